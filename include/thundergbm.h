@@ -153,6 +153,20 @@ int tgbm_predict_raw(int n_rows, const float *val, const int *row_ptr, const int
 int tgbm_predict_raw_timed(int n_rows, const float *val, const int *row_ptr, const int *col, const void *nodes, int n_rounds,
                      int trees_per_round, int n_nodes, float learning_rate, float base_score, float *out, float *kernel_ms);
 
+/* sparse_train_scikit / sparse_predict_scikit on a row-major matrix of floats (is_f64 = 0) or doubles (is_f64 = 1) in host
+ * memory, n_rows x n_cols with n_rows * n_cols < 2^31.  A zero is not stored, as in the CSR scipy.sparse.csr_matrix makes of
+ * the matrix: results are those of the two functions above on that CSR, which is made on the GPU. */
+void dense_train_scikit(int row_size, int n_cols, void *x, int is_f64, float *label, int depth, int n_trees,
+                        int n_device, float min_child_weight, float lambda, float gamma, int max_num_bin, int verbose,
+                        float column_sampling_rate, int bagging, int n_parallel_trees, float learning_rate,
+                        char *obj_type, int *num_class, char *tree_method, Tree **model, int *tree_per_iter,
+                        float *group_label, int *group, int num_group);
+void dense_predict_scikit(int row_size, int n_cols, void *x, int is_f64, float *y_pred, Tree **model,
+                          int n_trees, int trees_per_iter, char *objective, int num_class, float learning_rate,
+                          float *group_label, int verbose);
+/* number of distinct values (every NaN counts, +0 and -0 are one): the labels a group_label buffer must have room for */
+int tgbm_count_distinct(const float *v, long long n);
+
 /* Metric::get_score of the objective's default metric (the .cu files under src/thundergbm/metric, rank_metric.cpp) on raw scores
  * raw[t * n_rows + i]: RMSE, binary error, multi-class accuracy, MAP or NDCG.  `label` holds class indices for the
  * classification objectives.  Host pointers; device buffers and reduction scratch are allocated inside. */

@@ -15,6 +15,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "tgbm_input.h"
 #include "tgbm_kernels.cuh"
 #include "tgbm_hist_f32.cuh"
 #include "tgbm_exact.cuh"
@@ -44,8 +45,7 @@ struct BoosterImpl {
     std::vector<int> h_cut_ptr;
     std::vector<float> label;
 
-    DevBuf<int> d_row_ptr, d_col;  // the input CSR on the device, held from upload_csr() to the end of binning
-    DevBuf<float> d_val;
+    DeviceRows in;   // the stored values on the device, held from upload_rows() to the end of binning
     DevBuf<unsigned char> bins, binsT;
     // wide sparse data: CSR of global bin ids instead of the two dense matrices
     bool sparse = false;
@@ -131,7 +131,7 @@ struct BoosterImpl {
     }
 
     // ---------------------------------------------------------------- init helpers
-    void upload_csr(const DataSet &ds);
+    void upload_rows(const DataSet &ds);
     void find_cuts_and_bins(const DataSet &ds);
     // tree_method = exact (tgbm_exact.cuh)
     bool exact = false;
@@ -144,7 +144,7 @@ struct BoosterImpl {
     DevBuf<int> ex_pid_ptr, ex_nid, ex_any;
     DevBuf<unsigned long long> ex_best;
     DevBuf<unsigned char> ex_tmp;       // scratch of the radix sort and the scan by key
-    void init_exact(const DataSet &ds);
+    void init_exact();
     template <typename T> void exact_levels(int k, const void *gh_rows);
     void build_tree_exact(int round, int k);
     void column_builder_candidates(DevBuf<unsigned long long> &ukeys, DevBuf<long long> &ucopies, long long &nu);
@@ -157,37 +157,15 @@ struct BoosterImpl {
 
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
-// Host CSR -> device (asynchronous).  When the caller did not count the features (DataSet::n_features < 0) the largest
-// column index is found here, at HBM speed, instead of by a pass over the host copy.
-void BoosterImpl::upload_csr(const DataSet &ds) {
-    const size_t nnz = (size_t)ds.rp[N];
-    d_row_ptr.alloc(N + 1); d_col.alloc(std::max<size_t>(nnz, 1)); d_val.alloc(std::max<size_t>(nnz, 1));
-    // host threads that stage a pageable source (fewer per rank when the ranks of one process upload side by side)
-    const int up_threads = comm && comm->active() ? std::max(1, upload_threads() / comm->world) : upload_threads();
-    upload_h2d(d_row_ptr.p, ds.rp, sizeof(int) * (size_t)(N + 1), stream, up_threads);
-    upload_h2d(d_col.p, ds.ci, sizeof(int) * nnz, stream, up_threads);
-    upload_h2d(d_val.p, ds.vv, sizeof(float) * nnz, stream, up_threads);
-    // Largest and smallest column index, found here at HBM speed: the largest gives the feature count when the caller
-    // did not count (dataset.cpp:54-57), a negative one would send the binning kernels out of bounds.
-    const bool count_features = F < 0;
-    if (count_features) F = 1;
-    if (nnz) {
-        DevBuf<int> d_mm;
-        d_mm.alloc(2);
-        size_t tb = 0, tb2 = 0;
-        TGBM_CUDA(cub::DeviceReduce::Max(nullptr, tb, d_col.p, d_mm.p, (long long)nnz, stream));
-        TGBM_CUDA(cub::DeviceReduce::Min(nullptr, tb2, d_col.p, d_mm.p + 1, (long long)nnz, stream));
-        DevBuf<unsigned char> tmp;
-        tmp.alloc(std::max<size_t>(std::max(tb, tb2), 1));
-        TGBM_CUDA(cub::DeviceReduce::Max(tmp.p, tb, d_col.p, d_mm.p, (long long)nnz, stream));
-        TGBM_CUDA(cub::DeviceReduce::Min(tmp.p, tb2, d_col.p, d_mm.p + 1, (long long)nnz, stream));
-        int h_mm[2] = {0, 0};
-        TGBM_CUDA(cudaMemcpyAsync(h_mm, d_mm.p, sizeof(h_mm), cudaMemcpyDeviceToHost, stream));
-        TGBM_CUDA(cudaStreamSynchronize(stream));
-        TGBM_CHECK(h_mm[1] >= 0, "negative column index in the CSR input");
-        if (count_features) F = h_mm[0] + 1;
-        else TGBM_CHECK(h_mm[0] < F, "column index beyond the feature count");
-    }
+void BoosterImpl::upload_rows(const DataSet &ds) {
+    // fewer threads per rank when the ranks of one process upload side by side
+    in.upload(ds, stream, num_sms, comm && comm->active() ? std::max(1, upload_threads() / comm->world) : upload_threads());
+    nnz_local = (long long)in.nnz;
+    // the largest column gives the feature count when the caller did not count (dataset.cpp:54-57), a negative one would
+    // send the binning kernels out of bounds
+    TGBM_CHECK(in.min_col >= 0, "negative column index in the CSR input");
+    if (F < 0) F = std::max(1, in.max_col + 1);
+    else TGBM_CHECK(in.max_col < F, "column index beyond the feature count");
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -299,8 +277,9 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
         fprintf(stderr, "[tgbm init] %-28s %8.1f ms\n", what, std::chrono::duration<double, std::milli>(t - t_prev).count());
         t_prev = t;
     };
-    const size_t nnz = (size_t)ds.rp[N];
-    lap("H2D of the CSR");
+    const size_t nnz = (size_t)nnz_local;
+    (void)ds;
+    lap("H2D of the rows");
     long long nu = 0;
     DevBuf<unsigned long long> ukeys;
     const bool multi = comm && comm->active();
@@ -357,7 +336,7 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
         };
         if (local_err.empty()) {
             try {
-                if (nnz) k_make_keys<<<std::min(ceil_div(nnz, 256), num_sms * 16), 256, 0, stream>>>(d_val.p, d_col.p, nnz, keys.p);
+                if (nnz) k_make_keys<<<std::min(ceil_div(nnz, 256), num_sms * 16), 256, 0, stream>>>(in.val.p, in.col.p, in.full_cols, nnz, keys.p);
                 if (nnz && colb) k_fill_ll<<<std::min(ceil_div(nnz, 256), num_sms * 16), 256, 0, stream>>>(copies.p, nnz, 1);
                 nu = sort_unique(nnz);
             } catch (const std::exception &e) { local_err = e.what(); }
@@ -494,12 +473,12 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
         }
         TGBM_CHECK(sparse || (long long)F * 32 <= (1 << 21), "the dense bin matrix supports at most 65536 features");
     }
-    nnz_local = (long long)nnz;
     if (sparse) {
+        in.need_csr(N, stream, num_sms);
         sp_row_ptr.alloc(N + 1);
         sp_bin.alloc(std::max<size_t>(nnz, 1));
-        TGBM_CUDA(cudaMemcpyAsync(sp_row_ptr.p, d_row_ptr.p, sizeof(int) * (N + 1), cudaMemcpyDeviceToDevice, stream));
-        if (nnz) k_bin_csr<<<std::min(ceil_div(nnz, 256), num_sms * 16), 256, 0, stream>>>(d_col.p, d_val.p, nnz, cut_ptr.p, cut_val.p, sp_bin.p, colb ? 1 : 0);
+        TGBM_CUDA(cudaMemcpyAsync(sp_row_ptr.p, in.row_ptr.p, sizeof(int) * (N + 1), cudaMemcpyDeviceToDevice, stream));
+        if (nnz) k_bin_csr<<<std::min(ceil_div(nnz, 256), num_sms * 16), 256, 0, stream>>>(in.col.p, in.val.p, nnz, cut_ptr.p, cut_val.p, sp_bin.p, colb ? 1 : 0);
         // rows whose columns arrive unordered are put in ascending bin order (= ascending column order)
         if (nnz) {
             DevBuf<int> unsorted;
@@ -541,11 +520,11 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
         binsT.alloc((size_t)F * Npad);
         TGBM_CUDA(cudaMemsetAsync(bins.p, MISSING_BIN, bins.bytes(), stream));
         TGBM_CUDA(cudaMemsetAsync(binsT.p, MISSING_BIN, binsT.bytes(), stream));
-        if (N) k_bin_dense<<<ceil_div(N, 128), 128, 0, stream>>>(d_row_ptr.p, d_col.p, d_val.p, N, cut_ptr.p, cut_val.p, Fpad, Npad, bins.p, binsT.p, colb ? 1 : 0);
+        if (N) k_bin_dense<<<ceil_div(N, 128), 128, 0, stream>>>(in.row_ptr.p, in.col.p, in.val.p, in.full_cols, N, cut_ptr.p, cut_val.p, Fpad, Npad, bins.p, binsT.p, colb ? 1 : 0);
     }
     TGBM_CUDA(cudaStreamSynchronize(stream));
     TGBM_CUDA(cudaGetLastError());
-    d_row_ptr.release(); d_col.release(); d_val.release();
+    in.release();
     lap("binning");
 }
 
@@ -553,8 +532,9 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
 // Exact builder, set-up: the stored values by column, largest first (SparseColumns::csr2csc_gpu,
 // src/thundergbm/sparse_columns.cu:20-93 and :127) -- one stable radix sort of (column, complement of the value's ordered
 // image) keys with the row ids as payload -- and the buffers of the level loop, sized once.
-void BoosterImpl::init_exact(const DataSet &ds) {
-    const size_t nnz = (size_t)ds.rp[N];
+void BoosterImpl::init_exact() {
+    const size_t nnz = (size_t)nnz_local;
+    in.need_csr(N, stream, num_sms);
     ex_nnz = (long long)nnz;
     TGBM_CHECK(nnz < (1ull << 31), "the exact builder indexes stored values with 32 bits");
     TGBM_CHECK((double)F * (double)(1 << std::max(0, depth - 1)) < 4294967295.0, "columns x nodes of the last level must fit 32 bits");
@@ -564,8 +544,8 @@ void BoosterImpl::init_exact(const DataSet &ds) {
         DevBuf<unsigned long long> keys, keys2;
         DevBuf<int> rows;
         keys.alloc(n1); keys2.alloc(n1); rows.alloc(n1); ex_row.alloc(n1); ex_val.alloc(n1); ex_csc_ptr.alloc(F + 1);
-        if (N) k_exact_rows<<<std::min(ceil_div(N, 256), num_sms * 16), 256, 0, stream>>>(d_row_ptr.p, N, rows.p);
-        if (nnz) k_exact_csc_keys<<<grid, 256, 0, stream>>>(d_val.p, d_col.p, nnz, keys.p);
+        if (N) k_exact_rows<<<std::min(ceil_div(N, 256), num_sms * 16), 256, 0, stream>>>(in.row_ptr.p, N, rows.p);
+        if (nnz) k_exact_csc_keys<<<grid, 256, 0, stream>>>(in.val.p, in.col.p, nnz, keys.p);
         int end_bit = 32;
         while ((1ll << (end_bit - 32)) < F && end_bit < 64) ++end_bit;
         if (nnz) {
@@ -580,7 +560,7 @@ void BoosterImpl::init_exact(const DataSet &ds) {
         k_feature_bounds<<<ceil_div(F + 1, 128), 128, 0, stream>>>(keys2.p, (long long)nnz, F, ex_csc_ptr.p);
         TGBM_CUDA(cudaStreamSynchronize(stream));
     }
-    d_row_ptr.release(); d_col.release(); d_val.release();
+    in.release();
     // no cut points, no bin matrix
     B = 0; sparse = false;
     h_cut_ptr.assign(F + 1, 0);
@@ -718,7 +698,7 @@ void Booster::init(const DataSet &ds) {
     DevBuf<long long> mine, all;
     locally([&] {
         if (need_group_file(m.objective)) RankState::validate(ds, m.N);
-        m.upload_csr(ds);
+        m.upload_rows(ds);
         if (multi) { mine.alloc(3); all.alloc(3 * (size_t)m.comm->world); }
     });
     agree("loading its rows");
@@ -777,7 +757,7 @@ void Booster::init(const DataSet &ds) {
     m.exact = p.tree_method == "exact";
     if (m.exact) {
         TGBM_CHECK(!multi, "the exact builder runs on one GPU");
-        locally([&] { m.init_exact(ds); });
+        locally([&] { m.init_exact(); });
         agree("sorting its columns");
     } else {
         m.find_cuts_and_bins(ds);

@@ -81,6 +81,18 @@ std::vector<std::vector<Tree>> train_model(GBMParam &param, const DataSet &ds);
 // kernel_ms (optional): device time of the traversal kernel alone
 void predict_raw(const DataSet &ds, const std::vector<std::vector<Tree>> &model, float learning_rate, float base_score,
                  std::vector<float> &out, float *kernel_ms = nullptr);
+// The same on a model laid out for the GPU beforehand (kept with a model handle: nodes are not read again), followed by
+// the objective's predict_transform (OBJ_UNKNOWN: raw scores).  out: n_rows x trees_per_round floats, n_rows for multi:softmax.
+struct ModelRef {
+    int n_rounds = 0, K = 0, n_nodes = 0;
+    std::vector<const TreeNode *> trees;   // [round * K + class], n_nodes records each
+};
+class PredictPlan;
+std::shared_ptr<PredictPlan> make_predict_plan(const ModelRef &m);
+bool predict_plan_fits(const PredictPlan &plan, int n_rounds, int K);   // ... and is on the current device
+void predict(const DataSet &ds, PredictPlan &plan, float learning_rate, float base_score, int objective, const std::vector<float> &label,
+             float *out, float *kernel_ms = nullptr);
+void predict_release_workspaces() noexcept;
 // ObjectiveFunction::predict_transform on raw scores (in place; may shrink `y`)
 void predict_transform(int objective, int num_class, const std::vector<float> &label, int n_rows, std::vector<float> &y);
 // Metric::get_score on raw scores of `ds`

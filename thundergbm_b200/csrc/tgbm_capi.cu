@@ -4,6 +4,7 @@
 #include <climits>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -13,7 +14,11 @@
 #include "tgbm_device.cuh"
 
 // the opaque C handle is the C++ tree container
-struct Tree : tgbm::Tree {};
+struct Tree : tgbm::Tree {
+    // first tree of a model: the model as the prediction kernels want it, made by its first prediction (the trees behind
+    // a handle never change) and freed with it
+    std::shared_ptr<tgbm::PredictPlan> plan;
+};
 struct TgbmComm { tgbm::Comm *c; };
 struct TgbmBooster {
     tgbm::Booster *b = nullptr;
@@ -49,11 +54,28 @@ std::vector<std::vector<tgbm::Tree>> wrap_model(::Tree *model, int n_trees, int 
     return m;
 }
 
-::Tree *unwrap_model(const std::vector<std::vector<tgbm::Tree>> &m) {
+// the prediction plan of a model handle
+std::shared_ptr<tgbm::PredictPlan> plan_of(::Tree *model, int n_trees, int per_iter) {
+    TGBM_CHECK(model != nullptr, "model is null!");
+    static std::mutex m;   // one plan is made at a time; a prediction that finds one only copies the pointer
+    std::lock_guard<std::mutex> lock(m);
+    if (model->plan && tgbm::predict_plan_fits(*model->plan, n_trees, per_iter)) return model->plan;
+    tgbm::ModelRef ref;
+    ref.n_rounds = n_trees; ref.K = per_iter;
+    for (int i = 0; i < n_trees * per_iter; ++i) {
+        if (i == 0) ref.n_nodes = (int)model[0].nodes.size();
+        TGBM_CHECK((int)model[i].nodes.size() == ref.n_nodes, "ragged model");
+        ref.trees.push_back(model[i].nodes.data());
+    }
+    model->plan = tgbm::make_predict_plan(ref);
+    return model->plan;
+}
+
+::Tree *unwrap_model(std::vector<std::vector<tgbm::Tree>> &&m) {
     const size_t per = m.empty() ? 0 : m[0].size();
     ::Tree *out = new ::Tree[std::max<size_t>(1, m.size() * per)];
     for (size_t i = 0; i < m.size(); ++i)
-        for (size_t j = 0; j < per; ++j) out[i * per + j].nodes = m[i][j].nodes;
+        for (size_t j = 0; j < per; ++j) out[i * per + j].nodes = std::move(m[i][j].nodes);
     return out;
 }
 
@@ -158,11 +180,16 @@ std::vector<std::vector<tgbm::Tree>> train_in_process(tgbm::GBMParam &p, const t
                 tgbm::DataSet shard;
                 shard.n_rows = hi - lo;
                 shard.n_features = ds.n_features;
-                shard.row_ptr.resize(hi - lo + 1);
-                for (int i = lo; i <= hi; ++i) shard.row_ptr[i - lo] = ds.rp[i] - ds.rp[lo];
-                shard.rp = shard.row_ptr.data();
-                shard.ci = ds.ci + ds.rp[lo];
-                shard.vv = ds.vv + ds.rp[lo];
+                if (ds.dense) {
+                    shard.dense = static_cast<const char *>(ds.dense) + (size_t)lo * ds.dense_cols * (ds.dense_f64 ? 8 : 4);
+                    shard.dense_cols = ds.dense_cols; shard.dense_f64 = ds.dense_f64;
+                } else {
+                    shard.row_ptr.resize(hi - lo + 1);
+                    for (int i = lo; i <= hi; ++i) shard.row_ptr[i - lo] = ds.rp[i] - ds.rp[lo];
+                    shard.rp = shard.row_ptr.data();
+                    shard.ci = ds.ci + ds.rp[lo];
+                    shard.vv = ds.vv + ds.rp[lo];
+                }
                 const float *labels = ds.yv ? ds.yv : ds.y.data();
                 shard.yv = labels ? labels + lo : nullptr;
                 shard.labels_raw = ds.labels_raw;
@@ -247,6 +274,50 @@ tgbm::GBMParam param_from_c(const TgbmParam *cp) {
     p.tree_method = cp->exact_builder ? "exact" : "hist";
     return p;
 }
+
+// sparse_train_scikit / dense_train_scikit; `load` fills the data set from the caller's arrays
+template <typename Load>
+void train_scikit(Load &&load, int depth, int n_trees, int n_device, float min_child_weight, float lambda, float gamma, int max_num_bin,
+                  int verbose, float column_sampling_rate, int bagging, int n_parallel_trees, float learning_rate, char *obj_type,
+                  int *num_class, char *tree_method, ::Tree **model, int *tree_per_iter, float *group_label) {
+    if (model) *model = nullptr;
+    guard([&] {
+        tgbm::GBMParam p;
+        p.depth = depth; p.n_trees = n_trees; p.n_device = n_device; p.min_child_weight = min_child_weight;
+        p.lambda = lambda; p.gamma = gamma; p.max_num_bin = max_num_bin; p.verbose = verbose;
+        p.column_sampling_rate = column_sampling_rate; p.bagging = bagging != 0; p.n_parallel_trees = n_parallel_trees;
+        p.learning_rate = learning_rate; p.objective = obj_type; p.num_class = *num_class; p.tree_method = tree_method;
+        p.rt_eps = 1e-6f; p.tree_per_rounds = 1;
+        p.hist_mode = tgbm::default_hist_mode();
+        tgbm::set_verbosity(verbose);
+        TGBM_CHECK(n_device >= 1, "n_device must be at least 1");
+        tgbm::DataSet ds;
+        load(ds, p);
+        tgbm::log_info("#instances = %d", ds.n_rows);
+        *num_class = p.num_class;
+        auto m = tgbm::train_model(p, ds);
+        *num_class = p.num_class;
+        *tree_per_iter = m.empty() ? 1 : (int)m[0].size();
+        TGBM_CHECK((int)m.size() == n_trees, "trained fewer rounds than requested");
+        *model = unwrap_model(std::move(m));
+        for (size_t i = 0; i < ds.label.size(); ++i) group_label[i] = ds.label[i];
+    });
+}
+
+template <typename View>
+void predict_scikit(View &&view, float *y_pred, ::Tree **model, int n_trees, int trees_per_iter, char *objective, int num_class,
+                    float learning_rate, float *group_label, int verbose) {
+    guard([&] {
+        tgbm::DataSet ds;
+        view(ds);
+        tgbm::set_verbosity(verbose);
+        std::vector<float> label;
+        if (group_label) label.assign(group_label, group_label + std::max(0, num_class));
+        TGBM_CHECK(model && *model, "model is null!");
+        // base_score: never set on this path, scikit_tgbm.cpp:87-90
+        tgbm::predict(ds, *plan_of(*model, n_trees, trees_per_iter), learning_rate, 0.f, tgbm::objective_from_name(objective), label, y_pred);
+    });
+}
 }  // namespace
 
 namespace tgbm {
@@ -287,48 +358,34 @@ void sparse_train_scikit(int row_size, float *val, int *row_ptr, int *col_ptr, f
                          float column_sampling_rate, int bagging, int n_parallel_trees, float learning_rate,
                          char *obj_type, int *num_class, char *tree_method, ::Tree **model, int *tree_per_iter,
                          float *group_label, int *group, int num_group) {
-    if (model) *model = nullptr;
-    guard([&] {
-        tgbm::GBMParam p;
-        p.depth = depth; p.n_trees = n_trees; p.n_device = n_device; p.min_child_weight = min_child_weight;
-        p.lambda = lambda; p.gamma = gamma; p.max_num_bin = max_num_bin; p.verbose = verbose;
-        p.column_sampling_rate = column_sampling_rate; p.bagging = bagging != 0; p.n_parallel_trees = n_parallel_trees;
-        p.learning_rate = learning_rate; p.objective = obj_type; p.num_class = *num_class; p.tree_method = tree_method;
-        p.rt_eps = 1e-6f; p.tree_per_rounds = 1;
-        p.hist_mode = tgbm::default_hist_mode();
-        set_logger(verbose);
-        TGBM_CHECK(n_device >= 1, "n_device must be at least 1");
-        tgbm::DataSet ds;
-        ds.load_from_sparse(row_size, val, row_ptr, col_ptr, label, group, num_group, p, /*lazy=*/true);
-        tgbm::log_info("#instances = %d", ds.n_rows);
-        *num_class = p.num_class;
-        auto m = tgbm::train_model(p, ds);
-        *num_class = p.num_class;
-        *tree_per_iter = m.empty() ? 1 : (int)m[0].size();
-        TGBM_CHECK((int)m.size() == n_trees, "trained fewer rounds than requested");
-        *model = unwrap_model(m);
-        for (size_t i = 0; i < ds.label.size(); ++i) group_label[i] = ds.label[i];
-    });
+    train_scikit([&](tgbm::DataSet &ds, tgbm::GBMParam &p) { ds.load_from_sparse(row_size, val, row_ptr, col_ptr, label, group, num_group, p, /*lazy=*/true); },
+                 depth, n_trees, n_device, min_child_weight, lambda, gamma, max_num_bin, verbose, column_sampling_rate, bagging, n_parallel_trees,
+                 learning_rate, obj_type, num_class, tree_method, model, tree_per_iter, group_label);
+}
+
+void dense_train_scikit(int row_size, int n_cols, void *x, int is_f64, float *label, int depth, int n_trees,
+                        int n_device, float min_child_weight, float lambda, float gamma, int max_num_bin, int verbose,
+                        float column_sampling_rate, int bagging, int n_parallel_trees, float learning_rate,
+                        char *obj_type, int *num_class, char *tree_method, ::Tree **model, int *tree_per_iter,
+                        float *group_label, int *group, int num_group) {
+    train_scikit([&](tgbm::DataSet &ds, tgbm::GBMParam &p) { ds.load_from_dense(row_size, n_cols, x, is_f64 != 0, label, group, num_group, p); },
+                 depth, n_trees, n_device, min_child_weight, lambda, gamma, max_num_bin, verbose, column_sampling_rate, bagging, n_parallel_trees,
+                 learning_rate, obj_type, num_class, tree_method, model, tree_per_iter, group_label);
 }
 
 void sparse_predict_scikit(int row_size, float *val, int *row_ptr, int *col_ptr, float *y_pred, ::Tree **model,
                            int n_trees, int trees_per_iter, char *objective, int num_class, float learning_rate,
                            float *group_label, int *group, int num_group, int verbose) {
-    guard([&] {
-        tgbm::GBMParam p;
-        p.objective = objective; p.learning_rate = learning_rate; p.num_class = num_class;
-        tgbm::DataSet ds;
-        ds.load_from_sparse(row_size, val, row_ptr, col_ptr, nullptr, group, num_group, p);
-        set_logger(verbose);
-        ds.label.clear();
-        if (group_label) for (int i = 0; i < num_class; ++i) ds.label.push_back(group_label[i]);
-        TGBM_CHECK(model && *model, "model is null!");
-        auto m = wrap_model(*model, n_trees, trees_per_iter);
-        std::vector<float> y;
-        tgbm::predict_raw(ds, m, learning_rate, /*base_score: never set on this path, scikit_tgbm.cpp:87-90*/ 0.f, y);
-        tgbm::predict_transform(tgbm::objective_from_name(p.objective), num_class, ds.label, row_size, y);
-        std::copy(y.begin(), y.end(), y_pred);
-    });
+    (void)group; (void)num_group;
+    predict_scikit([&](tgbm::DataSet &ds) { ds.view_sparse(row_size, val, row_ptr, col_ptr); }, y_pred, model, n_trees, trees_per_iter,
+                   objective, num_class, learning_rate, group_label, verbose);
+}
+
+void dense_predict_scikit(int row_size, int n_cols, void *x, int is_f64, float *y_pred, ::Tree **model,
+                          int n_trees, int trees_per_iter, char *objective, int num_class, float learning_rate,
+                          float *group_label, int verbose) {
+    predict_scikit([&](tgbm::DataSet &ds) { ds.view_dense(row_size, n_cols, x, is_f64 != 0); }, y_pred, model, n_trees, trees_per_iter,
+                   objective, num_class, learning_rate, group_label, verbose);
 }
 
 void save(char *model_path, char *objective, float learning_rate, int num_class, int n_trees, int trees_per_iter,
@@ -355,7 +412,7 @@ void load_model(char *model_path, float *learning_rate, int *num_class, int *n_t
         *learning_rate = p.learning_rate; *num_class = p.num_class; *n_trees = p.n_trees;
         *trees_per_iter = m.empty() ? 1 : (int)m[0].size();
         TGBM_CHECK((int)m.size() == *n_trees, "model file: n_trees does not match the number of rounds stored");
-        *model = unwrap_model(m);
+        *model = unwrap_model(std::move(m));
     });
 }
 
@@ -558,7 +615,12 @@ void tgbm_booster_free(TgbmBooster *b) {
     delete b;
     tgbm::dev_trim();
 }
-void tgbm_release_device_memory(void) { tgbm::dev_release_all(); }
+void tgbm_release_device_memory(void) {
+    tgbm::predict_release_workspaces();
+    tgbm::dev_release_all();
+}
+
+int tgbm_count_distinct(const float *v, long long n) { return (int)tgbm::count_distinct(v, n); }
 
 int tgbm_metric_score(const char *objective, int n_rows, int trees_per_round, const float *label, const float *raw,
                       const int *group, int num_group, float *out) {
@@ -585,21 +647,14 @@ int tgbm_predict_raw(int n_rows, const float *val, const int *row_ptr, const int
 int tgbm_predict_raw_timed(int n_rows, const float *val, const int *row_ptr, const int *col, const void *nodes, int n_rounds,
                            int trees_per_round, int n_nodes, float learning_rate, float base_score, float *out, float *kernel_ms) {
     return guard([&] {
-        tgbm::GBMParam p;
         tgbm::DataSet ds;
-        ds.load_from_sparse(n_rows, val, row_ptr, col, nullptr, nullptr, 0, p);
+        ds.view_sparse(n_rows, val, row_ptr, col);
+        tgbm::ModelRef ref;
+        ref.n_rounds = n_rounds; ref.K = trees_per_round; ref.n_nodes = n_nodes;
         const tgbm::TreeNode *src = (const tgbm::TreeNode *)nodes;
-        std::vector<std::vector<tgbm::Tree>> m(n_rounds);
-        for (int r = 0; r < n_rounds; ++r) {
-            m[r].resize(trees_per_round);
-            for (int t = 0; t < trees_per_round; ++t) {
-                const tgbm::TreeNode *s = src + ((size_t)r * trees_per_round + t) * n_nodes;
-                m[r][t].nodes.assign(s, s + n_nodes);
-            }
-        }
-        std::vector<float> y;
-        tgbm::predict_raw(ds, m, learning_rate, base_score, y, kernel_ms);
-        std::copy(y.begin(), y.end(), out);
+        for (size_t t = 0; t < (size_t)n_rounds * trees_per_round; ++t) ref.trees.push_back(src + t * n_nodes);
+        if (n_rows == 0) return;
+        tgbm::predict(ds, *tgbm::make_predict_plan(ref), learning_rate, base_score, tgbm::OBJ_UNKNOWN, {}, out, kernel_ms);
     });
 }
 

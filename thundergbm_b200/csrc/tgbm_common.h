@@ -120,6 +120,11 @@ struct DataSet {
     // reference's copies) or pointing into the owned vectors below (load_from_file)
     const int *rp = nullptr, *ci = nullptr;
     const float *vv = nullptr;
+    // ... or, instead of a CSR, a borrowed row-major matrix of n_rows x dense_cols floats or doubles whose zeros are not
+    // stored (what scipy.sparse.csr_matrix makes of it); rp, ci and vv are null then
+    const void *dense = nullptr;
+    int dense_cols = 0;
+    bool dense_f64 = false;
     std::vector<int> row_ptr, col;
     std::vector<float> val, y;
     std::vector<int> group;
@@ -133,12 +138,20 @@ struct DataSet {
     // the device after the upload) and the labels are borrowed instead of copied.
     void load_from_sparse(int n, const float *v, const int *rp, const int *ci, const float *yy, const int *grp,
                           int num_group, GBMParam &param, bool lazy = false);
+    // rows to predict: a view of the caller's arrays, no labels, features not counted
+    void view_sparse(int n, const float *v, const int *rp, const int *ci);
+    void view_dense(int n, int cols, const void *x, bool f64);
+    // the same for a dense matrix (always lazy)
+    void load_from_dense(int n, int cols, const void *x, bool f64, const float *yy, const int *grp, int num_group, GBMParam &param);
+    void take_labels(const float *yy, const int *grp, int num_group, GBMParam &param, bool lazy);
     void distinct_labels(const float *yy, size_t n);
     int count_features() const;   // largest column index + 1, scanned by a few host threads
     void load_from_file(const std::string &file, GBMParam &param);
     void load_group_file(const std::string &file);
     void group_label();
 };
+
+long long count_distinct(const float *v, long long n);   // every NaN counts, +0 and -0 are one value
 
 // logging (verbosity as in set_logger: 0 silent, 1 info, 2 debug)
 void set_verbosity(int v);

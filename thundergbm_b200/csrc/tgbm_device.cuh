@@ -25,6 +25,12 @@ void dev_release_all() noexcept;
 // host -> device copy that also runs at the speed of the link when the source is pageable memory (then it returns
 // when the data is on the device; from page-locked memory it is cudaMemcpyAsync on `stream`)
 void upload_h2d(void *dst, const void *src, size_t bytes, cudaStream_t stream, int n_threads);
+// The values of a CSR, the same way; true when every row stores the columns 0 .. n_cols - 1 in order (a dense matrix handed
+// over as CSR): the column ids and row pointers then say nothing and need not follow.  They are checked by the host threads
+// while the values are copied: reading them costs less than sending them (half of the bytes of such a CSR).
+bool upload_csr_values(float *dst, const float *val, const int *row_ptr, const int *col, int n_rows, int n_cols, cudaStream_t stream, int n_threads);
+// device -> host copy, the same way; the data is there when it returns
+void download_d2h(void *dst, const void *src, size_t bytes, cudaStream_t stream, int n_threads);
 int upload_threads();   // host threads one upload may use: TGBM_UPLOAD_THREADS, else half of the cores, at most 8
 
 // RAII device buffer; everything is allocated once at init and reused for every tree.
@@ -45,6 +51,11 @@ struct DevBuf {
         release();
         n = count;
         if (count) p = static_cast<T *>(dev_alloc(sizeof(T) * count));
+    }
+    void take(DevBuf &o) {
+        release();
+        p = o.p; n = o.n;
+        o.p = nullptr; o.n = 0;
     }
     void zero(cudaStream_t s) {
         if (n) TGBM_CUDA(cudaMemsetAsync(p, 0, sizeof(T) * n, s));

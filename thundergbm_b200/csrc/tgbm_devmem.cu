@@ -18,8 +18,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <condition_variable>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
+#include <functional>
 #include <iterator>
 #include <map>
 #include <mutex>
@@ -164,16 +168,23 @@ static void trim_all(size_t keep, bool only_dirty) noexcept {
     if (cur >= 0) cudaSetDevice(cur);
 }
 
-// ---- large host -> device copies ---------------------------------------------------------------------------------
+// ---- copies between the device and pageable host memory ------------------------------------------------------------
 // cudaMemcpyAsync from pageable memory (what a NumPy caller hands over) is staged by the driver through one small
 // pinned buffer: 10.8 GB/s measured for the 2.4 GB of a Higgs-sized CSR, a fifth of what the link carries from pinned
-// memory (page-locking the caller's arrays in place with cudaHostRegister runs at 11 GB/s too).  upload_h2d does the staging itself: a few host threads copy 8 MB pieces into page-locked slots (two per
-// thread, kept for the next call) and send each slot on with cudaMemcpyAsync on the thread's own stream.  Page-locked
-// or registered sources, and small copies, go to cudaMemcpyAsync directly.
+// memory (page-locking the caller's arrays in place with cudaHostRegister runs at 11 GB/s too).  A few worker threads do
+// the staging instead: they copy pieces into page-locked slots (two per thread, kept for the next call) and send each
+// slot on with cudaMemcpyAsync on a stream of their own.  Page-locked or registered host memory, and copies of less than
+// STAGE_MIN bytes (which the driver finishes before the workers have woken up), go to cudaMemcpyAsync directly.
+//
+// The workers outlive a call: starting eight threads with a stream and two events each cost 0.6-1 ms per upload.  At
+// most WORKERS of them exist; several calling threads share them, a call that finds all of them busy waits.
 namespace {
 
-constexpr size_t STAGE_BYTES = 8u << 20;
-constexpr int STAGE_KEEP = 16;   // slots that stay allocated between calls (128 MB)
+constexpr size_t STAGE_BYTES = 8u << 20;       // size of a slot and largest piece
+constexpr size_t STAGE_PIECE_MIN = 256u << 10; // smallest piece
+constexpr size_t STAGE_MIN = 1u << 20;
+constexpr int WORKERS = 8;
+constexpr int STAGE_KEEP = 2 * WORKERS;        // slots that stay allocated between calls (128 MB)
 
 std::mutex &g_stage_mutex = *new std::mutex;
 std::vector<void *> &g_stage_free = *new std::vector<void *>;
@@ -203,71 +214,215 @@ bool host_is_pageable(const void *p) {
     return attr.type == cudaMemoryTypeUnregistered;
 }
 
+void check_cuda(cudaError_t e, const char *what) {
+    if (e != cudaSuccess) { cudaGetLastError(); throw Error(std::string("CUDA error: ") + cudaGetErrorString(e) + " in " + what); }
+}
+
+// stream and events of one worker on one device
+struct Lane {
+    cudaStream_t st = nullptr;
+    cudaEvent_t done[2] = {nullptr, nullptr};
+};
+
+struct Worker {
+    Lane lanes[MAX_DEVICES];
+    Lane &lane(int dev) {
+        Lane &l = lanes[dev];
+        if (!l.st) {
+            check_cuda(cudaStreamCreateWithFlags(&l.st, cudaStreamNonBlocking), "cudaStreamCreate");
+            for (int k = 0; k < 2; ++k) check_cuda(cudaEventCreateWithFlags(&l.done[k], cudaEventDisableTiming), "cudaEventCreate");
+        }
+        return l;
+    }
+};
+
+class Pool {
+public:
+    // runs f(worker, t) for t = 0 .. n - 1 on the workers and returns when all have returned; f must not throw
+    void run(int n, const std::function<void(Worker &, int)> &f) {
+        Job job{&f, n};
+        std::unique_lock<std::mutex> lock(mutex_);
+        for (int t = 0; t < n; ++t) queue_.push_back({&job, t});
+        for (; started_ < WORKERS && idle_ + starting_ < (int)queue_.size(); ++started_, ++starting_) std::thread(&Pool::loop, this).detach();
+        wake_.notify_all();
+        done_.wait(lock, [&] { return job.left == 0; });
+    }
+
+private:
+    struct Job { const std::function<void(Worker &, int)> *f; int left; };
+    struct Task { Job *job; int t; };
+    void loop() {
+        Worker w;
+        std::unique_lock<std::mutex> lock(mutex_);
+        --starting_;
+        for (;;) {
+            ++idle_;
+            wake_.wait(lock, [&] { return !queue_.empty(); });
+            --idle_;
+            const Task task = queue_.front();
+            queue_.pop_front();
+            lock.unlock();
+            (*task.job->f)(w, task.t);
+            lock.lock();
+            if (--task.job->left == 0) done_.notify_all();
+        }
+    }
+    std::mutex mutex_;
+    std::condition_variable wake_, done_;
+    std::deque<Task> queue_;
+    int started_ = 0, starting_ = 0, idle_ = 0;
+};
+
+// never destroyed: the workers wait on it until the process ends
+Pool &pool() {
+    static Pool *p = new Pool;
+    return *p;
+}
+
+// One copy cut into pieces that the workers take in turn.  A worker fills one of its slots while the other is on its way.
+struct Transfer {
+    char *dev;                 // device side
+    char *host;                // host side (read when up, written when down)
+    size_t bytes, piece;
+    bool up;
+    std::atomic<size_t> next{0};
+    Transfer(void *d, const void *h, size_t n, bool up_, int workers)
+        : dev(static_cast<char *>(d)), host(static_cast<char *>(const_cast<void *>(h))), bytes(n), up(up_) {
+        piece = std::min(STAGE_BYTES, std::max(STAGE_PIECE_MIN, (n / ((size_t)workers * 4) + 65535) / 65536 * 65536));
+    }
+    void work(Lane &l, void *const slot[2]) {
+        struct Pending { size_t off, len; } pending[2] = {{0, 0}, {0, 0}};
+        auto finish = [&](int k) {
+            if (!pending[k].len) return;
+            check_cuda(cudaEventSynchronize(l.done[k]), "cudaEventSynchronize");
+            if (!up) memcpy(host + pending[k].off, slot[k], pending[k].len);
+            pending[k].len = 0;
+        };
+        for (int k = 0;; k ^= 1) {
+            const size_t off = next.fetch_add(piece);
+            if (off >= bytes) break;
+            const size_t len = std::min(piece, bytes - off);
+            finish(k);
+            if (up) {
+                memcpy(slot[k], host + off, len);
+                check_cuda(cudaMemcpyAsync(dev + off, slot[k], len, cudaMemcpyHostToDevice, l.st), "cudaMemcpyAsync");
+            } else {
+                check_cuda(cudaMemcpyAsync(slot[k], dev + off, len, cudaMemcpyDeviceToHost, l.st), "cudaMemcpyAsync");
+            }
+            check_cuda(cudaEventRecord(l.done[k], l.st), "cudaEventRecord");
+            pending[k] = {off, len};
+        }
+        for (int k = 0; k < 2; ++k) finish(k);
+    }
+};
+
+// runs the transfer on the workers; `side` (may be empty) is called by every worker first
+void run_staged(Transfer *tr, int n_threads, const std::function<void(int)> &side) {
+    int dev = 0;
+    TGBM_CUDA(cudaGetDevice(&dev));
+    TGBM_CHECK(dev >= 0 && dev < MAX_DEVICES, "device index out of range");
+    const int T = std::max(1, std::min(n_threads, WORKERS));
+    std::vector<std::string> errors(T);
+    pool().run(T, [&](Worker &w, int t) {
+        void *slot[2] = {nullptr, nullptr};
+        Lane *l = nullptr;
+        try {
+            if (tr) {
+                check_cuda(cudaSetDevice(dev), "cudaSetDevice");
+                l = &w.lane(dev);
+                for (auto &p : slot)
+                    if (!(p = stage_acquire())) throw Error("no page-locked memory for a copy");
+                tr->work(*l, slot);
+            }
+            if (side) side(t);
+        } catch (const std::exception &e) {
+            errors[t] = e.what();
+            if (l) cudaStreamSynchronize(l->st);   // nothing may still use the slots when they go back
+        }
+        for (void *p : slot) stage_release(p);
+    });
+    for (const auto &e : errors)
+        if (!e.empty()) throw Error(e);
+}
+
+bool staging_on() {
+    static const bool on = getenv("TGBM_NO_STAGED_UPLOAD") == nullptr;
+    return on;
+}
+
 }  // namespace
 
 int upload_threads() {
     static const int n = [] {
-        if (const char *e = getenv("TGBM_UPLOAD_THREADS")) return std::max(1, std::min(STAGE_KEEP / 2, atoi(e)));
+        if (const char *e = getenv("TGBM_UPLOAD_THREADS")) return std::max(1, std::min(WORKERS, atoi(e)));
         const int hw = (int)std::thread::hardware_concurrency();
-        return std::max(1, std::min(8, hw / 2));   // 16 cores: 4 / 6 / 8 threads bring 2.4 GB over in 100 / 82 / 65 ms, 12 and more in 0.2-1.2 s
+        return std::max(1, std::min(WORKERS, hw / 2));   // 16 cores: 4 / 6 / 8 threads bring 2.4 GB over in 100 / 82 / 65 ms, 12 and more in 0.2-1.2 s
     }();
     return n;
 }
 
 void upload_h2d(void *dst, const void *src, size_t bytes, cudaStream_t stream, int n_threads) {
     if (bytes == 0) return;
-    static const bool staged = getenv("TGBM_NO_STAGED_UPLOAD") == nullptr;
-    if (!staged || bytes < 4 * STAGE_BYTES || n_threads < 1 || !host_is_pageable(src)) {
+    if (!staging_on() || bytes < STAGE_MIN || n_threads < 1 || !host_is_pageable(src)) {
         TGBM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
         return;
     }
-    int dev = 0;
-    TGBM_CUDA(cudaGetDevice(&dev));
-    const size_t n_chunks = (bytes + STAGE_BYTES - 1) / STAGE_BYTES;
-    const int T = (int)std::min<size_t>((size_t)n_threads, n_chunks);
-    std::vector<std::string> errors(T);
-    std::vector<std::thread> workers;
-    for (int t = 0; t < T; ++t)
-        workers.emplace_back([&, t] {
-            void *slot[2] = {nullptr, nullptr};
-            cudaEvent_t done[2] = {nullptr, nullptr};
-            bool busy[2] = {false, false};
-            cudaStream_t st = nullptr;
-            auto check = [&](cudaError_t e, const char *what) {
-                if (e != cudaSuccess) { cudaGetLastError(); throw Error(std::string("CUDA error: ") + cudaGetErrorString(e) + " in " + what); }
-            };
-            try {
-                check(cudaSetDevice(dev), "cudaSetDevice");
-                check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
-                for (int k = 0; k < 2; ++k) {
-                    slot[k] = stage_acquire();
-                    if (!slot[k]) throw Error("no page-locked memory for the upload");
-                    check(cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming), "cudaEventCreate");
-                }
-                int k = 0;
-                for (size_t c = t; c < n_chunks; c += T, k ^= 1) {
-                    const size_t off = c * STAGE_BYTES, len = std::min(STAGE_BYTES, bytes - off);
-                    if (busy[k]) check(cudaEventSynchronize(done[k]), "cudaEventSynchronize");
-                    memcpy(slot[k], static_cast<const char *>(src) + off, len);
-                    check(cudaMemcpyAsync(static_cast<char *>(dst) + off, slot[k], len, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
-                    check(cudaEventRecord(done[k], st), "cudaEventRecord");
-                    busy[k] = true;
-                }
-                check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
-            } catch (const std::exception &e) {
-                errors[t] = e.what();
-                if (st) cudaStreamSynchronize(st);   // nothing may still read the slots when they go back
-            }
-            for (int k = 0; k < 2; ++k) {
-                if (done[k]) cudaEventDestroy(done[k]);
-                stage_release(slot[k]);
-            }
-            if (st) cudaStreamDestroy(st);
-        });
-    for (auto &w : workers) w.join();
-    for (const auto &e : errors)
-        if (!e.empty()) throw Error(e);
-    (void)stream;   // the pieces are on the device when the workers return: whatever is queued next sees them
+    Transfer tr(dst, src, bytes, true, n_threads);
+    run_staged(&tr, n_threads, {});   // the pieces are on the device when the workers return: whatever is queued next sees them
+}
+
+bool upload_csr_values(float *dst, const float *val, const int *row_ptr, const int *col, int n_rows, int n_cols, cudaStream_t stream, int n_threads) {
+    const size_t nnz = (size_t)row_ptr[n_rows], bytes = sizeof(float) * nnz;
+    // candidates: every row of equal length, first and last row complete
+    bool dense = n_rows > 0 && n_cols > 0 && nnz == (size_t)n_rows * (size_t)n_cols && row_ptr[0] == 0 && row_ptr[1] == n_cols;
+    auto row_ok = [&](int r) {
+        int bad = row_ptr[r] ^ (r * n_cols);
+        const int *c = col + (size_t)r * n_cols;
+        for (int j = 0; j < n_cols; ++j) bad |= c[j] ^ j;
+        return bad == 0;
+    };
+    dense = dense && row_ok(0) && row_ok(n_rows - 1);
+    const bool threads = staging_on() && n_threads >= 1 && bytes >= STAGE_MIN;
+    const bool staged = threads && host_is_pageable(val);
+    if (!staged && bytes) TGBM_CUDA(cudaMemcpyAsync(dst, val, bytes, cudaMemcpyHostToDevice, stream));
+    if (!dense && !staged) return false;
+    std::atomic<bool> ok{dense};
+    if (!threads) {
+        for (int r = 0; r < n_rows && ok; ++r) ok = row_ok(r);
+        return ok;
+    }
+    std::atomic<int> next{0};
+    const int rows = std::max(1, (64 << 10) / std::max(1, n_cols));
+    auto check_rows = [&](int) {   // the column ids are read while the values are on their way
+        for (;;) {
+            const long long r0 = (long long)next.fetch_add(1) * rows;
+            if (r0 >= n_rows || !ok) return;
+            const int r1 = (int)std::min<long long>(n_rows, r0 + rows);
+            for (int r = (int)r0; r < r1; ++r)
+                if (!row_ok(r)) { ok = false; return; }
+        }
+    };
+    std::function<void(int)> side;
+    if (dense) side = check_rows;
+    if (staged) {
+        Transfer tr(dst, val, bytes, true, n_threads);
+        run_staged(&tr, n_threads, side);
+    } else {
+        run_staged(nullptr, n_threads, side);
+    }
+    return ok;
+}
+
+void download_d2h(void *dst, const void *src, size_t bytes, cudaStream_t stream, int n_threads) {
+    if (bytes == 0) return;
+    if (!staging_on() || bytes < STAGE_MIN || n_threads < 1 || !host_is_pageable(dst)) {
+        TGBM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream));
+        TGBM_CUDA(cudaStreamSynchronize(stream));
+        return;
+    }
+    TGBM_CUDA(cudaStreamSynchronize(stream));   // what the workers read has been written
+    Transfer tr(const_cast<void *>(src), dst, bytes, false, n_threads);
+    run_staged(&tr, n_threads, {});
 }
 
 void dev_trim() noexcept { trim_all(keep_bytes(), true); }

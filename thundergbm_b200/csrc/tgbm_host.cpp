@@ -35,7 +35,38 @@ void DataSet::load_from_sparse(int n, const float *v, const int *rp, const int *
     TGBM_CHECK(nnz >= 0, "bad CSR row_ptr");
     n_rows = n;
     row_ptr.clear(); col.clear(); val.clear();
+    dense = nullptr; dense_cols = 0;
     this->rp = rp; this->ci = ci; this->vv = v;  // borrowed: the 2.4 GB of a Higgs-sized CSR are not copied on the host
+    // n_features = largest column index + 1 (dataset.cpp:54-57), scanned by a few threads
+    n_features = -1;
+    if (!lazy) n_features = count_features();
+    take_labels(yy, grp, num_group, param, lazy);
+}
+
+void DataSet::view_sparse(int n, const float *v, const int *rp_, const int *ci_) {
+    TGBM_CHECK(n >= 0 && rp_ != nullptr, "bad CSR input");
+    TGBM_CHECK(rp_[n] >= 0, "bad CSR row_ptr");
+    n_rows = n; n_features = -1;
+    dense = nullptr; dense_cols = 0;
+    rp = rp_; ci = ci_; vv = v;
+}
+
+void DataSet::view_dense(int n, int cols, const void *x, bool f64) {
+    TGBM_CHECK(n >= 0 && cols >= 0 && (x != nullptr || n == 0 || cols == 0), "bad dense input");
+    TGBM_CHECK((long long)n * cols < (1ll << 31), "rows x columns of a dense matrix must fit 31 bits");
+    n_rows = n; n_features = -1;
+    rp = nullptr; ci = nullptr; vv = nullptr;
+    dense = x; dense_cols = cols; dense_f64 = f64;
+}
+
+void DataSet::load_from_dense(int n, int cols, const void *x, bool f64, const float *yy, const int *grp, int num_group, GBMParam &param) {
+    view_dense(n, cols, x, f64);
+    row_ptr.clear(); col.clear(); val.clear();
+    take_labels(yy, grp, num_group, param, /*lazy=*/true);
+}
+
+void DataSet::take_labels(const float *yy, const int *grp, int num_group, GBMParam &param, bool lazy) {
+    const int n = n_rows;
     const bool borrow = lazy && yy != nullptr;
     y.clear();
     if (!borrow) { if (yy) y.assign(yy, yy + n); else y.assign(n, 0.f); }
@@ -43,9 +74,6 @@ void DataSet::load_from_sparse(int n, const float *v, const int *rp, const int *
     labels_raw = false;
     label.clear();
     group.clear();
-    // n_features = largest column index + 1 (dataset.cpp:54-57), scanned by a few threads
-    n_features = -1;
-    if (!lazy) n_features = count_features();
     const int o = objective_from_name(param.objective);
     if (yy && need_group_label(o)) {
         if (borrow) { distinct_labels(yy, (size_t)n); labels_raw = true; }
@@ -57,6 +85,17 @@ void DataSet::load_from_sparse(int n, const float *v, const int *rp, const int *
 }
 
 int DataSet::count_features() const {
+    if (dense) {   // last column that holds a non-zero: rows from the last column down, most matrices end at the first row
+        int m = -1;
+        auto scan = [&](auto *x) {
+            for (int r = 0; r < n_rows && m < dense_cols - 1; ++r)
+                for (int c = dense_cols - 1; c > m; --c)
+                    if (x[(size_t)r * dense_cols + c] != 0) { m = c; break; }
+        };
+        if (dense_f64) scan(static_cast<const double *>(dense));
+        else scan(static_cast<const float *>(dense));
+        return m + 1;
+    }
     const long long nnz = rp ? rp[n_rows] : 0;
     const int nt = (int)std::max<long long>(1, std::min<long long>(16, nnz / (1 << 22)));
     std::vector<int> part(nt, -1);
@@ -103,6 +142,52 @@ void DataSet::distinct_labels(const float *yy, size_t n) {
     t.erase(std::unique(t.begin(), t.end()), t.end());
     label.clear();
     for (int v : t) label.push_back((float)v);
+}
+
+long long count_distinct(const float *v, long long n) {
+    // few values are the rule (class labels): a short list first, an open hash table of bit patterns beyond it
+    float seen[16];
+    int ns = 0;
+    long long i = 0, nans = 0;
+    for (; i < n; ++i) {
+        const float x = v[i];
+        if (x != x) { ++nans; continue; }
+        bool hit = false;
+        for (int k = 0; k < ns; ++k) hit |= seen[k] == x;
+        if (hit) continue;
+        if (ns == 16) break;
+        seen[ns++] = x;
+    }
+    if (i == n) return ns + nans;
+    size_t cap = 1024, used = 0;
+    while (cap < (size_t)(2 * std::min<long long>(n, 1 << 24))) cap <<= 1;
+    constexpr uint32_t EMPTY = 0xffffffffu;   // a NaN pattern
+    std::vector<uint32_t> table(cap, EMPTY);
+    auto put = [&](float x) {
+        uint32_t u;
+        if (x == 0.f) x = 0.f;   // one zero
+        memcpy(&u, &x, 4);
+        size_t h = (size_t)((u * 0x9E3779B97F4A7C15ull) >> 32) & (cap - 1);
+        while (table[h] != EMPTY && table[h] != u) h = (h + 1) & (cap - 1);
+        if (table[h] == u) return;
+        table[h] = u;
+        if (++used * 4 <= cap * 3) return;
+        std::vector<uint32_t> old(cap * 2, EMPTY);
+        old.swap(table);
+        cap *= 2;
+        for (uint32_t w : old) {
+            if (w == EMPTY) continue;
+            size_t g = (size_t)((w * 0x9E3779B97F4A7C15ull) >> 32) & (cap - 1);
+            while (table[g] != EMPTY) g = (g + 1) & (cap - 1);
+            table[g] = w;
+        }
+    };
+    for (int k = 0; k < ns; ++k) put(seen[k]);
+    for (; i < n; ++i) {
+        if (v[i] != v[i]) ++nans;
+        else put(v[i]);
+    }
+    return (long long)used + nans;
 }
 
 void DataSet::group_label() {

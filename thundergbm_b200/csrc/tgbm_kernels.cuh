@@ -61,13 +61,15 @@ struct SplitRec {  // best candidate of one (node, feature)
 
 // ------------------------------------------------------------------ cut points
 // key = feature id in the high word, order-preserving image of the float in the low word
-static __global__ void k_make_keys(const float *__restrict__ val, const int *__restrict__ col, size_t nnz,
+static __global__ void k_make_keys(const float *__restrict__ val, const int *__restrict__ col, int full_cols, size_t nnz,
                             unsigned long long *__restrict__ keys) {
+    // full_cols > 0: a matrix without missing values, `col` is not read
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nnz; i += (size_t)gridDim.x * blockDim.x) {
         unsigned u = __float_as_uint(val[i]);
         if (u == 0x80000000u) u = 0;  // -0.0f == 0.0f
         u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-        keys[i] = ((unsigned long long)(unsigned)col[i] << 32) | u;
+        const unsigned c = full_cols ? (unsigned)i % (unsigned)full_cols : (unsigned)col[i];
+        keys[i] = ((unsigned long long)c << 32) | u;
     }
 }
 
@@ -193,12 +195,13 @@ __device__ __forceinline__ int bin_search_down(const float *__restrict__ cut_val
 // HistTreeBuilder_single::get_bin_ids (hist_tree_builder_single.cu:81-119): clamped upper bound,
 // bin = min(#cuts <= v, n_cuts - 1); stored as the feature-local id in both layouts
 static __global__ void k_bin_dense(const int *__restrict__ row_ptr, const int *__restrict__ col, const float *__restrict__ val,
-                            int n_rows, const int *__restrict__ cut_ptr, const float *__restrict__ cut_val, int Fpad,
+                            int full_cols, int n_rows, const int *__restrict__ cut_ptr, const float *__restrict__ cut_val, int Fpad,
                             size_t Npad, unsigned char *__restrict__ bins, unsigned char *__restrict__ binsT, int multi) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n_rows) return;
-    for (int j = row_ptr[r]; j < row_ptr[r + 1]; ++j) {
-        const int f = col[j];
+    const int j0 = full_cols ? r * full_cols : row_ptr[r], j1 = full_cols ? j0 + full_cols : row_ptr[r + 1];
+    for (int j = j0; j < j1; ++j) {
+        const int f = full_cols ? j - j0 : col[j];
         const float v = val[j];
         const int b0 = cut_ptr[f];
         int lo = b0, hi = cut_ptr[f + 1] - 1;

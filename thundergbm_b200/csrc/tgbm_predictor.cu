@@ -2,8 +2,12 @@
 // predict_transform and the metric the predict CLI logs.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <future>
+#include <mutex>
 
 #include "tgbm_booster.h"
+#include "tgbm_input.h"
 #include "tgbm_kernels.cuh"
 #include "tgbm_rank.cuh"
 
@@ -31,7 +35,7 @@ k_predict_dense(const int *__restrict__ row_ptr, const int *__restrict__ col, co
     if (i < n_rows)
         for (int j = row_ptr[i]; j < row_ptr[i + 1]; ++j) {
             const int c = col[j];
-            if (c < F) dense[c * PRED_ROWS + threadIdx.x] = val[j];
+            if (c >= 0 && c < F) dense[c * PRED_ROWS + threadIdx.x] = val[j];
         }
     if (i >= n_rows) return;
     for (int t = 0; t < K; ++t) {
@@ -371,35 +375,29 @@ k_rank_rows(const int *__restrict__ row_ptr, const int *__restrict__ col, const 
     }
 }
 
-// Rows that store every feature, columns in order (a dense matrix handed over as CSR): one thread per row reads its F
-// values with 16-byte loads, checks its row pointer and the column ids against 0 .. F-1 as it goes (any other row raises `not_dense` and
-// the caller falls back to the kernel above) and ranks each value by an eight-step descent through the feature's
+// Rows that store every feature, columns in order (a dense matrix, or one handed over as CSR: the host threads that copy
+// the values check that): one thread per row reads its F values with 16-byte loads and ranks each value by an eight-step descent through the feature's
 // thresholds laid out as an implicit search tree (level by level: the lanes of a warp, all on the same feature, touch
 // consecutive words).  No row search, no address arithmetic per value: ncu counted 130 warp instructions per value in the
 // kernel above.
 constexpr int RD_THREADS = 256;
 template <bool DENSE_PATH>
 __global__ void __launch_bounds__(RD_THREADS)
-k_rank_dense_rows(const int *__restrict__ row_ptr, const int *__restrict__ col, const float *__restrict__ val, int n_rows, int F, const float *__restrict__ tree_thr,
-                  const int *__restrict__ thr_ptr, unsigned char *__restrict__ bins, int *__restrict__ not_dense) {
+k_rank_dense_rows(const float *__restrict__ val, int n_rows, int F, const float *__restrict__ tree_thr, const int *__restrict__ thr_ptr,
+                  unsigned char *__restrict__ bins) {
     extern __shared__ float s_tree[];   // [F][256]: 255 thresholds of the feature in level order, padded with +inf
     __shared__ int s_n[32];
     for (int i = threadIdx.x; i < F * 256; i += RD_THREADS) s_tree[i] = tree_thr[i];
     if (threadIdx.x < F) s_n[threadIdx.x] = thr_ptr[threadIdx.x + 1] - thr_ptr[threadIdx.x];
     __syncthreads();
     const int F4 = F / 4;   // F is a multiple of 4 here
-    bool bad = false;
     for (int r = blockIdx.x * RD_THREADS + threadIdx.x; r < n_rows; r += gridDim.x * RD_THREADS) {
         const float4 *vp = reinterpret_cast<const float4 *>(val + (size_t)r * F);
-        const int4 *cp = reinterpret_cast<const int4 *>(col + (size_t)r * F);
-        bad |= row_ptr[r] != r * F;
         uint32_t out[8] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             if (q < F4) {
                 const float4 v4 = vp[q];
-                const int4 c4 = cp[q];
-                bad |= c4.x != 4 * q || c4.y != 4 * q + 1 || c4.z != 4 * q + 2 || c4.w != 4 * q + 3;
                 const float v[4] = {v4.x, v4.y, v4.z, v4.w};
                 uint32_t word = 0;
 #pragma unroll
@@ -421,7 +419,6 @@ k_rank_dense_rows(const int *__restrict__ row_ptr, const int *__restrict__ col, 
         dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
         dst[1] = make_uint4(out[4], out[5], out[6], out[7]);
     }
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) *not_dense = 1;
 }
 
 constexpr int PR_THREADS = 512;
@@ -628,298 +625,104 @@ k_predict_planes(const unsigned char *__restrict__ bins, int Fpad, int n_rows, c
     }
 }
 
-void predict_raw(const DataSet &ds, const std::vector<std::vector<Tree>> &model, float learning_rate, float base_score,
-                 std::vector<float> &out, float *kernel_ms) {
-    const int N = ds.n_rows;
-    const int n_rounds = (int)model.size();
-    TGBM_CHECK(n_rounds > 0 && !model[0].empty(), "empty model");
-    const int K = (int)model[0].size();
-    const int n_nodes = (int)model[0][0].nodes.size();
-    out.assign((size_t)N * K, 0.f);
-    if (N == 0) return;
-    if (K > 1) base_score = 0;  // predictor.cu:81-83
-    std::vector<PNode> flat((size_t)n_rounds * K * n_nodes);
-    for (int r = 0; r < n_rounds; ++r)
-        for (int t = 0; t < K; ++t) {
-            TGBM_CHECK((int)model[r].size() == K && (int)model[r][t].nodes.size() == n_nodes, "ragged model");
-            for (int n = 0; n < n_nodes; ++n) {
-                const TreeNode &s = model[r][t].nodes[n];
-                PNode &d = flat[((size_t)r * K + t) * n_nodes + n];
-                d.lch = s.lch_index; d.rch = s.rch_index;
-                if (s.is_leaf) { d.v = s.base_weight; d.fid = (int)0x80000000; }
-                else { d.v = s.split_value; d.fid = (s.split_feature_id & 0x3fffffff) | (s.default_right ? 0x40000000 : 0); }
+// ---- few rows: straight from the matrix ------------------------------------------------------------------------------
+// One launch from the caller's rows to the scores.  Preparing ranks (below) pays for millions of rows; a request of one to
+// a few hundred thousand rows is over sooner when every tree is walked on the floats themselves: a block spreads out
+// the features of 2^rt_log rows in shared memory ([feature][row], padded so that neither the rows' columns nor a column's
+// rows collide), its threads take (tree, row) pairs -- a warp's 32 rows walk one tree, with fewer rows the lanes spread
+// over trees -- and read the 8-byte nodes through L1.  The leaf values meet in shared memory, where one thread per (row,
+// class) adds them in ascending round order: the sums are those of the kernels above bit for bit.
+// Bound by latency for single rows (6 levels x one L2 access), by L1/L2 node reads for large batches:
+// 50003 rows x 54 features, 210 trees of depth 8: 0.2 ms; the rank path needs 0.1 ms more to prepare than to walk there.
+constexpr int PD_THREADS = 256;
+enum PredictInput { IN_CSR = 0, IN_F32 = 1, IN_F64 = 2, IN_FULL = 3 };  // FULL: every cell is stored (a zero is a value)
+struct RowsIn {
+    const void *x;             // dense forms
+    const int *row_ptr, *col;  // CSR
+    const float *val;
+    int cols;                  // row length of the dense forms
+};
+
+template <bool DENSE_PATH>
+__global__ void __launch_bounds__(PD_THREADS)
+k_predict_direct(int kind, RowsIn in, int n_rows, int n_feat, const HNode *__restrict__ model, int n_rounds, int K, int n_nodes, int depth,
+                 int rt_log, int chunk_rounds, float lr, float base_score, float *__restrict__ out) {
+    extern __shared__ __align__(16) unsigned char pd_sm[];
+    const int RT = 1 << rt_log, stride = RT + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *acc = reinterpret_cast<double *>(pd_sm);                    // [K][RT] running sums (the CSR path keeps floats there)
+    float *leaf = reinterpret_cast<float *>(acc + (size_t)K * RT);      // [chunk_rounds * K][RT]
+    float *feat = leaf + (size_t)chunk_rounds * K * RT;                 // [n_feat][RT + 1]
+    const float absent = DENSE_PATH ? INFINITY : __uint_as_float(PRED_ABSENT);
+    const int row0 = blockIdx.x << rt_log, rows = min(RT, n_rows - row0);
+    if (kind == IN_CSR) {
+        for (int i = threadIdx.x; i < n_feat * stride; i += PD_THREADS) feat[i] = absent;
+        __syncthreads();
+    }
+    for (int r = warp; r < RT; r += PD_THREADS / 32) {
+        if (kind == IN_CSR) {
+            if (r >= rows) continue;
+            const int e1 = in.row_ptr[row0 + r + 1];
+            for (int e = in.row_ptr[row0 + r] + lane; e < e1; e += 32) {
+                const int c = in.col[e];
+                if (c >= 0 && c < n_feat) feat[c * stride + r] = in.val[e];
             }
-        }
-    // is every tree a heap (children of i at 2i+1, 2i+2)?  The trainers here and the reference's Tree::init2 build them so.
-    bool heap = ((n_nodes + 1) & n_nodes) == 0;
-    int depth = 0;
-    while ((2 << depth) - 1 < n_nodes) ++depth;
-    std::vector<HNode> hflat;
-    if (heap) {
-        hflat.resize(flat.size());
-        for (size_t i = 0; i < flat.size() && heap; ++i) {
-            const int n = (int)(i % n_nodes);
-            const PNode &s = flat[i];
-            if (!(s.fid & 0x80000000) && (s.lch != 2 * n + 1 || s.rch != 2 * n + 2 || s.rch >= n_nodes)) heap = false;
-            hflat[i].v = s.v;
-            hflat[i].fid = s.fid;
-        }
-    }
-    // streams and events are released on every way out, also when a CUDA call throws
-    struct Guard {
-        cudaStream_t st = nullptr;
-        cudaEvent_t e0 = nullptr, e1 = nullptr;
-        ~Guard() {
-            if (e0) cudaEventDestroy(e0);
-            if (e1) cudaEventDestroy(e1);
-            if (st) cudaStreamDestroy(st);
-        }
-    } gd;
-    TGBM_CUDA(cudaStreamCreateWithFlags(&gd.st, cudaStreamNonBlocking));
-    cudaStream_t st = gd.st;
-    const size_t nnz = (size_t)ds.rp[N];
-    DevBuf<int> d_rp, d_col;
-    DevBuf<float> d_val, d_out;
-    DevBuf<PNode> d_model;
-    DevBuf<HNode> d_hmodel;
-    d_rp.alloc(N + 1); d_col.alloc(std::max<size_t>(nnz, 1)); d_val.alloc(std::max<size_t>(nnz, 1)); d_out.alloc((size_t)N * K);
-    upload_h2d(d_rp.p, ds.rp, sizeof(int) * (size_t)(N + 1), st, upload_threads());
-    upload_h2d(d_col.p, ds.ci, sizeof(int) * nnz, st, upload_threads());
-    upload_h2d(d_val.p, ds.vv, sizeof(float) * nnz, st, upload_threads());
-    if (heap) {
-        d_hmodel.alloc(hflat.size());
-        TGBM_CUDA(cudaMemcpyAsync(d_hmodel.p, hflat.data(), sizeof(HNode) * hflat.size(), cudaMemcpyHostToDevice, st));
-    }
-    d_model.alloc(flat.size());
-    TGBM_CUDA(cudaMemcpyAsync(d_model.p, flat.data(), sizeof(PNode) * flat.size(), cudaMemcpyHostToDevice, st));
-    const int F = ds.n_features;
-    const size_t smem = (size_t)F * PRED_ROWS * sizeof(float);
-    int dev = 0, num_sms = 148;
-    TGBM_CUDA(cudaGetDevice(&dev));
-    TGBM_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
-    // The reference chooses its arithmetic by F * 128 * 4 <= 48 KB (predictor.cu:88); that choice is kept, the tiled
-    // kernel serves either whenever a tile of rows and a chunk of trees fit the shared memory of an SM.
-    const bool dense_path = smem <= 48 * 1024;
-    bool done = false;
-    DevBuf<double> d_partial;
-    const bool heap_ok = heap && getenv("TGBM_PREDICT_SIMPLE") == nullptr;
-    // ---- ranks: thresholds per feature, nodes with threshold ranks
-    std::vector<int> thr_ptr;
-    std::vector<float> thr;
-    std::vector<RNode> rflat;
-    // (the rank bytes are a dense N x Fpad matrix: not for wide sparse data, where it would dwarf the CSR itself)
-    const size_t rank_bytes = (size_t)N * (size_t)((F + 31) / 32 * 32);
-    bool ranks = heap_ok && getenv("TGBM_PREDICT_FLOAT") == nullptr && sizeof(RNode) * (size_t)n_nodes * std::min(8, n_rounds) <= 140 * 1024 && F < 65536 &&
-                 rank_bytes <= std::max<size_t>((size_t)64 << 20, 8 * nnz);
-    if (ranks) {
-        std::vector<std::vector<float>> per(F);
-        for (size_t i = 0; i < flat.size(); ++i) {
-            const PNode &nd = flat[i];
-            if (nd.fid & 0x80000000) continue;
-            const int f = nd.fid & 0x3fffffff;
-            if (f < F) per[f].push_back(nd.v == 0.f ? 0.f : nd.v);  // -0 and +0 compare equal: one threshold
-            if (nd.v != nd.v) ranks = false;                        // a NaN threshold has no rank
-        }
-        thr_ptr.assign(F + 1, 0);
-        for (int f = 0; f < F && ranks; ++f) {
-            std::sort(per[f].begin(), per[f].end());
-            per[f].erase(std::unique(per[f].begin(), per[f].end()), per[f].end());
-            if (per[f].size() > 254) ranks = false;
-            thr_ptr[f + 1] = thr_ptr[f] + (int)per[f].size();
-        }
-        if (ranks) {
-            thr.reserve(thr_ptr[F] + 1);
-            for (int f = 0; f < F; ++f) thr.insert(thr.end(), per[f].begin(), per[f].end());
-            rflat.resize(flat.size());
-            for (size_t i = 0; i < flat.size(); ++i) {
-                const PNode &nd = flat[i];
-                RNode &o = rflat[i];
-                if (nd.fid & 0x80000000) { o.flags = 0x200; o.weight = nd.v; continue; }
-                const int f = nd.fid & 0x3fffffff;
-                int t = 0;
-                if (f < F) t = (int)(std::lower_bound(per[f].begin(), per[f].end(), nd.v == 0.f ? 0.f : nd.v) - per[f].begin());
-                // rows of up to 32 features are walked on words: bits 16-31 = word index (8 = the word of absent marks, for a
-                // feature the data does not have), bits 10-14 = bit offset of the byte; else bits 16-31 = feature id
-                const unsigned hi = (F <= 32) ? (f < F ? (unsigned)(f >> 2) : 8u) : (unsigned)std::min(f, 65535);
-                o.flags = t | ((nd.fid & 0x40000000) ? 0x100 : 0) | ((F <= 32 && f < F) ? ((f & 3) * 8) << 10 : 0) | (int)(hi << 16);
-                o.weight = 0.f;
-            }
-        }
-    }
-    // complete trees for the two-plane walk (rows of at most 32 features; TGBM_PREDICT_RANKS=1 keeps the walk above)
-    const bool planes = ranks && F <= 32 && depth >= 1 && depth <= 12 && getenv("TGBM_PREDICT_RANKS") == nullptr;
-    std::vector<PlaneNode> pl_nodes;
-    std::vector<float> pl_leaves;
-    const int n_inner = (1 << depth) - 1, n_leaf = 1 << depth;
-    if (planes) {
-        pl_nodes.resize((size_t)n_rounds * K * n_inner);
-        pl_leaves.assign((size_t)n_rounds * K * n_leaf, 0.f);
-        const PlaneNode pass = plane_node(0, 255, PL_WORDS - 1);   // absent word of plane 0: 255 <= 255, left
-        for (int tr = 0; tr < n_rounds * K; ++tr) {
-            const RNode *src = rflat.data() + (size_t)tr * n_nodes;
-            PlaneNode *dn = pl_nodes.data() + (size_t)tr * n_inner;
-            float *dl = pl_leaves.data() + (size_t)tr * n_leaf;
-            // carry[i]: the node inherits a leaf from above (1) with weight w[i], or lies off every path (2)
-            std::vector<unsigned char> carry(n_nodes, 0);
-            std::vector<float> w(n_nodes, 0.f);
-            for (int i = 0; i < n_nodes; ++i) {
-                const bool leaf = carry[i] != 0 || (src[i].flags & 0x200);
-                const float wt = carry[i] == 1 ? w[i] : carry[i] == 2 ? 0.f : src[i].weight;
-                if (i >= n_inner) { dl[i - n_inner] = leaf ? wt : 0.f; continue; }
-                if (leaf) {
-                    dn[i] = pass;
-                    carry[2 * i + 1] = carry[i] == 2 ? 2 : 1; w[2 * i + 1] = wt;
-                    carry[2 * i + 2] = 2;
-                    continue;
-                }
-                const int fl = src[i].flags;
-                const unsigned word = (unsigned)fl >> 16, byte = (((unsigned)fl >> 10) & 31u) / 8u, t = (unsigned)fl & 0xffu;
-                const bool default_right = fl & 0x100;
-                // missing goes right: plane 0, rank <= t; missing goes left: plane 1 (ranks rotated by one), <= t + 1
-                dn[i] = plane_node(byte, default_right ? t : t + 1, word + (default_right ? 0u : (unsigned)PL_WORDS));
-            }
-        }
-    }
-    DevBuf<PlaneNode> d_pl_nodes;
-    DevBuf<float> d_pl_leaves;
-    DevBuf<int> d_thr_ptr;
-    DevBuf<float> d_thr;
-    DevBuf<RNode> d_rmodel;
-    DevBuf<unsigned char> d_bins;
-    const int Fpad = (F + 31) / 32 * 32;
-    int rk_chunk = 0;
-    if (ranks) {
-        d_thr_ptr.alloc(F + 1); d_thr.alloc(std::max<size_t>(thr.size(), 1)); d_rmodel.alloc(rflat.size()); d_bins.alloc((size_t)N * Fpad);
-        TGBM_CUDA(cudaMemcpyAsync(d_thr_ptr.p, thr_ptr.data(), sizeof(int) * (F + 1), cudaMemcpyHostToDevice, st));
-        if (!thr.empty()) TGBM_CUDA(cudaMemcpyAsync(d_thr.p, thr.data(), sizeof(float) * thr.size(), cudaMemcpyHostToDevice, st));
-        TGBM_CUDA(cudaMemcpyAsync(d_rmodel.p, rflat.data(), sizeof(RNode) * rflat.size(), cudaMemcpyHostToDevice, st));
-        const size_t rk_rows_bytes = F <= 32 ? sizeof(uint32_t) * 9 * PR_ROWS : 0;
-        rk_chunk = (int)std::min<size_t>((size_t)n_rounds, ((size_t)(216 * 1024) - rk_rows_bytes) / (sizeof(RNode) * (size_t)n_nodes));
-        if (planes) {
-            d_pl_nodes.alloc(pl_nodes.size()); d_pl_leaves.alloc(pl_leaves.size());
-            TGBM_CUDA(cudaMemcpyAsync(d_pl_nodes.p, pl_nodes.data(), sizeof(PlaneNode) * pl_nodes.size(), cudaMemcpyHostToDevice, st));
-            TGBM_CUDA(cudaMemcpyAsync(d_pl_leaves.p, pl_leaves.data(), sizeof(float) * pl_leaves.size(), cudaMemcpyHostToDevice, st));
-            const size_t per_tree = sizeof(PlaneNode) * (size_t)n_inner + sizeof(float) * (size_t)n_leaf;
-            const size_t row_bytes = sizeof(uint32_t) * 2 * PL_WORDS * PL_ROWS;
-            rk_chunk = (int)std::min<size_t>((size_t)n_rounds, ((size_t)(224 * 1024) - row_bytes) / per_tree);
-            TGBM_CHECK(rk_chunk >= 1, "a tree of this depth does not fit beside a tile of rows");
-        }
-        if (rk_chunk < n_rounds) d_partial.alloc((size_t)N * K);
-    }
-    const bool tiled = heap_ok && !ranks;
-    auto tiles = [&](bool plan_only) {
-        return dense_path ? launch_predict_tiles<true>(d_rp.p, d_col.p, d_val.p, N, F, d_hmodel.p, n_rounds, K, n_nodes, depth, learning_rate,
-                                                       base_score, d_out.p, num_sms, st, d_partial, plan_only)
-                          : launch_predict_tiles<false>(d_rp.p, d_col.p, d_val.p, N, F, d_hmodel.p, n_rounds, K, n_nodes, depth, learning_rate,
-                                                        base_score, d_out.p, num_sms, st, d_partial, plan_only);
-    };
-    if (tiled) tiles(true);  // scratch for the running sums is allocated here, outside the timed kernel
-    // dense fast path of the conversion: N * F stored values, F a multiple of 4 up to 32
-    bool dense_rows = ranks && planes && F % 4 == 0 && (size_t)N * F == nnz && getenv("TGBM_PREDICT_RANKS") == nullptr;
-    // (whether row i really starts at i * F and holds the columns 0 .. F-1 is checked by the kernel, row by row)
-    DevBuf<float> d_tree_thr;
-    DevBuf<int> d_not_dense;
-    if (dense_rows) {
-        std::vector<float> tree((size_t)F * 256, INFINITY);
-        for (int f = 0; f < F; ++f) {
-            std::vector<float> sorted(255, INFINITY);
-            std::copy(thr.begin() + thr_ptr[f], thr.begin() + thr_ptr[f + 1], sorted.begin());
-            // node k of the implicit tree holds the middle of its range; children 2k+1 (left half), 2k+2 (right half)
-            struct Range { int k, lo, hi; };
-            std::vector<Range> todo{{0, 0, 255}};
-            while (!todo.empty()) {
-                const Range g = todo.back();
-                todo.pop_back();
-                if (g.lo >= g.hi) continue;
-                const int mid = (g.lo + g.hi) / 2;
-                tree[(size_t)f * 256 + g.k] = sorted[mid];
-                todo.push_back({2 * g.k + 1, g.lo, mid});
-                todo.push_back({2 * g.k + 2, mid + 1, g.hi});
-            }
-        }
-        d_tree_thr.alloc(tree.size()); d_not_dense.alloc(1);
-        TGBM_CUDA(cudaMemcpyAsync(d_tree_thr.p, tree.data(), sizeof(float) * tree.size(), cudaMemcpyHostToDevice, st));
-        d_not_dense.zero(st);
-    }
-    if (ranks) {   // the kernels of this path are loaded before the clock starts (the first launch of a kernel loads it otherwise)
-        cudaFuncAttributes fa;
-        if (dense_rows) cudaFuncGetAttributes(&fa, dense_path ? k_rank_dense_rows<true> : k_rank_dense_rows<false>);
-        cudaFuncGetAttributes(&fa, dense_path ? k_rank_rows<true, true> : k_rank_rows<false, true>);
-        if (planes) cudaFuncGetAttributes(&fa, dense_path ? k_predict_planes<true> : k_predict_planes<false>);
-    }
-    if (kernel_ms) { TGBM_CUDA(cudaEventCreate(&gd.e0)); TGBM_CUDA(cudaEventCreate(&gd.e1)); TGBM_CUDA(cudaEventRecord(gd.e0, st)); }
-    if (tiled) done = tiles(false);
-    if (ranks) {
-        bool converted = false;
-        if (dense_rows) {
-            const size_t tree_smem = sizeof(float) * (size_t)F * 256;
-            auto kern = dense_path ? k_rank_dense_rows<true> : k_rank_dense_rows<false>;
-            kern<<<std::min((N + RD_THREADS - 1) / RD_THREADS, num_sms * 8), RD_THREADS, tree_smem, st>>>(d_rp.p, d_col.p, d_val.p, N, F, d_tree_thr.p,
-                                                                                                      d_thr_ptr.p, d_bins.p, d_not_dense.p);
-            int h_not_dense = 0;
-            TGBM_CUDA(cudaMemcpyAsync(&h_not_dense, d_not_dense.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-            TGBM_CUDA(cudaStreamSynchronize(st));
-            converted = h_not_dense == 0;
-        }
-        if (!converted) {
-        TGBM_CUDA(cudaMemsetAsync(d_bins.p, MISSING_BIN, d_bins.bytes(), st));
-        const int rk_blocks = std::min((N + RK_ROWS - 1) / RK_ROWS, num_sms * 8);   // persistent: a block walks several tiles of rows
-        const size_t thr_smem = sizeof(float) * (size_t)F * RK_THR_STRIDE;
-        const bool smem_thr = thr_smem <= 40 * 1024 && getenv("TGBM_PREDICT_RANKS") == nullptr;
-        if (smem_thr) {
-            if (dense_path) k_rank_rows<true, true><<<rk_blocks, RK_THREADS, thr_smem, st>>>(d_rp.p, d_col.p, d_val.p, N, F, Fpad, d_thr_ptr.p, d_thr.p, d_bins.p);
-            else k_rank_rows<false, true><<<rk_blocks, RK_THREADS, thr_smem, st>>>(d_rp.p, d_col.p, d_val.p, N, F, Fpad, d_thr_ptr.p, d_thr.p, d_bins.p);
         } else {
-            if (dense_path) k_rank_rows<true, false><<<rk_blocks, RK_THREADS, 0, st>>>(d_rp.p, d_col.p, d_val.p, N, F, Fpad, d_thr_ptr.p, d_thr.p, d_bins.p);
-            else k_rank_rows<false, false><<<rk_blocks, RK_THREADS, 0, st>>>(d_rp.p, d_col.p, d_val.p, N, F, Fpad, d_thr_ptr.p, d_thr.p, d_bins.p);
+            for (int c = lane; c < n_feat; c += 32) {
+                float v = absent;
+                if (r < rows && c < in.cols) {
+                    const size_t at = (size_t)(row0 + r) * in.cols + c;
+                    if (kind == IN_F64) { const double d = static_cast<const double *>(in.x)[at]; if (d != 0.0) v = (float)d; }
+                    else { const float d = static_cast<const float *>(in.x)[at]; if (kind == IN_FULL || d != 0.f) v = d; }
+                }
+                feat[c * stride + r] = v;
+            }
         }
-        }
-        const size_t rk_smem = sizeof(RNode) * (size_t)n_nodes * rk_chunk + (F <= 32 ? sizeof(uint32_t) * 9 * PR_ROWS : 0);
-        const int grid = std::max(1, std::min((N + PR_ROWS - 1) / PR_ROWS, num_sms));
-        if (getenv("TGBM_TIMING")) {  // how the time splits between the conversion and the walk
-            cudaEvent_t em;
-            cudaEventCreate(&em); cudaEventRecord(em, st); cudaEventSynchronize(em);
-            float ms = 0;
-            if (gd.e0) { cudaEventElapsedTime(&ms, gd.e0, em); fprintf(stderr, "[tgbm predict] rows -> ranks %8.3f ms\n", ms); }
-            cudaEventDestroy(em);
-        }
-        auto go = [&](auto kern) {
-            TGBM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem));
-            kern<<<grid, PR_THREADS, rk_smem, st>>>(d_bins.p, Fpad, F, N, d_rmodel.p, n_rounds, K, n_nodes, depth, rk_chunk, learning_rate, base_score,
-                                             d_out.p, d_partial.p);
-        };
-        if (planes) {
-            const size_t pl_smem = sizeof(uint32_t) * 2 * PL_WORDS * PL_ROWS +
-                                   (sizeof(PlaneNode) * (size_t)n_inner + sizeof(float) * (size_t)n_leaf) * rk_chunk;
-            const int pl_grid = std::max(1, std::min((N + PL_ROWS - 1) / PL_ROWS, num_sms));
-            auto go_planes = [&](auto kern) {
-                TGBM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl_smem));
-                kern<<<pl_grid, PL_THREADS, pl_smem, st>>>(d_bins.p, Fpad, N, d_pl_nodes.p, d_pl_leaves.p, n_rounds, K, depth, rk_chunk, learning_rate,
-                                                          base_score, d_out.p, d_partial.p);
-            };
-            if (dense_path) go_planes(k_predict_planes<true>); else go_planes(k_predict_planes<false>);
-        }
-        else if (dense_path) { if (F <= 32) go(k_predict_ranks<true, true>); else go(k_predict_ranks<true, false>); }
-        else { if (F <= 32) go(k_predict_ranks<false, true>); else go(k_predict_ranks<false, false>); }
-        done = true;
     }
-    if (done) {
-    } else if (dense_path) {
-        k_predict_dense<<<(N + PRED_ROWS - 1) / PRED_ROWS, PRED_ROWS, smem, st>>>(d_rp.p, d_col.p, d_val.p, N, F, d_model.p, n_rounds, K,
-                                                                                n_nodes, learning_rate, base_score, d_out.p);
-    } else if (smem <= 200 * 1024) {
-        TGBM_CUDA(cudaFuncSetAttribute(k_predict_csr_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_predict_csr_staged<<<(N + PRED_ROWS - 1) / PRED_ROWS, PRED_ROWS, smem, st>>>(d_rp.p, d_col.p, d_val.p, N, F, d_model.p, n_rounds,
-                                                                                     K, n_nodes, learning_rate, base_score, d_out.p);
-    } else {
-        k_predict_csr<<<(N + 127) / 128, 128, 0, st>>>(d_rp.p, d_col.p, d_val.p, N, d_model.p, n_rounds, K, n_nodes, learning_rate,
-                                                       base_score, d_out.p);
+    for (int i = threadIdx.x; i < K * RT; i += PD_THREADS) acc[i] = base_score;
+    for (int q0 = 0; q0 < n_rounds; q0 += chunk_rounds) {
+        const int nc = min(chunk_rounds, n_rounds - q0) * K;
+        __syncthreads();
+        const int r = threadIdx.x & (RT - 1);
+        const HNode *first = model + (size_t)q0 * K * n_nodes;
+        for (int q = threadIdx.x >> rt_log; q < nc; q += PD_THREADS >> rt_log) {
+            const HNode *nd = first + (size_t)q * n_nodes;
+            int cur = 0;
+            float v;
+            for (int lvl = 0;; ++lvl) {
+                const int2 raw = __ldg(reinterpret_cast<const int2 *>(nd + cur));
+                v = __int_as_float(raw.x);
+                if (raw.y < 0 || lvl == depth) break;
+                const int f = raw.y & 0x3fffffff;
+                const float fv = f < n_feat ? feat[f * stride + r] : absent;
+                const bool present = DENSE_PATH ? (fv < INFINITY) : (__float_as_uint(fv) != PRED_ABSENT);
+                const bool right = present ? !(fv < v) : (raw.y & 0x40000000) != 0;
+                cur = 2 * cur + 1 + (right ? 1 : 0);
+            }
+            leaf[q * RT + r] = v;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < K * RT; i += PD_THREADS) {
+            const int k = i >> rt_log, rr = i & (RT - 1);
+            const float *lw = leaf + (size_t)k * RT + rr;
+            const int n = nc / K, step = K * RT;
+            if (DENSE_PATH) {
+                double s = acc[i];
+#pragma unroll 4
+                for (int q = 0; q < n; ++q) s += (double)__fmul_rn(lr, lw[(size_t)q * step]);
+                acc[i] = s;
+            } else {
+                float s = (float)acc[i];   // a float survives the round trip through a double unchanged
+#pragma unroll 4
+                for (int q = 0; q < n; ++q) s = __fmaf_rn(lr, lw[(size_t)q * step], s);
+                acc[i] = s;
+            }
+        }
     }
-    TGBM_CUDA(cudaGetLastError());
-    if (kernel_ms) TGBM_CUDA(cudaEventRecord(gd.e1, st));
-    TGBM_CUDA(cudaMemcpyAsync(out.data(), d_out.p, sizeof(float) * out.size(), cudaMemcpyDeviceToHost, st));
-    TGBM_CUDA(cudaStreamSynchronize(st));
-    if (kernel_ms) TGBM_CUDA(cudaEventElapsedTime(kernel_ms, gd.e0, gd.e1));
+    // (a thread reads back only the sums it wrote)
+    for (int i = threadIdx.x; i < K * RT; i += PD_THREADS) {
+        const int k = i >> rt_log, rr = i & (RT - 1);
+        if (rr < rows) out[(size_t)k * n_rows + row0 + rr] = DENSE_PATH ? (float)(0.0 + acc[i]) : (float)acc[i];
+    }
 }
 
 // ---- predict_transform -------------------------------------------------------------------------
@@ -948,6 +751,586 @@ __global__ void k_transform(int objective, int K, int n, const float *__restrict
         }
         for (int k = 0; k < K; ++k) y[(size_t)k * n + i] = __fdiv_rn(y[(size_t)k * n + i], sum);
     }
+}
+
+// Stream and page-locked scratch of one prediction call.  A request of a few rows is over in tens of microseconds;
+// making a stream and allocating device buffers for it took longer than that.  Workspaces are kept for the next call (at
+// most WS_KEEP per device, 256 KB each; every calling thread takes one of its own) and given back by
+// tgbm_release_device_memory().  Inputs and scores that fit are read and written by the kernel through the mapping of the
+// page-locked buffer: no copy is queued at all.
+namespace {
+constexpr size_t WS_BYTES = 256 * 1024, WS_MAX_ITEM = 64 * 1024;
+constexpr int WS_KEEP = 8;
+struct WsBlock { int device; cudaStream_t st; char *host, *dev; };
+std::mutex &g_ws_mutex = *new std::mutex;
+std::vector<WsBlock> &g_ws_free = *new std::vector<WsBlock>;
+void ws_destroy(WsBlock &b) {
+    cudaStreamDestroy(b.st);
+    cudaFreeHost(b.host);
+}
+}  // namespace
+
+void predict_release_workspaces() noexcept {
+    std::vector<WsBlock> v;
+    {
+        std::lock_guard<std::mutex> lock(g_ws_mutex);
+        v.swap(g_ws_free);
+    }
+    for (auto &b : v) ws_destroy(b);
+}
+
+class PredictWorkspace {
+public:
+    PredictWorkspace() {
+        int dev = 0;
+        TGBM_CUDA(cudaGetDevice(&dev));
+        {
+            std::lock_guard<std::mutex> lock(g_ws_mutex);
+            for (size_t i = 0; i < g_ws_free.size(); ++i)
+                if (g_ws_free[i].device == dev) {
+                    b_ = g_ws_free[i];
+                    g_ws_free.erase(g_ws_free.begin() + i);
+                    return;
+                }
+        }
+        b_ = WsBlock{dev, nullptr, nullptr, nullptr};
+        TGBM_CUDA(cudaStreamCreateWithFlags(&b_.st, cudaStreamNonBlocking));
+        void *p = nullptr, *d = nullptr;
+        if (cudaHostAlloc(&p, WS_BYTES, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess || cudaHostGetDevicePointer(&d, p, 0) != cudaSuccess) {
+            cudaGetLastError();   // without it every item takes the device buffers
+            if (p) cudaFreeHost(p);
+            p = d = nullptr;
+        }
+        b_.host = static_cast<char *>(p); b_.dev = static_cast<char *>(d);
+    }
+    PredictWorkspace(const PredictWorkspace &) = delete;
+    PredictWorkspace &operator=(const PredictWorkspace &) = delete;
+    ~PredictWorkspace() {
+        cudaStreamSynchronize(b_.st);   // nothing of this call still uses the buffer
+        {
+            std::lock_guard<std::mutex> lock(g_ws_mutex);
+            if ((int)std::count_if(g_ws_free.begin(), g_ws_free.end(), [&](const WsBlock &o) { return o.device == b_.device; }) < WS_KEEP) {
+                g_ws_free.push_back(b_);
+                return;
+            }
+        }
+        ws_destroy(b_);
+    }
+    cudaStream_t stream() const { return b_.st; }
+    void *take(size_t bytes) {   // null: too large
+        const size_t n = (bytes + 255) / 256 * 256;
+        if (!b_.host || bytes > WS_MAX_ITEM || used_ + n > WS_BYTES) return nullptr;
+        void *p = b_.host + used_;
+        used_ += n;
+        return p;
+    }
+    void *device(void *host) const { return b_.dev + (static_cast<char *>(host) - b_.host); }
+
+private:
+    WsBlock b_;
+    size_t used_ = 0;
+};
+
+// ---- a model laid out for the kernels above ---------------------------------------------------------------------------
+// Made once per model handle (the C entry points keep it with the handle) or once per call of tgbm_predict_raw, whose
+// caller hands node records over every time.  The node records alone serve the direct walk; ranks, thresholds and
+// completed trees are added when a large input first asks for them.
+class PredictPlan {
+public:
+    int n_rounds = 0, K = 0, n_nodes = 0, depth = 0, max_fid = -1, device = 0;
+    bool heap = false;     // children of i at 2i+1, 2i+2: the trainers here and the reference's Tree::init2 build trees so
+    DevBuf<HNode> h;       // heap trees
+    DevBuf<PNode> p;       // any other
+
+    struct Ranks {
+        int F = 0;
+        bool ok = false, planes = false;
+        std::vector<int> thr_ptr;
+        std::vector<float> thr, tree_thr, leaves;
+        std::vector<RNode> nodes;
+        std::vector<PlaneNode> pl_nodes;
+        DevBuf<int> d_thr_ptr;
+        DevBuf<float> d_thr, d_tree_thr, d_leaves;
+        DevBuf<RNode> d_nodes;
+        DevBuf<PlaneNode> d_pl_nodes;
+        void upload(cudaStream_t st) {
+            auto put = [&](auto &dst, const auto &src) {
+                dst.alloc(std::max<size_t>(src.size(), 1));
+                if (!src.empty()) TGBM_CUDA(cudaMemcpyAsync(dst.p, src.data(), sizeof(src[0]) * src.size(), cudaMemcpyHostToDevice, st));
+            };
+            put(d_thr_ptr, thr_ptr); put(d_thr, thr); put(d_tree_thr, tree_thr);
+            if (planes) { put(d_pl_nodes, pl_nodes); put(d_leaves, leaves); }
+            else put(d_nodes, nodes);
+            TGBM_CUDA(cudaStreamSynchronize(st));
+        }
+    };
+
+    PredictPlan(const ModelRef &m, cudaStream_t st) : n_rounds(m.n_rounds), K(m.K), n_nodes(m.n_nodes) {
+        TGBM_CUDA(cudaGetDevice(&device));
+        while ((2 << depth) - 1 < n_nodes) ++depth;
+        heap = ((n_nodes + 1) & n_nodes) == 0;
+        const size_t total = m.trees.size() * (size_t)n_nodes;
+        flat_.resize(total);
+        for (size_t t = 0; t < m.trees.size(); ++t) {
+            const TreeNode *src = m.trees[t];
+            HNode *dst = flat_.data() + t * n_nodes;
+            bool ok = true;
+            int top = -1;
+            for (int n = 0; n < n_nodes; ++n) {
+                const TreeNode &s = src[n];
+                if (s.is_leaf) { dst[n] = HNode{s.base_weight, (int)0x80000000}; continue; }
+                const int f = s.split_feature_id & 0x3fffffff;
+                dst[n] = HNode{s.split_value, f | (s.default_right ? 0x40000000 : 0)};
+                ok &= s.lch_index == 2 * n + 1 && s.rch_index == 2 * n + 2 && s.rch_index < n_nodes;
+                if (s.split_feature_id >= 0) top = std::max(top, f);   // (nodes that were never reached carry -1)
+            }
+            heap = heap && ok;
+            max_fid = std::max(max_fid, top);
+        }
+        if (heap) {
+            h.alloc(total);
+            TGBM_CUDA(cudaMemcpyAsync(h.p, flat_.data(), sizeof(HNode) * total, cudaMemcpyHostToDevice, st));
+            return;
+        }
+        std::vector<PNode> any(total);
+        for (size_t i = 0; i < total; ++i) {
+            const TreeNode &s = m.trees[i / n_nodes][i % n_nodes];
+            any[i] = PNode{flat_[i].v, flat_[i].fid, s.lch_index, s.rch_index};
+        }
+        p.alloc(total);
+        TGBM_CUDA(cudaMemcpyAsync(p.p, any.data(), sizeof(PNode) * total, cudaMemcpyHostToDevice, st));
+        TGBM_CUDA(cudaStreamSynchronize(st));
+    }
+
+    // ranks for data of F features (host side; nothing is uploaded)
+    std::shared_ptr<Ranks> make_ranks(int F) const {
+        auto rk = std::make_shared<Ranks>();
+        Ranks &r = *rk;
+        r.F = F;
+        if (!heap || F >= 65536 || sizeof(RNode) * (size_t)n_nodes * std::min(8, n_rounds) > 140 * 1024) return rk;
+        auto zero = [](float v) { return v == 0.f ? 0.f : v; };   // -0 and +0 compare equal: one threshold
+        std::vector<int> at(F + 1, 0);
+        for (const HNode &nd : flat_) {
+            if (nd.fid < 0) continue;
+            const int f = nd.fid & 0x3fffffff;
+            if (nd.v != nd.v) return rk;   // a NaN threshold has no rank
+            if (f < F) ++at[f + 1];
+        }
+        for (int f = 0; f < F; ++f) at[f + 1] += at[f];
+        std::vector<float> all(at[F]);
+        {
+            std::vector<int> pos(at.begin(), at.end() - 1);
+            for (const HNode &nd : flat_) {
+                const int f = nd.fid & 0x3fffffff;
+                if (nd.fid >= 0 && f < F) all[pos[f]++] = zero(nd.v);
+            }
+        }
+        r.thr_ptr.assign(F + 1, 0);
+        for (int f = 0; f < F; ++f) {
+            std::sort(all.begin() + at[f], all.begin() + at[f + 1]);
+            const auto end = std::unique(all.begin() + at[f], all.begin() + at[f + 1]);
+            if (end - (all.begin() + at[f]) > 254) return rk;
+            r.thr.insert(r.thr.end(), all.begin() + at[f], end);
+            r.thr_ptr[f + 1] = (int)r.thr.size();
+        }
+        r.nodes.resize(flat_.size());
+        for (size_t i = 0; i < flat_.size(); ++i) {
+            const HNode &nd = flat_[i];
+            RNode &o = r.nodes[i];
+            if (nd.fid < 0) { o.flags = 0x200; o.weight = nd.v; continue; }
+            const int f = nd.fid & 0x3fffffff;
+            int t = 0;
+            if (f < F) t = (int)(std::lower_bound(r.thr.begin() + r.thr_ptr[f], r.thr.begin() + r.thr_ptr[f + 1], zero(nd.v)) - (r.thr.begin() + r.thr_ptr[f]));
+            // rows of up to 32 features are walked on words: bits 16-31 = word index (8 = the word of absent marks, for a
+            // feature the data does not have), bits 10-14 = bit offset of the byte; else bits 16-31 = feature id
+            const unsigned hi = (F <= 32) ? (f < F ? (unsigned)(f >> 2) : 8u) : (unsigned)std::min(f, 65535);
+            o.flags = t | ((nd.fid & 0x40000000) ? 0x100 : 0) | ((F <= 32 && f < F) ? ((f & 3) * 8) << 10 : 0) | (int)(hi << 16);
+            o.weight = 0.f;
+        }
+        r.ok = true;
+        r.planes = F <= 32 && depth >= 1 && depth <= 12 && getenv("TGBM_PREDICT_RANKS") == nullptr;
+        if (r.planes) {
+            complete_trees(r);
+            search_trees(r);
+        }
+        return rk;
+    }
+
+    // the ranks for data of F features, on the device; made and uploaded by the first caller
+    std::shared_ptr<Ranks> ranks(int F, cudaStream_t st, std::shared_ptr<Ranks> made) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (!ranks_ || ranks_->F != F) {
+            if (!made || made->F != F) made = make_ranks(F);
+            if (made->ok) made->upload(st);
+            ranks_ = std::move(made);
+        }
+        return ranks_;
+    }
+    // the nodes with their own child indices, for the kernels that take trees of any shape
+    const PNode *any_nodes(cudaStream_t st) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (!p.p) {
+            std::vector<PNode> any(flat_.size());
+            for (size_t i = 0; i < flat_.size(); ++i) {
+                const int n = (int)(i % (size_t)n_nodes);
+                any[i] = PNode{flat_[i].v, flat_[i].fid, 2 * n + 1, 2 * n + 2};
+            }
+            p.alloc(any.size());
+            TGBM_CUDA(cudaMemcpyAsync(p.p, any.data(), sizeof(PNode) * any.size(), cudaMemcpyHostToDevice, st));
+            TGBM_CUDA(cudaStreamSynchronize(st));
+        }
+        return p.p;
+    }
+    bool has_ranks(int F) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        return ranks_ && ranks_->F == F;
+    }
+
+private:
+    // complete trees for the two-plane walk
+    void complete_trees(Ranks &r) const {
+        const int n_inner = (1 << depth) - 1, n_leaf = 1 << depth, n_trees = n_rounds * K;
+        r.pl_nodes.resize((size_t)n_trees * n_inner);
+        r.leaves.assign((size_t)n_trees * n_leaf, 0.f);
+        const PlaneNode pass = plane_node(0, 255, PL_WORDS - 1);   // absent word of plane 0: 255 <= 255, left
+        std::vector<unsigned char> carry(n_nodes);
+        std::vector<float> w(n_nodes);
+        for (int tr = 0; tr < n_trees; ++tr) {
+            const RNode *src = r.nodes.data() + (size_t)tr * n_nodes;
+            PlaneNode *dn = r.pl_nodes.data() + (size_t)tr * n_inner;
+            float *dl = r.leaves.data() + (size_t)tr * n_leaf;
+            // carry[i]: the node inherits a leaf from above (1) with weight w[i], or lies off every path (2)
+            carry.assign(n_nodes, 0);
+            w.assign(n_nodes, 0.f);
+            for (int i = 0; i < n_nodes; ++i) {
+                const bool leaf = carry[i] != 0 || (src[i].flags & 0x200);
+                const float wt = carry[i] == 1 ? w[i] : carry[i] == 2 ? 0.f : src[i].weight;
+                if (i >= n_inner) { dl[i - n_inner] = leaf ? wt : 0.f; continue; }
+                if (leaf) {
+                    dn[i] = pass;
+                    carry[2 * i + 1] = carry[i] == 2 ? 2 : 1; w[2 * i + 1] = wt;
+                    carry[2 * i + 2] = 2;
+                    continue;
+                }
+                const int fl = src[i].flags;
+                const unsigned word = (unsigned)fl >> 16, byte = (((unsigned)fl >> 10) & 31u) / 8u, t = (unsigned)fl & 0xffu;
+                const bool default_right = fl & 0x100;
+                // missing goes right: plane 0, rank <= t; missing goes left: plane 1 (ranks rotated by one), <= t + 1
+                dn[i] = plane_node(byte, default_right ? t : t + 1, word + (default_right ? 0u : (unsigned)PL_WORDS));
+            }
+        }
+    }
+    // the thresholds of every feature as an implicit search tree of 255 nodes, padded with +inf
+    void search_trees(Ranks &r) const {
+        r.tree_thr.assign((size_t)r.F * 256, INFINITY);
+        for (int f = 0; f < r.F; ++f) {
+            const int n = r.thr_ptr[f + 1] - r.thr_ptr[f];
+            for (int k = 0; k < 255; ++k) {
+                // node k = the q-th of its level of 2^lv: it holds the middle of the q-th of 2^lv equal parts of 255 + 1 slots
+                int lv = 0;
+                while ((2 << lv) - 1 <= k) ++lv;
+                const int q = k - ((1 << lv) - 1), mid = (2 * q + 1) * (128 >> lv) - 1;
+                if (mid < n) r.tree_thr[(size_t)f * 256 + k] = r.thr[r.thr_ptr[f] + mid];
+            }
+        }
+    }
+
+    std::vector<HNode> flat_;
+    std::mutex mutex_;
+    std::shared_ptr<Ranks> ranks_;
+};
+std::shared_ptr<PredictPlan> make_predict_plan(const ModelRef &m) {
+    TGBM_CHECK(m.n_rounds > 0 && m.K > 0 && !m.trees.empty() && m.n_nodes > 0, "empty model");
+    PredictWorkspace ws;
+    auto plan = std::make_shared<PredictPlan>(m, ws.stream());
+    TGBM_CUDA(cudaStreamSynchronize(ws.stream()));
+    return plan;
+}
+bool predict_plan_fits(const PredictPlan &plan, int n_rounds, int K) {
+    int dev = 0;
+    TGBM_CUDA(cudaGetDevice(&dev));
+    return plan.n_rounds == n_rounds && plan.K == K && plan.device == dev;
+}
+
+// Node visits (rows x trees x levels) up to which rows are walked directly: below that the walk itself is over in less
+// time than the ranks of the large-input path take to make.
+constexpr double DIRECT_VISITS = 4e8;
+
+void predict(const DataSet &ds, PredictPlan &plan, float learning_rate, float base_score, int objective, const std::vector<float> &label,
+             float *out, float *kernel_ms) {
+    const int N = ds.n_rows, K = plan.K, n_rounds = plan.n_rounds, n_nodes = plan.n_nodes, depth = plan.depth;
+    if (N == 0) return;
+    if (K > 1) base_score = 0;  // predictor.cu:81-83
+    const bool transforms = objective == REG_LOGISTIC || objective == BINARY_LOGISTIC || objective == MULTI_SOFTMAX || objective == MULTI_SOFTPROB;
+    if (objective == BINARY_LOGISTIC) TGBM_CHECK(label.size() >= 2, "binary:logistic needs two class labels");
+    if (objective == MULTI_SOFTMAX) TGBM_CHECK((int)label.size() >= K, "multi:softmax needs one label per class");
+    const size_t n_out = objective == MULTI_SOFTMAX ? (size_t)N : (size_t)N * K;
+    PredictWorkspace ws;
+    cudaStream_t st = ws.stream();
+    int dev = 0, num_sms = 148;
+    TGBM_CUDA(cudaGetDevice(&dev));
+    TGBM_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
+    struct Events {
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+        ~Events() {
+            if (e0) cudaEventDestroy(e0);
+            if (e1) cudaEventDestroy(e1);
+        }
+    } ev;
+    if (kernel_ms) { TGBM_CUDA(cudaEventCreate(&ev.e0)); TGBM_CUDA(cudaEventCreate(&ev.e1)); }
+
+    // scores: small ones are written straight into page-locked memory
+    DevBuf<float> d_out;
+    float *scores = static_cast<float *>(ws.take(sizeof(float) * (size_t)N * K)), *scores_dev = nullptr;
+    if (scores) scores_dev = static_cast<float *>(ws.device(scores));
+    else { d_out.alloc((size_t)N * K); scores_dev = d_out.p; }
+    auto finish = [&]() {
+        TGBM_CUDA(cudaGetLastError());
+        if (kernel_ms) TGBM_CUDA(cudaEventRecord(ev.e1, st));
+        DevBuf<float> d_label;
+        if (transforms) {
+            const float *labels = nullptr;
+            if (!label.empty()) {
+                float *small = static_cast<float *>(ws.take(sizeof(float) * label.size()));
+                if (small) { memcpy(small, label.data(), sizeof(float) * label.size()); labels = static_cast<float *>(ws.device(small)); }
+                else {
+                    d_label.alloc(label.size());
+                    TGBM_CUDA(cudaMemcpyAsync(d_label.p, label.data(), sizeof(float) * label.size(), cudaMemcpyHostToDevice, st));
+                    labels = d_label.p;
+                }
+            }
+            k_transform<<<(N + 255) / 256, 256, 0, st>>>(objective, K, N, labels, scores_dev);
+            TGBM_CUDA(cudaGetLastError());
+        }
+        if (scores) {
+            TGBM_CUDA(cudaStreamSynchronize(st));
+            memcpy(out, scores, sizeof(float) * n_out);
+        } else {
+            download_d2h(out, d_out.p, sizeof(float) * n_out, st, upload_threads());
+        }
+        if (kernel_ms) TGBM_CUDA(cudaEventElapsedTime(kernel_ms, ev.e0, ev.e1));
+    };
+
+    // The reference chooses its arithmetic by F * 128 * 4 <= 48 KB (predictor.cu:88), F = largest column of the data + 1;
+    // that choice is kept whatever kernel serves it.
+    auto is_dense_path = [](int F) { return (size_t)F * PRED_ROWS * sizeof(float) <= 48 * 1024; };
+    const bool simple = getenv("TGBM_PREDICT_SIMPLE") != nullptr;
+    const bool heap_ok = plan.heap && !simple;
+    DeviceRows rows;
+    bool uploaded = false;
+    int F = ds.n_features;   // < 0: not counted yet
+
+    // ---- few rows: the direct walk
+    if (heap_ok && (double)N * n_rounds * K * std::max(depth, 1) <= DIRECT_VISITS && getenv("TGBM_PREDICT_FLOAT") == nullptr &&
+        getenv("TGBM_PREDICT_RANKS") == nullptr) {
+        RowsIn in{};
+        int kind = ds.dense ? (ds.dense_f64 ? IN_F64 : IN_F32) : IN_CSR;
+        DevBuf<unsigned char> d_x;
+        if (ds.dense) {
+            in.cols = ds.dense_cols;
+            if (F < 0) F = is_dense_path(in.cols) ? in.cols : ds.count_features();   // only the choice of the arithmetic depends on it
+            const size_t bytes = (size_t)N * in.cols * (ds.dense_f64 ? 8 : 4);
+            void *small = ws.take(bytes);
+            if (small) { memcpy(small, ds.dense, bytes); in.x = ws.device(small); }
+            else {
+                d_x.alloc(bytes);
+                upload_h2d(d_x.p, ds.dense, bytes, st, upload_threads());
+                in.x = d_x.p;
+            }
+        } else {
+            const size_t nnz = (size_t)ds.rp[N];
+            int *rp = static_cast<int *>(ws.take(sizeof(int) * (size_t)(N + 1)));
+            int *col = rp ? static_cast<int *>(ws.take(sizeof(int) * nnz)) : nullptr;
+            float *val = col ? static_cast<float *>(ws.take(sizeof(float) * nnz)) : nullptr;
+            if (val) {
+                memcpy(rp, ds.rp, sizeof(int) * (size_t)(N + 1));
+                memcpy(col, ds.ci, sizeof(int) * nnz);
+                memcpy(val, ds.vv, sizeof(float) * nnz);
+                if (F < 0) {
+                    int m = -1;
+                    for (size_t i = 0; i < nnz; ++i) m = std::max(m, col[i]);
+                    F = m + 1;
+                }
+                in.row_ptr = static_cast<int *>(ws.device(rp)); in.col = static_cast<int *>(ws.device(col)); in.val = static_cast<float *>(ws.device(val));
+            } else {
+                rows.upload(ds, st, num_sms, upload_threads());
+                uploaded = true;
+                if (F < 0) F = rows.max_col + 1;
+                if (rows.full_cols) { kind = IN_FULL; in.x = rows.val.p; in.cols = rows.full_cols; }
+                else { in.row_ptr = rows.row_ptr.p; in.col = rows.col.p; in.val = rows.val.p; }
+            }
+        }
+        const int n_feat = std::max(1, std::min(plan.max_fid + 1, kind == IN_CSR ? F : in.cols));
+        const size_t budget = 96 * 1024;   // two blocks per SM
+        int rt_log = 5, chunk = 0;
+        while (rt_log > 0 && (long long)(N >> rt_log) < 2LL * num_sms) --rt_log;   // at least two blocks per SM, then longer tiles
+        auto smem = [&]() {
+            const size_t fixed = ((size_t)8 * K << rt_log) + sizeof(float) * (size_t)n_feat * ((1 << rt_log) + 1), per_round = ((size_t)4 * K << rt_log);
+            chunk = fixed + per_round > budget ? 0 : (int)std::min<size_t>((size_t)n_rounds, (budget - fixed) / per_round);
+            return fixed + per_round * chunk;
+        };
+        size_t bytes = smem();
+        while (chunk < std::min(8, n_rounds) && rt_log > 0) { --rt_log; bytes = smem(); }
+        if (chunk > 0) {
+            auto kern = is_dense_path(F) ? k_predict_direct<true> : k_predict_direct<false>;
+            static std::once_flag once;
+            std::call_once(once, [&] {
+                cudaFuncSetAttribute(k_predict_direct<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
+                cudaFuncSetAttribute(k_predict_direct<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
+            });
+            if (kernel_ms) TGBM_CUDA(cudaEventRecord(ev.e0, st));
+            kern<<<(N + (1 << rt_log) - 1) >> rt_log, PD_THREADS, bytes, st>>>(kind, in, N, n_feat, plan.h.p, n_rounds, K, n_nodes, depth, rt_log,
+                                                                              chunk, learning_rate, base_score, scores_dev);
+            finish();
+            return;
+        }
+    }
+
+    // ---- many rows: stored values on the device, ranks, tiles.  The host side of the ranks is made while the values are
+    // copied when the feature count is known or can be read off the first row.
+    std::future<std::shared_ptr<PredictPlan::Ranks>> making;
+    if (!uploaded) {
+        const int guess = F >= 0 ? std::max(1, F) : ds.dense ? std::max(1, ds.dense_cols) : ds.rp[1];
+        if (heap_ok && guess >= 1 && guess <= 256 && !plan.has_ranks(guess)) making = std::async(std::launch::async, [&plan, guess] { return plan.make_ranks(guess); });
+        rows.upload(ds, st, num_sms, upload_threads());
+    }
+    std::shared_ptr<PredictPlan::Ranks> made;
+    if (making.valid()) made = making.get();
+    if (F < 0) F = rows.max_col + 1;
+    F = std::max(F, 1);
+    const bool dense_path = is_dense_path(F);
+    const size_t smem = (size_t)F * PRED_ROWS * sizeof(float);
+    const int Fpad = (F + 31) / 32 * 32;
+    // (the rank bytes are a dense N x Fpad matrix: not for wide sparse data, where it would dwarf the CSR itself)
+    const size_t rank_bytes = (size_t)N * (size_t)Fpad;
+    std::shared_ptr<PredictPlan::Ranks> rk;
+    if (heap_ok && getenv("TGBM_PREDICT_FLOAT") == nullptr && rank_bytes <= std::max<size_t>((size_t)64 << 20, 8 * rows.nnz)) {
+        rk = plan.ranks(F, st, made);
+        if (!rk->ok) rk.reset();
+    }
+    DevBuf<double> d_partial;
+    if (rk) {
+        DevBuf<unsigned char> d_bins;
+        d_bins.alloc((size_t)N * Fpad);
+        // dense fast path of the conversion: every cell stored, F a multiple of 4 up to 32
+        const bool dense_rows = rk->planes && rows.full_cols == F && F % 4 == 0;
+        if (!dense_rows) rows.need_csr(N, st, num_sms);
+        const int n_inner = (1 << depth) - 1, n_leaf = 1 << depth;
+        size_t rk_smem;
+        int chunk;
+        if (rk->planes) {
+            const size_t per_tree = sizeof(PlaneNode) * (size_t)n_inner + sizeof(float) * (size_t)n_leaf, row_bytes = sizeof(uint32_t) * 2 * PL_WORDS * PL_ROWS;
+            chunk = (int)std::min<size_t>((size_t)n_rounds, ((size_t)(224 * 1024) - row_bytes) / per_tree);
+            TGBM_CHECK(chunk >= 1, "a tree of this depth does not fit beside a tile of rows");
+            rk_smem = row_bytes + per_tree * chunk;
+        } else {
+            const size_t row_bytes = F <= 32 ? sizeof(uint32_t) * 9 * PR_ROWS : 0;
+            chunk = (int)std::min<size_t>((size_t)n_rounds, ((size_t)(216 * 1024) - row_bytes) / (sizeof(RNode) * (size_t)n_nodes));
+            rk_smem = sizeof(RNode) * (size_t)n_nodes * chunk + row_bytes;
+        }
+        if (chunk < n_rounds) d_partial.alloc((size_t)N * K);
+        {   // the kernels of this path are loaded before the clock starts (the first launch of a kernel loads it otherwise)
+            cudaFuncAttributes fa;
+            if (dense_rows) cudaFuncGetAttributes(&fa, dense_path ? k_rank_dense_rows<true> : k_rank_dense_rows<false>);
+            else cudaFuncGetAttributes(&fa, dense_path ? k_rank_rows<true, true> : k_rank_rows<false, true>);
+            if (rk->planes) cudaFuncGetAttributes(&fa, dense_path ? k_predict_planes<true> : k_predict_planes<false>);
+        }
+        if (kernel_ms) TGBM_CUDA(cudaEventRecord(ev.e0, st));
+        if (dense_rows) {
+            auto kern = dense_path ? k_rank_dense_rows<true> : k_rank_dense_rows<false>;
+            kern<<<std::min((N + RD_THREADS - 1) / RD_THREADS, num_sms * 8), RD_THREADS, sizeof(float) * (size_t)F * 256, st>>>(
+                rows.val.p, N, F, rk->d_tree_thr.p, rk->d_thr_ptr.p, d_bins.p);
+        } else {
+            TGBM_CUDA(cudaMemsetAsync(d_bins.p, MISSING_BIN, d_bins.bytes(), st));
+            const int rk_blocks = std::min((N + RK_ROWS - 1) / RK_ROWS, num_sms * 8);   // persistent: a block walks several tiles of rows
+            const size_t thr_smem = sizeof(float) * (size_t)F * RK_THR_STRIDE;
+            const bool smem_thr = thr_smem <= 40 * 1024 && getenv("TGBM_PREDICT_RANKS") == nullptr;
+            auto convert = [&](auto kern) {
+                kern<<<rk_blocks, RK_THREADS, smem_thr ? thr_smem : 0, st>>>(rows.row_ptr.p, rows.col.p, rows.val.p, N, F, Fpad, rk->d_thr_ptr.p,
+                                                                             rk->d_thr.p, d_bins.p);
+            };
+            if (smem_thr) { if (dense_path) convert(k_rank_rows<true, true>); else convert(k_rank_rows<false, true>); }
+            else { if (dense_path) convert(k_rank_rows<true, false>); else convert(k_rank_rows<false, false>); }
+        }
+        if (getenv("TGBM_TIMING") && ev.e0) {  // how the time splits between the conversion and the walk
+            cudaEvent_t em;
+            cudaEventCreate(&em); cudaEventRecord(em, st); cudaEventSynchronize(em);
+            float ms = 0;
+            cudaEventElapsedTime(&ms, ev.e0, em);
+            fprintf(stderr, "[tgbm predict] rows -> ranks %8.3f ms\n", ms);
+            cudaEventDestroy(em);
+        }
+        if (rk->planes) {
+            auto go = [&](auto kern) {
+                TGBM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem));
+                kern<<<std::max(1, std::min((N + PL_ROWS - 1) / PL_ROWS, num_sms)), PL_THREADS, rk_smem, st>>>(
+                    d_bins.p, Fpad, N, rk->d_pl_nodes.p, rk->d_leaves.p, n_rounds, K, depth, chunk, learning_rate, base_score, scores_dev, d_partial.p);
+            };
+            if (dense_path) go(k_predict_planes<true>); else go(k_predict_planes<false>);
+        } else {
+            auto go = [&](auto kern) {
+                TGBM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem));
+                kern<<<std::max(1, std::min((N + PR_ROWS - 1) / PR_ROWS, num_sms)), PR_THREADS, rk_smem, st>>>(
+                    d_bins.p, Fpad, F, N, rk->d_nodes.p, n_rounds, K, n_nodes, depth, chunk, learning_rate, base_score, scores_dev, d_partial.p);
+            };
+            if (dense_path) { if (F <= 32) go(k_predict_ranks<true, true>); else go(k_predict_ranks<true, false>); }
+            else { if (F <= 32) go(k_predict_ranks<false, true>); else go(k_predict_ranks<false, false>); }
+        }
+        finish();
+        return;
+    }
+    rows.need_csr(N, st, num_sms);
+    const int *rp = rows.row_ptr.p, *col = rows.col.p;
+    const float *val = rows.val.p;
+    if (heap_ok) {
+        auto tiles = [&](bool plan_only) {
+            return dense_path ? launch_predict_tiles<true>(rp, col, val, N, F, plan.h.p, n_rounds, K, n_nodes, depth, learning_rate, base_score,
+                                                           scores_dev, num_sms, st, d_partial, plan_only)
+                              : launch_predict_tiles<false>(rp, col, val, N, F, plan.h.p, n_rounds, K, n_nodes, depth, learning_rate, base_score,
+                                                            scores_dev, num_sms, st, d_partial, plan_only);
+        };
+        if (tiles(true)) {   // scratch for the running sums is allocated here, outside the timed kernel
+            if (kernel_ms) TGBM_CUDA(cudaEventRecord(ev.e0, st));
+            tiles(false);
+            finish();
+            return;
+        }
+    }
+    const PNode *any = plan.any_nodes(st);
+    if (kernel_ms) TGBM_CUDA(cudaEventRecord(ev.e0, st));
+    if (dense_path) {
+        k_predict_dense<<<(N + PRED_ROWS - 1) / PRED_ROWS, PRED_ROWS, smem, st>>>(rp, col, val, N, F, any, n_rounds, K, n_nodes, learning_rate, base_score, scores_dev);
+    } else if (smem <= 200 * 1024) {
+        TGBM_CUDA(cudaFuncSetAttribute(k_predict_csr_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_predict_csr_staged<<<(N + PRED_ROWS - 1) / PRED_ROWS, PRED_ROWS, smem, st>>>(rp, col, val, N, F, any, n_rounds, K, n_nodes, learning_rate, base_score, scores_dev);
+    } else {
+        k_predict_csr<<<(N + 127) / 128, 128, 0, st>>>(rp, col, val, N, any, n_rounds, K, n_nodes, learning_rate, base_score, scores_dev);
+    }
+    finish();
+}
+
+ModelRef model_ref(const std::vector<std::vector<Tree>> &model) {
+    ModelRef m;
+    m.n_rounds = (int)model.size();
+    TGBM_CHECK(m.n_rounds > 0 && !model[0].empty(), "empty model");
+    m.K = (int)model[0].size();
+    m.n_nodes = (int)model[0][0].nodes.size();
+    for (const auto &round : model) {
+        TGBM_CHECK((int)round.size() == m.K, "ragged model");
+        for (const auto &t : round) {
+            TGBM_CHECK((int)t.nodes.size() == m.n_nodes, "ragged model");
+            m.trees.push_back(t.nodes.data());
+        }
+    }
+    return m;
+}
+
+void predict_raw(const DataSet &ds, const std::vector<std::vector<Tree>> &model, float learning_rate, float base_score,
+                 std::vector<float> &out, float *kernel_ms) {
+    const ModelRef m = model_ref(model);
+    out.assign((size_t)ds.n_rows * m.K, 0.f);
+    if (ds.n_rows == 0) return;
+    predict(ds, *make_predict_plan(m), learning_rate, base_score, OBJ_UNKNOWN, {}, out.data(), kernel_ms);
 }
 
 void predict_transform(int objective, int num_class, const std::vector<float> &label, int n_rows, std::vector<float> &y) {
