@@ -78,9 +78,12 @@ typedef struct {
     int verbose;
     int profile;        /* time the histogram and partition kernels with CUDA events */
     unsigned rank_seed; /* LambdaRank partner sampling */
-    int hist_mode;      /* histogram arithmetic: 0 fp32 -- float (g,h) added value by value into one accumulator per bin,
-                           what the reference does (hist_tree_builder_single.cu:203-216, :485-505); 1 exact -- integer sums
-                           on a fixed-point grid, bit-identical from run to run and for any number of GPUs */
+    int hist_mode;      /* histogram arithmetic: 0 fp32 -- sums of the float (g,h): in the first round added value by value
+                           into one float accumulator per bin, what the reference does in every round
+                           (hist_tree_builder_single.cu:203-216, :485-505); in later rounds integer sums on a grid of 2^-30
+                           of the round's largest gradient, closer to the true sums than any order of float additions;
+                           1 exact -- integer sums on a fixed-point grid in every round, bit-identical from run to run and
+                           for any number of GPUs */
     int bagging;        /* RowSampler::do_bagging (src/thundergbm/row_sampler.cu:9-35): bootstrap multiplicities on (g,h) */
     float column_sampling_rate; /* Shard::column_sampling (src/thundergbm/builder/shard.cu:8-23); 1 = off */
     unsigned sample_seed;       /* seed of both samplers (the reference draws from std::rand()) */

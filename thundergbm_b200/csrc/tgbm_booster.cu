@@ -23,6 +23,8 @@
 
 namespace tgbm {
 
+constexpr int FINE_SMEM = 4 * 256 * 32 * 4;   // k_hist<., true>: low and high halves of g and h, [256 bins][32 features] each
+
 struct BoosterImpl {
     GBMParam p;
     const Comm *comm = nullptr;
@@ -68,6 +70,9 @@ struct BoosterImpl {
     // fp32 mode: the same two buffers hold float pairs; `hist_spread` receives the built histograms, their cells
     // `f32_stride(pairs)` float2 apart (see tgbm_hist_f32.cuh)
     bool f32 = false;
+    // the round sums floats value by value; fp32 mode's later rounds sum integers on a grid of FINE_BITS bits
+    bool float_round(int round) const { return f32 && (exact || round < FINE_FROM_ROUND); }
+    bool last_float = false;   // hist_full holds float pairs
     DevBuf<float2> hist_spread;
     DevBuf<double> sum_partial;
     CutOffsets f32_cuts{};                 // fp32 dense kernel: first bin of every feature, passed by value
@@ -854,8 +859,10 @@ void Booster::init(const DataSet &ds) {
     m.window_rows = (1 << (31 - p.quant_bits)) - HIST_THREADS;
     TGBM_CHECK(m.window_rows >= HIST_THREADS, "quant_bits too large for the int32 accumulation window");
     m.hist_smem = 2 * 256 * 32 * 4 + 2 * 256 * 32 * 8;  // int32 accumulators + int64 totals, both [2][256 bins][32 features]
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, m.hist_smem));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, m.hist_smem));
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, m.hist_smem));
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, m.hist_smem));
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FINE_SMEM));
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FINE_SMEM));
     TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
@@ -880,7 +887,7 @@ void BoosterImpl::gradient(int round) {
     const bool pointwise = objective == REG_LINEAR || objective == REG_LOGISTIC || objective == BINARY_LOGISTIC;
     const int logistic = objective == REG_LINEAR ? 0 : 1;
     // the pass that applied the previous tree has already found this round's gradient maxima
-    const bool have_max = pointwise && grad_max_ready && round >= 0 && !f32 && !p.bagging;
+    const bool have_max = pointwise && grad_max_ready && round >= 0 && !float_round(round) && !p.bagging;
     grad_max_ready = false;
     root_sum.zero(stream);
     if (!have_max) {
@@ -906,7 +913,7 @@ void BoosterImpl::gradient(int round) {
         k_bag_scale<<<std::max(1, std::min(ceil_div((long long)N * K, 256), num_sms * 8)), 256, 0, stream>>>(gh.p, bag_count.p, (size_t)N * K, maxbits.p);
         launches += 2;
     }
-    if (f32) {  // float gradients as they are; root sums in fp64, block partials combined in a fixed order
+    if (float_round(round)) {  // float gradients as they are; root sums in fp64, block partials combined in a fixed order
         k_sum_gh<<<dim3(SUM_BLOCKS, K), 256, 0, stream>>>(gh.p, N, sum_partial.p);
         k_sum_gh_final<<<K, 32, 0, stream>>>(sum_partial.p, SUM_BLOCKS, reinterpret_cast<double *>(root_sum.p));
         launches += 2;
@@ -915,8 +922,12 @@ void BoosterImpl::gradient(int round) {
     }
     if (comm && comm->active()) comm->allreduce(maxbits.p, 2, Comm::U32, Comm::MAX, stream);
     const int blocks = std::max(1, std::min(ceil_div(N, tb), num_sms * 8));
-    k_quantize<<<dim3(blocks, K), tb, 0, stream>>>(have_max ? nullptr : gh.p, N, maxbits.p, p.quant_bits, (uint32_t)round, (uint32_t)row_offset,
-                                                   ghq.p, root_sum.p, qinfo.p, y.p, ypred.p, logistic, round >= 0 ? rstate.p : nullptr);
+    auto quantize = [&](auto kern, int bits) {
+        kern<<<dim3(blocks, K), tb, 0, stream>>>(have_max ? nullptr : gh.p, N, maxbits.p, bits, (uint32_t)round, (uint32_t)row_offset,
+                                                 ghq.p, root_sum.p, qinfo.p, y.p, ypred.p, logistic, round >= 0 ? rstate.p : nullptr);
+    };
+    if (f32) quantize(k_quantize<true>, FINE_BITS);
+    else quantize(k_quantize<false>, p.quant_bits);
     ++launches;
     if (comm && comm->active()) comm->allreduce(root_sum.p, 2 * (size_t)K, Comm::I64, Comm::SUM, stream);
 }
@@ -954,7 +965,9 @@ void BoosterImpl::init_base_score() {
 
 void BoosterImpl::build_tree(int round, int k) {
     const int tree_index = round * K + k;
-    // fp32 mode: the records carry the float gradient pairs themselves (same 8 bytes)
+    const bool f32 = float_round(round), fine = this->f32 && !f32;
+    last_float = f32;
+    // float rounds: the records carry the float gradient pairs themselves (same 8 bytes)
     const int2 *gq = f32 ? reinterpret_cast<const int2 *>(gh.p + (size_t)k * N) : ghq.p + (size_t)k * N;
     const int hist_ctas = std::min(num_sms, HIST_MAX_CTAS);
     k_tree_init<<<ceil_div(n_nodes, 256), 256, 0, stream>>>(nodes.p, n_nodes, root_sum.p + 2 * k, qinfo.p, p.lambda, N,
@@ -1008,12 +1021,14 @@ void BoosterImpl::build_tree(int round, int k) {
             else
                 k_hist_sparse<true><<<sp_ctas, SPARSE_THREADS, sp_smem, stream>>>(sp_row_ptr.p, sp_bin.p, idx_in, gh_in, hist_work.p,
                                                                                   hist_tile_base.p, ctl.p, built, B);
-        } else if (level == 0)
-            k_hist<false><<<dim3(hist_ctas, G), HIST_THREADS, hist_smem, stream>>>(bins.p, Fpad, F, nullptr, gh_in, hist_cta_off.p, hist_seq.p,
-                                                                                   cut_ptr.p, cut_fid.p, built, B, window_rows);
-        else
-            k_hist<true><<<dim3(hist_ctas, G), HIST_THREADS, hist_smem, stream>>>(bins.p, Fpad, F, idx_in, gh_in, hist_cta_off.p, hist_seq.p,
-                                                                                  cut_ptr.p, cut_fid.p, built, B, window_rows);
+        } else {
+            auto hist = [&](auto kern) {
+                kern<<<dim3(hist_ctas, G), HIST_THREADS, fine ? FINE_SMEM : hist_smem, stream>>>(bins.p, Fpad, F, idx_in, gh_in, hist_cta_off.p,
+                                                                                                hist_seq.p, cut_ptr.p, cut_fid.p, built, B, window_rows);
+            };
+            if (level == 0) { if (fine) hist(k_hist<false, true>); else hist(k_hist<false, false>); }
+            else { if (fine) hist(k_hist<true, true>); else hist(k_hist<true, false>); }
+        }
         if (profile_on) { cudaEventRecord(ev.b, stream); events.push_back(ev); }
         int bs_eval = bs;   // distance of the cells the split search reads
         if (comm && comm->active()) {
@@ -1267,7 +1282,7 @@ HistProfile Booster::profile() {
     const TreeCtl &c0 = m.stat_base;
     r.hist_root_bytes = (double)(c.stat_rows_root - c0.stat_rows_root) * (row_bytes + 8);
     r.hist_bytes = r.hist_root_bytes + (double)(c.stat_rows_gather - c0.stat_rows_gather) * (row_bytes + 8 + 4) +
-                   (double)(c.stat_hists - c0.stat_hists) * m.B * (m.f32 ? 8.0 : 16.0);
+                   (double)(c.stat_hists - c0.stat_hists) * m.B * (m.last_float ? 8.0 : 16.0);
     r.partition_bytes = (double)(c.stat_part_rows - c0.stat_part_rows) * (4 + 1 + 4);
     r.hist_rows = (long long)((c.stat_rows_root - c0.stat_rows_root) + (c.stat_rows_gather - c0.stat_rows_gather));
     r.kernel_launches = m.launches;
@@ -1325,7 +1340,12 @@ std::vector<long long> Booster::get_root_hist() {
 std::vector<float> Booster::get_root_hist_f32() {
     sync();
     TGBM_CHECK(impl_->f32, "exact mode keeps integer histograms: use get_root_hist");
-    return to_host(reinterpret_cast<const float *>(impl_->hist_full.p), (size_t)impl_->B * 2);
+    if (impl_->last_float) return to_host(reinterpret_cast<const float *>(impl_->hist_full.p), (size_t)impl_->B * 2);
+    const auto h = to_host(impl_->hist_full.p, (size_t)impl_->B * 2);
+    const QuantInfo q = to_host(impl_->qinfo.p, 1)[0];
+    std::vector<float> out(h.size());
+    for (size_t i = 0; i < h.size(); ++i) out[i] = (float)((double)h[i] * ((i & 1) ? q.inv_sh : q.inv_sg));
+    return out;
 }
 std::vector<double> Booster::get_quant_scale() {
     sync();

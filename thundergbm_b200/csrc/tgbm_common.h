@@ -77,10 +77,11 @@ struct GBMParam {
     int n_device = 1;
     std::string tree_method = "auto";
     // additions of this implementation
-    // Histogram arithmetic.  0 "fp32": float (g,h) added per stored value into one accumulator per bin, float prefix
-    // sums -- the reference's own arithmetic (hist_tree_builder_single.cu:203-216), results depend on the order of
-    // the additions in the last bits.  1 "exact": gradients on a power-of-two grid, integer sums -- the deterministic
-    // mode: bit-identical from run to run and for any number of GPUs.
+    // Histogram arithmetic.  0 "fp32": sums of the float (g,h).  First round: added per stored value into one float
+    // accumulator per bin, float prefix sums -- the reference's own arithmetic (hist_tree_builder_single.cu:203-216),
+    // results depend on the order of the additions in the last bits.  Later rounds: integer sums on a grid of 2^-30 of the
+    // round's largest gradient (see FINE_FROM_ROUND).  1 "exact": gradients on a coarser, dithered power-of-two grid in
+    // every round -- the deterministic mode: bit-identical from run to run and for any number of GPUs.
     int hist_mode = 0;
     // 0: cut points, candidate order and child sums of the one-device builder (HistTreeBuilder_single, what the
     // reference runs for n_device = 1).  D >= 1: those of the column-sharded HistTreeBuilder the reference runs for

@@ -23,6 +23,9 @@ constexpr int PART_THREADS = 512;  // 512 x 4 records per tile measured best (10
 constexpr int PART_RPT = 4;         // records per thread
 constexpr int PART_TILE = PART_THREADS * PART_RPT;
 constexpr int MISSING_BIN = 255;
+constexpr int FINE_BITS = 30;          // value bits of the grid of fp32 mode's later rounds
+constexpr int FINE_WINDOW = 1 << 16;   // rows whose 16-bit low halves fit an unsigned accumulator
+constexpr int FINE_FROM_ROUND = 1;     // fp32 mode: rounds before it sum floats value by value (k_hist_f32)
 
 struct HistWork {  // one histogram to build at a level
     int begin, count, slab;
@@ -347,8 +350,12 @@ static __global__ void k_grad_softmax(const float *__restrict__ y, const float *
 // round-to-nearest would move every row that carries the same gradient the same way (in the first round all rows
 // of a class do), and those shifts would add up coherently in the histogram sums.
 //
+// FINE (fp32 mode from the second round on, FINE_BITS value bits): rounded to nearest -- the grid is 2^-30 of the largest
+// gradient, finer than the last bit of any float sum that a bin of the reference could hold.
+//
 // `gh` null: the gradients are those of a pointwise objective (`logistic` 0/1) and are computed again from y and the
 // scores here -- the pass that found their maxima (k_predict_walk) did not store them.
+template <bool FINE>
 static __global__ void k_quantize(const float2 *__restrict__ gh, int n, const unsigned *__restrict__ maxbits, int quant_bits,
                            uint32_t round, uint32_t row_offset, int2 *__restrict__ ghq,
                            unsigned long long *__restrict__ root_sum, QuantInfo *__restrict__ qinfo,
@@ -365,10 +372,15 @@ static __global__ void k_quantize(const float2 *__restrict__ gh, int n, const un
     long long tg = 0, th = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float2 v = gh ? gh[(size_t)k * n + i] : pointwise_gh(logistic, y[i], yp[i]);
+        int qg, qh;
+        if (FINE) {
+            qg = __double2int_rn((double)v.x * sg); qh = __double2int_rn((double)v.y * sh);
+        } else {
         const uint32_t row = row_offset + (uint32_t)i;
         const double ug = (double)mix32(0x9E3779B9u, round, (uint32_t)k, row) * (1.0 / 4294967296.0);
         const double uh = (double)mix32(0x9E3779B9u + 1u, round, (uint32_t)k, row) * (1.0 / 4294967296.0);
-        const int qg = (int)__double2ll_rd((double)v.x * sg + ug), qh = (int)__double2ll_rd((double)v.y * sh + uh);
+        qg = (int)__double2ll_rd((double)v.x * sg + ug); qh = (int)__double2ll_rd((double)v.y * sh + uh);
+        }
         ghq[(size_t)k * n + i] = make_int2(qg, qh);
         tg += qg; th += qh;
     }
@@ -637,20 +649,29 @@ __device__ __forceinline__ void xor_permute_half(uint32_t (&w)[4], int key) {
 // Persistent CTAs, one per SM; grid = (ctas, feature groups of 32).  Each CTA visits the tiles the level's plan
 // gave it (see hist_sequence).  A lane holds one 16-feature half of two rows; the shared-memory
 // accumulators are laid out [bin][32 features] so that the bank is the feature index, and at step j the 32 lanes
-// of a warp handle 32 different features, so every shared atomic of a warp hits 32 different banks.  Accumulators are int32.  Before they could overflow
-// (`window_rows` rows of at most 2^quant_bits each) they are drained into int64 totals, also in shared
-// memory; the totals go to the node's int64 histogram in global memory when the CTA moves on to another
-// node and at the end.
-template <bool GATHER>
+// of a warp handle 32 different features, so every shared atomic of a warp hits 32 different banks.
+//
+// !FINE (exact mode, values of at most quant_bits bits): accumulators are int32.  Before they could overflow
+// (`window_rows` rows of at most 2^quant_bits each) they are drained into int64 totals, also in shared memory.
+// FINE (fp32 mode after its first round, values of FINE_BITS bits and a sign): a value is added in two halves, the low 16
+// bits to an unsigned accumulator and the rest to a signed one.  Two plain 32-bit atomics per component are the cheapest
+// exact 31-bit addition there is: the bare shared-memory atomics of 294 M (row, feature) pairs take 0.134 ms so, 0.188 ms
+// as one returning atomic with a carry test, 0.290 ms as one 64-bit atomic, 0.320 ms as float atomics (compare-and-swap
+// loops); 0.073 ms with one 32-bit atomic per component.  FINE_WINDOW rows fill the low halves.
+// Totals or halves go to the node's int64 histogram in global memory when the CTA moves on to another node and at the end.
+template <bool GATHER, bool FINE>
 static __global__ void __launch_bounds__(HIST_THREADS, 1)
 k_hist(const unsigned char *__restrict__ bins, int Fpad, int F, const int *__restrict__ rec_idx,
        const int2 *__restrict__ rec_gh, const int *__restrict__ cta_off, const int4 *__restrict__ seq,
        const int *__restrict__ cut_ptr, const int *__restrict__ cut_fid,
        long long *__restrict__ slab, int B, int window_rows) {
-    extern __shared__ __align__(16) int sh_hist[];  // int32 g,h: [2][256][32]; int64 totals g,h: [2][256][32]
+    // int32 g,h: [2][256][32], then int64 totals g,h: [2][256][32]; FINE: low halves of g,h, high halves of g,h
+    extern __shared__ __align__(16) int sh_hist[];
+    constexpr int CELLS = 256 * 32;
     int *acc = sh_hist;
-    int *hg = acc;  // g accumulators; the h accumulators follow at +256*32
-    long long *tot = reinterpret_cast<long long *>(sh_hist + 2 * 256 * 32);
+    int *hg = acc;  // g accumulators; the h accumulators follow at +CELLS
+    long long *tot = reinterpret_cast<long long *>(sh_hist + 2 * CELLS);
+    int *high = sh_hist + 2 * CELLS;
 
     const int group = blockIdx.y;
     const int f0 = group * 32;
@@ -658,13 +679,13 @@ k_hist(const unsigned char *__restrict__ bins, int Fpad, int F, const int *__res
     const int lane = threadIdx.x & 31;
     const int i2 = cta_off[blockIdx.x], i_end = cta_off[blockIdx.x + 1];  // the CTA's tiles in seq[], see hist_sequence
     if (i2 >= i_end) return;
-    for (int i = threadIdx.x; i < 2 * 256 * 32; i += HIST_THREADS) { acc[i] = 0; tot[i] = 0; }
+    for (int i = threadIdx.x; i < (FINE ? 4 : 6) * CELLS; i += HIST_THREADS) sh_hist[i] = 0;
     __syncthreads();
 
     auto drain = [&]() {  // int32 window -> int64 totals, same [bin][feature] layout
         __syncthreads();
 #pragma unroll 4
-        for (int i = threadIdx.x; i < 2 * 256 * 32; i += HIST_THREADS) {
+        for (int i = threadIdx.x; i < 2 * CELLS; i += HIST_THREADS) {
             const int v = acc[i];
             if (v) { tot[i] += v; acc[i] = 0; }
         }
@@ -681,8 +702,15 @@ k_hist(const unsigned char *__restrict__ bins, int Fpad, int F, const int *__res
 #pragma unroll 2
         for (int i = threadIdx.x >> 5; i < 256; i += HIST_THREADS / 32) {
             const int s = i * 32 + flush_f;
-            const long long vg = tot[s] + acc[s], vh = tot[256 * 32 + s] + acc[256 * 32 + s];
-            tot[s] = 0; tot[256 * 32 + s] = 0; acc[s] = 0; acc[256 * 32 + s] = 0;
+            long long vg, vh;
+            if (FINE) {
+                vg = ((long long)high[s] << 16) + (unsigned)acc[s]; vh = ((long long)high[CELLS + s] << 16) + (unsigned)acc[CELLS + s];
+                high[s] = 0; high[CELLS + s] = 0;
+            } else {
+                vg = tot[s] + acc[s]; vh = tot[CELLS + s] + acc[CELLS + s];
+                tot[s] = 0; tot[CELLS + s] = 0;
+            }
+            acc[s] = 0; acc[CELLS + s] = 0;
             if (i < flush_nb) {
                 if (vg) atomicAdd(dst + 2 * i, (unsigned long long)vg);
                 if (vh) atomicAdd(dst + 2 * i + 1, (unsigned long long)vh);
@@ -748,11 +776,11 @@ k_hist(const unsigned char *__restrict__ bins, int Fpad, int F, const int *__res
         prefetch_rows();
         r1a = r2a; r1b = r2b;
         ids(i + 3, r2a, r2b);
-        if (slab_this != slab_cur) {  // the tile belongs to another node: hand the finished one over
+        if (slab_this != slab_cur || (FINE && since + HIST_THREADS > FINE_WINDOW)) {  // the tile belongs to another node: hand the finished one over
             flush(slab_cur);
             slab_cur = slab_this;
             since = 0;
-        } else if (since + HIST_THREADS > window_rows) {
+        } else if (!FINE && since + HIST_THREADS > window_rows) {
             drain();
             since = 0;
         }
@@ -763,6 +791,17 @@ k_hist(const unsigned char *__restrict__ bins, int Fpad, int F, const int *__res
         // mask.  No test for missing values: bin 255 (missing, and the padding columns beyond F) lands in row 255
         // of the table, which no feature ever reads back.
         char *const gbase = reinterpret_cast<char *>(hg);
+        auto add = [&](uint32_t off, const int2 v) {
+            if (FINE) {
+                atomicAdd(reinterpret_cast<unsigned *>(gbase + off), (unsigned)v.x & 0xffffu);
+                atomicAdd(reinterpret_cast<unsigned *>(gbase + off + CELLS * 4), (unsigned)v.y & 0xffffu);
+                atomicAdd(reinterpret_cast<int *>(gbase + off + 2 * CELLS * 4), v.x >> 16);
+                atomicAdd(reinterpret_cast<int *>(gbase + off + 3 * CELLS * 4), v.y >> 16);
+            } else {
+                atomicAdd(reinterpret_cast<int *>(gbase + off), v.x);
+                atomicAdd(reinterpret_cast<int *>(gbase + off + CELLS * 4), v.y);
+            }
+        };
         if (oka) {
             uint32_t w[4] = {a.x, a.y, a.z, a.w};
             xor_permute_half(w, lane >> 1);
@@ -771,8 +810,7 @@ k_hist(const unsigned char *__restrict__ bins, int Fpad, int F, const int *__res
                 const uint32_t word = w[j >> 2];
                 const uint32_t binoff = ((j & 3) == 0 ? (word << 7) : (word >> (8 * (j & 3) - 7))) & 0x7f80u;
                 const uint32_t off = binoff | (laneoff ^ (4u * j));
-                atomicAdd(reinterpret_cast<int *>(gbase + off), va.x);
-                atomicAdd(reinterpret_cast<int *>(gbase + off + 256 * 32 * 4), va.y);
+                add(off, va);
             }
         }
         if (okb) {
@@ -783,8 +821,7 @@ k_hist(const unsigned char *__restrict__ bins, int Fpad, int F, const int *__res
                 const uint32_t word = w[j >> 2];
                 const uint32_t binoff = ((j & 3) == 0 ? (word << 7) : (word >> (8 * (j & 3) - 7))) & 0x7f80u;
                 const uint32_t off = binoff | (laneoff ^ (4u * j));
-                atomicAdd(reinterpret_cast<int *>(gbase + off), vb.x);
-                atomicAdd(reinterpret_cast<int *>(gbase + off + 256 * 32 * 4), vb.y);
+                add(off, vb);
             }
         }
     }
