@@ -17,20 +17,17 @@
 
 #include "tgbm_input.h"
 #include "tgbm_kernels.cuh"
+#include "tgbm_level.cuh"
 #include "tgbm_hist_f32.cuh"
 #include "tgbm_exact.cuh"
 #include "tgbm_rank.cuh"
 
 namespace tgbm {
 
-constexpr int FINE_SMEM = 4 * 256 * 32 * 4;   // k_hist<., true>: low and high halves of g and h, [256 bins][32 features] each
-
 struct BoosterImpl {
     GBMParam p;
     const Comm *comm = nullptr;
     cudaStream_t stream = nullptr;
-    cudaStream_t stream2 = nullptr;          // side stream for planning kernels that run beside the scatter
-    cudaEvent_t ev_scan = nullptr, ev_plan = nullptr;
     int objective = REG_LINEAR;
     int N = 0, F = 0, Fpad = 0, G = 0, B = 0, K = 1, n_nodes = 0, depth = 0;
     long long N_global = 0;
@@ -62,9 +59,13 @@ struct BoosterImpl {
     DevBuf<unsigned long long> root_sum;
     DevBuf<QuantInfo> qinfo, qinfo_log;
     DevBuf<TreeNode> nodes, model;
+    // the trees of a round are built in batches of `batch` (see Batch): one tree's share of the buffers below lies a
+    // stride behind the one before
+    int batch = 1;
+    Batch bufs{};
     DevBuf<int> rec_idx[2];
     DevBuf<int2> rec_gh[2];
-    DevBuf<int> seg_begin[2], seg_cnt[2], gcnt;
+    DevBuf<int> seg_begin[2], seg_cnt[2];
     DevBuf<int> nid_keep;
     DevBuf<long long> hist_full, hist_built;
     // fp32 mode: the same two buffers hold float pairs; `hist_spread` receives the built histograms, their cells
@@ -73,6 +74,7 @@ struct BoosterImpl {
     // the round sums floats value by value; fp32 mode's later rounds sum integers on a grid of FINE_BITS bits
     bool float_round(int round) const { return f32 && (exact || round < FINE_FROM_ROUND); }
     bool last_float = false;   // hist_full holds float pairs
+    size_t last_tree_full = 0; // where the histograms of the tree built last start in it
     DevBuf<float2> hist_spread;
     DevBuf<double> sum_partial;
     CutOffsets f32_cuts{};                 // fp32 dense kernel: first bin of every feature, passed by value
@@ -89,8 +91,6 @@ struct BoosterImpl {
         while (s > 1 && (size_t)s * pairs * std::max(B, 1) > spread_cells) s >>= 1;
         return s;
     }
-    DevBuf<int> built_right, hist_tile_base;
-    DevBuf<HistWork> hist_work;
     bool prune_in_smem = true;
     TreeCtl stat_base{};  // counters of `ctl` when profiling was switched on
     DevBuf<RoundState> rstate;          // device copy of `rounds`
@@ -100,22 +100,16 @@ struct BoosterImpl {
     bool graphs_allowed = true;
     void run_round(int round);
     DevBuf<int> eval_ticket;  // k_eval: finished blocks per sibling pair, zero between launches
+    int part_ctas = 1;
     bool grad_max_ready = false;        // maxbits holds the maxima of the next round's gradients
     bool metric_partial_ready = false;  // metric_partial holds the finished round's partial sums
     int metric_blocks() const { return std::max(1, std::min((N + 255) / 256, 1024)); }
-    DevBuf<int> hist_cta_off;  // dense histogram kernel: tile sequence of every CTA
-    DevBuf<int4> hist_seq;
     DevBuf<SplitRec> recs;
-    DevBuf<int> node_tile0[2], tile_left, tile_node[2];
-    DevBuf<int> part_base;                    // single-pass partition: records of the nodes before a node
-    DevBuf<unsigned long long> part_status;   // single-pass partition: left count of every tile
-    DevBuf<unsigned long long> part_group;    // ... and of every aligned group of 32 tiles (count of contributors << 32 | sum)
-    bool part_one = false;
+    DevBuf<int> tile_left, tail_left;
     DevBuf<unsigned> bits;
     DevBuf<TreeCtl> ctl;
     DevBuf<double> metric_partial, metric_sum;
     int max_tiles = 0;
-    int hist_smem = 0;
     RankState rank;
 
     struct TimedEvent { cudaEvent_t a, b; int kind; };
@@ -125,13 +119,9 @@ struct BoosterImpl {
 
     ~BoosterImpl() {
         if (stream) cudaStreamSynchronize(stream);    // nothing of this booster is in flight when its buffers go
-        if (stream2) cudaStreamSynchronize(stream2);
         for (auto &e : events) { cudaEventDestroy(e.a); cudaEventDestroy(e.b); }
         if (round_exec) cudaGraphExecDestroy(round_exec);
         if (round_graph) cudaGraphDestroy(round_graph);
-        if (ev_scan) cudaEventDestroy(ev_scan);
-        if (ev_plan) cudaEventDestroy(ev_plan);
-        if (stream2) cudaStreamDestroy(stream2);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -155,9 +145,8 @@ struct BoosterImpl {
     void column_builder_candidates(DevBuf<unsigned long long> &ukeys, DevBuf<long long> &ucopies, long long &nu);
     void init_base_score();
     void gradient(int round);
-    void build_tree(int round, int k);
+    void build_trees(int round, int k0, int n_trees);
     void round_metric(int round);
-    size_t full_offset(int level) const { return ((size_t)(1 << level) - 1) * B * 2; }
 };
 
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
@@ -644,17 +633,17 @@ void BoosterImpl::exact_levels(int k, const void *gh_rows) {
 void BoosterImpl::build_tree_exact(int round, int k) {
     const int tree_index = round * K + k;
     k_tree_init<<<ceil_div(n_nodes, 256), 256, 0, stream>>>(nodes.p, n_nodes, root_sum.p + 2 * k, qinfo.p, p.lambda, N,
-                                                            seg_begin[0].p, seg_cnt[0].p, gcnt.p, ctl.p, f32 ? 1 : 0);
+                                                            seg_begin[0].p, seg_cnt[0].p, bufs.seg_stride, f32 ? 1 : 0);
     if (f32) exact_levels<float>(k, gh.p + (size_t)k * N);
     else exact_levels<long long>(k, ghq.p + (size_t)k * N);
-    k_prune<<<1, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream>>>(nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0);
+    k_prune<<<1, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream>>>(nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0, model.p, K, k,
+                                                                                         rstate.p);
     if (N) {
         int *nid_out = p.keep_nid ? nid_keep.p + (size_t)tree_index * N : nullptr;
         k_exact_predict<<<std::min(ceil_div(N, 256), num_sms * 8), 256, 0, stream>>>(ex_nid.p, N, nodes.p, p.learning_rate, ypred.p + (size_t)k * N, nid_out);
     }
     grad_max_ready = metric_partial_ready = false;
-    k_store_tree<<<std::min(ceil_div(n_nodes, 256), 64), 256, 0, stream>>>(nodes.p, model.p, n_nodes, K, k, rstate.p);
-    launches += 4;
+    launches += 3;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -679,9 +668,6 @@ void Booster::init(const DataSet &ds) {
     TGBM_CUDA(cudaGetDevice(&dev));
     TGBM_CUDA(cudaDeviceGetAttribute(&m.num_sms, cudaDevAttrMultiProcessorCount, dev));
     TGBM_CUDA(cudaStreamCreateWithFlags(&m.stream, cudaStreamNonBlocking));
-    TGBM_CUDA(cudaStreamCreateWithFlags(&m.stream2, cudaStreamNonBlocking));
-    TGBM_CUDA(cudaEventCreateWithFlags(&m.ev_scan, cudaEventDisableTiming));
-    TGBM_CUDA(cudaEventCreateWithFlags(&m.ev_plan, cudaEventDisableTiming));
     m.N = ds.n_rows;
     m.F = ds.n_features;
     m.depth = p.depth;
@@ -806,23 +792,53 @@ void Booster::init(const DataSet &ds) {
         TGBM_CUDA(cudaStreamSynchronize(m.stream));
     }
     m.qinfo_log.alloc(std::max(p.n_trees, 1) + 1);
-    m.nodes.alloc(m.n_nodes);
+    const size_t B1 = std::max(m.B, 1);
+    const int max_pairs = std::max(1, 1 << std::max(0, depth - 2));
+    m.max_tiles = ceil_div(N, PART_TILE) + (1 << depth) + 2;
+    {
+        // trees built side by side: all of a round's while their buffers stay within 6 GB
+        Batch &b = m.bufs;
+        b.half = (int)n1;
+        b.nodes_stride = m.n_nodes;
+        b.seg_stride = (size_t)1 << depth;
+        // left children in the first half, right children in the second; the bulk copies that stage a unit of records read
+        // up to a unit beyond the last record, from a 16-byte boundary
+        b.rec_stride = (2 * n1 + 2 * F32_THREADS + 3) / 4 * 4;
+        b.gh_stride = N;
+        b.full_stride = (((size_t)1 << depth) - 1) * B1 * 2;
+        b.built_stride = max_pairs * B1 * 2;
+        b.recs_stride = m.exact ? 1 : ((size_t)1 << (depth - 1)) * (m.sparse ? std::max(m.n_chunks, 1) : m.F);
+        b.bits_stride = (size_t)m.max_tiles * (PART_TILE / 32);
+        b.tile_stride = m.max_tiles;
+        b.ticket_stride = max_pairs;
+        const double per_tree = 24.0 * b.rec_stride + 8.0 * (b.full_stride + b.built_stride) + 4.0 * b.bits_stride;
+        m.batch = m.exact ? 1 : std::max(1, std::min(K, (int)(6e9 / per_tree)));
+        m.part_ctas = std::max(1, std::min(m.max_tiles, m.num_sms * (2048 / PART_THREADS) / m.batch));
+        b.tail_stride = m.part_ctas;
+        const size_t T = m.batch;
+        m.nodes.alloc(T * b.nodes_stride); b.nodes = m.nodes.p;
+        for (int i = 0; i < 2; ++i) {
+            m.rec_idx[i].alloc(T * b.rec_stride); m.rec_gh[i].alloc(T * b.rec_stride);
+            m.seg_begin[i].alloc(T * b.seg_stride); m.seg_cnt[i].alloc(T * b.seg_stride);
+            m.seg_begin[i].zero(m.stream); m.seg_cnt[i].zero(m.stream);
+            b.rec_idx[i] = m.rec_idx[i].p; b.rec_gh[i] = m.rec_gh[i].p;
+            b.seg_begin[i] = m.seg_begin[i].p; b.seg_cnt[i] = m.seg_cnt[i].p;
+        }
+        m.hist_full.alloc(T * b.full_stride); b.hist_full = m.hist_full.p;
+        m.hist_built.alloc(T * b.built_stride); b.hist_built = m.hist_built.p;
+        m.hist_built.zero(m.stream);   // the split search leaves it zeroed
+        m.recs.alloc(T * b.recs_stride); b.recs = m.recs.p;
+        m.bits.alloc(T * b.bits_stride); b.bits = m.bits.p;
+        m.tile_left.alloc(T * b.tile_stride); b.tile_left = m.tile_left.p;
+        m.tail_left.alloc(T * b.tail_stride); b.tail_left = m.tail_left.p;
+        m.eval_ticket.alloc(T * b.ticket_stride); b.ticket = m.eval_ticket.p;
+        m.eval_ticket.zero(m.stream);
+        m.ctl.alloc(1); b.ctl = m.ctl.p;
+        m.ctl.zero(m.stream);
+    }
     m.model.alloc((size_t)std::max(p.n_trees, 1) * K * m.n_nodes);
     m.metric.alloc(std::max(p.n_trees, 1));
-    for (int i = 0; i < 2; ++i) {
-        // left children in the first half, right children in the second (single-pass partition); the bulk copies that
-        // stage a unit of records read up to a unit beyond the last record
-        m.rec_idx[i].alloc(2 * n1 + 2 * F32_THREADS); m.rec_gh[i].alloc(2 * n1 + 2 * F32_THREADS);
-        m.seg_begin[i].alloc((size_t)1 << depth); m.seg_cnt[i].alloc((size_t)1 << depth);
-        m.seg_begin[i].zero(m.stream); m.seg_cnt[i].zero(m.stream);
-    }
-    m.gcnt.alloc((size_t)1 << depth);
-    m.gcnt.zero(m.stream);
     if (p.keep_nid) m.nid_keep.alloc(n1 * K * std::max(p.n_trees, 1));
-    const size_t B1 = std::max(m.B, 1);
-    m.hist_full.alloc((((size_t)1 << depth) - 1) * B1 * 2);
-    m.hist_built.alloc(std::max<size_t>(1, (size_t)1 << std::max(0, depth - 2)) * B1 * 2);
-    const int max_pairs = std::max(1, 1 << std::max(0, depth - 2));
     if (m.f32) {
         for (int f = 0; f < std::min(m.F, 256); ++f) m.f32_cuts.v[f] = m.h_cut_ptr[f];
         m.spread_cells = std::max<size_t>(std::min<size_t>((size_t)32 * max_pairs * B1, (size_t)8 << 20), (size_t)max_pairs * B1);  // <= 64 MB
@@ -832,44 +848,25 @@ void Booster::init(const DataSet &ds) {
         TGBM_CUDA(cudaMemcpyAsync(m.qinfo.p, &one, sizeof(one), cudaMemcpyHostToDevice, m.stream));
         TGBM_CUDA(cudaStreamSynchronize(m.stream));
     }
-    m.built_right.alloc(max_pairs); m.hist_work.alloc(max_pairs); m.hist_tile_base.alloc(max_pairs + 1);
-    m.hist_cta_off.alloc((size_t)m.num_sms + 1);
-    m.eval_ticket.alloc(max_pairs);
     m.rstate.alloc(1);
     m.rstate.zero(m.stream);
     m.graphs_allowed = getenv("TGBM_NO_GRAPH") == nullptr;
-    m.eval_ticket.zero(m.stream);
-    m.hist_seq.alloc((size_t)ceil_div(std::max(N, 1), HIST_THREADS) + max_pairs + 16);
-    m.recs.alloc(m.exact ? 1 : ((size_t)1 << (depth - 1)) * (m.sparse ? std::max(m.n_chunks, 1) : m.F));
-    m.max_tiles = ceil_div(N, PART_TILE) + (1 << depth) + 2;
-    m.tile_left.alloc(m.max_tiles);
-    m.tile_node[0].alloc(m.max_tiles); m.tile_node[1].alloc(m.max_tiles);
-    m.node_tile0[0].alloc(((size_t)1 << depth) + 1); m.node_tile0[1].alloc(((size_t)1 << depth) + 1);
-    m.bits.alloc((size_t)m.max_tiles * (PART_TILE / 32));
-    m.part_base.alloc((size_t)1 << depth);
-    m.part_status.alloc(m.max_tiles);
-    m.part_status.zero(m.stream);
-    m.part_group.alloc(m.max_tiles / 32 + 2);
-    m.part_group.zero(m.stream);
-    m.part_one = getenv("TGBM_PART_ONE") != nullptr;
     m.f32_staged = getenv("TGBM_NO_BULK_COPY") == nullptr;
-    m.ctl.alloc(1);
-    m.ctl.zero(m.stream);
     m.metric_partial.alloc(1024); m.metric_sum.alloc(1);
     m.window_rows = (1 << (31 - p.quant_bits)) - HIST_THREADS;
     TGBM_CHECK(m.window_rows >= HIST_THREADS, "quant_bits too large for the int32 accumulation window");
-    m.hist_smem = 2 * 256 * 32 * 4 + 2 * 256 * 32 * 8;  // int32 accumulators + int64 totals, both [2][256 bins][32 features]
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, m.hist_smem));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, m.hist_smem));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FINE_SMEM));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FINE_SMEM));
+    const int table = 4 * (max_pairs + 1);   // tiles before every pair of the deepest level
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_EXACT_SMEM + table));
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_EXACT_SMEM + table));
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
     TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16));
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
+    TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
     m.prune_in_smem = sizeof(TreeNode) * (size_t)m.n_nodes <= 200 * 1024;  // up to depth 11
-    if (m.prune_in_smem && sizeof(TreeNode) * (size_t)m.n_nodes > 48 * 1024)
+    if (m.prune_in_smem && sizeof(TreeNode) * (size_t)m.n_nodes > 40 * 1024)   // (the kernel has static shared memory beside it)
         TGBM_CUDA(cudaFuncSetAttribute(k_prune, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(TreeNode) * (size_t)m.n_nodes)));
     if (need_group_file(m.objective)) m.rank.init(ds, m.objective, m.N, m.stream, first_group, total_groups);
     });
@@ -963,193 +960,132 @@ void BoosterImpl::init_base_score() {
     if (N) k_fill<<<std::min(ceil_div(N, 256), num_sms * 8), 256, 0, stream>>>(ypred.p, (size_t)N, w);
 }
 
-void BoosterImpl::build_tree(int round, int k) {
-    const int tree_index = round * K + k;
-    const bool f32 = float_round(round), fine = this->f32 && !f32;
-    last_float = f32;
+// Trees k0 .. k0 + n_trees - 1 of the round, level by level side by side (n_trees <= batch).
+void BoosterImpl::build_trees(int round, int k0, int n_trees) {
+    const bool float_sums = float_round(round), fine = f32 && !float_sums;
+    last_float = float_sums;
+    last_tree_full = (size_t)(n_trees - 1) * bufs.full_stride;
+    Batch b = bufs;
     // float rounds: the records carry the float gradient pairs themselves (same 8 bytes)
-    const int2 *gq = f32 ? reinterpret_cast<const int2 *>(gh.p + (size_t)k * N) : ghq.p + (size_t)k * N;
-    const int hist_ctas = std::min(num_sms, HIST_MAX_CTAS);
-    k_tree_init<<<ceil_div(n_nodes, 256), 256, 0, stream>>>(nodes.p, n_nodes, root_sum.p + 2 * k, qinfo.p, p.lambda, N,
-                                                            seg_begin[0].p, seg_cnt[0].p, gcnt.p, ctl.p, f32 ? 1 : 0);
-    k_plan_root<<<1, 1024, 0, stream>>>(seg_begin[0].p, seg_cnt[0].p, gcnt.p, nodes.p, built_right.p, hist_work.p, hist_tile_base.p,
-                                        node_tile0[0].p, ctl.p, hist_ctas, hist_cta_off.p, hist_seq.p, depth, tile_node[0].p, part_base.p,
-                                        seg_begin[1].p, seg_cnt[1].p, part_group.p, (int)part_group.n);
-    launches += 2;
+    b.gh = float_sums ? reinterpret_cast<const int2 *>(gh.p + (size_t)k0 * N) : ghq.p + (size_t)k0 * N;
+    k_tree_init<<<dim3(ceil_div(n_nodes, 256), n_trees), 256, 0, stream>>>(nodes.p, n_nodes, root_sum.p + 2 * k0, qinfo.p, p.lambda, N,
+                                                                           seg_begin[0].p, seg_cnt[0].p, b.seg_stride, float_sums ? 1 : 0);
+    ++launches;
     const int by_hessian = (comm && comm->active()) ? 1 : 0;
     const int colb = p.column_shards > 0 ? 1 : 0;  // candidates, tie rule and child sums of the column-sharded builder
-    const int part_ctas = std::max(1, std::min(max_tiles, num_sms * (2048 / PART_THREADS)));
+    // one CTA per SM over all trees and feature groups: every further CTA is one more flush per node
+    const int hist_ctas = std::max(1, num_sms / (n_trees * (sparse ? 1 : G)));
     for (int level = 0; level < depth; ++level) {
-        const int cur = level & 1, nxt = cur ^ 1;
         const int nl = 1 << level, pairs = std::max(1, nl / 2);
-        const int *idx_in = level == 0 ? nullptr : rec_idx[cur].p;
-        const int2 *gh_in = level == 0 ? gq : rec_gh[cur].p;
-        // -- histogram of the root / of the smaller child of every pair
-        long long *built = level == 0 ? hist_full.p : hist_built.p;
-        const int bs = f32 ? f32_stride(pairs) : 1;  // fp32 mode: distance of two cells of the built histograms
-        float2 *built_f = bs != 1 ? hist_spread.p : reinterpret_cast<float2 *>(built);
-        if (f32) TGBM_CUDA(cudaMemsetAsync(built_f, 0, sizeof(float2) * (size_t)B * pairs * bs, stream));
-        else TGBM_CUDA(cudaMemsetAsync(built, 0, sizeof(long long) * 2 * (size_t)B * pairs, stream));
-        TimedEvent ev{};
-        if (profile_on) {
-            cudaEventCreate(&ev.a); cudaEventCreate(&ev.b);
-            ev.kind = level == 0 ? 0 : 1;
-            cudaEventRecord(ev.a, stream);
-        }
-        if (f32) {
-            const float2 *ghf = reinterpret_cast<const float2 *>(gh_in);
-            const int f32_ctas = num_sms * (2048 / F32_THREADS);
+        const size_t table = sizeof(int) * ((size_t)pairs + 1);
+        // -- histogram of the root / of the smaller child of every pair, and the choice of the splits
+        auto evaluate = [&](auto *built, int bs, int tree, int n) {
+            using T = std::remove_pointer_t<decltype(built)>;
             if (sparse) {
-                if (level == 0)
-                    k_hist_sparse_f32<false><<<f32_ctas, F32_THREADS, 0, stream>>>(sp_row_ptr.p, sp_bin.p, nullptr, ghf, hist_work.p, hist_tile_base.p,
-                                                                                   ctl.p, built_f, B, bs);
-                else
-                    k_hist_sparse_f32<true><<<f32_ctas, F32_THREADS, 0, stream>>>(sp_row_ptr.p, sp_bin.p, idx_in, ghf, hist_work.p, hist_tile_base.p,
-                                                                                  ctl.p, built_f, B, bs);
-            } else if (level == 0)
-                k_hist_f32<false><<<dim3(f32_ctas, G), F32_THREADS, 0, stream>>>(bins.p, Fpad, F, nullptr, ghf, hist_seq.p, ctl.p, cut_ptr.p, built_f, B, bs,
-                                                                                 f32_cuts, F <= 256, 0);
-            else
-                k_hist_f32<true><<<dim3(f32_ctas, G), F32_THREADS, 0, stream>>>(bins.p, Fpad, F, idx_in, ghf, hist_seq.p, ctl.p, cut_ptr.p, built_f, B, bs,
-                                                                                f32_cuts, F <= 256, f32_staged ? 1 : 0);
-        } else if (sparse) {
-            const int sp_ctas = num_sms;
-            const size_t sp_smem = (size_t)std::min(B, SPARSE_SMEM_BINS) * 16;
-            if (level == 0)
-                k_hist_sparse<false><<<sp_ctas, SPARSE_THREADS, sp_smem, stream>>>(sp_row_ptr.p, sp_bin.p, nullptr, gh_in, hist_work.p,
-                                                                                   hist_tile_base.p, ctl.p, built, B);
-            else
-                k_hist_sparse<true><<<sp_ctas, SPARSE_THREADS, sp_smem, stream>>>(sp_row_ptr.p, sp_bin.p, idx_in, gh_in, hist_work.p,
-                                                                                  hist_tile_base.p, ctl.p, built, B);
-        } else {
-            auto hist = [&](auto kern) {
-                kern<<<dim3(hist_ctas, G), HIST_THREADS, fine ? FINE_SMEM : hist_smem, stream>>>(bins.p, Fpad, F, idx_in, gh_in, hist_cta_off.p,
-                                                                                                hist_seq.p, cut_ptr.p, cut_fid.p, built, B, window_rows);
-            };
-            if (level == 0) { if (fine) hist(k_hist<false, true>); else hist(k_hist<false, false>); }
-            else { if (fine) hist(k_hist<true, true>); else hist(k_hist<true, false>); }
-        }
-        if (profile_on) { cudaEventRecord(ev.b, stream); events.push_back(ev); }
-        int bs_eval = bs;   // distance of the cells the split search reads
-        if (comm && comm->active()) {
-            if (f32) {
-                // the ranks' sums meet in a compact buffer: spread cells are gathered first (a pass over B x pairs cells)
-                float2 *compact = reinterpret_cast<float2 *>(built);
-                if (bs != 1) {
-                    const size_t cells = (size_t)B * pairs;
-                    k_compact_cells<<<std::min(ceil_div(cells, 256), num_sms * 8), 256, 0, stream>>>(built_f, compact, cells, bs);
-                    built_f = compact; bs_eval = 1; ++launches;
-                }
-                comm->allreduce(built_f, 2 * (size_t)B * pairs, Comm::F32, Comm::SUM, stream);
-            } else comm->allreduce(built, 2 * (size_t)B * pairs, Comm::I64, Comm::SUM, stream);
-        }
-        // -- split selection and tree update
-        if (f32) {
-            const float *parent_f = level == 0 ? nullptr : reinterpret_cast<const float *>(hist_full.p) + full_offset(level - 1);
-            float *full_f = reinterpret_cast<float *>(hist_full.p) + full_offset(level);
-            const float *bf = reinterpret_cast<const float *>(built_f);
-            if (sparse) {
-                k_eval_chunk<float><<<dim3(n_chunks, pairs), 64, 0, stream>>>(level, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_fid.p, nodes.p, built_right.p,
-                                                                              bf, parent_f, full_f, qinfo.p, p.min_child_weight, p.lambda, recs.p, bs_eval, ignored_all.p, rstate.p, F, colb);
-                k_best_apply<<<nl, 32, 0, stream>>>(level, n_chunks, cut_ptr.p, cut_val.p, recs.p, nodes.p, p.rt_eps, p.lambda, cut_fid.p, 1, colb);
+                k_eval_chunk<T><<<dim3(n_chunks, pairs, n), 64, 0, stream>>>(level, b, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_fid.p, built, bs, qinfo.p,
+                                                                             p.min_child_weight, p.lambda, ignored_all.p, rstate.p, F, colb, by_hessian, tree);
+                k_best_apply<<<dim3(nl, 1, n), 32, 0, stream>>>(level, b, n_chunks, cut_ptr.p, cut_val.p, p.rt_eps, p.lambda, cut_fid.p, 1, colb, tree);
+                launches += 2;
             } else {
-                k_eval<float><<<dim3(F, pairs), 64, 0, stream>>>(level, F, B, cut_ptr.p, nodes.p, built_right.p, bf, parent_f, full_f, qinfo.p,
-                                                                 p.min_child_weight, p.lambda, recs.p, cut_val.p, p.rt_eps, cut_fid.p, eval_ticket.p, bs_eval,
-                                                                 ignored_all.p, rstate.p, colb);
+                k_eval<T><<<dim3(F, pairs, n), EVAL_THREADS, 0, stream>>>(level, b, F, B, cut_ptr.p, built, bs, qinfo.p, p.min_child_weight, p.lambda,
+                                                                         cut_val.p, p.rt_eps, cut_fid.p, ignored_all.p, rstate.p, colb, by_hessian, tree);
+                ++launches;
+            }
+        };
+        auto timed = [&](int kind, auto &&work) {
+            TimedEvent ev{};
+            if (profile_on) {
+                cudaEventCreate(&ev.a); cudaEventCreate(&ev.b);
+                ev.kind = kind;
+                cudaEventRecord(ev.a, stream);
+            }
+            work();
+            if (profile_on) { cudaEventRecord(ev.b, stream); events.push_back(ev); }
+        };
+        if (float_sums) {
+            // Values are added one by one into cells `bs` float pairs apart, trees one after the other (they share the
+            // spread-out buffer).
+            const int bs = f32_stride(pairs), ctas = num_sms * (2048 / F32_THREADS);
+            for (int t = 0; t < n_trees; ++t) {
+                float2 *compact = reinterpret_cast<float2 *>(hist_built.p + t * b.built_stride), *cells = bs != 1 ? hist_spread.p : compact;
+                if (bs != 1) TGBM_CUDA(cudaMemsetAsync(cells, 0, sizeof(float2) * (size_t)B * pairs * bs, stream));
+                timed(level == 0 ? 0 : 1, [&] {
+                    if (sparse) {
+                        auto kern = level == 0 ? k_hist_sparse_f32<false> : k_hist_sparse_f32<true>;
+                        kern<<<ctas, F32_THREADS, table, stream>>>(level, b, sp_row_ptr.p, sp_bin.p, cells, B, bs, by_hessian, t);
+                    } else {
+                        auto kern = level == 0 ? k_hist_f32<false> : k_hist_f32<true>;
+                        kern<<<dim3(ctas, G), F32_THREADS, table, stream>>>(level, b, bins.p, Fpad, F, cut_ptr.p, cells, B, bs, f32_cuts, F <= 256,
+                                                                            f32_staged ? 1 : 0, by_hessian, t);
+                    }
+                });
+                ++launches;
+                if (comm && comm->active()) {
+                    // the ranks' sums meet in a compact buffer: spread cells are gathered first (a pass over B x pairs cells)
+                    if (bs != 1) {
+                        const size_t n = (size_t)B * pairs;
+                        k_compact_cells<<<std::min(ceil_div(n, 256), num_sms * 8), 256, 0, stream>>>(cells, compact, n, bs);
+                        ++launches;
+                    }
+                    comm->allreduce(compact, 2 * (size_t)B * pairs, Comm::F32, Comm::SUM, stream);
+                    evaluate(reinterpret_cast<float *>(compact), 1, t, 1);
+                } else evaluate(reinterpret_cast<float *>(cells), bs, t, 1);
             }
         } else {
-        const long long *parent_hist = level == 0 ? nullptr : hist_full.p + full_offset(level - 1);
-        if (sparse) {
-            k_eval_chunk<long long><<<dim3(n_chunks, pairs), 64, 0, stream>>>(level, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_fid.p, nodes.p, built_right.p,
-                                                                   built, parent_hist, hist_full.p + full_offset(level), qinfo.p,
-                                                                   p.min_child_weight, p.lambda, recs.p, 1, ignored_all.p, rstate.p, F, colb);
-            k_best_apply<<<nl, 32, 0, stream>>>(level, n_chunks, cut_ptr.p, cut_val.p, recs.p, nodes.p, p.rt_eps, p.lambda, cut_fid.p, 1, colb);
-        } else {
-            k_eval<long long><<<dim3(F, pairs), 64, 0, stream>>>(level, F, B, cut_ptr.p, nodes.p, built_right.p, built, parent_hist,
-                                                      hist_full.p + full_offset(level), qinfo.p, p.min_child_weight, p.lambda, recs.p,
-                                                      cut_val.p, p.rt_eps, cut_fid.p, eval_ticket.p, 1, ignored_all.p, rstate.p, colb);
-        }
+            timed(level == 0 ? 0 : 1, [&] {
+                if (sparse) {
+                    auto kern = level == 0 ? k_hist_sparse<false> : k_hist_sparse<true>;
+                    kern<<<dim3(hist_ctas, 1, n_trees), SPARSE_THREADS, (size_t)std::min(B, SPARSE_SMEM_BINS) * 16 + table, stream>>>(
+                        level, b, sp_row_ptr.p, sp_bin.p, B, by_hessian, 0);
+                } else {
+                    auto kern = level == 0 ? (fine ? k_hist<false, true> : k_hist<false, false>) : (fine ? k_hist<true, true> : k_hist<true, false>);
+                    kern<<<dim3(hist_ctas, G, n_trees), HIST_THREADS, (fine ? HIST_FINE_SMEM : HIST_EXACT_SMEM) + table, stream>>>(
+                        level, b, bins.p, Fpad, F, cut_ptr.p, B, window_rows, by_hessian, 0);
+                }
+            });
+            ++launches;
+            if (comm && comm->active())
+                for (int t = 0; t < n_trees; ++t) comm->allreduce(hist_built.p + t * b.built_stride, 2 * (size_t)B * pairs, Comm::I64, Comm::SUM, stream);
+            evaluate(hist_built.p, 1, 0, n_trees);
         }
         // -- move the rows (not after the last level: the finished tree is applied by walking it, see k_predict_walk)
-        launches += sparse ? 3 : 2;
         if (level == depth - 1) break;
-        TimedEvent pv{};
-        if (profile_on) { cudaEventCreate(&pv.a); cudaEventCreate(&pv.b); pv.kind = 2; cudaEventRecord(pv.a, stream); }
-        if (part_one) {
-            // one pass: count, look-back prefix inside every node and scatter; then the plan of the next level
-            const int n1 = std::max(N, 1);
-            if (sparse)
-                k_part_one<true><<<part_ctas, PART_THREADS, 0, stream>>>(level, nodes.p, seg_begin[cur].p, seg_cnt[cur].p, node_tile0[cur].p, tile_node[cur].p,
-                                                                         part_base.p, ctl.p, idx_in, gh_in, nullptr, Npad, sp_row_ptr.p, sp_bin.p, cut_ptr.p,
-                                                                         part_status.p, part_group.p, seg_begin[nxt].p, seg_cnt[nxt].p, rec_idx[nxt].p, rec_gh[nxt].p, n1, colb);
-            else
-                k_part_one<false><<<part_ctas, PART_THREADS, 0, stream>>>(level, nodes.p, seg_begin[cur].p, seg_cnt[cur].p, node_tile0[cur].p, tile_node[cur].p,
-                                                                          part_base.p, ctl.p, idx_in, gh_in, binsT.p, Npad, nullptr, nullptr, cut_ptr.p,
-                                                                          part_status.p, part_group.p, seg_begin[nxt].p, seg_cnt[nxt].p, rec_idx[nxt].p, rec_gh[nxt].p, n1, colb);
-            k_plan_next<<<1, 1024, 0, stream>>>(level, seg_begin[nxt].p, seg_cnt[nxt].p, seg_cnt[nxt].p, nodes.p, ctl.p, by_hessian, built_right.p,
-                                                hist_work.p, hist_tile_base.p, node_tile0[nxt].p, hist_ctas, hist_cta_off.p, hist_seq.p, depth, tile_node[nxt].p,
-                                                part_base.p, seg_begin[cur].p, seg_cnt[cur].p, part_group.p, (int)part_group.n);
-            if (profile_on) { cudaEventRecord(pv.b, stream); events.push_back(pv); }
-            launches += 2;
-            continue;
-        }
-        if (sparse)
-            k_part_count<true><<<part_ctas, PART_THREADS, 0, stream>>>(level, nodes.p, seg_begin[cur].p, seg_cnt[cur].p, node_tile0[cur].p, ctl.p,
-                                                                       idx_in, nullptr, Npad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, bits.p, tile_left.p, tile_node[cur].p, colb);
-        else
-            k_part_count<false><<<part_ctas, PART_THREADS, 0, stream>>>(level, nodes.p, seg_begin[cur].p, seg_cnt[cur].p, node_tile0[cur].p, ctl.p,
-                                                                        idx_in, binsT.p, Npad, nullptr, nullptr, cut_ptr.p, bits.p, tile_left.p, tile_node[cur].p, colb);
-        k_part_scan<<<1, 1024, 0, stream>>>(level, nodes.p, seg_cnt[cur].p, node_tile0[cur].p, tile_left.p,
-                                            seg_begin[nxt].p, seg_cnt[nxt].p, gcnt.p, ctl.p);
-        // the next level's plan runs beside the scatter: launched first so that it gets its SM slot, while the
-        // scatter leaves 1024 threads' worth of its block slots free
-        TGBM_CUDA(cudaEventRecord(ev_scan, stream));
-        TGBM_CUDA(cudaStreamWaitEvent(stream2, ev_scan, 0));
-        k_plan_next<<<1, 1024, 0, stream2>>>(level, seg_begin[nxt].p, seg_cnt[nxt].p, gcnt.p, nodes.p, ctl.p, by_hessian, built_right.p,
-                                             hist_work.p, hist_tile_base.p, node_tile0[nxt].p, hist_ctas, hist_cta_off.p, hist_seq.p, depth, tile_node[nxt].p,
-                                             part_base.p, nullptr, nullptr, nullptr, 0);
-        TGBM_CUDA(cudaEventRecord(ev_plan, stream2));
-        k_part_scatter<<<std::max(1, part_ctas - 1024 / PART_THREADS), PART_THREADS, 0, stream>>>(level, nodes.p, seg_begin[cur].p, seg_cnt[cur].p,
-                                                                                node_tile0[cur].p, ctl.p, idx_in, gh_in, bits.p, tile_left.p,
-                                                                                seg_begin[nxt].p, rec_idx[nxt].p, rec_gh[nxt].p, tile_node[cur].p);
-        TGBM_CUDA(cudaStreamWaitEvent(stream, ev_plan, 0));
-        if (profile_on) { cudaEventRecord(pv.b, stream); events.push_back(pv); }
-        launches += 4;
+        timed(2, [&] {
+            const dim3 grid(part_ctas, 1, n_trees);
+            const size_t nodes_table = sizeof(int) * ((size_t)nl + 1);
+            if (sparse) k_part_count<true><<<grid, PART_THREADS, nodes_table, stream>>>(level, b, nullptr, Npad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, colb, 0);
+            else k_part_count<false><<<grid, PART_THREADS, nodes_table, stream>>>(level, b, binsT.p, Npad, nullptr, nullptr, cut_ptr.p, colb, 0);
+            k_part_scatter<<<grid, PART_THREADS, 2 * nodes_table, stream>>>(level, b, 0);
+        });
+        launches += 2;
     }
-    k_prune<<<1, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream>>>(nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0);
+    k_prune<<<n_trees, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream>>>(nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0,
+                                                                                              model.p, K, k0, rstate.p);
     if (N) {
         const size_t per_node = sizeof(WalkNode) + (sparse ? sizeof(WalkSpan) : 0);
         const int in_smem = per_node * (size_t)n_nodes <= 160 * 1024;
         const size_t walk_smem = in_smem ? per_node * (size_t)n_nodes : 0;
-        float *yp = ypred.p + (size_t)k * N;
-        int *nid_out = p.keep_nid ? nid_keep.p + (size_t)tree_index * N : nullptr;
+        float *yp = ypred.p + (size_t)k0 * N;
+        int *nid_out = p.keep_nid ? nid_keep.p + ((size_t)round * K + k0) * N : nullptr;
         // One tree per round and a pointwise objective: the walk also adds up the round's metric and finds the maxima
         // of the next round's gradients (grid and order of additions are those of k_metric_partial).
         const bool fuse = K == 1 && (objective == REG_LINEAR || objective == REG_LOGISTIC || objective == BINARY_LOGISTIC);
-        const int walk_ctas = fuse ? metric_blocks() : std::min(ceil_div(N, 256), num_sms * 8);
+        const dim3 walk_ctas(fuse ? metric_blocks() : std::min(ceil_div(N, 256), num_sms * 8), n_trees);
         const int fo = fuse ? objective : -1;
         if (fuse) maxbits.zero(stream);
-        if (sparse)
-            k_predict_walk<2><<<walk_ctas, 256, walk_smem, stream>>>(nodes.p, n_nodes, in_smem, nullptr, Fpad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, N,
-                                                                     p.learning_rate, yp, nid_out, y.p, fo, metric_partial.p, maxbits.p, colb);
-        else if (Fpad == 32)
-            k_predict_walk<0><<<walk_ctas, 256, walk_smem, stream>>>(nodes.p, n_nodes, in_smem, bins.p, Fpad, nullptr, nullptr, cut_ptr.p, N,
-                                                                     p.learning_rate, yp, nid_out, y.p, fo, metric_partial.p, maxbits.p, colb);
-        else
-            k_predict_walk<1><<<walk_ctas, 256, walk_smem, stream>>>(nodes.p, n_nodes, in_smem, bins.p, Fpad, nullptr, nullptr, cut_ptr.p, N,
-                                                                     p.learning_rate, yp, nid_out, y.p, fo, metric_partial.p, maxbits.p, colb);
+        auto kern = sparse ? k_predict_walk<2> : Fpad == 32 ? k_predict_walk<0> : k_predict_walk<1>;
+        kern<<<walk_ctas, 256, walk_smem, stream>>>(nodes.p, n_nodes, in_smem, sparse ? nullptr : bins.p, Fpad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, N,
+                                                    p.learning_rate, yp, nid_out, y.p, fo, metric_partial.p, maxbits.p, colb);
         grad_max_ready = metric_partial_ready = fuse;
     }
     launches += 2;
-    k_store_tree<<<std::min(ceil_div(n_nodes, 256), 64), 256, 0, stream>>>(nodes.p, model.p, n_nodes, K, k, rstate.p);
-    ++launches;
 }
 
 void BoosterImpl::round_metric(int round) {
     const int log_len = (int)qinfo_log.n;
     if (need_group_file(objective)) {
         rank.metric(objective, ypred.p, nullptr, comm, N_global, stream);
-        k_round_end<<<1, 32, 0, stream>>>(objective, rank.sum.p, rank.n_group_total, metric.p, qinfo.p, qinfo_log.p, log_len, rstate.p);
+        k_round_end<<<1, 32, 0, stream>>>(objective, rank.sum.p, nullptr, 0, rank.n_group_total, metric.p, qinfo.p, qinfo_log.p, log_len, rstate.p);
         ++launches;
         return;
     }
@@ -1159,10 +1095,15 @@ void BoosterImpl::round_metric(int round) {
         ++launches;
     }
     metric_partial_ready = false;
-    k_metric_sum<<<1, 32, 0, stream>>>(metric_partial.p, blocks, metric_sum.p);
-    if (comm && comm->active()) comm->allreduce(metric_sum.p, 1, Comm::F64, Comm::SUM, stream);
-    k_round_end<<<1, 32, 0, stream>>>(objective, metric_sum.p, N_global, metric.p, qinfo.p, qinfo_log.p, log_len, rstate.p);
-    launches += 2;
+    const bool multi = comm && comm->active();
+    if (multi) {
+        k_metric_sum<<<1, 32, 0, stream>>>(metric_partial.p, blocks, metric_sum.p);
+        comm->allreduce(metric_sum.p, 1, Comm::F64, Comm::SUM, stream);
+        ++launches;
+    }
+    k_round_end<<<1, 32, 0, stream>>>(objective, metric_sum.p, multi ? nullptr : metric_partial.p, blocks, N_global, metric.p, qinfo.p, qinfo_log.p,
+                                      log_len, rstate.p);
+    ++launches;
 }
 
 // One boosting round.  From the second round on the launch sequence no longer changes (which kernels run is decided
@@ -1173,9 +1114,9 @@ void BoosterImpl::round_metric(int round) {
 void BoosterImpl::run_round(int round) {
     auto direct = [&]() {
         gradient(round);
-        for (int k = 0; k < K; ++k) {
+        for (int k = 0; k < K; k += batch) {
             if (exact) build_tree_exact(round, k);
-            else build_tree(round, k);
+            else build_trees(round, k, std::min(batch, K - k));
         }
         round_metric(round);
     };
@@ -1225,8 +1166,7 @@ void Booster::sync() {
     if (impl_->comm && impl_->comm->active()) impl_->comm->wait(impl_->stream);  // bounded: a rank may have left
     else TGBM_CUDA(cudaStreamSynchronize(impl_->stream));
     TGBM_CUDA(cudaGetLastError());
-    // bounded waits inside the kernels (look-back of the single-pass partition, bulk-copy barriers of the fp32 histogram
-    // kernel) report here instead of spinning: the results of the run are not to be trusted
+    // bounded waits inside the kernels (bulk-copy barriers of the float histogram kernel) report here instead of spinning: the results of the run are not to be trusted
     if (impl_->ctl.p) {
         int err = 0;
         TGBM_CUDA(cudaMemcpy(&err, reinterpret_cast<const char *>(impl_->ctl.p) + offsetof(TreeCtl, error), sizeof(int), cudaMemcpyDeviceToHost));
@@ -1260,7 +1200,7 @@ HistProfile Booster::profile() {
     for (auto &e : m.events) {
         float ms = 0;
         cudaEventElapsedTime(&ms, e.a, e.b);
-        if (e.kind == 2) { r.partition_ms += ms; r.partition_launches += 4; }
+        if (e.kind == 2) { r.partition_ms += ms; r.partition_launches += 2; }
         else {
             r.hist_ms += ms; r.hist_launches += 1;
             if (e.kind == 0) { r.hist_root_ms += ms; r.hist_root_launches += 1; }
@@ -1335,13 +1275,13 @@ std::vector<int> Booster::get_nid() {
 std::vector<long long> Booster::get_root_hist() {
     sync();
     TGBM_CHECK(!impl_->f32, "fp32 mode keeps float histograms: use get_root_hist_f32");
-    return to_host(impl_->hist_full.p, (size_t)impl_->B * 2);
+    return to_host(impl_->hist_full.p + impl_->last_tree_full, (size_t)impl_->B * 2);
 }
 std::vector<float> Booster::get_root_hist_f32() {
     sync();
     TGBM_CHECK(impl_->f32, "exact mode keeps integer histograms: use get_root_hist");
-    if (impl_->last_float) return to_host(reinterpret_cast<const float *>(impl_->hist_full.p), (size_t)impl_->B * 2);
-    const auto h = to_host(impl_->hist_full.p, (size_t)impl_->B * 2);
+    if (impl_->last_float) return to_host(reinterpret_cast<const float *>(impl_->hist_full.p + impl_->last_tree_full), (size_t)impl_->B * 2);
+    const auto h = to_host(impl_->hist_full.p + impl_->last_tree_full, (size_t)impl_->B * 2);
     const QuantInfo q = to_host(impl_->qinfo.p, 1)[0];
     std::vector<float> out(h.size());
     for (size_t i = 0; i < h.size(); ++i) out[i] = (float)((double)h[i] * ((i & 1) ? q.inv_sh : q.inv_sg));

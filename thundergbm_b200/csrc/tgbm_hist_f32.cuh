@@ -21,7 +21,7 @@
 //
 // The fixed-point kernels (k_hist, k_hist_sparse) serve the deterministic mode and the later rounds.
 #pragma once
-#include "tgbm_kernels.cuh"
+#include "tgbm_level.cuh"
 
 namespace tgbm {
 
@@ -69,15 +69,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
     return false;
 }
 
-// Dense layout.  grid = (CTAs, feature groups of 32); a CTA takes half a 1024-record tile of the level's tile
-// sequence at a time, a thread one record: its 32 bin bytes, its gradient pair, one reduction per present feature.
+// Dense layout.  grid = (CTAs, feature groups of 32); a CTA takes a unit of F32_THREADS records at a time, a thread one
+// record: its 32 bin bytes, its gradient pair, one reduction per present feature.
 template <bool GATHER>
 static __global__ void __launch_bounds__(F32_THREADS)
-k_hist_f32(const unsigned char *__restrict__ bins, int Fpad, int F, const int *__restrict__ rec_idx,
-           const float2 *__restrict__ rec_gh, const int4 *__restrict__ seq, TreeCtl *__restrict__ ctl,
-           const int *__restrict__ cut_ptr, float2 *__restrict__ slab, int B, int cell_stride,
-           const __grid_constant__ CutOffsets cuts, int cuts_in_param, int staged) {
-    __shared__ int s_cut[32];
+k_hist_f32(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpad, int F, const int *__restrict__ cut_ptr,
+           float2 *__restrict__ slab, int B, int cell_stride, const __grid_constant__ CutOffsets cuts, int cuts_in_param, int staged,
+           int by_hessian, int tree) {
+    extern __shared__ int s_base[];
+    __shared__ int s_cut[32], scratch[33];
     __shared__ __align__(16) int s_idx[2][STAGE_IDX];
     __shared__ __align__(16) float2 s_gh[2][STAGE_GH];
     __shared__ __align__(8) uint64_t s_bar[2];
@@ -86,17 +86,7 @@ k_hist_f32(const unsigned char *__restrict__ bins, int Fpad, int F, const int *_
     if (!cuts_in_param) {  // more than 256 features: the offsets of the CTA's group through shared memory
         if (threadIdx.x < 32) s_cut[threadIdx.x] = threadIdx.x < nf ? cut_ptr[f0 + threadIdx.x] : 0;
     }
-    constexpr int PER_TILE = HIST_THREADS / F32_THREADS;
-    const int units = ctl->n_hist_tiles * PER_TILE;
     const bool stage = GATHER && staged;
-    auto unit_first = [&](int u) { const int4 e = seq[u / PER_TILE]; return e.x + (u % PER_TILE) * F32_THREADS; };
-    auto issue = [&](int u, int buf) {  // thread 0: both pieces of unit u into buffer buf
-        const int p0 = unit_first(u);
-        const int a_idx = p0 & ~3, a_gh = p0 & ~1;
-        mbar_expect_tx(&s_bar[buf], (uint32_t)(STAGE_IDX * sizeof(int) + STAGE_GH * sizeof(float2)));
-        bulk_g2s(s_idx[buf], rec_idx + a_idx, (uint32_t)(STAGE_IDX * sizeof(int)), &s_bar[buf]);
-        bulk_g2s(s_gh[buf], rec_gh + a_gh, (uint32_t)(STAGE_GH * sizeof(float2)), &s_bar[buf]);
-    };
     if (stage) {
         if (threadIdx.x == 0) {
             mbar_init(&s_bar[0], 1); mbar_init(&s_bar[1], 1);
@@ -104,8 +94,29 @@ k_hist_f32(const unsigned char *__restrict__ bins, int Fpad, int F, const int *_
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
-    __syncthreads();
-    // A CTA takes a contiguous run of the unit sequence, so that at any moment the CTAs of the grid work on different
+    const int units = hist_items<F32_THREADS, F32_THREADS>(level, b, tree, by_hessian, s_base, scratch, blockIdx.x == 0 && blockIdx.y == 0);
+    const int pairs = level == 0 ? 1 : 1 << (level - 1);
+    const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
+    const TreeNode *nodes = b.nodes + tree * b.nodes_stride;
+    const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
+    const float2 *rec_gh = reinterpret_cast<const float2 *>(GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride);
+    auto unit = [&](int u) -> int3 {   // first record, records, histogram slot
+        int lo = 0, hi = pairs - 1;    // last item that starts at or before u
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if (s_base[mid] <= u) lo = mid; else hi = mid - 1;
+        }
+        const int node = level == 0 ? 0 : 2 * lo + built_side(level, lo, seg_cnt, nodes, by_hessian), at = (u - s_base[lo]) * F32_THREADS;
+        return make_int3(seg_begin[node] + at, min(F32_THREADS, seg_cnt[node] - at), lo);
+    };
+    auto issue = [&](int u, int buf) {  // thread 0: both pieces of unit u into buffer buf
+        const int p0 = unit(u).x;
+        const int a_idx = p0 & ~3, a_gh = p0 & ~1;
+        mbar_expect_tx(&s_bar[buf], (uint32_t)(STAGE_IDX * sizeof(int) + STAGE_GH * sizeof(float2)));
+        bulk_g2s(s_idx[buf], rec_idx + a_idx, (uint32_t)(STAGE_IDX * sizeof(int)), &s_bar[buf]);
+        bulk_g2s(s_gh[buf], rec_gh + a_gh, (uint32_t)(STAGE_GH * sizeof(float2)), &s_bar[buf]);
+    };
+    // A CTA takes a contiguous run of the units, so that at any moment the CTAs of the grid work on different
     // nodes: with all of them on the same node (units dealt out round-robin) every reduction in flight aims at that one
     // node's 57 KB of cells, the regime the L2 handles worst (86 G reductions/s against 181 G/s over 64 nodes).
     const int run = (units + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -113,16 +124,15 @@ k_hist_f32(const unsigned char *__restrict__ bins, int Fpad, int F, const int *_
     if (stage && threadIdx.x == 0 && u_begin < u_end) issue(u_begin, 0);
     int n_done = 0;  // units this CTA has consumed: buffer = n_done & 1, parity = (n_done >> 1) & 1
     for (int u = u_begin; u < u_end; ++u, ++n_done) {
-        const int4 e = seq[u / PER_TILE];  // first record, records, histogram slot
-        const int q = (u % PER_TILE) * F32_THREADS + threadIdx.x;
+        const int3 e = unit(u);
+        const int q = threadIdx.x;
         int r = -1;
         float2 v = make_float2(0.f, 0.f);
         if (stage) {
             const int buf = n_done & 1;
             if (threadIdx.x == 0 && u + 1 < u_end) issue(u + 1, buf ^ 1);  // one unit ahead
-            if (!mbar_wait(&s_bar[buf], (n_done >> 1) & 1)) { s_fail = 1; atomicCAS(&ctl->error, 0, 0x40000000 | u); }
-            const int p0 = e.x + (u % PER_TILE) * F32_THREADS;
-            if (q < e.y) { r = s_idx[buf][(p0 & 3) + threadIdx.x]; v = s_gh[buf][(p0 & 1) + threadIdx.x]; }
+            if (!mbar_wait(&s_bar[buf], (n_done >> 1) & 1)) { s_fail = 1; atomicCAS(&b.ctl->error, 0, 0x40000000 | u); }
+            if (q < e.y) { r = s_idx[buf][(e.x & 3) + threadIdx.x]; v = s_gh[buf][(e.x & 1) + threadIdx.x]; }
             __syncthreads();  // every thread holds its record: the buffer may be refilled two units from now
             if (s_fail) {  // leave only when the copy that is still on its way has landed (bounded as well)
                 if (threadIdx.x == 0 && u + 1 < u_end) mbar_wait(&s_bar[buf ^ 1], ((n_done + 1) >> 1) & 1);
@@ -136,8 +146,8 @@ k_hist_f32(const unsigned char *__restrict__ bins, int Fpad, int F, const int *_
         }
         if (r < 0) continue;
         const uint4 *row = reinterpret_cast<const uint4 *>(bins + (size_t)r * Fpad + f0);
-        const uint4 a = row[0], b = row[1];
-        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const uint4 a = row[0], bb = row[1];
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, bb.x, bb.y, bb.z, bb.w};
         float2 *dst = slab + (size_t)e.z * B * cell_stride;
 #pragma unroll
         for (int f = 0; f < 32; ++f) {
@@ -153,23 +163,29 @@ k_hist_f32(const unsigned char *__restrict__ bins, int Fpad, int F, const int *_
 // CSR layout: a warp per record, lanes over the row's stored values (global bin ids).
 template <bool GATHER>
 static __global__ void __launch_bounds__(F32_THREADS)
-k_hist_sparse_f32(const int *__restrict__ row_ptr, const int *__restrict__ bin, const int *__restrict__ rec_idx,
-                  const float2 *__restrict__ rec_gh, const HistWork *__restrict__ work, const int *__restrict__ tile_base,
-                  const TreeCtl *__restrict__ ctl, float2 *__restrict__ slab, int B, int cell_stride) {
-    const int total = ctl->n_hist_tiles, nwork = ctl->n_hist_work;
+k_hist_sparse_f32(int level, const Batch b, const int *__restrict__ row_ptr, const int *__restrict__ bin, float2 *__restrict__ slab, int B,
+                  int cell_stride, int by_hessian, int tree) {
+    extern __shared__ int s_base[];
+    __shared__ int scratch[33];
+    const int total = hist_items<F32_THREADS, HIST_THREADS>(level, b, tree, by_hessian, s_base, scratch, blockIdx.x == 0);
+    const int pairs = level == 0 ? 1 : 1 << (level - 1);
+    const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
+    const TreeNode *nodes = b.nodes + tree * b.nodes_stride;
+    const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
+    const float2 *rec_gh = reinterpret_cast<const float2 *>(GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int W = F32_THREADS / 32;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        int lo = 0, hi = nwork - 1;  // the work item of tile t: last w with tile_base[w] <= t
+        int lo = 0, hi = pairs - 1;  // the item of tile t: the last one that starts at or before it
         while (lo < hi) {
             const int mid = (lo + hi + 1) / 2;
-            if (tile_base[mid] <= t) lo = mid; else hi = mid - 1;
+            if (s_base[mid] <= t) lo = mid; else hi = mid - 1;
         }
-        const HistWork it = work[lo];
-        float2 *dst = slab + (size_t)it.slab * B * cell_stride;
-        const int first = (t - tile_base[lo]) * HIST_THREADS, last = min(it.count, first + HIST_THREADS);
+        const int node = level == 0 ? 0 : 2 * lo + built_side(level, lo, seg_cnt, nodes, by_hessian), begin = seg_begin[node];
+        float2 *dst = slab + (size_t)lo * B * cell_stride;
+        const int first = (t - s_base[lo]) * HIST_THREADS, last = min(seg_cnt[node], first + HIST_THREADS);
         for (int q = first + warp; q < last; q += W) {
-            const int p = it.begin + q;
+            const int p = begin + q;
             const int r = GATHER ? rec_idx[p] : p;
             const float2 v = rec_gh[p];
             const int j1 = row_ptr[r + 1];

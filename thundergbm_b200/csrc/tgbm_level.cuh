@@ -1,0 +1,1130 @@
+// Kernels of one tree level: histogram build, split search, row partition.
+//
+// A level is four launches -- k_hist (or its CSR / float forms), k_eval, k_part_count, k_part_scatter -- that hand over to
+// each other through the segment tables alone (seg_begin, seg_cnt: where the records of every node of the level sit).
+// What used to be planned by single-block kernels between them (which sibling to build, tile lists, prefix sums: 14 + 5 us
+// a level, most of the time of a small training) every block now works out for itself from those tables, in shared memory,
+// while its first loads are on their way.
+//
+// Trees of one round do not depend on each other (softmax builds one per class from the same scores), so every kernel
+// takes a batch of them: blockIdx.z is the tree, the buffers of consecutive trees lie `Batch::*_stride` apart.
+#pragma once
+#include "tgbm_kernels.cuh"
+
+namespace tgbm {
+
+struct Batch {
+    TreeNode *nodes;
+    int *seg_begin[2], *seg_cnt[2];   // by level parity
+    int *rec_idx[2];                  // row ids of the records, left children in the first half, right ones in the second
+    int2 *rec_gh[2];                  // their gradient pairs
+    const int2 *gh;                   // gradient pairs by row: the records of the root
+    long long *hist_full, *hist_built;
+    SplitRec *recs;
+    unsigned *bits;                   // partition: one bit per record of a tile, left = 1
+    int *tile_left, *tail_left, *ticket;
+    TreeCtl *ctl;
+    size_t nodes_stride, seg_stride, rec_stride, gh_stride, full_stride, built_stride, recs_stride, bits_stride, tile_stride, tail_stride,
+        ticket_stride;
+    int half;                         // offset of the right children in rec_idx / rec_gh
+};
+
+// ------------------------------------------------------------------ work lists
+// Exclusive prefix sums over n values inside one block of NT threads: out(i, prefix before i); returns the total.
+// `scratch` holds 33 ints of shared memory.  Every thread of the block must call it.
+template <int NT, typename In, typename Out>
+__device__ __forceinline__ int block_prefix(int n, In in, Out out, int *scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = 0;
+    for (int base = 0; base < n; base += NT) {
+        const int i = base + threadIdx.x;
+        const int x = i < n ? in(i) : 0;
+        int v = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+        __syncthreads();
+        if (lane == 31) scratch[warp] = v;
+        __syncthreads();
+        if (n - base <= 32) {   // one warp holds them all
+            const int total = scratch[0];
+            if (i < n) out(i, v - x + carry);
+            carry += total;
+            break;
+        }
+        if (warp == 0) {
+            int t = lane < NT / 32 ? scratch[lane] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, t, o); if (lane >= o) t += u; }
+            scratch[lane] = t;
+        }
+        __syncthreads();
+        if (i < n) out(i, v + (warp ? scratch[warp - 1] : 0) + carry - x);
+        carry += scratch[NT / 32 - 1];
+    }
+    __syncthreads();
+    return carry;
+}
+
+// Which child of pair j of a level >= 1 is built (the other one is the parent minus it): the one with fewer rows, ties ->
+// left (hist_tree_builder_single.cu:466); -1: neither holds rows.  With several ranks the row counts are rank-local, so
+// every rank takes the child with the smaller hessian sum from the replicated node table -- the same choice everywhere
+// without a collective; the histogram sums are integers, so built and subtracted ones are identical either way.
+__device__ __forceinline__ int built_side(int level, int j, const int *seg_cnt, const TreeNode *nodes, int by_hessian) {
+    if (by_hessian) {
+        const int off = (1 << level) - 1;
+        const TreeNode &l = nodes[off + 2 * j], &r = nodes[off + 2 * j + 1];
+        if (!l.is_valid || !r.is_valid) return -1;
+        return l.sum_h > r.sum_h ? 1 : 0;
+    }
+    const int2 c = *reinterpret_cast<const int2 *>(seg_cnt + 2 * j);
+    return max(c.x, c.y) == 0 ? -1 : (c.x > c.y ? 1 : 0);
+}
+
+// The histograms a level builds and their tiles of `TILE` records: s_base[j] = tiles before pair j, s_base[pairs] = total.
+// `node(j)`: the built node of the pair or -1.  The block that reports adds to the byte counters of the roofline.
+template <int NT, int TILE>
+__device__ __forceinline__ int hist_items(int level, const Batch &b, size_t tree, int by_hessian, int *s_base, int *scratch, bool report) {
+    const int pairs = level == 0 ? 1 : 1 << (level - 1);
+    const int *cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
+    const TreeNode *nodes = b.nodes + tree * b.nodes_stride;
+    __shared__ unsigned long long s_rows;
+    __shared__ int s_hists;
+    if (threadIdx.x == 0) { s_rows = 0; s_hists = 0; }
+    __syncthreads();
+    const int total = block_prefix<NT>(pairs,
+        [&](int j) {
+            const int r = level == 0 ? 0 : built_side(level, j, cnt, nodes, by_hessian);
+            const int n = r < 0 ? 0 : cnt[level == 0 ? 0 : 2 * j + r];
+            if (report && r >= 0) { atomicAdd(&s_rows, (unsigned long long)n); atomicAdd(&s_hists, 1); }
+            return (n + TILE - 1) / TILE;
+        },
+        [&](int j, int before) { s_base[j] = before; }, scratch);
+    if (threadIdx.x == 0) {
+        s_base[pairs] = total;
+        if (report) {
+            atomicAdd(level == 0 ? &b.ctl->stat_rows_root : &b.ctl->stat_rows_gather, s_rows);
+            atomicAdd(&b.ctl->stat_hists, (unsigned long long)s_hists);
+        }
+    }
+    __syncthreads();
+    return total;
+}
+
+// Order in which the dense histogram kernel visits the level's tiles.
+// The tiles are dealt out to `n_ctas * HIST_SHARES` shares in proportion to the items' sizes (cumulative rounding, so
+// the shares of different items are disjoint; an item too small for a share of its own rides on one).  Inside an item
+// tile t belongs to share v0 + t mod k.  CTA c owns HIST_SHARES consecutive shares and visits, item by item, the tiles
+// of its shares in ascending order: every CTA walks each of its (one or two, rarely more) lists once, front to back,
+// and since all CTAs carry about the same number of tiles, all lists are walked at the same relative pace.  Row ids
+// ascend inside every list, so at any time the whole GPU gathers rows from one moving window of the bin matrix:
+// DRAM pages and 64-byte sectors get shared between nodes.  A pure gather of 5.2 M of 10.5 M rows in 8 to 64 lists
+// takes 72 us this way and 100 to 110 us list after list.
+struct HistCursor {   // where a CTA stands in its list: item, remaining tiles of it, next tile = first record and records left from it
+    int w, w_end, left = 0, k = 1, width = 1, rr = 0, first = 0, rows = 0;
+};
+__device__ __forceinline__ void hist_share(const int *s_base, int w, int total, int n_shares, int &v0, int &k) {
+    const unsigned half = (unsigned)total / 2, a = (unsigned)s_base[w] * (unsigned)n_shares + half, z = (unsigned)s_base[w + 1] * (unsigned)n_shares + half;
+    v0 = (int)(a / (unsigned)total);
+    k = (int)(z / (unsigned)total) - v0;
+    if (k <= 0) { k = 1; v0 = min(v0, n_shares - 1); }
+}
+
+// Permute the 16 bin bytes of a half row so that byte j of the register array is the bin of slot (j XOR key),
+// key = 0..15: at step j the 16 lane pairs of a warp then address 16 different slots of either half.  Key bits 0-1
+// permute the bytes inside every word (one PRMT each), bits 2-3 exchange whole words.
+__device__ __forceinline__ void xor_permute_half(uint32_t (&w)[4], int key) {
+    const uint32_t sel = (key & 2) ? ((key & 1) ? 0x0123u : 0x1032u) : ((key & 1) ? 0x2301u : 0x3210u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __byte_perm(w[i], 0u, sel);
+    const int hi = key >> 2;
+#pragma unroll
+    for (int s = 1; s <= 2; s <<= 1) {
+        uint32_t t[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) t[i] = (hi & s) ? w[i ^ s] : w[i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = t[i];
+    }
+}
+
+// ------------------------------------------------------------------ histogram build, dense layout
+// Root: hist_tree_builder_single.cu:203-216, deeper levels: :485-505.
+// Persistent CTAs, one per SM; grid = (ctas, feature groups of 32, trees).  A lane holds one 16-feature half of two rows;
+// the shared-memory accumulators are laid out [bin][32 features] so that the bank is the feature index, and at step j the
+// 32 lanes of a warp handle 32 different features, so every shared atomic of a warp hits 32 different banks.
+//
+// !FINE (exact mode, values of at most quant_bits bits): accumulators are int32.  Before they could overflow
+// (`window_rows` rows of at most 2^quant_bits each) they are drained into int64 totals, also in shared memory.
+// FINE (fp32 mode after its first round, values of FINE_BITS bits and a sign): a value is added in two halves, the low 16
+// bits to an unsigned accumulator and the rest to a signed one.  Two plain 32-bit atomics per component are the cheapest
+// exact 31-bit addition there is: the bare shared-memory atomics of 294 M (row, feature) pairs take 0.134 ms so, 0.188 ms
+// as one returning atomic with a carry test, 0.290 ms as one 64-bit atomic, 0.320 ms as float atomics (compare-and-swap
+// loops); 0.073 ms with one 32-bit atomic per component.  FINE_WINDOW rows fill the low halves.
+//
+// When a CTA is done with a node its sums are laid out [feature][bin][g,h] as int64 in shared memory and added to the
+// node's histogram by one bulk reduction per feature (cp.reduce.async.bulk: the L2 takes whole lines; 148 CTAs flushing
+// 28 x 255 cells: 4.3 us into one node, 2.8 us into 64; 21.7 and 10.7 us as one RED.64 per cell and component, whose
+// lanes hit 32 different sectors).
+constexpr int HIST_CELLS = 256 * 32;                                   // per component
+constexpr int HIST_STAGE = 256 * 16 + 16;                              // bytes of a feature's int64 pairs; the pad keeps 8 lanes' 16-byte stores in different banks
+constexpr int HIST_FINE_SMEM = 32 * HIST_STAGE;                        // 4 int32 accumulators per cell (128 KB), staged in place
+constexpr int HIST_EXACT_SMEM = 2 * HIST_CELLS * 4 + 32 * HIST_STAGE;  // 2 int32 accumulators, then int64 totals = staging area
+
+__device__ __forceinline__ void bulk_add_u64(void *dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;"
+                 ::"l"(dst), "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(bytes) : "memory");
+}
+
+template <bool GATHER, bool FINE>
+static __global__ void __launch_bounds__(HIST_THREADS, 1)
+k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpad, int F, const int *__restrict__ cut_ptr, int B,
+       int window_rows, int by_hessian, int tree0) {
+    extern __shared__ __align__(128) unsigned char hist_sm[];
+    int *acc = reinterpret_cast<int *>(hist_sm);          // g, h (FINE: low halves)
+    int *high = acc + 2 * HIST_CELLS;                     // FINE: high halves of g, h
+    unsigned char *stage = hist_sm + (FINE ? 0 : 2 * HIST_CELLS * 4);
+    long long *tot = reinterpret_cast<long long *>(stage);  // !FINE: totals of g, then h, [bin][feature]
+    int *s_base = reinterpret_cast<int *>(hist_sm + (FINE ? HIST_FINE_SMEM : HIST_EXACT_SMEM));
+    __shared__ int scratch[33], s_ib, s_ie;
+    const int group = blockIdx.y, f0 = group * 32, nf = min(32, F - f0), lane = threadIdx.x & 31;
+    const size_t tree = tree0 + blockIdx.z;
+    for (int i = threadIdx.x; i < (FINE ? HIST_FINE_SMEM : HIST_EXACT_SMEM) / 16; i += HIST_THREADS)
+        reinterpret_cast<int4 *>(hist_sm)[i] = make_int4(0, 0, 0, 0);
+    if (threadIdx.x == 0) { s_ib = 0x7fffffff; s_ie = -1; }
+    const int total = hist_items<HIST_THREADS, HIST_THREADS>(level, b, tree, by_hessian, s_base, scratch, blockIdx.x == 0 && group == 0);
+    if (total == 0) return;
+    const int pairs = level == 0 ? 1 : 1 << (level - 1);
+    const int n_shares = (int)gridDim.x * HIST_SHARES, va = (int)blockIdx.x * HIST_SHARES, vb = va + HIST_SHARES;
+    const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
+    const TreeNode *nodes = b.nodes + tree * b.nodes_stride;
+    for (int w = threadIdx.x; w < pairs; w += HIST_THREADS) {   // items with a share among this CTA's
+        if (s_base[w + 1] == s_base[w]) continue;
+        int v0, k;
+        hist_share(s_base, w, total, n_shares, v0, k);
+        if (v0 < vb && v0 + k > va) { atomicMin(&s_ib, w); atomicMax(&s_ie, w); }
+    }
+    __syncthreads();
+    HistCursor c;
+    c.w = s_ib - 1; c.w_end = s_ie;
+    if (c.w_end < 0) return;
+    auto next = [&]() -> int3 {   // (first record, records, pair) of the CTA's next tile; records = 0 at the end
+        while (c.left == 0) {
+            if (++c.w > c.w_end) { c.w = c.w_end; return make_int3(0, 0, 0); }
+            const int T = s_base[c.w + 1] - s_base[c.w];
+            if (!T) continue;
+            int v0, k;
+            hist_share(s_base, c.w, total, n_shares, v0, k);
+            const int ra = max(va, v0) - v0, width = min(vb, v0 + k) - v0 - ra;
+            if (width <= 0) continue;
+            c.left = (T / k) * width + min(max(T % k - ra, 0), width);
+            c.k = k; c.width = width; c.rr = 0;
+            const int node = level == 0 ? 0 : 2 * c.w + built_side(level, c.w, seg_cnt, nodes, by_hessian);
+            c.first = seg_begin[node] + ra * HIST_THREADS; c.rows = seg_cnt[node] - ra * HIST_THREADS;
+        }
+        --c.left;
+        const int3 e = make_int3(c.first, min(HIST_THREADS, c.rows), c.w);
+        int step = HIST_THREADS;   // the share's tiles: `width` neighbours of every k
+        if (++c.rr == c.width) { c.rr = 0; step += (c.k - c.width) * HIST_THREADS; }
+        c.first += step; c.rows -= step;
+        return e;
+    };
+
+    const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
+    const int2 *rec_gh = GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride;
+    long long *slab = b.hist_built + tree * b.built_stride;
+
+    auto drain = [&]() {  // int32 window -> int64 totals, same [bin][feature] layout
+        __syncthreads();
+#pragma unroll 4
+        for (int i = threadIdx.x; i < 2 * HIST_CELLS; i += HIST_THREADS) {
+            const int v = acc[i];
+            if (v) { tot[i] += v; acc[i] = 0; }
+        }
+        __syncthreads();
+    };
+    const int flush_b0 = lane < nf ? cut_ptr[f0 + lane] : 0;   // first bin of this lane's feature
+    const int flush_nb = lane < nf ? cut_ptr[f0 + lane + 1] - flush_b0 : 0;
+    auto flush = [&](int pair, bool again) {
+        long long vg[8], vh[8];
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int s = ((threadIdx.x >> 5) + 32 * q) * 32 + lane;
+            if (FINE) {
+                vg[q] = ((long long)high[s] << 16) + (unsigned)acc[s]; vh[q] = ((long long)high[HIST_CELLS + s] << 16) + (unsigned)acc[HIST_CELLS + s];
+            } else {
+                vg[q] = tot[s] + acc[s]; vh[q] = tot[HIST_CELLS + s] + acc[HIST_CELLS + s];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            *reinterpret_cast<longlong2 *>(stage + lane * HIST_STAGE + ((threadIdx.x >> 5) + 32 * q) * 16) = make_longlong2(vg[q], vh[q]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            if (flush_nb > 0) bulk_add_u64(slab + ((size_t)pair * B + flush_b0) * 2, stage + lane * HIST_STAGE, (uint32_t)flush_nb * 16);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        }
+        if (!again) return;
+        __syncthreads();
+        for (int i = threadIdx.x; i < (FINE ? HIST_FINE_SMEM : HIST_EXACT_SMEM) / 16; i += HIST_THREADS)
+            reinterpret_cast<int4 *>(hist_sm)[i] = make_int4(0, 0, 0, 0);
+        __syncthreads();
+    };
+
+    // Two lanes share a row: lane l loads the 16-byte half (l & 1) of the rows at tile positions
+    // warp*32 + (l >> 1) ("A") and 16 further on ("B").  One load instruction of a warp therefore touches 16 rows
+    // (16 sectors) instead of 32 half-used ones, which halves the L1 wavefronts the gathered rows cost.
+    const int qa = (threadIdx.x & ~31) | (lane >> 1), qb = qa + 16;  // the lane's two tile positions
+    const uint32_t laneoff = ((uint32_t)(lane & 1) << 6) | ((uint32_t)(lane >> 1) << 2);  // 4 * (16*half + key)
+    // Software pipeline over the CTA's tiles.  While tile i is accumulated, the bin rows of tile i+1 are on their
+    // way into registers, those of tile i+2 have been asked into L2 (a prefetch holds no register), and the row ids
+    // of tile i+3 are being fetched.  The gather levels are bound by the bytes in flight (a loaded DRAM access takes
+    // 2-3 us here): one tile per warp in registers alone sustains only ~2.4 TB/s of sector traffic.
+    auto ids = [&](const int3 &e, int &ra, int &rb) {   // row ids of the lane's two positions, -1 = no record
+        ra = qa < e.y ? (GATHER ? rec_idx[e.x + qa] : e.x + qa) : -1;
+        rb = qb < e.y ? (GATHER ? rec_idx[e.x + qb] : e.x + qb) : -1;
+    };
+    const size_t half_off = (size_t)f0 + 16u * (lane & 1);
+    uint4 na = make_uint4(0, 0, 0, 0), nb = na;
+    int2 nva = make_int2(0, 0), nvb = nva;
+    auto load_rows = [&](const int3 &e, int ra, int rb) {
+        if (ra >= 0) { na = *reinterpret_cast<const uint4 *>(bins + (size_t)ra * Fpad + half_off); nva = rec_gh[e.x + qa]; }
+        if (rb >= 0) { nb = *reinterpret_cast<const uint4 *>(bins + (size_t)rb * Fpad + half_off); nvb = rec_gh[e.x + qb]; }
+    };
+    auto prefetch_rows = [&](int ra, int rb) {  // one lane of each pair asks for the row's sector
+        if (GATHER && !(lane & 1)) {
+            if (ra >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(bins + (size_t)ra * Fpad + f0));
+            if (rb >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(bins + (size_t)rb * Fpad + f0));
+        }
+    };
+    int3 e0 = next(), e1 = next(), e2 = next();
+    if (e0.y == 0) return;   // more shares than tiles
+    int r1a, r1b, r2a, r2b;
+    ids(e0, r1a, r1b);
+    ids(e1, r2a, r2b);
+    load_rows(e0, r1a, r1b);
+    prefetch_rows(r2a, r2b);
+    bool noka = r1a >= 0, nokb = r1b >= 0;
+    r1a = r2a; r1b = r2b;
+    ids(e2, r2a, r2b);
+    int pair_cur = e0.z, since = 0;
+    while (e0.y > 0) {
+        const uint4 a = na, bb = nb;
+        const int2 va2 = nva, vb2 = nvb;
+        const bool oka = noka, okb = nokb;
+        const int pair_this = e0.z;
+        e0 = e1; e1 = e2; e2 = next();
+        load_rows(e0, r1a, r1b);
+        noka = r1a >= 0; nokb = r1b >= 0;
+        prefetch_rows(r2a, r2b);
+        r1a = r2a; r1b = r2b;
+        ids(e2, r2a, r2b);
+        if (pair_this != pair_cur || (FINE && since + HIST_THREADS > FINE_WINDOW)) {  // another node: hand the finished one over
+            flush(pair_cur, true);
+            pair_cur = pair_this;
+            since = 0;
+        } else if (!FINE && since + HIST_THREADS > window_rows) {
+            drain();
+            since = 0;
+        }
+        since += HIST_THREADS;
+        // Step j adds a row to (bin of feature 16*half + (j ^ key), that feature), key = lane >> 1: the 32 lanes of a
+        // warp address 32 different features = 32 different banks.  Byte offset of the accumulator:
+        // bin * 128 | feature * 4 -- the bin field comes straight out of the packed word with one shift and one
+        // mask.  No test for missing values: bin 255 (missing, and the padding columns beyond F) lands in row 255
+        // of the table, which no feature ever reads back.
+        char *const gbase = reinterpret_cast<char *>(acc);
+        auto add = [&](uint32_t off, const int2 v) {
+            if (FINE) {
+                atomicAdd(reinterpret_cast<unsigned *>(gbase + off), (unsigned)v.x & 0xffffu);
+                atomicAdd(reinterpret_cast<unsigned *>(gbase + off + HIST_CELLS * 4), (unsigned)v.y & 0xffffu);
+                atomicAdd(reinterpret_cast<int *>(gbase + off + 2 * HIST_CELLS * 4), v.x >> 16);
+                atomicAdd(reinterpret_cast<int *>(gbase + off + 3 * HIST_CELLS * 4), v.y >> 16);
+            } else {
+                atomicAdd(reinterpret_cast<int *>(gbase + off), v.x);
+                atomicAdd(reinterpret_cast<int *>(gbase + off + HIST_CELLS * 4), v.y);
+            }
+        };
+        auto add_row = [&](const uint4 &row, const int2 v) {
+            uint32_t w[4] = {row.x, row.y, row.z, row.w};
+            xor_permute_half(w, lane >> 1);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const uint32_t word = w[j >> 2];
+                const uint32_t binoff = ((j & 3) == 0 ? (word << 7) : (word >> (8 * (j & 3) - 7))) & 0x7f80u;
+                add(binoff | (laneoff ^ (4u * j)), v);
+            }
+        };
+        if (oka) add_row(a, va2);
+        if (okb) add_row(bb, vb2);
+    }
+    flush(pair_cur, false);
+}
+
+// ------------------------------------------------------------------ histogram build, CSR of global bin ids
+// A histogram of ~100k bins does not fit in shared memory; with Zipf-like column frequencies most updates hit the lowest
+// column ids, so the first SPARSE_SMEM_BINS bins are accumulated per CTA in shared memory and the long tail goes straight to
+// the node's histogram with global int64 atomics (L2-resident: 16 B per bin).  One warp per row, lanes over its values; the
+// shared accumulators are the low and high halves of k_hist<., true> in either mode (exact values are narrower), which costs
+// four plain atomics per value: the int64 atomics they replace are compare-and-swap loops (root of 1 M rows x 30 values: 370 us).
+constexpr int SPARSE_SMEM_BINS = 12288;  // 192 KB: low and high halves of g and h
+constexpr int SPARSE_THREADS = 1024;     // one CTA per SM
+
+template <bool GATHER>
+static __global__ void __launch_bounds__(SPARSE_THREADS, 1)
+k_hist_sparse(int level, const Batch b, const int *__restrict__ row_ptr, const int *__restrict__ bin, int B, int by_hessian, int tree0) {
+    extern __shared__ __align__(16) int sh_sparse[];  // [4][nsm]: low g, low h, high g, high h; then s_base
+    __shared__ int scratch[33];
+    const int nsm = min(B, SPARSE_SMEM_BINS);
+    int *s_base = sh_sparse + 4 * nsm;
+    const size_t tree = tree0 + blockIdx.z;
+    for (int i = threadIdx.x; i < 4 * nsm; i += SPARSE_THREADS) sh_sparse[i] = 0;
+    const int total = hist_items<SPARSE_THREADS, HIST_THREADS>(level, b, tree, by_hessian, s_base, scratch, blockIdx.x == 0);
+    const int per = (total + gridDim.x - 1) / gridDim.x;
+    const int t_begin = min(total, (int)blockIdx.x * per), t_end = min(total, t_begin + per);
+    if (t_begin >= t_end) return;
+    const int pairs = level == 0 ? 1 : 1 << (level - 1);
+    const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
+    const TreeNode *nodes = b.nodes + tree * b.nodes_stride;
+    const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
+    const int2 *rec_gh = GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride;
+    long long *slab = b.hist_built + tree * b.built_stride;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto flush = [&](int pair, bool again) {
+        __syncthreads();
+        unsigned long long *dst = reinterpret_cast<unsigned long long *>(slab + (size_t)pair * B * 2);
+        for (int i = threadIdx.x; i < 2 * nsm; i += SPARSE_THREADS) {   // consecutive lanes: consecutive words of the histogram
+            const int s = (i & 1) * nsm + (i >> 1);
+            const long long v = ((long long)sh_sparse[2 * nsm + s] << 16) + (unsigned)sh_sparse[s];
+            if (v) atomicAdd(dst + i, (unsigned long long)v);
+            if (again) { sh_sparse[s] = 0; sh_sparse[2 * nsm + s] = 0; }
+        }
+        if (again) __syncthreads();
+    };
+    int w = 0;
+    {
+        int lo = 0, hi = pairs - 1;   // last item that starts at or before t_begin
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if (s_base[mid] <= t_begin) lo = mid; else hi = mid - 1;
+        }
+        w = lo;
+    }
+    int w_cur = w, since = 0, node = -1, begin = 0, count = 0;
+    for (int t = t_begin; t < t_end; ++t) {
+        while (t >= s_base[w + 1]) ++w;
+        if (w != w_cur || since + HIST_THREADS > FINE_WINDOW) { flush(w_cur, true); since = 0; }
+        since += HIST_THREADS;
+        if (w != w_cur || node < 0) {
+            w_cur = w;
+            node = level == 0 ? 0 : 2 * w + built_side(level, w, seg_cnt, nodes, by_hessian);
+            begin = seg_begin[node]; count = seg_cnt[node];
+        }
+        unsigned long long *dst = reinterpret_cast<unsigned long long *>(slab + (size_t)w * B * 2);
+        const int first = (t - s_base[w]) * HIST_THREADS;
+        const int last = min(count, first + HIST_THREADS);
+        // A warp takes every 32nd row of the tile.  Three rows are in flight per warp: the row pointers and gradients
+        // of the row after next, the first 32 bin ids of the next row, and the row being accumulated -- a row is a
+        // chain of three dependent loads (record -> row pointers -> bin ids) and would otherwise cost three memory
+        // latencies each.
+        constexpr int W = SPARSE_THREADS / 32;
+        auto meta = [&](int q, int &j0, int &j1, int2 &v) {
+            j0 = j1 = 0; v = make_int2(0, 0);
+            if (q < last) {
+                const int p = begin + q;
+                const int r = GATHER ? rec_idx[p] : p;
+                v = rec_gh[p];
+                j0 = row_ptr[r]; j1 = row_ptr[r + 1];
+            }
+        };
+        int q = first + warp;
+        int j0, j1, nj0, nj1, mj0, mj1;
+        int2 v, nv, mv;
+        meta(q, j0, j1, v);
+        meta(q + W, nj0, nj1, nv);
+        int b0 = j0 + lane < j1 ? bin[j0 + lane] : -1;
+        for (; q < last; q += W) {
+            meta(q + 2 * W, mj0, mj1, mv);
+            const int nb0 = nj0 + lane < nj1 ? bin[nj0 + lane] : -1;
+            int x = b0;
+            for (int j = j0 + lane; j < j1; j += 32) {
+                if (j != j0 + lane) x = bin[j];
+                if (x < nsm) {
+                    atomicAdd(reinterpret_cast<unsigned *>(sh_sparse + x), (unsigned)v.x & 0xffffu);
+                    atomicAdd(reinterpret_cast<unsigned *>(sh_sparse + nsm + x), (unsigned)v.y & 0xffffu);
+                    atomicAdd(sh_sparse + 2 * nsm + x, v.x >> 16);
+                    atomicAdd(sh_sparse + 3 * nsm + x, v.y >> 16);
+                } else {
+                    atomicAdd(dst + 2 * x, (unsigned long long)(long long)v.x);
+                    atomicAdd(dst + 2 * x + 1, (unsigned long long)(long long)v.y);
+                }
+            }
+            j0 = nj0; j1 = nj1; v = nv; b0 = nb0;
+            nj0 = mj0; nj1 = mj1; nv = mv;
+        }
+    }
+    flush(w_cur, false);
+}
+
+// ------------------------------------------------------------------ split evaluation
+// Histogram cells are `long long` sums on the round's fixed-point grid (exact mode) or `float` sums (fp32 mode, the
+// reference's own arithmetic: GHPair of floats, include/thundergbm/common.h:43-59).  The evaluation kernels are
+// written once over the cell type.
+template <typename T> __device__ __forceinline__ double cell_inv(const QuantInfo *q, int h);
+template <> __device__ __forceinline__ double cell_inv<long long>(const QuantInfo *q, int h) { return h ? q->inv_sh : q->inv_sg; }
+template <> __device__ __forceinline__ double cell_inv<float>(const QuantInfo *, int) { return 1.0; }
+__device__ __forceinline__ float cell_f(long long v, double inv_scale) { return q2f(v, inv_scale); }
+__device__ __forceinline__ float cell_f(float v, double) { return v; }
+__device__ __forceinline__ long long shfl_up_t(long long v, int d) { return shfl_up_ll(v, d); }
+__device__ __forceinline__ float shfl_up_t(float v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
+__device__ __forceinline__ long long shfl_t(long long v, int src) { return shfl_ll(v, src); }
+__device__ __forceinline__ float shfl_t(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+
+// one child's sums (g, h); the other child is the node minus it, `parent` the node's own term
+__device__ __forceinline__ float split_gain(float parent, float pg, float ph, float g, float h, float mcw, float lam) {
+    const float g2 = __fsub_rn(pg, g), h2 = __fsub_rn(ph, h);
+    if (h >= mcw && h2 >= mcw)
+        return __fsub_rn(__fadd_rn(__fdiv_rn(__fmul_rn(g, g), __fadd_rn(h, lam)), __fdiv_rn(__fmul_rn(g2, g2), __fadd_rn(h2, lam))), parent);
+    return 0.f;
+}
+__device__ __forceinline__ float split_gain(float pg, float ph, float lg, float lh, float rg, float rh, float mcw, float lam) {
+    // compute_gain, hist_tree_builder_single.cu:279-286 (no fused multiply-add: products feed divisions)
+    if (lh >= mcw && rh >= mcw)
+        return __fsub_rn(__fadd_rn(__fdiv_rn(__fmul_rn(lg, lg), __fadd_rn(lh, lam)), __fdiv_rn(__fmul_rn(rg, rg), __fadd_rn(rh, lam))),
+                         __fdiv_rn(__fmul_rn(pg, pg), __fadd_rn(ph, lam)));
+    return 0.f;
+}
+
+// Per-node argmax over the features, SplitPoint decode and update_tree
+// (hist_tree_builder_single.cu:365-389 and :847-902).  Called by one whole warp for node n of the level.  The records
+// may have been written by other blocks of the running kernel: they are read past L1.
+__device__ __forceinline__ SplitRec load_rec(const SplitRec *p) {
+    SplitRec r;
+    r.gain = __ldcg(&p->gain); r.bin = __ldcg(&p->bin);
+    r.lg = __ldcg(&p->lg); r.lh = __ldcg(&p->lh); r.mg = __ldcg(&p->mg); r.mh = __ldcg(&p->mh);
+    return r;
+}
+__device__ __forceinline__ void best_apply_node(int level, int n, int F, const int *__restrict__ cut_ptr,
+                                                const float *__restrict__ cut_val, const SplitRec *recs, TreeNode *nodes,
+                                                float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi) {
+    // chunked: F is the number of chunks and a record's bin is a global bin index (k_eval_chunk);
+    // otherwise one record per feature with a feature-local bin (k_eval).  Ties go to the smaller global bin either way.
+    const int lane = threadIdx.x & 31;
+    const int nid = (1 << level) - 1 + n;
+    if (!nodes[nid].is_valid) return;
+    unsigned long long key = 0;
+    int key_col = 0;  // record column (feature or chunk) of this lane's best key
+    for (int f = lane; f < F; f += 32) {
+        const SplitRec r = load_rec(recs + (size_t)n * F + f);
+        if (r.bin < 0) continue;
+        const unsigned long long k = ((unsigned long long)__float_as_uint(fabsf(r.gain)) << 32) |
+                                     (unsigned)(0x7fffffff - (chunked ? r.bin : f));
+        if (k > key) { key = k; key_col = f; }
+    }
+    // a record with gain 0 still has a key > 0, so 0 means "no record"
+    unsigned long long mk = key;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long other = (unsigned long long)shfl_xor_ll((long long)mk, o);
+        mk = other > mk ? other : mk;
+    }
+    const unsigned winners = __ballot_sync(0xffffffffu, key == mk);
+    const int win_col = __shfl_sync(0xffffffffu, key_col, __ffs(winners) - 1);
+    if (lane != 0) return;
+    TreeNode &nd = nodes[nid];
+    if (mk == 0) {  // no feature has a cut point: nothing to split on
+        nd.is_leaf = 1;
+        nodes[nd.lch_index].is_valid = 0;
+        nodes[nd.rch_index].is_valid = 0;
+        return;
+    }
+    int f = 0x7fffffff - (int)(mk & 0xffffffffull);
+    SplitRec r;
+    if (chunked) {
+        const int gbin = f;
+        f = cut_fid[gbin];
+        r = load_rec(recs + (size_t)n * F + win_col);
+        r.bin = gbin - cut_ptr[f];
+    } else {
+        r = load_rec(recs + (size_t)n * F + f);
+    }
+    const float gain = fabsf(r.gain);
+    if (gain > rt_eps) {
+        const bool default_right = r.gain < 0.f;
+        const int b0 = cut_ptr[f];
+        nd.gain = gain;
+        nd.split_feature_id = f;
+        nd.split_bid = (unsigned char)r.bin;
+        if (multi) {
+            // TreeBuilder::update_tree of the column-sharded builder (tree_builder.cu:9-60): the split value is the
+            // cut point itself, the record's sums are the right child's, the left child is the node minus it
+            nd.split_value = cut_val[b0 + r.bin];
+            TreeNode &l = nodes[nd.lch_index], &rc = nodes[nd.rch_index];
+            l.is_valid = 1; rc.is_valid = 1;
+            float rgs = r.lg, rhs = r.lh;
+            if (default_right) { rgs = __fadd_rn(rgs, r.mg); rhs = __fadd_rn(rhs, r.mh); nd.default_right = 1; }
+            else nd.default_right = 0;
+            rc.sum_g = rgs; rc.sum_h = rhs;
+            l.sum_g = __fsub_rn(nd.sum_g, rgs); l.sum_h = __fsub_rn(nd.sum_h, rhs);
+            l.base_weight = __fdiv_rn(-l.sum_g, __fadd_rn(l.sum_h, lam));
+            rc.base_weight = __fdiv_rn(-rc.sum_g, __fadd_rn(rc.sum_h, lam));
+            return;
+        }
+        if (r.bin == 0) {
+            const float c = cut_val[b0];
+            nd.split_value = (float)((double)__fsub_rn(c, fabsf(c)) - 1e-5);
+        } else {
+            nd.split_value = cut_val[b0 + r.bin - 1];
+        }
+        TreeNode &l = nodes[nd.lch_index], &rc = nodes[nd.rch_index];
+        l.is_valid = 1; rc.is_valid = 1;
+        float lgs = r.lg, lhs = r.lh;
+        if (!default_right) { lgs = __fadd_rn(lgs, r.mg); lhs = __fadd_rn(lhs, r.mh); nd.default_right = 0; }
+        else nd.default_right = 1;
+        l.sum_g = lgs; l.sum_h = lhs;
+        rc.sum_g = __fsub_rn(nd.sum_g, lgs); rc.sum_h = __fsub_rn(nd.sum_h, lhs);
+        l.base_weight = __fdiv_rn(-l.sum_g, __fadd_rn(l.sum_h, lam));
+        rc.base_weight = __fdiv_rn(-rc.sum_g, __fadd_rn(rc.sum_h, lam));
+    } else {
+        nd.is_leaf = 1;
+        nodes[nd.lch_index].is_valid = 0;
+        nodes[nd.rch_index].is_valid = 0;
+    }
+}
+
+// CSR layout: one warp per node of the level, after k_eval_chunk
+static __global__ void __launch_bounds__(32)
+k_best_apply(int level, const Batch b, int F, const int *__restrict__ cut_ptr, const float *__restrict__ cut_val,
+             float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi, int tree0) {
+    const size_t tree = tree0 + blockIdx.z;
+    best_apply_node(level, blockIdx.x, F, cut_ptr, cut_val, b.recs + tree * b.recs_stride, b.nodes + tree * b.nodes_stride, rt_eps, lam,
+                    cut_fid, chunked, multi);
+}
+
+// Sibling subtraction, per-feature prefix scan, missing sums, gains and per-feature argmax
+// (hist_tree_builder_single.cu:257-347 for the root, :538-540 and :614-704 for sibling pairs), then, by the block that
+// finishes a pair last (`ticket`, left at zero), the choice among the features and the tree update of the pair's nodes.
+// grid = (F, pairs, trees); a thread owns two bins of both children.  The gains are the work of this kernel -- four IEEE
+// divisions per bin and child -- and its time is latency: few bins per thread keep a block's chain short, few threads per
+// block keep many blocks resident.  The built histogram is zeroed as it is read, ready for the next level's reductions.
+//
+// multi: the column-sharded builder's candidates (hist_tree_builder.cu:299-352): the INCLUSIVE prefix along the
+// bins (they count down from the largest values there) is the right child, the left one is the node minus it,
+// missing values join the right child when that gains at least as much; the record then carries the right sums.
+// bs: distance of two cells of `built` in cells (1 unless the fp32 histogram kernel spread them out).
+// ignored: the round's column-sampling mask (Shard::column_sampling, src/thundergbm/builder/shard.cu:8-23; the
+// masked features take no part in the split search, hist_tree_builder_single.cu:304,663), or null.
+constexpr int EVAL_THREADS = 128, EVAL_BINS = 2;
+template <typename T> struct CellPair;
+template <> struct CellPair<long long> { typedef longlong2 type; };
+template <> struct CellPair<float> { typedef float2 type; };
+template <typename T>
+static __global__ void __launch_bounds__(EVAL_THREADS, 8)
+k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, T *__restrict__ built_all, int bs,
+       const QuantInfo *__restrict__ q, float mcw, float lam, const float *__restrict__ cut_val, float rt_eps,
+       const int *__restrict__ cut_fid, const unsigned char *__restrict__ ignored_all, const RoundState *__restrict__ rs, int multi,
+       int by_hessian, int tree0) {
+    constexpr int WARPS = EVAL_THREADS / 32, NB = EVAL_BINS;
+    __shared__ T s_sum[4][sizeof(T) == 4 ? 32 : WARPS];
+    __shared__ unsigned long long s_key[2][WARPS];
+    const int f = blockIdx.x, j = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i0 = threadIdx.x * NB;
+    const size_t tree = tree0 + blockIdx.z;
+    TreeNode *nodes = b.nodes + tree * b.nodes_stride;
+    SplitRec *recs = b.recs + tree * b.recs_stride;
+    int *ticket = b.ticket + tree * b.ticket_stride;
+    const int b0 = cut_ptr[f], nb = cut_ptr[f + 1] - b0, off = (1 << level) - 1, n_children = level == 0 ? 1 : 2;
+    const int br = level == 0 ? 0 : built_side(level, j, b.seg_cnt[level & 1] + tree * b.seg_stride, nodes, by_hessian);
+    const bool ignored = ignored_all && ignored_all[(size_t)rs->round * F + f];
+    T *full = reinterpret_cast<T *>(b.hist_full + tree * b.full_stride) + (size_t)off * B * 2;
+    T *built = built_all + (sizeof(T) == 8 ? tree * b.built_stride : 0) + ((size_t)j * B + b0) * 2 * bs;
+    using Pair = typename CellPair<T>::type;
+    // every load of the block is on its way before the first one is waited for (nothing here may alias: the compiler does
+    // not know and would wait between a store and the next load)
+    Pair cell[NB], above[NB];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+        const bool mine = i0 + n < nb && br >= 0;
+        cell[n] = above[n] = Pair{0, 0};
+        if (mine) cell[n] = *reinterpret_cast<const Pair *>(built + (size_t)2 * bs * (i0 + n));
+        if (mine && level > 0) above[n] = *reinterpret_cast<const Pair *>(full + 2 * (b0 + i0 + n) - (size_t)(1 << (level - 1)) * B * 2 + (size_t)j * B * 2);
+    }
+    bool valid[2];
+    float sum_g[2], sum_h[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const TreeNode &nd = nodes[off + (level == 0 ? 0 : 2 * j + c)];
+        valid[c] = nd.is_valid; sum_g[c] = nd.sum_g; sum_h[c] = nd.sum_h;
+    }
+    const double inv_sg = cell_inv<T>(q, 0), inv_sh = cell_inv<T>(q, 1);
+    T v[4][NB];   // g, h of the left child, g, h of the right one
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+        const T cg = cell[n].x, ch = cell[n].y, og = above[n].x - cg, oh = above[n].y - ch;
+        if (i0 + n < nb && br >= 0) {
+            *reinterpret_cast<Pair *>(built + (size_t)2 * bs * (i0 + n)) = Pair{0, 0};
+            T *own = full + 2 * (b0 + i0 + n);
+            if (level == 0) *reinterpret_cast<Pair *>(own) = cell[n];   // what the next level subtracts from
+            else {
+                *reinterpret_cast<Pair *>(own + (size_t)(2 * j + br) * B * 2) = cell[n];
+                *reinterpret_cast<Pair *>(own + (size_t)(2 * j + 1 - br) * B * 2) = Pair{og, oh};
+            }
+        }
+        v[0][n] = br == 1 ? og : cg; v[1][n] = br == 1 ? oh : ch;
+        v[2][n] = br == 1 ? cg : og; v[3][n] = br == 1 ? ch : oh;
+    }
+    const bool skip = nb == 0 || br < 0 || ignored;   // the same in the whole block
+    if (skip) {
+        if ((int)threadIdx.x < n_children) {
+            recs[(size_t)(level == 0 ? 0 : 2 * j + (int)threadIdx.x) * F + f] = SplitRec{0.f, -1, 0.f, 0.f, 0.f, 0.f};
+            __threadfence();
+        }
+    } else {
+        T base[4], tot[4], groups[4] = {0, 0, 0, 0};   // sum before the thread's first bin (float cells: in its group, before its group), sum over all bins
+        if constexpr (sizeof(T) == 4) {
+            // float cells (first round): eight bins one after the other, then a scan over the 32 groups of eight -- the order
+            // of additions this mode's parity with the reference was established with
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                T before = 0;   // sum of the group's bins before the thread's, group = four threads
+                T run = v[c][0] + v[c][1];
+#pragma unroll
+                for (int k = 1; k < 4; ++k) {
+                    const T u = shfl_up_t(run, 1);
+                    if ((lane & 3) == k) { before = u; run = (u + v[c][0]) + v[c][1]; }
+                }
+                if ((lane & 3) == 3) s_sum[c][threadIdx.x >> 2] = run;
+                base[c] = before;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                T t = s_sum[c][lane];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const T u = shfl_up_t(t, o); if (lane >= o) t += u; }
+                tot[c] = shfl_t(t, 31);
+                const int group = threadIdx.x >> 2;
+                const T g = shfl_t(t, max(group - 1, 0));
+                groups[c] = group == 0 ? T(0) : g;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const T own = v[c][0] + v[c][1];
+                T incl = own;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const T u = shfl_up_t(incl, o); if (lane >= o) incl += u; }
+                if (lane == 31) s_sum[c][warp] = incl;
+                base[c] = incl - own;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                T all = 0;
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) { if (w == warp) base[c] += all; all += s_sum[c][w]; }
+                tot[c] = all;
+            }
+        }
+        float best_gain[2], keep_g[2], keep_h[2], miss_g[2], miss_h[2];
+        unsigned long long key[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            key[c] = 0;
+            if (c >= n_children) continue;
+            const float pg = sum_g[c], ph = sum_h[c];
+            const float parent = __fdiv_rn(__fmul_rn(pg, pg), __fadd_rn(ph, lam));
+            const float mg = __fsub_rn(pg, cell_f(tot[2 * c], inv_sg)), mh = __fsub_rn(ph, cell_f(tot[2 * c + 1], inv_sh));
+            miss_g[c] = mg; miss_h[c] = mh;
+            T run_g = base[2 * c], run_h = base[2 * c + 1];
+#pragma unroll
+            for (int n = 0; n < NB; ++n) {
+                const int i = i0 + n;
+                T g = groups[2 * c] + run_g, h = groups[2 * c + 1] + run_h;
+                if (multi) { g += v[2 * c][n]; h += v[2 * c + 1][n]; }
+                run_g += v[2 * c][n]; run_h += v[2 * c + 1][n];
+                const float kg = cell_f(g, inv_sg), kh = cell_f(h, inv_sh);   // left sums (multi: right sums) without missing
+                const float kg2 = __fadd_rn(kg, mg), kh2 = __fadd_rn(kh, mh);
+                const float a = split_gain(parent, pg, ph, kg, kh, mcw, lam), z = split_gain(parent, pg, ph, kg2, kh2, mcw, lam);
+                const float gl = fmaxf(0.f, multi ? a : z), gr = fmaxf(0.f, multi ? z : a);   // missing values go left / right
+                const float gn = gl > gr ? gl : -gr;
+                // arg-abs-max, ties -> smaller bin (hist_tree_builder_single.cu:330-335)
+                const unsigned long long kk = ((unsigned long long)__float_as_uint(fabsf(gn)) << 32) | (unsigned)(0x7fffffff - i);
+                if (valid[c] && i < nb && kk > key[c]) { key[c] = kk; best_gain[c] = gn; keep_g[c] = kg; keep_h[c] = kh; }
+            }
+            // largest key of the warp: the gain first, then the bin among the lanes that hold it
+            const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(key[c] >> 32));
+            const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(key[c] >> 32) == hi ? (unsigned)key[c] : 0u);
+            if (lane == 0) s_key[c][warp] = ((unsigned long long)hi << 32) | lo;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            if (c >= n_children) continue;
+            unsigned long long mk = 0;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) mk = s_key[c][w] > mk ? s_key[c][w] : mk;
+            SplitRec *r = recs + (size_t)(level == 0 ? 0 : 2 * j + c) * F + f;
+            // the thread that writes the record also makes it visible before the block's ticket is
+            if (mk == 0) { if (threadIdx.x == 0) { *r = SplitRec{0.f, -1, 0.f, 0.f, 0.f, 0.f}; __threadfence(); } }   // the node is not valid
+            else if (key[c] == mk) {
+                *r = SplitRec{best_gain[c], 0x7fffffff - (int)(unsigned)(mk & 0xffffffffull), keep_g[c], keep_h[c], miss_g[c], miss_h[c]};
+                __threadfence();
+            }
+        }
+    }
+    __shared__ int last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(&ticket[j], 1) == (int)gridDim.x - 1;
+        if (last) ticket[j] = 0;
+    }
+    __syncthreads();
+    if (!last || warp >= n_children) return;
+    __threadfence();
+    best_apply_node(level, level == 0 ? 0 : 2 * j + warp, F, cut_ptr, cut_val, recs, nodes, rt_eps, lam, cut_fid, 0, multi);
+}
+
+// The same evaluation for data with many narrow features: one block handles a chunk of whole features whose bins
+// add up to at most 256 (a 100k-column one-hot-like data set has one or two bins per feature; a block per feature
+// would launch millions of near-empty blocks).  The scan is segmented by feature; the record of a (node, chunk) keeps
+// the GLOBAL bin index of its best candidate.  grid = (chunks, pairs); block = 64.
+template <typename T>
+static __global__ void __launch_bounds__(64)
+k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restrict__ chunk_bin0, const int *__restrict__ cut_ptr,
+             const int *__restrict__ cut_fid, T *__restrict__ built_all, int bs, const QuantInfo *__restrict__ q, float mcw, float lam,
+             const unsigned char *__restrict__ ignored_all, const RoundState *__restrict__ rs, int F, int multi, int by_hessian, int tree0) {
+    const size_t tree = tree0 + blockIdx.z;
+    const TreeNode *nodes = b_.nodes + tree * b_.nodes_stride;
+    SplitRec *recs = b_.recs + tree * b_.recs_stride;
+    T *full = reinterpret_cast<T *>(b_.hist_full + tree * b_.full_stride) + (size_t)((1 << level) - 1) * B * 2;
+    T *built = built_all + (sizeof(T) == 8 ? tree * b_.built_stride : 0);
+    __shared__ T sg[2][256], sh[2][256];
+    const unsigned char *ignored = ignored_all ? ignored_all + (size_t)rs->round * F : nullptr;
+    const int c = blockIdx.x, j = blockIdx.y;
+    const int b0 = chunk_bin0[c], nb = chunk_bin0[c + 1] - b0;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_children = level == 0 ? 1 : 2;
+    const int node_local = level == 0 ? 0 : 2 * j + warp;
+    const int off = (1 << level) - 1;
+    const SplitRec none = {0.f, -1, 0.f, 0.f, 0.f, 0.f};
+    const int br = level == 0 ? 0 : built_side(level, j, b_.seg_cnt[level & 1] + tree * b_.seg_stride, nodes, by_hessian);
+    if (nb == 0 || br < 0) {
+        if (lane == 0 && warp < n_children) recs[(size_t)node_local * n_chunks + c] = none;
+        return;
+    }
+    if (level == 0) {
+        for (int i = threadIdx.x; i < nb; i += 64) {
+            T *cell = built + (size_t)2 * bs * (b0 + i);
+            const T cg = cell[0], ch = cell[1];
+            cell[0] = 0; cell[1] = 0;   // zeroed as it is read, like in k_eval
+            sg[0][i] = cg; sh[0][i] = ch;
+            full[2 * (b0 + i)] = cg; full[2 * (b0 + i) + 1] = ch;
+        }
+    } else {
+        T *bp = built + (size_t)j * B * 2 * bs;
+        const T *pp = full - (size_t)(1 << (level - 1)) * B * 2 + (size_t)j * B * 2;
+        T *fb = full + (size_t)(2 * j + br) * B * 2, *fo = full + (size_t)(2 * j + 1 - br) * B * 2;
+        for (int i = threadIdx.x; i < nb; i += 64) {
+            T *cell = bp + (size_t)2 * bs * (b0 + i);
+            const T cg = cell[0], ch = cell[1];
+            cell[0] = 0; cell[1] = 0;
+            const T og = pp[2 * (b0 + i)] - cg, oh = pp[2 * (b0 + i) + 1] - ch;
+            sg[br][i] = cg; sh[br][i] = ch;
+            sg[1 - br][i] = og; sh[1 - br][i] = oh;
+            fb[2 * (b0 + i)] = cg; fb[2 * (b0 + i) + 1] = ch;
+            fo[2 * (b0 + i)] = og; fo[2 * (b0 + i) + 1] = oh;
+        }
+    }
+    __syncthreads();
+    if (warp >= n_children) return;
+    const TreeNode nd = nodes[off + node_local];
+    if (!nd.is_valid) {
+        if (lane == 0) recs[(size_t)node_local * n_chunks + c] = none;
+        return;
+    }
+    // lane-local pass over 8 consecutive bins; sums restart where a feature starts
+    T eg[8], eh[8];       // exclusive prefix inside the feature, as far as the lane can see
+    bool before_start[8];         // no feature start in this lane up to and including this bin -> add the carry
+    T rg = 0, rh = 0;
+    bool seen = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int b = lane * 8 + i;
+        if (b < nb) {
+            const int f = cut_fid[b0 + b];
+            if (cut_ptr[f] == b0 + b) { rg = 0; rh = 0; seen = true; }
+            eg[i] = rg; eh[i] = rh; before_start[i] = !seen;
+            rg += sg[warp][b]; rh += sh[warp][b];
+        } else { eg[i] = 0; eh[i] = 0; before_start[i] = false; }
+    }
+    // segmented inclusive scan of the lanes' open tails (rg, rh); flag = the lane contains a feature start
+    T vg = rg, vh = rh;
+    bool fl = seen;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T ug = shfl_up_t(vg, o), uh = shfl_up_t(vh, o);
+        const int uf = __shfl_up_sync(0xffffffffu, (int)fl, o);
+        if (lane >= o) {
+            if (!fl) { vg += ug; vh += uh; }
+            fl = fl || uf;
+        }
+    }
+    T cg = shfl_up_t(vg, 1), ch = shfl_up_t(vh, 1);  // carry into this lane = inclusive value of lane-1
+    if (lane == 0) { cg = 0; ch = 0; }
+    // inclusive prefix per bin back into shared memory: the last bin of a feature then holds the feature total
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int b = lane * 8 + i;
+        if (b < nb) {
+            if (before_start[i]) { eg[i] += cg; eh[i] += ch; }
+            const T ig = eg[i] + sg[warp][b], ih = eh[i] + sh[warp][b];
+            sg[warp][b] = ig; sh[warp][b] = ih;
+        }
+    }
+    __syncwarp();
+    const float pg = nd.sum_g, ph = nd.sum_h;
+    const double inv_sg = cell_inv<T>(q, 0), inv_sh = cell_inv<T>(q, 1);
+    float best = 0.f, best_lg = 0.f, best_lh = 0.f, best_mg = 0.f, best_mh = 0.f;
+    int best_bin = -1;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int b = lane * 8 + i;
+        if (b < nb && !(ignored && ignored[cut_fid[b0 + b]])) {
+            const int f = cut_fid[b0 + b];
+            const int lastb = cut_ptr[f + 1] - 1 - b0;
+            const float mg = __fsub_rn(pg, cell_f(sg[warp][lastb], inv_sg)), mh = __fsub_rn(ph, cell_f(sh[warp][lastb], inv_sh));
+            float gn, keep_g, keep_h;
+            if (multi) {  // inclusive prefix = right child, see eval_feature
+                const float rg = cell_f(sg[warp][b], inv_sg), rh = cell_f(sh[warp][b], inv_sh);
+                const float gl = fmaxf(0.f, split_gain(pg, ph, __fsub_rn(pg, rg), __fsub_rn(ph, rh), rg, rh, mcw, lam));
+                const float rg2 = __fadd_rn(rg, mg), rh2 = __fadd_rn(rh, mh);
+                const float gr = fmaxf(0.f, split_gain(pg, ph, __fsub_rn(pg, rg2), __fsub_rn(ph, rh2), rg2, rh2, mcw, lam));
+                gn = gl > gr ? gl : -gr; keep_g = rg; keep_h = rh;
+            } else {
+                const float lg = cell_f(eg[i], inv_sg), lh = cell_f(eh[i], inv_sh);
+                const float gr = fmaxf(0.f, split_gain(pg, ph, lg, lh, __fsub_rn(pg, lg), __fsub_rn(ph, lh), mcw, lam));
+                const float lg2 = __fadd_rn(lg, mg), lh2 = __fadd_rn(lh, mh);
+                const float gl = fmaxf(0.f, split_gain(pg, ph, lg2, lh2, __fsub_rn(pg, lg2), __fsub_rn(ph, lh2), mcw, lam));
+                gn = gl > gr ? gl : -gr; keep_g = lg; keep_h = lh;
+            }
+            if (best_bin < 0 || fabsf(gn) > fabsf(best)) { best = gn; best_bin = b0 + b; best_lg = keep_g; best_lh = keep_h; best_mg = mg; best_mh = mh; }
+        }
+    }
+    unsigned long long key = best_bin < 0 ? 0ull
+                                          : (((unsigned long long)__float_as_uint(fabsf(best)) << 32) | (unsigned)(0x7fffffff - best_bin));
+    unsigned long long mk = key;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long other = (unsigned long long)shfl_xor_ll((long long)mk, o);
+        mk = other > mk ? other : mk;
+    }
+    const unsigned win = __ballot_sync(0xffffffffu, key == mk && best_bin >= 0);
+    const int src = __ffs(win) - 1;
+    best = __shfl_sync(0xffffffffu, best, src);
+    best_bin = __shfl_sync(0xffffffffu, best_bin, src);
+    best_lg = __shfl_sync(0xffffffffu, best_lg, src);
+    best_lh = __shfl_sync(0xffffffffu, best_lh, src);
+    best_mg = __shfl_sync(0xffffffffu, best_mg, src);
+    best_mh = __shfl_sync(0xffffffffu, best_mh, src);
+    if (lane == 0) recs[(size_t)node_local * n_chunks + c] = SplitRec{best, best_bin, best_lg, best_lh, best_mg, best_mh};
+}
+
+
+// ------------------------------------------------------------------ instance partition
+// (replaces update_ins2node_id + the per-level radix sort, hist_tree_builder_single.cu:908-1020, :397-415)
+// Every node of the level that holds records gets ceil(count / PART_TILE) tiles of PART_TILE records; each block takes a
+// contiguous run of the tiles.  Two kernels: the first finds the direction of every record (one bit) and the left count of
+// every tile, the second moves the records.  What lies between them needs no kernel of its own: a block's records start
+// where the lefts of the node's tiles before its run end, and those are the tail counts (lefts in the last node of a
+// run) of the few blocks before it that lie in the same node.
+// Output: left children of all nodes in the first half of the record buffers, right children in the second, both at the
+// number of records of the nodes before theirs.  Stable: the rows of either child ascend like those of the node.  Records
+// of nodes that stopped splitting drop out.
+
+// prologue of both kernels: tiles (s_tile) and records (s_rec) before every node, total tiles
+__device__ __forceinline__ int part_items(int level, const int *seg_cnt, int *s_tile, int *s_rec, int *scratch) {
+    const int nl = 1 << level;
+    const int total = block_prefix<PART_THREADS>(nl, [&](int n) { return (seg_cnt[n] + PART_TILE - 1) / PART_TILE; }, [&](int n, int t) { s_tile[n] = t; }, scratch);
+    if (s_rec) block_prefix<PART_THREADS>(nl, [&](int n) { return seg_cnt[n]; }, [&](int n, int r) { s_rec[n] = r; }, scratch);
+    if (threadIdx.x == 0) s_tile[nl] = total;
+    __syncthreads();
+    return total;
+}
+// node that owns tile t: the n with s_tile[n] <= t < s_tile[n + 1]
+__device__ __forceinline__ int tile_owner(const int *s_tile, int nl, int t) {
+    int lo = 0, hi = nl;  // first n with s_tile[n] > t
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (s_tile[mid] > t) hi = mid; else lo = mid + 1;
+    }
+    return lo - 1;
+}
+
+// Direction of every record of a splittable node: left unless (missing and default right) or
+// bin >= split_bid (hist_tree_builder_single.cu:1003-1012).  A thread handles PART_RPT records of a tile so that their
+// loads overlap.
+// SPARSE: the row's bin of the split feature is searched in its CSR bin ids (hist_tree_builder_single.cu:941-966)
+// instead of being read from the column-major matrix.
+template <bool SPARSE>
+static __global__ void __launch_bounds__(PART_THREADS)
+k_part_count(int level, const Batch b, const unsigned char *__restrict__ binsT, size_t Npad, const int *__restrict__ sp_row_ptr,
+             const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr, int rev, int tree0) {
+    extern __shared__ int s_tile[];   // [nl + 1]
+    __shared__ int wsum[PART_THREADS / 32], scratch[33];
+    const int nl = 1 << level, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t tree = tree0 + blockIdx.z;
+    const TreeNode *nodes = b.nodes + tree * b.nodes_stride + nl - 1;
+    const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
+    const int *rec_idx = level == 0 ? nullptr : b.rec_idx[level & 1] + tree * b.rec_stride;
+    unsigned *bits = b.bits + tree * b.bits_stride;
+    const int total = part_items(level, seg_cnt, s_tile, nullptr, scratch);
+    const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x, t_begin = min(total, (int)blockIdx.x * per), t_end = min(total, t_begin + per);
+    int n = t_begin < t_end ? tile_owner(s_tile, nl, t_begin) : 0, tail = 0, fresh = -1;
+    TreeNode nd;
+    int begin = 0, end = 0;
+    for (int t = t_begin; t < t_end; ++t) {
+        while (t >= s_tile[n + 1]) ++n;
+        if (n != fresh) { fresh = n; nd = nodes[n]; begin = seg_begin[n]; end = begin + seg_cnt[n]; tail = 0; }
+        if (!(nd.is_valid && !nd.is_leaf)) continue;   // finished node
+        const int p0 = begin + (t - s_tile[n]) * PART_TILE;
+        const unsigned char *colp = SPARSE ? nullptr : binsT + (size_t)nd.split_feature_id * Npad;
+        int r[PART_RPT];
+#pragma unroll
+        for (int j = 0; j < PART_RPT; ++j) {
+            const int p = p0 + j * PART_THREADS + threadIdx.x;
+            r[j] = p < end ? (rec_idx ? rec_idx[p] : p) : -1;
+        }
+        unsigned char bin[PART_RPT];
+        if (SPARSE) {
+            const int c0 = cut_ptr[nd.split_feature_id], c1 = cut_ptr[nd.split_feature_id + 1];
+#pragma unroll
+            for (int j = 0; j < PART_RPT; ++j) {
+                bin[j] = MISSING_BIN;
+                if (r[j] >= 0) {
+                    int lo = sp_row_ptr[r[j]], hi = sp_row_ptr[r[j] + 1];  // bin ids ascend inside a row
+                    while (lo < hi) {
+                        const int mid = lo + (hi - lo) / 2, v = sp_bin[mid];
+                        if (v >= c0 && v < c1) { bin[j] = (unsigned char)(v - c0); break; }
+                        if (v < c0) lo = mid + 1; else hi = mid;
+                    }
+                }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < PART_RPT; ++j) bin[j] = r[j] >= 0 ? colp[r[j]] : 0;
+        }
+        int cnt = 0;
+#pragma unroll
+        for (int j = 0; j < PART_RPT; ++j) {
+            const bool left = r[j] >= 0 && ((bin[j] == MISSING_BIN) ? !nd.default_right : (rev ? bin[j] > nd.split_bid : bin[j] < nd.split_bid));
+            const unsigned m = __ballot_sync(0xffffffffu, left);
+            if (lane == 0) bits[(size_t)t * (PART_TILE / 32) + j * (PART_THREADS / 32) + warp] = m;
+            cnt += __popc(m);
+        }
+        __syncthreads();  // wsum of the previous tile has been read
+        if (lane == 0) wsum[warp] = cnt;
+        __syncthreads();
+        int v = lane < PART_THREADS / 32 ? wsum[lane] : 0;
+        v = __reduce_add_sync(0xffffffffu, v);
+        tail += v;
+        if (threadIdx.x == 0) b.tile_left[tree * b.tile_stride + t] = v;
+    }
+    if (threadIdx.x == 0) b.tail_left[tree * b.tail_stride + blockIdx.x] = tail;
+}
+
+// Stable scatter of the records into the child segments, and the segment table of the next level.  Same grid as k_part_count.
+static __global__ void __launch_bounds__(PART_THREADS, 2048 / PART_THREADS)
+k_part_scatter(int level, const Batch b, int tree0) {
+    constexpr int WORDS = PART_TILE / 32;
+    extern __shared__ int s_tile[];   // [nl + 1], then records before every node [nl]
+    __shared__ int wpre[WORDS], wtot[(WORDS + 31) / 32], scratch[33];
+    const int nl = 1 << level, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int *s_rec = s_tile + nl + 1;
+    const size_t tree = tree0 + blockIdx.z;
+    const TreeNode *nodes = b.nodes + tree * b.nodes_stride + nl - 1;
+    const int in = level & 1, nx = in ^ 1;
+    const int *seg_begin = b.seg_begin[in] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[in] + tree * b.seg_stride;
+    int *next_begin = b.seg_begin[nx] + tree * b.seg_stride, *next_cnt = b.seg_cnt[nx] + tree * b.seg_stride;
+    const int *rec_idx = level == 0 ? nullptr : b.rec_idx[in] + tree * b.rec_stride;
+    const int2 *rec_gh = level == 0 ? b.gh + tree * b.gh_stride : b.rec_gh[in] + tree * b.rec_stride;
+    int *out_idx = b.rec_idx[nx] + tree * b.rec_stride;
+    int2 *out_gh = b.rec_gh[nx] + tree * b.rec_stride;
+    const unsigned *bits = b.bits + tree * b.bits_stride;
+    const int *tile_left = b.tile_left + tree * b.tile_stride, *tail_left = b.tail_left + tree * b.tail_stride;
+    const int total = part_items(level, seg_cnt, s_tile, s_rec, scratch);
+    auto set_children = [&](int n, int left, int right) {
+        next_cnt[2 * n] = left; next_cnt[2 * n + 1] = right;
+        next_begin[2 * n] = s_rec[n]; next_begin[2 * n + 1] = b.half + s_rec[n];
+    };
+    if (blockIdx.x == 0) {
+        for (int n = threadIdx.x; n < nl; n += PART_THREADS)
+            if (s_tile[n] == s_tile[n + 1]) set_children(n, 0, 0);   // no tile, no block to do it
+        if (threadIdx.x == 0) atomicAdd(&b.ctl->stat_part_rows, (unsigned long long)(s_rec[nl - 1] + seg_cnt[nl - 1]));
+    }
+    const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x, t_begin = min(total, (int)blockIdx.x * per), t_end = min(total, t_begin + per);
+    if (t_begin >= t_end) return;
+    int n = tile_owner(s_tile, nl, t_begin), fresh = -1, before = 0;   // lefts of the node before the running tile
+    {
+        const int c0 = s_tile[n] / per;   // the block that holds the node's first tile
+        int v = 0;
+        for (int c = c0 + lane; c < (int)blockIdx.x; c += 32) v += tail_left[c];
+        before = __reduce_add_sync(0xffffffffu, v);   // (every warp for itself)
+    }
+    TreeNode nd;
+    int begin = 0, end = 0, base_l = 0, base_r = 0;
+    for (int t = t_begin; t < t_end; ++t) {
+        while (t >= s_tile[n + 1]) ++n;
+        if (n != fresh) {
+            if (fresh >= 0) before = 0;
+            fresh = n; nd = nodes[n]; begin = seg_begin[n]; end = begin + seg_cnt[n];
+            base_l = s_rec[n]; base_r = b.half + base_l;
+        }
+        if (!(nd.is_valid && !nd.is_leaf)) {   // finished node: its records leave the lists
+            if (t == s_tile[n] && threadIdx.x == 0) set_children(n, 0, 0);
+            continue;
+        }
+        const int p0 = begin + (t - s_tile[n]) * PART_TILE, here = tile_left[t];
+        // loads first, so that they overlap with the rank computation
+        int r[PART_RPT];
+        int2 g[PART_RPT];
+        unsigned m[PART_RPT];
+#pragma unroll
+        for (int j = 0; j < PART_RPT; ++j) {
+            const int p = p0 + j * PART_THREADS + threadIdx.x;
+            r[j] = p < end ? (rec_idx ? rec_idx[p] : p) : -1;
+            if (p < end) g[j] = rec_gh[p];
+            m[j] = bits[(size_t)t * WORDS + j * (PART_THREADS / 32) + warp];
+        }
+        __syncthreads();  // wpre / wtot of the previous tile have been read
+        // exclusive prefix of the left counts over the tile's ballot words (record order = word order)
+        if (threadIdx.x < WORDS) {
+            const int c = __popc(bits[(size_t)t * WORDS + threadIdx.x]);
+            int v = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+            wpre[threadIdx.x] = v - c;
+            if (lane == 31) wtot[warp] = v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < PART_RPT; ++j) {
+            if (r[j] < 0) continue;
+            const int w = j * (PART_THREADS / 32) + warp;
+            int pre = wpre[w];
+            for (int q = 0; q < (w >> 5); ++q) pre += wtot[q];
+            const bool left = (m[j] >> lane) & 1u;
+            const int lefts = before + pre + __popc(m[j] & ((1u << lane) - 1u));
+            const int d = left ? base_l + lefts : base_r + (p0 - begin + j * PART_THREADS + (int)threadIdx.x - lefts);
+            out_idx[d] = r[j];
+            out_gh[d] = g[j];
+        }
+        before += here;
+        if (t == s_tile[n + 1] - 1 && threadIdx.x == 0) set_children(n, before, end - begin - before);
+    }
+}
+
+}  // namespace tgbm
