@@ -19,6 +19,7 @@
 #include "tgbm_kernels.cuh"
 #include "tgbm_level.cuh"
 #include "tgbm_hist_f32.cuh"
+#include "tgbm_small.cuh"
 #include "tgbm_exact.cuh"
 #include "tgbm_rank.cuh"
 
@@ -146,6 +147,9 @@ struct BoosterImpl {
     void init_base_score();
     void gradient(int round);
     void build_trees(int round, int k0, int n_trees);
+    SmallPlan small{};   // cluster > 0: trees of integer rounds are built by k_small_tree
+    void plan_small_trees();
+    void launch_small_trees(int k0, int n_trees);
     void round_metric(int round);
 };
 
@@ -633,7 +637,7 @@ void BoosterImpl::exact_levels(int k, const void *gh_rows) {
 void BoosterImpl::build_tree_exact(int round, int k) {
     const int tree_index = round * K + k;
     k_tree_init<<<ceil_div(n_nodes, 256), 256, 0, stream>>>(nodes.p, n_nodes, root_sum.p + 2 * k, qinfo.p, p.lambda, N,
-                                                            seg_begin[0].p, seg_cnt[0].p, bufs.seg_stride, f32 ? 1 : 0);
+                                                            seg_begin[0].p, seg_cnt[0].p, bufs.seg_stride, f32 ? 1 : 0, maxbits.p);
     if (f32) exact_levels<float>(k, gh.p + (size_t)k * N);
     else exact_levels<long long>(k, ghq.p + (size_t)k * N);
     k_prune<<<1, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream>>>(nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0, model.p, K, k,
@@ -769,6 +773,7 @@ void Booster::init(const DataSet &ds) {
     }
     m.ypred.zero(m.stream);
     m.maxbits.alloc(2); m.root_sum.alloc(2 * (size_t)K); m.qinfo.alloc(1);
+    m.maxbits.zero(m.stream); m.root_sum.zero(m.stream);
     if (p.bagging) {
         TGBM_CHECK((unsigned long long)std::max(p.num_class, 1) * (unsigned long long)m.N_global < (1ull << 32), "bagging: num_class x rows must fit 32 bits");
         m.bag_count.alloc(n1 * K);
@@ -868,6 +873,7 @@ void Booster::init(const DataSet &ds) {
     m.prune_in_smem = sizeof(TreeNode) * (size_t)m.n_nodes <= 200 * 1024;  // up to depth 11
     if (m.prune_in_smem && sizeof(TreeNode) * (size_t)m.n_nodes > 40 * 1024)   // (the kernel has static shared memory beside it)
         TGBM_CUDA(cudaFuncSetAttribute(k_prune, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(TreeNode) * (size_t)m.n_nodes)));
+    m.plan_small_trees();
     if (need_group_file(m.objective)) m.rank.init(ds, m.objective, m.N, m.stream, first_group, total_groups);
     });
     agree("allocating its training buffers");
@@ -886,16 +892,15 @@ void BoosterImpl::gradient(int round) {
     // the pass that applied the previous tree has already found this round's gradient maxima
     const bool have_max = pointwise && grad_max_ready && round >= 0 && !float_round(round) && !p.bagging;
     grad_max_ready = false;
-    root_sum.zero(stream);
+    // (root_sum and maxbits are zero here: k_round_end and k_tree_init leave them so)
     if (!have_max) {
-        maxbits.zero(stream);
         if (N) {
             const int gb = std::max(1, std::min(ceil_div(N, tb), num_sms * 8));
             switch (objective) {
             case REG_LINEAR: case REG_LOGISTIC: case BINARY_LOGISTIC:
-                k_grad_pointwise<<<gb, tb, 0, stream>>>(y.p, ypred.p, N, logistic, gh.p, maxbits.p); break;
+                launch_after(k_grad_pointwise, gb, tb, 0, stream, y.p, ypred.p, N, logistic, gh.p, maxbits.p); break;
             case MULTI_SOFTMAX: case MULTI_SOFTPROB:
-                k_grad_softmax<<<gb, tb, 0, stream>>>(y.p, ypred.p, N, K, gh.p, maxbits.p); break;
+                launch_after(k_grad_softmax, gb, tb, 0, stream, y.p, ypred.p, N, K, gh.p, maxbits.p); break;
             case RANK_PAIRWISE: case RANK_NDCG:
                 rank.gradient(rstate.p, p.rank_seed, ypred.p, gh.p, maxbits.p, stream); break;
             }
@@ -911,8 +916,8 @@ void BoosterImpl::gradient(int round) {
         launches += 2;
     }
     if (float_round(round)) {  // float gradients as they are; root sums in fp64, block partials combined in a fixed order
-        k_sum_gh<<<dim3(SUM_BLOCKS, K), 256, 0, stream>>>(gh.p, N, sum_partial.p);
-        k_sum_gh_final<<<K, 32, 0, stream>>>(sum_partial.p, SUM_BLOCKS, reinterpret_cast<double *>(root_sum.p));
+        launch_after(k_sum_gh, dim3(SUM_BLOCKS, K), 256, 0, stream, gh.p, N, sum_partial.p);
+        launch_after(k_sum_gh_final, K, 32, 0, stream, sum_partial.p, SUM_BLOCKS, reinterpret_cast<double *>(root_sum.p));
         launches += 2;
         if (comm && comm->active()) comm->allreduce(root_sum.p, 2 * (size_t)K, Comm::F64, Comm::SUM, stream);
         return;
@@ -920,7 +925,7 @@ void BoosterImpl::gradient(int round) {
     if (comm && comm->active()) comm->allreduce(maxbits.p, 2, Comm::U32, Comm::MAX, stream);
     const int blocks = std::max(1, std::min(ceil_div(N, tb), num_sms * 8));
     auto quantize = [&](auto kern, int bits) {
-        kern<<<dim3(blocks, K), tb, 0, stream>>>(have_max ? nullptr : gh.p, N, maxbits.p, bits, (uint32_t)round, (uint32_t)row_offset,
+        launch_after(kern, dim3(blocks, K), tb, 0, stream, have_max ? nullptr : gh.p, N, maxbits.p, bits, (uint32_t)round, (uint32_t)row_offset,
                                                  ghq.p, root_sum.p, qinfo.p, y.p, ypred.p, logistic, round >= 0 ? rstate.p : nullptr);
     };
     if (f32) quantize(k_quantize<true>, FINE_BITS);
@@ -958,6 +963,63 @@ void BoosterImpl::init_base_score() {
     base_score = w;
     p.base_score = w;
     if (N) k_fill<<<std::min(ceil_div(N, 256), num_sms * 8), 256, 0, stream>>>(ypred.p, (size_t)N, w);
+    root_sum.zero(stream); maxbits.zero(stream);
+}
+
+// Is the data small enough for a tree per launch (tgbm_small.cuh)?  Every CTA of the cluster walks all rows for its share of
+// the features, so its time grows with rows x features per CTA and, deep down, with nodes x features per CTA, while a level
+// of the level kernels takes 25-30 us at any size up to a few hundred thousand rows.
+void BoosterImpl::plan_small_trees() {
+    small = SmallPlan{};
+    if (sparse || exact || (comm && comm->active()) || N < 1 || N > 32768 || depth < 1 || F > 4096) return;
+    SmallPlan pl{};
+    pl.cluster = 1;
+    while (pl.cluster < 16 && pl.cluster < F) pl.cluster *= 2;
+    const int max_nl = 1 << (depth - 1);
+    cudaFuncSetAttribute(k_small_tree, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (; pl.cluster >= 1; pl.cluster /= 2) {
+        pl.feats = ceil_div(F, pl.cluster);
+        pl.bins = 1;
+        for (int f = 0; f < F; f += pl.feats) pl.bins = std::max(pl.bins, h_cut_ptr[std::min(F, f + pl.feats)] - h_cut_ptr[f]);
+        if ((double)N * pl.feats > 8e4 || (double)max_nl * pl.feats > 512) return;
+        const size_t budget = 200 * 1024, fixed = (sizeof(TreeNode) * (size_t)n_nodes + 15) / 16 * 16 + sizeof(SmallPost) * 2 * max_nl + (size_t)(N + 7) / 8 * 16;
+        const size_t per_node = 16 * (size_t)pl.bins + sizeof(SplitRec) * pl.feats;
+        if (fixed + per_node > budget) return;
+        pl.nodes_pass = (int)std::min<size_t>(max_nl, (budget - fixed) / per_node);
+        if (max_nl > 8 * pl.nodes_pass) return;   // the rows would be walked over and over
+        pl.smem = fixed + per_node * pl.nodes_pass;
+        TGBM_CUDA(cudaFuncSetAttribute(k_small_tree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = pl.cluster; cfg.blockDim = SMALL_THREADS; cfg.dynamicSmemBytes = pl.smem;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = pl.cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr; cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, k_small_tree, &cfg) == cudaSuccess && fit >= 1) {
+            small = pl;
+            return;
+        }
+        cudaGetLastError();   // no GPC has room for a cluster of this size: half of it
+    }
+}
+
+void BoosterImpl::launch_small_trees(int k0, int n_trees) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = small.cluster * n_trees; cfg.blockDim = SMALL_THREADS; cfg.dynamicSmemBytes = small.smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = small.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    const int2 *gq = ghq.p + (size_t)k0 * N;
+    const unsigned long long *roots = root_sum.p + 2 * (size_t)k0;
+    TGBM_CUDA(cudaLaunchKernelEx(&cfg, k_small_tree, (SmallPlan)small, N, Npad, F, depth, (const unsigned char *)binsT.p, (const int *)cut_ptr.p,
+                                 (const float *)cut_val.p, gq, roots, (const QuantInfo *)qinfo.p, p.min_child_weight, p.lambda, p.rt_eps, p.gamma,
+                                 (const unsigned char *)ignored_all.p, (const RoundState *)rstate.p, p.column_shards > 0 ? 1 : 0, nodes.p, model.p, K, k0,
+                                 maxbits.p, ctl.p, hist_full.p, bufs.full_stride));
+    ++launches;
 }
 
 // Trees k0 .. k0 + n_trees - 1 of the round, level by level side by side (n_trees <= batch).
@@ -968,26 +1030,30 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
     Batch b = bufs;
     // float rounds: the records carry the float gradient pairs themselves (same 8 bytes)
     b.gh = float_sums ? reinterpret_cast<const int2 *>(gh.p + (size_t)k0 * N) : ghq.p + (size_t)k0 * N;
-    k_tree_init<<<dim3(ceil_div(n_nodes, 256), n_trees), 256, 0, stream>>>(nodes.p, n_nodes, root_sum.p + 2 * k0, qinfo.p, p.lambda, N,
-                                                                           seg_begin[0].p, seg_cnt[0].p, b.seg_stride, float_sums ? 1 : 0);
+    const bool one_launch = small.cluster > 0 && !float_sums && !profile_on;
+    if (one_launch) launch_small_trees(k0, n_trees);
+    else {
+    launch_after(k_tree_init, dim3(ceil_div(n_nodes, 256), n_trees), 256, 0, stream, nodes.p, n_nodes, root_sum.p + 2 * k0, qinfo.p, p.lambda, N,
+                                                                           seg_begin[0].p, seg_cnt[0].p, b.seg_stride, float_sums ? 1 : 0, maxbits.p);
     ++launches;
+    }
     const int by_hessian = (comm && comm->active()) ? 1 : 0;
     const int colb = p.column_shards > 0 ? 1 : 0;  // candidates, tie rule and child sums of the column-sharded builder
     // one CTA per SM over all trees and feature groups: every further CTA is one more flush per node
     const int hist_ctas = std::max(1, num_sms / (n_trees * (sparse ? 1 : G)));
-    for (int level = 0; level < depth; ++level) {
+    for (int level = 0; level < depth && !one_launch; ++level) {
         const int nl = 1 << level, pairs = std::max(1, nl / 2);
         const size_t table = sizeof(int) * ((size_t)pairs + 1);
         // -- histogram of the root / of the smaller child of every pair, and the choice of the splits
         auto evaluate = [&](auto *built, int bs, int tree, int n) {
             using T = std::remove_pointer_t<decltype(built)>;
             if (sparse) {
-                k_eval_chunk<T><<<dim3(n_chunks, pairs, n), 64, 0, stream>>>(level, b, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_fid.p, built, bs, qinfo.p,
+                launch_after(k_eval_chunk<T>, dim3(n_chunks, pairs, n), 64, 0, stream, level, b, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_fid.p, built, bs, qinfo.p,
                                                                              p.min_child_weight, p.lambda, ignored_all.p, rstate.p, F, colb, by_hessian, tree);
-                k_best_apply<<<dim3(nl, 1, n), 32, 0, stream>>>(level, b, n_chunks, cut_ptr.p, cut_val.p, p.rt_eps, p.lambda, cut_fid.p, 1, colb, tree);
+                launch_after(k_best_apply, dim3(nl, 1, n), 32, 0, stream, level, b, n_chunks, cut_ptr.p, cut_val.p, p.rt_eps, p.lambda, cut_fid.p, 1, colb, tree);
                 launches += 2;
             } else {
-                k_eval<T><<<dim3(F, pairs, n), EVAL_THREADS, 0, stream>>>(level, b, F, B, cut_ptr.p, built, bs, qinfo.p, p.min_child_weight, p.lambda,
+                launch_after(k_eval<T>, dim3(F, pairs, n), EVAL_THREADS, 0, stream, level, b, F, B, cut_ptr.p, built, bs, qinfo.p, p.min_child_weight, p.lambda,
                                                                          cut_val.p, p.rt_eps, cut_fid.p, ignored_all.p, rstate.p, colb, by_hessian, tree);
                 ++launches;
             }
@@ -1012,10 +1078,10 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
                 timed(level == 0 ? 0 : 1, [&] {
                     if (sparse) {
                         auto kern = level == 0 ? k_hist_sparse_f32<false> : k_hist_sparse_f32<true>;
-                        kern<<<ctas, F32_THREADS, table, stream>>>(level, b, sp_row_ptr.p, sp_bin.p, cells, B, bs, by_hessian, t);
+                        launch_after(kern, ctas, F32_THREADS, table, stream, level, b, sp_row_ptr.p, sp_bin.p, cells, B, bs, by_hessian, t);
                     } else {
                         auto kern = level == 0 ? k_hist_f32<false> : k_hist_f32<true>;
-                        kern<<<dim3(ctas, G), F32_THREADS, table, stream>>>(level, b, bins.p, Fpad, F, cut_ptr.p, cells, B, bs, f32_cuts, F <= 256,
+                        launch_after(kern, dim3(ctas, G), F32_THREADS, table, stream, level, b, bins.p, Fpad, F, cut_ptr.p, cells, B, bs, f32_cuts, F <= 256,
                                                                             f32_staged ? 1 : 0, by_hessian, t);
                     }
                 });
@@ -1024,7 +1090,7 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
                     // the ranks' sums meet in a compact buffer: spread cells are gathered first (a pass over B x pairs cells)
                     if (bs != 1) {
                         const size_t n = (size_t)B * pairs;
-                        k_compact_cells<<<std::min(ceil_div(n, 256), num_sms * 8), 256, 0, stream>>>(cells, compact, n, bs);
+                        launch_after(k_compact_cells, std::min(ceil_div(n, 256), num_sms * 8), 256, 0, stream, cells, compact, n, bs);
                         ++launches;
                     }
                     comm->allreduce(compact, 2 * (size_t)B * pairs, Comm::F32, Comm::SUM, stream);
@@ -1035,12 +1101,10 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
             timed(level == 0 ? 0 : 1, [&] {
                 if (sparse) {
                     auto kern = level == 0 ? k_hist_sparse<false> : k_hist_sparse<true>;
-                    kern<<<dim3(hist_ctas, 1, n_trees), SPARSE_THREADS, (size_t)std::min(B, SPARSE_SMEM_BINS) * 16 + table, stream>>>(
-                        level, b, sp_row_ptr.p, sp_bin.p, B, by_hessian, 0);
+                    launch_after(kern, dim3(hist_ctas, 1, n_trees), SPARSE_THREADS, (size_t)std::min(B, SPARSE_SMEM_BINS) * 16 + table, stream, level, b, sp_row_ptr.p, sp_bin.p, B, by_hessian, 0);
                 } else {
                     auto kern = level == 0 ? (fine ? k_hist<false, true> : k_hist<false, false>) : (fine ? k_hist<true, true> : k_hist<true, false>);
-                    kern<<<dim3(hist_ctas, G, n_trees), HIST_THREADS, (fine ? HIST_FINE_SMEM : HIST_EXACT_SMEM) + table, stream>>>(
-                        level, b, bins.p, Fpad, F, cut_ptr.p, B, window_rows, by_hessian, 0);
+                    launch_after(kern, dim3(hist_ctas, G, n_trees), HIST_THREADS, (fine ? HIST_FINE_SMEM : HIST_EXACT_SMEM) + table, stream, level, b, bins.p, Fpad, F, cut_ptr.p, B, window_rows, by_hessian, 0);
                 }
             });
             ++launches;
@@ -1053,13 +1117,13 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
         timed(2, [&] {
             const dim3 grid(part_ctas, 1, n_trees);
             const size_t nodes_table = sizeof(int) * ((size_t)nl + 1);
-            if (sparse) k_part_count<true><<<grid, PART_THREADS, nodes_table, stream>>>(level, b, nullptr, Npad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, colb, 0);
-            else k_part_count<false><<<grid, PART_THREADS, nodes_table, stream>>>(level, b, binsT.p, Npad, nullptr, nullptr, cut_ptr.p, colb, 0);
-            k_part_scatter<<<grid, PART_THREADS, 2 * nodes_table, stream>>>(level, b, 0);
+            if (sparse) launch_after(k_part_count<true>, grid, PART_THREADS, nodes_table, stream, level, b, nullptr, Npad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, colb, 0);
+            else launch_after(k_part_count<false>, grid, PART_THREADS, nodes_table, stream, level, b, binsT.p, Npad, nullptr, nullptr, cut_ptr.p, colb, 0);
+            launch_after(k_part_scatter, grid, PART_THREADS, 2 * nodes_table, stream, level, b, 0);
         });
         launches += 2;
     }
-    k_prune<<<n_trees, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream>>>(nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0,
+    if (!one_launch) launch_after(k_prune, n_trees, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream, nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0,
                                                                                               model.p, K, k0, rstate.p);
     if (N) {
         const size_t per_node = sizeof(WalkNode) + (sparse ? sizeof(WalkSpan) : 0);
@@ -1072,9 +1136,8 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
         const bool fuse = K == 1 && (objective == REG_LINEAR || objective == REG_LOGISTIC || objective == BINARY_LOGISTIC);
         const dim3 walk_ctas(fuse ? metric_blocks() : std::min(ceil_div(N, 256), num_sms * 8), n_trees);
         const int fo = fuse ? objective : -1;
-        if (fuse) maxbits.zero(stream);
         auto kern = sparse ? k_predict_walk<2> : Fpad == 32 ? k_predict_walk<0> : k_predict_walk<1>;
-        kern<<<walk_ctas, 256, walk_smem, stream>>>(nodes.p, n_nodes, in_smem, sparse ? nullptr : bins.p, Fpad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, N,
+        launch_after(kern, walk_ctas, 256, walk_smem, stream, nodes.p, n_nodes, in_smem, sparse ? nullptr : bins.p, Fpad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, N,
                                                     p.learning_rate, yp, nid_out, y.p, fo, metric_partial.p, maxbits.p, colb);
         grad_max_ready = metric_partial_ready = fuse;
     }
@@ -1085,13 +1148,13 @@ void BoosterImpl::round_metric(int round) {
     const int log_len = (int)qinfo_log.n;
     if (need_group_file(objective)) {
         rank.metric(objective, ypred.p, nullptr, comm, N_global, stream);
-        k_round_end<<<1, 32, 0, stream>>>(objective, rank.sum.p, nullptr, 0, rank.n_group_total, metric.p, qinfo.p, qinfo_log.p, log_len, rstate.p);
+        launch_after(k_round_end, 1, 32, 0, stream, objective, rank.sum.p, nullptr, 0, rank.n_group_total, metric.p, qinfo.p, qinfo_log.p, log_len, rstate.p, root_sum.p, 2 * K);
         ++launches;
         return;
     }
     const int blocks = metric_blocks();
     if (!metric_partial_ready) {  // else the walk that applied the round's tree has left the partial sums
-        k_metric_partial<<<blocks, 256, 0, stream>>>(objective, y.p, ypred.p, N, K, metric_partial.p);
+        launch_after(k_metric_partial, blocks, 256, 0, stream, objective, y.p, ypred.p, N, K, metric_partial.p);
         ++launches;
     }
     metric_partial_ready = false;
@@ -1101,8 +1164,8 @@ void BoosterImpl::round_metric(int round) {
         comm->allreduce(metric_sum.p, 1, Comm::F64, Comm::SUM, stream);
         ++launches;
     }
-    k_round_end<<<1, 32, 0, stream>>>(objective, metric_sum.p, multi ? nullptr : metric_partial.p, blocks, N_global, metric.p, qinfo.p, qinfo_log.p,
-                                      log_len, rstate.p);
+    launch_after(k_round_end, 1, 32, 0, stream, objective, metric_sum.p, multi ? nullptr : metric_partial.p, blocks, N_global, metric.p, qinfo.p, qinfo_log.p,
+                                      log_len, rstate.p, root_sum.p, 2 * K);
     ++launches;
 }
 

@@ -74,8 +74,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
 template <bool GATHER>
 static __global__ void __launch_bounds__(F32_THREADS)
 k_hist_f32(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpad, int F, const int *__restrict__ cut_ptr,
-           float2 *__restrict__ slab, int B, int cell_stride, const __grid_constant__ CutOffsets cuts, int cuts_in_param, int staged,
+           float2 *slab, int B, int cell_stride, const __grid_constant__ CutOffsets cuts, int cuts_in_param, int staged,
            int by_hessian, int tree) {
+    chain_wait();
     extern __shared__ int s_base[];
     __shared__ int s_cut[32], scratch[33];
     __shared__ __align__(16) int s_idx[2][STAGE_IDX];
@@ -163,8 +164,9 @@ k_hist_f32(int level, const Batch b, const unsigned char *__restrict__ bins, int
 // CSR layout: a warp per record, lanes over the row's stored values (global bin ids).
 template <bool GATHER>
 static __global__ void __launch_bounds__(F32_THREADS)
-k_hist_sparse_f32(int level, const Batch b, const int *__restrict__ row_ptr, const int *__restrict__ bin, float2 *__restrict__ slab, int B,
+k_hist_sparse_f32(int level, const Batch b, const int *__restrict__ row_ptr, const int *__restrict__ bin, float2 *slab, int B,
                   int cell_stride, int by_hessian, int tree) {
+    chain_wait();
     extern __shared__ int s_base[];
     __shared__ int scratch[33];
     const int total = hist_items<F32_THREADS, HIST_THREADS>(level, b, tree, by_hessian, s_base, scratch, blockIdx.x == 0);
@@ -198,7 +200,8 @@ k_hist_sparse_f32(int level, const Batch b, const int *__restrict__ row_ptr, con
 // pairs in the reference): fp64 partial sums per block in a fixed order, then one warp per class.
 constexpr int SUM_BLOCKS = 256;
 static __global__ void __launch_bounds__(256)
-k_sum_gh(const float2 *__restrict__ gh, int n, double *__restrict__ partial) {
+k_sum_gh(const float2 *gh, int n, double *partial) {
+    chain_wait();
     __shared__ double wg[8], wh[8];
     const int k = blockIdx.y;
     double sg = 0, sh = 0;
@@ -218,12 +221,14 @@ k_sum_gh(const float2 *__restrict__ gh, int n, double *__restrict__ partial) {
     }
 }
 // spread cells (`stride` float2 apart) -> consecutive cells: what the ranks all-reduce
-static __global__ void k_compact_cells(const float2 *__restrict__ spread, float2 *__restrict__ compact, size_t cells, int stride) {
+static __global__ void k_compact_cells(const float2 *spread, float2 *compact, size_t cells, int stride) {
+    chain_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x)
         compact[i] = spread[i * (size_t)stride];
 }
 
-static __global__ void k_sum_gh_final(const double *__restrict__ partial, int nb, double *__restrict__ out) {
+static __global__ void k_sum_gh_final(const double *partial, int nb, double *out) {
+    chain_wait();
     const int k = blockIdx.x;
     double tg = 0, th = 0;
     for (int i = threadIdx.x; i < nb; i += 32) { tg += partial[((size_t)k * nb + i) * 2]; th += partial[((size_t)k * nb + i) * 2 + 1]; }

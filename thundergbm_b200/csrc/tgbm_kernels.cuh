@@ -298,8 +298,9 @@ __device__ __forceinline__ double pointwise_metric_term(int objective, float y, 
     return (double)__fmul_rn(e, e);
 }
 
-static __global__ void k_grad_pointwise(const float *__restrict__ y, const float *__restrict__ yp, int n, int logistic,
-                                 float2 *__restrict__ gh, unsigned *__restrict__ maxbits) {
+static __global__ void k_grad_pointwise(const float *y, const float *yp, int n, int logistic,
+                                 float2 *gh, unsigned *maxbits) {
+    chain_wait();
     float mg = 0.f, mh = 0.f;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float2 v = pointwise_gh(logistic, y[i], yp[i]);
@@ -311,8 +312,9 @@ static __global__ void k_grad_pointwise(const float *__restrict__ y, const float
 }
 
 // Softmax::get_gradient (src/thundergbm/objective/multiclass_obj.cu:7-35), class-major gh[k*N+i]
-static __global__ void k_grad_softmax(const float *__restrict__ y, const float *__restrict__ yp, int n, int K,
-                               float2 *__restrict__ gh, unsigned *__restrict__ maxbits) {
+static __global__ void k_grad_softmax(const float *y, const float *yp, int n, int K,
+                               float2 *gh, unsigned *maxbits) {
+    chain_wait();
     float mg = 0.f, mh = 0.f;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float mx = yp[i];
@@ -345,11 +347,12 @@ static __global__ void k_grad_softmax(const float *__restrict__ y, const float *
 // `gh` null: the gradients are those of a pointwise objective (`logistic` 0/1) and are computed again from y and the
 // scores here -- the pass that found their maxima (k_predict_walk) did not store them.
 template <bool FINE>
-static __global__ void k_quantize(const float2 *__restrict__ gh, int n, const unsigned *__restrict__ maxbits, int quant_bits,
-                           uint32_t round, uint32_t row_offset, int2 *__restrict__ ghq,
-                           unsigned long long *__restrict__ root_sum, QuantInfo *__restrict__ qinfo,
-                           const float *__restrict__ y, const float *__restrict__ yp, int logistic,
-                           const RoundState *__restrict__ rs) {
+static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbits, int quant_bits,
+                           uint32_t round, uint32_t row_offset, int2 *ghq,
+                           unsigned long long *root_sum, QuantInfo *qinfo,
+                           const float *y, const float *yp, int logistic,
+                           const RoundState *rs) {
+    chain_wait();
     if (rs) round = (uint32_t)rs->round;  // the booster's rounds; the base-score pass gives its own
     const int k = blockIdx.y;
     const int eg = exp_above(__uint_as_float(maxbits[0])), eh = exp_above(__uint_as_float(maxbits[1]));
@@ -415,10 +418,13 @@ static __global__ void k_bag_scale(float2 *__restrict__ gh, const int *__restric
 // Tree::init2 (src/thundergbm/tree.cu:8-39)
 // root_is_f64: fp32 mode, the root sums are doubles (k_sum_gh_final) instead of integers on the fixed-point grid
 // grid.y = trees of the batch; seg tables: the root holds every row
-static __global__ void k_tree_init(TreeNode *__restrict__ nodes, int n_nodes, const unsigned long long *__restrict__ root_sum,
-                            const QuantInfo *__restrict__ q, float lambda, int n_rows, int *__restrict__ seg_begin,
-                            int *__restrict__ seg_cnt, size_t seg_stride, int root_is_f64) {
+static __global__ void k_tree_init(TreeNode *nodes, int n_nodes, const unsigned long long *root_sum,
+                            const QuantInfo *q, float lambda, int n_rows, int *seg_begin,
+                            int *seg_cnt, size_t seg_stride, int root_is_f64, unsigned *maxbits) {
+    // maxbits: the quantisation has used the round's maxima; those of the next round's gradients are collected from zero
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 2 && blockIdx.y == 0) maxbits[i] = 0;
     if (i >= n_nodes) return;
     const size_t tree = blockIdx.y;
     root_sum += 2 * tree;
@@ -478,20 +484,7 @@ __device__ inline int block_scan_excl(int n, In in, Out out, int *scratch) {
 // Tree::prune_self / try_prune_leaf / reorder_nid (src/thundergbm/tree.cu:85-128).  The reference walks the
 // leaves in index order and climbs while a parent has two leaf children and gain < gamma; the fixed point of that
 // walk does not depend on the order, so the levels are processed bottom-up with one thread per node.  One block.
-static __global__ void __launch_bounds__(1024)
-k_prune(TreeNode *__restrict__ nodes, int n_nodes, int depth, float gamma, int table_in_smem, TreeNode *__restrict__ model, int K, int k0,
-        const RoundState *__restrict__ rs) {
-    // grid = trees of the batch.  The finished tree also goes to its slot of the model, tree (round * K + class).
-    nodes += (size_t)blockIdx.x * n_nodes;
-    model += ((size_t)rs->round * K + k0 + blockIdx.x) * n_nodes;
-    extern __shared__ __align__(16) unsigned char sm[];
-    __shared__ int scratch[33];
-    // trees too large for shared memory (depth 12 to 14) are pruned in place in global memory
-    TreeNode *sn = table_in_smem ? reinterpret_cast<TreeNode *>(sm) : nodes;
-    if (table_in_smem) {
-        for (int i = threadIdx.x; i < n_nodes; i += blockDim.x) sn[i] = nodes[i];
-        __syncthreads();
-    }
+__device__ inline void prune_tree(TreeNode *sn, int n_nodes, int depth, float gamma, int *scratch) {   // called by 1024 threads
     for (int level = depth - 1; level >= 0; --level) {
         const int nl = 1 << level, off = nl - 1;
         for (int n = threadIdx.x; n < nl; n += blockDim.x) {
@@ -508,10 +501,29 @@ k_prune(TreeNode *__restrict__ nodes, int n_nodes, int depth, float gamma, int t
     block_scan_excl(n_nodes, [&](int i) { return (sn[i].is_valid && !sn[i].is_pruned) ? 1 : 0; },
                     [&](int i, int id) { if (sn[i].is_valid && !sn[i].is_pruned) sn[i].final_id = id; }, scratch);
     __syncthreads();
-    for (int i = threadIdx.x; i < n_nodes; i += blockDim.x) {
-        const TreeNode t = sn[i];
-        if (table_in_smem) nodes[i] = t;
-        model[i] = t;
+}
+static __global__ void __launch_bounds__(1024)
+k_prune(TreeNode *nodes, int n_nodes, int depth, float gamma, int table_in_smem, TreeNode *model, int K, int k0,
+        const RoundState *rs) {
+    chain_wait();
+    // grid = trees of the batch.  The finished tree also goes to its slot of the model, tree (round * K + class).
+    nodes += (size_t)blockIdx.x * n_nodes;
+    model += ((size_t)rs->round * K + k0 + blockIdx.x) * n_nodes;
+    extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ int scratch[33];
+    // trees too large for shared memory (depth 12 to 14) are pruned in place in global memory; the 48-byte records are
+    // copied as the 16-byte pieces they consist of
+    TreeNode *sn = table_in_smem ? reinterpret_cast<TreeNode *>(sm) : nodes;
+    const int pieces = n_nodes * (int)(sizeof(TreeNode) / 16);
+    if (table_in_smem) {
+        for (int i = threadIdx.x; i < pieces; i += blockDim.x) reinterpret_cast<int4 *>(sn)[i] = reinterpret_cast<const int4 *>(nodes)[i];
+        __syncthreads();
+    }
+    prune_tree(sn, n_nodes, depth, gamma, scratch);
+    for (int i = threadIdx.x; i < pieces; i += blockDim.x) {
+        const int4 t = reinterpret_cast<const int4 *>(sn)[i];
+        if (table_in_smem) reinterpret_cast<int4 *>(nodes)[i] = t;
+        reinterpret_cast<int4 *>(model)[i] = t;
     }
 }
 
@@ -528,7 +540,7 @@ k_prune(TreeNode *__restrict__ nodes, int n_nodes, int depth, float gamma, int t
 struct WalkNode { int flags; float weight; };
 struct WalkSpan { int c0, c1; };  // CSR layout: global bins [c0, c1) of the split feature
 
-__device__ __forceinline__ WalkNode walk_node(const TreeNode *__restrict__ nodes, int i, int rev) {
+__device__ __forceinline__ WalkNode walk_node(const TreeNode *nodes, int i, int rev) {
     const TreeNode nd = nodes[i];
     const bool split = nd.is_valid && nd.lch_index >= 0 && nodes[nd.lch_index].is_valid;
     WalkNode w;
@@ -537,7 +549,7 @@ __device__ __forceinline__ WalkNode walk_node(const TreeNode *__restrict__ nodes
     w.weight = nd.base_weight;
     return w;
 }
-__device__ __forceinline__ WalkSpan walk_span(const TreeNode *__restrict__ nodes, const int *__restrict__ cut_ptr, int i) {
+__device__ __forceinline__ WalkSpan walk_span(const TreeNode *nodes, const int *__restrict__ cut_ptr, int i) {
     const TreeNode nd = nodes[i];
     const bool split = nd.is_valid && nd.lch_index >= 0 && nodes[nd.lch_index].is_valid;
     const int f = split ? nd.split_feature_id : 0;
@@ -551,11 +563,12 @@ __device__ __forceinline__ WalkSpan walk_span(const TreeNode *__restrict__ nodes
 // memory at every step.
 template <int LAYOUT>
 static __global__ void __launch_bounds__(256)
-k_predict_walk(const TreeNode *__restrict__ nodes, int n_nodes, int table_in_smem, const unsigned char *__restrict__ bins, int Fpad,
+k_predict_walk(const TreeNode *nodes, int n_nodes, int table_in_smem, const unsigned char *__restrict__ bins, int Fpad,
                const int *__restrict__ sp_row_ptr, const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr,
-               int n, float lr, float *__restrict__ yp, int *__restrict__ nid_out,
-               const float *__restrict__ y, int fuse_objective, double *__restrict__ metric_partial,
-               unsigned *__restrict__ maxbits, int rev) {
+               int n, float lr, float *yp, int *__restrict__ nid_out,
+               const float *__restrict__ y, int fuse_objective, double *metric_partial,
+               unsigned *maxbits, int rev) {
+    chain_wait();
     // blockIdx.y: tree of the batch
     nodes += (size_t)blockIdx.y * n_nodes;
     yp += (size_t)blockIdx.y * n;
@@ -642,8 +655,9 @@ k_predict_walk(const TreeNode *__restrict__ nodes, int n_nodes, int table_in_sme
 // ------------------------------------------------------------------ metrics
 // per-block partial sums in a fixed order: RMSE (pointwise_metric.cu:8-22), binary error and
 // multi-class accuracy (multiclass_metric.cu:9-46)
-static __global__ void k_metric_partial(int objective, const float *__restrict__ y, const float *__restrict__ yp, int n, int K,
-                                 double *__restrict__ partial) {
+static __global__ void k_metric_partial(int objective, const float *__restrict__ y, const float *yp, int n, int K,
+                                 double *partial) {
+    chain_wait();
     __shared__ double ws[32];
     double s = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -687,12 +701,20 @@ static __global__ void k_metric_final(int objective, const double *__restrict__ 
 // End of a boosting round: the round's metric (for ranking `sum` and `n_total` are those of the query groups), the round's
 // fixed-point grid for the log, and the device round counter moves on.  One warp; `partial` not null: the sum is that of the
 // `nb` partial sums, added like k_metric_sum adds them.
-static __global__ void k_round_end(int objective, const double *__restrict__ sum, const double *__restrict__ partial, int nb, long long n_total,
-                                   float *__restrict__ metric, const QuantInfo *__restrict__ qinfo, QuantInfo *__restrict__ qinfo_log, int log_len,
-                                   RoundState *__restrict__ rs) {
+static __global__ void k_round_end(int objective, const double *sum, const double *partial, int nb, long long n_total,
+                                   float *metric, const QuantInfo *qinfo, QuantInfo *qinfo_log, int log_len,
+                                   RoundState *rs,
+                                   unsigned long long *root_sum, int n_root) {
+    chain_wait();
+    for (int i = threadIdx.x; i < n_root; i += 32) root_sum[i] = 0;   // the next round adds to them
     double t = 0;
     if (partial) {
-        for (int i = threadIdx.x; i < nb; i += 32) t += partial[i];
+        // (at most 1024 partial sums: all loads first, then the additions in the usual order)
+        double v[32];
+#pragma unroll
+        for (int u = 0; u < 32; ++u) v[u] = (int)threadIdx.x + 32 * u < nb ? partial[threadIdx.x + 32 * u] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 32; ++u) t += v[u];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     }

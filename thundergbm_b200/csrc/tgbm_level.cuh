@@ -190,6 +190,7 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
     const size_t tree = tree0 + blockIdx.z;
     for (int i = threadIdx.x; i < (FINE ? HIST_FINE_SMEM : HIST_EXACT_SMEM) / 16; i += HIST_THREADS)
         reinterpret_cast<int4 *>(hist_sm)[i] = make_int4(0, 0, 0, 0);
+    chain_wait();
     if (threadIdx.x == 0) { s_ib = 0x7fffffff; s_ie = -1; }
     const int total = hist_items<HIST_THREADS, HIST_THREADS>(level, b, tree, by_hessian, s_base, scratch, blockIdx.x == 0 && group == 0);
     if (total == 0) return;
@@ -382,6 +383,7 @@ k_hist_sparse(int level, const Batch b, const int *__restrict__ row_ptr, const i
     int *s_base = sh_sparse + 4 * nsm;
     const size_t tree = tree0 + blockIdx.z;
     for (int i = threadIdx.x; i < 4 * nsm; i += SPARSE_THREADS) sh_sparse[i] = 0;
+    chain_wait();
     const int total = hist_items<SPARSE_THREADS, HIST_THREADS>(level, b, tree, by_hessian, s_base, scratch, blockIdx.x == 0);
     const int per = (total + gridDim.x - 1) / gridDim.x;
     const int t_begin = min(total, (int)blockIdx.x * per), t_end = min(total, t_begin + per);
@@ -507,50 +509,10 @@ __device__ __forceinline__ SplitRec load_rec(const SplitRec *p) {
     r.lg = __ldcg(&p->lg); r.lh = __ldcg(&p->lh); r.mg = __ldcg(&p->mg); r.mh = __ldcg(&p->mh);
     return r;
 }
-__device__ __forceinline__ void best_apply_node(int level, int n, int F, const int *__restrict__ cut_ptr,
-                                                const float *__restrict__ cut_val, const SplitRec *recs, TreeNode *nodes,
-                                                float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi) {
-    // chunked: F is the number of chunks and a record's bin is a global bin index (k_eval_chunk);
-    // otherwise one record per feature with a feature-local bin (k_eval).  Ties go to the smaller global bin either way.
-    const int lane = threadIdx.x & 31;
-    const int nid = (1 << level) - 1 + n;
-    if (!nodes[nid].is_valid) return;
-    unsigned long long key = 0;
-    int key_col = 0;  // record column (feature or chunk) of this lane's best key
-    for (int f = lane; f < F; f += 32) {
-        const SplitRec r = load_rec(recs + (size_t)n * F + f);
-        if (r.bin < 0) continue;
-        const unsigned long long k = ((unsigned long long)__float_as_uint(fabsf(r.gain)) << 32) |
-                                     (unsigned)(0x7fffffff - (chunked ? r.bin : f));
-        if (k > key) { key = k; key_col = f; }
-    }
-    // a record with gain 0 still has a key > 0, so 0 means "no record"
-    unsigned long long mk = key;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long other = (unsigned long long)shfl_xor_ll((long long)mk, o);
-        mk = other > mk ? other : mk;
-    }
-    const unsigned winners = __ballot_sync(0xffffffffu, key == mk);
-    const int win_col = __shfl_sync(0xffffffffu, key_col, __ffs(winners) - 1);
-    if (lane != 0) return;
+// SplitPoint of candidate r (feature-local bin) of feature f into node nd and its children: TreeBuilder::update_tree
+__device__ __forceinline__ void apply_split(TreeNode *nodes, int nid, int f, const SplitRec &r, const int *__restrict__ cut_ptr,
+                                            const float *__restrict__ cut_val, float rt_eps, float lam, int multi) {
     TreeNode &nd = nodes[nid];
-    if (mk == 0) {  // no feature has a cut point: nothing to split on
-        nd.is_leaf = 1;
-        nodes[nd.lch_index].is_valid = 0;
-        nodes[nd.rch_index].is_valid = 0;
-        return;
-    }
-    int f = 0x7fffffff - (int)(mk & 0xffffffffull);
-    SplitRec r;
-    if (chunked) {
-        const int gbin = f;
-        f = cut_fid[gbin];
-        r = load_rec(recs + (size_t)n * F + win_col);
-        r.bin = gbin - cut_ptr[f];
-    } else {
-        r = load_rec(recs + (size_t)n * F + f);
-    }
     const float gain = fabsf(r.gain);
     if (gain > rt_eps) {
         const bool default_right = r.gain < 0.f;
@@ -595,10 +557,58 @@ __device__ __forceinline__ void best_apply_node(int level, int n, int F, const i
     }
 }
 
+__device__ __forceinline__ void best_apply_node(int level, int n, int F, const int *__restrict__ cut_ptr,
+                                                const float *__restrict__ cut_val, const SplitRec *recs, TreeNode *nodes,
+                                                float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi) {
+    // chunked: F is the number of chunks and a record's bin is a global bin index (k_eval_chunk);
+    // otherwise one record per feature with a feature-local bin (k_eval).  Ties go to the smaller global bin either way.
+    const int lane = threadIdx.x & 31;
+    const int nid = (1 << level) - 1 + n;
+    if (!nodes[nid].is_valid) return;
+    unsigned long long key = 0;
+    int key_col = 0;  // record column (feature or chunk) of this lane's best key
+    for (int f = lane; f < F; f += 32) {
+        const SplitRec r = load_rec(recs + (size_t)n * F + f);
+        if (r.bin < 0) continue;
+        const unsigned long long k = ((unsigned long long)__float_as_uint(fabsf(r.gain)) << 32) |
+                                     (unsigned)(0x7fffffff - (chunked ? r.bin : f));
+        if (k > key) { key = k; key_col = f; }
+    }
+    // a record with gain 0 still has a key > 0, so 0 means "no record"
+    unsigned long long mk = key;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long other = (unsigned long long)shfl_xor_ll((long long)mk, o);
+        mk = other > mk ? other : mk;
+    }
+    const unsigned winners = __ballot_sync(0xffffffffu, key == mk);
+    const int win_col = __shfl_sync(0xffffffffu, key_col, __ffs(winners) - 1);
+    if (lane != 0) return;
+    TreeNode &nd = nodes[nid];
+    if (mk == 0) {  // no feature has a cut point: nothing to split on
+        nd.is_leaf = 1;
+        nodes[nd.lch_index].is_valid = 0;
+        nodes[nd.rch_index].is_valid = 0;
+        return;
+    }
+    int f = 0x7fffffff - (int)(mk & 0xffffffffull);
+    SplitRec r;
+    if (chunked) {
+        const int gbin = f;
+        f = cut_fid[gbin];
+        r = load_rec(recs + (size_t)n * F + win_col);
+        r.bin = gbin - cut_ptr[f];
+    } else {
+        r = load_rec(recs + (size_t)n * F + f);
+    }
+    apply_split(nodes, nid, f, r, cut_ptr, cut_val, rt_eps, lam, multi);
+}
+
 // CSR layout: one warp per node of the level, after k_eval_chunk
 static __global__ void __launch_bounds__(32)
 k_best_apply(int level, const Batch b, int F, const int *__restrict__ cut_ptr, const float *__restrict__ cut_val,
              float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi, int tree0) {
+    chain_wait();
     const size_t tree = tree0 + blockIdx.z;
     best_apply_node(level, blockIdx.x, F, cut_ptr, cut_val, b.recs + tree * b.recs_stride, b.nodes + tree * b.nodes_stride, rt_eps, lam,
                     cut_fid, chunked, multi);
@@ -623,9 +633,9 @@ template <> struct CellPair<long long> { typedef longlong2 type; };
 template <> struct CellPair<float> { typedef float2 type; };
 template <typename T>
 static __global__ void __launch_bounds__(EVAL_THREADS, 8)
-k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, T *__restrict__ built_all, int bs,
-       const QuantInfo *__restrict__ q, float mcw, float lam, const float *__restrict__ cut_val, float rt_eps,
-       const int *__restrict__ cut_fid, const unsigned char *__restrict__ ignored_all, const RoundState *__restrict__ rs, int multi,
+k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, T *built_all, int bs,
+       const QuantInfo *q, float mcw, float lam, const float *__restrict__ cut_val, float rt_eps,
+       const int *__restrict__ cut_fid, const unsigned char *__restrict__ ignored_all, const RoundState *rs, int multi,
        int by_hessian, int tree0) {
     constexpr int WARPS = EVAL_THREADS / 32, NB = EVAL_BINS;
     __shared__ T s_sum[4][sizeof(T) == 4 ? 32 : WARPS];
@@ -636,6 +646,7 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
     SplitRec *recs = b.recs + tree * b.recs_stride;
     int *ticket = b.ticket + tree * b.ticket_stride;
     const int b0 = cut_ptr[f], nb = cut_ptr[f + 1] - b0, off = (1 << level) - 1, n_children = level == 0 ? 1 : 2;
+    chain_wait();
     const int br = level == 0 ? 0 : built_side(level, j, b.seg_cnt[level & 1] + tree * b.seg_stride, nodes, by_hessian);
     const bool ignored = ignored_all && ignored_all[(size_t)rs->round * F + f];
     T *full = reinterpret_cast<T *>(b.hist_full + tree * b.full_stride) + (size_t)off * B * 2;
@@ -794,8 +805,9 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
 template <typename T>
 static __global__ void __launch_bounds__(64)
 k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restrict__ chunk_bin0, const int *__restrict__ cut_ptr,
-             const int *__restrict__ cut_fid, T *__restrict__ built_all, int bs, const QuantInfo *__restrict__ q, float mcw, float lam,
-             const unsigned char *__restrict__ ignored_all, const RoundState *__restrict__ rs, int F, int multi, int by_hessian, int tree0) {
+             const int *__restrict__ cut_fid, T *built_all, int bs, const QuantInfo *q, float mcw, float lam,
+             const unsigned char *__restrict__ ignored_all, const RoundState *rs, int F, int multi, int by_hessian, int tree0) {
+    chain_wait();
     const size_t tree = tree0 + blockIdx.z;
     const TreeNode *nodes = b_.nodes + tree * b_.nodes_stride;
     SplitRec *recs = b_.recs + tree * b_.recs_stride;
@@ -815,27 +827,34 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
         if (lane == 0 && warp < n_children) recs[(size_t)node_local * n_chunks + c] = none;
         return;
     }
-    if (level == 0) {
-        for (int i = threadIdx.x; i < nb; i += 64) {
-            T *cell = built + (size_t)2 * bs * (b0 + i);
-            const T cg = cell[0], ch = cell[1];
-            cell[0] = 0; cell[1] = 0;   // zeroed as it is read, like in k_eval
-            sg[0][i] = cg; sh[0][i] = ch;
-            full[2 * (b0 + i)] = cg; full[2 * (b0 + i) + 1] = ch;
-        }
-    } else {
+    {
+        // (the loads of all four bins of a thread first: the stores below may alias them as far as the compiler knows)
+        using Pair = typename CellPair<T>::type;
+        Pair cell[4], above[4];
         T *bp = built + (size_t)j * B * 2 * bs;
-        const T *pp = full - (size_t)(1 << (level - 1)) * B * 2 + (size_t)j * B * 2;
-        T *fb = full + (size_t)(2 * j + br) * B * 2, *fo = full + (size_t)(2 * j + 1 - br) * B * 2;
-        for (int i = threadIdx.x; i < nb; i += 64) {
-            T *cell = bp + (size_t)2 * bs * (b0 + i);
-            const T cg = cell[0], ch = cell[1];
-            cell[0] = 0; cell[1] = 0;
-            const T og = pp[2 * (b0 + i)] - cg, oh = pp[2 * (b0 + i) + 1] - ch;
-            sg[br][i] = cg; sh[br][i] = ch;
-            sg[1 - br][i] = og; sh[1 - br][i] = oh;
-            fb[2 * (b0 + i)] = cg; fb[2 * (b0 + i) + 1] = ch;
-            fo[2 * (b0 + i)] = og; fo[2 * (b0 + i) + 1] = oh;
+        const T *pp = full - (level == 0 ? 0 : (size_t)(1 << (level - 1)) * B * 2) + (size_t)j * B * 2;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = threadIdx.x + 64 * u;
+            if (i < nb) {
+                cell[u] = *reinterpret_cast<const Pair *>(bp + (size_t)2 * bs * (b0 + i));
+                if (level > 0) above[u] = *reinterpret_cast<const Pair *>(pp + 2 * (size_t)(b0 + i));
+            }
+        }
+        T *fb = full + (level == 0 ? 0 : (size_t)(2 * j + br) * B * 2), *fo = full + (size_t)(2 * j + 1 - br) * B * 2;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = threadIdx.x + 64 * u;
+            if (i >= nb) continue;
+            *reinterpret_cast<Pair *>(bp + (size_t)2 * bs * (b0 + i)) = Pair{0, 0};   // zeroed as it is read, like in k_eval
+            *reinterpret_cast<Pair *>(fb + 2 * (size_t)(b0 + i)) = cell[u];
+            const int side = level == 0 ? 0 : br;
+            sg[side][i] = cell[u].x; sh[side][i] = cell[u].y;
+            if (level > 0) {
+                const T og = above[u].x - cell[u].x, oh = above[u].y - cell[u].y;
+                sg[1 - br][i] = og; sh[1 - br][i] = oh;
+                *reinterpret_cast<Pair *>(fo + 2 * (size_t)(b0 + i)) = Pair{og, oh};
+            }
         }
     }
     __syncthreads();
@@ -973,6 +992,7 @@ template <bool SPARSE>
 static __global__ void __launch_bounds__(PART_THREADS)
 k_part_count(int level, const Batch b, const unsigned char *__restrict__ binsT, size_t Npad, const int *__restrict__ sp_row_ptr,
              const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr, int rev, int tree0) {
+    chain_wait();
     extern __shared__ int s_tile[];   // [nl + 1]
     __shared__ int wsum[PART_THREADS / 32], scratch[33];
     const int nl = 1 << level, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1039,6 +1059,7 @@ k_part_count(int level, const Batch b, const unsigned char *__restrict__ binsT, 
 // Stable scatter of the records into the child segments, and the segment table of the next level.  Same grid as k_part_count.
 static __global__ void __launch_bounds__(PART_THREADS, 2048 / PART_THREADS)
 k_part_scatter(int level, const Batch b, int tree0) {
+    chain_wait();
     constexpr int WORDS = PART_TILE / 32;
     extern __shared__ int s_tile[];   // [nl + 1], then records before every node [nl]
     __shared__ int wpre[WORDS], wtot[(WORDS + 31) / 32], scratch[33];

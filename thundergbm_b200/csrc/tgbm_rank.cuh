@@ -52,9 +52,10 @@ __device__ inline float disc_gain(int label, int rank, const float *__restrict__
 
 // LambdaRank::get_gradient for one query group per CTA
 static __global__ void __launch_bounds__(256)
-k_lambdarank(const int *__restrict__ gptr, const float *__restrict__ y, const float *__restrict__ yp, const float *__restrict__ idcg,
-             const float *__restrict__ log2tab, int ndcg, uint32_t seed, const RoundState *__restrict__ rs, uint32_t group_offset,
-             float2 *__restrict__ gh, unsigned *__restrict__ maxbits) {
+k_lambdarank(const int *__restrict__ gptr, const float *__restrict__ y, const float *yp, const float *__restrict__ idcg,
+             const float *__restrict__ log2tab, int ndcg, uint32_t seed, const RoundState *rs, uint32_t group_offset,
+             float2 *gh, unsigned *maxbits) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char sm[];
     const uint32_t round = (uint32_t)rs->round;  // read on the device: the launch is the same every round
     const int k = blockIdx.x;
@@ -131,8 +132,9 @@ k_lambdarank(const int *__restrict__ gptr, const float *__restrict__ y, const fl
 // NDCG / MAP of one query group per CTA (src/thundergbm/metric/rank_metric.cpp:42-100):
 // documents ordered by score descending (ties by row), sequential sums in rank order
 static __global__ void __launch_bounds__(256)
-k_rank_metric(const int *__restrict__ gptr, const float *__restrict__ y, const float *__restrict__ yp, const float *__restrict__ idcg,
-              const float *__restrict__ log2tab, int ndcg, float *__restrict__ group_score) {
+k_rank_metric(const int *__restrict__ gptr, const float *__restrict__ y, const float *yp, const float *__restrict__ idcg,
+              const float *__restrict__ log2tab, int ndcg, float *group_score) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char sm[];
     const int k = blockIdx.x;
     const int s0 = gptr[k], len = gptr[k + 1] - s0;
@@ -144,27 +146,47 @@ k_rank_metric(const int *__restrict__ gptr, const float *__restrict__ y, const f
     for (int i = threadIdx.x; i < len; i += blockDim.x) { key[i] = desc_key(yp[s0 + i]); idx[i] = i; }
     __syncthreads();
     block_bitonic(key, idx, len, P);
+    // the terms by all threads (a chain of dependent global reads in one thread took 60 us for 120 documents), added in rank
+    // order by one
+    float *term = reinterpret_cast<float *>(key);
+    __syncthreads();
+    for (int i = threadIdx.x; i < len; i += blockDim.x) {
+        const float label = y[s0 + idx[i]];
+        term[i] = ndcg ? disc_gain((int)label, i, log2tab) : label;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         if (ndcg) {
             float dcg = 0.f;
-            for (int i = 0; i < len; ++i) dcg = __fadd_rn(dcg, disc_gain((int)y[s0 + idx[i]], i, log2tab));
+            for (int i = 0; i < len; ++i) dcg = __fadd_rn(dcg, term[i]);
             group_score[k] = __fdiv_rn(dcg, idcg[k]);
         } else {
             int nh = 0;
             double ap = 0;
             for (int i = 0; i < len; ++i)
-                if (y[s0 + idx[i]] != 0.f) { nh++; ap += (double)nh / (i + 1); }
+                if (term[i] != 0.f) { nh++; ap += (double)nh / (i + 1); }
             group_score[k] = nh ? (float)(ap / nh) : 1.f;
         }
     }
 }
 
-static __global__ void k_rank_metric_sum(const float *__restrict__ group_score, int n_group, double *__restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0;
-        for (int i = 0; i < n_group; ++i) s += (double)group_score[i];
-        *out = s;
-    }
+// sum of the group scores, in a fixed order (thread t adds the scores t, t + 1024, ...; then a fixed tree): one thread
+// adding 2500 scores one by one took 65 us
+static __global__ void __launch_bounds__(1024)
+k_rank_metric_sum(const float *group_score, int n_group, double *out) {
+    chain_wait();
+    __shared__ double part[32];
+    double s = 0;
+    for (int i = threadIdx.x; i < n_group; i += 1024) s += (double)group_score[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    s = part[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) *out = s;
 }
 static __global__ void k_rank_metric_final(const double *__restrict__ sum, long long n_group_total, float *__restrict__ out) {
     if (threadIdx.x == 0 && blockIdx.x == 0) *out = (float)(*sum / (double)n_group_total);
@@ -230,16 +252,15 @@ struct RankState {
 
     void gradient(const RoundState *rs, uint32_t seed, const float *yp, float2 *gh, unsigned *maxbits, cudaStream_t stream) {
         if (!n_group) return;
-        TGBM_CUDA(cudaMemsetAsync(gh, 0, sizeof(float2) * (size_t)N, stream));
         const int P = pow2_len();
-        k_lambdarank<<<n_group, 256, 40 * (size_t)P, stream>>>(gptr.p, y.p, yp, idcg.p, log2tab.p, idcg_used, seed, rs,
+        launch_after(k_lambdarank, n_group, 256, 40 * (size_t)P, stream, gptr.p, y.p, yp, idcg.p, log2tab.p, idcg_used, seed, rs,
                                                              group_offset, gh, maxbits);
     }
     // `out` null: the sum of the group scores stays in `sum` (the caller finishes the metric)
     void metric(int objective, const float *yp, float *out, const Comm *comm, long long, cudaStream_t stream) {
         const int P = pow2_len();
-        if (n_group) k_rank_metric<<<n_group, 256, 12 * (size_t)P, stream>>>(gptr.p, y.p, yp, idcg.p, log2tab.p, objective == RANK_NDCG, group_score.p);
-        k_rank_metric_sum<<<1, 32, 0, stream>>>(group_score.p, n_group, sum.p);
+        if (n_group) launch_after(k_rank_metric, n_group, 256, 12 * (size_t)P, stream, gptr.p, y.p, yp, idcg.p, log2tab.p, objective == RANK_NDCG, group_score.p);
+        launch_after(k_rank_metric_sum, 1, 1024, 0, stream, group_score.p, n_group, sum.p);
         if (comm && comm->active()) comm->allreduce(sum.p, 1, Comm::F64, Comm::SUM, stream);
         if (out) k_rank_metric_final<<<1, 32, 0, stream>>>(sum.p, n_group_total, out);
     }
