@@ -848,6 +848,7 @@ void Booster::init(const DataSet &ds) {
         for (int f = 0; f < std::min(m.F, 256); ++f) m.f32_cuts.v[f] = m.h_cut_ptr[f];
         m.spread_cells = std::max<size_t>(std::min<size_t>((size_t)32 * max_pairs * B1, (size_t)8 << 20), (size_t)max_pairs * B1);  // <= 64 MB
         m.hist_spread.alloc(m.spread_cells);
+        m.hist_spread.zero(m.stream);
         m.sum_partial.alloc((size_t)SUM_BLOCKS * K * 2);
         const QuantInfo one{1.0, 1.0, 1.0, 1.0};
         TGBM_CUDA(cudaMemcpyAsync(m.qinfo.p, &one, sizeof(one), cudaMemcpyHostToDevice, m.stream));
@@ -982,7 +983,8 @@ void BoosterImpl::plan_small_trees() {
         pl.bins = 1;
         for (int f = 0; f < F; f += pl.feats) pl.bins = std::max(pl.bins, h_cut_ptr[std::min(F, f + pl.feats)] - h_cut_ptr[f]);
         if ((double)N * pl.feats > 8e4 || (double)max_nl * pl.feats > 512) return;
-        const size_t budget = 200 * 1024, fixed = (sizeof(TreeNode) * (size_t)n_nodes + 15) / 16 * 16 + sizeof(SmallPost) * 2 * max_nl + (size_t)(N + 7) / 8 * 16;
+        const size_t budget = 200 * 1024, fixed = (sizeof(TreeNode) * (size_t)n_nodes + 15) / 16 * 16 + sizeof(SmallPost) * 2 * max_nl + (size_t)(N + 7) / 8 * 16 +
+                     4 * (size_t)((max_nl + 3) / 4 * 4) + 64;   // (64: roundings)
         const size_t per_node = 16 * (size_t)pl.bins + sizeof(SplitRec) * pl.feats;
         if (fixed + per_node > budget) return;
         pl.nodes_pass = (int)std::min<size_t>(max_nl, (budget - fixed) / per_node);
@@ -1074,7 +1076,8 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
             const int bs = f32_stride(pairs), ctas = num_sms * (2048 / F32_THREADS);
             for (int t = 0; t < n_trees; ++t) {
                 float2 *compact = reinterpret_cast<float2 *>(hist_built.p + t * b.built_stride), *cells = bs != 1 ? hist_spread.p : compact;
-                if (bs != 1) TGBM_CUDA(cudaMemsetAsync(cells, 0, sizeof(float2) * (size_t)B * pairs * bs, stream));
+                // (the split search leaves the cells it reads zeroed; between ranks it reads the gathered ones)
+                if (bs != 1 && comm && comm->active()) TGBM_CUDA(cudaMemsetAsync(cells, 0, sizeof(float2) * (size_t)B * pairs * bs, stream));
                 timed(level == 0 ? 0 : 1, [&] {
                     if (sparse) {
                         auto kern = level == 0 ? k_hist_sparse_f32<false> : k_hist_sparse_f32<true>;

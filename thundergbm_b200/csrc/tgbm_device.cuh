@@ -31,7 +31,6 @@ void upload_h2d(void *dst, const void *src, size_t bytes, cudaStream_t stream, i
 bool upload_csr_values(float *dst, const float *val, const int *row_ptr, const int *col, int n_rows, int n_cols, cudaStream_t stream, int n_threads);
 // device -> host copy, the same way; the data is there when it returns
 void download_d2h(void *dst, const void *src, size_t bytes, cudaStream_t stream, int n_threads);
-int upload_threads();   // host threads one upload may use: TGBM_UPLOAD_THREADS, else half of the cores, at most 8
 
 // RAII device buffer; everything is allocated once at init and reused for every tree.
 template <typename T>
@@ -137,6 +136,15 @@ __device__ inline int exp_above(float m) {
 }
 
 __device__ inline float q2f(long long v, double inv_scale) { return __double2float_rn((double)v * inv_scale); }
+// The same for many values on one grid.  Rounding the integer and scaling by a power of two gives the float that scaling in
+// double and rounding gives (up to 2^53, beyond it the former rounds once instead of twice), with one conversion instead of
+// two and a double multiply; grids so far out that the scaled float would not be a normal number keep the long way.
+struct GridScale {
+    double inv;
+    float inv_f;   // 0: take the long way
+    __device__ explicit GridScale(double i) : inv(i), inv_f(i > 1e-30 && i < 1e18 ? (float)i : 0.f) {}
+    __device__ __forceinline__ float operator()(long long v) const { return inv_f != 0.f ? __fmul_rn(__ll2float_rn(v), inv_f) : q2f(v, inv); }
+};
 
 __device__ inline long long shfl_ll(long long v, int src) {
     int lo = __shfl_sync(0xffffffffu, (int)(v & 0xffffffffll), src);

@@ -352,6 +352,16 @@ bool staging_on() {
 
 }  // namespace
 
+void host_parallel(int n, const std::function<void(int)> &f) {
+    if (n <= 1) { if (n == 1) f(0); return; }
+    std::vector<std::string> errors(n);
+    pool().run(n, [&](Worker &, int t) {
+        try { f(t); } catch (const std::exception &e) { errors[t] = e.what(); }
+    });
+    for (const auto &e : errors)
+        if (!e.empty()) throw Error(e);
+}
+
 int upload_threads() {
     static const int n = [] {
         if (const char *e = getenv("TGBM_UPLOAD_THREADS")) return std::max(1, std::min(WORKERS, atoi(e)));

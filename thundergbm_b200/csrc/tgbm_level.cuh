@@ -480,6 +480,8 @@ template <> __device__ __forceinline__ double cell_inv<long long>(const QuantInf
 template <> __device__ __forceinline__ double cell_inv<float>(const QuantInfo *, int) { return 1.0; }
 __device__ __forceinline__ float cell_f(long long v, double inv_scale) { return q2f(v, inv_scale); }
 __device__ __forceinline__ float cell_f(float v, double) { return v; }
+__device__ __forceinline__ float cell_f(long long v, const GridScale &s) { return s(v); }
+__device__ __forceinline__ float cell_f(float v, const GridScale &) { return v; }
 __device__ __forceinline__ long long shfl_up_t(long long v, int d) { return shfl_up_ll(v, d); }
 __device__ __forceinline__ float shfl_up_t(float v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
 __device__ __forceinline__ long long shfl_t(long long v, int src) { return shfl_ll(v, src); }
@@ -669,7 +671,7 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
         const TreeNode &nd = nodes[off + (level == 0 ? 0 : 2 * j + c)];
         valid[c] = nd.is_valid; sum_g[c] = nd.sum_g; sum_h[c] = nd.sum_h;
     }
-    const double inv_sg = cell_inv<T>(q, 0), inv_sh = cell_inv<T>(q, 1);
+    const GridScale inv_sg(cell_inv<T>(q, 0)), inv_sh(cell_inv<T>(q, 1));
     T v[4][NB];   // g, h of the left child, g, h of the right one
 #pragma unroll
     for (int n = 0; n < NB; ++n) {
@@ -906,7 +908,7 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
     }
     __syncwarp();
     const float pg = nd.sum_g, ph = nd.sum_h;
-    const double inv_sg = cell_inv<T>(q, 0), inv_sh = cell_inv<T>(q, 1);
+    const GridScale inv_sg(cell_inv<T>(q, 0)), inv_sh(cell_inv<T>(q, 1));
     float best = 0.f, best_lg = 0.f, best_lh = 0.f, best_mg = 0.f, best_mh = 0.f;
     int best_bin = -1;
 #pragma unroll

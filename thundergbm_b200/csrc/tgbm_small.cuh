@@ -9,7 +9,8 @@
 // others through the cluster -- behind one cluster barrier.
 //
 // Bound by the shared-memory atomics of the rows x own features (four 32-bit halves per value, random banks) and by the
-// division chains of the split search.  10000 rows x 32 features, depth 6: 72 us a tree against 185 us.
+// division chains of the split search.  10000 rows x 32 features, depth 6:
+// 130 us a tree against 185 us; 1605 rows x 119 features: 85 us against 165 us.
 // Same integer sums, gains, tie rules and node records as the level kernels, bit for bit.
 #pragma once
 #include <cooperative_groups.h>
@@ -34,7 +35,7 @@ struct SmallPlan {   // sizes fixed by the host (see small_plan in the booster)
 
 // best candidate of one (node, feature): the lanes of a warp own BPL consecutive bins each
 template <int BPL>
-__device__ __forceinline__ void small_eval(const int *cell, int words, int nb, float pg, float ph, double inv_sg, double inv_sh, float mcw,
+__device__ __forceinline__ void small_eval(const int *cell, int words, int nb, float pg, float ph, const GridScale &inv_sg, const GridScale &inv_sh, float mcw,
                                            float lam, int multi, SplitRec *out) {
     const int lane = threadIdx.x & 31;
     long long g[BPL], h[BPL], tg = 0, th = 0;
@@ -55,7 +56,7 @@ __device__ __forceinline__ void small_eval(const int *cell, int words, int nb, f
         if (lane >= o) { ig += ug; ih += uh; }
     }
     const long long all_g = shfl_ll(ig, 31), all_h = shfl_ll(ih, 31);
-    const float mg = __fsub_rn(pg, q2f(all_g, inv_sg)), mh = __fsub_rn(ph, q2f(all_h, inv_sh));
+    const float mg = __fsub_rn(pg, inv_sg(all_g)), mh = __fsub_rn(ph, inv_sh(all_h));
     const float parent = __fdiv_rn(__fmul_rn(pg, pg), __fadd_rn(ph, lam));
     long long rg = ig - tg, rh = ih - th;
     unsigned long long key = 0;
@@ -64,7 +65,7 @@ __device__ __forceinline__ void small_eval(const int *cell, int words, int nb, f
     for (int i = 0; i < BPL; ++i) {
         const int b = lane * BPL + i;
         if (multi) { rg += g[i]; rh += h[i]; }
-        const float kg = q2f(rg, inv_sg), kh = q2f(rh, inv_sh);   // see k_eval
+        const float kg = inv_sg(rg), kh = inv_sh(rh);   // see k_eval
         if (!multi) { rg += g[i]; rh += h[i]; }
         const float a = split_gain(parent, pg, ph, kg, kh, mcw, lam), z = split_gain(parent, pg, ph, __fadd_rn(kg, mg), __fadd_rn(kh, mh), mcw, lam);
         const float gl = fmaxf(0.f, multi ? a : z), gr = fmaxf(0.f, multi ? z : a);
@@ -90,7 +91,8 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
     TreeNode *nodes = reinterpret_cast<TreeNode *>(small_sm);
     SmallPost *posts = reinterpret_cast<SmallPost *>(small_sm + (sizeof(TreeNode) * n_nodes + 15) / 16 * 16);   // [2][max_nl]
     SplitRec *recs = reinterpret_cast<SplitRec *>(posts + 2 * max_nl);                                       // [nodes_pass][feats]
-    unsigned short *node_of = reinterpret_cast<unsigned short *>(recs + (size_t)plan.nodes_pass * plan.feats);   // [N, even]
+    unsigned *split = reinterpret_cast<unsigned *>(recs + (plan.nodes_pass * plan.feats + 1) / 2 * 2);   // [max_nl] what the level decided
+    unsigned short *node_of = reinterpret_cast<unsigned short *>(split + (max_nl + 3) / 4 * 4);            // [N, eights]
     int *acc = reinterpret_cast<int *>(node_of + (N + 7) / 8 * 8);                                               // [4][nodes_pass * bins]
     const cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), tree = blockIdx.x / plan.cluster, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -98,7 +100,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
     for (int r = threadIdx.x; r < N; r += SMALL_THREADS) node_of[r] = 0;
     chain_wait();
     const int2 *gq = ghq + (size_t)tree * N;
-    const double inv_sg = q->inv_sg, inv_sh = q->inv_sh;
+    const GridScale inv_sg(q->inv_sg), inv_sh(q->inv_sh);
     const unsigned char *ignored = ignored_all ? ignored_all + (size_t)rs->round * F : nullptr;
     for (int i = threadIdx.x; i < n_nodes; i += SMALL_THREADS) {   // Tree::init2, as k_tree_init
         TreeNode t;
@@ -109,8 +111,8 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
         if (i < n_nodes / 2) { t.is_leaf = 0; t.lch_index = 2 * i + 1; t.rch_index = 2 * i + 2; }
         else { t.is_leaf = 1; t.lch_index = -1; t.rch_index = -1; }
         if (i == 0) {
-            t.sum_g = q2f((long long)root_sum[2 * tree], inv_sg);
-            t.sum_h = q2f((long long)root_sum[2 * tree + 1], inv_sh);
+            t.sum_g = inv_sg((long long)root_sum[2 * tree]);
+            t.sum_h = inv_sh((long long)root_sum[2 * tree + 1]);
             t.is_valid = 1;
             t.base_weight = __fdiv_rn(-t.sum_g, __fadd_rn(t.sum_h, lam));
         }
@@ -134,20 +136,20 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
                     const int r = r0 + u * SMALL_THREADS;
                     n[u] = r < N ? (int)node_of[r] - n0 : -1;
                     if ((unsigned)n[u] >= (unsigned)here) n[u] = -1;
-                    else v[u] = gq[r];
+                    v[u] = r < N ? gq[r] : make_int2(0, 0);   // (does not wait for the node)
                 }
                 for (int f = 0; f < nf; ++f) {
                     const unsigned char *col = binsT + (size_t)(f0 + f) * Npad;
                     const int first = cut_ptr[f0 + f] - bin0;
                     int b[U];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) b[u] = n[u] >= 0 ? col[r0 + u * SMALL_THREADS] : MISSING_BIN;
+                    for (int u = 0; u < U; ++u) b[u] = r0 + u * SMALL_THREADS < N ? col[r0 + u * SMALL_THREADS] : MISSING_BIN;
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
-                        if (b[u] == MISSING_BIN) continue;
+                        if (b[u] == MISSING_BIN || n[u] < 0) continue;
                         int *cell = acc + n[u] * plan.bins + first + b[u];
                         atomicAdd(reinterpret_cast<unsigned *>(cell), (unsigned)v[u].x & 0xffffu);
-                        atomicAdd(reinterpret_cast<unsigned *>(cell + words), (unsigned)v[u].y & 0xffffu);
+                        if (v[u].y & 0xffff) atomicAdd(reinterpret_cast<unsigned *>(cell + words), (unsigned)v[u].y & 0xffffu);   // (a hessian of 1 has no low half)
                         atomicAdd(cell + 2 * words, v[u].x >> 16);
                         atomicAdd(cell + 3 * words, v[u].y >> 16);
                     }
@@ -190,46 +192,57 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
         }
         if (threadIdx.x == 0) s_split = 0;
         cluster.sync();   // every CTA's candidates are in place (and its reads of the level before are done)
-        for (int n = threadIdx.x; n < nl; n += SMALL_THREADS) {
-            if (!nodes[off + n].is_valid) continue;
-            unsigned long long best = 0;
-            int from = 0;
-            for (int c = 0; c < plan.cluster; ++c) {
-                const unsigned long long k = cluster.map_shared_rank(post, c)[n].key;
-                if (k > best) { best = k; from = c; }
+        // sixteen lanes per node: each reads one CTA's candidate
+        for (int base = (int)(threadIdx.x & ~31u); base < nl * 16; base += SMALL_THREADS) {
+            const int n = (base + lane) >> 4, c = lane & 15;
+            const bool valid = n < nl && nodes[off + n].is_valid;
+            unsigned long long best = valid && c < plan.cluster ? cluster.map_shared_rank(post, c)[n].key : 0;
+            int from = c;
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) {
+                const unsigned long long other = (unsigned long long)shfl_xor_ll((long long)best, o);
+                const int f = __shfl_xor_sync(0xffffffffu, from, o);
+                if (other > best) { best = other; from = f; }
             }
-            if (best == 0) {   // no feature has a cut point: nothing to split on
-                nodes[off + n].is_leaf = 1;
-                continue;
+            if (c == 0 && n < nl) {
+                split[n] = 0;
+                if (valid) {
+                    TreeNode &nd = nodes[off + n];
+                    if (best == 0) nd.is_leaf = 1;   // no feature has a cut point: nothing to split on
+                    else {
+                        const SplitRec r = cluster.map_shared_rank(post, from)[n].rec;
+                        apply_split(nodes, off + n, 0x7fffffff - (int)(unsigned)(best & 0xffffffffull), r, cut_ptr, cut_val, rt_eps, lam, multi);
+                    }
+                    if (!nd.is_leaf) {
+                        s_split = 1;
+                        split[n] = 0x80000000u | (nd.default_right ? 0x40000000u : 0u) | ((unsigned)nd.split_feature_id << 8) | nd.split_bid;
+                    }
+                }
             }
-            const SplitRec r = cluster.map_shared_rank(post, from)[n].rec;
-            apply_split(nodes, off + n, 0x7fffffff - (int)(unsigned)(best & 0xffffffffull), r, cut_ptr, cut_val, rt_eps, lam, multi);
-            if (!nodes[off + n].is_leaf) s_split = 1;
+            __syncwarp();
         }
         __syncthreads();
         if (!s_split || level == depth - 1) break;   // the same in every CTA
         // -- rows to the children
-        for (int r0 = threadIdx.x; r0 < N; r0 += 4 * SMALL_THREADS) {
-            int n[4], b[4];
+        // (every CTA for itself: moving a share each and storing it into all sixteen copies took twice the time)
+        constexpr int R = 8;   // rows in flight per thread
+        for (int r0 = threadIdx.x; r0 < N; r0 += R * SMALL_THREADS) {
+            int n[R];
+            unsigned sp[R];
+            unsigned char b[R];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < R; ++u) {
                 const int r = r0 + u * SMALL_THREADS;
                 n[u] = r < N ? (int)node_of[r] : (int)SMALL_NONE;
-                b[u] = 0;
-                if (n[u] != SMALL_NONE) {
-                    const TreeNode &nd = nodes[off + n[u]];
-                    if (!nd.is_valid || nd.is_leaf) { n[u] = -1; continue; }
-                    b[u] = binsT[(size_t)nd.split_feature_id * Npad + r];
-                }
+                sp[u] = n[u] != SMALL_NONE ? split[n[u]] : 0u;
+                b[u] = sp[u] ? binsT[(size_t)((sp[u] >> 8) & 0x3fffffu) * Npad + r] : (unsigned char)0;
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int r = r0 + u * SMALL_THREADS;
+            for (int u = 0; u < R; ++u) {
                 if (n[u] == SMALL_NONE) continue;
-                if (n[u] < 0) { node_of[r] = SMALL_NONE; continue; }
-                const TreeNode &nd = nodes[off + n[u]];
-                const bool left = b[u] == MISSING_BIN ? !nd.default_right : (multi ? b[u] > nd.split_bid : b[u] < nd.split_bid);
-                node_of[r] = (unsigned short)(2 * n[u] + (left ? 0 : 1));
+                const unsigned char bid = (unsigned char)sp[u];
+                const bool left = b[u] == MISSING_BIN ? !(sp[u] & 0x40000000u) : (multi ? b[u] > bid : b[u] < bid);
+                node_of[r0 + u * SMALL_THREADS] = sp[u] ? (unsigned short)(2 * n[u] + (left ? 0 : 1)) : SMALL_NONE;
             }
         }
         __syncthreads();
