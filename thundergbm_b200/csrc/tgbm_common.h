@@ -155,7 +155,7 @@ struct DataSet {
 
 // f(0) ... f(n - 1) on the library's standing worker threads (tgbm_devmem.cu); returns when all have returned
 void host_parallel(int n, const std::function<void(int)> &f);
-int upload_threads();   // how many of them one call should use: TGBM_UPLOAD_THREADS, else half of the cores, at most 8
+int upload_threads();   // how many of them one call should use: TGBM_UPLOAD_THREADS, else all cores but one, at most 15
 long long count_distinct(const float *v, long long n);   // every NaN counts, +0 and -0 are one value
 
 // logging (verbosity as in set_logger: 0 silent, 1 info, 2 debug)
