@@ -265,6 +265,39 @@ void BoosterImpl::column_builder_candidates(DevBuf<unsigned long long> &ukeys, D
 // Radix sort of (feature, value) keys and DeviceSelect::Unique come from CUB; this runs once, before
 // the boosting loop.  With several ranks every rank contributes its sorted distinct keys, all ranks merge the lists and
 // derive identical cut points from the union, so the bins equal the single-GPU ones.
+// A matrix without missing values is sorted column by column from BY_COLUMN_ROWS rows on: below, the launches of one sort
+// per column cost more than the shorter keys save.  28 columns of 1.05 / 2.1 / 10.5 M rows: 1.9 / 2.8 / 9.1 ms, as one sort
+// of 64-bit keys 1.7 / 3.4 / 16.6 ms.
+constexpr int BY_COLUMN_ROWS = 1 << 21;
+constexpr int SORT_LANES = 4;   // columns sorted side by side
+
+// streams that start after what `main` holds now; join() makes `main` wait for them
+struct SideStreams {
+    std::vector<cudaStream_t> st;
+    cudaStream_t main;
+    cudaEvent_t ev = nullptr;
+    SideStreams(cudaStream_t m, int n) : main(m) {
+        TGBM_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        TGBM_CUDA(cudaEventRecord(ev, main));
+        for (int i = 0; i < n; ++i) {
+            cudaStream_t s = nullptr;
+            TGBM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+            st.push_back(s);
+            TGBM_CUDA(cudaStreamWaitEvent(s, ev, 0));
+        }
+    }
+    void join() {
+        for (cudaStream_t s : st) {
+            TGBM_CUDA(cudaEventRecord(ev, s));
+            TGBM_CUDA(cudaStreamWaitEvent(main, ev, 0));
+        }
+    }
+    ~SideStreams() {
+        for (cudaStream_t s : st) { cudaStreamSynchronize(s); cudaStreamDestroy(s); }
+        if (ev) cudaEventDestroy(ev);
+    }
+};
+
 void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
     const bool timing = getenv("TGBM_TIMING") != nullptr;  // phase times of the set-up on stderr
     auto t_prev = std::chrono::steady_clock::now();
@@ -288,7 +321,58 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
     };
     const bool colb = p.column_shards > 0;   // the column-sharded builder's cut points need the multiplicity of every key
     DevBuf<long long> ucopies;
-    {
+    std::vector<int> h_stride(F);
+    h_cut_ptr.assign(F + 1, 0);
+    DevBuf<int> d_stride;
+    // strides and numbers of cut points from the number of distinct values of every feature
+    auto lay_out_cuts = [&](auto &&distinct) {
+        for (int f = 0; f < F; ++f) {
+            const long long u = distinct(f), st = u / p.max_num_bin;
+            h_stride[f] = (int)st;
+            h_cut_ptr[f + 1] = h_cut_ptr[f] + (int)(st == 0 ? u : p.max_num_bin);
+        }
+        B = h_cut_ptr[F];
+        d_stride.alloc(std::max(F, 1));
+        cut_ptr.alloc(F + 1); cut_val.alloc(std::max(B, 1)); cut_fid.alloc(std::max(B, 1));
+        TGBM_CUDA(cudaMemcpyAsync(d_stride.p, h_stride.data(), sizeof(int) * F, cudaMemcpyHostToDevice, stream));
+        TGBM_CUDA(cudaMemcpyAsync(cut_ptr.p, h_cut_ptr.data(), sizeof(int) * (F + 1), cudaMemcpyHostToDevice, stream));
+    };
+    const bool by_column = in.full_cols > 0 && in.full_cols == F && !multi && !colb && N >= BY_COLUMN_ROWS;
+    if (by_column) {
+        const int chunks = ceil_div(N, COL_CHUNK);
+        DevBuf<unsigned> a, c;
+        DevBuf<int> heads, distinct;
+        a.alloc(nnz); c.alloc(nnz); heads.alloc((size_t)chunks * F); distinct.alloc(F);
+        k_order_columns<<<dim3(ceil_div(N, 64), ceil_div(F, 32)), 256, 0, stream>>>(in.val.p, N, F, a.p);
+        size_t tb = 0;
+        cub::DoubleBuffer<unsigned> keys(a.p, c.p);
+        TGBM_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb, keys, N, 0, 32, stream));
+        tb = (std::max<size_t>(tb, 16) + 255) / 256 * 256;
+        DevBuf<unsigned char> tmp;
+        tmp.alloc(tb * SORT_LANES);
+        int side = 0;
+        {
+            SideStreams lanes(stream, std::min(F, SORT_LANES));
+            for (int f = 0; f < F; ++f) {
+                const int q = f % SORT_LANES;
+                keys = cub::DoubleBuffer<unsigned>(a.p + (size_t)f * N, c.p + (size_t)f * N);
+                TGBM_CUDA(cub::DeviceRadixSort::SortKeys(tmp.p + q * tb, tb, keys, N, 0, 32, lanes.st[q]));
+                TGBM_CHECK(f == 0 || keys.selector == side, "sorted columns in different buffers");
+                side = keys.selector;
+            }
+            lanes.join();
+        }
+        const unsigned *sorted = side ? c.p : a.p;
+        k_column_heads<<<dim3(chunks, F), 256, 0, stream>>>(sorted, N, heads.p);
+        k_column_prefix<<<F, 1024, 0, stream>>>(heads.p, chunks, distinct.p);
+        std::vector<int> h_distinct(F);
+        TGBM_CUDA(cudaMemcpyAsync(h_distinct.data(), distinct.p, sizeof(int) * F, cudaMemcpyDeviceToHost, stream));
+        TGBM_CUDA(cudaStreamSynchronize(stream));
+        lap("columns sorted");
+        lay_out_cuts([&](int f) { return (long long)h_distinct[f]; });
+        k_column_cuts<<<dim3(chunks, F), 256, 0, stream>>>(sorted, N, heads.p, d_stride.p, cut_ptr.p, p.max_num_bin, cut_val.p, cut_fid.p);
+        TGBM_CUDA(cudaStreamSynchronize(stream));
+    } else {
         DevBuf<unsigned long long> keys, keys2;
         DevBuf<long long> copies, copies2;
         DevBuf<long long> d_nu;
@@ -431,31 +515,21 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
         }
         TGBM_CUDA(cudaStreamSynchronize(stream));
     }
-    if (colb) column_builder_candidates(ukeys, ucopies, nu);
-    lap("sort + unique of the keys");
-    // distinct values per feature -> stride and number of cut points per feature (host, F+1 numbers)
-    DevBuf<long long> ustart;
-    ustart.alloc(F + 1);
-    k_feature_bounds<<<ceil_div(F + 1, 128), 128, 0, stream>>>(ukeys.p, nu, F, ustart.p);
-    std::vector<long long> h_ustart(F + 1);
-    TGBM_CUDA(cudaMemcpyAsync(h_ustart.data(), ustart.p, sizeof(long long) * (F + 1), cudaMemcpyDeviceToHost, stream));
-    TGBM_CUDA(cudaStreamSynchronize(stream));
-    std::vector<int> h_stride(F);
-    h_cut_ptr.assign(F + 1, 0);
-    for (int f = 0; f < F; ++f) {
-        const long long u = h_ustart[f + 1] - h_ustart[f];
-        const long long s = u / p.max_num_bin;
-        h_stride[f] = (int)s;
-        h_cut_ptr[f + 1] = h_cut_ptr[f] + (int)(s == 0 ? u : p.max_num_bin);
+    if (!by_column) {
+        if (colb) column_builder_candidates(ukeys, ucopies, nu);
+        lap("sort + unique of the keys");
+        // distinct values per feature -> stride and number of cut points per feature (host, F+1 numbers)
+        DevBuf<long long> ustart;
+        ustart.alloc(F + 1);
+        k_feature_bounds<<<ceil_div(F + 1, 128), 128, 0, stream>>>(ukeys.p, nu, F, ustart.p);
+        std::vector<long long> h_ustart(F + 1);
+        TGBM_CUDA(cudaMemcpyAsync(h_ustart.data(), ustart.p, sizeof(long long) * (F + 1), cudaMemcpyDeviceToHost, stream));
+        TGBM_CUDA(cudaStreamSynchronize(stream));
+        lay_out_cuts([&](int f) { return h_ustart[f + 1] - h_ustart[f]; });
+        if (nu) k_select_cuts<<<std::min(ceil_div(nu, 256), num_sms * 16), 256, 0, stream>>>(ukeys.p, nu, ustart.p, d_stride.p, cut_ptr.p,
+                                                                                             p.max_num_bin, cut_val.p, cut_fid.p, colb ? 1 : 0);
+        TGBM_CUDA(cudaStreamSynchronize(stream));   // the list of start positions goes
     }
-    B = h_cut_ptr[F];
-    DevBuf<int> d_stride;
-    d_stride.alloc(std::max(F, 1));
-    cut_ptr.alloc(F + 1); cut_val.alloc(std::max(B, 1)); cut_fid.alloc(std::max(B, 1));
-    TGBM_CUDA(cudaMemcpyAsync(d_stride.p, h_stride.data(), sizeof(int) * F, cudaMemcpyHostToDevice, stream));
-    TGBM_CUDA(cudaMemcpyAsync(cut_ptr.p, h_cut_ptr.data(), sizeof(int) * (F + 1), cudaMemcpyHostToDevice, stream));
-    if (nu) k_select_cuts<<<std::min(ceil_div(nu, 256), num_sms * 16), 256, 0, stream>>>(ukeys.p, nu, ustart.p, d_stride.p, cut_ptr.p,
-                                                                                         p.max_num_bin, cut_val.p, cut_fid.p, colb ? 1 : 0);
     h_cut_val.resize(B);
     TGBM_CUDA(cudaMemcpyAsync(h_cut_val.data(), cut_val.p, sizeof(float) * B, cudaMemcpyDeviceToHost, stream));
 

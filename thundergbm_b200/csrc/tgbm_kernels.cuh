@@ -480,6 +480,89 @@ __device__ inline int block_scan_excl(int n, In in, Out out, int *scratch) {
     return carry;
 }
 
+// ------------------------------------------------------------------ cut points of a matrix without missing values
+// Every column is sorted for itself: 32-bit keys instead of 64-bit ones that carry the column, and four passes over them
+// instead of five; distinct values are then counted and picked where they lie instead of being compacted first.
+constexpr int COL_CHUNK = 4096;   // sorted keys per block
+
+// values [n][c] -> order-preserving images by column [c][n]; a block transposes 64 rows of 32 columns
+static __global__ void __launch_bounds__(256)
+k_order_columns(const float *__restrict__ val, int n, int c, unsigned *__restrict__ out) {
+    __shared__ unsigned t[64][33];
+    const int r0 = blockIdx.x * 64, c0 = blockIdx.y * 32;
+    for (int i = threadIdx.x; i < 64 * 32; i += 256) {
+        const int r = r0 + (i >> 5), f = c0 + (i & 31);
+        if (r < n && f < c) {
+            unsigned u = __float_as_uint(val[(size_t)r * c + f]);
+            if (u == 0x80000000u) u = 0;  // -0.0f == 0.0f
+            t[i >> 5][i & 31] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 64 * 32; i += 256) {
+        const int r = r0 + (i & 63), f = c0 + (i >> 6);
+        if (r < n && f < c) out[(size_t)f * n + r] = t[i & 63][i >> 6];
+    }
+}
+
+// distinct values that start in every chunk of a sorted column; grid = (chunks, columns)
+static __global__ void __launch_bounds__(256)
+k_column_heads(const unsigned *__restrict__ keys, int n, int *__restrict__ heads) {
+    const unsigned *k = keys + (size_t)blockIdx.y * n;
+    int cnt = 0;
+    for (int u = 0; u < COL_CHUNK / 256; ++u) {
+        const int i = blockIdx.x * COL_CHUNK + u * 256 + threadIdx.x;
+        cnt += i < n && (i == 0 || k[i] != k[i - 1]);
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    __shared__ int w[8];
+    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = cnt;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int t = 0;
+        for (int i = 0; i < 8; ++i) t += w[i];
+        heads[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
+    }
+}
+
+// exclusive prefix over the chunks of a column in place, and its number of distinct values; one block of 1024 threads each
+static __global__ void __launch_bounds__(1024)
+k_column_prefix(int *__restrict__ heads, int chunks, int *__restrict__ distinct) {
+    __shared__ int scratch[33];
+    int *h = heads + (size_t)blockIdx.x * chunks;
+    const int total = block_scan_excl(chunks, [&](int i) { return h[i]; }, [&](int i, int before) { h[i] = before; }, scratch);
+    if (threadIdx.x == 0) distinct[blockIdx.x] = total;
+}
+
+// k_select_cuts on the sorted columns; grid as in k_column_heads
+static __global__ void __launch_bounds__(256)
+k_column_cuts(const unsigned *__restrict__ keys, int n, const int *__restrict__ before, const int *__restrict__ stride,
+              const int *__restrict__ cut_ptr, int max_bin, float *__restrict__ cut_val, int *__restrict__ cut_fid) {
+    const unsigned *k = keys + (size_t)blockIdx.y * n;
+    const int f = blockIdx.y, s = stride[f], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int rank0 = before[(size_t)f * gridDim.x + blockIdx.x];
+    __shared__ int w[8];
+    for (int u = 0; u < COL_CHUNK / 256; ++u) {
+        const int i = blockIdx.x * COL_CHUNK + u * 256 + threadIdx.x;
+        const unsigned key = i < n ? k[i] : 0u;
+        const bool head = i < n && (i == 0 || key != k[i - 1]);
+        const unsigned m = __ballot_sync(0xffffffffu, head);
+        __syncthreads();
+        if (lane == 0) w[warp] = __popc(m);
+        __syncthreads();
+        int t = rank0 + __popc(m & ((1u << lane) - 1u)), all = 0;
+        for (int q = 0; q < 8; ++q) { if (q < warp) t += w[q]; all += w[q]; }
+        if (head) {
+            const int pos = s == 0 ? t : (t % s == 0 && t / s < max_bin ? t / s : -1);
+            if (pos >= 0) {
+                cut_val[cut_ptr[f] + pos] = key_to_float((unsigned long long)key);
+                cut_fid[cut_ptr[f] + pos] = f;
+            }
+        }
+        rank0 += all;
+    }
+}
+
 // ------------------------------------------------------------------ end of tree
 // Tree::prune_self / try_prune_leaf / reorder_nid (src/thundergbm/tree.cu:85-128).  The reference walks the
 // leaves in index order and climbs while a parent has two leaf children and gain < gamma; the fixed point of that
