@@ -104,7 +104,7 @@ struct BoosterImpl {
     int part_ctas = 1;
     bool grad_max_ready = false;        // maxbits holds the maxima of the next round's gradients
     bool metric_partial_ready = false;  // metric_partial holds the finished round's partial sums
-    int metric_blocks() const { return std::max(1, std::min((N + 255) / 256, 1024)); }
+    int metric_blocks() const { return std::max(1, std::min((N + 255) / 256, std::min(num_sms * 8, METRIC_PARTS))); }   // of 256 threads: one full wave
     DevBuf<SplitRec> recs;
     DevBuf<int> tile_left, tail_left;
     DevBuf<unsigned> bits;
@@ -932,7 +932,7 @@ void Booster::init(const DataSet &ds) {
     m.rstate.zero(m.stream);
     m.graphs_allowed = getenv("TGBM_NO_GRAPH") == nullptr;
     m.f32_staged = getenv("TGBM_NO_BULK_COPY") == nullptr;
-    m.metric_partial.alloc(1024); m.metric_sum.alloc(1);
+    m.metric_partial.alloc(m.metric_blocks()); m.metric_sum.alloc(1);
     m.window_rows = (1 << (31 - p.quant_bits)) - HIST_THREADS;
     TGBM_CHECK(m.window_rows >= HIST_THREADS, "quant_bits too large for the int32 accumulation window");
     const int table = 4 * (max_pairs + 1);   // tiles before every pair of the deepest level
@@ -940,9 +940,9 @@ void Booster::init(const DataSet &ds) {
     TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_EXACT_SMEM + table));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
-    TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+    TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM));
+    TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM));
+    TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
     m.prune_in_smem = sizeof(TreeNode) * (size_t)m.n_nodes <= 200 * 1024;  // up to depth 11
@@ -1203,9 +1203,9 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
     if (!one_launch) launch_after(k_prune, n_trees, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream, nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0,
                                                                                               model.p, K, k0, rstate.p);
     if (N) {
-        const size_t per_node = sizeof(WalkNode) + (sparse ? sizeof(WalkSpan) : 0);
-        const int in_smem = per_node * (size_t)n_nodes <= 160 * 1024;
-        const size_t walk_smem = in_smem ? per_node * (size_t)n_nodes : 0;
+        const size_t walk_table = (sizeof(WalkNode) + sizeof(float) + (sparse ? sizeof(WalkSpan) : 0)) * (size_t)n_nodes + sizeof(float);
+        const int in_smem = walk_table <= WALK_SMEM;
+        const size_t walk_smem = in_smem ? walk_table : 0;
         float *yp = ypred.p + (size_t)k0 * N;
         int *nid_out = p.keep_nid ? nid_keep.p + ((size_t)round * K + k0) * N : nullptr;
         // One tree per round and a pointwise objective: the walk also adds up the round's metric and finds the maxima

@@ -25,6 +25,7 @@ constexpr int PART_THREADS = 512;  // 512 x 4 records per tile measured best (10
 constexpr int PART_RPT = 4;         // records per thread
 constexpr int PART_TILE = PART_THREADS * PART_RPT;
 constexpr int MISSING_BIN = 255;
+constexpr int METRIC_PARTS = 1280;  // most partial sums of a round's metric (148 SMs x 8 blocks use 1184)
 constexpr int FINE_BITS = 30;          // value bits of the grid of fp32 mode's later rounds
 constexpr int FINE_WINDOW = 1 << 16;   // rows whose 16-bit low halves fit an unsigned accumulator
 constexpr int FINE_FROM_ROUND = 1;     // fp32 mode: rounds before it sum floats value by value (k_hist_f32)
@@ -618,32 +619,40 @@ k_prune(TreeNode *nodes, int n_nodes, int depth, float gamma, int table_in_smem,
 // A node was split iff its children are valid; pruning only marks nodes, so the walk goes on below a pruned
 // parent to find the node the reference's table would hold (`nid_out`) while the score takes the weight of the
 // deepest node on the path that survived pruning.
-// Walk table entry: flags = split bin (bits 0-7) | default right (8) | was split (9) | pruned (10) |
-// bins count down, i.e. left means bin > split bin (11; the column-sharded builder's rule, hist_tree_builder.cu:455-459) | feature << 16
-struct WalkNode { int flags; float weight; };
+//
+// Table entry: test = feature << 16 | feature bits 3-4 at 14 | shift << 13 | threshold << 4 | feature bits 0-2,
+// left = table offset of the left child in bytes; the right child follows it.
+// A row goes left iff x = (bin + shift) mod 256 is below the threshold (not below, where bins count down: `rev`, the
+// column-sharded builder's rule, left means bin > split bin, hist_tree_builder.cu:455-459).  The missing value's bin 255
+// thereby takes the default direction without a test of its own: unshifted it lies above every bin, shifted below.  A node
+// that was not split sends every row left, to itself, so that all rows take the same number of steps.
+struct WalkNode { unsigned test; unsigned left; };
 struct WalkSpan { int c0, c1; };  // CSR layout: global bins [c0, c1) of the split feature
 
+__device__ __forceinline__ bool walk_split(const TreeNode *nodes, const TreeNode &nd) { return nd.is_valid && nd.lch_index >= 0 && nodes[nd.lch_index].is_valid; }
 __device__ __forceinline__ WalkNode walk_node(const TreeNode *nodes, int i, int rev) {
     const TreeNode nd = nodes[i];
-    const bool split = nd.is_valid && nd.lch_index >= 0 && nodes[nd.lch_index].is_valid;
-    WalkNode w;
-    w.flags = (int)nd.split_bid | (nd.default_right ? 0x100 : 0) | (split ? 0x200 : 0) | (nd.is_pruned ? 0x400 : 0) | (rev ? 0x800 : 0) |
-              (split ? (int)((unsigned)nd.split_feature_id << 16) : 0);
-    w.weight = nd.base_weight;
-    return w;
+    if (!walk_split(nodes, nd)) return WalkNode{rev ? 0u : 256u << 4, (unsigned)(i * sizeof(WalkNode))};
+    const unsigned f = (unsigned)nd.split_feature_id, shift = rev ? (nd.default_right ? 1 : 0) : (nd.default_right ? 0 : 1);
+    const unsigned threshold = (unsigned)nd.split_bid + shift + (rev ? 1 : 0);
+    return WalkNode{(f << 16) | ((f & 24) << 11) | (shift << 13) | (threshold << 4) | (f & 7), (unsigned)((2 * i + 1) * sizeof(WalkNode))};
+}
+__device__ __forceinline__ float walk_weight(const TreeNode *nodes, int i) {   // of the deepest node on the path that survived pruning
+    while (i > 0 && nodes[i].is_pruned) i = (i - 1) >> 1;
+    return nodes[i].base_weight;
 }
 __device__ __forceinline__ WalkSpan walk_span(const TreeNode *nodes, const int *__restrict__ cut_ptr, int i) {
     const TreeNode nd = nodes[i];
-    const bool split = nd.is_valid && nd.lch_index >= 0 && nodes[nd.lch_index].is_valid;
-    const int f = split ? nd.split_feature_id : 0;
+    const int f = walk_split(nodes, nd) ? nd.split_feature_id : 0;
     return WalkSpan{cut_ptr[f], cut_ptr[f + 1]};
 }
 
 // LAYOUT 0: dense rows of exactly 32 bytes, held in registers (two 16-byte loads per row; the byte of the split
-// feature is picked with selects, so that a step costs no memory access); 1: dense rows of any width, one byte load
-// per step; 2: CSR of global bin ids, binary search per step (the feature id does not fit the packed flags there).
-// `table_in_smem` = 0 for trees too large for shared memory (depth 13 and 14): the nodes are then decoded from global
+// feature is picked with six selects and a byte permutation, so that a step costs one shared-memory access); 1: dense rows
+// of any width, one byte load per step; 2: CSR of global bin ids, binary search per step.
+// `table_in_smem` = 0 for trees too large for shared memory (depth 14): the nodes are then decoded from global
 // memory at every step.
+constexpr int WALK_SMEM = 200 * 1024;
 template <int LAYOUT>
 static __global__ void __launch_bounds__(256)
 k_predict_walk(const TreeNode *nodes, int n_nodes, int table_in_smem, const unsigned char *__restrict__ bins, int Fpad,
@@ -663,16 +672,18 @@ k_predict_walk(const TreeNode *nodes, int n_nodes, int table_in_smem, const unsi
     const int fuse_logistic = fuse_objective == REG_LINEAR ? 0 : 1;
     double msum = 0;
     float mg = 0.f, mh = 0.f;
-    extern __shared__ __align__(16) unsigned char walk_sm[];
-    WalkNode *wn = reinterpret_cast<WalkNode *>(walk_sm);
-    WalkSpan *ws = reinterpret_cast<WalkSpan *>(walk_sm + sizeof(WalkNode) * n_nodes);
+    extern __shared__ __align__(16) unsigned char walk_sm[];   // WalkNode[n_nodes], float weight[n_nodes], LAYOUT 2: WalkSpan[n_nodes]
+    float *ww = reinterpret_cast<float *>(walk_sm + sizeof(WalkNode) * n_nodes);
+    WalkSpan *ws = reinterpret_cast<WalkSpan *>(walk_sm + (sizeof(WalkNode) * n_nodes + sizeof(float) * (n_nodes + 1)));
     if (table_in_smem) {
         for (int i = threadIdx.x; i < n_nodes; i += blockDim.x) {
-            wn[i] = walk_node(nodes, i, rev);
+            reinterpret_cast<WalkNode *>(walk_sm)[i] = walk_node(nodes, i, rev);
+            ww[i] = walk_weight(nodes, i);
             if (LAYOUT == 2) ws[i] = walk_span(nodes, cut_ptr, i);
         }
         __syncthreads();
     }
+    const int levels = 31 - __clz(n_nodes + 1) - 1;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         int lo0 = 0, hi0 = 0;
         uint32_t w[8];
@@ -682,53 +693,51 @@ k_predict_walk(const TreeNode *nodes, int n_nodes, int table_in_smem, const unsi
             const uint4 a = reinterpret_cast<const uint4 *>(row)[0], b = reinterpret_cast<const uint4 *>(row)[1];
             w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
         }
-        int nid = 0;
-        float weight = 0.f;
+        const float score0 = yp[r];
+        const float yr = fuse ? y[r] : 0.f;
+        unsigned at = 0;   // table offset of the row's node
 #pragma unroll 1
-        for (;;) {
-            const WalkNode wk = table_in_smem ? wn[nid] : walk_node(nodes, nid, rev);
-            if (!(wk.flags & 0x400)) weight = wk.weight;
-            if (!(wk.flags & 0x200)) break;
-            int b = MISSING_BIN;
+        for (int l = 0; l < levels; ++l) {
+            const WalkNode wk = table_in_smem ? *reinterpret_cast<const WalkNode *>(walk_sm + at) : walk_node(nodes, (int)(at / sizeof(WalkNode)), rev);
+            unsigned b;
             if (LAYOUT == 2) {
-                const WalkSpan sp = table_in_smem ? ws[nid] : walk_span(nodes, cut_ptr, nid);
-                int lo = lo0, hi = hi0;
+                const WalkSpan sp = table_in_smem ? ws[at / sizeof(WalkNode)] : walk_span(nodes, cut_ptr, (int)(at / sizeof(WalkNode)));
+                int lo = lo0, hi = wk.left == at ? lo0 : hi0;
+                b = MISSING_BIN;
                 while (lo < hi) {  // bin ids ascend inside a row
                     const int mid = lo + (hi - lo) / 2, v = sp_bin[mid];
                     if (v >= sp.c0 && v < sp.c1) { b = v - sp.c0; break; }
                     if (v < sp.c0) lo = mid + 1; else hi = mid;
                 }
             } else if (LAYOUT == 1) {
-                b = row[(unsigned)wk.flags >> 16];
+                b = row[wk.test >> 16];
             } else {
-                const unsigned f = (unsigned)wk.flags >> 16;
-                const uint32_t a0 = (f & 16) ? w[4] : w[0], a1 = (f & 16) ? w[5] : w[1], a2 = (f & 16) ? w[6] : w[2],
-                               a3 = (f & 16) ? w[7] : w[3];
-                const uint32_t b0 = (f & 8) ? a2 : a0, b1 = (f & 8) ? a3 : a1;
-                b = (((f & 4) ? b1 : b0) >> (8 * (f & 3))) & 0xffu;
+                const bool h16 = wk.test & 0x8000u, h8 = wk.test & 0x4000u;
+                const uint32_t a0 = h16 ? w[4] : w[0], a1 = h16 ? w[5] : w[1], a2 = h16 ? w[6] : w[2], a3 = h16 ? w[7] : w[3];
+                b = __byte_perm(h8 ? a2 : a0, h8 ? a3 : a1, wk.test);   // the low byte counts
             }
-            const bool left = (b == MISSING_BIN) ? !(wk.flags & 0x100) : ((wk.flags & 0x800) ? b > (wk.flags & 0xff) : b < (wk.flags & 0xff));
-            nid = 2 * nid + (left ? 1 : 2);
+            const unsigned x = (b + ((wk.test >> 13) & 1u)) & 0xffu, threshold = (wk.test >> 4) & 0x1ffu;
+            at = wk.left + ((x < threshold) != (rev != 0) ? 0u : (unsigned)sizeof(WalkNode));
         }
+        const int nid = (int)(at / sizeof(WalkNode));
         if (nid_out) nid_out[r] = nid;
-        const float score = __fmaf_rn(lr, weight, yp[r]);
+        const float score = __fmaf_rn(lr, table_in_smem ? ww[nid] : walk_weight(nodes, nid), score0);
         yp[r] = score;
         if (fuse) {
-            const float yr = y[r];
             msum += pointwise_metric_term(fuse_objective, yr, score);
             const float2 v = pointwise_gh(fuse_logistic, yr, score);
             mg = fmaxf(mg, fabsf(v.x)); mh = fmaxf(mh, v.y);
         }
     }
     if (fuse) {
-        __shared__ double ws[8];
+        __shared__ double part[8];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) msum += __shfl_xor_sync(0xffffffffu, msum, o);
-        if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = msum;
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = msum;
         __syncthreads();
         if (threadIdx.x == 0) {
             double t = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ws[w];
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
             metric_partial[blockIdx.x] = t;
         }
         track_max(mg, mh, maxbits);
@@ -792,12 +801,12 @@ static __global__ void k_round_end(int objective, const double *sum, const doubl
     for (int i = threadIdx.x; i < n_root; i += 32) root_sum[i] = 0;   // the next round adds to them
     double t = 0;
     if (partial) {
-        // (at most 1024 partial sums: all loads first, then the additions in the usual order)
-        double v[32];
+        // (all loads first, then the additions in the usual order)
+        double v[METRIC_PARTS / 32];
 #pragma unroll
-        for (int u = 0; u < 32; ++u) v[u] = (int)threadIdx.x + 32 * u < nb ? partial[threadIdx.x + 32 * u] : 0.0;
+        for (int u = 0; u < METRIC_PARTS / 32; ++u) v[u] = (int)threadIdx.x + 32 * u < nb ? partial[threadIdx.x + 32 * u] : 0.0;
 #pragma unroll
-        for (int u = 0; u < 32; ++u) t += v[u];
+        for (int u = 0; u < METRIC_PARTS / 32; ++u) t += v[u];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     }
