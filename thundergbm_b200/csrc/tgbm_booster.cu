@@ -132,14 +132,17 @@ struct BoosterImpl {
     // tree_method = exact (tgbm_exact.cuh)
     bool exact = false;
     long long ex_nnz = 0;
-    DevBuf<int> ex_row;                 // stored values by column, largest first: row ...
-    DevBuf<float> ex_val;               // ... and value
-    DevBuf<long long> ex_csc_ptr;
-    DevBuf<unsigned> ex_key[2], ex_idx[2];  // per level: partition id of every entry / sorted, entry of every sorted position
-    DevBuf<unsigned char> ex_sums;      // ExPair<T> per sorted position: (g,h) of its partition up to itself
-    DevBuf<int> ex_pid_ptr, ex_nid, ex_any;
+    // stored values by column, largest first ([0]), and grouped by (column, node) at the levels below the root (two in turn)
+    DevBuf<unsigned> ex_key[3];
+    DevBuf<int> ex_row[3];
+    DevBuf<float> ex_val[3];
+    DevBuf<unsigned char> ex_pre, ex_tile_sum, ex_tile_pre;   // prefix sums: see k_exact_sum
+    DevBuf<unsigned> ex_lr;
+    DevBuf<ExPair<int>> ex_tile_cnt, ex_tile_lr;
+    DevBuf<int2> ex_group, ex_gh[3];                // (group ranges; gradient pairs of the entries, float or quantised)
+    DevBuf<uint2> ex_side;
+    DevBuf<int> ex_live, ex_nid, ex_any, ex_ticket;   // ex_live[level]: entries of the level
     DevBuf<unsigned long long> ex_best;
-    DevBuf<unsigned char> ex_tmp;       // scratch of the radix sort and the scan by key
     void init_exact();
     template <typename T> void exact_levels(int k, const void *gh_rows);
     void build_tree_exact(int round, int k);
@@ -610,27 +613,26 @@ void BoosterImpl::init_exact() {
     ex_nnz = (long long)nnz;
     TGBM_CHECK(nnz < (1ull << 31), "the exact builder indexes stored values with 32 bits");
     TGBM_CHECK((double)F * (double)(1 << std::max(0, depth - 1)) < 4294967295.0, "columns x nodes of the last level must fit 32 bits");
-    const size_t n1 = std::max<size_t>(nnz, 1);
+    const size_t n1 = std::max<size_t>(nnz, 1), tiles = (n1 + EX_TILE - 1) / EX_TILE, padded = tiles * EX_TILE;   // whole tiles are loaded
     const int grid = std::max(1, std::min(ceil_div((long long)n1, 256), num_sms * 16));
     {
         DevBuf<unsigned long long> keys, keys2;
         DevBuf<int> rows;
-        keys.alloc(n1); keys2.alloc(n1); rows.alloc(n1); ex_row.alloc(n1); ex_val.alloc(n1); ex_csc_ptr.alloc(F + 1);
+        keys.alloc(n1); keys2.alloc(n1); rows.alloc(n1);
+        for (int i = 0; i < (depth > 1 ? 3 : 1); ++i) { ex_key[i].alloc(padded); ex_row[i].alloc(padded); ex_val[i].alloc(padded); ex_gh[i].alloc(padded); }
         if (N) k_exact_rows<<<std::min(ceil_div(N, 256), num_sms * 16), 256, 0, stream>>>(in.row_ptr.p, N, rows.p);
         if (nnz) k_exact_csc_keys<<<grid, 256, 0, stream>>>(in.val.p, in.col.p, nnz, keys.p);
         int end_bit = 32;
         while ((1ll << (end_bit - 32)) < F && end_bit < 64) ++end_bit;
         if (nnz) {
             size_t tb = 0;
-            cub::DeviceRadixSort::SortPairs(nullptr, tb, keys.p, keys2.p, rows.p, ex_row.p, (long long)nnz, 0, end_bit, stream);
+            cub::DeviceRadixSort::SortPairs(nullptr, tb, keys.p, keys2.p, rows.p, ex_row[0].p, (long long)nnz, 0, end_bit, stream);
             DevBuf<unsigned char> tmp;
             tmp.alloc(std::max<size_t>(tb, 1));
-            TGBM_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, keys.p, keys2.p, rows.p, ex_row.p, (long long)nnz, 0, end_bit, stream));
-            k_exact_csc_vals<<<grid, 256, 0, stream>>>(keys2.p, nnz, ex_val.p);
+            TGBM_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, keys.p, keys2.p, rows.p, ex_row[0].p, (long long)nnz, 0, end_bit, stream));
+            k_exact_csc_vals<<<grid, 256, 0, stream>>>(keys2.p, nnz, ex_val[0].p, ex_key[0].p);
             TGBM_CUDA(cudaStreamSynchronize(stream));
         }
-        k_feature_bounds<<<ceil_div(F + 1, 128), 128, 0, stream>>>(keys2.p, (long long)nnz, F, ex_csc_ptr.p);
-        TGBM_CUDA(cudaStreamSynchronize(stream));
     }
     in.release();
     // no cut points, no bin matrix
@@ -639,29 +641,20 @@ void BoosterImpl::init_exact() {
     cut_ptr.alloc(F + 1); cut_val.alloc(1); cut_fid.alloc(1);
     cut_ptr.zero(stream);
     const size_t max_nl = (size_t)1 << std::max(0, depth - 1);
-    for (int i = 0; i < 2; ++i) { ex_key[i].alloc(n1); ex_idx[i].alloc(n1); }
-    k_exact_iota<<<grid, 256, 0, stream>>>(ex_idx[0].p, n1);
-    ex_sums.alloc(n1 * (f32 ? sizeof(ExPair<float>) : sizeof(ExPair<long long>)));
-    ex_pid_ptr.alloc((size_t)F * max_nl + 2);
-    ex_nid.alloc(std::max(N, 1));
+    const size_t v = f32 ? sizeof(double) : sizeof(int), w = 8;
+    ex_pre.alloc(2 * v * padded); ex_tile_sum.alloc(2 * w * tiles); ex_tile_pre.alloc(2 * w * tiles);
+    ex_lr.alloc(padded); ex_tile_cnt.alloc(tiles); ex_tile_lr.alloc(tiles);
+    ex_group.alloc((size_t)F * max_nl + 1);
+    ex_live.alloc(depth + 1);
+    const int live = (int)nnz;
+    TGBM_CUDA(cudaMemcpyAsync(ex_live.p, &live, sizeof(int), cudaMemcpyHostToDevice, stream));
+    ex_nid.alloc(std::max(N, 1)); ex_side.alloc(N / 32 + 1);
     ex_best.alloc(max_nl);
     ex_best.zero(stream);
     ex_any.alloc(1);
     ex_any.zero(stream);
-    size_t tb_sort = 0, tb_scan = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb_sort, ex_key[0].p, ex_key[1].p, ex_idx[0].p, ex_idx[1].p, (long long)n1, 0, 32, stream);
-    if (f32) {
-        cub::TransformInputIterator<ExPair<float>, ExGather<float>, cub::CountingInputIterator<long long>> in(
-            cub::CountingInputIterator<long long>(0), ExGather<float>{ex_idx[1].p, ex_row.p, nullptr});
-        cub::DeviceScan::InclusiveScanByKey(nullptr, tb_scan, ex_key[1].p, in, reinterpret_cast<ExPair<float> *>(ex_sums.p), ExAdd<float>(),
-                                            (long long)n1, cub::Equality(), stream);
-    } else {
-        cub::TransformInputIterator<ExPair<long long>, ExGather<long long>, cub::CountingInputIterator<long long>> in(
-            cub::CountingInputIterator<long long>(0), ExGather<long long>{ex_idx[1].p, ex_row.p, nullptr});
-        cub::DeviceScan::InclusiveScanByKey(nullptr, tb_scan, ex_key[1].p, in, reinterpret_cast<ExPair<long long> *>(ex_sums.p), ExAdd<long long>(),
-                                            (long long)n1, cub::Equality(), stream);
-    }
-    ex_tmp.alloc(std::max<size_t>(std::max(tb_sort, tb_scan), 1));
+    ex_ticket.alloc(1);
+    ex_ticket.zero(stream);
     TGBM_CUDA(cudaFuncSetAttribute(k_exact_gain<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
     TGBM_CUDA(cudaFuncSetAttribute(k_exact_gain<long long>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
     TGBM_CUDA(cudaStreamSynchronize(stream));
@@ -673,37 +666,35 @@ void BoosterImpl::init_exact() {
 // quantised gradients, exact in any order.
 template <typename T>
 void BoosterImpl::exact_levels(int k, const void *gh_rows) {
-    const long long nnz = ex_nnz;
-    const int grid = std::max(1, std::min(ceil_div(std::max<long long>(nnz, 1), 256), num_sms * 16));
-    const int row_grid = std::max(1, std::min(ceil_div(std::max(N, 1), 256), num_sms * 8));
-    ExPair<T> *sums = reinterpret_cast<ExPair<T> *>(ex_sums.p);
+    typedef typename ExKind<T>::V V;
+    typedef typename ExKind<T>::W W;
     TGBM_CUDA(cudaMemsetAsync(ex_nid.p, 0, sizeof(int) * (size_t)std::max(N, 1), stream));
+    if (!ex_nnz) return;   // no stored value: the root stays as it is
+    const int grid = std::max(1, std::min(ceil_div(ex_nnz, EX_TILE), num_sms * 8));
+    const int row_grid = std::max(1, std::min(ceil_div(std::max(N, 1), 256), num_sms * 8));
+    ExPair<V> *pre = reinterpret_cast<ExPair<V> *>(ex_pre.p);
+    ExPair<W> *tile_sum = reinterpret_cast<ExPair<W> *>(ex_tile_sum.p), *tile_pre = reinterpret_cast<ExPair<W> *>(ex_tile_pre.p);
+    typedef typename ExKind<T>::In In;
+    auto gh_of = [&](int i) { return reinterpret_cast<In *>(ex_gh[i].p); };
     for (int level = 0; level < depth; ++level) {
-        const int nl = 1 << level;
-        const long long n_pid = (long long)F * nl;
-        if (nnz) {
-            k_exact_keys<<<grid, 256, 0, stream>>>(ex_row.p, nnz, ex_csc_ptr.p, F, ex_nid.p, level, ex_key[0].p);
-            int end_bit = 1;
-            while ((1ll << end_bit) <= n_pid && end_bit < 32) ++end_bit;   // the largest key, EX_NONE, has every bit set
-            size_t tb = ex_tmp.n;
-            TGBM_CUDA(cub::DeviceRadixSort::SortPairs(ex_tmp.p, tb, ex_key[0].p, ex_key[1].p, ex_idx[0].p, ex_idx[1].p, nnz, 0, end_bit, stream));
-            using Gather = ExGather<T>;
-            cub::TransformInputIterator<ExPair<T>, Gather, cub::CountingInputIterator<long long>> in(
-                cub::CountingInputIterator<long long>(0),
-                Gather{ex_idx[1].p, ex_row.p, reinterpret_cast<decltype(Gather::gh)>(gh_rows)});
-            tb = ex_tmp.n;
-            TGBM_CUDA(cub::DeviceScan::InclusiveScanByKey(ex_tmp.p, tb, ex_key[1].p, in, sums, ExAdd<T>(), nnz, cub::Equality(), stream));
-            k_exact_pid_ptr<<<std::max(1, std::min(ceil_div(n_pid + 1, 256), num_sms * 16)), 256, 0, stream>>>(ex_key[1].p, nnz, n_pid, ex_pid_ptr.p);
-            k_exact_gain<T><<<num_sms * 2, EX_THREADS, sizeof(unsigned long long) * (size_t)nl, stream>>>(
-                ex_key[1].p, ex_idx[1].p, ex_val.p, sums, ex_pid_ptr.p, nnz, level, nodes.p, qinfo.p, p.min_child_weight, p.lambda,
-                ignored_all.p, rstate.p, F, ex_best.p);
-            launches += 5;
-        }
-        k_exact_apply<T><<<ceil_div(nl, 128), 128, 0, stream>>>(ex_key[1].p, ex_idx[1].p, ex_val.p, sums, ex_pid_ptr.p, level, nodes.p, qinfo.p,
-                                                                 p.min_child_weight, p.lambda, p.rt_eps, ex_best.p, ex_any.p);
-        if (nnz) k_exact_move<<<grid, 256, 0, stream>>>(ex_row.p, ex_val.p, nnz, ex_csc_ptr.p, F, ex_nid.p, nodes.p, ex_any.p);
-        k_exact_move_missing<<<row_grid, 256, 0, stream>>>(ex_nid.p, N, level, nodes.p, ex_any.p);
-        launches += 3;
+        const int nl = 1 << level, a = level == 0 ? 0 : 1 + (level & 1), z = 1 + ((level + 1) & 1);   // this level's entries, the next one's
+        const int *live = ex_live.p + level;
+        launch_after(level == 0 ? k_exact_sum<T, true> : k_exact_sum<T, false>, grid, EX_THREADS, 0, stream, live, ex_key[a].p, ex_row[a].p,
+                     static_cast<const In *>(gh_rows), gh_of(a), pre, tile_sum, tile_pre, ex_group.p, ex_ticket.p);
+        const ExSearch<T> x{ex_key[a].p, ex_val[a].p, pre, tile_pre, ex_group.p};
+        launch_after(k_exact_gain<T>, grid, EX_THREADS, sizeof(unsigned long long) * (size_t)nl, stream, live, x, level, nodes.p, qinfo.p,
+                     p.min_child_weight, p.lambda, p.rt_eps, ignored_all.p, rstate.p, F, ex_best.p, ex_any.p, ex_ticket.p);
+        const int node_blocks = std::min(nl, 1024);
+        launch_after(k_exact_move, dim3(std::max(1, row_grid / node_blocks), node_blocks), 256, 0, stream, ex_row[a].p, ex_val[a].p, ex_group.p, level, ex_nid.p,
+                     nodes.p, ex_any.p);
+        launch_after(k_exact_move_missing, row_grid, 256, 0, stream, ex_nid.p, N, level, nodes.p, ex_any.p, ex_side.p);
+        launches += 4;
+        if (level + 1 == depth) break;
+        launch_after(k_exact_sides, grid, EX_THREADS, 0, stream, live, ex_row[a].p, ex_side.p, ex_lr.p, ex_tile_cnt.p, ex_tile_lr.p, ex_live.p + level + 1,
+                     ex_ticket.p);
+        launch_after(k_exact_scatter<In>, grid, EX_THREADS, 0, stream, live, ex_key[a].p, ex_row[a].p, ex_val[a].p, gh_of(a), ex_lr.p, ex_tile_lr.p, ex_group.p, ex_key[z].p,
+                     ex_row[z].p, ex_val[z].p, gh_of(z));
+        launches += 2;
     }
     (void)k;
 }
