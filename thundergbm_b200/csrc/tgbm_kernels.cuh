@@ -30,9 +30,10 @@ constexpr int FINE_BITS = 30;          // value bits of the grid of fp32 mode's 
 constexpr int FINE_WINDOW = 1 << 16;   // rows whose 16-bit low halves fit an unsigned accumulator
 constexpr int FINE_FROM_ROUND = 1;     // fp32 mode: rounds before it sum floats value by value (k_hist_f32)
 
-// Shares of the level's tiles per CTA of the dense histogram kernel.  More shares balance the CTAs better but widen the
-// window of rows the GPU works on at a time; 1 to 4 measure the same on 10.5 M rows, 16 is 10 % slower.
-constexpr int HIST_SHARES = 2;
+// Shares of the level's tiles per CTA of the dense histogram kernel: two when a CTA has HIST_SHARE_TILES tiles or more, else
+// one.  Two balance the CTAs better (7 trees of 581 k rows side by side, 22 tiles per CTA: 50.6 ms per training against 52.6),
+// but a CTA with few tiles then hands over the sums of twice as many nodes (1 M rows, 3 tiles per CTA: 54.3 ms against 52.2).
+constexpr int HIST_SHARES = 2, HIST_SHARE_TILES = 8;
 
 // Device copy of the booster's round counter: kernels whose work depends on the round read it here, so that the launch
 // sequence of a round is the same every round and can be replayed as a CUDA graph.

@@ -111,9 +111,9 @@ __device__ __forceinline__ int hist_items(int level, const Batch &b, size_t tree
 }
 
 // Order in which the dense histogram kernel visits the level's tiles.
-// The tiles are dealt out to `n_ctas * HIST_SHARES` shares in proportion to the items' sizes (cumulative rounding, so
+// The tiles are dealt out to shares, one or two per CTA, in proportion to the items' sizes (cumulative rounding, so
 // the shares of different items are disjoint; an item too small for a share of its own rides on one).  Inside an item
-// tile t belongs to share v0 + t mod k.  CTA c owns HIST_SHARES consecutive shares and visits, item by item, the tiles
+// tile t belongs to share v0 + t mod k.  CTA c owns its consecutive shares and visits, item by item, the tiles
 // of its shares in ascending order: every CTA walks each of its (one or two, rarely more) lists once, front to back,
 // and since all CTAs carry about the same number of tiles, all lists are walked at the same relative pace.  Row ids
 // ascend inside every list, so at any time the whole GPU gathers rows from one moving window of the bin matrix:
@@ -188,14 +188,16 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
     __shared__ int scratch[33], s_ib, s_ie;
     const int group = blockIdx.y, f0 = group * 32, nf = min(32, F - f0), lane = threadIdx.x & 31;
     const size_t tree = tree0 + blockIdx.z;
-    for (int i = threadIdx.x; i < (FINE ? HIST_FINE_SMEM : HIST_EXACT_SMEM) / 16; i += HIST_THREADS)
+    constexpr int ZERO_BYTES = FINE ? 4 * HIST_CELLS * 4 : 2 * HIST_CELLS * 4;   // the accumulators
+    for (int i = threadIdx.x; i < ZERO_BYTES / 16; i += HIST_THREADS)
         reinterpret_cast<int4 *>(hist_sm)[i] = make_int4(0, 0, 0, 0);
     chain_wait();
     if (threadIdx.x == 0) { s_ib = 0x7fffffff; s_ie = -1; }
     const int total = hist_items<HIST_THREADS, HIST_THREADS>(level, b, tree, by_hessian, s_base, scratch, blockIdx.x == 0 && group == 0);
     if (total == 0) return;
     const int pairs = level == 0 ? 1 : 1 << (level - 1);
-    const int n_shares = (int)gridDim.x * HIST_SHARES, va = (int)blockIdx.x * HIST_SHARES, vb = va + HIST_SHARES;
+    const int per_cta = total >= HIST_SHARE_TILES * (int)gridDim.x ? HIST_SHARES : 1;
+    const int n_shares = (int)gridDim.x * per_cta, va = (int)blockIdx.x * per_cta, vb = va + per_cta;
     const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
     const TreeNode *nodes = b.nodes + tree * b.nodes_stride;
     for (int w = threadIdx.x; w < pairs; w += HIST_THREADS) {   // items with a share among this CTA's
@@ -234,14 +236,17 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
     const int2 *rec_gh = GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride;
     long long *slab = b.hist_built + tree * b.built_stride;
 
+    bool drained = false;   // the totals hold something: few rows per node and CTA need none, so they are not zeroed either
     auto drain = [&]() {  // int32 window -> int64 totals, same [bin][feature] layout
         __syncthreads();
 #pragma unroll 4
         for (int i = threadIdx.x; i < 2 * HIST_CELLS; i += HIST_THREADS) {
             const int v = acc[i];
-            if (v) { tot[i] += v; acc[i] = 0; }
+            tot[i] = drained ? tot[i] + v : v;
+            acc[i] = 0;
         }
         __syncthreads();
+        drained = true;
     };
     const int flush_b0 = lane < nf ? cut_ptr[f0 + lane] : 0;   // first bin of this lane's feature
     const int flush_nb = lane < nf ? cut_ptr[f0 + lane + 1] - flush_b0 : 0;
@@ -254,7 +259,8 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
             if (FINE) {
                 vg[q] = ((long long)high[s] << 16) + (unsigned)acc[s]; vh[q] = ((long long)high[HIST_CELLS + s] << 16) + (unsigned)acc[HIST_CELLS + s];
             } else {
-                vg[q] = tot[s] + acc[s]; vh[q] = tot[HIST_CELLS + s] + acc[HIST_CELLS + s];
+                vg[q] = acc[s]; vh[q] = acc[HIST_CELLS + s];
+                if (drained) { vg[q] += tot[s]; vh[q] += tot[HIST_CELLS + s]; }
             }
         }
         __syncthreads();
@@ -270,8 +276,9 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
         }
         if (!again) return;
         __syncthreads();
-        for (int i = threadIdx.x; i < (FINE ? HIST_FINE_SMEM : HIST_EXACT_SMEM) / 16; i += HIST_THREADS)
+        for (int i = threadIdx.x; i < ZERO_BYTES / 16; i += HIST_THREADS)
             reinterpret_cast<int4 *>(hist_sm)[i] = make_int4(0, 0, 0, 0);
+        drained = false;
         __syncthreads();
     };
 
