@@ -1109,19 +1109,19 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
     // one CTA per SM over all trees and feature groups: every further CTA is one more flush per node
     const int hist_ctas = std::max(1, num_sms / (n_trees * (sparse ? 1 : G)));
     for (int level = 0; level < depth && !one_launch; ++level) {
-        const int nl = 1 << level, pairs = std::max(1, nl / 2);
+        const int nl = 1 << level, pairs = std::max(1, nl / 2), keep = level == 0 || level + 1 < depth;
         const size_t table = sizeof(int) * ((size_t)pairs + 1);
         // -- histogram of the root / of the smaller child of every pair, and the choice of the splits
         auto evaluate = [&](auto *built, int bs, int tree, int n) {
             using T = std::remove_pointer_t<decltype(built)>;
             if (sparse) {
                 launch_after(k_eval_chunk<T>, dim3(n_chunks, pairs, n), 64, 0, stream, level, b, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_fid.p, built, bs, qinfo.p,
-                                                                             p.min_child_weight, p.lambda, ignored_all.p, rstate.p, F, colb, by_hessian, tree);
+                                                                             p.min_child_weight, p.lambda, ignored_all.p, rstate.p, F, colb, by_hessian, keep, tree);
                 launch_after(k_best_apply, dim3(nl, 1, n), 32, 0, stream, level, b, n_chunks, cut_ptr.p, cut_val.p, p.rt_eps, p.lambda, cut_fid.p, 1, colb, tree);
                 launches += 2;
             } else {
                 launch_after(k_eval<T>, dim3(F, pairs, n), EVAL_THREADS, 0, stream, level, b, F, B, cut_ptr.p, built, bs, qinfo.p, p.min_child_weight, p.lambda,
-                                                                         cut_val.p, p.rt_eps, cut_fid.p, ignored_all.p, rstate.p, colb, by_hessian, tree);
+                                                                         cut_val.p, p.rt_eps, cut_fid.p, ignored_all.p, rstate.p, colb, by_hessian, keep, tree);
                 ++launches;
             }
         };

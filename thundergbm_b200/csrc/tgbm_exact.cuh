@@ -205,11 +205,11 @@ __device__ __forceinline__ ExCand exact_cand(const TreeNode &nd, const ExPair<W>
     return ExCand{exact_cell(right.g, inv_sg), exact_cell(right.h, inv_sh),
                   __fsub_rn(nd.sum_g, exact_cell(total.g, inv_sg)), __fsub_rn(nd.sum_h, exact_cell(total.h, inv_sh))};
 }
-__device__ __forceinline__ float exact_gain(float pg, float ph, const ExCand &c, float mcw, float lam) {
+__device__ __forceinline__ float exact_gain(float parent, float pg, float ph, const ExCand &c, float mcw, float lam) {
     // exact_tree_builder.cu:186-209 (gain, default direction)
-    const float gl = fmaxf(0.f, split_gain(pg, ph, __fsub_rn(pg, c.rg), __fsub_rn(ph, c.rh), c.rg, c.rh, mcw, lam));
+    const float gl = fmaxf(0.f, split_gain(parent, pg, ph, c.rg, c.rh, mcw, lam));
     const float rg2 = __fadd_rn(c.rg, c.mg), rh2 = __fadd_rn(c.rh, c.mh);
-    const float gr = fmaxf(0.f, split_gain(pg, ph, __fsub_rn(pg, rg2), __fsub_rn(ph, rh2), rg2, rh2, mcw, lam));
+    const float gr = fmaxf(0.f, split_gain(parent, pg, ph, rg2, rh2, mcw, lam));
     return gl > gr ? gl : -gr;
 }
 // the children's terms of the gain with fast divisions (2 units in the last place), the larger of the two directions
@@ -230,7 +230,8 @@ __device__ __forceinline__ void exact_apply(const ExSearch<T> &x, int level, int
     const int2 range = x.group[key];
     const ExPair<typename ExKind<T>::W> base = exact_before(x, (unsigned)range.x);
     const ExCand c = exact_cand(nd, exact_before(x, j + 1) - base, exact_before(x, (unsigned)range.y) - base, inv_sg, inv_sh);
-    const float gn = exact_gain(nd.sum_g, nd.sum_h, c, mcw, lam);
+    const float parent = __fdiv_rn(__fmul_rn(nd.sum_g, nd.sum_g), __fadd_rn(nd.sum_h, lam));
+    const float gn = exact_gain(parent, nd.sum_g, nd.sum_h, c, mcw, lam);
     const float gain = __uint_as_float((unsigned)(b >> 32));   // |gn|, or 0 for a column left out of the round
     if (gain > rt_eps) {
         const float v = x.val[j];
@@ -259,7 +260,7 @@ __device__ __forceinline__ void exact_apply(const ExSearch<T> &x, int level, int
 // the largest |gain| and among equals the smallest sorted position (exact_tree_builder.cu:218-258: smaller partition
 // id, i.e. smaller column, then larger value).  Per block the keys meet in shared memory (one slot per node of the
 // level), warps whose lanes all sit in one node reduce first.
-// Five exact divisions per direction are what a candidate costs: one that cannot reach its block's best so far is left out
+// Two exact divisions per direction are what a candidate costs: one that cannot reach its block's best so far is left out
 // by a bound with fast divisions, whose margin (1e-5) is far above their error.
 template <typename T>
 static __global__ void __launch_bounds__(EX_THREADS)
@@ -319,7 +320,7 @@ k_exact_gain(const int *live, const ExSearch<T> x, int level, TreeNode *nodes, c
                 c.rg = exact_cell(right.g, inv_sg); c.rh = exact_cell(right.h, inv_sh);
                 c.mg = __fsub_rn(pg, exact_cell(total.g, inv_sg)); c.mh = __fsub_rn(ph, exact_cell(total.h, inv_sh));
                 if (bar > 0.f && exact_terms(pg, ph, c, lam) * 1.00001f < (bar + parent) * 0.99999f) continue;
-                gn = exact_gain(pg, ph, c, mcw, lam);
+                gn = exact_gain(parent, pg, ph, c, mcw, lam);
             }
             const unsigned long long mine = ((unsigned long long)__float_as_uint(fabsf(gn)) << 32) | (0xffffffffu - i);
             if (cn >= 0 && cn != n) { atomicMax(&ex_best[cn], cand); cand = 0; }

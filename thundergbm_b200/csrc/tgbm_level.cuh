@@ -501,14 +501,6 @@ __device__ __forceinline__ float split_gain(float parent, float pg, float ph, fl
         return __fsub_rn(__fadd_rn(__fdiv_rn(__fmul_rn(g, g), __fadd_rn(h, lam)), __fdiv_rn(__fmul_rn(g2, g2), __fadd_rn(h2, lam))), parent);
     return 0.f;
 }
-__device__ __forceinline__ float split_gain(float pg, float ph, float lg, float lh, float rg, float rh, float mcw, float lam) {
-    // compute_gain, hist_tree_builder_single.cu:279-286 (no fused multiply-add: products feed divisions)
-    if (lh >= mcw && rh >= mcw)
-        return __fsub_rn(__fadd_rn(__fdiv_rn(__fmul_rn(lg, lg), __fadd_rn(lh, lam)), __fdiv_rn(__fmul_rn(rg, rg), __fadd_rn(rh, lam))),
-                         __fdiv_rn(__fmul_rn(pg, pg), __fadd_rn(ph, lam)));
-    return 0.f;
-}
-
 // Per-node argmax over the features, SplitPoint decode and update_tree
 // (hist_tree_builder_single.cu:365-389 and :847-902).  Called by one whole warp for node n of the level.  The records
 // may have been written by other blocks of the running kernel: they are read past L1.
@@ -645,7 +637,8 @@ static __global__ void __launch_bounds__(EVAL_THREADS, 8)
 k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, T *built_all, int bs,
        const QuantInfo *q, float mcw, float lam, const float *__restrict__ cut_val, float rt_eps,
        const int *__restrict__ cut_fid, const unsigned char *__restrict__ ignored_all, const RoundState *rs, int multi,
-       int by_hessian, int tree0) {
+       int by_hessian, int keep, int tree0) {
+    // keep = 0 at the last level: no level subtracts from its histograms, so they are not stored
     constexpr int WARPS = EVAL_THREADS / 32, NB = EVAL_BINS;
     __shared__ T s_sum[4][sizeof(T) == 4 ? 32 : WARPS];
     __shared__ unsigned long long s_key[2][WARPS];
@@ -687,7 +680,7 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
             *reinterpret_cast<Pair *>(built + (size_t)2 * bs * (i0 + n)) = Pair{0, 0};
             T *own = full + 2 * (b0 + i0 + n);
             if (level == 0) *reinterpret_cast<Pair *>(own) = cell[n];   // what the next level subtracts from
-            else {
+            else if (keep) {
                 *reinterpret_cast<Pair *>(own + (size_t)(2 * j + br) * B * 2) = cell[n];
                 *reinterpret_cast<Pair *>(own + (size_t)(2 * j + 1 - br) * B * 2) = Pair{og, oh};
             }
@@ -815,7 +808,7 @@ template <typename T>
 static __global__ void __launch_bounds__(64)
 k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restrict__ chunk_bin0, const int *__restrict__ cut_ptr,
              const int *__restrict__ cut_fid, T *built_all, int bs, const QuantInfo *q, float mcw, float lam,
-             const unsigned char *__restrict__ ignored_all, const RoundState *rs, int F, int multi, int by_hessian, int tree0) {
+             const unsigned char *__restrict__ ignored_all, const RoundState *rs, int F, int multi, int by_hessian, int keep, int tree0) {
     chain_wait();
     const size_t tree = tree0 + blockIdx.z;
     const TreeNode *nodes = b_.nodes + tree * b_.nodes_stride;
@@ -856,13 +849,13 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
             const int i = threadIdx.x + 64 * u;
             if (i >= nb) continue;
             *reinterpret_cast<Pair *>(bp + (size_t)2 * bs * (b0 + i)) = Pair{0, 0};   // zeroed as it is read, like in k_eval
-            *reinterpret_cast<Pair *>(fb + 2 * (size_t)(b0 + i)) = cell[u];
+            if (keep) *reinterpret_cast<Pair *>(fb + 2 * (size_t)(b0 + i)) = cell[u];   // not at the last level, like in k_eval
             const int side = level == 0 ? 0 : br;
             sg[side][i] = cell[u].x; sh[side][i] = cell[u].y;
             if (level > 0) {
                 const T og = above[u].x - cell[u].x, oh = above[u].y - cell[u].y;
                 sg[1 - br][i] = og; sh[1 - br][i] = oh;
-                *reinterpret_cast<Pair *>(fo + 2 * (size_t)(b0 + i)) = Pair{og, oh};
+                if (keep) *reinterpret_cast<Pair *>(fo + 2 * (size_t)(b0 + i)) = Pair{og, oh};
             }
         }
     }
@@ -914,7 +907,7 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
         }
     }
     __syncwarp();
-    const float pg = nd.sum_g, ph = nd.sum_h;
+    const float pg = nd.sum_g, ph = nd.sum_h, parent = __fdiv_rn(__fmul_rn(pg, pg), __fadd_rn(ph, lam));
     const GridScale inv_sg(cell_inv<T>(q, 0)), inv_sh(cell_inv<T>(q, 1));
     float best = 0.f, best_lg = 0.f, best_lh = 0.f, best_mg = 0.f, best_mh = 0.f;
     int best_bin = -1;
@@ -928,15 +921,15 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
             float gn, keep_g, keep_h;
             if (multi) {  // inclusive prefix = right child, see eval_feature
                 const float rg = cell_f(sg[warp][b], inv_sg), rh = cell_f(sh[warp][b], inv_sh);
-                const float gl = fmaxf(0.f, split_gain(pg, ph, __fsub_rn(pg, rg), __fsub_rn(ph, rh), rg, rh, mcw, lam));
+                const float gl = fmaxf(0.f, split_gain(parent, pg, ph, rg, rh, mcw, lam));
                 const float rg2 = __fadd_rn(rg, mg), rh2 = __fadd_rn(rh, mh);
-                const float gr = fmaxf(0.f, split_gain(pg, ph, __fsub_rn(pg, rg2), __fsub_rn(ph, rh2), rg2, rh2, mcw, lam));
+                const float gr = fmaxf(0.f, split_gain(parent, pg, ph, rg2, rh2, mcw, lam));
                 gn = gl > gr ? gl : -gr; keep_g = rg; keep_h = rh;
             } else {
                 const float lg = cell_f(eg[i], inv_sg), lh = cell_f(eh[i], inv_sh);
-                const float gr = fmaxf(0.f, split_gain(pg, ph, lg, lh, __fsub_rn(pg, lg), __fsub_rn(ph, lh), mcw, lam));
+                const float gr = fmaxf(0.f, split_gain(parent, pg, ph, lg, lh, mcw, lam));
                 const float lg2 = __fadd_rn(lg, mg), lh2 = __fadd_rn(lh, mh);
-                const float gl = fmaxf(0.f, split_gain(pg, ph, lg2, lh2, __fsub_rn(pg, lg2), __fsub_rn(ph, lh2), mcw, lam));
+                const float gl = fmaxf(0.f, split_gain(parent, pg, ph, lg2, lh2, mcw, lam));
                 gn = gl > gr ? gl : -gr; keep_g = lg; keep_h = lh;
             }
             if (best_bin < 0 || fabsf(gn) > fabsf(best)) { best = gn; best_bin = b0 + b; best_lg = keep_g; best_lh = keep_h; best_mg = mg; best_mh = mh; }
