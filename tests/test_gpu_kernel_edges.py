@@ -1,0 +1,96 @@
+"""Sizes at which the training kernels change over: edges of tiles, warps and shared memory, and the sizes on either side of
+the rules that choose between them.  Against the CPU oracle bit for bit, or against NumPy where the result is a plain count."""
+import numpy as np
+import pytest
+
+from thundergbm_b200.synth import CsrData
+
+pytestmark = pytest.mark.gpu
+
+
+def _csr(x, y):
+    n, f = x.shape
+    return CsrData(n, f, (np.arange(n + 1) * f).astype(np.int32), np.tile(np.arange(f, dtype=np.int32), n), np.ascontiguousarray(x, np.float32).ravel(),
+                   np.asarray(y, np.float32))
+
+
+def _holes(x, y, keep):
+    """The same with only the kept entries stored."""
+    n, f = x.shape
+    ptr = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    return CsrData(n, f, ptr, np.nonzero(keep)[1].astype(np.int32), np.ascontiguousarray(x[keep], np.float32), np.asarray(y, np.float32))
+
+
+def _data(n, f, classes, seed, holes=0.2, levels=40):
+    r = np.random.default_rng(seed)
+    x = r.integers(1, levels, (n, f)).astype(np.float32)   # few distinct values: ties and runs
+    y = r.integers(0, classes, n) if classes > 1 else x[:, 0] + 3 * (x[:, -1] > 20) + r.random(n)
+    return _holes(x, y, r.random((n, f)) >= holes) if holes else _csr(x, y)
+
+
+def _same_as_oracle(orc, d, **p):
+    from thundergbm_b200.booster import Booster
+    o = orc.train(d, hist_mode=1, keep_nid=0, **p)
+    b = Booster(d, hist_mode='exact', **p)
+    b.boost(p['n_trees'])
+    assert b.trees().tobytes() == o.trees.tobytes()
+    assert np.array_equal(b.ypred(), o.ypred)
+    assert np.array_equal(b.metrics(), o.metric)
+    b.close()
+
+
+# one cluster builds the tree up to 32768 rows, the level kernels from there on
+@pytest.mark.parametrize('n,f,depth,classes,extra', [
+    (1, 1, 1, 1, {}), (2, 3, 6, 1, {}), (31, 5, 4, 3, {}), (1023, 33, 6, 1, {}), (1025, 130, 9, 1, {}), (8191, 8, 10, 1, {}),
+    (3001, 600, 3, 1, {}), (4097, 17, 6, 7, dict(bagging=1, sample_seed=3)), (5000, 64, 7, 1, dict(column_sampling_rate=0.3, sample_seed=5)),
+    (32768, 20, 6, 1, {}), (32769, 20, 6, 1, {})])
+def test_small_trees(gpu, orc, n, f, depth, classes, extra):
+    d = _data(n, f, classes, n + f)
+    p = dict(depth=depth, n_trees=3, max_num_bin=64, learning_rate=0.5, objective='multi:softmax' if classes > 1 else 'reg:linear', num_class=classes, **extra)
+    _same_as_oracle(orc, d, **p)
+
+
+# tiles of 1024 entries, several columns in one and one column over several; groups that end at a tile's edge
+@pytest.mark.parametrize('n,f,depth,levels', [(1, 1, 2, 3), (1023, 1, 3, 500), (1024, 1, 6, 2), (1025, 2, 6, 10 ** 6), (512, 7, 4, 40), (300, 150, 9, 8),
+                                              (40_000, 3, 8, 10 ** 6)])
+@pytest.mark.parametrize('holes', [0, 0.5])
+def test_exact_splits(gpu, orc, n, f, depth, levels, holes):
+    d = _data(n, f, 1, 7 * n + f, holes, levels)
+    if holes:
+        d.y[: n // 3] = 0   # nodes that stop early: their entries leave
+    _same_as_oracle(orc, d, depth=depth, n_trees=3, learning_rate=0.5, objective='reg:linear', tree_method='exact')
+
+
+# from 2^21 rows on the columns of a full matrix are sorted one by one
+@pytest.mark.parametrize('n', [(1 << 21) - 1, 1 << 21, (1 << 21) + 4097])
+def test_cut_points_of_full_columns(gpu, n):
+    from thundergbm_b200.booster import Booster
+    r = np.random.default_rng(n)
+    x = np.stack([r.standard_normal(n), r.integers(-3, 4, n), np.full(n, -0.0), r.integers(0, 300, n) * 1e-3, np.linspace(-1, 1, n)], 1).astype(np.float32)
+    x[5, 2] = 0.0
+    b = Booster(_csr(x, x[:, 0]), depth=3, n_trees=1, max_num_bin=255, objective='reg:linear')
+    val, ptr = b.cuts()
+    for j in range(x.shape[1]):
+        u = np.unique(x[:, j])
+        s = len(u) // 255
+        want = u if s == 0 else u[np.arange(255) * s]
+        assert np.array_equal(val[ptr[j]:ptr[j + 1]], want)
+    b.close()
+
+
+# more rows per CTA than the 16-bit halves of one window hold: 149 groups of columns leave one CTA each
+def test_window_of_the_halved_sums(gpu):
+    from thundergbm_b200.booster import Booster
+    n, f = 70_001, 4 * 1200
+    r = np.random.default_rng(1)
+    cols = r.integers(1, 6, (n, 4)).astype(np.float32)
+    x = np.tile(cols, (1, f // 4))
+    b = Booster(_csr(x, 1e3 * cols[:, 0] + cols[:, 1]), depth=3, n_trees=3, max_num_bin=16, objective='reg:linear', hist_mode='fp32', keep_nid=1)
+    b.boost(3)
+    trees, nid = b.trees()[:, 0], b.nid().reshape(3, n)
+    for t in range(1, 3):   # hessian 1: a node's sum is its number of rows
+        for i in np.unique(nid[t]):
+            at, rows = int(i), nid[t] == i
+            assert trees[t, at]['sum_h'] == rows.sum()
+        assert trees[t, 0]['sum_h'] == n
+    b.close()

@@ -501,6 +501,7 @@ __device__ __forceinline__ float split_gain(float parent, float pg, float ph, fl
         return __fsub_rn(__fadd_rn(__fdiv_rn(__fmul_rn(g, g), __fadd_rn(h, lam)), __fdiv_rn(__fmul_rn(g2, g2), __fadd_rn(h2, lam))), parent);
     return 0.f;
 }
+
 // Per-node argmax over the features, SplitPoint decode and update_tree
 // (hist_tree_builder_single.cu:365-389 and :847-902).  Called by one whole warp for node n of the level.  The records
 // may have been written by other blocks of the running kernel: they are read past L1.
