@@ -119,9 +119,6 @@ __device__ __forceinline__ int hist_items(int level, const Batch &b, size_t tree
 // ascend inside every list, so at any time the whole GPU gathers rows from one moving window of the bin matrix:
 // DRAM pages and 64-byte sectors get shared between nodes.  A pure gather of 5.2 M of 10.5 M rows in 8 to 64 lists
 // takes 72 us this way and 100 to 110 us list after list.
-struct HistCursor {   // where a CTA stands in its list: item, remaining tiles of it, next tile = first record and records left from it
-    int w, w_end, left = 0, k = 1, width = 1, rr = 0, first = 0, rows = 0;
-};
 __device__ __forceinline__ void hist_share(const int *s_base, int w, int total, int n_shares, int &v0, int &k) {
     const unsigned half = (unsigned)total / 2, a = (unsigned)s_base[w] * (unsigned)n_shares + half, z = (unsigned)s_base[w + 1] * (unsigned)n_shares + half;
     v0 = (int)(a / (unsigned)total);
@@ -165,6 +162,7 @@ __device__ __forceinline__ void xor_permute_half(uint32_t (&w)[4], int key) {
 // node's histogram by one bulk reduction per feature (cp.reduce.async.bulk: the L2 takes whole lines; 148 CTAs flushing
 // 28 x 255 cells: 4.3 us into one node, 2.8 us into 64; 21.7 and 10.7 us as one RED.64 per cell and component, whose
 // lanes hit 32 different sectors).
+constexpr int HIST_SEQ = 32;                                           // tiles of a CTA laid down at a time
 constexpr int HIST_CELLS = 256 * 32;                                   // per component
 constexpr int HIST_STAGE = 256 * 16 + 16;                              // bytes of a feature's int64 pairs; the pad keeps 8 lanes' 16-byte stores in different banks
 constexpr int HIST_FINE_SMEM = 32 * HIST_STAGE;                        // 4 int32 accumulators per cell (128 KB), staged in place
@@ -175,17 +173,91 @@ __device__ __forceinline__ void bulk_add_u64(void *dst, const void *src, uint32_
                  ::"l"(dst), "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(bytes) : "memory");
 }
 
+// The rare parts of the kernel are functions of their own: inlined, their registers made the loop that adds up the rows
+// spill (64 registers per thread is all there is; 180 bytes spilled, 126 us per launch in exact mode at 10.5 M rows).
+
+// The CTA's t-th tile: first record, records (0 = no more), pair.
+struct HistTiles {
+    const int *s_base, *seg_begin, *seg_cnt;
+    const TreeNode *nodes;
+    int level, total, n_shares, va, vb, ib, ie, by_hessian;   // the CTA owns shares [va, vb), items ib .. ie may have some of them
+};
+__device__ __noinline__ int4 hist_tile(const HistTiles &x, int t) {
+    for (int w = x.ib; w <= x.ie; ++w) {
+        const int T = x.s_base[w + 1] - x.s_base[w];
+        if (!T) continue;
+        int v0, k;
+        hist_share(x.s_base, w, x.total, x.n_shares, v0, k);
+        const int ra = max(x.va, v0) - v0, width = min(x.vb, v0 + k) - v0 - ra;
+        if (width <= 0) continue;
+        const int n = (T / k) * width + min(max(T % k - ra, 0), width);   // the share's tiles: `width` neighbours of every k
+        if (t >= n) { t -= n; continue; }
+        const int at = (ra + (t / width) * k + t % width) * HIST_THREADS;
+        const int node = x.level == 0 ? 0 : 2 * w + built_side(x.level, w, x.seg_cnt, x.nodes, x.by_hessian);
+        return make_int4(x.seg_begin[node] + at, min(HIST_THREADS, x.seg_cnt[node] - at), w, 0);
+    }
+    return make_int4(0, 0, 0, 0);
+}
+
+// exact mode: int32 window -> int64 totals, same [bin][feature] layout
+__device__ __noinline__ void hist_drain(unsigned char *hist_sm, bool drained) {
+    int *acc = reinterpret_cast<int *>(hist_sm);
+    long long *tot = reinterpret_cast<long long *>(hist_sm + 2 * HIST_CELLS * 4);
+    __syncthreads();
+#pragma unroll 4
+    for (int i = threadIdx.x; i < 2 * HIST_CELLS; i += HIST_THREADS) {
+        const int v = acc[i];
+        tot[i] = drained ? tot[i] + v : v;
+        acc[i] = 0;
+    }
+    __syncthreads();
+}
+
+// the CTA's sums of a node to its histogram; dst, nb: first cell and bins of the lane's feature
+template <bool FINE>
+__device__ __noinline__ void hist_flush(unsigned char *hist_sm, long long *dst, int nb, bool drained, bool again) {
+    const int lane = threadIdx.x & 31;
+    int *acc = reinterpret_cast<int *>(hist_sm), *high = acc + 2 * HIST_CELLS;
+    unsigned char *stage = hist_sm + (FINE ? 0 : 2 * HIST_CELLS * 4);
+    const long long *tot = reinterpret_cast<const long long *>(stage);
+    long long vg[8], vh[8];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int s = ((threadIdx.x >> 5) + 32 * q) * 32 + lane;
+        if (FINE) {
+            vg[q] = ((long long)high[s] << 16) + (unsigned)acc[s]; vh[q] = ((long long)high[HIST_CELLS + s] << 16) + (unsigned)acc[HIST_CELLS + s];
+        } else {
+            vg[q] = acc[s]; vh[q] = acc[HIST_CELLS + s];
+            if (drained) { vg[q] += tot[s]; vh[q] += tot[HIST_CELLS + s]; }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<longlong2 *>(stage + lane * HIST_STAGE + ((threadIdx.x >> 5) + 32 * q) * 16) = make_longlong2(vg[q], vh[q]);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        if (nb > 0) bulk_add_u64(dst, stage + lane * HIST_STAGE, (uint32_t)nb * 16);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
+    if (!again) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < (FINE ? 4 : 2) * HIST_CELLS * 4 / 16; i += HIST_THREADS) reinterpret_cast<int4 *>(hist_sm)[i] = make_int4(0, 0, 0, 0);
+    __syncthreads();
+}
+
 template <bool GATHER, bool FINE>
 static __global__ void __launch_bounds__(HIST_THREADS, 1)
 k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpad, int F, const int *__restrict__ cut_ptr, int B,
        int window_rows, int by_hessian, int tree0) {
     extern __shared__ __align__(128) unsigned char hist_sm[];
     int *acc = reinterpret_cast<int *>(hist_sm);          // g, h (FINE: low halves)
-    int *high = acc + 2 * HIST_CELLS;                     // FINE: high halves of g, h
-    unsigned char *stage = hist_sm + (FINE ? 0 : 2 * HIST_CELLS * 4);
-    long long *tot = reinterpret_cast<long long *>(stage);  // !FINE: totals of g, then h, [bin][feature]
     int *s_base = reinterpret_cast<int *>(hist_sm + (FINE ? HIST_FINE_SMEM : HIST_EXACT_SMEM));
     __shared__ int scratch[33], s_ib, s_ie;
+    __shared__ int4 s_seq[HIST_SEQ + 4];
     const int group = blockIdx.y, f0 = group * 32, nf = min(32, F - f0), lane = threadIdx.x & 31;
     const size_t tree = tree0 + blockIdx.z;
     constexpr int ZERO_BYTES = FINE ? 4 * HIST_CELLS * 4 : 2 * HIST_CELLS * 4;   // the accumulators
@@ -207,79 +279,23 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
         if (v0 < vb && v0 + k > va) { atomicMin(&s_ib, w); atomicMax(&s_ie, w); }
     }
     __syncthreads();
-    HistCursor c;
-    c.w = s_ib - 1; c.w_end = s_ie;
-    if (c.w_end < 0) return;
-    auto next = [&]() -> int3 {   // (first record, records, pair) of the CTA's next tile; records = 0 at the end
-        while (c.left == 0) {
-            if (++c.w > c.w_end) { c.w = c.w_end; return make_int3(0, 0, 0); }
-            const int T = s_base[c.w + 1] - s_base[c.w];
-            if (!T) continue;
-            int v0, k;
-            hist_share(s_base, c.w, total, n_shares, v0, k);
-            const int ra = max(va, v0) - v0, width = min(vb, v0 + k) - v0 - ra;
-            if (width <= 0) continue;
-            c.left = (T / k) * width + min(max(T % k - ra, 0), width);
-            c.k = k; c.width = width; c.rr = 0;
-            const int node = level == 0 ? 0 : 2 * c.w + built_side(level, c.w, seg_cnt, nodes, by_hessian);
-            c.first = seg_begin[node] + ra * HIST_THREADS; c.rows = seg_cnt[node] - ra * HIST_THREADS;
-        }
-        --c.left;
-        const int3 e = make_int3(c.first, min(HIST_THREADS, c.rows), c.w);
-        int step = HIST_THREADS;   // the share's tiles: `width` neighbours of every k
-        if (++c.rr == c.width) { c.rr = 0; step += (c.k - c.width) * HIST_THREADS; }
-        c.first += step; c.rows -= step;
-        return e;
-    };
+    if (s_ie < 0) return;
+    // HIST_SEQ tiles at a time are laid down in shared memory
+    const HistTiles tiles{s_base, seg_begin, seg_cnt, nodes, level, total, n_shares, va, vb, s_ib, s_ie, by_hessian};
+    int seq0 = 0;   // position of s_seq[0]
+    if (threadIdx.x < HIST_SEQ + 4) s_seq[threadIdx.x] = hist_tile(tiles, (int)threadIdx.x);
+    __syncthreads();
 
     const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
     const int2 *rec_gh = GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride;
     long long *slab = b.hist_built + tree * b.built_stride;
 
     bool drained = false;   // the totals hold something: few rows per node and CTA need none, so they are not zeroed either
-    auto drain = [&]() {  // int32 window -> int64 totals, same [bin][feature] layout
-        __syncthreads();
-#pragma unroll 4
-        for (int i = threadIdx.x; i < 2 * HIST_CELLS; i += HIST_THREADS) {
-            const int v = acc[i];
-            tot[i] = drained ? tot[i] + v : v;
-            acc[i] = 0;
-        }
-        __syncthreads();
-        drained = true;
-    };
     const int flush_b0 = lane < nf ? cut_ptr[f0 + lane] : 0;   // first bin of this lane's feature
     const int flush_nb = lane < nf ? cut_ptr[f0 + lane + 1] - flush_b0 : 0;
     auto flush = [&](int pair, bool again) {
-        long long vg[8], vh[8];
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int s = ((threadIdx.x >> 5) + 32 * q) * 32 + lane;
-            if (FINE) {
-                vg[q] = ((long long)high[s] << 16) + (unsigned)acc[s]; vh[q] = ((long long)high[HIST_CELLS + s] << 16) + (unsigned)acc[HIST_CELLS + s];
-            } else {
-                vg[q] = acc[s]; vh[q] = acc[HIST_CELLS + s];
-                if (drained) { vg[q] += tot[s]; vh[q] += tot[HIST_CELLS + s]; }
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-            *reinterpret_cast<longlong2 *>(stage + lane * HIST_STAGE + ((threadIdx.x >> 5) + 32 * q) * 16) = make_longlong2(vg[q], vh[q]);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            if (flush_nb > 0) bulk_add_u64(slab + ((size_t)pair * B + flush_b0) * 2, stage + lane * HIST_STAGE, (uint32_t)flush_nb * 16);
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        }
-        if (!again) return;
-        __syncthreads();
-        for (int i = threadIdx.x; i < ZERO_BYTES / 16; i += HIST_THREADS)
-            reinterpret_cast<int4 *>(hist_sm)[i] = make_int4(0, 0, 0, 0);
+        hist_flush<FINE>(hist_sm, slab + ((size_t)pair * B + flush_b0) * 2, flush_nb, drained, again);
         drained = false;
-        __syncthreads();
     };
 
     // Two lanes share a row: lane l loads the 16-byte half (l & 1) of the rows at tile positions
@@ -291,51 +307,59 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
     // way into registers, those of tile i+2 have been asked into L2 (a prefetch holds no register), and the row ids
     // of tile i+3 are being fetched.  The gather levels are bound by the bytes in flight (a loaded DRAM access takes
     // 2-3 us here): one tile per warp in registers alone sustains only ~2.4 TB/s of sector traffic.
-    auto ids = [&](const int3 &e, int &ra, int &rb) {   // row ids of the lane's two positions, -1 = no record
+    auto ids = [&](int i, int &ra, int &rb) {   // row ids of the lane's two positions in tile i, -1 = no record
+        const int4 e = s_seq[i - seq0];
         ra = qa < e.y ? (GATHER ? rec_idx[e.x + qa] : e.x + qa) : -1;
         rb = qb < e.y ? (GATHER ? rec_idx[e.x + qb] : e.x + qb) : -1;
     };
     const size_t half_off = (size_t)f0 + 16u * (lane & 1);
     uint4 na = make_uint4(0, 0, 0, 0), nb = na;
     int2 nva = make_int2(0, 0), nvb = nva;
-    auto load_rows = [&](const int3 &e, int ra, int rb) {
-        if (ra >= 0) { na = *reinterpret_cast<const uint4 *>(bins + (size_t)ra * Fpad + half_off); nva = rec_gh[e.x + qa]; }
-        if (rb >= 0) { nb = *reinterpret_cast<const uint4 *>(bins + (size_t)rb * Fpad + half_off); nvb = rec_gh[e.x + qb]; }
+    int r1a, r1b, r2a, r2b, pair_next = 0;
+    bool noka = false, nokb = false;
+    auto load_rows = [&](int i) {   // rows of tile i (ids r1a, r1b) -> registers
+        const int4 e = s_seq[i - seq0];
+        pair_next = e.z;
+        noka = r1a >= 0; nokb = r1b >= 0;
+        if (noka) { na = *reinterpret_cast<const uint4 *>(bins + (size_t)r1a * Fpad + half_off); nva = rec_gh[e.x + qa]; }
+        if (nokb) { nb = *reinterpret_cast<const uint4 *>(bins + (size_t)r1b * Fpad + half_off); nvb = rec_gh[e.x + qb]; }
     };
-    auto prefetch_rows = [&](int ra, int rb) {  // one lane of each pair asks for the row's sector
+    auto prefetch_rows = [&]() {  // rows with ids r2a, r2b -> L2; one lane of each pair asks for the row's sector
         if (GATHER && !(lane & 1)) {
-            if (ra >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(bins + (size_t)ra * Fpad + f0));
-            if (rb >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(bins + (size_t)rb * Fpad + f0));
+            if (r2a >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(bins + (size_t)r2a * Fpad + f0));
+            if (r2b >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(bins + (size_t)r2b * Fpad + f0));
         }
     };
-    int3 e0 = next(), e1 = next(), e2 = next();
-    if (e0.y == 0) return;   // more shares than tiles
-    int r1a, r1b, r2a, r2b;
-    ids(e0, r1a, r1b);
-    ids(e1, r2a, r2b);
-    load_rows(e0, r1a, r1b);
-    prefetch_rows(r2a, r2b);
-    bool noka = r1a >= 0, nokb = r1b >= 0;
+    if (s_seq[0].y == 0) return;   // more shares than tiles
+    ids(0, r1a, r1b);
+    ids(1, r2a, r2b);
+    load_rows(0);
+    prefetch_rows();
     r1a = r2a; r1b = r2b;
-    ids(e2, r2a, r2b);
-    int pair_cur = e0.z, since = 0;
-    while (e0.y > 0) {
+    ids(2, r2a, r2b);
+    int pair_cur = pair_next, since = 0;
+    for (int i = 0; s_seq[i - seq0].y > 0; ++i) {
         const uint4 a = na, bb = nb;
         const int2 va2 = nva, vb2 = nvb;
         const bool oka = noka, okb = nokb;
-        const int pair_this = e0.z;
-        e0 = e1; e1 = e2; e2 = next();
-        load_rows(e0, r1a, r1b);
-        noka = r1a >= 0; nokb = r1b >= 0;
-        prefetch_rows(r2a, r2b);
+        const int pair_this = pair_next;
+        load_rows(i + 1);
+        prefetch_rows();
         r1a = r2a; r1b = r2b;
-        ids(e2, r2a, r2b);
+        ids(i + 3, r2a, r2b);
+        if (i + 1 - seq0 == HIST_SEQ) {
+            __syncthreads();
+            seq0 = i + 1;
+            if (threadIdx.x < HIST_SEQ + 4) s_seq[threadIdx.x] = hist_tile(tiles, seq0 + (int)threadIdx.x);
+            __syncthreads();
+        }
         if (pair_this != pair_cur || (FINE && since + HIST_THREADS > FINE_WINDOW)) {  // another node: hand the finished one over
             flush(pair_cur, true);
             pair_cur = pair_this;
             since = 0;
         } else if (!FINE && since + HIST_THREADS > window_rows) {
-            drain();
+            hist_drain(hist_sm, drained);
+            drained = true;
             since = 0;
         }
         since += HIST_THREADS;
