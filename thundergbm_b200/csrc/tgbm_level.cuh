@@ -176,12 +176,15 @@ __device__ __forceinline__ void bulk_add_u64(void *dst, const void *src, uint32_
 // The rare parts of the kernel are functions of their own: inlined, their registers made the loop that adds up the rows
 // spill (64 registers per thread is all there is; 180 bytes spilled, 126 us per launch in exact mode at 10.5 M rows).
 
-// The CTA's t-th tile: first record, records (0 = no more), pair.
+// What they need stands in shared memory for the same reason.
 struct HistTiles {
-    const int *s_base, *seg_begin, *seg_cnt;
+    const int *s_base, *seg_begin, *seg_cnt, *cut_ptr;
     const TreeNode *nodes;
+    long long *slab;
     int level, total, n_shares, va, vb, ib, ie, by_hessian;   // the CTA owns shares [va, vb), items ib .. ie may have some of them
+    int f0, nf, B;                                            // first feature of the group, features, bins of all features
 };
+// the CTA's t-th tile: first record, records (0 = no more), pair
 __device__ __noinline__ int4 hist_tile(const HistTiles &x, int t) {
     for (int w = x.ib; w <= x.ie; ++w) {
         const int T = x.s_base[w + 1] - x.s_base[w];
@@ -213,9 +216,9 @@ __device__ __noinline__ void hist_drain(unsigned char *hist_sm, bool drained) {
     __syncthreads();
 }
 
-// the CTA's sums of a node to its histogram; dst, nb: first cell and bins of the lane's feature
+// the CTA's sums of a pair's built node to its histogram
 template <bool FINE>
-__device__ __noinline__ void hist_flush(unsigned char *hist_sm, long long *dst, int nb, bool drained, bool again) {
+__device__ __noinline__ void hist_flush(const HistTiles &x, unsigned char *hist_sm, int pair, bool drained, bool again) {
     const int lane = threadIdx.x & 31;
     int *acc = reinterpret_cast<int *>(hist_sm), *high = acc + 2 * HIST_CELLS;
     unsigned char *stage = hist_sm + (FINE ? 0 : 2 * HIST_CELLS * 4);
@@ -239,7 +242,8 @@ __device__ __noinline__ void hist_flush(unsigned char *hist_sm, long long *dst, 
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32) {
-        if (nb > 0) bulk_add_u64(dst, stage + lane * HIST_STAGE, (uint32_t)nb * 16);
+        const int b0 = lane < x.nf ? x.cut_ptr[x.f0 + lane] : 0, nb = lane < x.nf ? x.cut_ptr[x.f0 + lane + 1] - b0 : 0;   // the lane's feature
+        if (nb > 0) bulk_add_u64(x.slab + ((size_t)pair * x.B + b0) * 2, stage + lane * HIST_STAGE, (uint32_t)nb * 16);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
@@ -258,7 +262,8 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
     int *s_base = reinterpret_cast<int *>(hist_sm + (FINE ? HIST_FINE_SMEM : HIST_EXACT_SMEM));
     __shared__ int scratch[33], s_ib, s_ie;
     __shared__ int4 s_seq[HIST_SEQ + 4];
-    const int group = blockIdx.y, f0 = group * 32, nf = min(32, F - f0), lane = threadIdx.x & 31;
+    __shared__ HistTiles tiles;
+    const int group = blockIdx.y, f0 = group * 32, lane = threadIdx.x & 31;
     const size_t tree = tree0 + blockIdx.z;
     constexpr int ZERO_BYTES = FINE ? 4 * HIST_CELLS * 4 : 2 * HIST_CELLS * 4;   // the accumulators
     for (int i = threadIdx.x; i < ZERO_BYTES / 16; i += HIST_THREADS)
@@ -281,22 +286,18 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
     __syncthreads();
     if (s_ie < 0) return;
     // HIST_SEQ tiles at a time are laid down in shared memory
-    const HistTiles tiles{s_base, seg_begin, seg_cnt, nodes, level, total, n_shares, va, vb, s_ib, s_ie, by_hessian};
+    if (threadIdx.x == 0)
+        tiles = HistTiles{s_base, seg_begin, seg_cnt, cut_ptr, nodes, b.hist_built + tree * b.built_stride, level, total, n_shares, va, vb, s_ib, s_ie, by_hessian,
+                          f0, min(32, F - f0), B};
+    __syncthreads();
     int seq0 = 0;   // position of s_seq[0]
     if (threadIdx.x < HIST_SEQ + 4) s_seq[threadIdx.x] = hist_tile(tiles, (int)threadIdx.x);
     __syncthreads();
 
     const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
     const int2 *rec_gh = GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride;
-    long long *slab = b.hist_built + tree * b.built_stride;
 
     bool drained = false;   // the totals hold something: few rows per node and CTA need none, so they are not zeroed either
-    const int flush_b0 = lane < nf ? cut_ptr[f0 + lane] : 0;   // first bin of this lane's feature
-    const int flush_nb = lane < nf ? cut_ptr[f0 + lane + 1] - flush_b0 : 0;
-    auto flush = [&](int pair, bool again) {
-        hist_flush<FINE>(hist_sm, slab + ((size_t)pair * B + flush_b0) * 2, flush_nb, drained, again);
-        drained = false;
-    };
 
     // Two lanes share a row: lane l loads the 16-byte half (l & 1) of the rows at tile positions
     // warp*32 + (l >> 1) ("A") and 16 further on ("B").  One load instruction of a warp therefore touches 16 rows
@@ -354,7 +355,8 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
             __syncthreads();
         }
         if (pair_this != pair_cur || (FINE && since + HIST_THREADS > FINE_WINDOW)) {  // another node: hand the finished one over
-            flush(pair_cur, true);
+            hist_flush<FINE>(tiles, hist_sm, pair_cur, drained, true);
+            drained = false;
             pair_cur = pair_this;
             since = 0;
         } else if (!FINE && since + HIST_THREADS > window_rows) {
@@ -393,7 +395,7 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
         if (oka) add_row(a, va2);
         if (okb) add_row(bb, vb2);
     }
-    flush(pair_cur, false);
+    hist_flush<FINE>(tiles, hist_sm, pair_cur, drained, false);
 }
 
 // ------------------------------------------------------------------ histogram build, CSR of global bin ids
