@@ -11,7 +11,8 @@ launched by torch.distributed.run) and the total work stays fixed ("strong" scal
 Prints one JSON line on rank 0:
   value     seconds per 100 boosting rounds for the boosting loop with the bin matrix resident in HBM (the scope of
             the reference's own "training time" line, src/thundergbm/trainer.cu:42-50), in the library's default
-            histogram arithmetic (fp32: the reference's own, one float accumulator per bin)
+            histogram arithmetic (fp32: float sums value by value in the first round, like the reference, then
+            integer sums of the float gradients on a grid of 2^-30 of the largest)
   deterministic_mode   the same loop in the exact fixed-point mode (bit-identical from run to run and for any number
             of GPUs), with the roofline of its histogram kernel
   e2e       the same unit through the reference's C entry point (sparse_train_scikit) with host CSR buffers: copies,
@@ -419,7 +420,7 @@ def main():
         hist_gbs = gbs(prof.hist_bytes, prof.hist_ms)
         root_gbs = gbs(prof.hist_root_bytes, prof.hist_root_ms)
         part_gbs = gbs(prof.partition_bytes, prof.partition_ms)
-        kernel = {'fp32': 'k_hist_f32 (one float accumulator per bin, vector reductions in L2; all levels)',
+        kernel = {'fp32': 'k_hist (shared-memory integer sums of the float gradients on a 2^-30 grid; all levels)',
                   'exact': 'k_hist (shared-memory integer histograms; all levels)'}[mode]
         if info.csr_layout:
             kernel = kernel.replace('k_hist', 'k_hist_sparse')
@@ -431,14 +432,15 @@ def main():
                 'hist_share_of_step': prof.hist_ms / ms_prof if ms_prof > 0 else None,
                 'partition_share_of_step': prof.partition_ms / ms_prof if ms_prof > 0 else None,
                 'measured_on': f'{k_prof} rounds directly after the timed region, per-kernel CUDA events (ms_per_step there {ms_prof / k_prof:.3f})'}
-        if mode == 'fp32':
-            # the kernel is bound by the rate at which the L2 performs float reductions, not by HBM: say so with numbers
-            reds = float(prof.hist_rows) * data.nnz / max(1, data.n_rows)  # one reduction per stored value of a processed row
-            roof['limiter'] = 'L2 float-reduction rate (one red.global.add.v2.f32 per stored value of a row)'
-            roof['reductions_per_s'] = reds / (prof.hist_ms * 1e-3) if prof.hist_ms > 0 else None
-            roof['reduction_peak_per_s'] = 191e9
-            roof['limiter_frac'] = roof['reductions_per_s'] / 191e9 if roof['reductions_per_s'] else None
-            roof['reduction_peak_kind'] = 'microbenchmark on this pool: 10.5 M rows x 28 bare reductions into cells 256 bytes apart (1, 8 or 64 nodes: 190-192 G/s)'
+        # the kernel is bound by its shared-memory atomics, not by HBM: one 32-bit atomic per component and (row, feature) in
+        # exact mode, two (low and high half of a 31-bit value) in fp32 mode
+        pair_peak = {'fp32': 294e6 / 0.134e-3, 'exact': 294e6 / 0.073e-3}[mode]
+        pairs = float(prof.hist_rows) * data.nnz / max(1, data.n_rows)  # (row, feature) pairs of the processed rows
+        roof['limiter'] = 'shared-memory atomics (%d per row and feature)' % (4 if mode == 'fp32' else 2)
+        roof['pairs_per_s'] = pairs / (prof.hist_ms * 1e-3) if prof.hist_ms > 0 else None
+        roof['pair_peak_per_s'] = pair_peak
+        roof['limiter_frac'] = roof['pairs_per_s'] / pair_peak if roof['pairs_per_s'] else None
+        roof['pair_peak_kind'] = 'microbenchmark on this pool: the bare atomics of 294 M (row, feature) pairs, conflict-free'
         return dict(ms_max=ms_max, launches=launches_timed, roofline=roof, t_init=t_init, info=info, trees=trees, logloss=ll,
                     final_metric=float(metrics_timed[w + k - 1]) if len(metrics_timed) >= w + k else None)
 
@@ -512,7 +514,8 @@ def main():
         'n_gpus': world, 'steps': k, 'warmup': w, 'ms_per_step': head['ms_max'] / k, 'higher_is_better': False,
         'scaling': 'strong', 'vs_baseline': None, 'dtype': 'f32' if head_mode == 'fp32' else 'i64', 'data': 'synthetic',
         'config': {'workload': wl, 'config': args.config, 'hist_mode': head_mode,
-                   'hist_mode_note': 'fp32 = float (g,h) added value by value into one accumulator per bin, the reference\'s arithmetic; '
+                   'hist_mode_note': 'fp32 = first round as the reference adds (floats, value by value into one accumulator per bin), later rounds '
+                                     'integer sums of the float gradients on a 2^-30 grid; '
                                      'exact = integer sums on a fixed-point grid (deterministic)',
                    'rows_per_gpu': hi - lo, 'parallelism': f'rows sharded over {world} GPU(s), NCCL all-reduce of level histograms',
                    'l2': 'inputs larger than L2 (bin data %.0f MB per GPU)' % (max(data.nnz, (hi - lo) * info.fpad) / 1e6),
