@@ -94,3 +94,29 @@ def test_window_of_the_halved_sums(gpu):
             assert trees[t, at]['sum_h'] == rows.sum()
         assert trees[t, 0]['sum_h'] == n
     b.close()
+
+
+# column ids travel as 16-bit numbers where all of them fit; page-locked arrays are copied as they are
+@pytest.mark.parametrize('top', [65535, 65536])
+def test_column_ids_of_a_large_csr(gpu, top):
+    import torch
+    from thundergbm_b200.booster import Booster
+    r = np.random.default_rng(top)
+    n = 150_001
+    col = np.sort(r.choice(2000, (n, 5), replace=True) * 2 + np.arange(5), 1).astype(np.int32)
+    keep = np.concatenate([np.ones((n, 1), bool), np.diff(col, axis=1) > 0], 1)
+    keep[0] = True
+    col[0] = [0, 1, 2, 3, 4]
+    col[n // 2, -1] = top
+    keep[n // 2] = [True, False, False, False, True]
+    d = _holes(r.integers(1, 9, (n, 5)).astype(np.float32), col[:, 0] % 7 + r.random(n), keep)
+    d.n_cols, d.col = top + 1, col[keep]
+    pinned = CsrData(n, top + 1, *[torch.from_numpy(a).pin_memory().numpy() for a in (d.row_ptr, d.col, d.val, d.y)])
+    got = []
+    for data in (d, pinned):
+        b = Booster(data, depth=4, n_trees=2, max_num_bin=16, objective='reg:linear', hist_mode='exact')
+        b.boost(2)
+        assert b.info.n_features == top + 1
+        got.append((b.trees().tobytes(), b.ypred().tobytes()))
+        b.close()
+    assert got[0] == got[1]

@@ -25,6 +25,9 @@ void dev_release_all() noexcept;
 // host -> device copy that also runs at the speed of the link when the source is pageable memory (then it returns
 // when the data is on the device; from page-locked memory it is cudaMemcpyAsync on `stream`)
 void upload_h2d(void *dst, const void *src, size_t bytes, cudaStream_t stream, int n_threads);
+// Ints from pageable host memory as 16-bit ones; false (nothing usable on the device) when one does not fit, or where the
+// staging threads are not used.  The staged copy of a CSR is bound by host memory and the link: half the bytes of the ids.
+bool upload_ids16(uint16_t *dst, const int *src, size_t n, int n_threads);
 // The values of a CSR, the same way; true when every row stores the columns 0 .. n_cols - 1 in order (a dense matrix handed
 // over as CSR): the column ids and row pointers then say nothing and need not follow.  They are checked by the host threads
 // while the values are copied: reading them costs less than sending them (half of the bytes of such a CSR).

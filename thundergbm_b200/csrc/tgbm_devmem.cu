@@ -24,6 +24,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstdlib>
+#include <cstdint>
 #include <cstring>
 #include <deque>
 #include <functional>
@@ -253,6 +254,35 @@ void copy_past_cache(void *dst, const void *src, size_t n) {
     memcpy(dst, src, n);
 }
 
+// the low halves of n ints; false if one of them does not fit 16 bits
+#if defined(__x86_64__)
+__attribute__((target("avx2"))) bool copy_low16_avx2(uint16_t *dst, const int *src, size_t n) {   // dst on a 32-byte boundary
+    __m256i high = _mm256_setzero_si256();
+    const __m256i mask = _mm256_set1_epi32((int)0xffff0000u);
+    size_t i = 0;
+    for (; i + 32 <= n; i += 32) {
+        const __m256i a = _mm256_loadu_si256((const __m256i *)(src + i)), b = _mm256_loadu_si256((const __m256i *)(src + i + 8));
+        const __m256i c = _mm256_loadu_si256((const __m256i *)(src + i + 16)), d = _mm256_loadu_si256((const __m256i *)(src + i + 24));
+        high = _mm256_or_si256(high, _mm256_and_si256(mask, _mm256_or_si256(_mm256_or_si256(a, b), _mm256_or_si256(c, d))));
+        _mm256_stream_si256((__m256i *)(dst + i), _mm256_permute4x64_epi64(_mm256_packus_epi32(a, b), 0xd8));
+        _mm256_stream_si256((__m256i *)(dst + i + 16), _mm256_permute4x64_epi64(_mm256_packus_epi32(c, d), 0xd8));
+    }
+    _mm_sfence();
+    int rest = 0;
+    for (; i < n; ++i) { dst[i] = (uint16_t)src[i]; rest |= src[i]; }
+    return _mm256_testz_si256(high, high) && !((unsigned)rest >> 16);
+}
+#endif
+bool copy_low16(uint16_t *dst, const int *src, size_t n) {
+#if defined(__x86_64__)
+    static const bool avx2 = __builtin_cpu_supports("avx2");
+    if (avx2) return copy_low16_avx2(dst, src, n);
+#endif
+    int all = 0;
+    for (size_t i = 0; i < n; ++i) { dst[i] = (uint16_t)src[i]; all |= src[i]; }
+    return !((unsigned)all >> 16);
+}
+
 struct Worker {
     Lane lanes[MAX_DEVICES];
     Lane &lane(int dev) {
@@ -314,6 +344,8 @@ struct Transfer {
     char *host;                // host side (read when up, written when down)
     size_t bytes, piece;
     bool up;
+    bool narrow = false;       // up: the host side is ints, the device side their low halves
+    std::atomic<bool> fits{true};
     std::atomic<size_t> next{0};
     Transfer(void *d, const void *h, size_t n, bool up_, int workers)
         : dev(static_cast<char *>(d)), host(static_cast<char *>(const_cast<void *>(h))), bytes(n), up(up_) {
@@ -333,7 +365,8 @@ struct Transfer {
             const size_t len = std::min(piece, bytes - off);
             finish(k);
             if (up) {
-                copy_past_cache(slot[k], host + off, len);
+                if (!narrow) copy_past_cache(slot[k], host + off, len);
+                else if (!fits || !copy_low16(static_cast<uint16_t *>(slot[k]), reinterpret_cast<const int *>(host + 2 * off), len / 2)) { fits = false; break; }
                 check_cuda(cudaMemcpyAsync(dev + off, slot[k], len, cudaMemcpyHostToDevice, l.st), "cudaMemcpyAsync");
             } else {
                 check_cuda(cudaMemcpyAsync(slot[k], dev + off, len, cudaMemcpyDeviceToHost, l.st), "cudaMemcpyAsync");
@@ -410,6 +443,16 @@ void upload_h2d(void *dst, const void *src, size_t bytes, cudaStream_t stream, i
     }
     Transfer tr(dst, src, bytes, true, n_threads);
     run_staged(&tr, n_threads, {});   // the pieces are on the device when the workers return: whatever is queued next sees them
+}
+
+bool upload_ids16(uint16_t *dst, const int *src, size_t n, int n_threads) {
+    if (!staging_on() || sizeof(uint16_t) * n < STAGE_MIN || n_threads < 1 || !host_is_pageable(src)) return false;
+    for (size_t i = 0; i < n; i += n / 64 + 1)
+        if ((unsigned)src[i] > 0xffffu) return false;   // a glance first
+    Transfer tr(dst, src, sizeof(uint16_t) * n, true, n_threads);
+    tr.narrow = true;
+    run_staged(&tr, n_threads, {});
+    return tr.fits;
 }
 
 bool upload_csr_values(float *dst, const float *val, const int *row_ptr, const int *col, int n_rows, int n_cols, cudaStream_t stream, int n_threads) {

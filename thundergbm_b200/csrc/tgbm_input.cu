@@ -66,6 +66,10 @@ static __global__ void k_full_row_ptr(int *__restrict__ row_ptr, int n, int c) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) row_ptr[i] = i * c;
 }
 
+static __global__ void k_widen_ids(const uint16_t *__restrict__ in, size_t n, int *__restrict__ out) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) out[i] = in[i];
+}
+
 // The largest and smallest column index are found on the device, at HBM speed, instead of by a pass over the host copy.
 void DeviceRows::upload(const DataSet &ds, cudaStream_t stream, int num_sms, int up_threads) {
     const int N = ds.n_rows;
@@ -83,7 +87,16 @@ void DeviceRows::upload(const DataSet &ds, cudaStream_t stream, int num_sms, int
     }
     row_ptr.alloc(N + 1); col.alloc(std::max<size_t>(nnz, 1));
     upload_h2d(row_ptr.p, ds.rp, sizeof(int) * (size_t)(N + 1), stream, up_threads);
-    upload_h2d(col.p, ds.ci, sizeof(int) * nnz, stream, up_threads);
+    {
+        DevBuf<uint16_t> narrow;
+        narrow.alloc(std::max<size_t>(nnz, 1));
+        if (upload_ids16(narrow.p, ds.ci, nnz, up_threads)) {
+            k_widen_ids<<<(int)std::min<size_t>((nnz + 255) / 256, (size_t)num_sms * 16), 256, 0, stream>>>(narrow.p, nnz, col.p);
+            TGBM_CUDA(cudaStreamSynchronize(stream));
+        } else {
+            upload_h2d(col.p, ds.ci, sizeof(int) * nnz, stream, up_threads);
+        }
+    }
     if (nnz) {
         DevBuf<int> d_mm;
         d_mm.alloc(2);
