@@ -136,9 +136,9 @@ struct BoosterImpl {
     DevBuf<unsigned> ex_key[3];
     DevBuf<int> ex_row[3];
     DevBuf<float> ex_val[3];
-    DevBuf<unsigned char> ex_pre, ex_tile_sum, ex_tile_pre;   // prefix sums: see k_exact_sum
+    DevBuf<unsigned char> ex_pre, ex_tile_pre, ex_run;   // prefix sums: see k_exact_sum; ex_run: sums and prefixes of the blocks' runs
     DevBuf<unsigned> ex_lr;
-    DevBuf<ExPair<int>> ex_tile_cnt, ex_tile_lr;
+    DevBuf<ExPair<int>> ex_tile_lr, ex_run_lr;
     DevBuf<int2> ex_group, ex_gh[3];                // (group ranges; gradient pairs of the entries, float or quantised)
     DevBuf<uint2> ex_side;
     DevBuf<int> ex_live, ex_nid, ex_any, ex_ticket;   // ex_live[level]: entries of the level
@@ -642,8 +642,8 @@ void BoosterImpl::init_exact() {
     cut_ptr.zero(stream);
     const size_t max_nl = (size_t)1 << std::max(0, depth - 1);
     const size_t v = f32 ? sizeof(double) : sizeof(int), w = 8;
-    ex_pre.alloc(2 * v * padded); ex_tile_sum.alloc(2 * w * tiles); ex_tile_pre.alloc(2 * w * tiles);
-    ex_lr.alloc(padded); ex_tile_cnt.alloc(tiles); ex_tile_lr.alloc(tiles);
+    ex_pre.alloc(2 * v * padded); ex_tile_pre.alloc(2 * w * tiles); ex_run.alloc(2 * 2 * w * num_sms * 8);
+    ex_lr.alloc(padded); ex_tile_lr.alloc(tiles); ex_run_lr.alloc(2 * num_sms * 8);
     ex_group.alloc((size_t)F * max_nl + 1);
     ex_live.alloc(depth + 1);
     const int live = (int)nnz;
@@ -673,15 +673,16 @@ void BoosterImpl::exact_levels(int k, const void *gh_rows) {
     const int grid = std::max(1, std::min(ceil_div(ex_nnz, EX_TILE), num_sms * 8));
     const int row_grid = std::max(1, std::min(ceil_div(std::max(N, 1), 256), num_sms * 8));
     ExPair<V> *pre = reinterpret_cast<ExPair<V> *>(ex_pre.p);
-    ExPair<W> *tile_sum = reinterpret_cast<ExPair<W> *>(ex_tile_sum.p), *tile_pre = reinterpret_cast<ExPair<W> *>(ex_tile_pre.p);
+    ExPair<W> *tile_pre = reinterpret_cast<ExPair<W> *>(ex_tile_pre.p), *run_sum = reinterpret_cast<ExPair<W> *>(ex_run.p), *run_pre = run_sum + num_sms * 8;
+    ExPair<int> *run_cnt = ex_run_lr.p, *run_lr = ex_run_lr.p + num_sms * 8;
     typedef typename ExKind<T>::In In;
     auto gh_of = [&](int i) { return reinterpret_cast<In *>(ex_gh[i].p); };
     for (int level = 0; level < depth; ++level) {
         const int nl = 1 << level, a = level == 0 ? 0 : 1 + (level & 1), z = 1 + ((level + 1) & 1);   // this level's entries, the next one's
         const int *live = ex_live.p + level;
         launch_after(level == 0 ? k_exact_sum<T, true> : k_exact_sum<T, false>, grid, EX_THREADS, 0, stream, live, ex_key[a].p, ex_row[a].p,
-                     static_cast<const In *>(gh_rows), gh_of(a), pre, tile_sum, tile_pre, ex_group.p, ex_ticket.p);
-        const ExSearch<T> x{ex_key[a].p, ex_val[a].p, pre, tile_pre, ex_group.p};
+                     static_cast<const In *>(gh_rows), gh_of(a), pre, tile_pre, run_sum, run_pre, ex_group.p, ex_ticket.p);
+        const ExSearch<T> x{ex_key[a].p, ex_val[a].p, pre, tile_pre, run_pre, ex_group.p};
         launch_after(k_exact_gain<T>, grid, EX_THREADS, sizeof(unsigned long long) * (size_t)nl, stream, live, x, level, nodes.p, qinfo.p,
                      p.min_child_weight, p.lambda, p.rt_eps, ignored_all.p, rstate.p, F, ex_best.p, ex_any.p, ex_ticket.p);
         const int node_blocks = std::min(nl, 1024);
@@ -690,9 +691,9 @@ void BoosterImpl::exact_levels(int k, const void *gh_rows) {
         launch_after(k_exact_move_missing, row_grid, 256, 0, stream, ex_nid.p, N, level, nodes.p, ex_any.p, ex_side.p);
         launches += 4;
         if (level + 1 == depth) break;
-        launch_after(k_exact_sides, grid, EX_THREADS, 0, stream, live, ex_row[a].p, ex_side.p, ex_lr.p, ex_tile_cnt.p, ex_tile_lr.p, ex_live.p + level + 1,
+        launch_after(k_exact_sides, grid, EX_THREADS, 0, stream, live, ex_row[a].p, ex_side.p, ex_lr.p, ex_tile_lr.p, run_cnt, run_lr, ex_live.p + level + 1,
                      ex_ticket.p);
-        launch_after(k_exact_scatter<In>, grid, EX_THREADS, 0, stream, live, ex_key[a].p, ex_row[a].p, ex_val[a].p, gh_of(a), ex_lr.p, ex_tile_lr.p, ex_group.p, ex_key[z].p,
+        launch_after(k_exact_scatter<In>, grid, EX_THREADS, 0, stream, live, ex_key[a].p, ex_row[a].p, ex_val[a].p, gh_of(a), ex_lr.p, ex_tile_lr.p, run_lr, ex_group.p, ex_key[z].p,
                      ex_row[z].p, ex_val[z].p, gh_of(z));
         launches += 2;
     }
