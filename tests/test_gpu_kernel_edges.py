@@ -120,3 +120,16 @@ def test_column_ids_of_a_large_csr(gpu, top):
         got.append((b.trees().tobytes(), b.ypred().tobytes()))
         b.close()
     assert got[0] == got[1]
+
+
+# CSR layout: rows around the 32 values that a warp adds up at a time
+@pytest.mark.parametrize('longest', [1, 32, 33, 64, 65, 400])
+def test_rows_of_the_csr_layout(gpu, orc, monkeypatch, longest):
+    monkeypatch.setenv('TGBM_LAYOUT', 'sparse')
+    r = np.random.default_rng(longest)
+    n, f = 3001, 400
+    keep = r.random((n, f)).argsort(1) < r.integers(0, longest + 1, n)[:, None]
+    keep[0] = np.arange(f) < longest
+    x = r.integers(1, 9, (n, f)).astype(np.float32)
+    d = _holes(x, (x * keep)[:, :20].sum(1) + r.random(n), keep)
+    _same_as_oracle(orc, d, depth=6, n_trees=3, max_num_bin=16, learning_rate=0.5, objective='reg:linear')
