@@ -65,9 +65,9 @@ WORKLOADS = {
            dict(objective='rank:ndcg', depth=8, max_num_bin=255, learning_rate=0.1, **COMMON),
            'mslr-shape 2.27M x 136 f32 in query groups of Poisson(120), rank:ndcg, depth 8, 255 bins, lr 0.1'),
 }
-# dram__bytes_read.sum + dram__bytes_write.sum per launch of the histogram kernel of either mode on config 2, from the
+# dram__bytes_read.sum + dram__bytes_write.sum per launch (mean over a tree) of the histogram kernel of either mode on config 2, from the
 # ncu captures summarised under profiles/ (None: no capture of that kernel yet)
-NCU_TRAFFIC_BYTES_PER_LAUNCH = {'exact': 363.1e6, 'fp32': 443.8e6}
+NCU_TRAFFIC_BYTES_PER_LAUNCH = {'exact': 356.1e6, 'fp32': 350.3e6}
 
 
 def make_shard(config, n_rows, rank, world):
