@@ -31,34 +31,34 @@ struct Batch {
 
 // ------------------------------------------------------------------ work lists
 // Exclusive prefix sums over n values inside one block of NT threads: out(i, prefix before i); returns the total.
-// `scratch` holds 33 ints of shared memory.  Every thread of the block must call it.
-template <int NT, typename In, typename Out>
-__device__ __forceinline__ int block_prefix(int n, In in, Out out, int *scratch) {
+// `scratch` holds 33 values of shared memory.  Every thread of the block must call it.
+template <int NT, typename V, typename In, typename Out>
+__device__ __forceinline__ V block_prefix(int n, In in, Out out, V *scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int carry = 0;
+    V carry = 0;
     for (int base = 0; base < n; base += NT) {
         const int i = base + threadIdx.x;
-        const int x = i < n ? in(i) : 0;
-        int v = x;
+        const V x = i < n ? in(i) : V(0);
+        V v = x;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+        for (int o = 1; o < 32; o <<= 1) { const V u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
         __syncthreads();
         if (lane == 31) scratch[warp] = v;
         __syncthreads();
         if (n - base <= 32) {   // one warp holds them all
-            const int total = scratch[0];
+            const V total = scratch[0];
             if (i < n) out(i, v - x + carry);
             carry += total;
             break;
         }
         if (warp == 0) {
-            int t = lane < NT / 32 ? scratch[lane] : 0;
+            V t = lane < NT / 32 ? scratch[lane] : V(0);
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, t, o); if (lane >= o) t += u; }
+            for (int o = 1; o < 32; o <<= 1) { const V u = __shfl_up_sync(0xffffffffu, t, o); if (lane >= o) t += u; }
             scratch[lane] = t;
         }
         __syncthreads();
-        if (i < n) out(i, v + (warp ? scratch[warp - 1] : 0) + carry - x);
+        if (i < n) out(i, v + (warp ? scratch[warp - 1] : V(0)) + carry - x);
         carry += scratch[NT / 32 - 1];
     }
     __syncthreads();
@@ -993,11 +993,19 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
 // number of records of the nodes before theirs.  Stable: the rows of either child ascend like those of the node.  Records
 // of nodes that stopped splitting drop out.
 
-// prologue of both kernels: tiles (s_tile) and records (s_rec) before every node, total tiles
-__device__ __forceinline__ int part_items(int level, const int *seg_cnt, int *s_tile, int *s_rec, int *scratch) {
+// prologue of both kernels: tiles (s_tile) before every node and total tiles; with a 64-bit scratch also the records before
+// every node (s_rec), both prefixes in one pass (the records of a level fit the low half)
+template <typename V>
+__device__ __forceinline__ int part_items(int level, const int *seg_cnt, int *s_tile, int *s_rec, V *scratch) {
     const int nl = 1 << level;
-    const int total = block_prefix<PART_THREADS>(nl, [&](int n) { return (seg_cnt[n] + PART_TILE - 1) / PART_TILE; }, [&](int n, int t) { s_tile[n] = t; }, scratch);
-    if (s_rec) block_prefix<PART_THREADS>(nl, [&](int n) { return seg_cnt[n]; }, [&](int n, int r) { s_rec[n] = r; }, scratch);
+    auto tiles = [&](int n) { return (seg_cnt[n] + PART_TILE - 1) / PART_TILE; };
+    int total;
+    if constexpr (sizeof(V) == 8) {
+        total = (int)(block_prefix<PART_THREADS>(nl, [&](int n) { return ((V)tiles(n) << 32) | (unsigned)seg_cnt[n]; },
+                                                 [&](int n, V before) { s_tile[n] = (int)(before >> 32); s_rec[n] = (int)before; }, scratch) >> 32);
+    } else {
+        total = block_prefix<PART_THREADS>(nl, tiles, [&](int n, int t) { s_tile[n] = t; }, scratch);
+    }
     if (threadIdx.x == 0) s_tile[nl] = total;
     __syncthreads();
     return total;
@@ -1091,7 +1099,8 @@ k_part_scatter(int level, const Batch b, int tree0) {
     chain_wait();
     constexpr int WORDS = PART_TILE / 32;
     extern __shared__ int s_tile[];   // [nl + 1], then records before every node [nl]
-    __shared__ int wpre[WORDS], wtot[(WORDS + 31) / 32], scratch[33];
+    __shared__ int wpre[WORDS], wtot[(WORDS + 31) / 32];
+    __shared__ long long scratch[33];
     const int nl = 1 << level, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int *s_rec = s_tile + nl + 1;
     const size_t tree = tree0 + blockIdx.z;
