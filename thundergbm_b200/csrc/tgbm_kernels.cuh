@@ -363,12 +363,17 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
         qinfo->sg = sg; qinfo->sh = sh;
         qinfo->inv_sg = pow2d(eg - quant_bits); qinfo->inv_sh = pow2d(eh - quant_bits);
     }
+    const bool in_float = sg < 1e38 && sh < 1e38;
+    const float fg = (float)sg, fh = (float)sh;
     long long tg = 0, th = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float2 v = gh ? gh[(size_t)k * n + i] : pointwise_gh(logistic, y[i], yp[i]);
         int qg, qh;
         if (FINE) {
-            qg = __double2int_rn((double)v.x * sg); qh = __double2int_rn((double)v.y * sh);
+            // the scale is a power of two: where a float holds it, the product is exact in float, and the conversions to and from
+            // double (a sixteenth of the float rate) can go
+            if (in_float) { qg = __float2int_rn(__fmul_rn(v.x, fg)); qh = __float2int_rn(__fmul_rn(v.y, fh)); }
+            else { qg = __double2int_rn((double)v.x * sg); qh = __double2int_rn((double)v.y * sh); }
         } else {
         const uint32_t row = row_offset + (uint32_t)i;
         const double ug = (double)mix32(0x9E3779B9u, round, (uint32_t)k, row) * (1.0 / 4294967296.0);
