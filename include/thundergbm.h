@@ -80,8 +80,9 @@ typedef struct {
     unsigned rank_seed; /* LambdaRank partner sampling */
     int hist_mode;      /* histogram arithmetic: 0 fp32 -- sums of the float (g,h): in the first round added value by value
                            into one float accumulator per bin, what the reference does in every round
-                           (hist_tree_builder_single.cu:203-216, :485-505); in later rounds integer sums on a grid of 2^-30
-                           of the round's largest gradient, closer to the true sums than any order of float additions;
+                           (hist_tree_builder_single.cu:203-216, :485-505); in later rounds integer sums of the gradients, each
+                           rounded by at most 2^-30 of the round's largest, as long as that is no worse than float sums;
+                           rounds whose gradients differ too much in size for it sum floats as in the first;
                            1 exact -- integer sums on a fixed-point grid in every round, bit-identical from run to run and
                            for any number of GPUs */
     int bagging;        /* RowSampler::do_bagging (src/thundergbm/row_sampler.cu:9-35): bootstrap multiplicities on (g,h) */

@@ -73,7 +73,8 @@ struct BoosterImpl {
     // `f32_stride(pairs)` float2 apart (see tgbm_hist_f32.cuh)
     bool f32 = false;
     // the round sums floats value by value; fp32 mode's later rounds sum integers on a grid of FINE_BITS bits
-    bool float_round(int round) const { return f32 && (exact || round < FINE_FROM_ROUND); }
+    bool float_round(int round) const { return f32 && (exact || round < FINE_FROM_ROUND || force_float); }
+    bool force_float = false;  // the round's gradients do not fit the grid (settle)
     bool last_float = false;   // hist_full holds float pairs
     size_t last_tree_full = 0; // where the histograms of the tree built last start in it
     DevBuf<float2> hist_spread;
@@ -100,6 +101,9 @@ struct BoosterImpl {
     long long round_graph_launches = 0;
     bool graphs_allowed = true;
     void run_round(int round);
+    void queue_round(int round);   // its launches one by one
+    void wait() const;
+    bool settle();
     DevBuf<int> eval_ticket;  // k_eval: finished blocks per sibling pair, zero between launches
     int part_ctas = 1;
     bool grad_max_ready = false;        // maxbits holds the maxima of the next round's gradients
@@ -703,7 +707,7 @@ void BoosterImpl::exact_levels(int k, const void *gh_rows) {
 void BoosterImpl::build_tree_exact(int round, int k) {
     const int tree_index = round * K + k;
     k_tree_init<<<ceil_div(n_nodes, 256), 256, 0, stream>>>(nodes.p, n_nodes, root_sum.p + 2 * k, qinfo.p, p.lambda, N,
-                                                            seg_begin[0].p, seg_cnt[0].p, bufs.seg_stride, f32 ? 1 : 0, maxbits.p);
+                                                            seg_begin[0].p, seg_cnt[0].p, bufs.seg_stride, f32 ? 1 : 0, maxbits.p, 0, ctl.p);
     if (f32) exact_levels<float>(k, gh.p + (size_t)k * N);
     else exact_levels<long long>(k, ghq.p + (size_t)k * N);
     k_prune<<<1, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream>>>(nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0, model.p, K, k,
@@ -838,7 +842,7 @@ void Booster::init(const DataSet &ds) {
         TGBM_CUDA(cudaStreamSynchronize(m.stream));
     }
     m.ypred.zero(m.stream);
-    m.maxbits.alloc(2); m.root_sum.alloc(2 * (size_t)K); m.qinfo.alloc(1);
+    m.maxbits.alloc(2); m.root_sum.alloc(2 * (size_t)K + 2); m.qinfo.alloc(1);
     m.maxbits.zero(m.stream); m.root_sum.zero(m.stream);
     if (p.bagging) {
         TGBM_CHECK((unsigned long long)std::max(p.num_class, 1) * (unsigned long long)m.N_global < (1ull << 32), "bagging: num_class x rows must fit 32 bits");
@@ -993,12 +997,12 @@ void BoosterImpl::gradient(int round) {
     const int blocks = std::max(1, std::min(ceil_div(N, tb), num_sms * 8));
     auto quantize = [&](auto kern, int bits) {
         launch_after(kern, dim3(blocks, K), tb, 0, stream, have_max ? nullptr : gh.p, N, maxbits.p, bits, (uint32_t)round, (uint32_t)row_offset,
-                                                 ghq.p, root_sum.p, qinfo.p, y.p, ypred.p, logistic, round >= 0 ? rstate.p : nullptr);
+                                                 ghq.p, root_sum.p, qinfo.p, y.p, ypred.p, logistic, round >= 0 ? rstate.p : nullptr, root_sum.p + 2 * K);
     };
-    if (f32) quantize(k_quantize<true>, FINE_BITS);
+    if (f32) quantize(k_quantize<true>, FINE_BITS);   // (its two words on the spread follow the root sums)
     else quantize(k_quantize<false>, p.quant_bits);
     ++launches;
-    if (comm && comm->active()) comm->allreduce(root_sum.p, 2 * (size_t)K, Comm::I64, Comm::SUM, stream);
+    if (comm && comm->active()) comm->allreduce(root_sum.p, 2 * (size_t)K + (f32 ? 2 : 0), Comm::I64, Comm::SUM, stream);
 }
 
 // Base score (include/thundergbm/objective/regression_obj.h:35-53 and :95-114): gradients at y_pred = 0,
@@ -1086,7 +1090,7 @@ void BoosterImpl::launch_small_trees(int k0, int n_trees) {
     TGBM_CUDA(cudaLaunchKernelEx(&cfg, k_small_tree, (SmallPlan)small, N, Npad, F, depth, (const unsigned char *)binsT.p, (const int *)cut_ptr.p,
                                  (const float *)cut_val.p, gq, roots, (const QuantInfo *)qinfo.p, p.min_child_weight, p.lambda, p.rt_eps, p.gamma,
                                  (const unsigned char *)ignored_all.p, (const RoundState *)rstate.p, p.column_shards > 0 ? 1 : 0, nodes.p, model.p, K, k0,
-                                 maxbits.p, ctl.p, hist_full.p, bufs.full_stride));
+                                 maxbits.p, f32 && k0 == 0 ? K : 0, ctl.p, hist_full.p, bufs.full_stride));
     ++launches;
 }
 
@@ -1102,7 +1106,7 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
     if (one_launch) launch_small_trees(k0, n_trees);
     else {
     launch_after(k_tree_init, dim3(ceil_div(n_nodes, 256), n_trees), 256, 0, stream, nodes.p, n_nodes, root_sum.p + 2 * k0, qinfo.p, p.lambda, N,
-                                                                           seg_begin[0].p, seg_cnt[0].p, b.seg_stride, float_sums ? 1 : 0, maxbits.p);
+                                                                           seg_begin[0].p, seg_cnt[0].p, b.seg_stride, float_sums ? 1 : 0, maxbits.p, fine && k0 == 0 ? K : 0, ctl.p);
     ++launches;
     }
     const int by_hessian = (comm && comm->active()) ? 1 : 0;
@@ -1207,7 +1211,7 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
         const int fo = fuse ? objective : -1;
         auto kern = sparse ? k_predict_walk<2> : Fpad == 32 ? k_predict_walk<0> : k_predict_walk<1>;
         launch_after(kern, walk_ctas, 256, walk_smem, stream, nodes.p, n_nodes, in_smem, sparse ? nullptr : bins.p, Fpad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, N,
-                                                    p.learning_rate, yp, nid_out, y.p, fo, metric_partial.p, maxbits.p, colb);
+                                                    p.learning_rate, yp, nid_out, y.p, fo, metric_partial.p, maxbits.p, colb, ctl.p);
         grad_max_ready = metric_partial_ready = fuse;
     }
     launches += 2;
@@ -1217,7 +1221,7 @@ void BoosterImpl::round_metric(int round) {
     const int log_len = (int)qinfo_log.n;
     if (need_group_file(objective)) {
         rank.metric(objective, ypred.p, nullptr, comm, N_global, stream);
-        launch_after(k_round_end, 1, 32, 0, stream, objective, rank.sum.p, nullptr, 0, rank.n_group_total, metric.p, qinfo.p, qinfo_log.p, log_len, rstate.p, root_sum.p, 2 * K);
+        launch_after(k_round_end, 1, 32, 0, stream, objective, rank.sum.p, nullptr, 0, rank.n_group_total, metric.p, qinfo.p, qinfo_log.p, log_len, rstate.p, root_sum.p, 2 * K + 2, ctl.p);
         ++launches;
         return;
     }
@@ -1234,7 +1238,7 @@ void BoosterImpl::round_metric(int round) {
         ++launches;
     }
     launch_after(k_round_end, 1, 32, 0, stream, objective, metric_sum.p, multi ? nullptr : metric_partial.p, blocks, N_global, metric.p, qinfo.p, qinfo_log.p,
-                                      log_len, rstate.p, root_sum.p, 2 * K);
+                                      log_len, rstate.p, root_sum.p, 2 * K + 2, ctl.p);
     ++launches;
 }
 
@@ -1243,15 +1247,15 @@ void BoosterImpl::round_metric(int round) {
 // on the device), so it is captured once into a CUDA graph and replayed: one launch per round instead of ~60, no
 // gaps between the small per-level kernels.  Not with profiling events or a kept row->node table.  With a communicator
 // the NCCL calls of the round are captured with it (every rank captures and replays the same sequence).
+void BoosterImpl::queue_round(int round) {
+    gradient(round);
+    for (int k = 0; k < K; k += batch) {
+        if (exact) build_tree_exact(round, k);
+        else build_trees(round, k, std::min(batch, K - k));
+    }
+    round_metric(round);
+}
 void BoosterImpl::run_round(int round) {
-    auto direct = [&]() {
-        gradient(round);
-        for (int k = 0; k < K; k += batch) {
-            if (exact) build_tree_exact(round, k);
-            else build_trees(round, k, std::min(batch, K - k));
-        }
-        round_metric(round);
-    };
     static const bool graph_with_comm = getenv("TGBM_NO_GRAPH_COMM") == nullptr;  // the round's collectives are captured with it
     // Ranks that are threads of ONE process do not replay graphs: instantiating a graph allocates device memory, and with
     // peer access enabled such a call can wait for the other devices of the process -- whose collective kernels may
@@ -1259,12 +1263,12 @@ void BoosterImpl::run_round(int round) {
     const bool in_process_group = comm && comm->active() && comm->host;
     const bool graph_ok = graphs_allowed && round >= 1 && !profile_on && !p.keep_nid && !in_process_group &&
                           (graph_with_comm || !(comm && comm->active()));
-    if (!graph_ok) { direct(); return; }
+    if (!graph_ok) { queue_round(round); return; }
     if (!round_exec) {
         const long long before = launches;
         TGBM_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         bool ok = true;
-        try { direct(); } catch (...) { ok = false; }
+        try { queue_round(round); } catch (...) { ok = false; }
         cudaGraph_t g = nullptr;
         const cudaError_t rc = cudaStreamEndCapture(stream, &g);
         round_graph_launches = launches - before;
@@ -1274,7 +1278,7 @@ void BoosterImpl::run_round(int round) {
             cudaGetLastError();
             graphs_allowed = false;
             TGBM_CHECK(ok, "capturing a boosting round failed");
-            direct();
+            queue_round(round);
             return;
         }
         round_graph = g;
@@ -1282,6 +1286,59 @@ void BoosterImpl::run_round(int round) {
     }
     TGBM_CUDA(cudaGraphLaunch(round_exec, stream));
     launches += round_graph_launches;
+    last_float = float_round(round);
+}
+
+void BoosterImpl::wait() const {
+    if (comm && comm->active()) comm->wait(stream);  // bounded: a rank may have left
+    else TGBM_CUDA(cudaStreamSynchronize(stream));
+}
+
+// Fine rounds of fp32 mode are queued before it is known whether their gradients fit the grid.  One whose do not leaves the
+// scores, the metric and the round counter alone (TreeCtl::coarse), and so does every round queued behind it.  Here, with the
+// queue empty, it is built again from float sums, and the rounds after it are queued once more: in steps that start at one
+// round and double, so that what is thrown away stays in proportion; one that does not fit either is found before it is built.
+// Returns whether there was such a round.
+bool BoosterImpl::settle() {
+    if (!f32 || exact || rounds <= FINE_FROM_ROUND) return false;
+    auto coarse = [&] {
+        int v = 0;
+        TGBM_CUDA(cudaMemcpyAsync(&v, &ctl.p->coarse, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        wait();
+        return v != 0;
+    };
+    auto float_again = [&](int round) {
+        static const QuantInfo one{1.0, 1.0, 1.0, 1.0};
+        TGBM_CUDA(cudaMemsetAsync(&ctl.p->coarse, 0, sizeof(int), stream));
+        TGBM_CUDA(cudaMemcpyAsync(qinfo.p, &one, sizeof(one), cudaMemcpyHostToDevice, stream));   // (what the log of the grids shows)
+        force_float = true;
+        queue_round(round);
+        force_float = false;
+    };
+    bool again = false;
+    for (int queued = rounds, step = 1;;) {
+        if (coarse()) {
+            RoundState at;
+            TGBM_CUDA(cudaMemcpy(&at, rstate.p, sizeof(at), cudaMemcpyDeviceToHost));
+            again = true;
+            step = 1;
+            float_again(at.round);
+            for (queued = at.round + 1; queued < rounds; ++queued) {
+                const bool have_max = grad_max_ready;
+                gradient(queued);
+                grad_max_ready = have_max;   // the maxima are still there
+                k_grid_check<<<1, 1, 0, stream>>>(root_sum.p, K, ctl.p);
+                root_sum.zero(stream);
+                ++launches;
+                if (!coarse()) break;
+                float_again(queued);
+            }
+        } else if (queued == rounds) {
+            return again;
+        }
+        for (int i = 0; i < step && queued < rounds; ++i) run_round(queued++);
+        step *= 2;
+    }
 }
 
 void Booster::boost(int n_rounds) {
@@ -1292,11 +1349,12 @@ void Booster::boost(int n_rounds) {
         ++m.rounds;
     }
     TGBM_CUDA(cudaGetLastError());
+    if (m.comm && m.comm->active()) m.settle();   // together: the ranks need not all ask for results, or at the same time
 }
 
-void Booster::sync() {
-    if (impl_->comm && impl_->comm->active()) impl_->comm->wait(impl_->stream);  // bounded: a rank may have left
-    else TGBM_CUDA(cudaStreamSynchronize(impl_->stream));
+bool Booster::sync() {
+    const bool again = impl_->settle();
+    impl_->wait();
     TGBM_CUDA(cudaGetLastError());
     // bounded waits inside the kernels (bulk-copy barriers of the float histogram kernel) report here instead of spinning: the results of the run are not to be trusted
     if (impl_->ctl.p) {
@@ -1304,6 +1362,7 @@ void Booster::sync() {
         TGBM_CUDA(cudaMemcpy(&err, reinterpret_cast<const char *>(impl_->ctl.p) + offsetof(TreeCtl, error), sizeof(int), cudaMemcpyDeviceToHost));
         TGBM_CHECK(err == 0, "a bounded wait inside a kernel ran out (code " + std::to_string(err) + "); the trees of this run are invalid");
     }
+    return again;
 }
 
 int Booster::rounds_done() const { return impl_->rounds; }

@@ -40,7 +40,7 @@ public:
     void init(const DataSet &ds);
     // rounds [done, done+n) ; asynchronous on the booster's stream
     void boost(int n_rounds);
-    void sync();
+    bool sync();   // waits; fp32 mode: builds the rounds again whose gradients did not fit the integer grid (true: there were some)
 
     int rounds_done() const;
     int trees_per_round() const;

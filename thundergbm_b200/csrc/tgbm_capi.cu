@@ -565,7 +565,10 @@ int tgbm_booster_boost_timed(TgbmBooster *b, int n_rounds, float *elapsed_ms) {
         TGBM_CUDA(cudaEventRecord(e0, b->b->stream()));
         b->b->boost(n_rounds);
         TGBM_CUDA(cudaEventRecord(e1, b->b->stream()));
-        b->b->sync();
+        if (b->b->sync()) {   // rounds were built again
+            TGBM_CUDA(cudaEventRecord(e1, b->b->stream()));
+            b->b->sync();
+        }
         TGBM_CUDA(cudaEventElapsedTime(elapsed_ms, e0, e1));
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);

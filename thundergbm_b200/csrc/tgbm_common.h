@@ -80,8 +80,8 @@ struct GBMParam {
     // additions of this implementation
     // Histogram arithmetic.  0 "fp32": sums of the float (g,h).  First round: added per stored value into one float
     // accumulator per bin, float prefix sums -- the reference's own arithmetic (hist_tree_builder_single.cu:203-216),
-    // results depend on the order of the additions in the last bits.  Later rounds: integer sums on a grid of 2^-30 of the
-    // round's largest gradient (see FINE_FROM_ROUND).  1 "exact": gradients on a coarser, dithered power-of-two grid in
+    // results depend on the order of the additions in the last bits.  Later rounds: integer sums, every gradient rounded by
+    // at most 2^-30 of the round's largest (FINE_FROM_ROUND), unless their spread is too wide for that (grid_too_coarse).  1 "exact": gradients on a coarser, dithered power-of-two grid in
     // every round -- the deterministic mode: bit-identical from run to run and for any number of GPUs.
     int hist_mode = 0;
     // 0: cut points, candidate order and child sums of the one-device builder (HistTreeBuilder_single, what the

@@ -1,4 +1,5 @@
-// Histogram build in the reference's own arithmetic (first round of the fp32 mode).
+// Histogram build in the reference's own arithmetic (fp32 mode: the first round, and rounds whose gradients do not fit the
+// integer grid, see grid_too_coarse).
 //
 // The reference keeps ONE float (g,h) accumulator per bin of a node in global memory and adds every stored value
 // to it with atomicAdd (src/thundergbm/builder/hist_tree_builder_single.cu:203-216 for the root, :485-505 for the
@@ -6,12 +7,13 @@
 // and when many equal values meet in one bin (first boosting round of a classification objective: every row of a
 // class carries the same hessian) that accumulation drifts by a few 1e-5 relative, whatever the order.  Sums that
 // are first collected per CTA and then combined -- or exact integer sums -- do not reproduce the drift, and the
-// gains computed from them sit a few 1e-4 away from the reference's.  So the first round keeps the reference's scheme:
+// gains computed from them sit a few 1e-4 away from the reference's.  So the first round keeps the reference's scheme,
+// for every objective (that of reg:linear and the ranking ones have no common gradient, and did not need it):
 // one accumulator per (node, bin) for the whole GPU, every (row, feature) pair issues one vector reduction
-// `red.global.add.v2.f32` that the L2 performs in arrival order.  From the second round on the gradients differ from row
-// to row, the rounding errors of the reference's sums no longer have a common sign and its sums agree with the true
-// ones to the noise that two of its own runs differ by; those rounds take integer sums in shared memory (k_hist<., true>),
-// which are closer to the true sums and 4 to 7 times faster (10.5 M rows x 28, depth 8: 4.6 -> 1.0 ms per tree).
+// `red.global.add.v2.f32` that the L2 performs in arrival order.  From the second round on the rows of a class carry as many
+// gradients as the tree has leaves (more with every further tree), the rounding errors of the reference's sums partly cancel,
+// and its recorded runs agree with integer sums to the noise that two of them differ by; those rounds take integer sums in
+// shared memory (k_hist<., true>), 4 to 7 times faster (10.5 M rows x 28, depth 8: 4.6 -> 1.0 ms per tree for the histograms).
 //
 // The L2 performs the reductions that aim at one line one after the other, so cells packed 16 to a line are its
 // worst case (measured with the bare reductions of 10.5 M rows x 28: 87 G/s into 8-byte cells of one node, 165 G/s

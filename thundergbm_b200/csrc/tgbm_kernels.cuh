@@ -28,7 +28,8 @@ constexpr int MISSING_BIN = 255;
 constexpr int METRIC_PARTS = 1280;  // most partial sums of a round's metric (148 SMs x 8 blocks use 1184)
 constexpr int FINE_BITS = 30;          // value bits of the grid of fp32 mode's later rounds
 constexpr int FINE_WINDOW = 1 << 16;   // rows whose 16-bit low halves fit an unsigned accumulator
-constexpr int FINE_FROM_ROUND = 1;     // fp32 mode: rounds before it sum floats value by value (k_hist_f32)
+constexpr int FINE_FROM_ROUND = 1;     // fp32 mode: rounds before it sum floats value by value (k_hist_f32), and so do those that grid_too_coarse finds
+constexpr int FINE_MEAN_BITS = 19;     // see grid_too_coarse
 
 // Shares of the level's tiles per CTA of the dense histogram kernel: two when a CTA has HIST_SHARE_TILES tiles or more, else
 // one.  Two balance the CTAs better (7 trees of 581 k rows side by side, 22 tiles per CTA: 50.6 ms per training against 52.6),
@@ -44,6 +45,7 @@ struct RoundState {
 struct TreeCtl {  // device-side scalars of the booster
     unsigned long long stat_rows_root, stat_rows_gather, stat_hists, stat_part_rows;  // what the level kernels processed
     int error;   // non-zero when a bounded wait inside a kernel gave up; the host reads it after a sync
+    int coarse;  // the running round's gradients do not fit the grid: scores, metric and round counter stay as they are
 };
 
 struct SplitRec {  // best candidate of one (node, feature)
@@ -343,8 +345,9 @@ static __global__ void k_grad_softmax(const float *y, const float *yp, int n, in
 // round-to-nearest would move every row that carries the same gradient the same way (in the first round all rows
 // of a class do), and those shifts would add up coherently in the histogram sums.
 //
-// FINE (fp32 mode from the second round on, FINE_BITS value bits): rounded to nearest -- the grid is 2^-30 of the largest
-// gradient, finer than the last bit of any float sum that a bin of the reference could hold.
+// FINE (fp32 mode from the second round on, FINE_BITS value bits): rounded to nearest, so a value moves by at most 2^-30 of
+// the round's largest one, however small it is itself.  What that means for the sums depends on the spread of the values: `spread` (behind the root
+// sums) collects what grid_too_coarse decides by.
 //
 // `gh` null: the gradients are those of a pointwise objective (`logistic` 0/1) and are computed again from y and the
 // scores here -- the pass that found their maxima (k_predict_walk) did not store them.
@@ -353,7 +356,7 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
                            uint32_t round, uint32_t row_offset, int2 *ghq,
                            unsigned long long *root_sum, QuantInfo *qinfo,
                            const float *y, const float *yp, int logistic,
-                           const RoundState *rs) {
+                           const RoundState *rs, unsigned long long *spread) {
     chain_wait();
     if (rs) round = (uint32_t)rs->round;  // the booster's rounds; the base-score pass gives its own
     const int k = blockIdx.y;
@@ -365,6 +368,8 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
     }
     const bool in_float = sg < 1e38 && sh < 1e38;
     const float fg = (float)sg, fh = (float)sh;
+    unsigned long long rounded = 0;
+    int bad = 0;
     long long tg = 0, th = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float2 v = gh ? gh[(size_t)k * n + i] : pointwise_gh(logistic, y[i], yp[i]);
@@ -372,8 +377,18 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
         if (FINE) {
             // the scale is a power of two: where a float holds it, the product is exact in float, and the conversions to and from
             // double (a sixteenth of the float rate) can go
-            if (in_float) { qg = __float2int_rn(__fmul_rn(v.x, fg)); qh = __float2int_rn(__fmul_rn(v.y, fh)); }
-            else { qg = __double2int_rn((double)v.x * sg); qh = __double2int_rn((double)v.y * sh); }
+            bool off;   // the gradient is not on the grid
+            if (in_float) {
+                const float pg = __fmul_rn(v.x, fg);
+                qg = __float2int_rn(pg); qh = __float2int_rn(__fmul_rn(v.y, fh));
+                off = __int2float_rn(qg) != pg;
+            } else {
+                const double pg = (double)v.x * sg;
+                qg = __double2int_rn(pg); qh = __double2int_rn((double)v.y * sh);
+                off = (double)qg != pg;
+            }
+            if (off) rounded += (unsigned)qh >> (31 - __clz(abs(qg) | 1));
+            bad += !(fabsf(v.x) < INFINITY) || !(v.y < INFINITY);
         } else {
         const uint32_t row = row_offset + (uint32_t)i;
         const double ug = (double)mix32(0x9E3779B9u, round, (uint32_t)k, row) * (1.0 / 4294967296.0);
@@ -385,16 +400,48 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) { tg += shfl_xor_ll(tg, o); th += shfl_xor_ll(th, o); }
+    if (FINE) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) rounded += (unsigned long long)shfl_xor_ll((long long)rounded, o);
+        bad = __reduce_add_sync(0xffffffffu, bad);
+    }
     // one pair of atomics per block: all go to the same two words, and one pair per warp made 19 k of them at 1 M rows, 12 of
     // the kernel's 19 us
-    __shared__ long long part[2][8];
-    if ((threadIdx.x & 31) == 0) { part[0][threadIdx.x >> 5] = tg; part[1][threadIdx.x >> 5] = th; }
+    __shared__ long long part[4][8];
+    if ((threadIdx.x & 31) == 0) {
+        part[0][threadIdx.x >> 5] = tg; part[1][threadIdx.x >> 5] = th;
+        if (FINE) { part[2][threadIdx.x >> 5] = (long long)rounded; part[3][threadIdx.x >> 5] = bad; }
+    }
     __syncthreads();
-    if (threadIdx.x < 2) {
+    if (threadIdx.x < (FINE ? 4 : 2)) {
         long long t = 0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[threadIdx.x][w];
-        atomicAdd(root_sum + 2 * k + threadIdx.x, (unsigned long long)t);
+        if (threadIdx.x < 2) atomicAdd(root_sum + 2 * k + threadIdx.x, (unsigned long long)t);
+        else if (t) atomicAdd(spread + threadIdx.x - 2, (unsigned long long)t);
     }
+}
+
+// Is the grid of a fine round too coarse for its gradients?  Called by one thread, after k_quantize and the ranks' sums.
+//
+// root_sum[2 K]: 2 * hessian * 2^-bits summed over the gradients that the grid had to round, bits = those left of the value.
+// 2^-bits bounds the relative error of a gradient, the hessian is the row's weight in -sum g / (sum h + lambda): divided by
+// the sum of all hessians it is the mean relative error of what the leaf weights are made of.  On normal residuals with a few
+// outliers, integer and float sums were both compared with float64 on the same gradients: the weights of the nodes without
+// outliers are at least as good from the integers down to 2^-18 for 4 k rows (outliers 300 times the rest; their error in
+// units of 2^-24 of the rms gradient, rms over the nodes: 0.4 against 1.3; 1.0 against 0.4 at 2^-16.7), down to 2^-15 for
+// 400 k rows.  Lambda gradients come to 2^-21 to 2^-23, everything else of ordinary data to 2^-28 and less, since most
+// gradients are multiples of the grid; one label of 1e9 among normal ones to 2^-1.
+// Hessians need no such test: sum h + lambda loses at most 2^-31 of the largest per row, the float sums lose 2^-24 of the
+// node's whole sum to one of its children (what the node's sum and the sum over its bins differ by counts as missing rows).
+// root_sum[2 K + 1]: gradients that are not finite.  One is enough: float sums carry it on, the grid does not.
+__device__ inline bool grid_too_coarse(const unsigned long long *root_sum, int K) {
+    unsigned long long h = 0;
+    for (int k = 0; k < K; ++k) h += root_sum[2 * k + 1];
+    return root_sum[2 * K + 1] != 0 || root_sum[2 * K] > h >> (FINE_MEAN_BITS - 1);
+}
+// the same for a round that is not built yet
+static __global__ void k_grid_check(const unsigned long long *root_sum, int K, TreeCtl *ctl) {
+    if (grid_too_coarse(root_sum, K)) ctl->coarse = 1;
 }
 
 
@@ -428,16 +475,22 @@ static __global__ void k_bag_scale(float2 *__restrict__ gh, const int *__restric
 }
 
 // ------------------------------------------------------------------ tree set-up
+// The quantisation has used the round's maxima; those of the next round's gradients are collected from zero -- unless the
+// round will be built again, on the same gradients.  fine_K > 0: the first trees of a fine round of fine_K trees.
+__device__ inline void next_maxima(const unsigned long long *root_sum, int fine_K, unsigned *maxbits, TreeCtl *ctl) {
+    if (fine_K && grid_too_coarse(root_sum, fine_K)) ctl->coarse = 1;
+    if (!ctl->coarse) maxbits[0] = maxbits[1] = 0;
+}
+
 // Tree::init2 (src/thundergbm/tree.cu:8-39)
 // root_is_f64: fp32 mode, the root sums are doubles (k_sum_gh_final) instead of integers on the fixed-point grid
 // grid.y = trees of the batch; seg tables: the root holds every row
 static __global__ void k_tree_init(TreeNode *nodes, int n_nodes, const unsigned long long *root_sum,
                             const QuantInfo *q, float lambda, int n_rows, int *seg_begin,
-                            int *seg_cnt, size_t seg_stride, int root_is_f64, unsigned *maxbits) {
-    // maxbits: the quantisation has used the round's maxima; those of the next round's gradients are collected from zero
+                            int *seg_cnt, size_t seg_stride, int root_is_f64, unsigned *maxbits, int fine_K, TreeCtl *ctl) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 2 && blockIdx.y == 0) maxbits[i] = 0;
+    if (i == 0 && blockIdx.y == 0) next_maxima(root_sum, fine_K, maxbits, ctl);
     if (i >= n_nodes) return;
     const size_t tree = blockIdx.y;
     root_sum += 2 * tree;
@@ -671,8 +724,9 @@ k_predict_walk(const TreeNode *nodes, int n_nodes, int table_in_smem, const unsi
                const int *__restrict__ sp_row_ptr, const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr,
                int n, float lr, float *yp, int *__restrict__ nid_out,
                const float *__restrict__ y, int fuse_objective, double *metric_partial,
-               unsigned *maxbits, int rev) {
+               unsigned *maxbits, int rev, const TreeCtl *ctl) {
     chain_wait();
+    const int coarse = ctl->coarse;
     // blockIdx.y: tree of the batch
     nodes += (size_t)blockIdx.y * n_nodes;
     yp += (size_t)blockIdx.y * n;
@@ -695,6 +749,7 @@ k_predict_walk(const TreeNode *nodes, int n_nodes, int table_in_smem, const unsi
         }
         __syncthreads();
     }
+    if (coarse) return;   // the round will be built again
     const int levels = 31 - __clz(n_nodes + 1) - 1;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         int lo0 = 0, hi0 = 0;
@@ -808,9 +863,10 @@ static __global__ void k_metric_final(int objective, const double *__restrict__ 
 static __global__ void k_round_end(int objective, const double *sum, const double *partial, int nb, long long n_total,
                                    float *metric, const QuantInfo *qinfo, QuantInfo *qinfo_log, int log_len,
                                    RoundState *rs,
-                                   unsigned long long *root_sum, int n_root) {
+                                   unsigned long long *root_sum, int n_root, const TreeCtl *ctl) {
     chain_wait();
     for (int i = threadIdx.x; i < n_root; i += 32) root_sum[i] = 0;   // the next round adds to them
+    if (ctl->coarse) return;   // this one will be built again
     double t = 0;
     if (partial) {
         // (all loads first, then the additions in the usual order)

@@ -83,7 +83,7 @@ static __global__ void __launch_bounds__(SMALL_THREADS, 1)
 k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const unsigned char *__restrict__ binsT, const int *__restrict__ cut_ptr,
              const float *__restrict__ cut_val, const int2 *ghq, const unsigned long long *root_sum, const QuantInfo *q, float mcw, float lam,
              float rt_eps, float gamma, const unsigned char *__restrict__ ignored_all, const RoundState *rs, int multi, TreeNode *nodes_out,
-             TreeNode *model, int K, int k0, unsigned *maxbits, TreeCtl *ctl, long long *hist_full, size_t full_stride) {
+             TreeNode *model, int K, int k0, unsigned *maxbits, int fine_K, TreeCtl *ctl, long long *hist_full, size_t full_stride) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char small_sm[];
     __shared__ int scratch[33], s_split;
@@ -250,7 +250,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
     cluster.sync();   // nobody reads this CTA's candidates any more
     if (rank != 0) return;
     // -- pruning and the finished tree (k_prune)
-    if (blockIdx.x == 0 && threadIdx.x < 2) maxbits[threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) next_maxima(root_sum, fine_K, maxbits, ctl);
     if (threadIdx.x == 0) {
         atomicAdd(&ctl->stat_rows_root, (unsigned long long)N);
         atomicAdd(&ctl->stat_hists, 1ull);
