@@ -74,3 +74,20 @@ def test_every_walk_equals_the_oracle(gpu, orc, n, f, rounds, k, depth, full):
     trees = _random_trees(rounds, k, depth, f, rng)
     want = orc.predict_raw(d, trees, 0.3, 0.25)
     assert np.array_equal(predict_raw(d, trees, 0.3, 0.25), want)
+
+
+# the walk from the matrix keeps more than 48 KB of leaf values in shared memory, a limit that every device has of its own
+def test_large_direct_walk_on_every_device(gpu):
+    import torch
+    from thundergbm_b200.booster import predict_raw
+    if torch.cuda.device_count() < 2:
+        pytest.skip('needs two GPUs')
+    rng = np.random.default_rng(1)
+    d = synth.dense_to_csr(rng.standard_normal((20_000, 12)).astype(np.float32), np.zeros(20_000, np.float32))
+    trees = _random_trees(100, 7, 4, 12, rng)
+    got = []
+    for dev in (0, 1, 0):
+        torch.cuda.set_device(dev)
+        got.append(predict_raw(d, trees, 0.3, 0.0))
+    torch.cuda.set_device(0)
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])

@@ -1173,11 +1173,8 @@ void predict(const DataSet &ds, PredictPlan &plan, float learning_rate, float ba
         while (chunk < std::min(8, n_rounds) && rt_log > 0) { --rt_log; bytes = smem(); }
         if (chunk > 0) {
             auto kern = is_dense_path(F) ? k_predict_direct<true> : k_predict_direct<false>;
-            static std::once_flag once;
-            std::call_once(once, [&] {
-                cudaFuncSetAttribute(k_predict_direct<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
-                cudaFuncSetAttribute(k_predict_direct<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
-            });
+            if (bytes > 48 * 1024)   // (a limit of the kernel on the current device)
+                TGBM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
             if (kernel_ms) TGBM_CUDA(cudaEventRecord(ev.e0, st));
             kern<<<(N + (1 << rt_log) - 1) >> rt_log, PD_THREADS, bytes, st>>>(kind, in, N, n_feat, plan.h.p, n_rounds, K, n_nodes, depth, rt_log,
                                                                               chunk, learning_rate, base_score, scores_dev);
