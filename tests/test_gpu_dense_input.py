@@ -91,3 +91,18 @@ def test_large_direct_walk_on_every_device(gpu):
         got.append(predict_raw(d, trees, 0.3, 0.0))
     torch.cuda.set_device(0)
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
+# a matrix of no columns has no cells and may be a null pointer: rows of missing values, like a CSR that stores nothing
+@pytest.mark.parametrize('n', [5, 3_000_000])   # walked directly, by ranks
+def test_matrix_without_columns(gpu, n):
+    import ctypes as C
+    from thundergbm_b200.thundergbm import TGBMModel
+    x = _matrix(1000, 4, 0.5, np.float32)
+    m = TGBMModel(depth=5, n_trees=30, learning_rate=0.5, verbose=0, objective='reg:linear', tree_method='hist').fit(x, np.arange(1000) % 7)
+    got = np.full(n, np.nan, np.float32)
+    m._lib.dense_predict_scikit(n, 0, None, 0, got.ctypes.data_as(C.c_void_p), C.byref(m.model), m.n_trees, m.tree_per_iter, b'reg:linear', m.num_class,
+                                m.learning_rate, None, 0)
+    assert not m._lib.tgbm_last_error()
+    want = m.predict(sp.csr_matrix((n, 4), dtype=np.float32))
+    assert np.array_equal(got, want)

@@ -180,8 +180,8 @@ std::vector<std::vector<tgbm::Tree>> train_in_process(tgbm::GBMParam &p, const t
                 tgbm::DataSet shard;
                 shard.n_rows = hi - lo;
                 shard.n_features = ds.n_features;
-                if (ds.dense) {
-                    shard.dense = static_cast<const char *>(ds.dense) + (size_t)lo * ds.dense_cols * (ds.dense_f64 ? 8 : 4);
+                if (ds.is_dense()) {
+                    shard.dense = ds.dense == nullptr ? nullptr : static_cast<const char *>(ds.dense) + (size_t)lo * ds.dense_cols * (ds.dense_f64 ? 8 : 4);
                     shard.dense_cols = ds.dense_cols; shard.dense_f64 = ds.dense_f64;
                 } else {
                     shard.row_ptr.resize(hi - lo + 1);

@@ -127,6 +127,7 @@ struct DataSet {
     const void *dense = nullptr;
     int dense_cols = 0;
     bool dense_f64 = false;
+    bool is_dense() const { return !rp; }   // (a matrix without cells may be a null pointer)
     std::vector<int> row_ptr, col;
     std::vector<float> val, y;
     std::vector<int> group;

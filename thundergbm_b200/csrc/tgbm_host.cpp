@@ -85,7 +85,7 @@ void DataSet::take_labels(const float *yy, const int *grp, int num_group, GBMPar
 }
 
 int DataSet::count_features() const {
-    if (dense) {   // last column that holds a non-zero: rows from the last column down, most matrices end at the first row
+    if (is_dense()) {   // last column that holds a non-zero: rows from the last column down, most matrices end at the first row
         int m = -1;
         auto scan = [&](auto *x) {
             for (int r = 0; r < n_rows && m < dense_cols - 1; ++r)
@@ -96,7 +96,7 @@ int DataSet::count_features() const {
         else scan(static_cast<const float *>(dense));
         return m + 1;
     }
-    const long long nnz = rp ? rp[n_rows] : 0;
+    const long long nnz = rp[n_rows];
     const int nt = (int)std::max<long long>(1, std::min<long long>(16, nnz / (1 << 22)));
     std::vector<int> part(nt, -1);
     std::vector<std::thread> th;

@@ -73,7 +73,7 @@ static __global__ void k_widen_ids(const uint16_t *__restrict__ in, size_t n, in
 // The largest and smallest column index are found on the device, at HBM speed, instead of by a pass over the host copy.
 void DeviceRows::upload(const DataSet &ds, cudaStream_t stream, int num_sms, int up_threads) {
     const int N = ds.n_rows;
-    if (ds.dense || !ds.rp) {
+    if (ds.is_dense()) {
         upload_dense(ds, stream, num_sms, up_threads);
         return;
     }

@@ -1124,14 +1124,17 @@ void predict(const DataSet &ds, PredictPlan &plan, float learning_rate, float ba
     if (heap_ok && (double)N * n_rounds * K * std::max(depth, 1) <= DIRECT_VISITS && getenv("TGBM_PREDICT_FLOAT") == nullptr &&
         getenv("TGBM_PREDICT_RANKS") == nullptr) {
         RowsIn in{};
-        int kind = ds.dense ? (ds.dense_f64 ? IN_F64 : IN_F32) : IN_CSR;
+        int kind = ds.is_dense() ? (ds.dense_f64 ? IN_F64 : IN_F32) : IN_CSR;
         DevBuf<unsigned char> d_x;
-        if (ds.dense) {
+        if (ds.is_dense()) {
             in.cols = ds.dense_cols;
             if (F < 0) F = is_dense_path(in.cols) ? in.cols : ds.count_features();   // only the choice of the arithmetic depends on it
             const size_t bytes = (size_t)N * in.cols * (ds.dense_f64 ? 8 : 4);
             void *small = ws.take(bytes);
-            if (small) { memcpy(small, ds.dense, bytes); in.x = ws.device(small); }
+            if (small) {
+                if (bytes) memcpy(small, ds.dense, bytes);
+                in.x = ws.device(small);
+            }
             else {
                 d_x.alloc(bytes);
                 upload_h2d(d_x.p, ds.dense, bytes, st, upload_threads());
@@ -1187,7 +1190,7 @@ void predict(const DataSet &ds, PredictPlan &plan, float learning_rate, float ba
     // copied when the feature count is known or can be read off the first row.
     std::future<std::shared_ptr<PredictPlan::Ranks>> making;
     if (!uploaded) {
-        const int guess = F >= 0 ? std::max(1, F) : ds.dense ? std::max(1, ds.dense_cols) : ds.rp[1];
+        const int guess = F >= 0 ? std::max(1, F) : ds.is_dense() ? std::max(1, ds.dense_cols) : ds.rp[1];
         if (heap_ok && guess >= 1 && guess <= 256 && !plan.has_ranks(guess)) making = std::async(std::launch::async, [&plan, guess] { return plan.make_ranks(guess); });
         rows.upload(ds, st, num_sms, upload_threads());
     }
