@@ -106,3 +106,14 @@ def test_matrix_without_columns(gpu, n):
     assert not m._lib.tgbm_last_error()
     want = m.predict(sp.csr_matrix((n, 4), dtype=np.float32))
     assert np.array_equal(got, want)
+
+
+# the labels of a model are those it was fitted with, whatever becomes of the caller's array
+@pytest.mark.parametrize('n', [300, 70_000])   # counted before, and beside the training
+def test_labels_of_the_model_are_its_own(gpu, n):
+    from thundergbm_b200.thundergbm import TGBMRegressor
+    x = _matrix(n, 3, 0, np.float32)
+    y = np.arange(n, dtype=np.float32) % 251
+    m = TGBMRegressor(depth=3, n_trees=2, verbose=0, tree_method='hist').fit(x, y)
+    y[:] = 1
+    assert m.group_label == [0.0] * 251

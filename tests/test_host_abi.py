@@ -92,6 +92,18 @@ def test_default_param_matches_reference_parser(lib):
     assert p.objective == b'reg:linear'
 
 
+@pytest.mark.parametrize('n,values', [(0, 1), (1, 1), (16, 16), (17, 17), (4096, 10 ** 6), (4097, 10 ** 6), (9000, 20), (300_000, 10 ** 9), (300_000, 40)])
+def test_distinct_labels_are_counted(lib, n, values):
+    """Every NaN counts, +0 and -0 are one."""
+    r = np.random.default_rng(n)
+    y = (r.integers(0, values, n) - values // 2).astype(np.float32)
+    y[::7] *= -1   # a -0 among the zeros
+    if n > 100:
+        y[5:9] = np.nan
+    want = len(np.unique(y[~np.isnan(y)] + 0.0)) + int(np.isnan(y).sum())
+    assert lib.tgbm_count_distinct(y.ctypes.data_as(C.c_void_p), n) == want
+
+
 def test_no_cpu_fallback_in_the_product():
     """The product never reaches for the oracle."""
     pkg = os.path.join(ROOT, 'thundergbm_b200')

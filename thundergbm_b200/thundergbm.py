@@ -13,6 +13,7 @@ predict() for 400009 x 28 values, against 20 ms of training on the GPU).
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 import scipy.sparse as sp
@@ -76,18 +77,18 @@ class TGBMModel:
     @property
     def group_label(self):
         """Labels of the model as the reference's wrapper keeps them: one entry per distinct value of y, zeros for the
-        objectives without classes (counted here when somebody asks: nothing uses them)."""
-        if self._group_label is None and self._label_source is not None:
-            self._group_label = [0.0] * max(1, self._lib.tgbm_count_distinct(_vp(self._label_source), self._label_source.size))
+        objectives without classes."""
+        if self._group_label is None and self._n_labels:
+            self._group_label = [0.0] * self._n_labels
         return self._group_label
 
     @group_label.setter
     def group_label(self, value):
-        self._group_label, self._label_source = value, None
+        self._group_label, self._n_labels = value, 0
 
     def _label_buffer(self):
         if self._group_label is None:
-            return None if self._label_source is None else (C.c_float * max(1, self.num_class))()
+            return (C.c_float * max(1, self.num_class))() if self._n_labels else None
         return (C.c_float * max(len(self._group_label), self.num_class))(*self._group_label)
 
     # -- API ---------------------------------------------------------------------------------------
@@ -103,7 +104,13 @@ class TGBMModel:
             raise ValueError('X and y have different numbers of rows')
         grp = None if groups is None else np.ascontiguousarray(groups, np.int32)
         labelled = self.objective in _LABELLED
-        n_labels = max(1, self._lib.tgbm_count_distinct(_vp(y), y.size)) if labelled else 1
+        count, counter = [1], None
+        if labelled or y.size < 4096:
+            count[0] = max(1, self._lib.tgbm_count_distinct(_vp(y), y.size))
+        else:  # beside the training, which does not need it (10 k / 400 k / 10.5 M different labels: 0.3 / 6 / 145 ms)
+            counter = threading.Thread(target=lambda: count.append(self._lib.tgbm_count_distinct(_vp(y), y.size)))
+            counter.start()
+        n_labels = count[0]
         group_label = (C.c_float * n_labels)()
         n_class = C.c_int(self.num_class)
         per_iter = C.c_int(0)
@@ -116,13 +123,15 @@ class TGBMModel:
             self._lib.dense_train_scikit(n, X.shape[1], _vp(dense[0]), dense[1], *rest)
         else:
             self._lib.sparse_train_scikit(n, _vp(val), _vp(indptr), _vp(indices), *rest)
+        if counter is not None:
+            counter.join()
         if not model.value:
             raise RuntimeError('training failed: ' + self._lib.tgbm_last_error().decode())
         self.model, self.num_class, self.tree_per_iter = model, n_class.value, per_iter.value
         if labelled:
             self.group_label = [group_label[i] for i in range(n_labels)]
         else:
-            self._group_label, self._label_source = None, y
+            self._group_label, self._n_labels = None, count[-1]
         return self
 
     def predict(self, X, groups=None):
