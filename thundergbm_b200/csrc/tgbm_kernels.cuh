@@ -400,7 +400,7 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) { tg += shfl_xor_ll(tg, o); th += shfl_xor_ll(th, o); }
-    if (FINE) {
+    if (FINE && __any_sync(0xffffffffu, rounded != 0 || bad != 0)) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) rounded += (unsigned long long)shfl_xor_ll((long long)rounded, o);
         bad = __reduce_add_sync(0xffffffffu, bad);
@@ -478,8 +478,9 @@ static __global__ void k_bag_scale(float2 *__restrict__ gh, const int *__restric
 // The quantisation has used the round's maxima; those of the next round's gradients are collected from zero -- unless the
 // round will be built again, on the same gradients.  fine_K > 0: the first trees of a fine round of fine_K trees.
 __device__ inline void next_maxima(const unsigned long long *root_sum, int fine_K, unsigned *maxbits, TreeCtl *ctl) {
-    if (fine_K && grid_too_coarse(root_sum, fine_K)) ctl->coarse = 1;
-    if (!ctl->coarse) maxbits[0] = maxbits[1] = 0;
+    const bool again = ctl->coarse, now = fine_K && grid_too_coarse(root_sum, fine_K);
+    if (now) ctl->coarse = 1;
+    if (!again && !now) maxbits[0] = maxbits[1] = 0;
 }
 
 // Tree::init2 (src/thundergbm/tree.cu:8-39)
@@ -865,8 +866,8 @@ static __global__ void k_round_end(int objective, const double *sum, const doubl
                                    RoundState *rs,
                                    unsigned long long *root_sum, int n_root, const TreeCtl *ctl) {
     chain_wait();
+    const int coarse = ctl->coarse;
     for (int i = threadIdx.x; i < n_root; i += 32) root_sum[i] = 0;   // the next round adds to them
-    if (ctl->coarse) return;   // this one will be built again
     double t = 0;
     if (partial) {
         // (all loads first, then the additions in the usual order)
@@ -878,7 +879,7 @@ static __global__ void k_round_end(int objective, const double *sum, const doubl
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     }
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
+    if (threadIdx.x == 0 && blockIdx.x == 0 && !coarse) {   // (else the round will be built again)
         const int r = rs->round;
         if (objective >= 0) metric[r] = metric_from_sum(objective, partial ? t : *sum, n_total);
         if (r < log_len) qinfo_log[r] = *qinfo;

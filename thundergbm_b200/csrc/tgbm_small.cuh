@@ -99,6 +99,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
     const int f0 = min(F, rank * plan.feats), nf = min(F, f0 + plan.feats) - f0, bin0 = cut_ptr[f0], words = plan.nodes_pass * plan.bins;
     for (int r = threadIdx.x; r < N; r += SMALL_THREADS) node_of[r] = 0;
     chain_wait();
+    if (blockIdx.x == 0 && threadIdx.x == SMALL_THREADS - 1) next_maxima(root_sum, fine_K, maxbits, ctl);   // (a thread that has nothing else to do yet)
     const int2 *gq = ghq + (size_t)tree * N;
     const GridScale inv_sg(q->inv_sg), inv_sh(q->inv_sh);
     const unsigned char *ignored = ignored_all ? ignored_all + (size_t)rs->round * F : nullptr;
@@ -250,7 +251,6 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
     cluster.sync();   // nobody reads this CTA's candidates any more
     if (rank != 0) return;
     // -- pruning and the finished tree (k_prune)
-    if (blockIdx.x == 0 && threadIdx.x == 0) next_maxima(root_sum, fine_K, maxbits, ctl);
     if (threadIdx.x == 0) {
         atomicAdd(&ctl->stat_rows_root, (unsigned long long)N);
         atomicAdd(&ctl->stat_hists, 1ull);
