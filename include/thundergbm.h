@@ -168,7 +168,8 @@ void dense_train_scikit(int row_size, int n_cols, void *x, int is_f64, float *la
 void dense_predict_scikit(int row_size, int n_cols, void *x, int is_f64, float *y_pred, Tree **model,
                           int n_trees, int trees_per_iter, char *objective, int num_class, float learning_rate,
                           float *group_label, int verbose);
-/* number of distinct values (every NaN counts, +0 and -0 are one): the labels a group_label buffer must have room for */
+/* number of distinct values (every NaN counts, +0 and -0 are one): the labels a group_label buffer must have room for;
+ * -1 when there is no memory to count them in (tgbm_last_error()) */
 int tgbm_count_distinct(const float *v, long long n);
 
 /* Metric::get_score of the objective's default metric (the .cu files under src/thundergbm/metric, rank_metric.cpp) on raw scores

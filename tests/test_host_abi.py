@@ -4,6 +4,8 @@ import ctypes as C
 import os
 import re
 import struct
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -102,6 +104,23 @@ def test_distinct_labels_are_counted(lib, n, values):
         y[5:9] = np.nan
     want = len(np.unique(y[~np.isnan(y)] + 0.0)) + int(np.isnan(y).sum())
     assert lib.tgbm_count_distinct(y.ctypes.data_as(C.c_void_p), n) == want
+
+
+def test_counting_labels_without_memory_is_an_error(lib):
+    """No C++ exception leaves a C entry point: it would end the process."""
+    code = '''
+import ctypes as C, re, resource, sys
+import numpy as np
+from thundergbm_b200 import _lib
+lib = _lib.lib()
+lib.set_logger(0)
+y = np.arange(1 << 24, dtype=np.float32)
+used = int(re.search(r"VmSize:\\s+(\\d+)", open("/proc/self/status").read()).group(1)) << 10
+resource.setrlimit(resource.RLIMIT_AS, (used + (32 << 20), resource.RLIM_INFINITY))
+assert lib.tgbm_count_distinct(y.ctypes.data_as(C.c_void_p), y.size) == -1 and lib.tgbm_last_error()
+'''
+    r = subprocess.run([sys.executable, '-c', code], cwd=ROOT, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 def test_no_cpu_fallback_in_the_product():

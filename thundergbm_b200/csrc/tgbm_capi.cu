@@ -623,7 +623,11 @@ void tgbm_release_device_memory(void) {
     tgbm::dev_release_all();
 }
 
-int tgbm_count_distinct(const float *v, long long n) { return (int)tgbm::count_distinct(v, n); }
+int tgbm_count_distinct(const float *v, long long n) {
+    int r = -1;
+    guard([&] { r = (int)tgbm::count_distinct(v, n); });
+    return r;
+}
 
 int tgbm_metric_score(const char *objective, int n_rows, int trees_per_round, const float *label, const float *raw,
                       const int *group, int num_group, float *out) {
