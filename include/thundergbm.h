@@ -171,6 +171,10 @@ void dense_predict_scikit(int row_size, int n_cols, void *x, int is_f64, float *
 /* number of distinct values (every NaN counts, +0 and -0 are one): the labels a group_label buffer must have room for;
  * -1 when there is no memory to count them in (tgbm_last_error()) */
 int tgbm_count_distinct(const float *v, long long n);
+/* The same on a thread of its own.  `v` is read until tgbm_count_distinct_wait() returns, which gives the number and frees the
+ * handle; null / -1: as above. */
+void *tgbm_count_distinct_start(const float *v, long long n);
+int tgbm_count_distinct_wait(void *count);
 
 /* Metric::get_score of the objective's default metric (the .cu files under src/thundergbm/metric, rank_metric.cpp) on raw scores
  * raw[t * n_rows + i]: RMSE, binary error, multi-class accuracy, MAP or NDCG.  `label` holds class indices for the

@@ -117,3 +117,10 @@ def test_labels_of_the_model_are_its_own(gpu, n):
     m = TGBMRegressor(depth=3, n_trees=2, verbose=0, tree_method='hist').fit(x, y)
     y[:] = 1
     assert m.group_label == [0.0] * 251
+
+
+def test_failed_training_says_why(gpu):
+    from thundergbm_b200.thundergbm import TGBMRegressor
+    x = _matrix(70_000, 3, 0, np.float32)
+    with pytest.raises(RuntimeError, match='depth must be in'):
+        TGBMRegressor(depth=40, n_trees=2, verbose=0, tree_method='hist').fit(x, x[:, 0])

@@ -104,6 +104,7 @@ def test_distinct_labels_are_counted(lib, n, values):
         y[5:9] = np.nan
     want = len(np.unique(y[~np.isnan(y)] + 0.0)) + int(np.isnan(y).sum())
     assert lib.tgbm_count_distinct(y.ctypes.data_as(C.c_void_p), n) == want
+    assert lib.tgbm_count_distinct_wait(lib.tgbm_count_distinct_start(y.ctypes.data_as(C.c_void_p), n)) == want
 
 
 def test_counting_labels_without_memory_is_an_error(lib):

@@ -70,6 +70,8 @@ def load() -> C.CDLL:
     lib.dense_train_scikit.argtypes = [C.c_int, C.c_int, vp, C.c_int, vp] + lib.sparse_train_scikit.argtypes[5:]
     lib.dense_predict_scikit.argtypes = [C.c_int, C.c_int, vp, C.c_int, vp, vp, C.c_int, C.c_int, C.c_char_p, C.c_int, C.c_float, vp, C.c_int]
     lib.tgbm_count_distinct.argtypes = [vp, C.c_longlong]
+    lib.tgbm_count_distinct_start.argtypes, lib.tgbm_count_distinct_start.restype = [vp, C.c_longlong], vp
+    lib.tgbm_count_distinct_wait.argtypes = [vp]
     lib.save.argtypes = [C.c_char_p, C.c_char_p, C.c_float, C.c_int, C.c_int, C.c_int, vp, vp]
     lib.load_model.argtypes = [C.c_char_p, fp, ip, ip, ip, vp]
     lib.load_config.argtypes = [C.c_char_p, vp]

@@ -3,6 +3,7 @@
 #include <chrono>
 #include <climits>
 #include <cstring>
+#include <future>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -626,6 +627,23 @@ void tgbm_release_device_memory(void) {
 int tgbm_count_distinct(const float *v, long long n) {
     int r = -1;
     guard([&] { r = (int)tgbm::count_distinct(v, n); });
+    return r;
+}
+void *tgbm_count_distinct_start(const float *v, long long n) {
+    std::unique_ptr<std::future<long long>> f;
+    guard([&] {
+        f.reset(new std::future<long long>);
+        *f = std::async(std::launch::async, [v, n] { return tgbm::count_distinct(v, n); });
+    });
+    return f && f->valid() ? f.release() : nullptr;
+}
+int tgbm_count_distinct_wait(void *count) {
+    int r = -1;
+    guard([&] {
+        std::unique_ptr<std::future<long long>> f(static_cast<std::future<long long> *>(count));
+        TGBM_CHECK(f != nullptr, "no count was started");
+        r = (int)f->get();
+    });
     return r;
 }
 
