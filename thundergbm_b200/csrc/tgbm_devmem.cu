@@ -22,11 +22,9 @@
 
 #include <algorithm>
 #include <atomic>
-#include <condition_variable>
 #include <cstdlib>
 #include <cstdint>
 #include <cstring>
-#include <deque>
 #include <functional>
 #include <iterator>
 #include <map>
@@ -38,6 +36,7 @@
 
 #include "tgbm_common.h"
 #include "tgbm_device.cuh"
+#include "tgbm_workers.h"
 
 namespace tgbm {
 namespace {
@@ -285,6 +284,16 @@ bool copy_low16(uint16_t *dst, const int *src, size_t n) {
 
 struct Worker {
     Lane lanes[MAX_DEVICES];
+    Worker() = default;
+    Worker(const Worker &) = delete;
+    Worker &operator=(const Worker &) = delete;
+    ~Worker() {   // (of a caller that works itself; the threads keep theirs)
+        for (Lane &l : lanes) {
+            for (cudaEvent_t e : l.done)
+                if (e) cudaEventDestroy(e);
+            if (l.st) cudaStreamDestroy(l.st);
+        }
+    }
     Lane &lane(int dev) {
         Lane &l = lanes[dev];
         if (!l.st) {
@@ -295,46 +304,11 @@ struct Worker {
     }
 };
 
-class Pool {
-public:
-    // runs f(worker, t) for t = 0 .. n - 1 on the workers and returns when all have returned; f must not throw
-    void run(int n, const std::function<void(Worker &, int)> &f) {
-        Job job{&f, n};
-        std::unique_lock<std::mutex> lock(mutex_);
-        for (int t = 0; t < n; ++t) queue_.push_back({&job, t});
-        for (; started_ < WORKERS && idle_ + starting_ < (int)queue_.size(); ++started_, ++starting_) std::thread(&Pool::loop, this).detach();
-        wake_.notify_all();
-        done_.wait(lock, [&] { return job.left == 0; });
-    }
-
-private:
-    struct Job { const std::function<void(Worker &, int)> *f; int left; };
-    struct Task { Job *job; int t; };
-    void loop() {
-        Worker w;
-        std::unique_lock<std::mutex> lock(mutex_);
-        --starting_;
-        for (;;) {
-            ++idle_;
-            wake_.wait(lock, [&] { return !queue_.empty(); });
-            --idle_;
-            const Task task = queue_.front();
-            queue_.pop_front();
-            lock.unlock();
-            (*task.job->f)(w, task.t);
-            lock.lock();
-            if (--task.job->left == 0) done_.notify_all();
-        }
-    }
-    std::mutex mutex_;
-    std::condition_variable wake_, done_;
-    std::deque<Task> queue_;
-    int started_ = 0, starting_ = 0, idle_ = 0;
-};
+using Pool = WorkerPool<Worker>;
 
 // never destroyed: the workers wait on it until the process ends
 Pool &pool() {
-    static Pool *p = new Pool;
+    static Pool *p = new Pool(WORKERS);
     return *p;
 }
 
