@@ -16,6 +16,7 @@
 // back to TGBM_POOL_KEEP_MB megabytes per device (default 16384; 0 = keep nothing), largest blocks first.
 // TGBM_NO_POOL=1 selects plain cudaMalloc / cudaFree.
 #include <cuda_runtime.h>
+#include <pthread.h>
 #if defined(__x86_64__)
 #include <immintrin.h>
 #endif
@@ -306,9 +307,18 @@ struct Worker {
 
 using Pool = WorkerPool<Worker>;
 
-// never destroyed: the workers wait on it until the process ends
+// Never destroyed: the workers wait on it until the process ends.  A process that fork() made has no workers, so it gets a
+// pool of its own.
 Pool &pool() {
-    static Pool *p = new Pool(WORKERS);
+    static std::atomic<Pool *> current{nullptr};
+    static const int registered = pthread_atfork(nullptr, nullptr, [] { current = nullptr; });
+    (void)registered;
+    Pool *p = current;
+    if (!p) {
+        Pool *made = new Pool(WORKERS);
+        if (current.compare_exchange_strong(p, made)) p = made;
+        else delete made;
+    }
     return *p;
 }
 
