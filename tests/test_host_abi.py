@@ -124,6 +124,20 @@ assert lib.tgbm_count_distinct(y.ctypes.data_as(C.c_void_p), y.size) == -1 and l
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+@pytest.mark.parametrize('n,builder,refused', [((1 << 30) - 2048, 'hist', False), ((1 << 30) - 2047, 'hist', True), ((1 << 30) - 2047, 'exact', False)])
+def test_rows_beyond_the_record_lists_are_refused(lib, n, builder, refused):
+    """Before anything is allocated.  (The arrays are zeros that nobody touches: no memory behind them.)"""
+    from thundergbm_b200.booster import Booster
+    from thundergbm_b200.synth import CsrData
+    import torch
+    if torch.cuda.is_available():
+        pytest.skip('what is not refused would be trained')
+    empty = np.zeros(0, np.float32)
+    with pytest.raises(RuntimeError) as e:
+        Booster(CsrData(n, 1, np.zeros(n + 1, np.int32), np.zeros(0, np.int32), empty, np.zeros(n, np.float32)), tree_method=builder)
+    assert ('rows per GPU' in str(e.value)) == refused   # (without a GPU the others end at the first CUDA call)
+
+
 def test_no_cpu_fallback_in_the_product():
     """The product never reaches for the oracle."""
     pkg = os.path.join(ROOT, 'thundergbm_b200')

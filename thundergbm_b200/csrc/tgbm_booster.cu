@@ -737,6 +737,21 @@ void Booster::init(const DataSet &ds) {
     TGBM_CHECK(p.quant_bits >= 8 && p.quant_bits <= 20, "quant_bits must be in [8, 20]");
     TGBM_CHECK(p.hist_mode == 0 || p.hist_mode == 1, "hist_mode must be 0 (fp32) or 1 (exact)");
     m.f32 = p.hist_mode == 0;
+    // Every phase that can fail on one rank alone (a check of this rank's input, an allocation) runs under `locally`
+    // and is followed by an agreement of all ranks, so that no rank enters a collective its peers will never join.
+    const bool multi = m.comm && m.comm->active();
+    std::string local_err;
+    auto locally = [&](auto &&phase) {
+        if (!local_err.empty()) return;
+        try { phase(); } catch (const std::exception &e) { local_err = e.what(); }
+    };
+    auto agree = [&](const char *what) {
+        if (multi) m.comm->agree(local_err, what, m.stream);
+        else if (!local_err.empty()) throw Error(local_err);
+    };
+    auto check_rows = [&] { TGBM_CHECK(ds.n_rows <= MAX_HIST_ROWS, "at most " + std::to_string(MAX_HIST_ROWS) + " rows per GPU"); };
+    if (p.tree_method == "hist") locally(check_rows);
+    if (!multi) agree("");   // (nothing has been allocated; ranks tell each other below)
     TGBM_CHECK(p.column_sampling_rate > 0.f, "column_sampling_rate must be positive");
     int dev = 0;
     TGBM_CUDA(cudaGetDevice(&dev));
@@ -747,23 +762,13 @@ void Booster::init(const DataSet &ds) {
     m.depth = p.depth;
     m.n_nodes = (1 << (p.depth + 1)) - 1;
     m.label = ds.label;
-    const bool multi = m.comm && m.comm->active();
-    // Every phase that can fail on one rank alone (a check of this rank's input, an allocation) runs under `locally`
-    // and is followed by an agreement of all ranks, so that no rank enters a collective its peers will never join.
-    std::string local_err;
-    auto locally = [&](auto &&phase) {
-        try { phase(); } catch (const std::exception &e) { local_err = e.what(); }
-    };
-    auto agree = [&](const char *what) {
-        if (multi) m.comm->agree(local_err, what, m.stream);
-        else if (!local_err.empty()) throw Error(local_err);
-    };
     // (buffers of the collectives are allocated inside the local phases too: between an agreement and the launch of the
     // collective no rank makes a call that could wait for another device -- cudaMalloc can, once peer access is on)
     DevBuf<long long> mine, all;
     locally([&] {
         if (need_group_file(m.objective)) RankState::validate(ds, m.N);
         m.upload_rows(ds);
+        if (p.tree_method == "auto" && m.F <= 20000) check_rows();   // (it will be the histogram builder)
         if (multi) { mine.alloc(3); all.alloc(3 * (size_t)m.comm->world); }
     });
     agree("loading its rows");

@@ -154,6 +154,10 @@ struct DataSet {
     void group_label();
 };
 
+// The histogram builder's record lists hold the right children behind the left ones, at most twice the rows, and a kernel
+// looks up to a tile beyond the last: positions are ints.
+constexpr int MAX_HIST_ROWS = (1 << 30) - 2048;
+
 // f(0) ... f(n - 1) on the library's standing worker threads (tgbm_devmem.cu); returns when all have returned
 void host_parallel(int n, const std::function<void(int)> &f);
 int upload_threads();   // how many of them one call should use: TGBM_UPLOAD_THREADS, else all cores but one, at most 15
