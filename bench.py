@@ -12,7 +12,8 @@ Prints one JSON line on rank 0:
   value     seconds per 100 boosting rounds for the boosting loop with the bin matrix resident in HBM (the scope of
             the reference's own "training time" line, src/thundergbm/trainer.cu:42-50), in the library's default
             histogram arithmetic (fp32: float sums value by value in the first round, like the reference, then
-            integer sums of the float gradients on a grid of 2^-30 of the largest)
+            integer sums of the float gradients on a grid of 2^-30 of the largest).  The warm-up rounds come first, so
+            the first round is not in it; it is in e2e, which trains from the start
   deterministic_mode   the same loop in the exact fixed-point mode (bit-identical from run to run and for any number
             of GPUs), with the roofline of its histogram kernel
   e2e       the same unit through the reference's C entry point (sparse_train_scikit) with host CSR buffers: copies,
@@ -68,6 +69,19 @@ WORKLOADS = {
 # dram__bytes_read.sum + dram__bytes_write.sum per launch (mean over a tree) of the histogram kernel of either mode on config 2, from the
 # ncu captures summarised under profiles/ (None: no capture of that kernel yet)
 NCU_TRAFFIC_BYTES_PER_LAUNCH = {'exact': 356.1e6, 'fp32': 350.3e6}
+
+
+def hist_limiter(mode, csr, pairs_per_s):
+    """What the histogram kernel issues per (row, feature) pair, and its rate against that of the bare operations."""
+    if csr:   # no rate of the bare operations was measured for this mix
+        return {'limiter': 'four 32-bit shared-memory atomics per value of the first 12288 bins, two 64-bit global reductions per other value (either mode)',
+                'pairs_per_s': pairs_per_s, 'pair_peak_per_s': None, 'limiter_frac': None, 'pair_peak_kind': None}
+    # dense layout: one 32-bit atomic per component in exact mode, two (low and high half of a 31-bit value) in fp32 mode.  In
+    # fp32 mode they bound the kernel; in exact mode it reaches a quarter of their rate and what bounds it is not known.
+    peak = {'fp32': 294e6 / 0.134e-3, 'exact': 294e6 / 0.073e-3}[mode]
+    return {'limiter': {'fp32': 'shared-memory atomics (4 per row and feature)', 'exact': 'not known (2 shared-memory atomics per row and feature)'}[mode],
+            'pairs_per_s': pairs_per_s, 'pair_peak_per_s': peak, 'limiter_frac': pairs_per_s / peak if pairs_per_s else None,
+            'pair_peak_kind': 'microbenchmark on a B200: the bare atomics of 294 M (row, feature) pairs, conflict-free'}
 
 
 def make_shard(config, n_rows, rank, world):
@@ -432,15 +446,8 @@ def main():
                 'hist_share_of_step': prof.hist_ms / ms_prof if ms_prof > 0 else None,
                 'partition_share_of_step': prof.partition_ms / ms_prof if ms_prof > 0 else None,
                 'measured_on': f'{k_prof} rounds directly after the timed region, per-kernel CUDA events (ms_per_step there {ms_prof / k_prof:.3f})'}
-        # the kernel is bound by its shared-memory atomics, not by HBM: one 32-bit atomic per component and (row, feature) in
-        # exact mode, two (low and high half of a 31-bit value) in fp32 mode
-        pair_peak = {'fp32': 294e6 / 0.134e-3, 'exact': 294e6 / 0.073e-3}[mode]
         pairs = float(prof.hist_rows) * data.nnz / max(1, data.n_rows)  # (row, feature) pairs of the processed rows
-        roof['limiter'] = 'shared-memory atomics (%d per row and feature)' % (4 if mode == 'fp32' else 2)
-        roof['pairs_per_s'] = pairs / (prof.hist_ms * 1e-3) if prof.hist_ms > 0 else None
-        roof['pair_peak_per_s'] = pair_peak
-        roof['limiter_frac'] = roof['pairs_per_s'] / pair_peak if roof['pairs_per_s'] else None
-        roof['pair_peak_kind'] = 'microbenchmark on this pool: the bare atomics of 294 M (row, feature) pairs, conflict-free'
+        roof.update(hist_limiter(mode, bool(info.csr_layout), pairs / (prof.hist_ms * 1e-3) if prof.hist_ms > 0 else None))
         return dict(ms_max=ms_max, launches=launches_timed, roofline=roof, t_init=t_init, info=info, trees=trees, logloss=ll,
                     final_metric=float(metrics_timed[w + k - 1]) if len(metrics_timed) >= w + k else None)
 
