@@ -352,7 +352,8 @@ static __global__ void k_grad_softmax(const float *y, const float *yp, int n, in
 // `gh` null: the gradients are those of a pointwise objective (`logistic` 0/1) and are computed again from y and the
 // scores here -- the pass that found their maxima (k_predict_walk) did not store them.
 template <bool FINE>
-static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbits, int quant_bits,
+static __global__ void __launch_bounds__(256, 8)   // (the grid is one full wave of eight blocks per SM)
+k_quantize(const float2 *gh, int n, const unsigned *maxbits, int quant_bits,
                            uint32_t round, uint32_t row_offset, int2 *ghq,
                            unsigned long long *root_sum, QuantInfo *qinfo,
                            const float *y, const float *yp, int logistic,
@@ -369,7 +370,7 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
     const bool in_float = sg < 1e38 && sh < 1e38;
     const float fg = (float)sg, fh = (float)sh;
     unsigned long long rounded = 0;
-    int bad = 0;
+    bool bad = false;
     long long tg = 0, th = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float2 v = gh ? gh[(size_t)k * n + i] : pointwise_gh(logistic, y[i], yp[i]);
@@ -377,18 +378,18 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
         if (FINE) {
             // the scale is a power of two: where a float holds it, the product is exact in float, and the conversions to and from
             // double (a sixteenth of the float rate) can go
-            bool off;   // the gradient is not on the grid
+            bool off;   // the gradient is not on the grid (one of 23 bits and more counts as if it were)
             if (in_float) {
                 const float pg = __fmul_rn(v.x, fg);
                 qg = __float2int_rn(pg); qh = __float2int_rn(__fmul_rn(v.y, fh));
-                off = __int2float_rn(qg) != pg;
+                off = fabsf(pg) < 4194304.f && __fadd_rn(__fadd_rn(pg, 12582912.f), -12582912.f) != pg;
             } else {
                 const double pg = (double)v.x * sg;
                 qg = __double2int_rn(pg); qh = __double2int_rn((double)v.y * sh);
                 off = (double)qg != pg;
             }
             if (off) rounded += (unsigned)qh >> (31 - __clz(abs(qg) | 1));
-            bad += !(fabsf(v.x) < INFINITY) || !(v.y < INFINITY);
+            bad |= !(fabsf(v.x) + v.y < INFINITY);   // (hessians are not negative)
         } else {
         const uint32_t row = row_offset + (uint32_t)i;
         const double ug = (double)mix32(0x9E3779B9u, round, (uint32_t)k, row) * (1.0 / 4294967296.0);
@@ -400,10 +401,10 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) { tg += shfl_xor_ll(tg, o); th += shfl_xor_ll(th, o); }
-    if (FINE && __any_sync(0xffffffffu, rounded != 0 || bad != 0)) {
+    if (FINE && __any_sync(0xffffffffu, rounded != 0 || bad)) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) rounded += (unsigned long long)shfl_xor_ll((long long)rounded, o);
-        bad = __reduce_add_sync(0xffffffffu, bad);
+        bad = __any_sync(0xffffffffu, bad);
     }
     // one pair of atomics per block: all go to the same two words, and one pair per warp made 19 k of them at 1 M rows, 12 of
     // the kernel's 19 us
@@ -433,7 +434,7 @@ static __global__ void k_quantize(const float2 *gh, int n, const unsigned *maxbi
 // gradients are multiples of the grid; one label of 1e9 among normal ones to 2^-1.
 // Hessians need no such test: sum h + lambda loses at most 2^-31 of the largest per row, the float sums lose 2^-24 of the
 // node's whole sum to one of its children (what the node's sum and the sum over its bins differ by counts as missing rows).
-// root_sum[2 K + 1]: gradients that are not finite.  One is enough: float sums carry it on, the grid does not.
+// root_sum[2 K + 1]: not zero if a gradient is not finite.  One is enough: float sums carry it on, the grid does not.
 __device__ inline bool grid_too_coarse(const unsigned long long *root_sum, int K) {
     unsigned long long h = 0;
     for (int k = 0; k < K; ++k) h += root_sum[2 * k + 1];
