@@ -138,6 +138,15 @@ def test_rows_beyond_the_record_lists_are_refused(lib, n, builder, refused):
     assert ('rows per GPU' in str(e.value)) == refused   # (without a GPU the others end at the first CUDA call)
 
 
+@pytest.mark.parametrize('rounds,per_round', [(0, 1), (1, 0)])
+def test_an_empty_model_is_refused_whatever_the_rows(lib, rounds, per_round):
+    rp, out = np.zeros(1, np.int32), np.zeros(1, np.float32)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    lib.set_logger(0)
+    assert lib.tgbm_predict_raw(0, None, p(rp), None, p(np.zeros(144, np.uint8)), rounds, per_round, 3, 0.1, 0.0, p(out)) != 0
+    assert b'empty model' in lib.tgbm_last_error()
+
+
 def test_no_cpu_fallback_in_the_product():
     """The product never reaches for the oracle."""
     pkg = os.path.join(ROOT, 'thundergbm_b200')

@@ -674,6 +674,7 @@ int tgbm_predict_raw_timed(int n_rows, const float *val, const int *row_ptr, con
     return guard([&] {
         tgbm::DataSet ds;
         ds.view_sparse(n_rows, val, row_ptr, col);
+        TGBM_CHECK(n_rounds > 0 && trees_per_round > 0, "empty model");
         tgbm::ModelRef ref;
         ref.n_rounds = n_rounds; ref.K = trees_per_round; ref.n_nodes = n_nodes;
         const tgbm::TreeNode *src = (const tgbm::TreeNode *)nodes;
