@@ -775,6 +775,7 @@ void Booster::init(const DataSet &ds) {
 
     // global row count, this rank's row offset, global feature count, query groups before this rank's
     m.N_global = m.N;
+    long long most_rows = m.N;   // of a rank
     m.row_offset = 0;
     long long first_group = 0, total_groups = (long long)ds.group.size();
     if (multi) {
@@ -789,6 +790,7 @@ void Booster::init(const DataSet &ds) {
         for (int r = 0; r < m.comm->world; ++r) {
             if (r < m.comm->rank) { m.row_offset += ha[3 * r]; first_group += ha[3 * r + 2]; }
             m.N_global += ha[3 * r];
+            most_rows = std::max(most_rows, ha[3 * r]);
             m.F = std::max<int>(m.F, (int)ha[3 * r + 1]);
             total_groups += ha[3 * r + 2];
         }
@@ -891,7 +893,8 @@ void Booster::init(const DataSet &ds) {
         b.bits_stride = (size_t)m.max_tiles * (PART_TILE / 32);
         b.tile_stride = m.max_tiles;
         b.ticket_stride = max_pairs;
-        const double per_tree = 24.0 * b.rec_stride + 8.0 * (b.full_stride + b.built_stride) + 4.0 * b.bits_stride;
+        // (the same number on every rank: it decides the order of the collectives)
+        const double per_tree = 48.0 * (double)(std::max(most_rows, 1ll) + F32_THREADS) + 8.0 * (b.full_stride + b.built_stride) + (double)most_rows / 8;
         m.batch = m.exact ? 1 : std::max(1, std::min(K, (int)(6e9 / per_tree)));
         m.part_ctas = std::max(1, std::min(m.max_tiles, m.num_sms * (2048 / PART_THREADS) / m.batch));
         b.tail_stride = m.part_ctas;
