@@ -623,7 +623,7 @@ void BoosterImpl::init_exact() {
         DevBuf<unsigned long long> keys, keys2;
         DevBuf<int> rows;
         keys.alloc(n1); keys2.alloc(n1); rows.alloc(n1);
-        for (int i = 0; i < (depth > 1 ? 3 : 1); ++i) { ex_key[i].alloc(padded); ex_row[i].alloc(padded); ex_val[i].alloc(padded); ex_gh[i].alloc(padded); }
+        ex_key[0].alloc(padded); ex_row[0].alloc(padded); ex_val[0].alloc(padded);
         if (N) k_exact_rows<<<std::min(ceil_div(N, 256), num_sms * 16), 256, 0, stream>>>(in.row_ptr.p, N, rows.p);
         if (nnz) k_exact_csc_keys<<<grid, 256, 0, stream>>>(in.val.p, in.col.p, nnz, keys.p);
         int end_bit = 32;
@@ -639,6 +639,9 @@ void BoosterImpl::init_exact() {
         }
     }
     in.release();
+    // (not before the sort's buffers are gone: with them 2 G stored values would not fit)
+    ex_gh[0].alloc(padded);
+    for (int i = 1; i < (depth > 1 ? 3 : 1); ++i) { ex_key[i].alloc(padded); ex_row[i].alloc(padded); ex_val[i].alloc(padded); ex_gh[i].alloc(padded); }
     // no cut points, no bin matrix
     B = 0; sparse = false;
     h_cut_ptr.assign(F + 1, 0);
