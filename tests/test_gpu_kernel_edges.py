@@ -133,3 +133,25 @@ def test_rows_of_the_csr_layout(gpu, orc, monkeypatch, longest):
     x = r.integers(1, 9, (n, f)).astype(np.float32)
     d = _holes(x, (x * keep)[:, :20].sum(1) + r.random(n), keep)
     _same_as_oracle(orc, d, depth=6, n_trees=3, max_num_bin=16, learning_rate=0.5, objective='reg:linear')
+
+
+# the trees of a round stand side by side in as much memory as there is, one by one if need be: the same trees
+def test_softmax_trees_in_little_memory(gpu):
+    import torch
+    from thundergbm_b200 import _lib
+    from thundergbm_b200.booster import Booster
+    r = np.random.default_rng(3)
+    x = r.standard_normal((3000, 30)).astype(np.float32)
+    d = _csr(x, (x[:, 0] > 0) + 2 * (x[:, 1] > 0) + 3 * (x[:, 2] > 1))
+    got = []
+    for fill in (False, True):
+        _lib.lib().tgbm_release_device_memory()
+        torch.cuda.empty_cache()
+        filler = torch.empty(torch.cuda.mem_get_info()[0] - (1500 << 20), dtype=torch.uint8, device='cuda') if fill else None
+        b = Booster(d, depth=12, n_trees=2, objective='multi:softmax', num_class=7, hist_mode='exact')   # 0.6 GB per tree
+        b.boost(2)
+        got.append((b.trees().tobytes(), b.ypred().tobytes()))
+        b.close()
+        del filler
+    torch.cuda.empty_cache()
+    assert got[0] == got[1]

@@ -881,7 +881,8 @@ void Booster::init(const DataSet &ds) {
     const int max_pairs = std::max(1, 1 << std::max(0, depth - 2));
     m.max_tiles = ceil_div(N, PART_TILE) + (1 << depth) + 2;
     {
-        // trees built side by side: all of a round's while their buffers stay within 6 GB
+        // trees built side by side: all of a round's while their buffers stay within 6 GB, and within an eighth of what is free
+        // on a single GPU (ranks must agree on the number)
         Batch &b = m.bufs;
         b.half = (int)n1;
         b.nodes_stride = m.n_nodes;
@@ -898,7 +899,13 @@ void Booster::init(const DataSet &ds) {
         b.ticket_stride = max_pairs;
         // (the same number on every rank: it decides the order of the collectives)
         const double per_tree = 48.0 * (double)(std::max(most_rows, 1ll) + F32_THREADS) + 8.0 * (b.full_stride + b.built_stride) + (double)most_rows / 8;
-        m.batch = m.exact ? 1 : std::max(1, std::min(K, (int)(6e9 / per_tree)));
+        double room = 6e9;
+        if (K > 1 && !multi) {
+            size_t free_bytes = 0, all_bytes = 0;
+            TGBM_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes));
+            room = std::min(room, free_bytes / 8.0);
+        }
+        m.batch = m.exact ? 1 : std::max(1, std::min(K, (int)(room / per_tree)));
         m.part_ctas = std::max(1, std::min(m.max_tiles, m.num_sms * (2048 / PART_THREADS) / m.batch));
         b.tail_stride = m.part_ctas;
         const size_t T = m.batch;
