@@ -78,7 +78,7 @@ def test_cut_points_of_full_columns(gpu, n):
     b.close()
 
 
-# more rows per CTA than the 16-bit halves of one window hold: 149 groups of columns leave one CTA each
+# more rows per CTA than the 16-bit halves of one window hold: 150 groups of columns leave one CTA each
 def test_window_of_the_halved_sums(gpu):
     from thundergbm_b200.booster import Booster
     n, f = 70_001, 4 * 1200
@@ -88,6 +88,7 @@ def test_window_of_the_halved_sums(gpu):
     b = Booster(_csr(x, 1e3 * cols[:, 0] + cols[:, 1]), depth=3, n_trees=3, max_num_bin=16, objective='reg:linear', hist_mode='fp32', keep_nid=1)
     b.boost(3)
     trees, nid = b.trees()[:, 0], b.nid().reshape(3, n)
+    assert (b.quant_scale()[1:] != 1).all()   # the later rounds did sum on the grid
     for t in range(1, 3):   # hessian 1: a node's sum is its number of rows
         for i in np.unique(nid[t]):
             at, rows = int(i), nid[t] == i
