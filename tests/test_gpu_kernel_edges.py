@@ -156,3 +156,13 @@ def test_softmax_trees_in_little_memory(gpu):
         del filler
     torch.cuda.empty_cache()
     assert got[0] == got[1]
+
+
+# chunks of 1024 rows with remainders, few and many children, several chunks per block; trees side by side in chunks of 2048 rows
+@pytest.mark.parametrize('n,f,depth,classes,layout', [(1, 3, 3, 1, 'sparse'), (255, 5, 4, 1, 'sparse'), (1025, 5, 6, 1, 'sparse'), (2049, 3, 9, 1, 'sparse'),
+                                                      (32_769, 4, 1, 1, 'dense'), (33_793, 4, 2, 1, 'dense'), (40_961, 5, 10, 1, 'dense'),
+                                                      (180_225, 4, 5, 7, 'dense')])
+def test_rows_to_children(gpu, orc, monkeypatch, n, f, depth, classes, layout):
+    monkeypatch.setenv('TGBM_LAYOUT', layout)
+    p = dict(depth=depth, n_trees=3, max_num_bin=64, learning_rate=0.5, objective='multi:softmax' if classes > 1 else 'reg:linear', num_class=classes)
+    _same_as_oracle(orc, _data(n, f, classes, n), **p)

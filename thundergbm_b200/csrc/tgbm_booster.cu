@@ -64,9 +64,11 @@ struct BoosterImpl {
     // stride behind the one before
     int batch = 1;
     Batch bufs{};
-    DevBuf<int> rec_idx[2];
-    DevBuf<int2> rec_gh[2];
-    DevBuf<int> seg_begin[2], seg_cnt[2];
+    DevBuf<int> rec_idx;
+    DevBuf<unsigned short> nid;
+    DevBuf<int> seg_begin[2], seg_cnt[2], origin[2];
+    DevBuf<float> leaf_weight;
+    DevBuf<AssignRule> leaf_rule;
     DevBuf<int> nid_keep;
     DevBuf<long long> hist_full, hist_built;
     // fp32 mode: the same two buffers hold float pairs; `hist_spread` receives the built histograms, their cells
@@ -105,16 +107,19 @@ struct BoosterImpl {
     void wait() const;
     bool settle();
     DevBuf<int> eval_ticket;  // k_eval: finished blocks per sibling pair, zero between launches
-    int part_ctas = 1;
+    int assign_ctas = 1, assign_rpt = 4;
+    auto assign_kernel(int level) const {
+        auto pick = [&](auto many, auto k0, auto k1, auto k2) { return level == 0 ? k0 : level == 1 ? k1 : level == 2 ? k2 : many; };
+        if (sparse) return pick(k_assign<true, 4, 0>, k_assign<true, 4, 1>, k_assign<true, 4, 2>, k_assign<true, 4, 3>);
+        if (assign_rpt == 8) return pick(k_assign<false, 8, 0>, k_assign<false, 8, 1>, k_assign<false, 8, 2>, k_assign<false, 8, 3>);
+        return pick(k_assign<false, 4, 0>, k_assign<false, 4, 1>, k_assign<false, 4, 2>, k_assign<false, 4, 3>);
+    }
     bool grad_max_ready = false;        // maxbits holds the maxima of the next round's gradients
     bool metric_partial_ready = false;  // metric_partial holds the finished round's partial sums
     int metric_blocks() const { return std::max(1, std::min((N + 255) / 256, std::min(num_sms * 8, METRIC_PARTS))); }   // of 256 threads: one full wave
     DevBuf<SplitRec> recs;
-    DevBuf<int> tile_left, tail_left;
-    DevBuf<unsigned> bits;
     DevBuf<TreeCtl> ctl;
     DevBuf<double> metric_partial, metric_sum;
-    int max_tiles = 0;
     RankState rank;
 
     struct TimedEvent { cudaEvent_t a, b; int kind; };
@@ -161,6 +166,11 @@ struct BoosterImpl {
 };
 
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+// shared memory of k_assign at a level: rules, counts, offsets (up to depth 13: 32 bytes per node), staged rows
+static inline size_t assign_smem(int level, int rpt) {
+    const size_t nl = (size_t)1 << level;
+    return sizeof(ChunkRule) * (nl + 1) + sizeof(unsigned) * ASSIGN_THREADS * rpt + 3 * sizeof(int) * (2 * nl + 1);
+}
 
 void BoosterImpl::upload_rows(const DataSet &ds) {
     // fewer threads per rank when the ranks of one process upload side by side
@@ -596,7 +606,7 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
         TGBM_CUDA(cudaStreamSynchronize(stream));
     } else {
         bins.alloc((size_t)N * Fpad);
-        binsT.alloc((size_t)F * Npad);
+        binsT.alloc((size_t)F * Npad + ASSIGN_CHUNK);   // (k_assign reads the first column to the end of a chunk)
         TGBM_CUDA(cudaMemsetAsync(bins.p, MISSING_BIN, bins.bytes(), stream));
         TGBM_CUDA(cudaMemsetAsync(binsT.p, MISSING_BIN, binsT.bytes(), stream));
         if (N) k_bin_dense<<<ceil_div(N, 128), 128, 0, stream>>>(in.row_ptr.p, in.col.p, in.val.p, in.full_cols, N, cut_ptr.p, cut_val.p, Fpad, Npad, bins.p, binsT.p, colb ? 1 : 0);
@@ -714,7 +724,7 @@ void BoosterImpl::build_tree_exact(int round, int k) {
     if (f32) exact_levels<float>(k, gh.p + (size_t)k * N);
     else exact_levels<long long>(k, ghq.p + (size_t)k * N);
     k_prune<<<1, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream>>>(nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0, model.p, K, k,
-                                                                                         rstate.p);
+                                                                                         rstate.p, nullptr, nullptr, 0, 0);
     if (N) {
         int *nid_out = p.keep_nid ? nid_keep.p + (size_t)tree_index * N : nullptr;
         k_exact_predict<<<std::min(ceil_div(N, 256), num_sms * 8), 256, 0, stream>>>(ex_nid.p, N, nodes.p, p.learning_rate, ypred.p + (size_t)k * N, nid_out);
@@ -879,7 +889,6 @@ void Booster::init(const DataSet &ds) {
     m.qinfo_log.alloc(std::max(p.n_trees, 1) + 1);
     const size_t B1 = std::max(m.B, 1);
     const int max_pairs = std::max(1, 1 << std::max(0, depth - 2));
-    m.max_tiles = ceil_div(N, PART_TILE) + (1 << depth) + 2;
     {
         // trees built side by side: all of a round's while their buffers stay within 6 GB, and within an eighth of what is free
         // on a single GPU (ranks must agree on the number)
@@ -887,18 +896,18 @@ void Booster::init(const DataSet &ds) {
         b.half = (int)n1;
         b.nodes_stride = m.n_nodes;
         b.seg_stride = (size_t)1 << depth;
-        // left children in the first half, right children in the second; the bulk copies that stage a unit of records read
-        // up to a unit beyond the last record, from a 16-byte boundary
+        // left children in the first half, right children in the second; the bulk copies that stage a unit of row ids read
+        // up to a unit beyond the last one, from a 16-byte boundary
         b.rec_stride = (2 * n1 + 2 * F32_THREADS + 3) / 4 * 4;
+        b.nid_stride = (n1 + ASSIGN_CHUNK - 1) / ASSIGN_CHUNK * ASSIGN_CHUNK;
         b.gh_stride = N;
         b.full_stride = (((size_t)1 << depth) - 1) * B1 * 2;
         b.built_stride = max_pairs * B1 * 2;
         b.recs_stride = m.exact ? 1 : ((size_t)1 << (depth - 1)) * (m.sparse ? std::max(m.n_chunks, 1) : m.F);
-        b.bits_stride = (size_t)m.max_tiles * (PART_TILE / 32);
-        b.tile_stride = m.max_tiles;
         b.ticket_stride = max_pairs;
+        b.rule_stride = (size_t)1 << (depth - 1);
         // (the same number on every rank: it decides the order of the collectives)
-        const double per_tree = 48.0 * (double)(std::max(most_rows, 1ll) + F32_THREADS) + 8.0 * (b.full_stride + b.built_stride) + (double)most_rows / 8;
+        const double per_tree = 10.0 * (double)(std::max(most_rows, 1ll) + F32_THREADS) + 8.0 * (b.full_stride + b.built_stride);
         double room = 6e9;
         if (K * per_tree > 512e6 && K > 1 && !multi) {   // (asking takes 0.4 ms)
             size_t free_bytes = 0, all_bytes = 0;
@@ -906,24 +915,24 @@ void Booster::init(const DataSet &ds) {
             room = std::min(room, free_bytes / 8.0);
         }
         m.batch = m.exact ? 1 : std::max(1, std::min(K, (int)(room / per_tree)));
-        m.part_ctas = std::max(1, std::min(m.max_tiles, m.num_sms * (2048 / PART_THREADS) / m.batch));
-        b.tail_stride = m.part_ctas;
+        m.assign_rpt = !m.sparse && (long long)N * m.batch >= 4ll * m.num_sms * 8 * ASSIGN_THREADS ? 8 : 4;
+        m.assign_ctas = std::max(1, std::min(ceil_div(N, ASSIGN_THREADS * m.assign_rpt), m.num_sms * (m.assign_rpt == 8 ? 4 : 6) / m.batch));
         const size_t T = m.batch;
         m.nodes.alloc(T * b.nodes_stride); b.nodes = m.nodes.p;
         for (int i = 0; i < 2; ++i) {
-            m.rec_idx[i].alloc(T * b.rec_stride); m.rec_gh[i].alloc(T * b.rec_stride);
-            m.seg_begin[i].alloc(T * b.seg_stride); m.seg_cnt[i].alloc(T * b.seg_stride);
+            m.seg_begin[i].alloc(T * b.seg_stride); m.seg_cnt[i].alloc(T * b.seg_stride); m.origin[i].alloc(T * b.seg_stride);
             m.seg_begin[i].zero(m.stream); m.seg_cnt[i].zero(m.stream);
-            b.rec_idx[i] = m.rec_idx[i].p; b.rec_gh[i] = m.rec_gh[i].p;
-            b.seg_begin[i] = m.seg_begin[i].p; b.seg_cnt[i] = m.seg_cnt[i].p;
+            b.seg_begin[i] = m.seg_begin[i].p; b.seg_cnt[i] = m.seg_cnt[i].p; b.origin[i] = m.origin[i].p;
         }
+        m.rec_idx.alloc(T * b.rec_stride); b.rec_idx = m.rec_idx.p;
+        m.nid.alloc(T * b.nid_stride); b.nid = m.nid.p;
+        m.nid.zero(m.stream);   // (what lies behind the rows stays so)
+        m.leaf_weight.alloc(T * b.nodes_stride); b.weight = m.leaf_weight.p;
+        m.leaf_rule.alloc(T * b.rule_stride); b.rule = m.leaf_rule.p;
         m.hist_full.alloc(T * b.full_stride); b.hist_full = m.hist_full.p;
         m.hist_built.alloc(T * b.built_stride); b.hist_built = m.hist_built.p;
         m.hist_built.zero(m.stream);   // the split search leaves it zeroed
         m.recs.alloc(T * b.recs_stride); b.recs = m.recs.p;
-        m.bits.alloc(T * b.bits_stride); b.bits = m.bits.p;
-        m.tile_left.alloc(T * b.tile_stride); b.tile_left = m.tile_left.p;
-        m.tail_left.alloc(T * b.tail_stride); b.tail_left = m.tail_left.p;
         m.eval_ticket.alloc(T * b.ticket_stride); b.ticket = m.eval_ticket.p;
         m.eval_ticket.zero(m.stream);
         m.ctl.alloc(1); b.ctl = m.ctl.p;
@@ -954,9 +963,8 @@ void Booster::init(const DataSet &ds) {
     TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_EXACT_SMEM + table));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
-    TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM));
-    TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM));
-    TGBM_CUDA(cudaFuncSetAttribute(k_predict_walk<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM));
+    const size_t assign_most = assign_smem(std::max(0, depth - 2), m.assign_rpt);
+    if (assign_most > 48 * 1024) TGBM_CUDA(cudaFuncSetAttribute(m.assign_kernel(depth - 2), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)assign_most));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
     m.prune_in_smem = sizeof(TreeNode) * (size_t)m.n_nodes <= 200 * 1024;  // up to depth 11
@@ -1108,7 +1116,7 @@ void BoosterImpl::launch_small_trees(int k0, int n_trees) {
     TGBM_CUDA(cudaLaunchKernelEx(&cfg, k_small_tree, (SmallPlan)small, N, Npad, F, depth, (const unsigned char *)binsT.p, (const int *)cut_ptr.p,
                                  (const float *)cut_val.p, gq, roots, (const QuantInfo *)qinfo.p, p.min_child_weight, p.lambda, p.rt_eps, p.gamma,
                                  (const unsigned char *)ignored_all.p, (const RoundState *)rstate.p, p.column_shards > 0 ? 1 : 0, nodes.p, model.p, K, k0,
-                                 maxbits.p, f32 && k0 == 0 ? K : 0, ctl.p, hist_full.p, bufs.full_stride));
+                                 maxbits.p, f32 && k0 == 0 ? K : 0, ctl.p, hist_full.p, bufs.full_stride, nid.p, bufs.nid_stride, leaf_weight.p, leaf_rule.p, bufs.rule_stride));
     ++launches;
 }
 
@@ -1203,33 +1211,25 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
                 for (int t = 0; t < n_trees; ++t) comm->allreduce(hist_built.p + t * b.built_stride, 2 * (size_t)B * pairs, Comm::I64, Comm::SUM, stream);
             evaluate(hist_built.p, 1, 0, n_trees);
         }
-        // -- move the rows (not after the last level: the finished tree is applied by walking it, see k_predict_walk)
+        // -- rows to their children (after the last level k_apply_tree does it)
         if (level == depth - 1) break;
         timed(2, [&] {
-            const dim3 grid(part_ctas, 1, n_trees);
-            const size_t nodes_table = sizeof(int) * ((size_t)nl + 1);
-            if (sparse) launch_after(k_part_count<true>, grid, PART_THREADS, nodes_table, stream, level, b, nullptr, Npad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, colb, 0);
-            else launch_after(k_part_count<false>, grid, PART_THREADS, nodes_table, stream, level, b, binsT.p, Npad, nullptr, nullptr, cut_ptr.p, colb, 0);
-            launch_after(k_part_scatter, grid, PART_THREADS, 2 * nodes_table, stream, level, b, 0);
+            launch_after(assign_kernel(level), dim3(assign_ctas, 1, n_trees), ASSIGN_THREADS, assign_smem(level, assign_rpt), stream, level, b, N, binsT.p, Npad, sp_row_ptr.p,
+                         sp_bin.p, cut_ptr.p, colb);
         });
-        launches += 2;
+        ++launches;
     }
     if (!one_launch) launch_after(k_prune, n_trees, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream, nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0,
-                                                                                              model.p, K, k0, rstate.p);
+                                                                                              model.p, K, k0, rstate.p, leaf_weight.p, leaf_rule.p, b.rule_stride, colb);
     if (N) {
-        const size_t walk_table = (sizeof(WalkNode) + sizeof(float) + (sparse ? sizeof(WalkSpan) : 0)) * (size_t)n_nodes + sizeof(float);
-        const int in_smem = walk_table <= WALK_SMEM;
-        const size_t walk_smem = in_smem ? walk_table : 0;
         float *yp = ypred.p + (size_t)k0 * N;
         int *nid_out = p.keep_nid ? nid_keep.p + ((size_t)round * K + k0) * N : nullptr;
-        // One tree per round and a pointwise objective: the walk also adds up the round's metric and finds the maxima
+        // One tree per round and a pointwise objective: the pass also adds up the round's metric and finds the maxima
         // of the next round's gradients (grid and order of additions are those of k_metric_partial).
         const bool fuse = K == 1 && (objective == REG_LINEAR || objective == REG_LOGISTIC || objective == BINARY_LOGISTIC);
-        const dim3 walk_ctas(fuse ? metric_blocks() : std::min(ceil_div(N, 256), num_sms * 8), n_trees);
-        const int fo = fuse ? objective : -1;
-        auto kern = sparse ? k_predict_walk<2> : Fpad == 32 ? k_predict_walk<0> : k_predict_walk<1>;
-        launch_after(kern, walk_ctas, 256, walk_smem, stream, nodes.p, n_nodes, in_smem, sparse ? nullptr : bins.p, Fpad, sp_row_ptr.p, sp_bin.p, cut_ptr.p, N,
-                                                    p.learning_rate, yp, nid_out, y.p, fo, metric_partial.p, maxbits.p, colb, ctl.p);
+        const dim3 ctas(fuse ? metric_blocks() : std::min(ceil_div(N, 256), num_sms * 8), n_trees);
+        launch_after(sparse ? k_apply_tree<true> : k_apply_tree<false>, ctas, 256, 0, stream, b, N, depth - 1, binsT.p, Npad, sp_row_ptr.p, sp_bin.p,
+                     cut_ptr.p, p.learning_rate, yp, nid_out, y.p, fuse ? objective : -1, metric_partial.p, maxbits.p, colb);
         grad_max_ready = metric_partial_ready = fuse;
     }
     launches += 2;
@@ -1244,7 +1244,7 @@ void BoosterImpl::round_metric(int round) {
         return;
     }
     const int blocks = metric_blocks();
-    if (!metric_partial_ready) {  // else the walk that applied the round's tree has left the partial sums
+    if (!metric_partial_ready) {  // else the pass that applied the round's tree has left the partial sums
         launch_after(k_metric_partial, blocks, 256, 0, stream, objective, y.p, ypred.p, N, K, metric_partial.p);
         ++launches;
     }
@@ -1409,7 +1409,7 @@ HistProfile Booster::profile() {
     for (auto &e : m.events) {
         float ms = 0;
         cudaEventElapsedTime(&ms, e.a, e.b);
-        if (e.kind == 2) { r.partition_ms += ms; r.partition_launches += 2; }
+        if (e.kind == 2) { r.partition_ms += ms; r.partition_launches += 1; }
         else {
             r.hist_ms += ms; r.hist_launches += 1;
             if (e.kind == 0) { r.hist_root_ms += ms; r.hist_root_launches += 1; }

@@ -38,15 +38,14 @@ constexpr int F32_THREADS = 512;
 struct CutOffsets { int v[256]; };
 
 // ---- bulk-copy staging of the record tiles (gather levels) ---------------------------------------------------------
-// At the levels below the root a CTA reads, for every unit of F32_THREADS records, the unit's row ids and gradient
-// pairs: two contiguous pieces of rec_idx / rec_gh.  They are brought into shared memory by the copy engine
+// At the levels below the root a CTA reads, for every unit of F32_THREADS records, the unit's row ids, a contiguous piece of
+// rec_idx.  They are brought into shared memory by the copy engine
 // (cp.async.bulk global -> shared, completion counted on an mbarrier; a plain one-CTA copy from this GPU's own memory)
-// one unit ahead of the threads, so that the only global loads left on a thread's critical path are its bin row and the
-// reductions.  A bulk copy needs 16-byte aligned addresses and sizes: a unit starts at any record, so the copy starts
+// one unit ahead of the threads, so that the only global loads left on a thread's critical path are its bin row and
+// gradients and the reductions.  A bulk copy needs 16-byte aligned addresses and sizes: a unit starts at any record, so the copy starts
 // at the aligned record before it and is a few records longer; the threads index from the remainder.
 // Every wait on the barrier is bounded; a wait that runs out records itself in ctl->error and the CTA stops.
 constexpr int STAGE_IDX = F32_THREADS + 4;   // ints per staged row-id piece   (2064 bytes)
-constexpr int STAGE_GH = F32_THREADS + 2;    // float2 per staged gradient piece (4112 bytes)
 constexpr int STAGE_WAIT_LIMIT = 1 << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -82,7 +81,6 @@ k_hist_f32(int level, const Batch b, const unsigned char *__restrict__ bins, int
     extern __shared__ int s_base[];
     __shared__ int s_cut[32], scratch[33];
     __shared__ __align__(16) int s_idx[2][STAGE_IDX];
-    __shared__ __align__(16) float2 s_gh[2][STAGE_GH];
     __shared__ __align__(8) uint64_t s_bar[2];
     __shared__ int s_fail;
     const int f0 = blockIdx.y * 32, nf = min(32, F - f0);
@@ -101,8 +99,8 @@ k_hist_f32(int level, const Batch b, const unsigned char *__restrict__ bins, int
     const int pairs = level == 0 ? 1 : 1 << (level - 1);
     const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
     const TreeNode *nodes = b.nodes + tree * b.nodes_stride;
-    const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
-    const float2 *rec_gh = reinterpret_cast<const float2 *>(GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride);
+    const int *rec_idx = b.rec_idx + tree * b.rec_stride;
+    const float2 *gh = reinterpret_cast<const float2 *>(b.gh + tree * b.gh_stride);
     auto unit = [&](int u) -> int3 {   // first record, records, histogram slot
         int lo = 0, hi = pairs - 1;    // last item that starts at or before u
         while (lo < hi) {
@@ -112,12 +110,9 @@ k_hist_f32(int level, const Batch b, const unsigned char *__restrict__ bins, int
         const int node = level == 0 ? 0 : 2 * lo + built_side(level, lo, seg_cnt, nodes, by_hessian), at = (u - s_base[lo]) * F32_THREADS;
         return make_int3(seg_begin[node] + at, min(F32_THREADS, seg_cnt[node] - at), lo);
     };
-    auto issue = [&](int u, int buf) {  // thread 0: both pieces of unit u into buffer buf
-        const int p0 = unit(u).x;
-        const int a_idx = p0 & ~3, a_gh = p0 & ~1;
-        mbar_expect_tx(&s_bar[buf], (uint32_t)(STAGE_IDX * sizeof(int) + STAGE_GH * sizeof(float2)));
-        bulk_g2s(s_idx[buf], rec_idx + a_idx, (uint32_t)(STAGE_IDX * sizeof(int)), &s_bar[buf]);
-        bulk_g2s(s_gh[buf], rec_gh + a_gh, (uint32_t)(STAGE_GH * sizeof(float2)), &s_bar[buf]);
+    auto issue = [&](int u, int buf) {  // thread 0: the row ids of unit u into buffer buf
+        mbar_expect_tx(&s_bar[buf], (uint32_t)(STAGE_IDX * sizeof(int)));
+        bulk_g2s(s_idx[buf], rec_idx + (unit(u).x & ~3), (uint32_t)(STAGE_IDX * sizeof(int)), &s_bar[buf]);
     };
     // A CTA takes a contiguous run of the units, so that at any moment the CTAs of the grid work on different
     // nodes: with all of them on the same node (units dealt out round-robin) every reduction in flight aims at that one
@@ -130,12 +125,11 @@ k_hist_f32(int level, const Batch b, const unsigned char *__restrict__ bins, int
         const int3 e = unit(u);
         const int q = threadIdx.x;
         int r = -1;
-        float2 v = make_float2(0.f, 0.f);
         if (stage) {
             const int buf = n_done & 1;
             if (threadIdx.x == 0 && u + 1 < u_end) issue(u + 1, buf ^ 1);  // one unit ahead
             if (!mbar_wait(&s_bar[buf], (n_done >> 1) & 1)) { s_fail = 1; atomicCAS(&b.ctl->error, 0, 0x40000000 | u); }
-            if (q < e.y) { r = s_idx[buf][(e.x & 3) + threadIdx.x]; v = s_gh[buf][(e.x & 1) + threadIdx.x]; }
+            if (q < e.y) r = s_idx[buf][(e.x & 3) + threadIdx.x];
             __syncthreads();  // every thread holds its record: the buffer may be refilled two units from now
             if (s_fail) {  // leave only when the copy that is still on its way has landed (bounded as well)
                 if (threadIdx.x == 0 && u + 1 < u_end) mbar_wait(&s_bar[buf ^ 1], ((n_done + 1) >> 1) & 1);
@@ -145,9 +139,9 @@ k_hist_f32(int level, const Batch b, const unsigned char *__restrict__ bins, int
         } else if (q < e.y) {
             const int p = e.x + q;
             r = GATHER ? rec_idx[p] : p;
-            v = rec_gh[p];
         }
         if (r < 0) continue;
+        const float2 v = gh[r];
         const uint4 *row = reinterpret_cast<const uint4 *>(bins + (size_t)r * Fpad + f0);
         const uint4 a = row[0], bb = row[1];
         const uint32_t w[8] = {a.x, a.y, a.z, a.w, bb.x, bb.y, bb.z, bb.w};
@@ -175,8 +169,8 @@ k_hist_sparse_f32(int level, const Batch b, const int *__restrict__ row_ptr, con
     const int pairs = level == 0 ? 1 : 1 << (level - 1);
     const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
     const TreeNode *nodes = b.nodes + tree * b.nodes_stride;
-    const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
-    const float2 *rec_gh = reinterpret_cast<const float2 *>(GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride);
+    const int *rec_idx = b.rec_idx + tree * b.rec_stride;
+    const float2 *gh = reinterpret_cast<const float2 *>(b.gh + tree * b.gh_stride);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int W = F32_THREADS / 32;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
@@ -191,7 +185,7 @@ k_hist_sparse_f32(int level, const Batch b, const int *__restrict__ row_ptr, con
         for (int q = first + warp; q < last; q += W) {
             const int p = begin + q;
             const int r = GATHER ? rec_idx[p] : p;
-            const float2 v = rec_gh[p];
+            const float2 v = gh[r];
             const int j1 = row_ptr[r + 1];
             for (int j = row_ptr[r] + lane; j < j1; j += 32) red_add_gh(dst + (size_t)bin[j] * cell_stride, v.x, v.y);
         }

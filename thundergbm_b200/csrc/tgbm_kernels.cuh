@@ -5,12 +5,12 @@
 // Data layout in HBM (one rank = one contiguous block of rows):
 //   bins   uint8 [N][Fpad]   row-major local bin ids, Fpad = F rounded up to 32, 255 = missing.
 //                            One 32-byte sector holds 32 features of one row.
-//   binsT  uint8 [F][Npad]   the same matrix column-major; read by the partition step, which
+//   binsT  uint8 [F][Npad]   the same matrix column-major; read by k_assign, which
 //                            needs one feature of many rows.
 //   gh     float2 [K][N]     gradient pairs of the round, class-major like the reference.
 //   ghq    int2   [K][N]     the same on the round's fixed-point grid.
-//   rec_idx/rec_gh [2][2N]   per-level record lists: rows grouped by tree node, ascending row id
-//                            inside a node (stable partition), ping-pong between levels.
+//   nid    uint16 [N]        node of every row.
+//   rec_idx [2N]             per-level row lists: rows grouped by tree node, roughly ascending inside a node.
 //   hist   int64 [node][B][2] per-node histograms on the fixed-point grid.
 //
 // All sums on the fixed-point grid are integer sums, so they do not depend on the order of
@@ -21,9 +21,7 @@
 namespace tgbm {
 
 constexpr int HIST_THREADS = 1024;  // one CTA per SM: 64 KB of int32 accumulators + up to 128 KB of int64 totals
-constexpr int PART_THREADS = 512;  // 512 x 4 records per tile measured best (1024: fewer tiles in flight per SM, 256: longer tile scan)
-constexpr int PART_RPT = 4;         // records per thread
-constexpr int PART_TILE = PART_THREADS * PART_RPT;
+constexpr int ASSIGN_THREADS = 256, ASSIGN_CHUNK = 8 * ASSIGN_THREADS;   // rows that k_assign takes at a time, at most
 constexpr int MISSING_BIN = 255;
 constexpr int METRIC_PARTS = 1280;  // most partial sums of a round's metric (148 SMs x 8 blocks use 1184)
 constexpr int FINE_BITS = 30;          // value bits of the grid of fp32 mode's later rounds
@@ -232,7 +230,7 @@ static __global__ void k_bin_csr(const int *__restrict__ col, const float *__res
     }
 }
 
-// flag = 1 when some row's bin ids do not ascend (the partition looks a feature up by binary search inside the row)
+// flag = 1 when some row's bin ids do not ascend (k_assign looks a feature up by binary search inside the row)
 static __global__ void k_rows_unsorted(const int *__restrict__ row_ptr, const int *__restrict__ bin, int n_rows, int *__restrict__ flag) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += gridDim.x * blockDim.x) {
         bool bad = false;
@@ -350,7 +348,7 @@ static __global__ void k_grad_softmax(const float *y, const float *yp, int n, in
 // sums) collects what grid_too_coarse decides by.
 //
 // `gh` null: the gradients are those of a pointwise objective (`logistic` 0/1) and are computed again from y and the
-// scores here -- the pass that found their maxima (k_predict_walk) did not store them.
+// scores here -- the pass that found their maxima (k_apply_tree) did not store them.
 template <bool FINE>
 static __global__ void __launch_bounds__(256, 8)   // (the grid is one full wave of eight blocks per SM)
 k_quantize(const float2 *gh, int n, const unsigned *maxbits, int quant_bits,
@@ -631,6 +629,18 @@ k_column_cuts(const unsigned *__restrict__ keys, int n, const int *__restrict__ 
     }
 }
 
+// ------------------------------------------------------------------ splits as the rows meet them
+// Direction (hist_tree_builder_single.cu:1003-1012; `rev`: the column-sharded builder's bins count down, left means bin >
+// split bin, hist_tree_builder.cu:455-459): a row goes left iff x = (bin + shift) mod 256 is below the threshold (rev: not
+// below).  The missing value's bin 255 thereby takes the default direction without a test of its own: unshifted it lies above
+// every bin, shifted below.
+struct AssignRule { int feature; unsigned test; };   // test = threshold << 1 | shift
+constexpr unsigned ASSIGN_NONE = 0xffffffffu;        // test of a node that was not split
+__device__ __forceinline__ AssignRule assign_rule(const TreeNode &nd, bool split, int rev) {
+    const unsigned shift = rev ? (nd.default_right ? 1 : 0) : (nd.default_right ? 0 : 1);
+    return split ? AssignRule{nd.split_feature_id, (((unsigned)nd.split_bid + shift + (rev ? 1u : 0u)) << 1) | shift} : AssignRule{0, ASSIGN_NONE};
+}
+__device__ __forceinline__ bool assign_left(unsigned test, unsigned bin, int rev) { return (((bin + (test & 1u)) & 0xffu) < (test >> 1)) != (rev != 0); }
 // ------------------------------------------------------------------ end of tree
 // Tree::prune_self / try_prune_leaf / reorder_nid (src/thundergbm/tree.cu:85-128).  The reference walks the
 // leaves in index order and climbs while a parent has two leaf children and gain < gamma; the fixed point of that
@@ -653,9 +663,22 @@ __device__ inline void prune_tree(TreeNode *sn, int n_nodes, int depth, float ga
                     [&](int i, int id) { if (sn[i].is_valid && !sn[i].is_pruned) sn[i].final_id = id; }, scratch);
     __syncthreads();
 }
+// what k_apply_tree needs of a finished tree
+__device__ inline void leave_rules(const TreeNode *sn, int n_nodes, int depth, int rev, float *weight, AssignRule *rule) {
+    for (int i = threadIdx.x; i < n_nodes; i += blockDim.x) {
+        int k = i;
+        while (k > 0 && sn[k].is_pruned) k = (k - 1) >> 1;
+        weight[i] = sn[k].base_weight;
+    }
+    const int nl = 1 << (depth - 1);
+    for (int i = threadIdx.x; i < nl; i += blockDim.x) {
+        const TreeNode &nd = sn[nl - 1 + i];
+        rule[i] = assign_rule(nd, nd.is_valid && sn[nd.lch_index].is_valid, rev);
+    }
+}
 static __global__ void __launch_bounds__(1024)
 k_prune(TreeNode *nodes, int n_nodes, int depth, float gamma, int table_in_smem, TreeNode *model, int K, int k0,
-        const RoundState *rs) {
+        const RoundState *rs, float *weight, AssignRule *rule, size_t rule_stride, int rev) {
     chain_wait();
     // grid = trees of the batch.  The finished tree also goes to its slot of the model, tree (round * K + class).
     nodes += (size_t)blockIdx.x * n_nodes;
@@ -671,145 +694,11 @@ k_prune(TreeNode *nodes, int n_nodes, int depth, float gamma, int table_in_smem,
         __syncthreads();
     }
     prune_tree(sn, n_nodes, depth, gamma, scratch);
+    if (weight) leave_rules(sn, n_nodes, depth, rev, weight + (size_t)blockIdx.x * n_nodes, rule + blockIdx.x * rule_stride);
     for (int i = threadIdx.x; i < pieces; i += blockDim.x) {
         const int4 t = reinterpret_cast<const int4 *>(sn)[i];
         if (table_in_smem) reinterpret_cast<int4 *>(nodes)[i] = t;
         reinterpret_cast<int4 *>(model)[i] = t;
-    }
-}
-
-// TreeBuilder::predict_in_training (src/thundergbm/builder/tree_builder.cu:62-74); nvcc contracts the
-// reference's `y += lr * w` into one fused multiply-add, written out here.
-// The reference looks the row's node up in ins2node_id; here every row walks the finished tree on its own bin
-// ids instead (the same comparisons the partition made, so the same node), in row order: the bin rows and the
-// scores are streamed once, nothing is scattered, and the last level needs no partition at all.
-// A node was split iff its children are valid; pruning only marks nodes, so the walk goes on below a pruned
-// parent to find the node the reference's table would hold (`nid_out`) while the score takes the weight of the
-// deepest node on the path that survived pruning.
-//
-// Table entry: test = feature << 16 | feature bits 3-4 at 14 | shift << 13 | threshold << 4 | feature bits 0-2,
-// left = table offset of the left child in bytes; the right child follows it.
-// A row goes left iff x = (bin + shift) mod 256 is below the threshold (not below, where bins count down: `rev`, the
-// column-sharded builder's rule, left means bin > split bin, hist_tree_builder.cu:455-459).  The missing value's bin 255
-// thereby takes the default direction without a test of its own: unshifted it lies above every bin, shifted below.  A node
-// that was not split sends every row left, to itself, so that all rows take the same number of steps.
-struct WalkNode { unsigned test; unsigned left; };
-struct WalkSpan { int c0, c1; };  // CSR layout: global bins [c0, c1) of the split feature
-
-__device__ __forceinline__ bool walk_split(const TreeNode *nodes, const TreeNode &nd) { return nd.is_valid && nd.lch_index >= 0 && nodes[nd.lch_index].is_valid; }
-__device__ __forceinline__ WalkNode walk_node(const TreeNode *nodes, int i, int rev) {
-    const TreeNode nd = nodes[i];
-    if (!walk_split(nodes, nd)) return WalkNode{rev ? 0u : 256u << 4, (unsigned)(i * sizeof(WalkNode))};
-    const unsigned f = (unsigned)nd.split_feature_id, shift = rev ? (nd.default_right ? 1 : 0) : (nd.default_right ? 0 : 1);
-    const unsigned threshold = (unsigned)nd.split_bid + shift + (rev ? 1 : 0);
-    return WalkNode{(f << 16) | ((f & 24) << 11) | (shift << 13) | (threshold << 4) | (f & 7), (unsigned)((2 * i + 1) * sizeof(WalkNode))};
-}
-__device__ __forceinline__ float walk_weight(const TreeNode *nodes, int i) {   // of the deepest node on the path that survived pruning
-    while (i > 0 && nodes[i].is_pruned) i = (i - 1) >> 1;
-    return nodes[i].base_weight;
-}
-__device__ __forceinline__ WalkSpan walk_span(const TreeNode *nodes, const int *__restrict__ cut_ptr, int i) {
-    const TreeNode nd = nodes[i];
-    const int f = walk_split(nodes, nd) ? nd.split_feature_id : 0;
-    return WalkSpan{cut_ptr[f], cut_ptr[f + 1]};
-}
-
-// LAYOUT 0: dense rows of exactly 32 bytes, held in registers (two 16-byte loads per row; the byte of the split
-// feature is picked with six selects and a byte permutation, so that a step costs one shared-memory access); 1: dense rows
-// of any width, one byte load per step; 2: CSR of global bin ids, binary search per step.
-// `table_in_smem` = 0 for trees too large for shared memory (depth 14): the nodes are then decoded from global
-// memory at every step.
-constexpr int WALK_SMEM = 200 * 1024;
-template <int LAYOUT>
-static __global__ void __launch_bounds__(256)
-k_predict_walk(const TreeNode *nodes, int n_nodes, int table_in_smem, const unsigned char *__restrict__ bins, int Fpad,
-               const int *__restrict__ sp_row_ptr, const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr,
-               int n, float lr, float *yp, int *__restrict__ nid_out,
-               const float *__restrict__ y, int fuse_objective, double *metric_partial,
-               unsigned *maxbits, int rev, const TreeCtl *ctl) {
-    chain_wait();
-    const int coarse = ctl->coarse;
-    // blockIdx.y: tree of the batch
-    nodes += (size_t)blockIdx.y * n_nodes;
-    yp += (size_t)blockIdx.y * n;
-    if (nid_out) nid_out += (size_t)blockIdx.y * n;
-    // fuse_objective >= 0 (a pointwise objective, one tree per round): the same pass adds up the round's training
-    // metric (same grid, same order of additions as k_metric_partial) and finds the maxima of the next round's
-    // gradients, so that neither needs a pass of its own over y and the scores.
-    const bool fuse = fuse_objective >= 0;
-    const int fuse_logistic = fuse_objective == REG_LINEAR ? 0 : 1;
-    double msum = 0;
-    float mg = 0.f, mh = 0.f;
-    extern __shared__ __align__(16) unsigned char walk_sm[];   // WalkNode[n_nodes], float weight[n_nodes], LAYOUT 2: WalkSpan[n_nodes]
-    float *ww = reinterpret_cast<float *>(walk_sm + sizeof(WalkNode) * n_nodes);
-    WalkSpan *ws = reinterpret_cast<WalkSpan *>(walk_sm + (sizeof(WalkNode) * n_nodes + sizeof(float) * (n_nodes + 1)));
-    if (table_in_smem) {
-        for (int i = threadIdx.x; i < n_nodes; i += blockDim.x) {
-            reinterpret_cast<WalkNode *>(walk_sm)[i] = walk_node(nodes, i, rev);
-            ww[i] = walk_weight(nodes, i);
-            if (LAYOUT == 2) ws[i] = walk_span(nodes, cut_ptr, i);
-        }
-        __syncthreads();
-    }
-    if (coarse) return;   // the round will be built again
-    const int levels = 31 - __clz(n_nodes + 1) - 1;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        int lo0 = 0, hi0 = 0;
-        uint32_t w[8];
-        const unsigned char *row = bins + (size_t)r * Fpad;
-        if (LAYOUT == 2) { lo0 = sp_row_ptr[r]; hi0 = sp_row_ptr[r + 1]; }
-        if (LAYOUT == 0) {
-            const uint4 a = reinterpret_cast<const uint4 *>(row)[0], b = reinterpret_cast<const uint4 *>(row)[1];
-            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-        }
-        const float score0 = yp[r];
-        const float yr = fuse ? y[r] : 0.f;
-        unsigned at = 0;   // table offset of the row's node
-#pragma unroll 1
-        for (int l = 0; l < levels; ++l) {
-            const WalkNode wk = table_in_smem ? *reinterpret_cast<const WalkNode *>(walk_sm + at) : walk_node(nodes, (int)(at / sizeof(WalkNode)), rev);
-            unsigned b;
-            if (LAYOUT == 2) {
-                const WalkSpan sp = table_in_smem ? ws[at / sizeof(WalkNode)] : walk_span(nodes, cut_ptr, (int)(at / sizeof(WalkNode)));
-                int lo = lo0, hi = wk.left == at ? lo0 : hi0;
-                b = MISSING_BIN;
-                while (lo < hi) {  // bin ids ascend inside a row
-                    const int mid = lo + (hi - lo) / 2, v = sp_bin[mid];
-                    if (v >= sp.c0 && v < sp.c1) { b = v - sp.c0; break; }
-                    if (v < sp.c0) lo = mid + 1; else hi = mid;
-                }
-            } else if (LAYOUT == 1) {
-                b = row[wk.test >> 16];
-            } else {
-                const bool h16 = wk.test & 0x8000u, h8 = wk.test & 0x4000u;
-                const uint32_t a0 = h16 ? w[4] : w[0], a1 = h16 ? w[5] : w[1], a2 = h16 ? w[6] : w[2], a3 = h16 ? w[7] : w[3];
-                b = __byte_perm(h8 ? a2 : a0, h8 ? a3 : a1, wk.test);   // the low byte counts
-            }
-            const unsigned x = (b + ((wk.test >> 13) & 1u)) & 0xffu, threshold = (wk.test >> 4) & 0x1ffu;
-            at = wk.left + ((x < threshold) != (rev != 0) ? 0u : (unsigned)sizeof(WalkNode));
-        }
-        const int nid = (int)(at / sizeof(WalkNode));
-        if (nid_out) nid_out[r] = nid;
-        const float score = __fmaf_rn(lr, table_in_smem ? ww[nid] : walk_weight(nodes, nid), score0);
-        yp[r] = score;
-        if (fuse) {
-            msum += pointwise_metric_term(fuse_objective, yr, score);
-            const float2 v = pointwise_gh(fuse_logistic, yr, score);
-            mg = fmaxf(mg, fabsf(v.x)); mh = fmaxf(mh, v.y);
-        }
-    }
-    if (fuse) {
-        __shared__ double part[8];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) msum += __shfl_xor_sync(0xffffffffu, msum, o);
-        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = msum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
-            metric_partial[blockIdx.x] = t;
-        }
-        track_max(mg, mh, maxbits);
     }
 }
 

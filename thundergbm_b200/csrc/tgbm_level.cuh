@@ -1,7 +1,7 @@
 // Kernels of one tree level: histogram build, split search, row partition.
 //
-// A level is four launches -- k_hist (or its CSR / float forms), k_eval, k_part_count, k_part_scatter -- that hand over to
-// each other through the segment tables alone (seg_begin, seg_cnt: where the records of every node of the level sit).
+// A level is three launches -- k_hist (or its CSR / float forms), k_eval, k_assign -- that hand over to each other through
+// the segment tables alone (seg_begin, seg_cnt: where the row list of every node of the level sits).
 // What used to be planned by single-block kernels between them (which sibling to build, tile lists, prefix sums: 14 + 5 us
 // a level, most of the time of a small training) every block now works out for itself from those tables, in shared memory,
 // while its first loads are on their way.
@@ -16,17 +16,18 @@ namespace tgbm {
 struct Batch {
     TreeNode *nodes;
     int *seg_begin[2], *seg_cnt[2];   // by level parity
-    int *rec_idx[2];                  // row ids of the records, left children in the first half, right ones in the second
-    int2 *rec_gh[2];                  // their gradient pairs
-    const int2 *gh;                   // gradient pairs by row: the records of the root
+    int *origin[2];                   // by level parity: rows of the nodes before a node, where its children's lists start
+    int *rec_idx;                     // row ids of the level's lists, left children in the first half, right ones in the second
+    unsigned short *nid;              // node of every row
+    const int2 *gh;                   // gradient pairs by row
     long long *hist_full, *hist_built;
     SplitRec *recs;
-    unsigned *bits;                   // partition: one bit per record of a tile, left = 1
-    int *tile_left, *tail_left, *ticket;
+    int *ticket;
+    float *weight;                    // finished tree: weight of the deepest surviving node on the way to a node
+    AssignRule *rule;                 // ... and the splits of the last level
     TreeCtl *ctl;
-    size_t nodes_stride, seg_stride, rec_stride, gh_stride, full_stride, built_stride, recs_stride, bits_stride, tile_stride, tail_stride,
-        ticket_stride;
-    int half;                         // offset of the right children in rec_idx / rec_gh
+    size_t nodes_stride, seg_stride, rec_stride, nid_stride, gh_stride, full_stride, built_stride, recs_stride, ticket_stride, rule_stride;
+    int half;                         // offset of the right children in rec_idx
 };
 
 // ------------------------------------------------------------------ work lists
@@ -294,8 +295,8 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
     if (threadIdx.x < HIST_SEQ + 4) s_seq[threadIdx.x] = hist_tile(tiles, (int)threadIdx.x);
     __syncthreads();
 
-    const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
-    const int2 *rec_gh = GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride;
+    const int *rec_idx = b.rec_idx + tree * b.rec_stride;
+    const int2 *gh = b.gh + tree * b.gh_stride;
 
     bool drained = false;   // the totals hold something: few rows per node and CTA need none, so they are not zeroed either
 
@@ -319,13 +320,14 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
     int r1a, r1b, r2a, r2b, pair_next = 0;
     bool noka = false, nokb = false;
     auto load_rows = [&](int i) {   // rows of tile i (ids r1a, r1b) -> registers
-        const int4 e = s_seq[i - seq0];
-        pair_next = e.z;
+        pair_next = s_seq[i - seq0].z;
         noka = r1a >= 0; nokb = r1b >= 0;
-        if (noka) { na = *reinterpret_cast<const uint4 *>(bins + (size_t)r1a * Fpad + half_off); nva = rec_gh[e.x + qa]; }
-        if (nokb) { nb = *reinterpret_cast<const uint4 *>(bins + (size_t)r1b * Fpad + half_off); nvb = rec_gh[e.x + qb]; }
+        if (noka) { na = *reinterpret_cast<const uint4 *>(bins + (size_t)r1a * Fpad + half_off); nva = gh[r1a]; }
+        if (nokb) { nb = *reinterpret_cast<const uint4 *>(bins + (size_t)r1b * Fpad + half_off); nvb = gh[r1b]; }
     };
-    auto prefetch_rows = [&]() {  // rows with ids r2a, r2b -> L2; one lane of each pair asks for the row's sector
+    // rows with ids r2a, r2b -> L2; one lane of each pair asks for the row's sector.  (Asking for the gradients too costs more
+    // than it brings, 67.5 against 66.1 ms per training of 10.5 M rows: lines of eight rows, most are there already.)
+    auto prefetch_rows = [&]() {
         if (GATHER && !(lane & 1)) {
             if (r2a >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(bins + (size_t)r2a * Fpad + f0));
             if (r2b >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(bins + (size_t)r2b * Fpad + f0));
@@ -425,8 +427,8 @@ k_hist_sparse(int level, const Batch b, const int *__restrict__ row_ptr, const i
     const int pairs = level == 0 ? 1 : 1 << (level - 1);
     const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
     const TreeNode *nodes = b.nodes + tree * b.nodes_stride;
-    const int *rec_idx = b.rec_idx[level & 1] + tree * b.rec_stride;
-    const int2 *rec_gh = GATHER ? b.rec_gh[level & 1] + tree * b.rec_stride : b.gh + tree * b.gh_stride;
+    const int *rec_idx = b.rec_idx + tree * b.rec_stride;
+    const int2 *gh = b.gh + tree * b.gh_stride;
     long long *slab = b.hist_built + tree * b.built_stride;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto flush = [&](int pair, bool again) {
@@ -472,7 +474,7 @@ k_hist_sparse(int level, const Batch b, const int *__restrict__ row_ptr, const i
             if (q < last) {
                 const int p = begin + q;
                 const int r = GATHER ? rec_idx[p] : p;
-                v = rec_gh[p];
+                v = gh[r];
                 j0 = row_ptr[r]; j1 = row_ptr[r + 1];
             }
         };
@@ -633,12 +635,23 @@ __device__ __forceinline__ void best_apply_node(int level, int n, int F, const i
     apply_split(nodes, nid, f, r, cut_ptr, cut_val, rt_eps, lam, multi);
 }
 
+// Where the row lists of node n's children start, their lengths zeroed for k_assign to count up.  A node's children take
+// the places of its own rows in either half of the lists, and the rows before it are known from its pair alone.
+__device__ __forceinline__ void open_children(int level, int n, const Batch &b, size_t tree) {
+    const size_t t = tree * b.seg_stride;
+    const int in = level & 1, o = level == 0 ? 0 : b.origin[in ^ 1][t + (n >> 1)] + ((n & 1) ? b.seg_cnt[in][t + n - 1] : 0);
+    b.origin[in][t + n] = o;
+    *reinterpret_cast<int2 *>(b.seg_begin[in ^ 1] + t + 2 * n) = make_int2(o, b.half + o);
+    *reinterpret_cast<int2 *>(b.seg_cnt[in ^ 1] + t + 2 * n) = make_int2(0, 0);
+}
+
 // CSR layout: one warp per node of the level, after k_eval_chunk
 static __global__ void __launch_bounds__(32)
 k_best_apply(int level, const Batch b, int F, const int *__restrict__ cut_ptr, const float *__restrict__ cut_val,
              float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi, int tree0) {
     chain_wait();
     const size_t tree = tree0 + blockIdx.z;
+    if (threadIdx.x == 0) open_children(level, blockIdx.x, b, tree);
     best_apply_node(level, blockIdx.x, F, cut_ptr, cut_val, b.recs + tree * b.recs_stride, b.nodes + tree * b.nodes_stride, rt_eps, lam,
                     cut_fid, chunked, multi);
 }
@@ -678,6 +691,7 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
     const int b0 = cut_ptr[f], nb = cut_ptr[f + 1] - b0, off = (1 << level) - 1, n_children = level == 0 ? 1 : 2;
     chain_wait();
     const int br = level == 0 ? 0 : built_side(level, j, b.seg_cnt[level & 1] + tree * b.seg_stride, nodes, by_hessian);
+    if (f == 0 && (int)threadIdx.x < n_children) open_children(level, level == 0 ? 0 : 2 * j + (int)threadIdx.x, b, tree);
     const bool ignored = ignored_all && ignored_all[(size_t)rs->round * F + f];
     T *full = reinterpret_cast<T *>(b.hist_full + tree * b.full_stride) + (size_t)off * B * 2;
     T *built = built_all + (sizeof(T) == 8 ? tree * b.built_stride : 0) + ((size_t)j * B + b0) * 2 * bs;
@@ -983,207 +997,233 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
 }
 
 
-// ------------------------------------------------------------------ instance partition
+// ------------------------------------------------------------------ rows to their children
 // (replaces update_ins2node_id + the per-level radix sort, hist_tree_builder_single.cu:908-1020, :397-415)
-// Every node of the level that holds records gets ceil(count / PART_TILE) tiles of PART_TILE records; each block takes a
-// contiguous run of the tiles.  Two kernels: the first finds the direction of every record (one bit) and the left count of
-// every tile, the second moves the records.  What lies between them needs no kernel of its own: a block's records start
-// where the lefts of the node's tiles before its run end, and those are the tail counts (lefts in the last node of a
-// run) of the few blocks before it that lie in the same node.
-// Output: left children of all nodes in the first half of the record buffers, right children in the second, both at the
-// number of records of the nodes before theirs.  Stable: the rows of either child ascend like those of the node.  Records
-// of nodes that stopped splitting drop out.
-
-// prologue of both kernels: tiles (s_tile) before every node and total tiles; with a 64-bit scratch also the records before
-// every node (s_rec), both prefixes in one pass (the records of a level fit the low half)
-template <typename V>
-__device__ __forceinline__ int part_items(int level, const int *seg_cnt, int *s_tile, int *s_rec, V *scratch) {
-    const int nl = 1 << level;
-    auto tiles = [&](int n) { return (seg_cnt[n] + PART_TILE - 1) / PART_TILE; };
-    int total;
-    if constexpr (sizeof(V) == 8) {
-        total = (int)(block_prefix<PART_THREADS>(nl, [&](int n) { return ((V)tiles(n) << 32) | (unsigned)seg_cnt[n]; },
-                                                 [&](int n, V before) { s_tile[n] = (int)(before >> 32); s_rec[n] = (int)before; }, scratch) >> 32);
-    } else {
-        total = block_prefix<PART_THREADS>(nl, tiles, [&](int n, int t) { s_tile[n] = t; }, scratch);
-    }
-    if (threadIdx.x == 0) s_tile[nl] = total;
-    __syncthreads();
-    return total;
-}
-// node that owns tile t: the n with s_tile[n] <= t < s_tile[n + 1]
-__device__ __forceinline__ int tile_owner(const int *s_tile, int nl, int t) {
-    int lo = 0, hi = nl;  // first n with s_tile[n] > t
+// One pass over the rows in row order.  10.5 M rows: 35 us at the root, 41 to 53 below; moving records of row id and gradients
+// instead, a pass to count and one to scatter them, took 64 to 88.  (The gradients by row cost the histogram kernels 8 of 58 ms
+// per 100 trees; the final walk through all levels, 133 us, became one step of 81.)  Every row keeps its node (`nid`, two bytes), looks up the split, and its id is written
+// to the list of its child.  The gradients are not moved: the histogram kernels fetch them by row.  A block handles a chunk of
+// neighbouring rows: rank of every row among the chunk's rows of its child (ballots and one shared atomic per warp and child), one
+// global atomic per child for the chunk's place in the list, and the ids, sorted by child in shared memory, go out as runs.
+// The chunks of a list therefore stand in the order their blocks came by, roughly ascending; the sums do not depend on it.
+// Rows of nodes that stopped splitting keep their node and are in no list.
+// CSR layout: the row's bin among the bins [span.x, span.y) of a feature, searched in its ascending bin ids (hist_tree_builder_single.cu:941-966)
+__device__ __forceinline__ unsigned csr_bin(const int *__restrict__ row_ptr, const int *__restrict__ bin, int2 span, int r) {
+    const int c0 = span.x, c1 = span.y;
+    if (c0 == c1) return MISSING_BIN;
+    int lo = row_ptr[r], hi = row_ptr[r + 1];
     while (lo < hi) {
-        const int mid = (lo + hi) / 2;
-        if (s_tile[mid] > t) hi = mid; else lo = mid + 1;
+        const int mid = lo + (hi - lo) / 2, v = bin[mid];
+        if (v >= c0 && v < c1) return (unsigned)(v - c0);
+        if (v < c0) lo = mid + 1; else hi = mid;
     }
-    return lo - 1;
+    return MISSING_BIN;
 }
 
-// Direction of every record of a splittable node: left unless (missing and default right) or
-// bin >= split_bid (hist_tree_builder_single.cu:1003-1012).  A thread handles PART_RPT records of a tile so that their
-// loads overlap.
-// SPARSE: the row's bin of the split feature is searched in its CSR bin ids (hist_tree_builder_single.cu:941-966)
-// instead of being read from the column-major matrix.
-template <bool SPARSE>
-static __global__ void __launch_bounds__(PART_THREADS)
-k_part_count(int level, const Batch b, const unsigned char *__restrict__ binsT, size_t Npad, const int *__restrict__ sp_row_ptr,
-             const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr, int rev, int tree0) {
-    chain_wait();
-    extern __shared__ int s_tile[];   // [nl + 1]
-    __shared__ int wsum[PART_THREADS / 32], scratch[33];
-    const int nl = 1 << level, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t tree = tree0 + blockIdx.z;
-    const TreeNode *nodes = b.nodes + tree * b.nodes_stride + nl - 1;
-    const int *seg_begin = b.seg_begin[level & 1] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[level & 1] + tree * b.seg_stride;
-    const int *rec_idx = level == 0 ? nullptr : b.rec_idx[level & 1] + tree * b.rec_stride;
-    unsigned *bits = b.bits + tree * b.bits_stride;
-    const int total = part_items(level, seg_cnt, s_tile, nullptr, scratch);
-    const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x, t_begin = min(total, (int)blockIdx.x * per), t_end = min(total, t_begin + per);
-    int n = t_begin < t_end ? tile_owner(s_tile, nl, t_begin) : 0, tail = 0, fresh = -1;
-    TreeNode nd;
-    int begin = 0, end = 0;
-    for (int t = t_begin; t < t_end; ++t) {
-        while (t >= s_tile[n + 1]) ++n;
-        if (n != fresh) { fresh = n; nd = nodes[n]; begin = seg_begin[n]; end = begin + seg_cnt[n]; tail = 0; }
-        if (!(nd.is_valid && !nd.is_leaf)) continue;   // finished node
-        const int p0 = begin + (t - s_tile[n]) * PART_TILE;
-        const unsigned char *colp = SPARSE ? nullptr : binsT + (size_t)nd.split_feature_id * Npad;
-        int r[PART_RPT];
-#pragma unroll
-        for (int j = 0; j < PART_RPT; ++j) {
-            const int p = p0 + j * PART_THREADS + threadIdx.x;
-            r[j] = p < end ? (rec_idx ? rec_idx[p] : p) : -1;
-        }
-        unsigned char bin[PART_RPT];
-        if (SPARSE) {
-            const int c0 = cut_ptr[nd.split_feature_id], c1 = cut_ptr[nd.split_feature_id + 1];
-#pragma unroll
-            for (int j = 0; j < PART_RPT; ++j) {
-                bin[j] = MISSING_BIN;
-                if (r[j] >= 0) {
-                    int lo = sp_row_ptr[r[j]], hi = sp_row_ptr[r[j] + 1];  // bin ids ascend inside a row
-                    while (lo < hi) {
-                        const int mid = lo + (hi - lo) / 2, v = sp_bin[mid];
-                        if (v >= c0 && v < c1) { bin[j] = (unsigned char)(v - c0); break; }
-                        if (v < c0) lo = mid + 1; else hi = mid;
-                    }
-                }
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < PART_RPT; ++j) bin[j] = r[j] >= 0 ? colp[r[j]] : 0;
-        }
-        int cnt = 0;
-#pragma unroll
-        for (int j = 0; j < PART_RPT; ++j) {
-            const bool left = r[j] >= 0 && ((bin[j] == MISSING_BIN) ? !nd.default_right : (rev ? bin[j] > nd.split_bid : bin[j] < nd.split_bid));
-            const unsigned m = __ballot_sync(0xffffffffu, left);
-            if (lane == 0) bits[(size_t)t * (PART_TILE / 32) + j * (PART_THREADS / 32) + warp] = m;
-            cnt += __popc(m);
-        }
-        __syncthreads();  // wsum of the previous tile has been read
-        if (lane == 0) wsum[warp] = cnt;
-        __syncthreads();
-        int v = lane < PART_THREADS / 32 ? wsum[lane] : 0;
-        v = __reduce_add_sync(0xffffffffu, v);
-        tail += v;
-        if (threadIdx.x == 0) b.tile_left[tree * b.tile_stride + t] = v;
-    }
-    if (threadIdx.x == 0) b.tail_left[tree * b.tail_stride + blockIdx.x] = tail;
-}
-
-// Stable scatter of the records into the child segments, and the segment table of the next level.  Same grid as k_part_count.
-static __global__ void __launch_bounds__(PART_THREADS, 2048 / PART_THREADS)
-k_part_scatter(int level, const Batch b, int tree0) {
-    chain_wait();
-    constexpr int WORDS = PART_TILE / 32;
-    extern __shared__ int s_tile[];   // [nl + 1], then records before every node [nl]
-    __shared__ int wpre[WORDS], wtot[(WORDS + 31) / 32];
-    __shared__ long long scratch[33];
-    const int nl = 1 << level, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int *s_rec = s_tile + nl + 1;
-    const size_t tree = tree0 + blockIdx.z;
-    const TreeNode *nodes = b.nodes + tree * b.nodes_stride + nl - 1;
-    const int in = level & 1, nx = in ^ 1;
-    const int *seg_begin = b.seg_begin[in] + tree * b.seg_stride, *seg_cnt = b.seg_cnt[in] + tree * b.seg_stride;
-    int *next_begin = b.seg_begin[nx] + tree * b.seg_stride, *next_cnt = b.seg_cnt[nx] + tree * b.seg_stride;
-    const int *rec_idx = level == 0 ? nullptr : b.rec_idx[in] + tree * b.rec_stride;
-    const int2 *rec_gh = level == 0 ? b.gh + tree * b.gh_stride : b.rec_gh[in] + tree * b.rec_stride;
-    int *out_idx = b.rec_idx[nx] + tree * b.rec_stride;
-    int2 *out_gh = b.rec_gh[nx] + tree * b.rec_stride;
-    const unsigned *bits = b.bits + tree * b.bits_stride;
-    const int *tile_left = b.tile_left + tree * b.tile_stride, *tail_left = b.tail_left + tree * b.tail_stride;
-    const int total = part_items(level, seg_cnt, s_tile, s_rec, scratch);
-    auto set_children = [&](int n, int left, int right) {
-        next_cnt[2 * n] = left; next_cnt[2 * n + 1] = right;
-        next_begin[2 * n] = s_rec[n]; next_begin[2 * n + 1] = b.half + s_rec[n];
+// The pass is bound by the instructions per row (127 in a first version with a test per row for every special case: 60 us at
+// any level of 10.5 M rows), hence: rows that go nowhere have a dummy child behind the others, whose rows are ranked and staged
+// like the rest and never read; a node's rule comes as one 16-byte word with the column's address; the next chunk's nodes and
+// bins are on their way while a chunk is ranked.
+// BITS: 1 to 3, the levels whose children (2^BITS) are few, ranked by ballots and one shared atomic per warp and child;
+// 0: many children, one shared atomic per row, the lanes seldom meet.
+struct alignas(16) ChunkRule {
+    union {
+        const unsigned char *col;   // dense: bins of the feature by row
+        int2 span;                  // CSR: the feature's bins
     };
-    if (blockIdx.x == 0) {
-        for (int n = threadIdx.x; n < nl; n += PART_THREADS)
-            if (s_tile[n] == s_tile[n + 1]) set_children(n, 0, 0);   // no tile, no block to do it
-        if (threadIdx.x == 0) atomicAdd(&b.ctl->stat_part_rows, (unsigned long long)(s_rec[nl - 1] + seg_cnt[nl - 1]));
-    }
-    const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x, t_begin = min(total, (int)blockIdx.x * per), t_end = min(total, t_begin + per);
-    if (t_begin >= t_end) return;
-    int n = tile_owner(s_tile, nl, t_begin), fresh = -1, before = 0;   // lefts of the node before the running tile
-    {
-        const int c0 = s_tile[n] / per;   // the block that holds the node's first tile
-        int v = 0;
-        for (int c = c0 + lane; c < (int)blockIdx.x; c += 32) v += tail_left[c];
-        before = __reduce_add_sync(0xffffffffu, v);   // (every warp for itself)
-    }
-    TreeNode nd;
-    int begin = 0, end = 0, base_l = 0, base_r = 0;
-    for (int t = t_begin; t < t_end; ++t) {
-        while (t >= s_tile[n + 1]) ++n;
-        if (n != fresh) {
-            if (fresh >= 0) before = 0;
-            fresh = n; nd = nodes[n]; begin = seg_begin[n]; end = begin + seg_cnt[n];
-            base_l = s_rec[n]; base_r = b.half + base_l;
-        }
-        if (!(nd.is_valid && !nd.is_leaf)) {   // finished node: its records leave the lists
-            if (t == s_tile[n] && threadIdx.x == 0) set_children(n, 0, 0);
-            continue;
-        }
-        const int p0 = begin + (t - s_tile[n]) * PART_TILE, here = tile_left[t];
-        // loads first, so that they overlap with the rank computation
-        int r[PART_RPT];
-        int2 g[PART_RPT];
-        unsigned m[PART_RPT];
+    unsigned code;                  // threshold << 23 | first child << 8 | shift
+    unsigned pad;
+};
+template <bool SPARSE, int RPT, int BITS>
+static __global__ void __launch_bounds__(ASSIGN_THREADS, RPT == 8 ? 4 : 6)
+k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__ binsT, size_t Npad, const int *__restrict__ sp_row_ptr,
+         const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr, int rev) {
+    constexpr int ROWS = RPT * ASSIGN_THREADS;   // at most 8192: 13 bits of a staged entry
+    extern __shared__ __align__(16) unsigned char assign_sm[];
+    __shared__ int scratch[33];
+    if (BITS) level = BITS - 1;
+    const int nl = 1 << level, lane = threadIdx.x & 31, in = level & 1;
+    ChunkRule *rule = reinterpret_cast<ChunkRule *>(assign_sm);          // [nl + 1], the last one for rows of finished nodes
+    unsigned *stage = reinterpret_cast<unsigned *>(rule + nl + 1);        // [ROWS] child << 13 | row of the chunk
+    int *s_cnt = reinterpret_cast<int *>(stage + ROWS);                   // [2 nl + 1] rows of the chunk per child
+    int *s_pre = s_cnt + 2 * nl + 1, *s_to = s_pre + 2 * nl + 1;          // [2 nl + 1] those before the child's; list position less that
+    const size_t tree = blockIdx.z;
+    const TreeNode *nodes = b.nodes + tree * b.nodes_stride + nl - 1;
+    unsigned short *nid = b.nid + tree * b.nid_stride;
+    const int *next_begin = b.seg_begin[in ^ 1] + tree * b.seg_stride;
+    int *next_cnt = b.seg_cnt[in ^ 1] + tree * b.seg_stride, *list = b.rec_idx + tree * b.rec_stride;
+    for (int i = threadIdx.x; i <= 2 * nl; i += ASSIGN_THREADS) s_cnt[i] = 0;
+    chain_wait();
+    const int chunks = (n_rows + ROWS - 1) / ROWS;
+    unsigned at[RPT];   // level's node of the rows to come, nl: none
+    auto load_nodes = [&](int chunk) {   // (the table ends with a whole chunk; what lies behind the rows stays at node 0)
+        const unsigned short *p = nid + (size_t)chunk * ROWS + threadIdx.x;
 #pragma unroll
-        for (int j = 0; j < PART_RPT; ++j) {
-            const int p = p0 + j * PART_THREADS + threadIdx.x;
-            r[j] = p < end ? (rec_idx ? rec_idx[p] : p) : -1;
-            if (p < end) g[j] = rec_gh[p];
-            m[j] = bits[(size_t)t * WORDS + j * (PART_THREADS / 32) + warp];
+        for (int u = 0; u < RPT; ++u) {
+            if (BITS == 1) at[u] = chunk * ROWS + u * ASSIGN_THREADS + (int)threadIdx.x < n_rows ? 0u : 1u;
+            else at[u] = (unsigned)p[u * ASSIGN_THREADS];
         }
-        __syncthreads();  // wpre / wtot of the previous tile have been read
-        // exclusive prefix of the left counts over the tile's ballot words (record order = word order)
-        if (threadIdx.x < WORDS) {
-            const int c = __popc(bits[(size_t)t * WORDS + threadIdx.x]);
-            int v = c;
+    };
+    int chunk = blockIdx.x;
+    if (chunk < chunks) load_nodes(chunk);
+    for (int i = threadIdx.x; i <= nl; i += ASSIGN_THREADS) {
+        AssignRule r{0, ASSIGN_NONE};
+        if (i < nl) r = assign_rule(nodes[i], nodes[i].is_valid && !nodes[i].is_leaf, rev);
+        const bool none = r.test == ASSIGN_NONE;   // always left, to the dummy
+        ChunkRule x;
+        if (SPARSE) x.span = none ? make_int2(0, 0) : make_int2(cut_ptr[r.feature], cut_ptr[r.feature + 1]);
+        else x.col = binsT + (size_t)r.feature * Npad;
+        x.code = none ? ((rev ? 0u : 256u) << 23) | ((unsigned)(2 * nl) << 8) : ((r.test >> 1) << 23) | ((unsigned)(2 * i) << 8) | (r.test & 1u);
+        x.pad = 0;
+        rule[i] = x;
+    }
+    if (blockIdx.x == 0) {   // rows that are looked at, for the byte counter
+        int rows = 0;
+        for (int i = threadIdx.x; i < nl; i += ASSIGN_THREADS) rows += b.seg_cnt[in][tree * b.seg_stride + i];
+        rows = __reduce_add_sync(0xffffffffu, rows);
+        if (lane == 0 && rows) atomicAdd(&b.ctl->stat_part_rows, (unsigned long long)rows);
+    }
+    __syncthreads();
+    unsigned code[RPT], bin[RPT];
+    auto load_bins = [&](int chunk) {
+        const int mine = chunk * ROWS + threadIdx.x;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
-            wpre[threadIdx.x] = v - c;
-            if (lane == 31) wtot[warp] = v;
+        for (int u = 0; u < RPT; ++u) {
+            const ChunkRule q = rule[BITS == 1 ? at[u] : min(at[u] - (unsigned)(nl - 1), (unsigned)nl)];   // (a node further up: beyond nl)
+            code[u] = q.code;
+            const int r = mine + u * ASSIGN_THREADS;
+            if (SPARSE) bin[u] = csr_bin(sp_row_ptr, sp_bin, q.span, r);
+            else bin[u] = q.col[r];   // (behind the last row: the first column's, allocated to the end of a chunk)
+        }
+    };
+    if (chunk < chunks) load_bins(chunk);
+    for (; chunk < chunks; chunk += gridDim.x) {
+        const int row0 = chunk * ROWS;
+        unsigned c[RPT];
+#pragma unroll
+        for (int u = 0; u < RPT; ++u) {
+            const bool left = (((bin[u] + code[u]) & 0xffu) < (code[u] >> 23)) != (rev != 0);
+            c[u] = (code[u] >> 8 & 0x7fffu) + (left ? 0u : 1u);
+            if (BITS == 1 || c[u] < (unsigned)(2 * nl))
+                nid[(size_t)row0 + u * ASSIGN_THREADS + threadIdx.x] = (unsigned short)(c[u] < (unsigned)(2 * nl) ? 2 * nl - 1 + c[u] : 0u);
+        }
+        const bool more = chunk + (int)gridDim.x < chunks;
+        if (more) load_nodes(chunk + gridDim.x);
+        int rank[RPT];
+#pragma unroll
+        for (int u = 0; u < RPT; ++u) {
+            if (BITS == 0) rank[u] = atomicAdd(&s_cnt[c[u]], 1);
+            else {
+                unsigned same = __ballot_sync(0xffffffffu, c[u] < (unsigned)(2 * nl));   // lanes with the same child
+#pragma unroll
+                for (int k = 0; k < BITS; ++k) {
+                    const unsigned v = __ballot_sync(0xffffffffu, c[u] >> k & 1u);
+                    same &= c[u] >> k & 1u ? v : ~v;
+                }
+                const unsigned below = same & ((1u << lane) - 1u);
+                int first = 0;
+                if (c[u] < (unsigned)(2 * nl) && below == 0) first = atomicAdd(&s_cnt[c[u]], __popc(same));
+                rank[u] = __shfl_sync(0xffffffffu, first, __ffs(same) - 1) + __popc(below);
+            }
+        }
+        if (more) load_bins(chunk + gridDim.x);
+        __syncthreads();
+        const int total = block_prefix<ASSIGN_THREADS>(2 * nl, [&](int i) { return s_cnt[i]; }, [&](int i, int before) { s_pre[i] = before; }, scratch);
+        for (int i = threadIdx.x; i < 2 * nl; i += ASSIGN_THREADS) {   // (on its way while the rows are staged)
+            const int n = s_cnt[i];
+            s_cnt[i] = 0;
+            if (n) s_to[i] = next_begin[i] + atomicAdd(next_cnt + i, n) - s_pre[i];
+        }
+        if (threadIdx.x == 0) { s_cnt[2 * nl] = 0; }
+#pragma unroll
+        for (int u = 0; u < RPT; ++u) {
+            const unsigned v = (c[u] << 13) | (unsigned)(u * ASSIGN_THREADS + threadIdx.x);
+            if (c[u] < (unsigned)(2 * nl)) stage[s_pre[c[u]] + rank[u]] = v;
         }
         __syncthreads();
-#pragma unroll
-        for (int j = 0; j < PART_RPT; ++j) {
-            if (r[j] < 0) continue;
-            const int w = j * (PART_THREADS / 32) + warp;
-            int pre = wpre[w];
-            for (int q = 0; q < (w >> 5); ++q) pre += wtot[q];
-            const bool left = (m[j] >> lane) & 1u;
-            const int lefts = before + pre + __popc(m[j] & ((1u << lane) - 1u));
-            const int d = left ? base_l + lefts : base_r + (p0 - begin + j * PART_THREADS + (int)threadIdx.x - lefts);
-            out_idx[d] = r[j];
-            out_gh[d] = g[j];
+#pragma unroll 4
+        for (int i = threadIdx.x; i < total; i += ASSIGN_THREADS) {
+            const unsigned w = stage[i];
+            list[s_to[w >> 13] + i] = row0 + (int)(w & 8191u);
         }
-        before += here;
-        if (t == s_tile[n + 1] - 1 && threadIdx.x == 0) set_children(n, before, end - begin - before);
+    }
+}
+
+// ------------------------------------------------------------------ end of tree
+// TreeBuilder::predict_in_training (src/thundergbm/builder/tree_builder.cu:62-74); nvcc contracts the reference's
+// `y += lr * w` into one fused multiply-add, written out here.  The last level's split is applied on the way.  A node was split iff its children are valid; pruning only marks nodes, so the row's node is the
+// one the reference's table would hold (`nid_out`) while the score takes the weight of the deepest node on the path that
+// survived pruning (`weight`, left by prune_tree like the rules of the last level).
+constexpr int APPLY_RPT = 4;   // rows in flight per thread
+template <bool SPARSE>
+static __global__ void __launch_bounds__(256)
+k_apply_tree(const Batch b, int n_rows, int last_level, const unsigned char *__restrict__ binsT, size_t Npad, const int *__restrict__ sp_row_ptr,
+             const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr, float lr, float *yp, int *__restrict__ nid_out,
+             const float *__restrict__ y, int fuse_objective, double *metric_partial, unsigned *maxbits, int rev) {
+    chain_wait();
+    // fuse_objective >= 0 (a pointwise objective, one tree per round): the same pass adds up the round's training
+    // metric (same grid, same order of additions as k_metric_partial) and finds the maxima of the next round's
+    // gradients, so that neither needs a pass of its own over y and the scores.
+    const bool fuse = fuse_objective >= 0;
+    const int fuse_logistic = fuse_objective == REG_LINEAR ? 0 : 1;
+    const size_t tree = blockIdx.y;
+    const unsigned short *nid = b.nid + tree * b.nid_stride;
+    const float *weight = b.weight + tree * b.nodes_stride;
+    const AssignRule *rule = b.rule + tree * b.rule_stride;
+    yp += tree * n_rows;
+    if (nid_out) nid_out += tree * n_rows;
+    if (b.ctl->coarse) return;   // the round will be built again
+    const unsigned off = (1u << last_level) - 1u;
+    double msum = 0;
+    float mg = 0.f, mh = 0.f;
+    const int step = gridDim.x * blockDim.x;
+    for (int r0 = blockIdx.x * blockDim.x + threadIdx.x; r0 < n_rows; r0 += APPLY_RPT * step) {
+        unsigned at[APPLY_RPT], bin[APPLY_RPT];
+        float score[APPLY_RPT], yr[APPLY_RPT];
+        AssignRule x[APPLY_RPT];
+#pragma unroll
+        for (int u = 0; u < APPLY_RPT; ++u) {
+            const int r = r0 + u * step;
+            const bool in = r < n_rows;
+            at[u] = in && last_level != 0 ? nid[r] : 0u;
+            score[u] = in ? yp[r] : 0.f;
+            yr[u] = in && fuse ? y[r] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < APPLY_RPT; ++u) x[u] = at[u] >= off ? rule[at[u] - off] : AssignRule{0, ASSIGN_NONE};
+#pragma unroll
+        for (int u = 0; u < APPLY_RPT; ++u) {
+            const int r = r0 + u * step;
+            bin[u] = 0;
+            if (x[u].test != ASSIGN_NONE && r < n_rows) bin[u] = SPARSE ? csr_bin(sp_row_ptr, sp_bin, make_int2(cut_ptr[x[u].feature], cut_ptr[x[u].feature + 1]), r) : binsT[(size_t)x[u].feature * Npad + r];
+        }
+#pragma unroll
+        for (int u = 0; u < APPLY_RPT; ++u) {
+            const int r = r0 + u * step;
+            if (r >= n_rows) break;
+            if (x[u].test != ASSIGN_NONE) at[u] = 2 * at[u] + (assign_left(x[u].test, bin[u], rev) ? 1u : 2u);
+            if (nid_out) nid_out[r] = (int)at[u];
+            const float s = __fmaf_rn(lr, weight[at[u]], score[u]);
+            yp[r] = s;
+            if (fuse) {
+                msum += pointwise_metric_term(fuse_objective, yr[u], s);
+                const float2 v = pointwise_gh(fuse_logistic, yr[u], s);
+                mg = fmaxf(mg, fabsf(v.x)); mh = fmaxf(mh, v.y);
+            }
+        }
+    }
+    if (fuse) {
+        __shared__ double part[8];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) msum += __shfl_xor_sync(0xffffffffu, msum, o);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = msum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double t = 0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
+            metric_partial[blockIdx.x] = t;
+        }
+        track_max(mg, mh, maxbits);
     }
 }
 

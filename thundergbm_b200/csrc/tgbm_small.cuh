@@ -20,7 +20,6 @@
 namespace tgbm {
 
 constexpr int SMALL_THREADS = 1024;
-constexpr unsigned short SMALL_NONE = 0xffff;   // node of a row that left the tree's active part
 
 struct SmallPost {   // a CTA's best candidate of a node: |gain| bits << 32 | (0x7fffffff - feature), 0 = none
     unsigned long long key;
@@ -83,7 +82,8 @@ static __global__ void __launch_bounds__(SMALL_THREADS, 1)
 k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const unsigned char *__restrict__ binsT, const int *__restrict__ cut_ptr,
              const float *__restrict__ cut_val, const int2 *ghq, const unsigned long long *root_sum, const QuantInfo *q, float mcw, float lam,
              float rt_eps, float gamma, const unsigned char *__restrict__ ignored_all, const RoundState *rs, int multi, TreeNode *nodes_out,
-             TreeNode *model, int K, int k0, unsigned *maxbits, int fine_K, TreeCtl *ctl, long long *hist_full, size_t full_stride) {
+             TreeNode *model, int K, int k0, unsigned *maxbits, int fine_K, TreeCtl *ctl, long long *hist_full, size_t full_stride,
+             unsigned short *nid, size_t nid_stride, float *weight, AssignRule *rule, size_t rule_stride) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char small_sm[];
     __shared__ int scratch[33], s_split;
@@ -97,6 +97,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
     const cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), tree = blockIdx.x / plan.cluster, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int f0 = min(F, rank * plan.feats), nf = min(F, f0 + plan.feats) - f0, bin0 = cut_ptr[f0], words = plan.nodes_pass * plan.bins;
+    const int share = (N + plan.cluster - 1) / plan.cluster, share0 = min(N, rank * share), share1 = min(N, share0 + share);   // rows whose node this CTA reports
     for (int r = threadIdx.x; r < N; r += SMALL_THREADS) node_of[r] = 0;
     chain_wait();
     if (blockIdx.x == 0 && threadIdx.x == SMALL_THREADS - 1) next_maxima(root_sum, fine_K, maxbits, ctl);   // (a thread that has nothing else to do yet)
@@ -121,7 +122,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
     }
     __syncthreads();
     for (int level = 0; level < depth; ++level) {
-        const int nl = 1 << level, off = nl - 1;
+        const int nl = 1 << level, off = nl - 1;   // (a row's node: from `off` on when it is still on its way)
         SmallPost *post = posts + (level & 1) * max_nl;
         for (int n0 = 0; n0 < nl; n0 += plan.nodes_pass) {
             const int here = min(plan.nodes_pass, nl - n0);
@@ -135,7 +136,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int r = r0 + u * SMALL_THREADS;
-                    n[u] = r < N ? (int)node_of[r] - n0 : -1;
+                    n[u] = r < N ? (int)node_of[r] - off - n0 : -1;
                     if ((unsigned)n[u] >= (unsigned)here) n[u] = -1;
                     v[u] = r < N ? gq[r] : make_int2(0, 0);   // (does not wait for the node)
                 }
@@ -223,31 +224,31 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
             __syncwarp();
         }
         __syncthreads();
-        if (!s_split || level == depth - 1) break;   // the same in every CTA
+        if (!s_split || level == depth - 1) break;   // the same in every CTA (k_apply_tree makes the last move)
         // -- rows to the children
         // (every CTA for itself: moving a share each and storing it into all sixteen copies took twice the time)
         constexpr int R = 8;   // rows in flight per thread
         for (int r0 = threadIdx.x; r0 < N; r0 += R * SMALL_THREADS) {
-            int n[R];
-            unsigned sp[R];
+            unsigned at[R], sp[R];
             unsigned char b[R];
 #pragma unroll
             for (int u = 0; u < R; ++u) {
                 const int r = r0 + u * SMALL_THREADS;
-                n[u] = r < N ? (int)node_of[r] : (int)SMALL_NONE;
-                sp[u] = n[u] != SMALL_NONE ? split[n[u]] : 0u;
+                at[u] = r < N ? node_of[r] : 0u;
+                sp[u] = r < N && at[u] >= (unsigned)off ? split[at[u] - off] : 0u;   // 0: not split
                 b[u] = sp[u] ? binsT[(size_t)((sp[u] >> 8) & 0x3fffffu) * Npad + r] : (unsigned char)0;
             }
 #pragma unroll
             for (int u = 0; u < R; ++u) {
-                if (n[u] == SMALL_NONE) continue;
+                if (!sp[u]) continue;
                 const unsigned char bid = (unsigned char)sp[u];
                 const bool left = b[u] == MISSING_BIN ? !(sp[u] & 0x40000000u) : (multi ? b[u] > bid : b[u] < bid);
-                node_of[r0 + u * SMALL_THREADS] = sp[u] ? (unsigned short)(2 * n[u] + (left ? 0 : 1)) : SMALL_NONE;
+                node_of[r0 + u * SMALL_THREADS] = (unsigned short)(2 * at[u] + (left ? 1u : 2u));
             }
         }
         __syncthreads();
     }
+    for (int r = share0 + (int)threadIdx.x; r < share1; r += SMALL_THREADS) nid[(size_t)tree * nid_stride + r] = node_of[r];
     cluster.sync();   // nobody reads this CTA's candidates any more
     if (rank != 0) return;
     // -- pruning and the finished tree (k_prune)
@@ -256,6 +257,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
         atomicAdd(&ctl->stat_hists, 1ull);
     }
     prune_tree(nodes, n_nodes, depth, gamma, scratch);
+    leave_rules(nodes, n_nodes, depth, multi, weight + (size_t)tree * n_nodes, rule + tree * rule_stride);
     TreeNode *out = nodes_out + (size_t)tree * n_nodes, *mod = model + ((size_t)rs->round * K + k0 + tree) * n_nodes;
     for (int i = threadIdx.x; i < n_nodes * (int)(sizeof(TreeNode) / 16); i += SMALL_THREADS) {
         const int4 t = reinterpret_cast<const int4 *>(nodes)[i];
