@@ -127,3 +127,32 @@ def test_gradients_that_are_not_numbers(gpu):
     trees, _, scores = _rounds(_csr(x, np.ones((n, 3), bool), y), depth=3, n_trees=4, learning_rate=0.5, objective='reg:linear')
     assert np.isnan(trees[:, 0]['base_weight']).all()   # as float sums have it, in every round
     assert np.isnan(scores[-1]).all()
+
+
+# the first round of a softmax objective: its trees are built side by side from float sums, in cells spread out or, where they
+# are too many for that, close together.  All rows of a class carry the same gradient, so the nodes' sums are counts.
+@pytest.mark.parametrize('classes,features,depth', [(3, 2, 1), (3, 5, 4), (7, 40, 6), (12, 33, 9)])
+@pytest.mark.parametrize('layout', ['dense', 'sparse'])
+def test_first_round_of_several_trees(gpu, monkeypatch, classes, features, depth, layout):
+    from thundergbm_b200.booster import Booster
+    monkeypatch.setenv('TGBM_LAYOUT', layout)
+    n = 6007
+    r = np.random.default_rng(classes)
+    x = np.where(r.random((n, features)) < 0.5, 1.0, r.integers(1, 250, (n, features)))   # one bin with half of the rows
+    y = r.integers(0, classes, n)
+    b = Booster(_csr(x, r.random((n, features)) < 0.8, y), hist_mode='fp32', keep_nid=1, depth=depth, n_trees=1, max_num_bin=255, learning_rate=1.0,
+                objective='multi:softmax', num_class=classes, min_child_weight=0.0, gamma=0.0)
+    b.boost(1)
+    trees, nid = b.trees()[0], b.nid().reshape(classes, n)
+    b.close()
+    g = 1 / classes - (y[None, :] == np.arange(classes)[:, None])
+    h = 2 / classes * (1 - 1 / classes)
+    for k in range(classes):
+        # m values added one after the other, every addition rounding the running sum by half a unit at most: m 2^-24 of the sum.
+        # (Equal values drift: the rounding errors do not cancel.)  A level's sums inherit what their ancestors' were off.
+        noise_g, noise_h = n * 2.0 ** -24 * np.abs(g[k]).sum(), n * 2.0 ** -24 * n * h
+        assert (trees[k]['is_valid'] != 0).sum() >= 3
+        for node in np.nonzero(trees[k]['is_valid'])[0]:
+            rows = _rows_below(nid[k], node, depth)
+            assert abs(trees[k]['sum_g'][node] - g[k][rows].sum()) <= noise_g * (depth + 1)
+            assert abs(trees[k]['sum_h'][node] - h * rows.sum()) <= noise_h * (depth + 1)

@@ -943,7 +943,7 @@ void Booster::init(const DataSet &ds) {
     if (p.keep_nid) m.nid_keep.alloc(n1 * K * std::max(p.n_trees, 1));
     if (m.f32) {
         for (int f = 0; f < std::min(m.F, 256); ++f) m.f32_cuts.v[f] = m.h_cut_ptr[f];
-        m.spread_cells = std::max<size_t>(std::min<size_t>((size_t)32 * max_pairs * B1, (size_t)8 << 20), (size_t)max_pairs * B1);  // <= 64 MB
+        m.spread_cells = std::min<size_t>((size_t)32 * m.batch * max_pairs * B1, (size_t)8 << 20);   // 64 MB: they stay in L2
         m.hist_spread.alloc(m.spread_cells);
         m.hist_spread.zero(m.stream);
         m.sum_partial.alloc((size_t)SUM_BLOCKS * K * 2);
@@ -1143,16 +1143,16 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
         const int nl = 1 << level, pairs = std::max(1, nl / 2), keep = level == 0 || level + 1 < depth;
         const size_t table = sizeof(int) * ((size_t)pairs + 1);
         // -- histogram of the root / of the smaller child of every pair, and the choice of the splits
-        auto evaluate = [&](auto *built, int bs, int tree, int n) {
+        auto evaluate = [&](auto *built, size_t tree_cells, int bs) {
             using T = std::remove_pointer_t<decltype(built)>;
             if (sparse) {
-                launch_after(k_eval_chunk<T>, dim3(n_chunks, pairs, n), 64, 0, stream, level, b, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_fid.p, built, bs, qinfo.p,
-                                                                             p.min_child_weight, p.lambda, ignored_all.p, rstate.p, F, colb, by_hessian, keep, tree);
-                launch_after(k_best_apply, dim3(nl, 1, n), 32, 0, stream, level, b, n_chunks, cut_ptr.p, cut_val.p, p.rt_eps, p.lambda, cut_fid.p, 1, colb, tree);
+                launch_after(k_eval_chunk<T>, dim3(n_chunks, pairs, n_trees), 64, 0, stream, level, b, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_fid.p, built, tree_cells, bs,
+                             qinfo.p, p.min_child_weight, p.lambda, ignored_all.p, rstate.p, F, colb, by_hessian, keep);
+                launch_after(k_best_apply, dim3(nl, 1, n_trees), 32, 0, stream, level, b, n_chunks, cut_ptr.p, cut_val.p, p.rt_eps, p.lambda, cut_fid.p, 1, colb);
                 launches += 2;
             } else {
-                launch_after(k_eval<T>, dim3(F, pairs, n), EVAL_THREADS, 0, stream, level, b, F, B, cut_ptr.p, built, bs, qinfo.p, p.min_child_weight, p.lambda,
-                                                                         cut_val.p, p.rt_eps, cut_fid.p, ignored_all.p, rstate.p, colb, by_hessian, keep, tree);
+                launch_after(k_eval<T>, dim3(F, pairs, n_trees), EVAL_THREADS, 0, stream, level, b, F, B, cut_ptr.p, built, tree_cells, bs, qinfo.p, p.min_child_weight, p.lambda,
+                             cut_val.p, p.rt_eps, cut_fid.p, ignored_all.p, rstate.p, colb, by_hessian, keep);
                 ++launches;
             }
         };
@@ -1167,49 +1167,51 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
             if (profile_on) { cudaEventRecord(ev.b, stream); events.push_back(ev); }
         };
         if (float_sums) {
-            // Values are added one by one into cells `bs` float pairs apart, trees one after the other (they share the
-            // spread-out buffer).
-            const int bs = f32_stride(pairs), ctas = num_sms * (2048 / F32_THREADS);
-            for (int t = 0; t < n_trees; ++t) {
-                float2 *compact = reinterpret_cast<float2 *>(hist_built.p + t * b.built_stride), *cells = bs != 1 ? hist_spread.p : compact;
-                // (the split search leaves the cells it reads zeroed; between ranks it reads the gathered ones)
-                if (bs != 1 && comm && comm->active()) TGBM_CUDA(cudaMemsetAsync(cells, 0, sizeof(float2) * (size_t)B * pairs * bs, stream));
-                timed(level == 0 ? 0 : 1, [&] {
-                    if (sparse) {
-                        auto kern = level == 0 ? k_hist_sparse_f32<false> : k_hist_sparse_f32<true>;
-                        launch_after(kern, ctas, F32_THREADS, table, stream, level, b, sp_row_ptr.p, sp_bin.p, cells, B, bs, by_hessian, t);
-                    } else {
-                        auto kern = level == 0 ? k_hist_f32<false> : k_hist_f32<true>;
-                        launch_after(kern, dim3(ctas, G), F32_THREADS, table, stream, level, b, bins.p, Fpad, F, cut_ptr.p, cells, B, bs, f32_cuts, F <= 256,
-                                                                            f32_staged ? 1 : 0, by_hessian, t);
-                    }
-                });
-                ++launches;
-                if (comm && comm->active()) {
-                    // the ranks' sums meet in a compact buffer: spread cells are gathered first (a pass over B x pairs cells)
-                    if (bs != 1) {
-                        const size_t n = (size_t)B * pairs;
-                        launch_after(k_compact_cells, std::min(ceil_div(n, 256), num_sms * 8), 256, 0, stream, cells, compact, n, bs);
+            // Values are added one by one into cells `bs` float pairs apart
+            const int bs = f32_stride(pairs * n_trees), ctas = std::max(1, num_sms * (2048 / F32_THREADS) / n_trees);
+            const bool spread = bs != 1, multi = comm && comm->active();
+            const size_t level_cells = (size_t)B * pairs, compact_cells = b.built_stride;
+            float2 *compact = reinterpret_cast<float2 *>(hist_built.p), *cells = spread ? hist_spread.p : compact;
+            const size_t tree_cells = spread ? level_cells * bs : compact_cells;
+            // (the split search leaves the cells it reads zeroed; between ranks it reads the gathered ones)
+            if (spread && multi) TGBM_CUDA(cudaMemsetAsync(cells, 0, sizeof(float2) * tree_cells * n_trees, stream));
+            timed(level == 0 ? 0 : 1, [&] {
+                if (sparse) {
+                    auto kern = level == 0 ? k_hist_sparse_f32<false> : k_hist_sparse_f32<true>;
+                    launch_after(kern, dim3(ctas, 1, n_trees), F32_THREADS, table, stream, level, b, sp_row_ptr.p, sp_bin.p, cells, tree_cells, B, bs, by_hessian);
+                } else {
+                    auto kern = level == 0 ? k_hist_f32<false> : k_hist_f32<true>;
+                    launch_after(kern, dim3(ctas, G, n_trees), F32_THREADS, table, stream, level, b, bins.p, Fpad, F, cut_ptr.p, cells, tree_cells, B, bs, f32_cuts, F <= 256,
+                                 f32_staged ? 1 : 0, by_hessian);
+                }
+            });
+            ++launches;
+            if (multi) {
+                // the ranks' sums meet in compact buffers: spread cells are gathered first (a pass over B x pairs cells)
+                for (int t = 0; t < n_trees; ++t) {
+                    if (spread) {
+                        launch_after(k_compact_cells, std::min(ceil_div(level_cells, 256), num_sms * 8), 256, 0, stream, cells + t * tree_cells, compact + t * compact_cells,
+                                     level_cells, bs);
                         ++launches;
                     }
-                    comm->allreduce(compact, 2 * (size_t)B * pairs, Comm::F32, Comm::SUM, stream);
-                    evaluate(reinterpret_cast<float *>(compact), 1, t, 1);
-                } else evaluate(reinterpret_cast<float *>(cells), bs, t, 1);
-            }
+                    comm->allreduce(compact + t * compact_cells, 2 * level_cells, Comm::F32, Comm::SUM, stream);
+                }
+                evaluate(reinterpret_cast<float *>(compact), 2 * compact_cells, 1);
+            } else evaluate(reinterpret_cast<float *>(cells), 2 * tree_cells, bs);
         } else {
             timed(level == 0 ? 0 : 1, [&] {
                 if (sparse) {
                     auto kern = level == 0 ? k_hist_sparse<false> : k_hist_sparse<true>;
-                    launch_after(kern, dim3(hist_ctas, 1, n_trees), SPARSE_THREADS, (size_t)std::min(B, SPARSE_SMEM_BINS) * 16 + table, stream, level, b, sp_row_ptr.p, sp_bin.p, B, by_hessian, 0);
+                    launch_after(kern, dim3(hist_ctas, 1, n_trees), SPARSE_THREADS, (size_t)std::min(B, SPARSE_SMEM_BINS) * 16 + table, stream, level, b, sp_row_ptr.p, sp_bin.p, B, by_hessian);
                 } else {
                     auto kern = level == 0 ? (fine ? k_hist<false, true> : k_hist<false, false>) : (fine ? k_hist<true, true> : k_hist<true, false>);
-                    launch_after(kern, dim3(hist_ctas, G, n_trees), HIST_THREADS, (fine ? HIST_FINE_SMEM : HIST_EXACT_SMEM) + table, stream, level, b, bins.p, Fpad, F, cut_ptr.p, B, window_rows, by_hessian, 0);
+                    launch_after(kern, dim3(hist_ctas, G, n_trees), HIST_THREADS, (fine ? HIST_FINE_SMEM : HIST_EXACT_SMEM) + table, stream, level, b, bins.p, Fpad, F, cut_ptr.p, B, window_rows, by_hessian);
                 }
             });
             ++launches;
             if (comm && comm->active())
                 for (int t = 0; t < n_trees; ++t) comm->allreduce(hist_built.p + t * b.built_stride, 2 * (size_t)B * pairs, Comm::I64, Comm::SUM, stream);
-            evaluate(hist_built.p, 1, 0, n_trees);
+            evaluate(hist_built.p, b.built_stride, 1);
         }
         // -- rows to their children (after the last level k_apply_tree does it)
         if (level == depth - 1) break;

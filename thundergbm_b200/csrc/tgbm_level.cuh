@@ -257,7 +257,7 @@ __device__ __noinline__ void hist_flush(const HistTiles &x, unsigned char *hist_
 template <bool GATHER, bool FINE>
 static __global__ void __launch_bounds__(HIST_THREADS, 1)
 k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpad, int F, const int *__restrict__ cut_ptr, int B,
-       int window_rows, int by_hessian, int tree0) {
+       int window_rows, int by_hessian) {
     extern __shared__ __align__(128) unsigned char hist_sm[];
     int *acc = reinterpret_cast<int *>(hist_sm);          // g, h (FINE: low halves)
     int *s_base = reinterpret_cast<int *>(hist_sm + (FINE ? HIST_FINE_SMEM : HIST_EXACT_SMEM));
@@ -265,7 +265,7 @@ k_hist(int level, const Batch b, const unsigned char *__restrict__ bins, int Fpa
     __shared__ int4 s_seq[HIST_SEQ + 4];
     __shared__ HistTiles tiles;
     const int group = blockIdx.y, f0 = group * 32, lane = threadIdx.x & 31;
-    const size_t tree = tree0 + blockIdx.z;
+    const size_t tree = blockIdx.z;
     constexpr int ZERO_BYTES = FINE ? 4 * HIST_CELLS * 4 : 2 * HIST_CELLS * 4;   // the accumulators
     for (int i = threadIdx.x; i < ZERO_BYTES / 16; i += HIST_THREADS)
         reinterpret_cast<int4 *>(hist_sm)[i] = make_int4(0, 0, 0, 0);
@@ -412,12 +412,12 @@ constexpr int SPARSE_THREADS = 1024;     // one CTA per SM
 
 template <bool GATHER>
 static __global__ void __launch_bounds__(SPARSE_THREADS, 1)
-k_hist_sparse(int level, const Batch b, const int *__restrict__ row_ptr, const int *__restrict__ bin, int B, int by_hessian, int tree0) {
+k_hist_sparse(int level, const Batch b, const int *__restrict__ row_ptr, const int *__restrict__ bin, int B, int by_hessian) {
     extern __shared__ __align__(16) int sh_sparse[];  // [4][nsm]: low g, low h, high g, high h; then s_base
     __shared__ int scratch[33];
     const int nsm = min(B, SPARSE_SMEM_BINS);
     int *s_base = sh_sparse + 4 * nsm;
-    const size_t tree = tree0 + blockIdx.z;
+    const size_t tree = blockIdx.z;
     for (int i = threadIdx.x; i < 4 * nsm; i += SPARSE_THREADS) sh_sparse[i] = 0;
     chain_wait();
     const int total = hist_items<SPARSE_THREADS, HIST_THREADS>(level, b, tree, by_hessian, s_base, scratch, blockIdx.x == 0);
@@ -648,9 +648,9 @@ __device__ __forceinline__ void open_children(int level, int n, const Batch &b, 
 // CSR layout: one warp per node of the level, after k_eval_chunk
 static __global__ void __launch_bounds__(32)
 k_best_apply(int level, const Batch b, int F, const int *__restrict__ cut_ptr, const float *__restrict__ cut_val,
-             float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi, int tree0) {
+             float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi) {
     chain_wait();
-    const size_t tree = tree0 + blockIdx.z;
+    const size_t tree = blockIdx.z;
     if (threadIdx.x == 0) open_children(level, blockIdx.x, b, tree);
     best_apply_node(level, blockIdx.x, F, cut_ptr, cut_val, b.recs + tree * b.recs_stride, b.nodes + tree * b.nodes_stride, rt_eps, lam,
                     cut_fid, chunked, multi);
@@ -666,7 +666,8 @@ k_best_apply(int level, const Batch b, int F, const int *__restrict__ cut_ptr, c
 // multi: the column-sharded builder's candidates (hist_tree_builder.cu:299-352): the INCLUSIVE prefix along the
 // bins (they count down from the largest values there) is the right child, the left one is the node minus it,
 // missing values join the right child when that gains at least as much; the record then carries the right sums.
-// bs: distance of two cells of `built` in cells (1 unless the fp32 histogram kernel spread them out).
+// bs: distance of two cells of `built` in cells (1 unless the fp32 histogram kernel spread them out); tree_cells: from tree to
+// tree, in T.
 // ignored: the round's column-sampling mask (Shard::column_sampling, src/thundergbm/builder/shard.cu:8-23; the
 // masked features take no part in the split search, hist_tree_builder_single.cu:304,663), or null.
 constexpr int EVAL_THREADS = 128, EVAL_BINS = 2;
@@ -675,16 +676,16 @@ template <> struct CellPair<long long> { typedef longlong2 type; };
 template <> struct CellPair<float> { typedef float2 type; };
 template <typename T>
 static __global__ void __launch_bounds__(EVAL_THREADS, 8)
-k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, T *built_all, int bs,
+k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, T *built_all, size_t tree_cells, int bs,
        const QuantInfo *q, float mcw, float lam, const float *__restrict__ cut_val, float rt_eps,
        const int *__restrict__ cut_fid, const unsigned char *__restrict__ ignored_all, const RoundState *rs, int multi,
-       int by_hessian, int keep, int tree0) {
+       int by_hessian, int keep) {
     // keep = 0 at the last level: no level subtracts from its histograms, so they are not stored
     constexpr int WARPS = EVAL_THREADS / 32, NB = EVAL_BINS;
     __shared__ T s_sum[4][sizeof(T) == 4 ? 32 : WARPS];
     __shared__ unsigned long long s_key[2][WARPS];
     const int f = blockIdx.x, j = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i0 = threadIdx.x * NB;
-    const size_t tree = tree0 + blockIdx.z;
+    const size_t tree = blockIdx.z;
     TreeNode *nodes = b.nodes + tree * b.nodes_stride;
     SplitRec *recs = b.recs + tree * b.recs_stride;
     int *ticket = b.ticket + tree * b.ticket_stride;
@@ -694,7 +695,7 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
     if (f == 0 && (int)threadIdx.x < n_children) open_children(level, level == 0 ? 0 : 2 * j + (int)threadIdx.x, b, tree);
     const bool ignored = ignored_all && ignored_all[(size_t)rs->round * F + f];
     T *full = reinterpret_cast<T *>(b.hist_full + tree * b.full_stride) + (size_t)off * B * 2;
-    T *built = built_all + (sizeof(T) == 8 ? tree * b.built_stride : 0) + ((size_t)j * B + b0) * 2 * bs;
+    T *built = built_all + tree * tree_cells + ((size_t)j * B + b0) * 2 * bs;
     using Pair = typename CellPair<T>::type;
     // every load of the block is on its way before the first one is waited for (nothing here may alias: the compiler does
     // not know and would wait between a store and the next load)
@@ -849,14 +850,14 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
 template <typename T>
 static __global__ void __launch_bounds__(64)
 k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restrict__ chunk_bin0, const int *__restrict__ cut_ptr,
-             const int *__restrict__ cut_fid, T *built_all, int bs, const QuantInfo *q, float mcw, float lam,
-             const unsigned char *__restrict__ ignored_all, const RoundState *rs, int F, int multi, int by_hessian, int keep, int tree0) {
+             const int *__restrict__ cut_fid, T *built_all, size_t tree_cells, int bs, const QuantInfo *q, float mcw, float lam,
+             const unsigned char *__restrict__ ignored_all, const RoundState *rs, int F, int multi, int by_hessian, int keep) {
     chain_wait();
-    const size_t tree = tree0 + blockIdx.z;
+    const size_t tree = blockIdx.z;
     const TreeNode *nodes = b_.nodes + tree * b_.nodes_stride;
     SplitRec *recs = b_.recs + tree * b_.recs_stride;
     T *full = reinterpret_cast<T *>(b_.hist_full + tree * b_.full_stride) + (size_t)((1 << level) - 1) * B * 2;
-    T *built = built_all + (sizeof(T) == 8 ? tree * b_.built_stride : 0);
+    T *built = built_all + tree * tree_cells;
     __shared__ T sg[2][256], sh[2][256];
     const unsigned char *ignored = ignored_all ? ignored_all + (size_t)rs->round * F : nullptr;
     const int c = blockIdx.x, j = blockIdx.y;
