@@ -51,6 +51,9 @@ struct BoosterImpl {
     bool sparse = false;
     long long nnz_local = 0;
     DevBuf<int> sp_row_ptr, sp_bin, chunk_bin0;
+    DevBuf<int> col_row, col_bin, col_ptr;   // the same values by column (SparseColumns)
+    SparseColumns columns() const { return SparseColumns{col_row.p, col_bin.p, col_ptr.p}; }
+    void sort_columns();
     int n_chunks = 0;
     DevBuf<float> cut_val, y, ypred, metric;
     DevBuf<int> cut_ptr, cut_fid;
@@ -108,11 +111,14 @@ struct BoosterImpl {
     bool settle();
     DevBuf<int> eval_ticket;  // k_eval: finished blocks per sibling pair, zero between launches
     int assign_ctas = 1, assign_rpt = 4;
-    auto assign_kernel(int level) const {
+    DevBuf<int> assign_table;   // float rounds: rows per block and child
+    auto assign_kernel(int level, bool ordered) const {
         auto pick = [&](auto many, auto k0, auto k1, auto k2) { return level == 0 ? k0 : level == 1 ? k1 : level == 2 ? k2 : many; };
-        if (sparse) return pick(k_assign<true, 4, 0>, k_assign<true, 4, 1>, k_assign<true, 4, 2>, k_assign<true, 4, 3>);
-        if (assign_rpt == 8) return pick(k_assign<false, 8, 0>, k_assign<false, 8, 1>, k_assign<false, 8, 2>, k_assign<false, 8, 3>);
-        return pick(k_assign<false, 4, 0>, k_assign<false, 4, 1>, k_assign<false, 4, 2>, k_assign<false, 4, 3>);
+        if (ordered && sparse) return pick(k_assign<true, 4, 0, true>, k_assign<true, 4, 1, true>, k_assign<true, 4, 2, true>, k_assign<true, 4, 3, true>);
+        if (ordered) return pick(k_assign<false, 4, 0, true>, k_assign<false, 4, 1, true>, k_assign<false, 4, 2, true>, k_assign<false, 4, 3, true>);
+        if (sparse) return pick(k_assign<true, 4, 0, false>, k_assign<true, 4, 1, false>, k_assign<true, 4, 2, false>, k_assign<true, 4, 3, false>);
+        if (assign_rpt == 8) return pick(k_assign<false, 8, 0, false>, k_assign<false, 8, 1, false>, k_assign<false, 8, 2, false>, k_assign<false, 8, 3, false>);
+        return pick(k_assign<false, 4, 0, false>, k_assign<false, 4, 1, false>, k_assign<false, 4, 2, false>, k_assign<false, 4, 3, false>);
     }
     bool grad_max_ready = false;        // maxbits holds the maxima of the next round's gradients
     bool metric_partial_ready = false;  // metric_partial holds the finished round's partial sums
@@ -314,6 +320,33 @@ struct SideStreams {
         if (ev) cudaEventDestroy(ev);
     }
 };
+
+// The stored values of the CSR layout once more by column, for the kernels that look for the rows of a column: one sort by bin
+// id, the rows stay in order.  Not where a row stores a column twice (which of its values counts is up to the search then).
+void BoosterImpl::sort_columns() {
+    const size_t nnz = (size_t)nnz_local;
+    if (!nnz || nnz >= ((size_t)1 << 31)) return;
+    const int grid = std::min(ceil_div(N, 8), num_sms * 16);
+    DevBuf<int> twice, rows;
+    twice.alloc(1);
+    twice.zero(stream);
+    k_rows_repeat<<<grid, 256, 0, stream>>>(sp_row_ptr.p, sp_bin.p, cut_fid.p, N, twice.p);
+    int h_twice = 0;
+    TGBM_CUDA(cudaMemcpyAsync(&h_twice, twice.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    TGBM_CUDA(cudaStreamSynchronize(stream));
+    if (h_twice) return;
+    rows.alloc(nnz); col_row.alloc(nnz); col_bin.alloc(nnz); col_ptr.alloc(B + 1);
+    k_value_rows<<<grid, 256, 0, stream>>>(sp_row_ptr.p, N, rows.p);
+    int end_bit = 1;
+    while ((1ll << end_bit) < B) ++end_bit;
+    size_t tb = 0;
+    TGBM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, sp_bin.p, col_bin.p, rows.p, col_row.p, (long long)nnz, 0, end_bit, stream));
+    DevBuf<unsigned char> tmp;
+    tmp.alloc(std::max<size_t>(tb, 1));
+    TGBM_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, sp_bin.p, col_bin.p, rows.p, col_row.p, (long long)nnz, 0, end_bit, stream));
+    k_bin_starts<<<std::min(ceil_div(B + 1, 256), num_sms * 8), 256, 0, stream>>>(col_bin.p, (int)nnz, B, col_ptr.p);
+    TGBM_CUDA(cudaStreamSynchronize(stream));
+}
 
 void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
     const bool timing = getenv("TGBM_TIMING") != nullptr;  // phase times of the set-up on stderr
@@ -591,6 +624,7 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
                 TGBM_CUDA(cudaStreamSynchronize(stream));
             }
         }
+        sort_columns();
         // chunks of whole features with at most 256 bins for the split evaluation
         std::vector<int> cb(1, 0);
         int cur = 0;
@@ -634,7 +668,7 @@ void BoosterImpl::init_exact() {
         DevBuf<int> rows;
         keys.alloc(n1); keys2.alloc(n1); rows.alloc(n1);
         ex_key[0].alloc(padded); ex_row[0].alloc(padded); ex_val[0].alloc(padded);
-        if (N) k_exact_rows<<<std::min(ceil_div(N, 256), num_sms * 16), 256, 0, stream>>>(in.row_ptr.p, N, rows.p);
+        if (N) k_value_rows<<<std::min(ceil_div(N, 8), num_sms * 16), 256, 0, stream>>>(in.row_ptr.p, N, rows.p);
         if (nnz) k_exact_csc_keys<<<grid, 256, 0, stream>>>(in.val.p, in.col.p, nnz, keys.p);
         int end_bit = 32;
         while ((1ll << (end_bit - 32)) < F && end_bit < 64) ++end_bit;
@@ -724,7 +758,7 @@ void BoosterImpl::build_tree_exact(int round, int k) {
     if (f32) exact_levels<float>(k, gh.p + (size_t)k * N);
     else exact_levels<long long>(k, ghq.p + (size_t)k * N);
     k_prune<<<1, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream>>>(nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0, model.p, K, k,
-                                                                                         rstate.p, nullptr, nullptr, 0, 0);
+                                                                                         rstate.p, nullptr, nullptr, 0, 0, nullptr, 0, nullptr, nullptr);
     if (N) {
         int *nid_out = p.keep_nid ? nid_keep.p + (size_t)tree_index * N : nullptr;
         k_exact_predict<<<std::min(ceil_div(N, 256), num_sms * 8), 256, 0, stream>>>(ex_nid.p, N, nodes.p, p.learning_rate, ypred.p + (size_t)k * N, nid_out);
@@ -916,7 +950,7 @@ void Booster::init(const DataSet &ds) {
         }
         m.batch = m.exact ? 1 : std::max(1, std::min(K, (int)(room / per_tree)));
         m.assign_rpt = !m.sparse && (long long)N * m.batch >= 4ll * m.num_sms * 8 * ASSIGN_THREADS ? 8 : 4;
-        m.assign_ctas = std::max(1, std::min(ceil_div(N, ASSIGN_THREADS * m.assign_rpt), m.num_sms * (m.assign_rpt == 8 ? 4 : 6) / m.batch));
+        m.assign_ctas = std::max(1, std::min(ceil_div(N, ASSIGN_THREADS * m.assign_rpt), m.num_sms * (m.sparse || m.assign_rpt == 8 ? 4 : 6) / m.batch));
         const size_t T = m.batch;
         m.nodes.alloc(T * b.nodes_stride); b.nodes = m.nodes.p;
         for (int i = 0; i < 2; ++i) {
@@ -929,6 +963,7 @@ void Booster::init(const DataSet &ds) {
         m.nid.zero(m.stream);   // (what lies behind the rows stays so)
         m.leaf_weight.alloc(T * b.nodes_stride); b.weight = m.leaf_weight.p;
         m.leaf_rule.alloc(T * b.rule_stride); b.rule = m.leaf_rule.p;
+        if (m.f32 && !m.exact) m.assign_table.alloc(T * m.assign_ctas * b.rule_stride);   // (a level's children are at most the last level's nodes)
         m.hist_full.alloc(T * b.full_stride); b.hist_full = m.hist_full.p;
         m.hist_built.alloc(T * b.built_stride); b.hist_built = m.hist_built.p;
         m.hist_built.zero(m.stream);   // the split search leaves it zeroed
@@ -964,7 +999,10 @@ void Booster::init(const DataSet &ds) {
     TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
     const size_t assign_most = assign_smem(std::max(0, depth - 2), m.assign_rpt);
-    if (assign_most > 48 * 1024) TGBM_CUDA(cudaFuncSetAttribute(m.assign_kernel(depth - 2), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)assign_most));
+    if (assign_most > 48 * 1024) {
+        TGBM_CUDA(cudaFuncSetAttribute(m.assign_kernel(depth - 2, false), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)assign_most));
+        TGBM_CUDA(cudaFuncSetAttribute(m.assign_kernel(depth - 2, true), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)assign_most));
+    }
     TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
     TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
     m.prune_in_smem = sizeof(TreeNode) * (size_t)m.n_nodes <= 200 * 1024;  // up to depth 11
@@ -1200,7 +1238,9 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
             } else evaluate(reinterpret_cast<float *>(cells), 2 * tree_cells, bs);
         } else {
             timed(level == 0 ? 0 : 1, [&] {
-                if (sparse) {
+                if (sparse && level == 0 && col_ptr.p) {
+                    launch_after(k_hist_columns, dim3(std::max(1, num_sms * 8 / n_trees), 1, n_trees), 256, 0, stream, b, columns(), (int)nnz_local);
+                } else if (sparse) {
                     auto kern = level == 0 ? k_hist_sparse<false> : k_hist_sparse<true>;
                     launch_after(kern, dim3(hist_ctas, 1, n_trees), SPARSE_THREADS, (size_t)std::min(B, SPARSE_SMEM_BINS) * 16 + table, stream, level, b, sp_row_ptr.p, sp_bin.p, B, by_hessian);
                 } else {
@@ -1214,15 +1254,25 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
             evaluate(hist_built.p, b.built_stride, 1);
         }
         // -- rows to their children (after the last level k_apply_tree does it)
+        if (sparse && col_ptr.p) {
+            const int node_blocks = std::min(nl, 1024);
+            launch_after(k_assign_stored, dim3(std::max(1, num_sms * 8 / (node_blocks * n_trees)), node_blocks, n_trees), 256, 0, stream, level, b, columns(), cut_ptr.p, colb);
+            ++launches;
+        }
         if (level == depth - 1) break;
         timed(2, [&] {
-            launch_after(assign_kernel(level), dim3(assign_ctas, 1, n_trees), ASSIGN_THREADS, assign_smem(level, assign_rpt), stream, level, b, N, binsT.p, Npad, sp_row_ptr.p,
-                         sp_bin.p, cut_ptr.p, colb);
+            auto assign = [&](int order) {
+                launch_after(assign_kernel(level, float_sums), dim3(assign_ctas, 1, n_trees), ASSIGN_THREADS, assign_smem(level, assign_rpt), stream, level, b, N, binsT.p, Npad, sp_row_ptr.p,
+                             sp_bin.p, cut_ptr.p, columns(), colb, order, assign_table.p);
+                ++launches;
+            };
+            if (float_sums) { assign(ASSIGN_COUNT); assign(ASSIGN_PLACE); }
+            else assign(ASSIGN_ANY);
         });
-        ++launches;
     }
     if (!one_launch) launch_after(k_prune, n_trees, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream, nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0,
-                                                                                              model.p, K, k0, rstate.p, leaf_weight.p, leaf_rule.p, b.rule_stride, colb);
+                                                                                              model.p, K, k0, rstate.p, leaf_weight.p, leaf_rule.p, b.rule_stride, colb,
+                                   seg_cnt[(depth - 1) & 1].p, b.seg_stride, cut_ptr.p, sparse ? col_ptr.p : nullptr);
     if (N) {
         float *yp = ypred.p + (size_t)k0 * N;
         int *nid_out = p.keep_nid ? nid_keep.p + ((size_t)round * K + k0) * N : nullptr;

@@ -48,11 +48,6 @@ template <typename E> __device__ __forceinline__ void exact_store4(E *p, const E
     for (int u = 0; u < (int)(sizeof(E) / 4); ++u) reinterpret_cast<int4 *>(p)[u] = w[u];
 }
 
-// row id of every stored value (CSR order)
-static __global__ void k_exact_rows(const int *__restrict__ row_ptr, int n_rows, int *__restrict__ out) {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += gridDim.x * blockDim.x)
-        for (int j = row_ptr[r]; j < row_ptr[r + 1]; ++j) out[j] = r;
-}
 // (column, complement of the value's ordered image): ascending keys = columns ascending, values descending
 static __global__ void k_exact_csc_keys(const float *__restrict__ val, const int *__restrict__ col, size_t nnz, unsigned long long *__restrict__ keys) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nnz; i += (size_t)gridDim.x * blockDim.x)

@@ -239,6 +239,33 @@ static __global__ void k_rows_unsorted(const int *__restrict__ row_ptr, const in
     }
 }
 
+// flag = 1 when some row stores a column twice (bin ids ascend inside a row)
+static __global__ void k_rows_repeat(const int *__restrict__ row_ptr, const int *__restrict__ bin, const int *__restrict__ cut_fid, int n_rows, int *__restrict__ flag) {
+    const int lane = threadIdx.x & 31;
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rows; r += (gridDim.x * blockDim.x) >> 5) {
+        bool bad = false;
+        for (int i = row_ptr[r] + 1 + lane; i < row_ptr[r + 1]; i += 32) bad |= cut_fid[bin[i - 1]] == cut_fid[bin[i]];
+        if (bad) *flag = 1;
+    }
+}
+// row of every stored value (CSR order)
+static __global__ void k_value_rows(const int *__restrict__ row_ptr, int n_rows, int *__restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rows; r += (gridDim.x * blockDim.x) >> 5)
+        for (int j = row_ptr[r] + lane, j1 = row_ptr[r + 1]; j < j1; j += 32) out[j] = r;
+}
+// bin_ptr[x] = first of the sorted bin ids that is x or larger
+static __global__ void k_bin_starts(const int *__restrict__ bin, int n, int n_bins, int *__restrict__ bin_ptr) {
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x <= n_bins; x += gridDim.x * blockDim.x) {
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = lo + (hi - lo) / 2;
+            if (bin[mid] < x) lo = mid + 1; else hi = mid;
+        }
+        bin_ptr[x] = lo;
+    }
+}
+
 // y[i] <- index of y[i] among the ascending `label` values, 0 when it is not one of them
 // (DataSet::group_label, src/thundergbm/dataset.cpp:83-101)
 static __global__ void k_map_labels(float *__restrict__ y, int n, const float *__restrict__ label, int n_label) {
@@ -663,8 +690,14 @@ __device__ inline void prune_tree(TreeNode *sn, int n_nodes, int depth, float ga
                     [&](int i, int id) { if (sn[i].is_valid && !sn[i].is_pruned) sn[i].final_id = id; }, scratch);
     __syncthreads();
 }
+// Does k_assign_stored move the rows of a node that store its split column, bins [span.x, span.y)?  Not if the column is much
+// longer than the node's list: searching the rows' values costs about as much as four entries of the column.
+__device__ __forceinline__ bool by_column(const int *bin_ptr, int2 span, int rows) {
+    return bin_ptr && (long long)bin_ptr[span.y] - bin_ptr[span.x] <= 4ll * rows;
+}
 // what k_apply_tree needs of a finished tree
-__device__ inline void leave_rules(const TreeNode *sn, int n_nodes, int depth, int rev, float *weight, AssignRule *rule) {
+__device__ inline void leave_rules(const TreeNode *sn, int n_nodes, int depth, int rev, float *weight, AssignRule *rule, const int *last_cnt, const int *cut_ptr,
+                                   const int *bin_ptr) {
     for (int i = threadIdx.x; i < n_nodes; i += blockDim.x) {
         int k = i;
         while (k > 0 && sn[k].is_pruned) k = (k - 1) >> 1;
@@ -673,12 +706,15 @@ __device__ inline void leave_rules(const TreeNode *sn, int n_nodes, int depth, i
     const int nl = 1 << (depth - 1);
     for (int i = threadIdx.x; i < nl; i += blockDim.x) {
         const TreeNode &nd = sn[nl - 1 + i];
-        rule[i] = assign_rule(nd, nd.is_valid && sn[nd.lch_index].is_valid, rev);
+        AssignRule r = assign_rule(nd, nd.is_valid && sn[nd.lch_index].is_valid, rev);
+        if (bin_ptr && r.test != ASSIGN_NONE && by_column(bin_ptr, make_int2(cut_ptr[r.feature], cut_ptr[r.feature + 1]), last_cnt[i])) r.feature = -1;
+        rule[i] = r;
     }
 }
 static __global__ void __launch_bounds__(1024)
 k_prune(TreeNode *nodes, int n_nodes, int depth, float gamma, int table_in_smem, TreeNode *model, int K, int k0,
-        const RoundState *rs, float *weight, AssignRule *rule, size_t rule_stride, int rev) {
+        const RoundState *rs, float *weight, AssignRule *rule, size_t rule_stride, int rev, const int *last_cnt, size_t cnt_stride, const int *cut_ptr,
+        const int *bin_ptr) {
     chain_wait();
     // grid = trees of the batch.  The finished tree also goes to its slot of the model, tree (round * K + class).
     nodes += (size_t)blockIdx.x * n_nodes;
@@ -694,7 +730,7 @@ k_prune(TreeNode *nodes, int n_nodes, int depth, float gamma, int table_in_smem,
         __syncthreads();
     }
     prune_tree(sn, n_nodes, depth, gamma, scratch);
-    if (weight) leave_rules(sn, n_nodes, depth, rev, weight + (size_t)blockIdx.x * n_nodes, rule + blockIdx.x * rule_stride);
+    if (weight) leave_rules(sn, n_nodes, depth, rev, weight + (size_t)blockIdx.x * n_nodes, rule + blockIdx.x * rule_stride, last_cnt + blockIdx.x * cnt_stride, cut_ptr, bin_ptr);
     for (int i = threadIdx.x; i < pieces; i += blockDim.x) {
         const int4 t = reinterpret_cast<const int4 *>(sn)[i];
         if (table_in_smem) reinterpret_cast<int4 *>(nodes)[i] = t;

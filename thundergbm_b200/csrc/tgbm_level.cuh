@@ -507,6 +507,78 @@ k_hist_sparse(int level, const Batch b, const int *__restrict__ row_ptr, const i
     flush(w_cur, false);
 }
 
+// The same stored values by column (rows ascend inside a bin), where no row stores a column twice: built once, see
+// BoosterImpl::sort_columns.
+struct SparseColumns {
+    const int *row, *bin;   // [values] sorted by bin
+    const int *bin_ptr;     // [bins + 1] first value of every bin; null: not there
+};
+
+// Root histogram bin by bin: a warp takes COLUMN_RUN neighbouring values, adds up those of a bin in registers and hands over two
+// sums per bin.  What it costs is the gradients, 8 bytes from anywhere in an array that stays in L2, a 32-byte sector each (popular
+// columns: up to four rows a sector): 36 M values of 1 M rows take 165 us, 5.6 TB/s of L2 sectors.  Row by row (k_hist_sparse) they
+// take 198 us: 181 for the 23 M values that meet in shared memory, where popular columns make the same few cells hot.  Bins of a
+// few values only: two reductions per value as there.  grid = (blocks, 1, trees)
+constexpr int COLUMN_RUN = 1024;
+static __global__ void __launch_bounds__(256)
+k_hist_columns(const Batch b, const SparseColumns c, int nnz) {
+    chain_wait();
+    const size_t tree = blockIdx.z;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // the byte counters, see hist_items
+        atomicAdd(&b.ctl->stat_rows_root, (unsigned long long)b.seg_cnt[0][tree * b.seg_stride]);
+        atomicAdd(&b.ctl->stat_hists, 1ull);
+    }
+    const int2 *gh = b.gh + tree * b.gh_stride;
+    unsigned long long *dst = reinterpret_cast<unsigned long long *>(b.hist_built + tree * b.built_stride);
+    const int lane = threadIdx.x & 31;
+    for (long long run = (long long)(blockIdx.x * 8 + (threadIdx.x >> 5)) * COLUMN_RUN; run < nnz; run += (long long)gridDim.x * 8 * COLUMN_RUN) {
+        const int end = (int)min((long long)nnz, run + COLUMN_RUN);
+        int cur = -1;   // bin that g and h belong to, the same in the whole warp
+        long long g = 0, h = 0;
+        auto hand_over = [&]() {
+            if (cur < 0) return;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) { g += shfl_xor_ll(g, o); h += shfl_xor_ll(h, o); }
+            if (lane < 2) atomicAdd(dst + 2 * (size_t)cur + lane, (unsigned long long)(lane ? h : g));
+            g = h = 0;
+        };
+        constexpr int U = 4;   // windows of 32 values in flight
+        for (int e0 = (int)run; e0 < end; e0 += 32 * U) {
+            int x[U], r[U];
+            int2 v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int e = e0 + 32 * u + lane;
+                x[u] = e < end ? c.bin[e] : -1;
+                r[u] = e < end ? c.row[e] : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = r[u] >= 0 ? gh[r[u]] : make_int2(0, 0);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                unsigned left = __ballot_sync(0xffffffffu, x[u] >= 0);
+                const int before = __shfl_up_sync(0xffffffffu, x[u], 1);
+                const int starts = __popc(__ballot_sync(0xffffffffu, x[u] >= 0 && lane > 0 && x[u] != before));
+                if (starts > 4) {
+                    if (x[u] >= 0) {
+                        atomicAdd(dst + 2 * (size_t)x[u], (unsigned long long)(long long)v[u].x);
+                        atomicAdd(dst + 2 * (size_t)x[u] + 1, (unsigned long long)(long long)v[u].y);
+                    }
+                    continue;
+                }
+                while (left) {
+                    const int bin = __shfl_sync(0xffffffffu, x[u], __ffs(left) - 1);
+                    if (bin != cur) { hand_over(); cur = bin; }
+                    const bool mine = x[u] == bin;
+                    if (mine) { g += v[u].x; h += v[u].y; }
+                    left &= ~__ballot_sync(0xffffffffu, mine);
+                }
+            }
+        }
+        hand_over();
+    }
+}
+
 // ------------------------------------------------------------------ split evaluation
 // Histogram cells are `long long` sums on the round's fixed-point grid (exact mode) or `float` sums (fp32 mode, the
 // reference's own arithmetic: GHPair of floats, include/thundergbm/common.h:43-59).  The evaluation kernels are
@@ -1025,8 +1097,13 @@ __device__ __forceinline__ unsigned csr_bin(const int *__restrict__ row_ptr, con
 // any level of 10.5 M rows), hence: rows that go nowhere have a dummy child behind the others, whose rows are ranked and staged
 // like the rest and never read; a node's rule comes as one 16-byte word with the column's address; the next chunk's nodes and
 // bins are on their way while a chunk is ranked.
+// order: ASSIGN_ANY as above.  The float rounds keep the lists in row order, as what their sums come to depends on it (with lists in
+// order to the chunk only, 7 % of trainings of 100 k rows fell on the other side of a near-tie that row order decides one
+// way): two launches, ASSIGN_COUNT leaves the children's rows of every block's run of chunks in `table` ([blocks][2 nl] a tree),
+// ASSIGN_PLACE starts from the rows of the blocks before.
 // BITS: 1 to 3, the levels whose children (2^BITS) are few, ranked by ballots and one shared atomic per warp and child;
 // 0: many children, one shared atomic per row, the lanes seldom meet.
+enum AssignOrder { ASSIGN_ANY = 0, ASSIGN_COUNT = 1, ASSIGN_PLACE = 2 };
 struct alignas(16) ChunkRule {
     union {
         const unsigned char *col;   // dense: bins of the feature by row
@@ -1035,10 +1112,35 @@ struct alignas(16) ChunkRule {
     unsigned code;                  // threshold << 23 | first child << 8 | shift
     unsigned pad;
 };
-template <bool SPARSE, int RPT, int BITS>
-static __global__ void __launch_bounds__(ASSIGN_THREADS, RPT == 8 ? 4 : 6)
+
+// CSR layout with sorted columns: the rows that store the split column of their node go first, found in the column instead of
+// searching the column in every row (1 M rows x 36 values: 45 us a level searching, five dependent reads a row).  grid = (blocks, nodes, trees)
+static __global__ void __launch_bounds__(256)
+k_assign_stored(int level, const Batch b, const SparseColumns c, const int *__restrict__ cut_ptr, int rev) {
+    chain_wait();
+    const size_t tree = blockIdx.z;
+    const int nl = 1 << level;
+    unsigned short *nid = b.nid + tree * b.nid_stride;
+    for (int n = blockIdx.y; n < nl; n += gridDim.y) {
+        const TreeNode &nd = b.nodes[tree * b.nodes_stride + nl - 1 + n];
+        if (!nd.is_valid || nd.is_leaf) continue;
+        const int2 span = make_int2(cut_ptr[nd.split_feature_id], cut_ptr[nd.split_feature_id + 1]);
+        if (!by_column(c.bin_ptr, span, b.seg_cnt[level & 1][tree * b.seg_stride + n])) continue;
+        // bins below the split bin go left (rev: those beyond it, the split bin itself goes right)
+        const int split = c.bin_ptr[span.x + nd.split_bid + (rev ? 1 : 0)], end = c.bin_ptr[span.y];
+        const unsigned short me = (unsigned short)(nl - 1 + n), left = (unsigned short)(2 * me + 1), right = (unsigned short)(2 * me + 2);
+        for (int e = c.bin_ptr[span.x] + blockIdx.x * 256 + threadIdx.x; e < end; e += gridDim.x * 256) {
+            const int r = c.row[e];
+            if (nid[r] == me) nid[r] = (e < split) != (rev != 0) ? left : right;
+        }
+    }
+}
+
+template <bool SPARSE, int RPT, int BITS, bool ORDERED>
+static __global__ void __launch_bounds__(ASSIGN_THREADS, SPARSE || RPT == 8 ? 4 : 6)
 k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__ binsT, size_t Npad, const int *__restrict__ sp_row_ptr,
-         const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr, int rev) {
+         const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr, const SparseColumns cols, int rev, int how, int *table) {
+    const int order = ORDERED ? how : (int)ASSIGN_ANY;
     constexpr int ROWS = RPT * ASSIGN_THREADS;   // at most 8192: 13 bits of a staged entry
     extern __shared__ __align__(16) unsigned char assign_sm[];
     __shared__ int scratch[33];
@@ -1061,24 +1163,37 @@ k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__
         const unsigned short *p = nid + (size_t)chunk * ROWS + threadIdx.x;
 #pragma unroll
         for (int u = 0; u < RPT; ++u) {
-            if (BITS == 1) at[u] = chunk * ROWS + u * ASSIGN_THREADS + (int)threadIdx.x < n_rows ? 0u : 1u;
+            if (BITS == 1) at[u] = chunk * ROWS + u * ASSIGN_THREADS + (int)threadIdx.x >= n_rows ? 3u : SPARSE ? (unsigned)p[u * ASSIGN_THREADS] : 0u;
             else at[u] = (unsigned)p[u * ASSIGN_THREADS];
         }
     };
-    int chunk = blockIdx.x;
-    if (chunk < chunks) load_nodes(chunk);
+    const int run = order == ASSIGN_ANY ? 1 : (chunks + (int)gridDim.x - 1) / (int)gridDim.x, step = order == ASSIGN_ANY ? (int)gridDim.x : 1;
+    int chunk = blockIdx.x * run;
+    const int chunk_end = order == ASSIGN_ANY ? chunks : min(chunks, chunk + run);
+    if (chunk < chunk_end) load_nodes(chunk);
     for (int i = threadIdx.x; i <= nl; i += ASSIGN_THREADS) {
         AssignRule r{0, ASSIGN_NONE};
         if (i < nl) r = assign_rule(nodes[i], nodes[i].is_valid && !nodes[i].is_leaf, rev);
         const bool none = r.test == ASSIGN_NONE;   // always left, to the dummy
         ChunkRule x;
-        if (SPARSE) x.span = none ? make_int2(0, 0) : make_int2(cut_ptr[r.feature], cut_ptr[r.feature + 1]);
+        if (SPARSE) {
+            x.span = none ? make_int2(0, 0) : make_int2(cut_ptr[r.feature], cut_ptr[r.feature + 1]);
+            if (!none && by_column(cols.bin_ptr, x.span, b.seg_cnt[in][tree * b.seg_stride + i])) x.span = make_int2(0, 0);   // who is still here stores no value
+        }
         else x.col = binsT + (size_t)r.feature * Npad;
         x.code = none ? ((rev ? 0u : 256u) << 23) | ((unsigned)(2 * nl) << 8) : ((r.test >> 1) << 23) | ((unsigned)(2 * i) << 8) | (r.test & 1u);
         x.pad = 0;
         rule[i] = x;
     }
-    if (blockIdx.x == 0) {   // rows that are looked at, for the byte counter
+    table += (tree * gridDim.x) * (size_t)(2 * nl);
+    if (order == ASSIGN_PLACE)   // rows of the blocks before, by child; in s_to from here on: where the child's next rows go
+        for (int i = threadIdx.x >> 5; i < 2 * nl; i += ASSIGN_THREADS / 32) {
+            int before = 0;
+            for (int k = lane; k < (int)blockIdx.x; k += 32) before += table[(size_t)k * (2 * nl) + i];
+            before = __reduce_add_sync(0xffffffffu, before);
+            if (lane == 0) s_to[i] = next_begin[i] + before;
+        }
+    if (blockIdx.x == 0 && order != ASSIGN_COUNT) {   // rows that are looked at, for the byte counter
         int rows = 0;
         for (int i = threadIdx.x; i < nl; i += ASSIGN_THREADS) rows += b.seg_cnt[in][tree * b.seg_stride + i];
         rows = __reduce_add_sync(0xffffffffu, rows);
@@ -1090,30 +1205,43 @@ k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__
         const int mine = chunk * ROWS + threadIdx.x;
 #pragma unroll
         for (int u = 0; u < RPT; ++u) {
-            const ChunkRule q = rule[BITS == 1 ? at[u] : min(at[u] - (unsigned)(nl - 1), (unsigned)nl)];   // (a node further up: beyond nl)
+            const unsigned from = at[u] - (unsigned)(nl - 1);
+            const ChunkRule q = rule[min(from, (unsigned)nl)];   // (a node further up: beyond nl)
             code[u] = q.code;
+            // gone already, by its stored value
+            if (SPARSE && from - (unsigned)nl < (unsigned)(2 * nl)) code[u] = ((rev ? 0u : 256u) << 23) | ((from - (unsigned)nl) << 8);
             const int r = mine + u * ASSIGN_THREADS;
             if (SPARSE) bin[u] = csr_bin(sp_row_ptr, sp_bin, q.span, r);
             else bin[u] = q.col[r];   // (behind the last row: the first column's, allocated to the end of a chunk)
         }
     };
-    if (chunk < chunks) load_bins(chunk);
-    for (; chunk < chunks; chunk += gridDim.x) {
+    if (chunk < chunk_end) load_bins(chunk);
+    for (; chunk < chunk_end; chunk += step) {
         const int row0 = chunk * ROWS;
         unsigned c[RPT];
 #pragma unroll
         for (int u = 0; u < RPT; ++u) {
             const bool left = (((bin[u] + code[u]) & 0xffu) < (code[u] >> 23)) != (rev != 0);
             c[u] = (code[u] >> 8 & 0x7fffu) + (left ? 0u : 1u);
-            if (BITS == 1 || c[u] < (unsigned)(2 * nl))
+            if (order != ASSIGN_COUNT && (BITS == 1 || c[u] < (unsigned)(2 * nl)))
                 nid[(size_t)row0 + u * ASSIGN_THREADS + threadIdx.x] = (unsigned short)(c[u] < (unsigned)(2 * nl) ? 2 * nl - 1 + c[u] : 0u);
         }
-        const bool more = chunk + (int)gridDim.x < chunks;
-        if (more) load_nodes(chunk + gridDim.x);
+        const bool more = chunk + step < chunk_end;
+        if (more) load_nodes(chunk + step);
         int rank[RPT];
 #pragma unroll
         for (int u = 0; u < RPT; ++u) {
-            if (BITS == 0) rank[u] = atomicAdd(&s_cnt[c[u]], 1);
+            if (order == ASSIGN_PLACE) {   // warp after warp
+                const unsigned same = __match_any_sync(0xffffffffu, c[u]), below = same & ((1u << lane) - 1u);
+                for (int w = 0; w < ASSIGN_THREADS / 32; ++w) {
+                    if ((int)(threadIdx.x >> 5) == w) {
+                        int first = 0;
+                        if (below == 0) first = atomicAdd(&s_cnt[c[u]], __popc(same));
+                        rank[u] = __shfl_sync(0xffffffffu, first, __ffs(same) - 1) + __popc(below);
+                    }
+                    __syncthreads();
+                }
+            } else if (BITS == 0) rank[u] = atomicAdd(&s_cnt[c[u]], 1);
             else {
                 unsigned same = __ballot_sync(0xffffffffu, c[u] < (unsigned)(2 * nl));   // lanes with the same child
 #pragma unroll
@@ -1127,15 +1255,19 @@ k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__
                 rank[u] = __shfl_sync(0xffffffffu, first, __ffs(same) - 1) + __popc(below);
             }
         }
-        if (more) load_bins(chunk + gridDim.x);
+        if (more) load_bins(chunk + step);
+        if (order == ASSIGN_COUNT) continue;
         __syncthreads();
         const int total = block_prefix<ASSIGN_THREADS>(2 * nl, [&](int i) { return s_cnt[i]; }, [&](int i, int before) { s_pre[i] = before; }, scratch);
         for (int i = threadIdx.x; i < 2 * nl; i += ASSIGN_THREADS) {   // (on its way while the rows are staged)
             const int n = s_cnt[i];
             s_cnt[i] = 0;
-            if (n) s_to[i] = next_begin[i] + atomicAdd(next_cnt + i, n) - s_pre[i];
+            if (order == ASSIGN_PLACE) {
+                s_to[i] -= s_pre[i];
+                s_cnt[i] = n;   // (for the next chunk's place, below)
+            } else if (n) s_to[i] = next_begin[i] + atomicAdd(next_cnt + i, n) - s_pre[i];
         }
-        if (threadIdx.x == 0) { s_cnt[2 * nl] = 0; }
+        if (threadIdx.x == 0) s_cnt[2 * nl] = 0;
 #pragma unroll
         for (int u = 0; u < RPT; ++u) {
             const unsigned v = (c[u] << 13) | (unsigned)(u * ASSIGN_THREADS + threadIdx.x);
@@ -1147,6 +1279,17 @@ k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__
             const unsigned w = stage[i];
             list[s_to[w >> 13] + i] = row0 + (int)(w & 8191u);
         }
+        if (order == ASSIGN_PLACE) {
+            __syncthreads();
+            for (int i = threadIdx.x; i < 2 * nl; i += ASSIGN_THREADS) { s_to[i] += s_pre[i] + s_cnt[i]; s_cnt[i] = 0; }
+            __syncthreads();
+        }
+    }
+    if (order == ASSIGN_ANY) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * nl; i += ASSIGN_THREADS) {
+        if (order == ASSIGN_COUNT) table[(size_t)blockIdx.x * (2 * nl) + i] = s_cnt[i];
+        else if (blockIdx.x == gridDim.x - 1) next_cnt[i] = s_to[i] - next_begin[i];
     }
 }
 
@@ -1154,7 +1297,8 @@ k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__
 // TreeBuilder::predict_in_training (src/thundergbm/builder/tree_builder.cu:62-74); nvcc contracts the reference's
 // `y += lr * w` into one fused multiply-add, written out here.  The last level's split is applied on the way.  A node was split iff its children are valid; pruning only marks nodes, so the row's node is the
 // one the reference's table would hold (`nid_out`) while the score takes the weight of the deepest node on the path that
-// survived pruning (`weight`, left by prune_tree like the rules of the last level).
+// survived pruning (`weight`, left by leave_rules like the rules of the last level; feature < 0: who stores the split column has
+// gone, see k_assign_stored).
 constexpr int APPLY_RPT = 4;   // rows in flight per thread
 template <bool SPARSE>
 static __global__ void __launch_bounds__(256)
@@ -1168,13 +1312,14 @@ k_apply_tree(const Batch b, int n_rows, int last_level, const unsigned char *__r
     const bool fuse = fuse_objective >= 0;
     const int fuse_logistic = fuse_objective == REG_LINEAR ? 0 : 1;
     const size_t tree = blockIdx.y;
-    const unsigned short *nid = b.nid + tree * b.nid_stride;
+    unsigned short *nid = b.nid + tree * b.nid_stride;
     const float *weight = b.weight + tree * b.nodes_stride;
     const AssignRule *rule = b.rule + tree * b.rule_stride;
     yp += tree * n_rows;
     if (nid_out) nid_out += tree * n_rows;
-    if (b.ctl->coarse) return;   // the round will be built again
-    const unsigned off = (1u << last_level) - 1u;
+    const bool coarse = b.ctl->coarse;   // the round will be built again
+    if (coarse && !SPARSE) return;
+    const unsigned nl = 1u << last_level, off = nl - 1u;
     double msum = 0;
     float mg = 0.f, mh = 0.f;
     const int step = gridDim.x * blockDim.x;
@@ -1186,22 +1331,26 @@ k_apply_tree(const Batch b, int n_rows, int last_level, const unsigned char *__r
         for (int u = 0; u < APPLY_RPT; ++u) {
             const int r = r0 + u * step;
             const bool in = r < n_rows;
-            at[u] = in && last_level != 0 ? nid[r] : 0u;
+            at[u] = in && (SPARSE || last_level != 0) ? nid[r] : 0u;
+            if (SPARSE && in) nid[r] = 0;   // the next tree's stored values look for the root there
             score[u] = in ? yp[r] : 0.f;
             yr[u] = in && fuse ? y[r] : 0.f;
         }
 #pragma unroll
-        for (int u = 0; u < APPLY_RPT; ++u) x[u] = at[u] >= off ? rule[at[u] - off] : AssignRule{0, ASSIGN_NONE};
+        for (int u = 0; u < APPLY_RPT; ++u) x[u] = at[u] - off < nl ? rule[at[u] - off] : AssignRule{0, ASSIGN_NONE};
 #pragma unroll
         for (int u = 0; u < APPLY_RPT; ++u) {
             const int r = r0 + u * step;
             bin[u] = 0;
-            if (x[u].test != ASSIGN_NONE && r < n_rows) bin[u] = SPARSE ? csr_bin(sp_row_ptr, sp_bin, make_int2(cut_ptr[x[u].feature], cut_ptr[x[u].feature + 1]), r) : binsT[(size_t)x[u].feature * Npad + r];
+            if (x[u].test == ASSIGN_NONE || r >= n_rows) continue;
+            if (!SPARSE) bin[u] = binsT[(size_t)x[u].feature * Npad + r];
+            else if (x[u].feature < 0) bin[u] = MISSING_BIN;
+            else bin[u] = csr_bin(sp_row_ptr, sp_bin, make_int2(cut_ptr[x[u].feature], cut_ptr[x[u].feature + 1]), r);
         }
 #pragma unroll
         for (int u = 0; u < APPLY_RPT; ++u) {
             const int r = r0 + u * step;
-            if (r >= n_rows) break;
+            if (r >= n_rows || coarse) break;
             if (x[u].test != ASSIGN_NONE) at[u] = 2 * at[u] + (assign_left(x[u].test, bin[u], rev) ? 1u : 2u);
             if (nid_out) nid_out[r] = (int)at[u];
             const float s = __fmaf_rn(lr, weight[at[u]], score[u]);
@@ -1213,7 +1362,7 @@ k_apply_tree(const Batch b, int n_rows, int last_level, const unsigned char *__r
             }
         }
     }
-    if (fuse) {
+    if (fuse && !coarse) {
         __shared__ double part[8];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) msum += __shfl_xor_sync(0xffffffffu, msum, o);

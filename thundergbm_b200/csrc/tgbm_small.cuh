@@ -257,7 +257,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
         atomicAdd(&ctl->stat_hists, 1ull);
     }
     prune_tree(nodes, n_nodes, depth, gamma, scratch);
-    leave_rules(nodes, n_nodes, depth, multi, weight + (size_t)tree * n_nodes, rule + tree * rule_stride);
+    leave_rules(nodes, n_nodes, depth, multi, weight + (size_t)tree * n_nodes, rule + tree * rule_stride, nullptr, nullptr, nullptr);
     TreeNode *out = nodes_out + (size_t)tree * n_nodes, *mod = model + ((size_t)rs->round * K + k0 + tree) * n_nodes;
     for (int i = threadIdx.x; i < n_nodes * (int)(sizeof(TreeNode) / 16); i += SMALL_THREADS) {
         const int4 t = reinterpret_cast<const int4 *>(nodes)[i];
