@@ -1118,8 +1118,9 @@ void BoosterImpl::plan_small_trees() {
         for (int f = 0; f < F; f += pl.feats) pl.bins = std::max(pl.bins, h_cut_ptr[std::min(F, f + pl.feats)] - h_cut_ptr[f]);
         if ((double)N * pl.feats > 8e4 || (double)max_nl * pl.feats > 512) return;
         const size_t budget = 200 * 1024, fixed = (sizeof(TreeNode) * (size_t)n_nodes + 15) / 16 * 16 + sizeof(SmallPost) * 2 * max_nl + (size_t)(N + 7) / 8 * 16 +
-                     4 * (size_t)((max_nl + 3) / 4 * 4) + 64;   // (64: roundings)
-        const size_t per_node = 16 * (size_t)pl.bins + sizeof(SplitRec) * pl.feats;
+                     4 * (size_t)((max_nl + 3) / 4 * 4) + 4 * (size_t)(pl.feats + 1 + pl.bins) + 64;   // (64: roundings)
+        pl.cells = small_feature_at(pl.bins, pl.feats);
+        const size_t per_node = 16 * (size_t)pl.cells + sizeof(SplitRec) * pl.feats;
         if (fixed + per_node > budget) return;
         pl.nodes_pass = (int)std::min<size_t>(max_nl, (budget - fixed) / per_node);
         if (max_nl > 8 * pl.nodes_pass) return;   // the rows would be walked over and over

@@ -613,20 +613,24 @@ __device__ __forceinline__ SplitRec load_rec(const SplitRec *p) {
     return r;
 }
 // SplitPoint of candidate r (feature-local bin) of feature f into node nd and its children: TreeBuilder::update_tree
-__device__ __forceinline__ void apply_split(TreeNode *nodes, int nid, int f, const SplitRec &r, const int *__restrict__ cut_ptr,
-                                            const float *__restrict__ cut_val, float rt_eps, float lam, int multi) {
+// split value of a feature's candidate, from the feature's cut points
+__device__ __forceinline__ float split_at(const float *cuts, int bin, int multi) {
+    if (multi) return cuts[bin];   // the column-sharded builder: the cut point itself (tree_builder.cu:9-60)
+    if (bin) return cuts[bin - 1];
+    return (float)((double)__fsub_rn(cuts[0], fabsf(cuts[0])) - 1e-5);
+}
+__device__ __forceinline__ void apply_split(TreeNode *nodes, int nid, int f, const SplitRec &r, float value, float rt_eps, float lam, int multi) {
     TreeNode &nd = nodes[nid];
     const float gain = fabsf(r.gain);
     if (gain > rt_eps) {
         const bool default_right = r.gain < 0.f;
-        const int b0 = cut_ptr[f];
         nd.gain = gain;
         nd.split_feature_id = f;
         nd.split_bid = (unsigned char)r.bin;
+        nd.split_value = value;
         if (multi) {
-            // TreeBuilder::update_tree of the column-sharded builder (tree_builder.cu:9-60): the split value is the
-            // cut point itself, the record's sums are the right child's, the left child is the node minus it
-            nd.split_value = cut_val[b0 + r.bin];
+            // TreeBuilder::update_tree of the column-sharded builder (tree_builder.cu:9-60): the record's sums are the right
+            // child's, the left child is the node minus it
             TreeNode &l = nodes[nd.lch_index], &rc = nodes[nd.rch_index];
             l.is_valid = 1; rc.is_valid = 1;
             float rgs = r.lg, rhs = r.lh;
@@ -637,12 +641,6 @@ __device__ __forceinline__ void apply_split(TreeNode *nodes, int nid, int f, con
             l.base_weight = __fdiv_rn(-l.sum_g, __fadd_rn(l.sum_h, lam));
             rc.base_weight = __fdiv_rn(-rc.sum_g, __fadd_rn(rc.sum_h, lam));
             return;
-        }
-        if (r.bin == 0) {
-            const float c = cut_val[b0];
-            nd.split_value = (float)((double)__fsub_rn(c, fabsf(c)) - 1e-5);
-        } else {
-            nd.split_value = cut_val[b0 + r.bin - 1];
         }
         TreeNode &l = nodes[nd.lch_index], &rc = nodes[nd.rch_index];
         l.is_valid = 1; rc.is_valid = 1;
@@ -704,7 +702,7 @@ __device__ __forceinline__ void best_apply_node(int level, int n, int F, const i
     } else {
         r = load_rec(recs + (size_t)n * F + f);
     }
-    apply_split(nodes, nid, f, r, cut_ptr, cut_val, rt_eps, lam, multi);
+    apply_split(nodes, nid, f, r, split_at(cut_val + cut_ptr[f], r.bin, multi), rt_eps, lam, multi);
 }
 
 // Where the row lists of node n's children start, their lengths zeroed for k_assign to count up.  A node's children take
