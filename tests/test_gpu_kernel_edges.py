@@ -184,3 +184,15 @@ def test_columns_of_the_csr_layout(gpu, orc, monkeypatch, n, f, depth, twice):
         at = d.row_ptr[:-1]
         d = CsrData(n, f, (d.row_ptr + np.arange(n + 1)).astype(np.int32), np.insert(d.col, at, d.col[at]), np.insert(d.val, at, d.val[at]), d.y)
     _same_as_oracle(orc, d, depth=depth, n_trees=3, max_num_bin=255, learning_rate=0.5, objective='reg:linear', num_class=1, min_child_weight=0.5)
+
+
+# blocks of the split search that take one feature or four: features of 64, 65 and 1 bins, none at all, numbers of them that leave a
+# block part empty, left-out columns in one of four
+@pytest.mark.parametrize('widths,extra', [([64] * 4, {}), ([65, 64, 1], {}), ([2], {}), ([1] * 6 + [200], {}), ([0, 3, 0, 70, 64, 2, 9], {}),
+                                          ([2] * 21, dict(column_sampling_rate=0.4, sample_seed=2))])
+def test_blocks_of_the_split_search(gpu, orc, widths, extra):
+    n, r = 33_000, np.random.default_rng(len(widths))     # (beyond the sizes of a tree per launch)
+    x = np.stack([r.integers(1, w + 1, n) if w else np.ones(n) for w in widths], 1).astype(np.float32)
+    keep = r.random(x.shape) < np.where(np.array(widths) > 0, 0.85, 0.0)
+    y = x @ r.normal(size=len(widths)) + keep[:, 0] + r.random(n)
+    _same_as_oracle(orc, _holes(x, y, keep), depth=6, n_trees=2, max_num_bin=255, learning_rate=0.5, objective='reg:linear', num_class=1, **extra)

@@ -109,6 +109,8 @@ struct BoosterImpl {
     void queue_round(int round);   // its launches one by one
     void wait() const;
     bool settle();
+    DevBuf<int4> eval_items;  // k_eval: features a block each, or four of few bins (n_eval_items = 0: all a block each)
+    int n_eval_items = 0;
     DevBuf<int> eval_ticket;  // k_eval: finished blocks per sibling pair, zero between launches
     int assign_ctas = 1, assign_rpt = 4;
     DevBuf<int> assign_table;   // float rounds: rows per block and child
@@ -986,6 +988,22 @@ void Booster::init(const DataSet &ds) {
         TGBM_CUDA(cudaMemcpyAsync(m.qinfo.p, &one, sizeof(one), cudaMemcpyHostToDevice, m.stream));
         TGBM_CUDA(cudaStreamSynchronize(m.stream));
     }
+    if (!m.exact && !m.sparse) {
+        std::vector<int4> one, four;
+        for (int f = 0; f < m.F; ++f) {
+            if (m.h_cut_ptr[f + 1] - m.h_cut_ptr[f] > EVAL_SMALL) { one.push_back(make_int4(f, -2, -2, -2)); continue; }
+            if (four.empty() || four.back().w >= 0) { four.push_back(make_int4(f, -1, -1, -1)); continue; }
+            int4 &t = four.back();
+            (t.y < 0 ? t.y : t.z < 0 ? t.z : t.w) = f;
+        }
+        if (four.size() > 1 || (four.size() == 1 && four[0].y >= 0)) {   // (the long ones first)
+            one.insert(one.end(), four.begin(), four.end());
+            m.n_eval_items = (int)one.size();
+            m.eval_items.alloc(one.size());
+            TGBM_CUDA(cudaMemcpyAsync(m.eval_items.p, one.data(), sizeof(int4) * one.size(), cudaMemcpyHostToDevice, m.stream));
+            TGBM_CUDA(cudaStreamSynchronize(m.stream));
+        }
+    }
     m.rstate.alloc(1);
     m.rstate.zero(m.stream);
     m.graphs_allowed = getenv("TGBM_NO_GRAPH") == nullptr;
@@ -1185,13 +1203,14 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
         auto evaluate = [&](auto *built, size_t tree_cells, int bs) {
             using T = std::remove_pointer_t<decltype(built)>;
             if (sparse) {
-                launch_after(k_eval_chunk<T>, dim3(n_chunks, pairs, n_trees), 64, 0, stream, level, b, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_fid.p, built, tree_cells, bs,
+                launch_after(k_eval_chunk<T>, dim3(n_chunks, pairs, n_trees), 64, 0, stream, level, b, n_chunks, B, chunk_bin0.p, cut_ptr.p, cut_val.p, cut_fid.p, built, tree_cells, bs,
                              qinfo.p, p.min_child_weight, p.lambda, ignored_all.p, rstate.p, F, colb, by_hessian, keep);
-                launch_after(k_best_apply, dim3(nl, 1, n_trees), 32, 0, stream, level, b, n_chunks, cut_ptr.p, cut_val.p, p.rt_eps, p.lambda, cut_fid.p, 1, colb);
+                launch_after(k_best_apply, dim3(nl, 1, n_trees), 32, 0, stream, level, b, n_chunks, cut_ptr.p, p.rt_eps, p.lambda, colb);
                 launches += 2;
             } else {
-                launch_after(k_eval<T>, dim3(F, pairs, n_trees), EVAL_THREADS, 0, stream, level, b, F, B, cut_ptr.p, built, tree_cells, bs, qinfo.p, p.min_child_weight, p.lambda,
-                             cut_val.p, p.rt_eps, cut_fid.p, ignored_all.p, rstate.p, colb, by_hessian, keep);
+                const bool items = sizeof(T) == 8 && n_eval_items > 0;
+                launch_after(k_eval<T>, dim3(items ? n_eval_items : F, pairs, n_trees), EVAL_THREADS, 0, stream, level, b, items ? eval_items.p : nullptr, F, B, cut_ptr.p, built, tree_cells, bs, qinfo.p, p.min_child_weight, p.lambda,
+                             cut_val.p, p.rt_eps, ignored_all.p, rstate.p, colb, by_hessian, keep);
                 ++launches;
             }
         };

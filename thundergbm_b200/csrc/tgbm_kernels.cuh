@@ -46,11 +46,13 @@ struct TreeCtl {  // device-side scalars of the booster
     int coarse;  // the running round's gradients do not fit the grid: scores, metric and round counter stay as they are
 };
 
-struct SplitRec {  // best candidate of one (node, feature)
+struct alignas(16) SplitRec {  // best candidate of one (node, feature)
     float gain;     // signed like the reference: negative = missing goes right
     int bin;        // local bin of the candidate, -1 = none
     float lg, lh;   // left sum without missing
     float mg, mh;   // missing sum of the feature in this node
+    float value;    // where it splits
+    int feature;
 };
 
 // ------------------------------------------------------------------ cut points

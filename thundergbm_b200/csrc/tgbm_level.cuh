@@ -603,106 +603,75 @@ __device__ __forceinline__ float split_gain(float parent, float pg, float ph, fl
     return 0.f;
 }
 
-// Per-node argmax over the features, SplitPoint decode and update_tree
-// (hist_tree_builder_single.cu:365-389 and :847-902).  Called by one whole warp for node n of the level.  The records
-// may have been written by other blocks of the running kernel: they are read past L1.
-__device__ __forceinline__ SplitRec load_rec(const SplitRec *p) {
-    SplitRec r;
-    r.gain = __ldcg(&p->gain); r.bin = __ldcg(&p->bin);
-    r.lg = __ldcg(&p->lg); r.lh = __ldcg(&p->lh); r.mg = __ldcg(&p->mg); r.mh = __ldcg(&p->mh);
-    return r;
-}
-// SplitPoint of candidate r (feature-local bin) of feature f into node nd and its children: TreeBuilder::update_tree
 // split value of a feature's candidate, from the feature's cut points
+__device__ __forceinline__ float split_below(float first) { return (float)((double)__fsub_rn(first, fabsf(first)) - 1e-5); }   // of the first bin
 __device__ __forceinline__ float split_at(const float *cuts, int bin, int multi) {
     if (multi) return cuts[bin];   // the column-sharded builder: the cut point itself (tree_builder.cu:9-60)
-    if (bin) return cuts[bin - 1];
-    return (float)((double)__fsub_rn(cuts[0], fabsf(cuts[0])) - 1e-5);
+    return bin ? cuts[bin - 1] : split_below(cuts[0]);
 }
-__device__ __forceinline__ void apply_split(TreeNode *nodes, int nid, int f, const SplitRec &r, float value, float rt_eps, float lam, int multi) {
-    TreeNode &nd = nodes[nid];
+// SplitPoint of candidate r (feature-local bin) into node nid of sums (sum_g, sum_h) and its children: TreeBuilder::update_tree.
+// The table is a heap (Tree::init2): no index is read from it.
+__device__ __forceinline__ void apply_split(TreeNode *nodes, int nid, const SplitRec &r, float sum_g, float sum_h, float rt_eps, float lam, int multi) {
+    TreeNode &nd = nodes[nid], &left = nodes[2 * nid + 1], &right = nodes[2 * nid + 2];
     const float gain = fabsf(r.gain);
-    if (gain > rt_eps) {
-        const bool default_right = r.gain < 0.f;
-        nd.gain = gain;
-        nd.split_feature_id = f;
-        nd.split_bid = (unsigned char)r.bin;
-        nd.split_value = value;
-        if (multi) {
-            // TreeBuilder::update_tree of the column-sharded builder (tree_builder.cu:9-60): the record's sums are the right
-            // child's, the left child is the node minus it
-            TreeNode &l = nodes[nd.lch_index], &rc = nodes[nd.rch_index];
-            l.is_valid = 1; rc.is_valid = 1;
-            float rgs = r.lg, rhs = r.lh;
-            if (default_right) { rgs = __fadd_rn(rgs, r.mg); rhs = __fadd_rn(rhs, r.mh); nd.default_right = 1; }
-            else nd.default_right = 0;
-            rc.sum_g = rgs; rc.sum_h = rhs;
-            l.sum_g = __fsub_rn(nd.sum_g, rgs); l.sum_h = __fsub_rn(nd.sum_h, rhs);
-            l.base_weight = __fdiv_rn(-l.sum_g, __fadd_rn(l.sum_h, lam));
-            rc.base_weight = __fdiv_rn(-rc.sum_g, __fadd_rn(rc.sum_h, lam));
-            return;
-        }
-        TreeNode &l = nodes[nd.lch_index], &rc = nodes[nd.rch_index];
-        l.is_valid = 1; rc.is_valid = 1;
-        float lgs = r.lg, lhs = r.lh;
-        if (!default_right) { lgs = __fadd_rn(lgs, r.mg); lhs = __fadd_rn(lhs, r.mh); nd.default_right = 0; }
-        else nd.default_right = 1;
-        l.sum_g = lgs; l.sum_h = lhs;
-        rc.sum_g = __fsub_rn(nd.sum_g, lgs); rc.sum_h = __fsub_rn(nd.sum_h, lhs);
-        l.base_weight = __fdiv_rn(-l.sum_g, __fadd_rn(l.sum_h, lam));
-        rc.base_weight = __fdiv_rn(-rc.sum_g, __fadd_rn(rc.sum_h, lam));
-    } else {
+    if (!(gain > rt_eps)) {
         nd.is_leaf = 1;
-        nodes[nd.lch_index].is_valid = 0;
-        nodes[nd.rch_index].is_valid = 0;
+        left.is_valid = 0;
+        right.is_valid = 0;
+        return;
     }
+    const bool default_right = r.gain < 0.f;
+    nd.gain = gain;
+    nd.split_feature_id = r.feature;
+    nd.split_bid = (unsigned char)r.bin;
+    nd.split_value = r.value;
+    nd.default_right = default_right ? 1 : 0;
+    // the record's sums are the left child's -- the right one's where the column-sharded builder's candidates are taken
+    // (`multi`, tree_builder.cu:9-60) --, the other child is the node minus it
+    float g = r.lg, h = r.lh;
+    if (default_right == (multi != 0)) { g = __fadd_rn(g, r.mg); h = __fadd_rn(h, r.mh); }
+    const float og = __fsub_rn(sum_g, g), oh = __fsub_rn(sum_h, h), w = __fdiv_rn(-g, __fadd_rn(h, lam)), ow = __fdiv_rn(-og, __fadd_rn(oh, lam));
+    left.is_valid = 1; right.is_valid = 1;
+    left.sum_g = multi ? og : g; left.sum_h = multi ? oh : h; left.base_weight = multi ? ow : w;
+    right.sum_g = multi ? g : og; right.sum_h = multi ? h : oh; right.base_weight = multi ? w : ow;
 }
 
-__device__ __forceinline__ void best_apply_node(int level, int n, int F, const int *__restrict__ cut_ptr,
-                                                const float *__restrict__ cut_val, const SplitRec *recs, TreeNode *nodes,
-                                                float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi) {
-    // chunked: F is the number of chunks and a record's bin is a global bin index (k_eval_chunk);
-    // otherwise one record per feature with a feature-local bin (k_eval).  Ties go to the smaller global bin either way.
-    const int lane = threadIdx.x & 31;
-    const int nid = (1 << level) - 1 + n;
-    if (!nodes[nid].is_valid) return;
+// Per-node argmax over the records, SplitPoint decode and update_tree (hist_tree_builder_single.cu:365-389 and :847-902) of node n
+// of the level, whose sums the caller knows.  Called by one whole warp; the records may have been written by other blocks of the
+// running kernel: they are read past L1.  chunked: F is the number of chunks and a record's bin is a global bin index
+// (k_eval_chunk); otherwise one record per feature with a feature-local bin (k_eval).  Ties go to the smaller global bin.
+__device__ __forceinline__ SplitRec load_rec(const SplitRec *p) {
+    int4 w[2] = {__ldcg(reinterpret_cast<const int4 *>(p)), __ldcg(reinterpret_cast<const int4 *>(p) + 1)};
+    SplitRec r;
+    memcpy(&r, w, sizeof(r));
+    return r;
+}
+__device__ __forceinline__ void best_apply_node(int level, int n, int F, const SplitRec *recs, TreeNode *nodes, float sum_g, float sum_h, float rt_eps, float lam,
+                                                const int *__restrict__ cut_ptr, int chunked, int multi) {
+    const int lane = threadIdx.x & 31, nid = (1 << level) - 1 + n;
     unsigned long long key = 0;
-    int key_col = 0;  // record column (feature or chunk) of this lane's best key
+    SplitRec best;
+    best.bin = -1;
     for (int f = lane; f < F; f += 32) {
         const SplitRec r = load_rec(recs + (size_t)n * F + f);
         if (r.bin < 0) continue;
-        const unsigned long long k = ((unsigned long long)__float_as_uint(fabsf(r.gain)) << 32) |
-                                     (unsigned)(0x7fffffff - (chunked ? r.bin : f));
-        if (k > key) { key = k; key_col = f; }
+        const unsigned long long k = ((unsigned long long)__float_as_uint(fabsf(r.gain)) << 32) | (unsigned)(0x7fffffff - (chunked ? r.bin : f));
+        if (k > key) { key = k; best = r; }
     }
     // a record with gain 0 still has a key > 0, so 0 means "no record"
-    unsigned long long mk = key;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long other = (unsigned long long)shfl_xor_ll((long long)mk, o);
-        mk = other > mk ? other : mk;
-    }
-    const unsigned winners = __ballot_sync(0xffffffffu, key == mk);
-    const int win_col = __shfl_sync(0xffffffffu, key_col, __ffs(winners) - 1);
-    if (lane != 0) return;
-    TreeNode &nd = nodes[nid];
-    if (mk == 0) {  // no feature has a cut point: nothing to split on
-        nd.is_leaf = 1;
-        nodes[nd.lch_index].is_valid = 0;
-        nodes[nd.rch_index].is_valid = 0;
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32) == hi ? (unsigned)key : 0u);
+    if (lo == 0) {  // no feature has a cut point: nothing to split on
+        if (lane == 0) {
+            nodes[nid].is_leaf = 1;
+            nodes[2 * nid + 1].is_valid = 0;
+            nodes[2 * nid + 2].is_valid = 0;
+        }
         return;
     }
-    int f = 0x7fffffff - (int)(mk & 0xffffffffull);
-    SplitRec r;
-    if (chunked) {
-        const int gbin = f;
-        f = cut_fid[gbin];
-        r = load_rec(recs + (size_t)n * F + win_col);
-        r.bin = gbin - cut_ptr[f];
-    } else {
-        r = load_rec(recs + (size_t)n * F + f);
-    }
-    apply_split(nodes, nid, f, r, split_at(cut_val + cut_ptr[f], r.bin, multi), rt_eps, lam, multi);
+    if (key != (((unsigned long long)hi << 32) | lo)) return;   // one lane holds it
+    if (chunked) best.bin -= cut_ptr[best.feature];
+    apply_split(nodes, nid, best, sum_g, sum_h, rt_eps, lam, multi);
 }
 
 // Where the row lists of node n's children start, their lengths zeroed for k_assign to count up.  A node's children take
@@ -717,19 +686,22 @@ __device__ __forceinline__ void open_children(int level, int n, const Batch &b, 
 
 // CSR layout: one warp per node of the level, after k_eval_chunk
 static __global__ void __launch_bounds__(32)
-k_best_apply(int level, const Batch b, int F, const int *__restrict__ cut_ptr, const float *__restrict__ cut_val,
-             float rt_eps, float lam, const int *__restrict__ cut_fid, int chunked, int multi) {
+k_best_apply(int level, const Batch b, int F, const int *__restrict__ cut_ptr, float rt_eps, float lam, int multi) {
     chain_wait();
     const size_t tree = blockIdx.z;
     if (threadIdx.x == 0) open_children(level, blockIdx.x, b, tree);
-    best_apply_node(level, blockIdx.x, F, cut_ptr, cut_val, b.recs + tree * b.recs_stride, b.nodes + tree * b.nodes_stride, rt_eps, lam,
-                    cut_fid, chunked, multi);
+    TreeNode *nodes = b.nodes + tree * b.nodes_stride;
+    const TreeNode &nd = nodes[(1 << level) - 1 + blockIdx.x];
+    if (nd.is_valid) best_apply_node(level, blockIdx.x, F, b.recs + tree * b.recs_stride, nodes, nd.sum_g, nd.sum_h, rt_eps, lam, cut_ptr, 1, multi);
 }
 
 // Sibling subtraction, per-feature prefix scan, missing sums, gains and per-feature argmax
 // (hist_tree_builder_single.cu:257-347 for the root, :538-540 and :614-704 for sibling pairs), then, by the block that
 // finishes a pair last (`ticket`, left at zero), the choice among the features and the tree update of the pair's nodes.
-// grid = (F, pairs, trees); a thread owns two bins of both children.  The gains are the work of this kernel -- four IEEE
+// grid = (items, pairs, trees), an item is a feature or, of features of up to EVAL_SMALL bins, four, a warp each (`items`: the
+// features, -2 behind a single one, -1 for a warp without; null: an item per feature; one-hot columns have one or two bins, and
+// a block each made 24 k blocks of a level of seven trees: 109 us, 44 of 54 columns with two bins); a thread owns two bins of both
+// children.  The gains are the work of this kernel -- four IEEE
 // divisions per bin and child -- and its time is latency: few bins per thread keep a block's chain short, few threads per
 // block keep many blocks resident.  The built histogram is zeroed as it is read, ready for the next level's reductions.
 //
@@ -740,30 +712,36 @@ k_best_apply(int level, const Batch b, int F, const int *__restrict__ cut_ptr, c
 // tree, in T.
 // ignored: the round's column-sampling mask (Shard::column_sampling, src/thundergbm/builder/shard.cu:8-23; the
 // masked features take no part in the split search, hist_tree_builder_single.cu:304,663), or null.
-constexpr int EVAL_THREADS = 128, EVAL_BINS = 2;
+constexpr int EVAL_THREADS = 128, EVAL_BINS = 2, EVAL_SMALL = 32 * EVAL_BINS;
 template <typename T> struct CellPair;
 template <> struct CellPair<long long> { typedef longlong2 type; };
 template <> struct CellPair<float> { typedef float2 type; };
 template <typename T>
 static __global__ void __launch_bounds__(EVAL_THREADS, 8)
-k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, T *built_all, size_t tree_cells, int bs,
+k_eval(int level, const Batch b, const int4 *__restrict__ items, int F, int B, const int *__restrict__ cut_ptr, T *built_all, size_t tree_cells, int bs,
        const QuantInfo *q, float mcw, float lam, const float *__restrict__ cut_val, float rt_eps,
-       const int *__restrict__ cut_fid, const unsigned char *__restrict__ ignored_all, const RoundState *rs, int multi,
-       int by_hessian, int keep) {
+       const unsigned char *__restrict__ ignored_all, const RoundState *rs, int multi, int by_hessian, int keep) {
     // keep = 0 at the last level: no level subtracts from its histograms, so they are not stored
     constexpr int WARPS = EVAL_THREADS / 32, NB = EVAL_BINS;
     __shared__ T s_sum[4][sizeof(T) == 4 ? 32 : WARPS];
     __shared__ unsigned long long s_key[2][WARPS];
-    const int f = blockIdx.x, j = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i0 = threadIdx.x * NB;
+    const int j = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int4 item = sizeof(T) == 8 && items ? items[blockIdx.x] : make_int4(blockIdx.x, -2, -2, -2);
+    const bool packed = sizeof(T) == 8 && item.y != -2;
+    const int f = !packed || warp == 0 ? item.x : warp == 1 ? item.y : warp == 2 ? item.z : item.w, i0 = (packed ? lane : (int)threadIdx.x) * NB;
     const size_t tree = blockIdx.z;
     TreeNode *nodes = b.nodes + tree * b.nodes_stride;
     SplitRec *recs = b.recs + tree * b.recs_stride;
     int *ticket = b.ticket + tree * b.ticket_stride;
-    const int b0 = cut_ptr[f], nb = cut_ptr[f + 1] - b0, off = (1 << level) - 1, n_children = level == 0 ? 1 : 2;
+    const int b0 = cut_ptr[max(f, 0)], nb = f < 0 ? 0 : cut_ptr[f + 1] - b0, off = (1 << level) - 1, n_children = level == 0 ? 1 : 2;
+    // the cut points around the thread's bins: the split value goes with the record
+    float cut[NB + 1];
+#pragma unroll
+    for (int n = 0; n <= NB; ++n) cut[n] = i0 + n - 1 < nb && i0 < nb ? cut_val[b0 + max(i0 + n - 1, 0)] : 0.f;
     chain_wait();
     const int br = level == 0 ? 0 : built_side(level, j, b.seg_cnt[level & 1] + tree * b.seg_stride, nodes, by_hessian);
-    if (f == 0 && (int)threadIdx.x < n_children) open_children(level, level == 0 ? 0 : 2 * j + (int)threadIdx.x, b, tree);
-    const bool ignored = ignored_all && ignored_all[(size_t)rs->round * F + f];
+    if (blockIdx.x == 0 && (int)threadIdx.x < n_children) open_children(level, level == 0 ? 0 : 2 * j + (int)threadIdx.x, b, tree);
+    const bool ignored = ignored_all && f >= 0 && ignored_all[(size_t)rs->round * F + f];
     T *full = reinterpret_cast<T *>(b.hist_full + tree * b.full_stride) + (size_t)off * B * 2;
     T *built = built_all + tree * tree_cells + ((size_t)j * B + b0) * 2 * bs;
     using Pair = typename CellPair<T>::type;
@@ -801,10 +779,12 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
         v[0][n] = br == 1 ? og : cg; v[1][n] = br == 1 ? oh : ch;
         v[2][n] = br == 1 ? cg : og; v[3][n] = br == 1 ? ch : oh;
     }
-    const bool skip = nb == 0 || br < 0 || ignored;   // the same in the whole block
+    const SplitRec none{0.f, -1, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
+    const bool skip = nb == 0 || br < 0 || ignored;   // the same in the whole block, or warp
     if (skip) {
-        if ((int)threadIdx.x < n_children) {
-            recs[(size_t)(level == 0 ? 0 : 2 * j + (int)threadIdx.x) * F + f] = SplitRec{0.f, -1, 0.f, 0.f, 0.f, 0.f};
+        const int c = packed ? lane : (int)threadIdx.x;
+        if (c < n_children && f >= 0) {
+            recs[(size_t)(level == 0 ? 0 : 2 * j + c) * F + f] = none;
             __threadfence();
         }
     } else {
@@ -844,18 +824,21 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
                 for (int o = 1; o < 32; o <<= 1) { const T u = shfl_up_t(incl, o); if (lane >= o) incl += u; }
                 if (lane == 31) s_sum[c][warp] = incl;
                 base[c] = incl - own;
+                tot[c] = packed ? shfl_t(incl, 31) : T(0);
             }
-            __syncthreads();
+            if (!packed) {
+                __syncthreads();
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                T all = 0;
+                for (int c = 0; c < 4; ++c) {
+                    T all = 0;
 #pragma unroll
-                for (int w = 0; w < WARPS; ++w) { if (w == warp) base[c] += all; all += s_sum[c][w]; }
-                tot[c] = all;
+                    for (int w = 0; w < WARPS; ++w) { if (w == warp) base[c] += all; all += s_sum[c][w]; }
+                    tot[c] = all;
+                }
             }
         }
-        float best_gain[2], keep_g[2], keep_h[2], miss_g[2], miss_h[2];
-        unsigned long long key[2];
+        float best_gain[2], keep_g[2], keep_h[2], miss_g[2], miss_h[2], value[2];
+        unsigned long long key[2], top[2];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             key[c] = 0;
@@ -878,25 +861,31 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
                 const float gn = gl > gr ? gl : -gr;
                 // arg-abs-max, ties -> smaller bin (hist_tree_builder_single.cu:330-335)
                 const unsigned long long kk = ((unsigned long long)__float_as_uint(fabsf(gn)) << 32) | (unsigned)(0x7fffffff - i);
-                if (valid[c] && i < nb && kk > key[c]) { key[c] = kk; best_gain[c] = gn; keep_g[c] = kg; keep_h[c] = kh; }
+                if (valid[c] && i < nb && kk > key[c]) {
+                    key[c] = kk; best_gain[c] = gn; keep_g[c] = kg; keep_h[c] = kh;
+                    value[c] = multi ? cut[n + 1] : i ? cut[n] : split_below(cut[n]);
+                }
             }
             // largest key of the warp: the gain first, then the bin among the lanes that hold it
             const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(key[c] >> 32));
             const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(key[c] >> 32) == hi ? (unsigned)key[c] : 0u);
-            if (lane == 0) s_key[c][warp] = ((unsigned long long)hi << 32) | lo;
+            top[c] = ((unsigned long long)hi << 32) | lo;
+            if (lane == 0) s_key[c][warp] = top[c];
         }
-        __syncthreads();
+        if (!packed) __syncthreads();
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             if (c >= n_children) continue;
-            unsigned long long mk = 0;
+            unsigned long long mk = top[c];
+            if (!packed) {
 #pragma unroll
-            for (int w = 0; w < WARPS; ++w) mk = s_key[c][w] > mk ? s_key[c][w] : mk;
+                for (int w = 0; w < WARPS; ++w) mk = s_key[c][w] > mk ? s_key[c][w] : mk;
+            }
             SplitRec *r = recs + (size_t)(level == 0 ? 0 : 2 * j + c) * F + f;
             // the thread that writes the record also makes it visible before the block's ticket is
-            if (mk == 0) { if (threadIdx.x == 0) { *r = SplitRec{0.f, -1, 0.f, 0.f, 0.f, 0.f}; __threadfence(); } }   // the node is not valid
+            if (mk == 0) { if (packed ? lane == 0 : threadIdx.x == 0) { *r = none; __threadfence(); } }   // the node is not valid
             else if (key[c] == mk) {
-                *r = SplitRec{best_gain[c], 0x7fffffff - (int)(unsigned)(mk & 0xffffffffull), keep_g[c], keep_h[c], miss_g[c], miss_h[c]};
+                *r = SplitRec{best_gain[c], 0x7fffffff - (int)(unsigned)(mk & 0xffffffffull), keep_g[c], keep_h[c], miss_g[c], miss_h[c], value[c], f};
                 __threadfence();
             }
         }
@@ -908,9 +897,9 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
         if (last) ticket[j] = 0;
     }
     __syncthreads();
-    if (!last || warp >= n_children) return;
+    if (!last || warp >= n_children || !(warp ? valid[1] : valid[0])) return;
     __threadfence();
-    best_apply_node(level, level == 0 ? 0 : 2 * j + warp, F, cut_ptr, cut_val, recs, nodes, rt_eps, lam, cut_fid, 0, multi);
+    best_apply_node(level, level == 0 ? 0 : 2 * j + warp, F, recs, nodes, warp ? sum_g[1] : sum_g[0], warp ? sum_h[1] : sum_h[0], rt_eps, lam, cut_ptr, 0, multi);
 }
 
 // The same evaluation for data with many narrow features: one block handles a chunk of whole features whose bins
@@ -920,7 +909,7 @@ k_eval(int level, const Batch b, int F, int B, const int *__restrict__ cut_ptr, 
 template <typename T>
 static __global__ void __launch_bounds__(64)
 k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restrict__ chunk_bin0, const int *__restrict__ cut_ptr,
-             const int *__restrict__ cut_fid, T *built_all, size_t tree_cells, int bs, const QuantInfo *q, float mcw, float lam,
+             const float *__restrict__ cut_val, const int *__restrict__ cut_fid, T *built_all, size_t tree_cells, int bs, const QuantInfo *q, float mcw, float lam,
              const unsigned char *__restrict__ ignored_all, const RoundState *rs, int F, int multi, int by_hessian, int keep) {
     chain_wait();
     const size_t tree = blockIdx.z;
@@ -936,7 +925,7 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
     const int n_children = level == 0 ? 1 : 2;
     const int node_local = level == 0 ? 0 : 2 * j + warp;
     const int off = (1 << level) - 1;
-    const SplitRec none = {0.f, -1, 0.f, 0.f, 0.f, 0.f};
+    const SplitRec none{0.f, -1, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
     const int br = level == 0 ? 0 : built_side(level, j, b_.seg_cnt[level & 1] + tree * b_.seg_stride, nodes, by_hessian);
     if (nb == 0 || br < 0) {
         if (lane == 0 && warp < n_children) recs[(size_t)node_local * n_chunks + c] = none;
@@ -1056,15 +1045,11 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
         const unsigned long long other = (unsigned long long)shfl_xor_ll((long long)mk, o);
         mk = other > mk ? other : mk;
     }
-    const unsigned win = __ballot_sync(0xffffffffu, key == mk && best_bin >= 0);
-    const int src = __ffs(win) - 1;
-    best = __shfl_sync(0xffffffffu, best, src);
-    best_bin = __shfl_sync(0xffffffffu, best_bin, src);
-    best_lg = __shfl_sync(0xffffffffu, best_lg, src);
-    best_lh = __shfl_sync(0xffffffffu, best_lh, src);
-    best_mg = __shfl_sync(0xffffffffu, best_mg, src);
-    best_mh = __shfl_sync(0xffffffffu, best_mh, src);
-    if (lane == 0) recs[(size_t)node_local * n_chunks + c] = SplitRec{best, best_bin, best_lg, best_lh, best_mg, best_mh};
+    if (mk == 0) { if (lane == 0) recs[(size_t)node_local * n_chunks + c] = none; }   // every column of the chunk is left out
+    else if (key == mk) {
+        const int f = cut_fid[best_bin];
+        recs[(size_t)node_local * n_chunks + c] = SplitRec{best, best_bin, best_lg, best_lh, best_mg, best_mh, split_at(cut_val + cut_ptr[f], best_bin - cut_ptr[f], multi), f};
+    }
 }
 
 

@@ -24,7 +24,6 @@ constexpr int SMALL_THREADS = 1024;
 struct SmallPost {   // a CTA's best candidate of a node: |gain| bits << 32 | (0x7fffffff - feature), 0 = none
     unsigned long long key;
     SplitRec rec;
-    float value;           // where it splits
 };
 
 // A feature's bins stand one word further apart every eighth bin, so that the lanes of the split search, eight consecutive bins
@@ -131,7 +130,7 @@ __device__ __noinline__ void small_eval(const SmallSearch &x, const int *cell, i
     }
     if (!active) return;
     if (top == 0) { if (lane == 0) out->bin = -1; }   // (a part without bins)
-    else if (key == top) *out = SplitRec{best, 0x7fffffff - (int)(unsigned)top, keep_g, keep_h, mg, mh};
+    else if (key == top) *out = SplitRec{best, 0x7fffffff - (int)(unsigned)top, keep_g, keep_h, mg, mh, 0.f, 0};
 }
 
 // grid = trees x plan.cluster, clusters of plan.cluster CTAs
@@ -152,7 +151,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
     TreeNode *nodes = reinterpret_cast<TreeNode *>(small_sm);
     SmallPost *posts = reinterpret_cast<SmallPost *>(small_sm + (sizeof(TreeNode) * n_nodes + 15) / 16 * 16);   // [2][max_nl]
     SplitRec *recs = reinterpret_cast<SplitRec *>(posts + 2 * max_nl);                                       // [nodes_pass][feats]
-    unsigned *split = reinterpret_cast<unsigned *>(recs + (plan.nodes_pass * plan.feats + 1) / 2 * 2);   // [max_nl] what the level decided
+    unsigned *split = reinterpret_cast<unsigned *>(recs + plan.nodes_pass * plan.feats);                 // [max_nl] what the level decided
     unsigned short *node_of = reinterpret_cast<unsigned short *>(split + (max_nl + 3) / 4 * 4);            // [N, eights]
     int *s_first = reinterpret_cast<int *>(node_of + (N + 7) / 8 * 8);                                           // [feats + 1] bins before the own features
     float *s_cut = reinterpret_cast<float *>(s_first + plan.feats + 1);                                          // [bins] their cut points
@@ -312,7 +311,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
                     const SplitRec r = recs[n * plan.feats + f];
                     if (r.bin < 0) continue;
                     const unsigned long long k = ((unsigned long long)__float_as_uint(fabsf(r.gain)) << 32) | (unsigned)(0x7fffffff - (f0 + f));
-                    if (k > p.key) { p.key = k; p.rec = r; p.value = split_at(s_cut + s_first[f], r.bin, multi); }
+                    if (k > p.key) { p.key = k; p.rec = r; p.rec.value = split_at(s_cut + s_first[f], r.bin, multi); p.rec.feature = f0 + f; }
                 }
                 post[n0 + n] = p;
             }
@@ -338,9 +337,8 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
                     TreeNode &nd = nodes[off + n];
                     if (best == 0) nd.is_leaf = 1;   // no feature has a cut point: nothing to split on
                     else {
-                        const SmallPost &p = cluster.map_shared_rank(post, from)[n];
-                        const SplitRec r = p.rec;
-                        apply_split(nodes, off + n, 0x7fffffff - (int)(unsigned)(best & 0xffffffffull), r, p.value, rt_eps, lam, multi);
+                        const SplitRec r = cluster.map_shared_rank(post, from)[n].rec;
+                        apply_split(nodes, off + n, r, nd.sum_g, nd.sum_h, rt_eps, lam, multi);
                     }
                     if (!nd.is_leaf) {
                         s_split = 1;
