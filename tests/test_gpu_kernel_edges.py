@@ -196,3 +196,42 @@ def test_blocks_of_the_split_search(gpu, orc, widths, extra):
     keep = r.random(x.shape) < np.where(np.array(widths) > 0, 0.85, 0.0)
     y = x @ r.normal(size=len(widths)) + keep[:, 0] + r.random(n)
     _same_as_oracle(orc, _holes(x, y, keep), depth=6, n_trees=2, max_num_bin=255, learning_rate=0.5, objective='reg:linear', num_class=1, **extra)
+
+
+# columns that exclude each other share a byte of the row-major matrix: groups of one-hot columns, of columns with several bins that
+# just fit a byte or do not, an empty column between them, one row that stores two of a group, rows whose columns come unordered
+@pytest.mark.parametrize('widths,both,shuffle', [([1] * 60 + [30], False, False), ([85] * 3 + [1] * 50, False, False), ([86] * 3 + [1] * 50, False, True),
+                                                 ([5] * 20 + [0] + [5] * 20, False, False), ([2] * 50, True, False)])
+@pytest.mark.parametrize('mode', ['exact', 'fp32'])
+def test_columns_that_share_a_byte(gpu, orc, widths, both, shuffle, mode):
+    from thundergbm_b200.booster import Booster
+    n, f, r = 33_000, len(widths) + 2, np.random.default_rng(len(widths))
+    x, keep = np.zeros((n, f), np.float32), np.zeros((n, f), bool)
+    of = r.choice(np.nonzero(widths)[0], n)           # every row stores one of the group
+    row = np.arange(n)
+    x[row, of] = 1 + r.integers(0, np.array(widths)[of])
+    keep[row, of] = r.random(n) < 0.9
+    if both:
+        x[7, 3] = x[7, 30] = 1
+        keep[7, [3, 30]] = True
+    x[:, -2:] = r.integers(1, 200, (n, 2))            # two columns of their own
+    keep[:, -2:] = r.random((n, 2)) < 0.8
+    d = _holes(x, x[:, -1] / 50 + np.sin(of) + x.sum(1) / 100 + r.random(n), keep)
+    in_order = d                                      # (what the oracle expects)
+    if shuffle:
+        ptr, col, val = d.row_ptr, d.col.copy(), d.val.copy()
+        for i in range(0, n, 3):
+            col[ptr[i]:ptr[i + 1]], val[ptr[i]:ptr[i + 1]] = d.col[ptr[i]:ptr[i + 1]][::-1], d.val[ptr[i]:ptr[i + 1]][::-1]
+        d = CsrData(n, f, ptr, col, val, d.y)
+    p = dict(depth=6, n_trees=3, max_num_bin=255, learning_rate=0.5, objective='reg:linear', num_class=1)
+    o = orc.train(in_order, hist_mode=int(mode == 'exact'), **p)
+    b = Booster(d, hist_mode=mode, **p)
+    cut_val, cut_ptr, bins = orc.bin_only(in_order, 255)
+    assert np.array_equal(b.bins(), orc.bins_to_dense(in_order, bins, cut_ptr, b.info.fpad))
+    b.boost(3)
+    if mode == 'exact':
+        assert b.trees().tobytes() == o.trees.tobytes() and np.array_equal(b.ypred(), o.ypred)
+    root, want = b.trees()[0, 0][0], o.trees[0, 0][0]
+    assert root['split_feature_id'] == want['split_feature_id'] and root['split_bid'] == want['split_bid']
+    assert np.max(np.abs(b.metrics() - o.metric)) <= 1e-4 * np.max(o.metric)
+    b.close()

@@ -30,7 +30,7 @@ struct BoosterImpl {
     const Comm *comm = nullptr;
     cudaStream_t stream = nullptr;
     int objective = REG_LINEAR;
-    int N = 0, F = 0, Fpad = 0, G = 0, B = 0, K = 1, n_nodes = 0, depth = 0;
+    int N = 0, F = 0, Fpad = 0, B = 0, K = 1, n_nodes = 0, depth = 0;
     long long N_global = 0;
     long long row_offset = 0;  // global id of local row 0
     size_t Npad = 0;
@@ -47,6 +47,11 @@ struct BoosterImpl {
 
     DeviceRows in;   // the stored values on the device, held from upload_rows() to the end of binning
     DevBuf<unsigned char> bins, binsT;
+    // slots of `bins`: features, or neighbouring ones that share a byte (k_last_before)
+    int S = 0, Spad = 0;
+    std::vector<int> h_slot_ptr;   // first bin of every slot
+    DevBuf<int> slot_ptr;
+    void bundle_columns();
     // wide sparse data: CSR of global bin ids instead of the two dense matrices
     bool sparse = false;
     long long nnz_local = 0;
@@ -322,6 +327,42 @@ struct SideStreams {
         if (ev) cudaEventDestroy(ev);
     }
 };
+
+// Fewer bytes per row for the histogram kernels, which take 32 slots of a row at a time whatever they hold: used where whole
+// groups of 32 go.  (581 k rows x 54 columns, 44 of them two one-hot groups: 12 slots.)
+void BoosterImpl::bundle_columns() {
+    S = F; Spad = Fpad;
+    h_slot_ptr = h_cut_ptr;
+    if (in.full_cols == F || Fpad == 32 || F > 8192 || !N) return;   // (a full matrix has no two columns that exclude each other)
+    DevBuf<int> last;
+    last.alloc(F);
+    TGBM_CUDA(cudaMemsetAsync(last.p, 0xff, sizeof(int) * F, stream));
+    k_last_before<<<std::min(ceil_div(N, 256), num_sms * 4), 256, sizeof(int) * F, stream>>>(bins.p, N, Fpad, F, last.p);
+    std::vector<int> h_last(F), slot(F), shift(F), ptr;
+    TGBM_CUDA(cudaMemcpyAsync(h_last.data(), last.p, sizeof(int) * F, cudaMemcpyDeviceToHost, stream));
+    TGBM_CUDA(cudaStreamSynchronize(stream));
+    int a = -1;   // first feature of the running slot
+    for (int f = 0; f < F; ++f) {
+        if (a < 0 || h_last[f] >= a || h_cut_ptr[f + 1] - h_cut_ptr[a] > MISSING_BIN) { a = f; ptr.push_back(h_cut_ptr[f]); }
+        slot[f] = (int)ptr.size() - 1;
+        shift[f] = h_cut_ptr[f] - h_cut_ptr[a];
+    }
+    const int slots = (int)ptr.size(), pad = (slots + 31) / 32 * 32;
+    if (pad == Fpad) return;
+    ptr.push_back(B);
+    DevBuf<int> d_slot, d_shift;
+    DevBuf<unsigned char> packed;
+    d_slot.alloc(F); d_shift.alloc(F); slot_ptr.alloc(slots + 1); packed.alloc((size_t)N * pad);
+    TGBM_CUDA(cudaMemcpyAsync(d_slot.p, slot.data(), sizeof(int) * F, cudaMemcpyHostToDevice, stream));
+    TGBM_CUDA(cudaMemcpyAsync(d_shift.p, shift.data(), sizeof(int) * F, cudaMemcpyHostToDevice, stream));
+    TGBM_CUDA(cudaMemcpyAsync(slot_ptr.p, ptr.data(), sizeof(int) * ptr.size(), cudaMemcpyHostToDevice, stream));
+    TGBM_CUDA(cudaMemsetAsync(packed.p, MISSING_BIN, packed.bytes(), stream));
+    k_bundle<<<std::min(ceil_div(N, 256), num_sms * 8), 256, 0, stream>>>(bins.p, N, Fpad, F, d_slot.p, d_shift.p, pad, packed.p);
+    TGBM_CUDA(cudaStreamSynchronize(stream));
+    bins.take(packed);
+    S = slots; Spad = pad;
+    h_slot_ptr = ptr;
+}
 
 // The stored values of the CSR layout once more by column, for the kernels that look for the rows of a column: one sort by bin
 // id, the rows stay in order.  Not where a row stores a column twice (which of its values counts is up to the search then).
@@ -646,6 +687,7 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
         TGBM_CUDA(cudaMemsetAsync(bins.p, MISSING_BIN, bins.bytes(), stream));
         TGBM_CUDA(cudaMemsetAsync(binsT.p, MISSING_BIN, binsT.bytes(), stream));
         if (N) k_bin_dense<<<ceil_div(N, 128), 128, 0, stream>>>(in.row_ptr.p, in.col.p, in.val.p, in.full_cols, N, cut_ptr.p, cut_val.p, Fpad, Npad, bins.p, binsT.p, colb ? 1 : 0);
+        bundle_columns();
     }
     TGBM_CUDA(cudaStreamSynchronize(stream));
     TGBM_CUDA(cudaGetLastError());
@@ -847,7 +889,6 @@ void Booster::init(const DataSet &ds) {
     TGBM_CHECK(m.N_global < (1ll << 31), "row count must fit 32 bits");
     TGBM_CHECK(m.F >= 1, "data set has no features");
     m.Fpad = (m.F + 31) / 32 * 32;
-    m.G = m.Fpad / 32;
     m.Npad = ((size_t)m.N + 127) / 128 * 128;
 
     // number of classes / trees per round (src/thundergbm/trainer.cu:26-37)
@@ -979,7 +1020,7 @@ void Booster::init(const DataSet &ds) {
     m.metric.alloc(std::max(p.n_trees, 1));
     if (p.keep_nid) m.nid_keep.alloc(n1 * K * std::max(p.n_trees, 1));
     if (m.f32) {
-        for (int f = 0; f < std::min(m.F, 256); ++f) m.f32_cuts.v[f] = m.h_cut_ptr[f];
+        for (int f = 0; f < std::min(m.S, 256); ++f) m.f32_cuts.v[f] = m.h_slot_ptr[f];
         m.spread_cells = std::min<size_t>((size_t)32 * m.batch * max_pairs * B1, (size_t)8 << 20);   // 64 MB: they stay in L2
         m.hist_spread.alloc(m.spread_cells);
         m.hist_spread.zero(m.stream);
@@ -1194,8 +1235,9 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
     }
     const int by_hessian = (comm && comm->active()) ? 1 : 0;
     const int colb = p.column_shards > 0 ? 1 : 0;  // candidates, tie rule and child sums of the column-sharded builder
-    // one CTA per SM over all trees and feature groups: every further CTA is one more flush per node
-    const int hist_ctas = std::max(1, num_sms / (n_trees * (sparse ? 1 : G)));
+    // one CTA per SM over all trees and groups of slots: every further CTA is one more flush per node
+    const int G = sparse ? 1 : Spad / 32, hist_ctas = std::max(1, num_sms / (n_trees * G));
+    const int *slots = slot_ptr.p ? slot_ptr.p : cut_ptr.p;
     for (int level = 0; level < depth && !one_launch; ++level) {
         const int nl = 1 << level, pairs = std::max(1, nl / 2), keep = level == 0 || level + 1 < depth;
         const size_t table = sizeof(int) * ((size_t)pairs + 1);
@@ -1239,7 +1281,7 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
                     launch_after(kern, dim3(ctas, 1, n_trees), F32_THREADS, table, stream, level, b, sp_row_ptr.p, sp_bin.p, cells, tree_cells, B, bs, by_hessian);
                 } else {
                     auto kern = level == 0 ? k_hist_f32<false> : k_hist_f32<true>;
-                    launch_after(kern, dim3(ctas, G, n_trees), F32_THREADS, table, stream, level, b, bins.p, Fpad, F, cut_ptr.p, cells, tree_cells, B, bs, f32_cuts, F <= 256,
+                    launch_after(kern, dim3(ctas, G, n_trees), F32_THREADS, table, stream, level, b, bins.p, Spad, S, slots, cells, tree_cells, B, bs, f32_cuts, S <= 256,
                                  f32_staged ? 1 : 0, by_hessian);
                 }
             });
@@ -1265,7 +1307,7 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
                     launch_after(kern, dim3(hist_ctas, 1, n_trees), SPARSE_THREADS, (size_t)std::min(B, SPARSE_SMEM_BINS) * 16 + table, stream, level, b, sp_row_ptr.p, sp_bin.p, B, by_hessian);
                 } else {
                     auto kern = level == 0 ? (fine ? k_hist<false, true> : k_hist<false, false>) : (fine ? k_hist<true, true> : k_hist<true, false>);
-                    launch_after(kern, dim3(hist_ctas, G, n_trees), HIST_THREADS, (fine ? HIST_FINE_SMEM : HIST_EXACT_SMEM) + table, stream, level, b, bins.p, Fpad, F, cut_ptr.p, B, window_rows, by_hessian);
+                    launch_after(kern, dim3(hist_ctas, G, n_trees), HIST_THREADS, (fine ? HIST_FINE_SMEM : HIST_EXACT_SMEM) + table, stream, level, b, bins.p, Spad, S, slots, B, window_rows, by_hessian);
                 }
             });
             ++launches;
@@ -1540,7 +1582,13 @@ std::vector<int> Booster::get_cut_ptr() const { return impl_->h_cut_ptr; }
 std::vector<unsigned char> Booster::get_bins() {
     sync();
     TGBM_CHECK(!impl_->sparse, "the booster holds the CSR layout: use get_bins_csr");
-    return to_host(impl_->bins.p, (size_t)impl_->N * impl_->Fpad);
+    const BoosterImpl &m = *impl_;
+    if (m.S == m.F) return to_host(m.bins.p, (size_t)m.N * m.Fpad);
+    const auto columns = to_host(m.binsT.p, (size_t)m.F * m.Npad);   // (several features share a byte of the other matrix)
+    std::vector<unsigned char> rows((size_t)m.N * m.Fpad, MISSING_BIN);
+    for (int f = 0; f < m.F; ++f)
+        for (int r = 0; r < m.N; ++r) rows[(size_t)r * m.Fpad + f] = columns[(size_t)f * m.Npad + r];
+    return rows;
 }
 std::vector<int> Booster::get_bins_csr() {
     sync();

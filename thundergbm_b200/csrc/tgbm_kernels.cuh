@@ -3,8 +3,9 @@
 // (the kernels of a tree level are in tgbm_level.cuh)
 //
 // Data layout in HBM (one rank = one contiguous block of rows):
-//   bins   uint8 [N][Fpad]   row-major local bin ids, Fpad = F rounded up to 32, 255 = missing.
-//                            One 32-byte sector holds 32 features of one row.
+//   bins   uint8 [N][Spad]   row-major bin ids by slot, Spad = slots rounded up to 32, 255 = missing.  A slot is a feature, or
+//                            neighbouring features of which no row stores two (one-hot groups): its bins are theirs one after
+//                            the other.  One 32-byte sector holds 32 slots of one row.
 //   binsT  uint8 [F][Npad]   the same matrix column-major; read by k_assign, which
 //                            needs one feature of many rows.
 //   gh     float2 [K][N]     gradient pairs of the round, class-major like the reference.
@@ -211,6 +212,45 @@ static __global__ void k_bin_dense(const int *__restrict__ row_ptr, const int *_
         const unsigned char b = (unsigned char)(lo - b0);
         bins[(size_t)r * Fpad + f] = b;
         binsT[(size_t)f * Npad + r] = b;
+    }
+}
+
+// Neighbouring features of which no row stores two may share a byte of the row-major matrix (exclusive feature bundling, Ke et
+// al., "LightGBM", NIPS 2017, section 4, without its tolerance for conflicts).  last[f] = the largest feature below f that a row
+// with a value of f stores as well, -1 if none: [a, f] may share a byte if last is below a for all of them but a.
+static __global__ void __launch_bounds__(256)
+k_last_before(const unsigned char *__restrict__ bins, int n_rows, int Fpad, int F, int *__restrict__ last) {
+    extern __shared__ int s_last[];   // [F]
+    for (int f = threadIdx.x; f < F; f += 256) s_last[f] = -1;
+    __syncthreads();
+    for (int r = blockIdx.x * 256 + threadIdx.x; r < n_rows; r += gridDim.x * 256) {
+        const uint4 *row = reinterpret_cast<const uint4 *>(bins + (size_t)r * Fpad);
+        int before = -1;
+        for (int q = 0; q < Fpad / 16; ++q) {
+            const uint4 v = row[q];
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                if (((w[k >> 2] >> (8 * (k & 3))) & 0xffu) == MISSING_BIN) continue;
+                const int f = q * 16 + k;
+                if (before > *(volatile int *)&s_last[f]) atomicMax(&s_last[f], before);
+                before = f;
+            }
+        }
+    }
+    __syncthreads();
+    for (int f = threadIdx.x; f < F; f += 256)
+        if (s_last[f] >= 0) atomicMax(last + f, s_last[f]);
+}
+// the matrix by slot: feature f's bins start at `shift[f]` of slot `slot[f]`
+static __global__ void __launch_bounds__(256)
+k_bundle(const unsigned char *__restrict__ bins, int n_rows, int Fpad, int F, const int *__restrict__ slot, const int *__restrict__ shift, int Spad,
+         unsigned char *__restrict__ out) {
+    for (int r = blockIdx.x * 256 + threadIdx.x; r < n_rows; r += gridDim.x * 256) {
+        const unsigned char *row = bins + (size_t)r * Fpad;
+        unsigned char *to = out + (size_t)r * Spad;
+        for (int f = 0; f < F; ++f)
+            if (row[f] != MISSING_BIN) to[slot[f]] = (unsigned char)(row[f] + shift[f]);
     }
 }
 
