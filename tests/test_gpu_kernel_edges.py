@@ -235,3 +235,29 @@ def test_columns_that_share_a_byte(gpu, orc, widths, both, shuffle, mode):
     assert root['split_feature_id'] == want['split_feature_id'] and root['split_bid'] == want['split_bid']
     assert np.max(np.abs(b.metrics() - o.metric)) <= 1e-4 * np.max(o.metric)
     b.close()
+
+
+# binning: full rows with and without 16-byte alignment, groups of 32 with remainders, CSR rows of few and of many values; features
+# of 1, 2, 254 and more distinct values, infinities and zeros of either sign
+@pytest.mark.parametrize('n,f,holes', [(1, 1, 0), (257, 4, 0), (1000, 33, 0), (300, 64, 0), (16_384, 30, 0.1), (16_385, 67, 0.3), (17_000, 40, 0.6)])
+def test_bins(gpu, n, f, holes):
+    from thundergbm_b200.booster import Booster
+    r = np.random.default_rng(n + f)
+    x = r.standard_normal((n, f)).astype(np.float32)
+    for j, levels in enumerate([1, 2, 253, 254, 255, 256, 600]):
+        if j < f:
+            x[:, j] = r.integers(0, levels, n) - levels // 2
+    if n > 100:
+        x[5:9, f - 1] = np.inf, -np.inf, 0.0, -0.0
+    keep = r.random((n, f)) >= holes
+    d = _holes(x, r.random(n), keep) if holes else _csr(x, r.random(n))
+    b = Booster(d, depth=2, n_trees=1, objective='reg:linear', tree_method='hist')
+    cut, ptr = b.cuts()
+    got = b.bins()
+    want = np.full(got.shape, 255, np.uint8)
+    for j in range(f):
+        c = cut[ptr[j]:ptr[j + 1]]
+        if len(c):
+            want[:, j] = np.where(keep[:, j], np.minimum(np.searchsorted(c, x[:, j], 'right'), len(c) - 1), 255)
+    assert np.array_equal(got, want)
+    b.close()

@@ -300,6 +300,9 @@ void BoosterImpl::column_builder_candidates(DevBuf<unsigned long long> &ukeys, D
 // of 64-bit keys 1.7 / 3.4 / 16.6 ms.
 constexpr int BY_COLUMN_ROWS = 1 << 21;
 constexpr int SORT_LANES = 4;   // columns sorted side by side
+// CSR rows binned by k_bin_rows: from so many rows on laying out the search trees of all columns pays, from so many values a row
+// a warp per row (300 k rows x 136: 1.3 ms with a thread per row, 0.2 so; 581 k rows x 12 values: 0.09 against 0.16)
+constexpr int BIN_ROWS_FROM = 16384, BIN_ROWS_VALUES = 24;
 
 // streams that start after what `main` holds now; join() makes `main` wait for them
 struct SideStreams {
@@ -333,7 +336,8 @@ struct SideStreams {
 void BoosterImpl::bundle_columns() {
     S = F; Spad = Fpad;
     h_slot_ptr = h_cut_ptr;
-    if (in.full_cols == F || Fpad == 32 || F > 8192 || !N) return;   // (a full matrix has no two columns that exclude each other)
+    // (a full matrix has no two columns that exclude each other; up to SMALL_ROWS the trees are mostly built without these rows)
+    if (in.full_cols == F || Fpad == 32 || F > 8192 || N <= SMALL_ROWS) return;
     DevBuf<int> last;
     last.alloc(F);
     TGBM_CUDA(cudaMemsetAsync(last.p, 0xff, sizeof(int) * F, stream));
@@ -684,9 +688,20 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
     } else {
         bins.alloc((size_t)N * Fpad);
         binsT.alloc((size_t)F * Npad + ASSIGN_CHUNK);   // (k_assign reads the first column to the end of a chunk)
-        TGBM_CUDA(cudaMemsetAsync(bins.p, MISSING_BIN, bins.bytes(), stream));
-        TGBM_CUDA(cudaMemsetAsync(binsT.p, MISSING_BIN, binsT.bytes(), stream));
-        if (N) k_bin_dense<<<ceil_div(N, 128), 128, 0, stream>>>(in.row_ptr.p, in.col.p, in.val.p, in.full_cols, N, cut_ptr.p, cut_val.p, Fpad, Npad, bins.p, binsT.p, colb ? 1 : 0);
+        const size_t tree_smem = sizeof(float) * (size_t)F * (BIN_TREE + 1);
+        if (N && !colb && in.full_cols == F) {
+            auto kern = F % 4 == 0 ? k_bin_full<true> : k_bin_full<false>;
+            kern<<<dim3(std::min(ceil_div(N, 256), num_sms * 4), Fpad / 32), 256, 0, stream>>>(in.val.p, N, F, cut_ptr.p, cut_val.p, Fpad, Npad, bins.p, binsT.p);
+        } else if (N && !colb && !in.full_cols && tree_smem <= BIN_ROWS_SMEM && N >= BIN_ROWS_FROM && nnz >= BIN_ROWS_VALUES * (size_t)N) {
+            TGBM_CUDA(cudaFuncSetAttribute(k_bin_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, BIN_ROWS_SMEM));
+            TGBM_CUDA(cudaMemsetAsync(bins.p, MISSING_BIN, bins.bytes(), stream));
+            k_bin_rows<<<std::min(ceil_div(N, 32), num_sms), 1024, tree_smem, stream>>>(in.row_ptr.p, in.col.p, in.val.p, N, F, cut_ptr.p, cut_val.p, Fpad, bins.p);
+            k_bins_by_column<<<dim3((unsigned)(Npad / 128), Fpad / 32), 256, 0, stream>>>(bins.p, N, F, Fpad, Npad, binsT.p);
+        } else {
+            TGBM_CUDA(cudaMemsetAsync(bins.p, MISSING_BIN, bins.bytes(), stream));
+            TGBM_CUDA(cudaMemsetAsync(binsT.p, MISSING_BIN, binsT.bytes(), stream));
+            if (N) k_bin_dense<<<ceil_div(N, 128), 128, 0, stream>>>(in.row_ptr.p, in.col.p, in.val.p, in.full_cols, N, cut_ptr.p, cut_val.p, Fpad, Npad, bins.p, binsT.p, colb ? 1 : 0);
+        }
         bundle_columns();
     }
     TGBM_CUDA(cudaStreamSynchronize(stream));
@@ -1165,7 +1180,7 @@ void BoosterImpl::init_base_score() {
 // of the level kernels takes 25-30 us at any size up to a few hundred thousand rows.
 void BoosterImpl::plan_small_trees() {
     small = SmallPlan{};
-    if (sparse || exact || (comm && comm->active()) || N < 1 || N > 32768 || depth < 1 || F > 4096) return;
+    if (sparse || exact || (comm && comm->active()) || N < 1 || N > SMALL_ROWS || depth < 1 || F > 4096) return;
     SmallPlan pl{};
     pl.cluster = 1;
     while (pl.cluster < 16 && pl.cluster < F) pl.cluster *= 2;

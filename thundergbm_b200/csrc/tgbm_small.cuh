@@ -19,7 +19,7 @@
 
 namespace tgbm {
 
-constexpr int SMALL_THREADS = 1024;
+constexpr int SMALL_THREADS = 1024, SMALL_ROWS = 32768;   // most rows
 
 struct SmallPost {   // a CTA's best candidate of a node: |gain| bits << 32 | (0x7fffffff - feature), 0 = none
     unsigned long long key;
