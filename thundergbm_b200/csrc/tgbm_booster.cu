@@ -780,7 +780,7 @@ void BoosterImpl::exact_levels(int k, const void *gh_rows) {
     typedef typename ExKind<T>::W W;
     TGBM_CUDA(cudaMemsetAsync(ex_nid.p, 0, sizeof(int) * (size_t)std::max(N, 1), stream));
     if (!ex_nnz) return;   // no stored value: the root stays as it is
-    const int grid = std::max(1, std::min(ceil_div(ex_nnz, EX_TILE), num_sms * 8));
+    const int tiles = std::max(1, ceil_div(ex_nnz, EX_TILE)), grid = std::min(tiles, num_sms * EX_SEARCH_BLOCKS), move_grid = std::min(tiles, num_sms * EX_MOVE_BLOCKS);
     const int row_grid = std::max(1, std::min(ceil_div(std::max(N, 1), 256), num_sms * 8));
     ExPair<V> *pre = reinterpret_cast<ExPair<V> *>(ex_pre.p);
     ExPair<W> *tile_pre = reinterpret_cast<ExPair<W> *>(ex_tile_pre.p), *run_sum = reinterpret_cast<ExPair<W> *>(ex_run.p), *run_pre = run_sum + num_sms * 8;
@@ -801,9 +801,9 @@ void BoosterImpl::exact_levels(int k, const void *gh_rows) {
         launch_after(k_exact_move_missing, row_grid, 256, 0, stream, ex_nid.p, N, level, nodes.p, ex_any.p, ex_side.p);
         launches += 4;
         if (level + 1 == depth) break;
-        launch_after(k_exact_sides, grid, EX_THREADS, 0, stream, live, ex_row[a].p, ex_side.p, ex_lr.p, ex_tile_lr.p, run_cnt, run_lr, ex_live.p + level + 1,
+        launch_after(k_exact_sides, move_grid, EX_THREADS, 0, stream, live, ex_row[a].p, ex_side.p, ex_lr.p, ex_tile_lr.p, run_cnt, run_lr, ex_live.p + level + 1,
                      ex_ticket.p);
-        launch_after(k_exact_scatter<In>, grid, EX_THREADS, 0, stream, live, ex_key[a].p, ex_row[a].p, ex_val[a].p, gh_of(a), ex_lr.p, ex_tile_lr.p, run_lr, ex_group.p, ex_key[z].p,
+        launch_after(k_exact_scatter<In>, move_grid, EX_THREADS, 0, stream, live, ex_key[a].p, ex_row[a].p, ex_val[a].p, gh_of(a), ex_lr.p, ex_tile_lr.p, run_lr, ex_group.p, ex_key[z].p,
                      ex_row[z].p, ex_val[z].p, gh_of(z));
         launches += 2;
     }

@@ -21,6 +21,11 @@ namespace tgbm {
 
 constexpr int EX_THREADS = 256, EX_ITEMS = 4, EX_TILE = EX_THREADS * EX_ITEMS;   // entries are handled in tiles, four neighbours per thread
 
+// Blocks per SM of the passes over the entries, all resident at once: the two of a pair share the runs of tiles, so they have the same
+// grid.  (Eight per SM, of which three to six fit, are 1.3 to 2.7 waves: 39 us for the sums of 5.6 M entries and 25 for the sides
+// that take 29 and 21 so.  With 5 and 6 per SM 28 and 22, but the scatter 60 instead of 48; with 3 and 4 the gains 59 instead of 52.)
+constexpr int EX_SEARCH_BLOCKS = 4, EX_MOVE_BLOCKS = 5;
+
 template <typename T> struct ExPair { T g, h; };
 template <typename T> __device__ __forceinline__ ExPair<T> operator+(const ExPair<T> &a, const ExPair<T> &b) { return ExPair<T>{a.g + b.g, a.h + b.h}; }
 template <typename T> __device__ __forceinline__ ExPair<T> operator-(const ExPair<T> &a, const ExPair<T> &b) { return ExPair<T>{a.g - b.g, a.h - b.h}; }
@@ -29,8 +34,8 @@ template <typename T> __device__ __forceinline__ ExPair<T> operator-(const ExPai
 template <typename T> struct ExKind;
 template <> struct ExKind<long long> { typedef int2 In; typedef int V; typedef long long W; };
 template <> struct ExKind<float> { typedef float2 In; typedef double V; typedef double W; };
-__device__ __forceinline__ float exact_cell(long long v, double inv) { return cell_f(v, inv); }
-__device__ __forceinline__ float exact_cell(double v, double) { return __double2float_rn(v); }
+__device__ __forceinline__ float exact_cell(long long v, const GridScale &s) { return s(v); }
+__device__ __forceinline__ float exact_cell(double v, const GridScale &) { return __double2float_rn(v); }
 
 // four neighbours at once, 16 bytes per access (one access each of 8 bytes: every 32-byte sector four times)
 template <typename E> __device__ __forceinline__ void exact_load4(const E *p, E (&v)[4]) {
@@ -129,7 +134,7 @@ __device__ __forceinline__ ExPair<W> exact_scan_runs(const ExPair<W> *sums, ExPa
 // The root fetches the gradients by row (GATHER, a 32-byte sector for 8 bytes) and writes them down; from there on they
 // travel with the entries.
 template <typename T, bool GATHER>
-static __global__ void __launch_bounds__(EX_THREADS)
+static __global__ void __launch_bounds__(EX_THREADS, EX_SEARCH_BLOCKS)
 k_exact_sum(const int *live, const unsigned *key, const int *row, const typename ExKind<T>::In *gh_rows,
             typename ExKind<T>::In *gh, ExPair<typename ExKind<T>::V> *pre,
             ExPair<typename ExKind<T>::W> *tile_pre, ExPair<typename ExKind<T>::W> *run_sum, ExPair<typename ExKind<T>::W> *run_pre, int2 *group, int *ticket) {
@@ -204,7 +209,7 @@ __device__ __forceinline__ ExPair<typename ExKind<T>::W> exact_before(const ExSe
 // right-child candidate sums and missing sums of a node
 struct ExCand { float rg, rh, mg, mh; };
 template <typename W>
-__device__ __forceinline__ ExCand exact_cand(const TreeNode &nd, const ExPair<W> &right, const ExPair<W> &total, double inv_sg, double inv_sh) {
+__device__ __forceinline__ ExCand exact_cand(const TreeNode &nd, const ExPair<W> &right, const ExPair<W> &total, const GridScale &inv_sg, const GridScale &inv_sh) {
     // exact_tree_builder.cu:160-167 (missing = node sum - sum of the stored values)
     return ExCand{exact_cell(right.g, inv_sg), exact_cell(right.h, inv_sh),
                   __fsub_rn(nd.sum_g, exact_cell(total.g, inv_sg)), __fsub_rn(nd.sum_h, exact_cell(total.h, inv_sh))};
@@ -225,7 +230,7 @@ __device__ __forceinline__ float exact_terms(float pg, float ph, const ExCand &c
 // SplitPoint of the best candidate and TreeBuilder::update_tree (exact_tree_builder.cu:262-296, :137-151 for the split
 // value; tree_builder.cu:9-60) of node n of the level.
 template <typename T>
-__device__ __forceinline__ void exact_apply(const ExSearch<T> &x, int level, int n, unsigned long long b, TreeNode *nodes, double inv_sg, double inv_sh,
+__device__ __forceinline__ void exact_apply(const ExSearch<T> &x, int level, int n, unsigned long long b, TreeNode *nodes, const GridScale &inv_sg, const GridScale &inv_sh,
                                             float mcw, float lam, float rt_eps, int per) {
     const int off = (1 << level) - 1;
     TreeNode &nd = nodes[off + n];
@@ -264,10 +269,11 @@ __device__ __forceinline__ void exact_apply(const ExSearch<T> &x, int level, int
 // the largest |gain| and among equals the smallest sorted position (exact_tree_builder.cu:218-258: smaller partition
 // id, i.e. smaller column, then larger value).  Per block the keys meet in shared memory (one slot per node of the
 // level), warps whose lanes all sit in one node reduce first.
+// What is the same for a group's candidates is worked out when a thread meets the group.
 // Two exact divisions per direction are what a candidate costs: one that cannot reach its block's best so far is left out
 // by a bound with fast divisions, whose margin (1e-5) is far above their error.
 template <typename T>
-static __global__ void __launch_bounds__(EX_THREADS)
+static __global__ void __launch_bounds__(EX_THREADS, EX_SEARCH_BLOCKS)
 k_exact_gain(const int *live, const ExSearch<T> x, int level, TreeNode *nodes, const QuantInfo *q, float mcw, float lam, float rt_eps,
              const unsigned char *__restrict__ ignored_all, const RoundState *rs, int F,
              unsigned long long *best, int *any_split, int *ticket) {
@@ -278,13 +284,13 @@ k_exact_gain(const int *live, const ExSearch<T> x, int level, TreeNode *nodes, c
     for (int n = threadIdx.x; n < nl; n += EX_THREADS) ex_best[n] = 0;
     __syncthreads();
     const unsigned char *ignored = ignored_all ? ignored_all + (size_t)rs->round * F : nullptr;
-    const double inv_sg = cell_inv<T>(q, 0), inv_sh = cell_inv<T>(q, 1);
+    const GridScale inv_sg(cell_inv<T>(q, 0)), inv_sh(cell_inv<T>(q, 1));
     const unsigned n_live = (unsigned)*live;
     const int tiles = (int)((n_live + EX_TILE - 1) / EX_TILE), per = exact_run(tiles);
     unsigned cur = 0xffffffffu;      // group the values below belong to
     unsigned end = 0;
-    ExPair<W> base{0, 0}, total{0, 0};
-    float pg = 0.f, ph = 0.f, parent = 0.f;
+    ExPair<W> base{0, 0};
+    float pg = 0.f, ph = 0.f, parent = 0.f, mg = 0.f, mh = 0.f;
     bool skipped = false;
     for (int t = blockIdx.x * per, t_end = min(tiles, t + per); t < t_end; ++t) {   // (neighbouring tiles: the threads seldom change the group)
         const unsigned i0 = (unsigned)t * EX_TILE + threadIdx.x * EX_ITEMS;
@@ -309,8 +315,9 @@ k_exact_gain(const int *live, const ExSearch<T> x, int level, TreeNode *nodes, c
                 const int2 range = x.group[cur];
                 end = (unsigned)range.y;
                 base = exact_before(x, (unsigned)range.x, per);
-                total = exact_before(x, end, per) - base;
+                const ExPair<W> total = exact_before(x, end, per) - base;
                 pg = nodes[off + n].sum_g; ph = nodes[off + n].sum_h;
+                mg = __fsub_rn(pg, exact_cell(total.g, inv_sg)); mh = __fsub_rn(ph, exact_cell(total.h, inv_sh));
                 parent = __fdiv_rn(__fmul_rn(pg, pg), __fadd_rn(ph, lam));
                 skipped = ignored && ignored[cur >> level];
             }
@@ -321,7 +328,7 @@ k_exact_gain(const int *live, const ExSearch<T> x, int level, TreeNode *nodes, c
                 const float bar = __uint_as_float((unsigned)(*(volatile unsigned long long *)&ex_best[n] >> 32));
                 ExCand c;
                 c.rg = exact_cell(right.g, inv_sg); c.rh = exact_cell(right.h, inv_sh);
-                c.mg = __fsub_rn(pg, exact_cell(total.g, inv_sg)); c.mh = __fsub_rn(ph, exact_cell(total.h, inv_sh));
+                c.mg = mg; c.mh = mh;
                 if (bar > 0.f && exact_terms(pg, ph, c, lam) * 1.00001f < (bar + parent) * 0.99999f) continue;
                 gn = exact_gain(parent, pg, ph, c, mcw, lam);
             }
@@ -396,7 +403,7 @@ static __global__ void k_exact_move_missing(int *nid, int n_rows, int level, con
 
 // lr[i] = entries of the tile up to and with i that go left (low half) and right (high half); tile_lr, run_lr: those before
 // tile t in its run, and before the run
-static __global__ void __launch_bounds__(EX_THREADS)
+static __global__ void __launch_bounds__(EX_THREADS, EX_MOVE_BLOCKS)
 k_exact_sides(const int *live, const int *row, const uint2 *side, unsigned *lr,
               ExPair<int> *tile_lr, ExPair<int> *run_cnt, ExPair<int> *run_lr, int *next_live, int *ticket) {
     chain_wait();
@@ -435,7 +442,7 @@ k_exact_sides(const int *live, const int *row, const uint2 *side, unsigned *lr,
 // Entry i of group [b, e) goes to (entries kept before b) + (lefts of the group before it), or behind all lefts of the group.
 // Neighbouring lanes hold neighbouring entries, so that either side's stores run on.
 template <typename In>
-static __global__ void __launch_bounds__(EX_THREADS)
+static __global__ void __launch_bounds__(EX_THREADS, EX_MOVE_BLOCKS)
 k_exact_scatter(const int *live, const unsigned *key, const int *row, const float *val, const In *gh, const unsigned *lr, const ExPair<int> *tile_lr,
                 const ExPair<int> *run_lr, const int2 *group, unsigned *key_out, int *row_out, float *val_out, In *gh_out) {
     chain_wait();
