@@ -66,9 +66,9 @@ WORKLOADS = {
            dict(objective='rank:ndcg', depth=8, max_num_bin=255, learning_rate=0.1, **COMMON),
            'mslr-shape 2.27M x 136 f32 in query groups of Poisson(120), rank:ndcg, depth 8, 255 bins, lr 0.1'),
 }
-# dram__bytes_read.sum + dram__bytes_write.sum per launch (mean over a tree) of the histogram kernel of either mode on config 2, from the
-# ncu captures summarised under profiles/ (None: no capture of that kernel yet)
-NCU_TRAFFIC_BYTES_PER_LAUNCH = {'exact': 356.1e6, 'fp32': 350.3e6}
+# dram__bytes_read.sum + dram__bytes_write.sum per launch (mean over a tree) of the histogram kernel of either mode on config 2: ncu at
+# 5 M rows (194 MB, profiles/k_assign_and_apply_higgs_5M_x28.md) times 2.1 (None: no capture of that kernel yet)
+NCU_TRAFFIC_BYTES_PER_LAUNCH = {'exact': 407e6, 'fp32': 407e6}
 
 
 def hist_limiter(mode, csr, pairs_per_s):
@@ -437,7 +437,7 @@ def main():
         kernel = {'fp32': 'k_hist (shared-memory integer sums of the float gradients on a 2^-30 grid; all levels)',
                   'exact': 'k_hist (shared-memory integer histograms; all levels)'}[mode]
         if info.csr_layout:
-            kernel = kernel.replace('k_hist', 'k_hist_sparse')
+            kernel = kernel.replace('k_hist', 'k_hist_columns, k_hist_sparse')
         roof = {'bound': 'hbm', 'kernel': kernel, 'achieved': hist_gbs, 'peak': peak, 'unit': 'GB/s', 'frac': hist_gbs / peak,
                 'peak_kind': peak_kind, 'traffic': NCU_TRAFFIC_BYTES_PER_LAUNCH[mode] if args.config == 'c2' and n_rows == rows_default and world == 1 else None,
                 'launches': int(prof.hist_launches), 'avg_launch_us': prof.hist_ms * 1e3 / max(1, prof.hist_launches),

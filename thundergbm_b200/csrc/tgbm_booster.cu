@@ -382,14 +382,18 @@ void BoosterImpl::sort_columns() {
     TGBM_CUDA(cudaMemcpyAsync(&h_twice, twice.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
     TGBM_CUDA(cudaStreamSynchronize(stream));
     if (h_twice) return;
-    rows.alloc(nnz); col_row.alloc(nnz); col_bin.alloc(nnz); col_ptr.alloc(B + 1);
-    k_value_rows<<<grid, 256, 0, stream>>>(sp_row_ptr.p, N, rows.p);
     int end_bit = 1;
     while ((1ll << end_bit) < B) ++end_bit;
     size_t tb = 0;
     TGBM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, sp_bin.p, col_bin.p, rows.p, col_row.p, (long long)nnz, 0, end_bit, stream));
     DevBuf<unsigned char> tmp;
-    tmp.alloc(std::max<size_t>(tb, 1));
+    try {
+        rows.alloc(nnz); col_row.alloc(nnz); col_bin.alloc(nnz); tmp.alloc(std::max<size_t>(tb, 1)); col_ptr.alloc(B + 1);
+    } catch (const Error &) {   // no room for them: the kernels search the rows
+        col_row.release(); col_bin.release(); col_ptr.release();
+        return;
+    }
+    k_value_rows<<<grid, 256, 0, stream>>>(sp_row_ptr.p, N, rows.p);
     TGBM_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, sp_bin.p, col_bin.p, rows.p, col_row.p, (long long)nnz, 0, end_bit, stream));
     k_bin_starts<<<std::min(ceil_div(B + 1, 256), num_sms * 8), 256, 0, stream>>>(col_bin.p, (int)nnz, B, col_ptr.p);
     TGBM_CUDA(cudaStreamSynchronize(stream));
@@ -1239,7 +1243,7 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
     last_float = float_sums;
     last_tree_full = (size_t)(n_trees - 1) * bufs.full_stride;
     Batch b = bufs;
-    // float rounds: the records carry the float gradient pairs themselves (same 8 bytes)
+    // float rounds: the float gradient pairs themselves (same 8 bytes)
     b.gh = float_sums ? reinterpret_cast<const int2 *>(gh.p + (size_t)k0 * N) : ghq.p + (size_t)k0 * N;
     const bool one_launch = small.cluster > 0 && !float_sums && !profile_on;
     if (one_launch) launch_small_trees(k0, n_trees);

@@ -117,7 +117,7 @@ __device__ __forceinline__ int hist_items(int level, const Batch &b, size_t tree
 // tile t belongs to share v0 + t mod k.  CTA c owns its consecutive shares and visits, item by item, the tiles
 // of its shares in ascending order: every CTA walks each of its (one or two, rarely more) lists once, front to back,
 // and since all CTAs carry about the same number of tiles, all lists are walked at the same relative pace.  Row ids
-// ascend inside every list, so at any time the whole GPU gathers rows from one moving window of the bin matrix:
+// ascend inside every list (to the chunks of k_assign), so at any time the whole GPU gathers rows from one moving window of the bin matrix:
 // DRAM pages and 64-byte sectors get shared between nodes.  A pure gather of 5.2 M of 10.5 M rows in 8 to 64 lists
 // takes 72 us this way and 100 to 110 us list after list.
 __device__ __forceinline__ void hist_share(const int *s_base, int w, int total, int n_shares, int &v0, int &k) {
