@@ -261,3 +261,21 @@ def test_bins(gpu, n, f, holes):
             want[:, j] = np.where(keep[:, j], np.minimum(np.searchsorted(c, x[:, j], 'right'), len(c) - 1), 255)
     assert np.array_equal(got, want)
     b.close()
+
+
+# query groups of one document to more than a block's threads, at the sizes where the sort changes its exchanges; groups of one
+# label, and of one document among others of another label (all of them draw it)
+@pytest.mark.parametrize('sizes', [[1, 2, 3, 31, 32, 33], [64, 65, 127, 128, 129, 1], [255, 256, 257, 40], [600, 5, 1025], [50] * 40])
+@pytest.mark.parametrize('objective', ['rank:ndcg', 'rank:pairwise'])
+def test_query_groups(gpu, orc, sizes, objective):
+    n, r = sum(sizes), np.random.default_rng(len(sizes))
+    x = r.integers(1, 20, (n, 6)).astype(np.float32)
+    y = np.minimum(r.poisson(x[:, 0] / 10), 4)
+    end = np.cumsum(sizes)
+    y[end[-1] - sizes[-1]:] = 1              # the last group: one label ...
+    if sizes[-1] > 1:
+        y[-1] = 2                            # ... but for one document
+    y[end[1] - sizes[1]:end[1]] = 3
+    d = _csr(x, y)
+    d.group = np.array(sizes, np.int32)
+    _same_as_oracle(orc, d, depth=4, n_trees=4, max_num_bin=32, learning_rate=0.3, objective=objective, min_child_weight=0.0)

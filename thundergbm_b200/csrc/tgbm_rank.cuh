@@ -15,6 +15,7 @@
 namespace tgbm {
 
 constexpr int RANK_MAX_GROUP = 4096;
+constexpr int RANK_FEW = 32;   // partners that a document looks through once per partner
 
 __device__ inline uint32_t desc_key(float v) {  // larger float -> smaller key
     uint32_t u = __float_as_uint(v);
@@ -43,6 +44,43 @@ __device__ inline void block_bitonic(unsigned long long *key, int *idx, int n, i
             __syncthreads();
         }
     }
+}
+
+// The same with an element per thread where P is at most the block's threads (thread i has put element i down): partners of a warp
+// exchange by shuffles, so 120 documents take 3 exchanges through shared memory instead of 28 with a barrier each.  Bound by its
+// instructions: warps without elements take part in the barriers only.  PACKED: the low half of a key is its idx.
+template <bool PACKED>
+__device__ inline void block_sort(unsigned long long *key, int *idx, int n, int P) {
+    if (P > (int)blockDim.x) {
+        __syncthreads();
+        block_bitonic(key, idx, n, P);
+        return;
+    }
+    const int i = threadIdx.x;
+    unsigned long long a = i < n ? key[i] : ~0ull;
+    int ia = !PACKED && i < n ? idx[i] : 0x7fffffff;
+    const bool some = (i & ~31) < P;
+    for (int k = 2; k <= P; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            unsigned long long b = a;
+            int ib = ia;
+            if (j < 32) {
+                if (!some) continue;
+                b = __shfl_xor_sync(0xffffffffu, a, j);
+                if (!PACKED) ib = __shfl_xor_sync(0xffffffffu, ia, j);
+            } else {
+                __syncthreads();
+                if (i < P) { key[i] = a; if (!PACKED) idx[i] = ia; }
+                __syncthreads();
+                if (i < P) { b = key[i ^ j]; if (!PACKED) ib = idx[i ^ j]; }
+            }
+            const bool larger = a > b || (a == b && ia > ib), keep_small = ((i & j) == 0) == ((i & k) == 0);
+            if (larger == keep_small) { a = b; ia = ib; }
+        }
+    }
+    __syncthreads();
+    if (i < P) { key[i] = a; idx[i] = PACKED ? (int)(unsigned)a : ia; }
+    __syncthreads();
 }
 
 __device__ inline float disc_gain(int label, int rank, const float *__restrict__ log2tab) {
@@ -74,9 +112,10 @@ k_lambdarank(const int *__restrict__ gptr, const float *__restrict__ y, const fl
         key[i] = ((unsigned long long)desc_key(y[s0 + i]) << 32) | desc_key(yp[s0 + i]);
         idx[i] = i;
     }
-    __syncthreads();
-    block_bitonic(key, idx, len, P);
-    for (int i = threadIdx.x; i < len; i += blockDim.x) { lab[i] = y[s0 + idx[i]]; sc[i] = yp[s0 + idx[i]]; }
+    block_sort<false>(key, idx, len, P);
+    // (the keys have served)
+    int *head = reinterpret_cast<int *>(key), *next = head + P;   // positions that drew a document as partner, in no order
+    for (int i = threadIdx.x; i < len; i += blockDim.x) { lab[i] = y[s0 + idx[i]]; sc[i] = yp[s0 + idx[i]]; head[i] = -1; }
     __syncthreads();
     const float id = ndcg ? idcg[k] : 1.f;
     for (int l = threadIdx.x; l < len; l += blockDim.x) {
@@ -107,26 +146,41 @@ k_lambdarank(const int *__restrict__ gptr, const float *__restrict__ y, const fl
             const float adz = fabsf(dz);
             const float rho = __fdiv_rn(1.0f, __fadd_rn(1.0f, portable_expf(__fsub_rn(sc[high], sc[low]))));
             hi[l] = high; lo[l] = low;
+            const int partner = m < nleft ? high : low;
+            next[l] = atomicExch(&head[partner], l);
             lam[l] = -__fmul_rn(adz, rho);
             hes[l] = __fmul_rn(2.0f, fmaxf(__fmul_rn(__fmul_rn(adz, rho), __fsub_rn(1.0f, rho)), 1e-16f));
         }
     }
     __syncthreads();
-    // every document sums what it receives in ascending l, the order of the reference's sequential loop
+    // every document sums what it receives in ascending l, the order of the reference's sequential loop: from its own draw and from
+    // the few that drew it (looking for them among all positions of a group is quadratic)
     float mg = 0.f, mh = 0.f;
     for (int t = threadIdx.x; t < len; t += blockDim.x) {
         float g = 0.f, h = 0.f;
-        for (int l = 0; l < len; ++l) {
-            if (hi[l] == t) { g = __fadd_rn(g, lam[l]); h = __fadd_rn(h, hes[l]); }
-            else if (lo[l] == t) { g = __fadd_rn(g, -lam[l]); h = __fadd_rn(h, hes[l]); }
+        auto receive = [&](int l) {
+            g = __fadd_rn(g, hi[l] == t ? lam[l] : -lam[l]);
+            h = __fadd_rn(h, hes[l]);
+        };
+        const bool own = hi[t] >= 0;
+        int n = 0;
+        for (int l = head[t]; l >= 0 && n <= RANK_FEW; l = next[l]) ++n;
+        if (n > RANK_FEW) {   // one of few documents with another label
+            for (int l = 0; l < len; ++l)
+                if (hi[l] == t || lo[l] == t) receive(l);
+        } else {
+            for (int q = 0, last = -1; q < n + (own ? 1 : 0); ++q) {
+                int first = own && t > last ? t : 0x7fffffff;
+                for (int l = head[t]; l >= 0; l = next[l])
+                    if (l > last && l < first) first = l;
+                receive(first);
+                last = first;
+            }
         }
         gh[s0 + idx[t]] = make_float2(g, h);
         mg = fmaxf(mg, fabsf(g)); mh = fmaxf(mh, h);
     }
-    unsigned ua = __float_as_uint(mg), ub = __float_as_uint(mh);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) { ua = max(ua, __shfl_xor_sync(0xffffffffu, ua, o)); ub = max(ub, __shfl_xor_sync(0xffffffffu, ub, o)); }
-    if ((threadIdx.x & 31) == 0) { atomicMax(maxbits, ua); atomicMax(maxbits + 1, ub); }
+    track_max(mg, mh, maxbits);
 }
 
 // NDCG / MAP of one query group per CTA (src/thundergbm/metric/rank_metric.cpp:42-100):
@@ -143,9 +197,8 @@ k_rank_metric(const int *__restrict__ gptr, const float *__restrict__ y, const f
     unsigned long long *key = reinterpret_cast<unsigned long long *>(sm);
     int *idx = reinterpret_cast<int *>(key + P);
     if (ndcg && idcg[k] == 0.f) { if (threadIdx.x == 0) group_score[k] = 1.f; return; }
-    for (int i = threadIdx.x; i < len; i += blockDim.x) { key[i] = desc_key(yp[s0 + i]); idx[i] = i; }
-    __syncthreads();
-    block_bitonic(key, idx, len, P);
+    for (int i = threadIdx.x; i < len; i += blockDim.x) { key[i] = ((unsigned long long)desc_key(yp[s0 + i]) << 32) | (unsigned)i; idx[i] = i; }
+    block_sort<true>(key, idx, len, P);
     // the terms by all threads (a chain of dependent global reads in one thread took 60 us for 120 documents), added in rank
     // order by one
     float *term = reinterpret_cast<float *>(key);
@@ -237,9 +290,9 @@ struct RankState {
                 }
             });
         }
-        // one thread per document of an ordinary group: with 256 for groups of 120 half of them wait at every barrier of the sort
-        threads = 64;
-        while (threads < 256 && (long long)threads * n_group < n_rows) threads *= 2;
+        // one thread per document, so that the sort exchanges by shuffles (300 k rows in groups of about 120: gradients 63 -> 36 us a
+        // round, metric 30 -> 21)
+        threads = std::max(64, std::min(256, pow2_len()));
         gptr.alloc(n_group + 1); idcg.alloc(hid.size()); log2tab.alloc(ltab.size()); y.alloc(std::max(n_rows, 1));
         group_score.alloc(std::max(n_group, 1)); sum.alloc(1);
         TGBM_CUDA(cudaMemcpyAsync(gptr.p, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice, stream));
