@@ -279,3 +279,33 @@ def test_query_groups(gpu, orc, sizes, objective):
     d = _csr(x, y)
     d.group = np.array(sizes, np.int32)
     _same_as_oracle(orc, d, depth=4, n_trees=4, max_num_bin=32, learning_rate=0.3, objective=objective, min_child_weight=0.0)
+
+
+# a row that stores a column twice: the last value counts, whether a thread walks the row or the lanes of a warp share it.  Columns
+# that ascend but for the repeats, in any order, and repeats a window of lanes or more apart
+@pytest.mark.parametrize('n,f,per', [(3000, 40, 30), (16_384, 40, 30), (16_385, 218, 70), (17_000, 3, 100)])
+@pytest.mark.parametrize('order', ['sorted', 'any', 'apart'])
+def test_columns_stored_twice(gpu, n, f, per, order):
+    from thundergbm_b200.booster import Booster
+    r = np.random.default_rng(n + f)
+    col = r.integers(0, f, (n, per))
+    if order != 'any':
+        col.sort(1)
+        col[::2] = np.arange(per) * f // per     # (every other row: no repeats where it has no more values than there are columns)
+    if order == 'apart':
+        col[:, -1] = col[:, 0]
+        col[1::3, per // 2] = col[1::3, 0]
+    x = r.integers(1, 200, (n, per)).astype(np.float32)
+    d = CsrData(n, f, (np.arange(n + 1) * per).astype(np.int32), col.astype(np.int32).ravel(), x.ravel(), r.random(n).astype(np.float32))
+    b = Booster(d, depth=2, n_trees=1, objective='reg:linear', tree_method='hist')
+    cut, ptr = b.cuts()
+    got = b.bins()
+    b.close()
+    want = np.full(got.shape, 255, np.uint8)
+    row = np.arange(n)
+    for k in range(per):     # one value after the other
+        c = col[:, k]
+        for j in np.unique(c):
+            at, cuts = row[c == j], cut[ptr[j]:ptr[j + 1]]
+            want[at, j] = np.minimum(np.searchsorted(cuts, x[at, k], 'right'), len(cuts) - 1)
+    assert np.array_equal(got, want)

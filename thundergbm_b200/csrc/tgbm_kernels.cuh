@@ -17,6 +17,8 @@
 // All sums on the fixed-point grid are integer sums, so they do not depend on the order of
 // the atomics, on the CTA count or on the number of ranks.
 #pragma once
+#include <climits>
+
 #include "tgbm_device.cuh"
 
 namespace tgbm {
@@ -272,7 +274,9 @@ k_bin_full(const float *__restrict__ val, int n_rows, int F, const int *__restri
         to[1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
 }
-// CSR rows: a warp per row, lanes over its values, row-major only (k_bins_by_column follows); `bins` comes filled with 255
+// CSR rows: a warp per row, lanes over its values, row-major only (k_bins_by_column follows); `bins` comes filled with 255.
+// Of a column that a row stores twice the last value counts, as above.  While the row's columns ascend no two lanes meet; from
+// the first window on where they do not, windows are stored one after the other, and of lanes with the same column the last stores.
 constexpr int BIN_ROWS_SMEM = 220 * 1024;
 static __global__ void __launch_bounds__(1024, 1)
 k_bin_rows(const int *__restrict__ row_ptr, const int *__restrict__ col, const float *__restrict__ val, int n_rows, int F, const int *__restrict__ cut_ptr,
@@ -286,18 +290,32 @@ k_bin_rows(const int *__restrict__ row_ptr, const int *__restrict__ col, const f
     constexpr int U = 2;   // values in flight per lane
     for (int r = blockIdx.x * 32 + (threadIdx.x >> 5); r < n_rows; r += gridDim.x * 32) {
         const int j1 = row_ptr[r + 1];
-        for (int j0 = row_ptr[r] + lane; j0 < j1; j0 += 32 * U) {
+        int last = -1;   // column before the window
+        bool ascend = true;
+        for (int j0 = row_ptr[r]; j0 < j1; j0 += 32 * U) {   // (the same in the whole warp)
             int c[U];
             float v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int j = j0 + 32 * u;
-                c[u] = j < j1 ? col[j] : -1;
+                const int j = j0 + 32 * u + lane;
+                c[u] = j < j1 ? col[j] : INT_MAX;
                 v[u] = j < j1 ? val[j] : 0.f;
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (c[u] >= 0) bins[(size_t)r * Fpad + c[u]] = (unsigned char)bin_of(bin_sm + c[u] * BIN_TREE, cuts[c[u]], v[u]);
+            for (int u = 0; u < U; ++u) {
+                const bool stored = c[u] != INT_MAX;
+                const int left = __shfl_up_sync(0xffffffffu, c[u], 1);
+                ascend = ascend && __all_sync(0xffffffffu, !stored || c[u] > (lane ? left : last));
+                last = __shfl_sync(0xffffffffu, c[u], 31);
+                const unsigned char b = stored ? (unsigned char)bin_of(bin_sm + c[u] * BIN_TREE, cuts[c[u]], v[u]) : (unsigned char)0;
+                bool mine = stored;
+                if (!ascend) {
+                    const unsigned same = __match_any_sync(0xffffffffu, c[u]);
+                    mine = mine && same >> lane == 1u;
+                    __syncwarp();   // what earlier windows stored comes before
+                }
+                if (mine) bins[(size_t)r * Fpad + c[u]] = b;
+            }
         }
     }
 }
