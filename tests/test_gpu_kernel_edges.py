@@ -309,3 +309,38 @@ def test_columns_stored_twice(gpu, n, f, per, order):
             at, cuts = row[c == j], cut[ptr[j]:ptr[j + 1]]
             want[at, j] = np.minimum(np.searchsorted(cuts, x[at, k], 'right'), len(cuts) - 1)
     assert np.array_equal(got, want)
+
+
+# shared memory that the kernels may ask for grows with the depth and, for ranking, with the longest query group: it is allowed to a
+# kernel, not to a booster, so a booster made in between must not take away what another one needs
+@pytest.mark.parametrize('layout,n,deep,shallow', [('dense', 33_000, 9, 2), ('dense', 33_000, 14, 12), ('dense', 33_000, 11, 10), ('sparse', 3000, 9, 2)])
+def test_boosters_of_different_depths_side_by_side(gpu, orc, monkeypatch, layout, n, deep, shallow):
+    from thundergbm_b200.booster import Booster
+    monkeypatch.setenv('TGBM_LAYOUT', layout)
+    d = _data(n, 4, 1, deep)
+    for mode in ('exact', 'fp32'):
+        p = [dict(depth=x, n_trees=2, max_num_bin=64, learning_rate=0.5, objective='reg:linear') for x in (deep, shallow)]
+        b = [Booster(d, hist_mode=mode, **q) for q in p]
+        for x, q in zip(b, p):
+            x.boost(2)
+            if mode == 'exact':
+                o = orc.train(d, hist_mode=1, keep_nid=0, **q)
+                assert x.trees().tobytes() == o.trees.tobytes() and np.array_equal(x.ypred(), o.ypred)
+            assert x.info.rounds_done == 2 and np.isfinite(x.metrics()).all()
+            x.close()
+
+
+def test_rankings_of_different_group_sizes_side_by_side(gpu, orc):
+    from thundergbm_b200.booster import Booster
+    r = np.random.default_rng(4)
+    p = dict(depth=3, n_trees=2, max_num_bin=32, learning_rate=0.5, objective='rank:ndcg')
+    data = []
+    for longest in (4096, 1300):
+        d = _csr(r.integers(1, 20, (longest + 9, 3)), r.integers(0, 4, longest + 9))
+        d.group = np.array([9, longest], np.int32)
+        data.append(d)
+    b = [Booster(d, hist_mode='exact', **p) for d in data]
+    for x, d in zip(b, data):
+        x.boost(2)
+        assert x.trees().tobytes() == orc.train(d, hist_mode=1, keep_nid=0, **p).trees.tobytes()
+        x.close()

@@ -179,6 +179,7 @@ struct BoosterImpl {
 };
 
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+constexpr size_t PRUNE_SMEM = 200 * 1024;   // node tables that k_prune holds in shared memory
 // shared memory of k_assign at a level: rules, counts, offsets (up to depth 13: 32 bytes per node), staged rows
 static inline size_t assign_smem(int level, int rpt) {
     const size_t nl = (size_t)1 << level;
@@ -697,7 +698,7 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
             auto kern = F % 4 == 0 ? k_bin_full<true> : k_bin_full<false>;
             kern<<<dim3(std::min(ceil_div(N, 256), num_sms * 4), Fpad / 32), 256, 0, stream>>>(in.val.p, N, F, cut_ptr.p, cut_val.p, Fpad, Npad, bins.p, binsT.p);
         } else if (N && !colb && !in.full_cols && tree_smem <= BIN_ROWS_SMEM && N >= BIN_ROWS_FROM && nnz >= BIN_ROWS_VALUES * (size_t)N) {
-            TGBM_CUDA(cudaFuncSetAttribute(k_bin_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, BIN_ROWS_SMEM));
+            allow_shared(k_bin_rows, BIN_ROWS_SMEM);
             TGBM_CUDA(cudaMemsetAsync(bins.p, MISSING_BIN, bins.bytes(), stream));
             k_bin_rows<<<std::min(ceil_div(N, 32), num_sms), 1024, tree_smem, stream>>>(in.row_ptr.p, in.col.p, in.val.p, N, F, cut_ptr.p, cut_val.p, Fpad, bins.p);
             k_bins_by_column<<<dim3((unsigned)(Npad / 128), Fpad / 32), 256, 0, stream>>>(bins.p, N, F, Fpad, Npad, binsT.p);
@@ -769,8 +770,8 @@ void BoosterImpl::init_exact() {
     ex_any.zero(stream);
     ex_ticket.alloc(1);
     ex_ticket.zero(stream);
-    TGBM_CUDA(cudaFuncSetAttribute(k_exact_gain<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-    TGBM_CUDA(cudaFuncSetAttribute(k_exact_gain<long long>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+    allow_shared(k_exact_gain<float>, 64 * 1024);
+    allow_shared(k_exact_gain<long long>, 64 * 1024);
     TGBM_CUDA(cudaStreamSynchronize(stream));
     TGBM_CUDA(cudaGetLastError());
 }
@@ -842,7 +843,7 @@ void Booster::init(const DataSet &ds) {
     GBMParam &p = m.p;
     m.objective = objective_from_name(p.objective);
     TGBM_CHECK(m.objective != OBJ_UNKNOWN, "undefined objective " + p.objective);
-    TGBM_CHECK(p.depth >= 1 && p.depth <= 14, "depth must be in [1, 14]");
+    TGBM_CHECK(p.depth >= 1 && p.depth <= MAX_DEPTH, "depth must be in [1, " + std::to_string(MAX_DEPTH) + "]");
     TGBM_CHECK(p.max_num_bin >= 1 && p.max_num_bin <= 255, "max_num_bin must be in [1, 255] (bin ids are bytes, 255 marks a missing value)");
     TGBM_CHECK(p.quant_bits >= 8 && p.quant_bits <= 20, "quant_bits must be in [8, 20]");
     TGBM_CHECK(p.hist_mode == 0 || p.hist_mode == 1, "hist_mode must be 0 (fp32) or 1 (exact)");
@@ -1071,21 +1072,20 @@ void Booster::init(const DataSet &ds) {
     m.metric_partial.alloc(m.metric_blocks()); m.metric_sum.alloc(1);
     m.window_rows = (1 << (31 - p.quant_bits)) - HIST_THREADS;
     TGBM_CHECK(m.window_rows >= HIST_THREADS, "quant_bits too large for the int32 accumulation window");
-    const int table = 4 * (max_pairs + 1);   // tiles before every pair of the deepest level
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_EXACT_SMEM + table));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_EXACT_SMEM + table));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_FINE_SMEM + table));
-    const size_t assign_most = assign_smem(std::max(0, depth - 2), m.assign_rpt);
-    if (assign_most > 48 * 1024) {
-        TGBM_CUDA(cudaFuncSetAttribute(m.assign_kernel(depth - 2, false), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)assign_most));
-        TGBM_CUDA(cudaFuncSetAttribute(m.assign_kernel(depth - 2, true), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)assign_most));
+    constexpr size_t table = 4 * ((1 << (MAX_DEPTH - 2)) + 1);   // tiles before every pair of the deepest level
+    allow_shared(k_hist<true, false>, HIST_EXACT_SMEM + table);
+    allow_shared(k_hist<false, false>, HIST_EXACT_SMEM + table);
+    allow_shared(k_hist<true, true>, HIST_FINE_SMEM + table);
+    allow_shared(k_hist<false, true>, HIST_FINE_SMEM + table);
+    if (assign_smem(std::max(0, depth - 2), m.assign_rpt) > 48 * 1024) {   // (depth 12 and beyond: one kernel for all levels with many children)
+        allow_shared(m.assign_kernel(depth - 2, false), assign_smem(MAX_DEPTH - 2, ASSIGN_CHUNK / ASSIGN_THREADS));
+        allow_shared(m.assign_kernel(depth - 2, true), assign_smem(MAX_DEPTH - 2, ASSIGN_CHUNK / ASSIGN_THREADS));
     }
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
-    TGBM_CUDA(cudaFuncSetAttribute(k_hist_sparse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPARSE_SMEM_BINS * 16 + table));
-    m.prune_in_smem = sizeof(TreeNode) * (size_t)m.n_nodes <= 200 * 1024;  // up to depth 11
+    allow_shared(k_hist_sparse<true>, SPARSE_SMEM_BINS * 16 + table);
+    allow_shared(k_hist_sparse<false>, SPARSE_SMEM_BINS * 16 + table);
+    m.prune_in_smem = sizeof(TreeNode) * (size_t)m.n_nodes <= PRUNE_SMEM;  // up to depth 11
     if (m.prune_in_smem && sizeof(TreeNode) * (size_t)m.n_nodes > 40 * 1024)   // (the kernel has static shared memory beside it)
-        TGBM_CUDA(cudaFuncSetAttribute(k_prune, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(TreeNode) * (size_t)m.n_nodes)));
+        allow_shared(k_prune, PRUNE_SMEM);
     m.plan_small_trees();
     if (need_group_file(m.objective)) m.rank.init(ds, m.objective, m.N, m.stream, first_group, total_groups);
     });
@@ -1203,7 +1203,7 @@ void BoosterImpl::plan_small_trees() {
         pl.nodes_pass = (int)std::min<size_t>(max_nl, (budget - fixed) / per_node);
         if (max_nl > 8 * pl.nodes_pass) return;   // the rows would be walked over and over
         pl.smem = fixed + per_node * pl.nodes_pass;
-        TGBM_CUDA(cudaFuncSetAttribute(k_small_tree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+        allow_shared(k_small_tree, budget);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = pl.cluster; cfg.blockDim = SMALL_THREADS; cfg.dynamicSmemBytes = pl.smem;
         cudaLaunchAttribute attr;

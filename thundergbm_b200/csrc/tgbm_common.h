@@ -114,6 +114,8 @@ struct Error : std::runtime_error {
         if (!(cond)) throw ::tgbm::Error(std::string(msg) + " (" #cond ") at " __FILE__ ":" + std::to_string(__LINE__)); \
     } while (0)
 
+constexpr int MAX_DEPTH = 14;
+
 // host data set: CSR + labels (src/thundergbm/dataset.cpp)
 struct DataSet {
     int n_rows = 0;

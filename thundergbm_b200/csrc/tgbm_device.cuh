@@ -87,6 +87,14 @@ inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
     TGBM_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
+// Shared memory that a kernel may be launched with.  It is a setting of the kernel on the device, for every booster, model and
+// thread of the process, so all of them set it to the same number: `most`, a constant, the most that any launch of the kernel
+// takes.  (Set to what one booster needs, it would take from another one what that needs.)
+template <typename... P>
+inline void allow_shared(void (*kernel)(P...), size_t most) {
+    TGBM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+}
+
 // ---- portable expf ------------------------------------------------------------------------
 // Cody-Waite reduction and a degree-5 polynomial written with explicit IEEE fp32 operations
 // only, so that a host restatement of the same lines gives the same bits.  Replaces expf in

@@ -276,7 +276,7 @@ static bool launch_predict_tiles(const int *rp, const int *col, const float *val
         const int tiles = (N + PT_THREADS * rpt - 1) / (PT_THREADS * rpt);
         const int grid = std::max(1, std::min(tiles, num_sms));
         auto go = [&](auto kern) {
-            TGBM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            allow_shared(kern, budget);
             kern<<<grid, PT_THREADS, smem, st>>>(rp, col, val, N, F, model, n_rounds, K, n_nodes, depth, chunk, lr, base_score, out, partial.p);
         };
         if (rpt == 2) go(k_predict_tiles<DENSE_PATH, 2>);
@@ -1176,8 +1176,7 @@ void predict(const DataSet &ds, PredictPlan &plan, float learning_rate, float ba
         while (chunk < std::min(8, n_rounds) && rt_log > 0) { --rt_log; bytes = smem(); }
         if (chunk > 0) {
             auto kern = is_dense_path(F) ? k_predict_direct<true> : k_predict_direct<false>;
-            if (bytes > 48 * 1024)   // (a limit of the kernel on the current device)
-                TGBM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+            if (bytes > 48 * 1024) allow_shared(kern, budget);
             if (kernel_ms) TGBM_CUDA(cudaEventRecord(ev.e0, st));
             kern<<<(N + (1 << rt_log) - 1) >> rt_log, PD_THREADS, bytes, st>>>(kind, in, N, n_feat, plan.h.p, n_rounds, K, n_nodes, depth, rt_log,
                                                                               chunk, learning_rate, base_score, scores_dev);
@@ -1216,16 +1215,17 @@ void predict(const DataSet &ds, PredictPlan &plan, float learning_rate, float ba
         const bool dense_rows = rk->planes && rows.full_cols == F && F % 4 == 0;
         if (!dense_rows) rows.need_csr(N, st, num_sms);
         const int n_inner = (1 << depth) - 1, n_leaf = 1 << depth;
+        const size_t planes_budget = 224 * 1024, ranks_budget = 216 * 1024;
         size_t rk_smem;
         int chunk;
         if (rk->planes) {
             const size_t per_tree = sizeof(PlaneNode) * (size_t)n_inner + sizeof(float) * (size_t)n_leaf, row_bytes = sizeof(uint32_t) * 2 * PL_WORDS * PL_ROWS;
-            chunk = (int)std::min<size_t>((size_t)n_rounds, ((size_t)(224 * 1024) - row_bytes) / per_tree);
+            chunk = (int)std::min<size_t>((size_t)n_rounds, (planes_budget - row_bytes) / per_tree);
             TGBM_CHECK(chunk >= 1, "a tree of this depth does not fit beside a tile of rows");
             rk_smem = row_bytes + per_tree * chunk;
         } else {
             const size_t row_bytes = F <= 32 ? sizeof(uint32_t) * 9 * PR_ROWS : 0;
-            chunk = (int)std::min<size_t>((size_t)n_rounds, ((size_t)(216 * 1024) - row_bytes) / (sizeof(RNode) * (size_t)n_nodes));
+            chunk = (int)std::min<size_t>((size_t)n_rounds, (ranks_budget - row_bytes) / (sizeof(RNode) * (size_t)n_nodes));
             rk_smem = sizeof(RNode) * (size_t)n_nodes * chunk + row_bytes;
         }
         if (chunk < n_rounds) d_partial.alloc((size_t)N * K);
@@ -1262,14 +1262,14 @@ void predict(const DataSet &ds, PredictPlan &plan, float learning_rate, float ba
         }
         if (rk->planes) {
             auto go = [&](auto kern) {
-                TGBM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem));
+                allow_shared(kern, planes_budget);
                 kern<<<std::max(1, std::min((N + PL_ROWS - 1) / PL_ROWS, num_sms)), PL_THREADS, rk_smem, st>>>(
                     d_bins.p, Fpad, N, rk->d_pl_nodes.p, rk->d_leaves.p, n_rounds, K, depth, chunk, learning_rate, base_score, scores_dev, d_partial.p);
             };
             if (dense_path) go(k_predict_planes<true>); else go(k_predict_planes<false>);
         } else {
             auto go = [&](auto kern) {
-                TGBM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem));
+                allow_shared(kern, ranks_budget);
                 kern<<<std::max(1, std::min((N + PR_ROWS - 1) / PR_ROWS, num_sms)), PR_THREADS, rk_smem, st>>>(
                     d_bins.p, Fpad, F, N, rk->d_nodes.p, n_rounds, K, n_nodes, depth, chunk, learning_rate, base_score, scores_dev, d_partial.p);
             };
@@ -1300,8 +1300,8 @@ void predict(const DataSet &ds, PredictPlan &plan, float learning_rate, float ba
     if (kernel_ms) TGBM_CUDA(cudaEventRecord(ev.e0, st));
     if (dense_path) {
         k_predict_dense<<<(N + PRED_ROWS - 1) / PRED_ROWS, PRED_ROWS, smem, st>>>(rp, col, val, N, F, any, n_rounds, K, n_nodes, learning_rate, base_score, scores_dev);
-    } else if (smem <= 200 * 1024) {
-        TGBM_CUDA(cudaFuncSetAttribute(k_predict_csr_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    } else if (constexpr size_t most = 200 * 1024; smem <= most) {
+        allow_shared(k_predict_csr_staged, most);
         k_predict_csr_staged<<<(N + PRED_ROWS - 1) / PRED_ROWS, PRED_ROWS, smem, st>>>(rp, col, val, N, F, any, n_rounds, K, n_nodes, learning_rate, base_score, scores_dev);
     } else {
         k_predict_csr<<<(N + 127) / 128, 128, 0, st>>>(rp, col, val, N, any, n_rounds, K, n_nodes, learning_rate, base_score, scores_dev);

@@ -306,9 +306,7 @@ struct RankState {
         int P = 1;
         while (P < max_len) P <<= 1;
         const int smem = 40 * P;
-        if (smem > 48 * 1024) {
-            TGBM_CUDA(cudaFuncSetAttribute(k_lambdarank, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        }
+        if (smem > 48 * 1024) allow_shared(k_lambdarank, 40 * RANK_MAX_GROUP);
     }
     int pow2_len() const { int P = 1; while (P < max_len) P <<= 1; return P; }
 
