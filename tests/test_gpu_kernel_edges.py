@@ -311,6 +311,33 @@ def test_columns_stored_twice(gpu, n, f, per, order):
     assert np.array_equal(got, want)
 
 
+
+def _trained_in(d, spare, rounds, **p):
+    """Trees and scores of a training that finds `spare` bytes of free device memory (0: all there is)."""
+    import torch
+    from thundergbm_b200 import _lib
+    from thundergbm_b200.booster import Booster
+    _lib.lib().tgbm_release_device_memory()
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - spare, dtype=torch.uint8, device='cuda') if spare else None
+    b = Booster(d, n_trees=rounds, hist_mode='exact', objective='reg:linear', **p)
+    b.boost(rounds)
+    got = b.trees().tobytes(), b.ypred().tobytes()
+    b.close()
+    del filler
+    torch.cuda.empty_cache()
+    return got
+
+
+# the values by column (240 MB that stay, 360 more while they are sorted) only where the level buffers (1.6 GB) leave room for them
+def test_columns_of_the_csr_layout_in_little_memory(gpu):
+    r = np.random.default_rng(1)
+    n, per, f = 750_000, 40, 20_000
+    col = (np.arange(per) * (f // per) + r.integers(0, f // per, (n, per))).astype(np.int32)
+    d = CsrData(n, f, np.arange(0, n * per + 1, per, dtype=np.int32), col.ravel(), np.ones(n * per, np.float32), (col[:, 0] % 5 + r.random(n)).astype(np.float32))
+    assert _trained_in(d, 0, 12, depth=12) == _trained_in(d, 1850 << 20, 12, depth=12)
+
+
 # shared memory that the kernels may ask for grows with the depth and, for ranking, with the longest query group: it is allowed to a
 # kernel, not to a booster, so a booster made in between must not take away what another one needs
 @pytest.mark.parametrize('layout,n,deep,shallow', [('dense', 33_000, 9, 2), ('dense', 33_000, 14, 12), ('dense', 33_000, 11, 10), ('sparse', 3000, 9, 2)])
