@@ -55,7 +55,8 @@ def test_outliers_among_normal_labels(gpu, monkeypatch, n, layout):
     x[11:13, 0] = 9, 10
     stored[11:13, 1] = False
     depth = 3
-    trees, nid, scores = _rounds(_csr(x, stored, y), depth=depth, n_trees=7, max_num_bin=16, learning_rate=1.0, objective='reg:linear', gamma=0.0,
+    rounds = 12 if layout == 'sparse' else 7     # (from ten on the CSR layout has its values by column)
+    trees, nid, scores = _rounds(_csr(x, stored, y), depth=depth, n_trees=rounds, max_num_bin=16, learning_rate=1.0, objective='reg:linear', gamma=0.0,
                                  min_child_weight=2.0, **{'lambda': 3.0})
     for t in (5, 6):
         g = (scores[t] - y.astype(np.float32)).astype(np.float64)

@@ -168,10 +168,12 @@ def test_rows_to_children(gpu, orc, monkeypatch, n, f, depth, classes, layout):
     _same_as_oracle(orc, _data(n, f, classes, n), **p)
 
 
-# the CSR layout with its columns sorted: more bins than the shared ones (columns of one value, of a few, of runs that span
-# several warps), columns too long for the nodes that split on them, and rows that store a column twice (no sorted columns)
+# the CSR layout with its columns sorted (from ten trees on) and without: more bins than the shared ones (columns of one value,
+# of a few, of runs that span several warps), columns too long for the nodes that split on them, and rows that store a column twice
+# (no sorted columns)
 @pytest.mark.parametrize('n,f,depth,twice', [(700, 14_000, 4, False), (3000, 60, 5, False), (40_000, 130, 6, False), (2000, 60, 4, True)])
-def test_columns_of_the_csr_layout(gpu, orc, monkeypatch, n, f, depth, twice):
+@pytest.mark.parametrize('trees', [9, 10])
+def test_columns_of_the_csr_layout(gpu, orc, monkeypatch, n, f, depth, twice, trees):
     monkeypatch.setenv('TGBM_LAYOUT', 'sparse')
     r = np.random.default_rng(n)
     share = np.clip(1.5 / np.arange(1, f + 1) ** 0.6, 3 / n, 0.98)     # popular columns first, rare ones last
@@ -183,7 +185,7 @@ def test_columns_of_the_csr_layout(gpu, orc, monkeypatch, n, f, depth, twice):
     if twice:   # every row gets its first value once more, the same one: whichever counts, the row goes the same way
         at = d.row_ptr[:-1]
         d = CsrData(n, f, (d.row_ptr + np.arange(n + 1)).astype(np.int32), np.insert(d.col, at, d.col[at]), np.insert(d.val, at, d.val[at]), d.y)
-    _same_as_oracle(orc, d, depth=depth, n_trees=3, max_num_bin=255, learning_rate=0.5, objective='reg:linear', num_class=1, min_child_weight=0.5)
+    _same_as_oracle(orc, d, depth=depth, n_trees=trees, max_num_bin=255, learning_rate=0.5, objective='reg:linear', num_class=1, min_child_weight=0.5)
 
 
 # blocks of the split search that take one feature or four: features of 64, 65 and 1 bins, none at all, numbers of them that leave a

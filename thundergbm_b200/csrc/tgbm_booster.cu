@@ -304,6 +304,11 @@ constexpr int SORT_LANES = 4;   // columns sorted side by side
 // CSR rows binned by k_bin_rows: from so many rows on laying out the search trees of all columns pays, from so many values a row
 // a warp per row (300 k rows x 136: 1.3 ms with a thread per row, 0.2 so; 581 k rows x 12 values: 0.09 against 0.16)
 constexpr int BIN_ROWS_FROM = 16384, BIN_ROWS_VALUES = 24;
+// CSR layout: trees from which on sorting the values by column pays.  What it takes, ms, and saves per tree, us: 1 M rows x 30 of
+// 100 k columns of very different popularity 1.05 and 240, 100 k rows 0.19 and 30; columns alike, 40 values of 5 k columns in 200 k
+// rows 0.38 and 27, of 10 k in 20 k rows 0.14 and 46; 12 distinct values, 20 of 1 k columns in 500 k rows 0.29 and 27.  Even after 3 to
+// 16 trees, then; a training of ten is between 6 % faster and 2 % slower.
+constexpr int COLUMNS_TREES = 10;
 
 // streams that start after what `main` holds now; join() makes `main` wait for them
 struct SideStreams {
@@ -1094,7 +1099,7 @@ void Booster::init(const DataSet &ds) {
         allow_shared(k_prune, PRUNE_SMEM);
     m.plan_small_trees();
     if (need_group_file(m.objective)) m.rank.init(ds, m.objective, m.N, m.stream, first_group, total_groups);
-    if (m.sparse) m.sort_columns();
+    if (m.sparse && (long long)p.n_trees * K >= COLUMNS_TREES) m.sort_columns();
     });
     agree("allocating its training buffers");
     lap("training buffers");
