@@ -340,6 +340,18 @@ def test_columns_of_the_csr_layout_in_little_memory(gpu):
     assert _trained_in(d, 0, 12, depth=12) == _trained_in(d, 1850 << 20, 12, depth=12)
 
 
+# the bytes by slot (224 MB here) beside those by feature (twice 256 MB) only where there is room for them
+def test_columns_that_share_a_byte_in_little_memory(gpu):
+    r = np.random.default_rng(1)
+    n, f = 1_000_000, 256
+    a, b = r.integers(40, f, n), r.integers(40, f - 1, n)
+    b += b >= a
+    col = np.stack([r.integers(0, 40, n), np.minimum(a, b), np.maximum(a, b)], 1).astype(np.int32)   # forty exclude each other
+    d = CsrData(n, f, np.arange(0, 3 * n + 1, 3, dtype=np.int32), col.ravel(), r.integers(1, 4, 3 * n).astype(np.float32),
+                (col[:, 0] % 5 + r.random(n)).astype(np.float32))
+    assert _trained_in(d, 0, 2, depth=4) == _trained_in(d, 640 << 20, 2, depth=4)
+
+
 # shared memory that the kernels may ask for grows with the depth and, for ranking, with the longest query group: it is allowed to a
 # kernel, not to a booster, so a booster made in between must not take away what another one needs
 @pytest.mark.parametrize('layout,n,deep,shallow', [('dense', 33_000, 9, 2), ('dense', 33_000, 14, 12), ('dense', 33_000, 11, 10), ('sparse', 3000, 9, 2)])

@@ -338,7 +338,8 @@ struct SideStreams {
 };
 
 // Fewer bytes per row for the histogram kernels, which take 32 slots of a row at a time whatever they hold: used where whole
-// groups of 32 go.  (581 k rows x 54 columns, 44 of them two one-hot groups: 12 slots.)
+// groups of 32 go.  (581 k rows x 54 columns, 44 of them two one-hot groups: 12 slots.)  The matrix by feature stays where there is
+// no memory for another one beside it.
 void BoosterImpl::bundle_columns() {
     S = F; Spad = Fpad;
     h_slot_ptr = h_cut_ptr;
@@ -362,7 +363,12 @@ void BoosterImpl::bundle_columns() {
     ptr.push_back(B);
     DevBuf<int> d_slot, d_shift;
     DevBuf<unsigned char> packed;
-    d_slot.alloc(F); d_shift.alloc(F); slot_ptr.alloc(slots + 1); packed.alloc((size_t)N * pad);
+    try {
+        d_slot.alloc(F); d_shift.alloc(F); slot_ptr.alloc(slots + 1); packed.alloc((size_t)N * pad);
+    } catch (const Error &) {
+        slot_ptr.release();
+        return;
+    }
     TGBM_CUDA(cudaMemcpyAsync(d_slot.p, slot.data(), sizeof(int) * F, cudaMemcpyHostToDevice, stream));
     TGBM_CUDA(cudaMemcpyAsync(d_shift.p, shift.data(), sizeof(int) * F, cudaMemcpyHostToDevice, stream));
     TGBM_CUDA(cudaMemcpyAsync(slot_ptr.p, ptr.data(), sizeof(int) * ptr.size(), cudaMemcpyHostToDevice, stream));
