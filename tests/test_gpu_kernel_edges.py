@@ -283,6 +283,36 @@ def test_query_groups(gpu, orc, sizes, objective):
     _same_as_oracle(orc, d, depth=4, n_trees=4, max_num_bin=32, learning_rate=0.3, objective=objective, min_child_weight=0.0)
 
 
+# NaNs with the sign set are the first cut point of a column, and no value compares above them
+@pytest.mark.parametrize('n,f,holes', [(300, 33, 0), (17_000, 40, 0.2)])
+def test_bins_of_columns_with_nans(gpu, n, f, holes):
+    from thundergbm_b200.booster import Booster
+    r = np.random.default_rng(f)
+    nan = np.copysign(np.float32(np.nan), np.float32(-1))
+    x = r.integers(1, 4, (n, f)).astype(np.float32)
+    x[:, 0] = 1
+    x[::3, :3] = nan
+    x[:, 3] = nan
+    x[::3, 4] = np.nan
+    keep = r.random((n, f)) >= holes
+    d = _holes(x, r.random(n), keep) if holes else _csr(x, r.random(n))
+    b = Booster(d, depth=2, n_trees=1, objective='reg:linear', tree_method='hist')
+    cut, ptr = b.cuts()
+    got = b.bins()
+    b.close()
+    want = np.full(got.shape, 255, np.uint8)
+    for j in range(f):
+        c = cut[ptr[j]:ptr[j + 1]]
+        assert np.isnan(c[0]) == (j < 4)
+        lo, hi = np.zeros(n, int), np.full(n, len(c) - 1)
+        for _ in range(9):
+            mid = (lo + hi) // 2
+            up = c[mid] <= x[:, j]
+            lo, hi = np.where((lo < hi) & up, mid + 1, lo), np.where((lo < hi) & ~up, mid, hi)
+        want[:, j] = np.where(keep[:, j], lo, 255)
+    assert np.array_equal(got, want)
+
+
 # a row that stores a column twice: the last value counts, whether a thread walks the row or the lanes of a warp share it.  Columns
 # that ascend but for the repeats, in any order, and repeats a window of lanes or more apart
 @pytest.mark.parametrize('n,f,per', [(3000, 40, 30), (16_384, 40, 30), (16_385, 218, 70), (17_000, 3, 100)])

@@ -711,10 +711,14 @@ void BoosterImpl::find_cuts_and_bins(const DataSet &ds) {
         bins.alloc((size_t)N * Fpad);
         binsT.alloc((size_t)F * Npad + ASSIGN_CHUNK);   // (k_assign reads the first column to the end of a chunk)
         const size_t tree_smem = sizeof(float) * (size_t)F * (BIN_TREE + 1);
-        if (N && !colb && in.full_cols == F) {
+        // a cut point that is a NaN with its sign set comes first, and no value is above it: what a search finds then depends on the
+        // cut points that it looks at, so those of k_bin_dense decide
+        bool ordered = !colb;
+        for (int f = 0; f < F; ++f) ordered = ordered && !(h_cut_ptr[f] < h_cut_ptr[f + 1] && std::isnan(h_cut_val[h_cut_ptr[f]]));
+        if (N && ordered && in.full_cols == F) {
             auto kern = F % 4 == 0 ? k_bin_full<true> : k_bin_full<false>;
             kern<<<dim3(std::min(ceil_div(N, 256), num_sms * 4), Fpad / 32), 256, 0, stream>>>(in.val.p, N, F, cut_ptr.p, cut_val.p, Fpad, Npad, bins.p, binsT.p);
-        } else if (N && !colb && !in.full_cols && tree_smem <= BIN_ROWS_SMEM && N >= BIN_ROWS_FROM && nnz >= BIN_ROWS_VALUES * (size_t)N) {
+        } else if (N && ordered && !in.full_cols && tree_smem <= BIN_ROWS_SMEM && N >= BIN_ROWS_FROM && nnz >= BIN_ROWS_VALUES * (size_t)N) {
             allow_shared(k_bin_rows, BIN_ROWS_SMEM);
             TGBM_CUDA(cudaMemsetAsync(bins.p, MISSING_BIN, bins.bytes(), stream));
             k_bin_rows<<<std::min(ceil_div(N, 32), num_sms), 1024, tree_smem, stream>>>(in.row_ptr.p, in.col.p, in.val.p, N, F, cut_ptr.p, cut_val.p, Fpad, bins.p);
