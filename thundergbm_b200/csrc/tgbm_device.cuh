@@ -4,6 +4,7 @@
 #include <cstdint>
 
 #include "tgbm_common.h"
+#include "tgbm_steps.h"
 
 namespace tgbm {
 

@@ -194,8 +194,7 @@ k_hist_sparse_f32(int level, const Batch b, const int *__restrict__ row_ptr, con
             const int p = begin + q;
             const int r = GATHER ? rec_idx[p] : p;
             const float2 v = gh[r];
-            const int j1 = row_ptr[r + 1];
-            for (int j = row_ptr[r] + lane; j < j1; j += 32) red_add_gh(dst + (size_t)bin[j] * cell_stride, v.x, v.y);
+            each_step(row_ptr[r], row_ptr[r + 1], lane, 32, [&](unsigned j) { red_add_gh(dst + (size_t)bin[j] * cell_stride, v.x, v.y); });
         }
     }
 }

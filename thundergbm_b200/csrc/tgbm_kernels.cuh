@@ -292,14 +292,14 @@ k_bin_rows(const int *__restrict__ row_ptr, const int *__restrict__ col, const f
         const int j1 = row_ptr[r + 1];
         int last = -1;   // column before the window
         bool ascend = true;
-        for (int j0 = row_ptr[r]; j0 < j1; j0 += 32 * U) {   // (the same in the whole warp)
+        each_step(row_ptr[r], j1, 0, 32 * U, [&](unsigned j0) {   // (the same in the whole warp)
             int c[U];
             float v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int j = j0 + 32 * u + lane;
-                c[u] = j < j1 ? col[j] : INT_MAX;
-                v[u] = j < j1 ? val[j] : 0.f;
+                const unsigned j = j0 + 32 * u + lane;
+                c[u] = j < (unsigned)j1 ? col[j] : INT_MAX;
+                v[u] = j < (unsigned)j1 ? val[j] : 0.f;
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -316,7 +316,7 @@ k_bin_rows(const int *__restrict__ row_ptr, const int *__restrict__ col, const f
                 }
                 if (mine) bins[(size_t)r * Fpad + c[u]] = b;
             }
-        }
+        });
     }
 }
 // bins [row][feature] -> binsT [feature][row], to the end of the padded rows; a block transposes 128 rows of 32 features
@@ -411,7 +411,7 @@ static __global__ void k_rows_repeat(const int *__restrict__ row_ptr, const int 
     const int lane = threadIdx.x & 31;
     for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rows; r += (gridDim.x * blockDim.x) >> 5) {
         bool bad = false;
-        for (int i = row_ptr[r] + 1 + lane; i < row_ptr[r + 1]; i += 32) bad |= cut_fid[bin[i - 1]] == cut_fid[bin[i]];
+        each_step(row_ptr[r], row_ptr[r + 1], 1 + lane, 32, [&](unsigned i) { bad |= cut_fid[bin[i - 1]] == cut_fid[bin[i]]; });
         if (bad) *flag = 1;
     }
 }
@@ -419,7 +419,7 @@ static __global__ void k_rows_repeat(const int *__restrict__ row_ptr, const int 
 static __global__ void k_value_rows(const int *__restrict__ row_ptr, int n_rows, int *__restrict__ out) {
     const int lane = threadIdx.x & 31;
     for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rows; r += (gridDim.x * blockDim.x) >> 5)
-        for (int j = row_ptr[r] + lane, j1 = row_ptr[r + 1]; j < j1; j += 32) out[j] = r;
+        each_step(row_ptr[r], row_ptr[r + 1], lane, 32, [&](unsigned j) { out[j] = r; });
 }
 // bin_ptr[x] = first of the sorted bin ids that is x or larger
 static __global__ void k_bin_starts(const int *__restrict__ bin, int n, int n_bins, int *__restrict__ bin_ptr) {

@@ -483,13 +483,13 @@ k_hist_sparse(int level, const Batch b, const int *__restrict__ row_ptr, const i
         int2 v, nv, mv;
         meta(q, j0, j1, v);
         meta(q + W, nj0, nj1, nv);
-        int b0 = j0 + lane < j1 ? bin[j0 + lane] : -1;
+        int b0 = lane < j1 - j0 ? bin[j0 + lane] : -1;
         for (; q < last; q += W) {
             meta(q + 2 * W, mj0, mj1, mv);
-            const int nb0 = nj0 + lane < nj1 ? bin[nj0 + lane] : -1;
+            const int nb0 = lane < nj1 - nj0 ? bin[nj0 + lane] : -1;
             int x = b0;
-            for (int j = j0 + lane; j < j1; j += 32) {
-                if (j != j0 + lane) x = bin[j];
+            each_step(j0, j1, lane, 32, [&](unsigned j) {
+                if (j != (unsigned)j0 + lane) x = bin[j];
                 if (x < nsm) {
                     atomicAdd(reinterpret_cast<unsigned *>(sh_sparse + x), (unsigned)v.x & 0xffffu);
                     atomicAdd(reinterpret_cast<unsigned *>(sh_sparse + nsm + x), (unsigned)v.y & 0xffffu);
@@ -499,7 +499,7 @@ k_hist_sparse(int level, const Batch b, const int *__restrict__ row_ptr, const i
                     atomicAdd(dst + 2 * x, (unsigned long long)(long long)v.x);
                     atomicAdd(dst + 2 * x + 1, (unsigned long long)(long long)v.y);
                 }
-            }
+            });
             j0 = nj0; j1 = nj1; v = nv; b0 = nb0;
             nj0 = mj0; nj1 = mj1; nv = mv;
         }
@@ -543,14 +543,14 @@ k_hist_columns(const Batch b, const SparseColumns c, int nnz) {
             g = h = 0;
         };
         constexpr int U = 4;   // windows of 32 values in flight
-        for (int e0 = (int)run; e0 < end; e0 += 32 * U) {
+        each_step((int)run, end, 0, 32 * U, [&](unsigned e0) {
             int x[U], r[U];
             int2 v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int e = e0 + 32 * u + lane;
-                x[u] = e < end ? c.bin[e] : -1;
-                r[u] = e < end ? c.row[e] : -1;
+                const unsigned e = e0 + 32 * u + lane;
+                x[u] = e < (unsigned)end ? c.bin[e] : -1;
+                r[u] = e < (unsigned)end ? c.row[e] : -1;
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) v[u] = r[u] >= 0 ? gh[r[u]] : make_int2(0, 0);
@@ -574,7 +574,7 @@ k_hist_columns(const Batch b, const SparseColumns c, int nnz) {
                     left &= ~__ballot_sync(0xffffffffu, mine);
                 }
             }
-        }
+        });
         hand_over();
     }
 }
@@ -1110,12 +1110,12 @@ k_assign_stored(int level, const Batch b, const SparseColumns c, const int *__re
         const int2 span = make_int2(cut_ptr[nd.split_feature_id], cut_ptr[nd.split_feature_id + 1]);
         if (!by_column(c.bin_ptr, span, b.seg_cnt[level & 1][tree * b.seg_stride + n])) continue;
         // bins below the split bin go left (rev: those beyond it, the split bin itself goes right)
-        const int split = c.bin_ptr[span.x + nd.split_bid + (rev ? 1 : 0)], end = c.bin_ptr[span.y];
+        const unsigned split = c.bin_ptr[span.x + nd.split_bid + (rev ? 1 : 0)];
         const unsigned short me = (unsigned short)(nl - 1 + n), left = (unsigned short)(2 * me + 1), right = (unsigned short)(2 * me + 2);
-        for (int e = c.bin_ptr[span.x] + blockIdx.x * 256 + threadIdx.x; e < end; e += gridDim.x * 256) {
+        each_step(c.bin_ptr[span.x], c.bin_ptr[span.y], blockIdx.x * 256 + threadIdx.x, gridDim.x * 256, [&](unsigned e) {
             const int r = c.row[e];
             if (nid[r] == me) nid[r] = (e < split) != (rev != 0) ? left : right;
-        }
+        });
     }
 }
 
