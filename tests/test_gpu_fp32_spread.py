@@ -157,3 +157,30 @@ def test_first_round_of_several_trees(gpu, monkeypatch, classes, features, depth
             rows = _rows_below(nid[k], node, depth)
             assert abs(trees[k]['sum_g'][node] - g[k][rows].sum()) <= noise_g * (depth + 1)
             assert abs(trees[k]['sum_h'][node] - h * rows.sum()) <= noise_h * (depth + 1)
+
+
+# rows to their children in row order: every block's place in a child's list from the rows of the blocks before, added up by the block
+# or, from 8192 (block, child) pairs on, by a pass of its own; the last level's children of 9 blocks are on that side, those of 8 at it
+@pytest.mark.parametrize('n', [8192, 9001])
+@pytest.mark.parametrize('layout', ['dense', 'sparse'])
+def test_row_lists_of_many_children(gpu, monkeypatch, n, layout):
+    from thundergbm_b200.booster import Booster
+    monkeypatch.setenv('TGBM_LAYOUT', layout)
+    depth, classes, r = 12, 3, np.random.default_rng(n)
+    x = r.integers(1, 120, (n, 6))
+    y = r.integers(0, classes, n)
+    b = Booster(_csr(x, r.random((n, 6)) < 0.9, y), hist_mode='fp32', keep_nid=1, depth=depth, n_trees=1, max_num_bin=255, learning_rate=1.0,
+                objective='multi:softmax', num_class=classes, min_child_weight=0.0, gamma=0.0)
+    b.boost(1)
+    trees, nid = b.trees()[0], b.nid().reshape(classes, n)
+    b.close()
+    h = 2 / classes * (1 - 1 / classes)
+    for k in range(classes):
+        valid = trees[k]['is_valid'] != 0
+        assert valid[1023:2047].sum() > 100 and valid[2047:4095].sum() > 100   # (it is as deep as it is meant to be)
+        _, noise = sum_noise(np.stack([np.zeros(n), np.full(n, h)], 1), n // 50)   # of one level; inherited by the levels below
+        rows = np.zeros(valid.size)
+        np.add.at(rows, nid[k], 1)
+        for node in range(valid.size // 2 - 1, -1, -1):   # the rows of the children were the node's
+            rows[node] += rows[2 * node + 1] + rows[2 * node + 2]
+        assert rows[0] == n and np.abs(trees[k]['sum_h'][valid] - h * rows[valid]).max() <= noise * (depth + 1) < h / 2

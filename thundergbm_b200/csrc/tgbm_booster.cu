@@ -1369,8 +1369,15 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
                              sp_bin.p, cut_ptr.p, columns(), colb, order, assign_table.p);
                 ++launches;
             };
-            if (float_sums) { assign(ASSIGN_COUNT); assign(ASSIGN_PLACE); }
-            else assign(ASSIGN_ANY);
+            if (float_sums) {
+                const bool add = 2ll * nl * assign_ctas <= ASSIGN_ADD;
+                assign(ASSIGN_COUNT);
+                if (!add) {
+                    launch_after(k_assign_before, dim3(ceil_div(2 * nl, 32), 1, n_trees), 1024, 0, stream, assign_ctas, 2 * nl, assign_table.p);
+                    ++launches;
+                }
+                assign(add ? ASSIGN_PLACE_ADD : ASSIGN_PLACE);
+            } else assign(ASSIGN_ANY);
         });
     }
     if (!one_launch) launch_after(k_prune, n_trees, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream, nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0,

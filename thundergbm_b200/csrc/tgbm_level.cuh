@@ -1082,11 +1082,11 @@ __device__ __forceinline__ unsigned csr_bin(const int *__restrict__ row_ptr, con
 // bins are on their way while a chunk is ranked.
 // order: ASSIGN_ANY as above.  The float rounds keep the lists in row order, as what their sums come to depends on it (with lists in
 // order to the chunk only, 7 % of trainings of 100 k rows fell on the other side of a near-tie that row order decides one
-// way): two launches, ASSIGN_COUNT leaves the children's rows of every block's run of chunks in `table` ([blocks][2 nl] a tree),
-// ASSIGN_PLACE starts from the rows of the blocks before.
+// way): ASSIGN_COUNT leaves the children's rows of every block's run of chunks in `table` ([blocks][2 nl] a tree), ASSIGN_PLACE
+// starts from those of the blocks before, which it adds up (ASSIGN_PLACE_ADD) or finds there (k_assign_before has been).
 // BITS: 1 to 3, the levels whose children (2^BITS) are few, ranked by ballots and one shared atomic per warp and child;
 // 0: many children, one shared atomic per row, the lanes seldom meet.
-enum AssignOrder { ASSIGN_ANY = 0, ASSIGN_COUNT = 1, ASSIGN_PLACE = 2 };
+enum AssignOrder { ASSIGN_ANY = 0, ASSIGN_COUNT = 1, ASSIGN_PLACE = 2, ASSIGN_PLACE_ADD = 3 };
 struct alignas(16) ChunkRule {
     union {
         const unsigned char *col;   // dense: bins of the feature by row
@@ -1119,11 +1119,40 @@ k_assign_stored(int level, const Batch b, const SparseColumns c, const int *__re
     }
 }
 
+// Row counts of the blocks -> those of the blocks before, child by child.  A block takes 32 children, a warp 1/32 of the table's
+// rows of them.  Its 9 us (888 blocks) are latency.  Up to ASSIGN_ADD entries of the table every block of ASSIGN_PLACE_ADD adds up the
+// rows before its own instead, which reads half of the table per block: 888 blocks with 8 children 2 us, with 16 and 32 30 on average,
+// with 2048 6.4 ms.  grid = (children / 32, 1, trees)
+constexpr int ASSIGN_ADD = 8192;
+static __global__ void __launch_bounds__(1024)
+k_assign_before(int blocks, int children, int *table) {
+    chain_wait();
+    __shared__ int part[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane, run = (blocks + 31) / 32;
+    const int k0 = min(blocks, warp * run), k1 = min(blocks, k0 + run);
+    int *at = table + (size_t)blockIdx.z * blocks * children + c;
+    int sum = 0;
+    if (c < children)
+#pragma unroll 8
+        for (int k = k0; k < k1; ++k) sum += at[(size_t)k * children];
+    part[warp][lane] = sum;
+    __syncthreads();
+    if (c >= children) return;
+    int before = 0;
+    for (int w = 0; w < warp; ++w) before += part[w][lane];
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) {
+        const int n = at[(size_t)k * children];
+        at[(size_t)k * children] = before;
+        before += n;
+    }
+}
+
 template <bool SPARSE, int RPT, int BITS, bool ORDERED>
 static __global__ void __launch_bounds__(ASSIGN_THREADS, SPARSE || RPT == 8 ? 4 : 6)
 k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__ binsT, size_t Npad, const int *__restrict__ sp_row_ptr,
          const int *__restrict__ sp_bin, const int *__restrict__ cut_ptr, const SparseColumns cols, int rev, int how, int *table) {
-    const int order = ORDERED ? how : (int)ASSIGN_ANY;
+    const int order = !ORDERED ? (int)ASSIGN_ANY : how == ASSIGN_PLACE_ADD ? (int)ASSIGN_PLACE : how;
     constexpr int ROWS = RPT * ASSIGN_THREADS;   // at most 8192: 13 bits of a staged entry
     extern __shared__ __align__(16) unsigned char assign_sm[];
     __shared__ int scratch[33];
@@ -1168,14 +1197,17 @@ k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__
         x.pad = 0;
         rule[i] = x;
     }
-    table += (tree * gridDim.x) * (size_t)(2 * nl);
-    if (order == ASSIGN_PLACE)   // rows of the blocks before, by child; in s_to from here on: where the child's next rows go
+    // in s_to from here on: where the child's next rows go
+    table += (tree * gridDim.x + blockIdx.x) * (size_t)(2 * nl);
+    if (ORDERED && how == ASSIGN_PLACE_ADD)
         for (int i = threadIdx.x >> 5; i < 2 * nl; i += ASSIGN_THREADS / 32) {
             int before = 0;
-            for (int k = lane; k < (int)blockIdx.x; k += 32) before += table[(size_t)k * (2 * nl) + i];
+            for (int k = lane; k < (int)blockIdx.x; k += 32) before += table[i - (long long)(k + 1) * (2 * nl)];
             before = __reduce_add_sync(0xffffffffu, before);
             if (lane == 0) s_to[i] = next_begin[i] + before;
         }
+    else if (order == ASSIGN_PLACE)
+        for (int i = threadIdx.x; i < 2 * nl; i += ASSIGN_THREADS) s_to[i] = next_begin[i] + table[i];
     if (blockIdx.x == 0 && order != ASSIGN_COUNT) {   // rows that are looked at, for the byte counter
         int rows = 0;
         for (int i = threadIdx.x; i < nl; i += ASSIGN_THREADS) rows += b.seg_cnt[in][tree * b.seg_stride + i];
@@ -1271,7 +1303,7 @@ k_assign(int level, const Batch b, int n_rows, const unsigned char *__restrict__
     if (order == ASSIGN_ANY) return;
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * nl; i += ASSIGN_THREADS) {
-        if (order == ASSIGN_COUNT) table[(size_t)blockIdx.x * (2 * nl) + i] = s_cnt[i];
+        if (order == ASSIGN_COUNT) table[i] = s_cnt[i];
         else if (blockIdx.x == gridDim.x - 1) next_cnt[i] = s_to[i] - next_begin[i];
     }
 }
