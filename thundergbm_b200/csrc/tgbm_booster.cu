@@ -1292,7 +1292,8 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
                 launches += 2;
             } else {
                 const bool items = sizeof(T) == 8 && n_eval_items > 0;
-                launch_after(k_eval<T>, dim3(items ? n_eval_items : F, pairs, n_trees), EVAL_THREADS, 0, stream, level, b, items ? eval_items.p : nullptr, F, B, cut_ptr.p, built, tree_cells, bs, qinfo.p, p.min_child_weight, p.lambda,
+                auto kern = items ? k_eval<T, sizeof(T) == 8> : k_eval<T, false>;
+                launch_after(kern, dim3(items ? n_eval_items : F, pairs, n_trees), EVAL_THREADS, 0, stream, level, b, items ? eval_items.p : nullptr, F, B, cut_ptr.p, built, tree_cells, bs, qinfo.p, p.min_child_weight, p.lambda,
                              cut_val.p, p.rt_eps, ignored_all.p, rstate.p, colb, by_hessian, keep);
                 ++launches;
             }

@@ -715,7 +715,8 @@ k_best_apply(int level, const Batch b, int F, const int *__restrict__ cut_ptr, f
 // (hist_tree_builder_single.cu:257-347 for the root, :538-540 and :614-704 for sibling pairs), then, by the block that
 // finishes a pair last (`ticket`, left at zero), the choice among the features and the tree update of the pair's nodes.
 // grid = (items, pairs, trees), an item is a feature or, of features of up to EVAL_SMALL bins, four, a warp each (`items`: the
-// features, -2 behind a single one, -1 for a warp without; null: an item per feature; one-hot columns have one or two bins, and
+// features, -2 behind a single one, -1 for a warp without; PACKED = false: an item per feature, in a kernel of its own, as asking
+// costs: 390 -> 367 us for the last level of 300 k rows x 28, depth 14; one-hot columns have one or two bins, and
 // a block each made 24 k blocks of a level of seven trees: 109 us, 44 of 54 columns with two bins); a thread owns two bins of both
 // children.  The gains are the work of this kernel -- four IEEE
 // divisions per bin and child -- and its time is latency: few bins per thread keep a block's chain short, few threads per
@@ -732,7 +733,7 @@ constexpr int EVAL_THREADS = 128, EVAL_BINS = 2, EVAL_SMALL = 32 * EVAL_BINS;
 template <typename T> struct CellPair;
 template <> struct CellPair<long long> { typedef longlong2 type; };
 template <> struct CellPair<float> { typedef float2 type; };
-template <typename T>
+template <typename T, bool PACKED>
 static __global__ void __launch_bounds__(EVAL_THREADS, 8)
 k_eval(int level, const Batch b, const int4 *__restrict__ items, int F, int B, const int *__restrict__ cut_ptr, T *built_all, size_t tree_cells, int bs,
        const QuantInfo *q, float mcw, float lam, const float *__restrict__ cut_val, float rt_eps,
@@ -742,8 +743,8 @@ k_eval(int level, const Batch b, const int4 *__restrict__ items, int F, int B, c
     __shared__ T s_sum[4][sizeof(T) == 4 ? 32 : WARPS];
     __shared__ unsigned long long s_key[2][WARPS];
     const int j = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int4 item = sizeof(T) == 8 && items ? items[blockIdx.x] : make_int4(blockIdx.x, -2, -2, -2);
-    const bool packed = sizeof(T) == 8 && item.y != -2;
+    const int4 item = PACKED ? items[blockIdx.x] : make_int4(blockIdx.x, -2, -2, -2);
+    const bool packed = PACKED && item.y != -2;
     const int f = !packed || warp == 0 ? item.x : warp == 1 ? item.y : warp == 2 ? item.z : item.w, i0 = (packed ? lane : (int)threadIdx.x) * NB;
     const size_t tree = blockIdx.z;
     TreeNode *nodes = b.nodes + tree * b.nodes_stride;
