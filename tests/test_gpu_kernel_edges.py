@@ -415,3 +415,27 @@ def test_rankings_of_different_group_sizes_side_by_side(gpu, orc):
         x.boost(2)
         assert x.trees().tobytes() == orc.train(d, hist_mode=1, keep_nid=0, **p).trees.tobytes()
         x.close()
+
+
+def _profiled(d, rounds, **p):
+    from thundergbm_b200.booster import Booster
+    b = Booster(d, n_trees=rounds, objective='reg:linear', **p)
+    b.set_profile(True)
+    b.boost(rounds)
+    got = b.profile()
+    b.close()
+    return got
+
+
+# what the counters call the bytes of a row: one per column, or per group of columns that share it
+def test_bytes_of_the_profile(gpu):
+    n, r = 40_000, np.random.default_rng(2)
+    x, keep = np.zeros((n, 62), np.float32), np.zeros((n, 62), bool)
+    of = r.integers(0, 60, n)
+    x[np.arange(n), of] = 1
+    keep[np.arange(n), of] = True
+    x[:, 60:] = r.integers(1, 200, (n, 2))
+    keep[:, 60:] = True
+    d = _holes(x, of % 7 + r.random(n), keep)
+    assert _profiled(d, 2, depth=3).hist_root_bytes == 2 * n * (3 + 8)          # sixty share one, two have their own
+    assert _profiled(_csr(x[:, 55:], d.y), 2, depth=3).hist_root_bytes == 2 * n * (7 + 8)

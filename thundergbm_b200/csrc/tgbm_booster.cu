@@ -1588,9 +1588,9 @@ HistProfile Booster::profile() {
     r = m.profile_acc;
     TreeCtl c;
     TGBM_CUDA(cudaMemcpy(&c, m.ctl.p, sizeof(c), cudaMemcpyDeviceToHost));
-    // algorithmic bytes: rows * (F bin bytes + 8 gradient bytes [+ 4 row index]) + histograms * B * 16 written
-    // per row: its bin ids (F bytes dense; 4 bytes per stored value + a row pointer in the CSR layout), 8 gradient bytes
-    const double row_bytes = m.sparse ? 4.0 * (double)m.nnz_local / std::max(1, m.N) + 4.0 : (double)m.F;
+    // algorithmic bytes: rows * (bin bytes + 8 gradient bytes [+ 4 row index]) + histograms * B * 16 written
+    // bin bytes of a row: a byte per slot (S: a feature, or several that share it) dense; 4 per stored value + a row pointer in the CSR layout
+    const double row_bytes = m.sparse ? 4.0 * (double)m.nnz_local / std::max(1, m.N) + 4.0 : (double)m.S;
     const TreeCtl &c0 = m.stat_base;
     r.hist_root_bytes = (double)(c.stat_rows_root - c0.stat_rows_root) * (row_bytes + 8);
     r.hist_bytes = r.hist_root_bytes + (double)(c.stat_rows_gather - c0.stat_rows_gather) * (row_bytes + 8 + 4) +
