@@ -439,3 +439,13 @@ def test_bytes_of_the_profile(gpu):
     d = _holes(x, of % 7 + r.random(n), keep)
     assert _profiled(d, 2, depth=3).hist_root_bytes == 2 * n * (3 + 8)          # sixty share one, two have their own
     assert _profiled(_csr(x[:, 55:], d.y), 2, depth=3).hist_root_bytes == 2 * n * (7 + 8)
+
+
+# launches that move rows: one a level but the last; two, and a third for many children, in float rounds; of the CSR layout with its
+# values by column one more at every level
+@pytest.mark.parametrize('layout,mode,trees,each', [('dense', 'exact', 10, [1, 1, 1, 0]), ('dense', 'fp32', 1, [2, 2, 2, 0]), ('sparse', 'exact', 9, [1, 1, 1, 0]),
+                                                    ('sparse', 'exact', 10, [2, 2, 2, 1])])
+def test_launches_of_the_profile(gpu, monkeypatch, layout, mode, trees, each):
+    monkeypatch.setenv('TGBM_LAYOUT', layout)
+    got = _profiled(_data(33_000, 5, 1, 3), trees, depth=4, hist_mode=mode)
+    assert got.partition_launches == trees * sum(each) and got.partition_ms > 0 and got.kernel_launches > got.partition_launches + got.hist_launches

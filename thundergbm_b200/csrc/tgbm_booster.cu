@@ -135,7 +135,7 @@ struct BoosterImpl {
     DevBuf<double> metric_partial, metric_sum;
     RankState rank;
 
-    struct TimedEvent { cudaEvent_t a, b; int kind; };
+    struct TimedEvent { cudaEvent_t a, b; int kind; long long launches; };
     std::vector<TimedEvent> events;
     HistProfile profile_acc;  // kernel times of the events already read and destroyed
     long long launches = 0;
@@ -1305,7 +1305,9 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
                 ev.kind = kind;
                 cudaEventRecord(ev.a, stream);
             }
+            const long long before = launches;
             work();
+            ev.launches = launches - before;
             if (profile_on) { cudaEventRecord(ev.b, stream); events.push_back(ev); }
         };
         if (float_sums) {
@@ -1358,13 +1360,15 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
             evaluate(hist_built.p, b.built_stride, 1);
         }
         // -- rows to their children (after the last level k_apply_tree does it)
-        if (sparse && col_ptr.p) {
-            const int node_blocks = std::min(nl, 1024);
-            launch_after(k_assign_stored, dim3(std::max(1, num_sms * 8 / (node_blocks * n_trees)), node_blocks, n_trees), 256, 0, stream, level, b, columns(), cut_ptr.p, colb);
-            ++launches;
-        }
-        if (level == depth - 1) break;
+        const bool by_columns = sparse && col_ptr.p, last = level == depth - 1;
+        if (last && !by_columns) break;
         timed(2, [&] {
+            if (by_columns) {
+                const int node_blocks = std::min(nl, 1024);
+                launch_after(k_assign_stored, dim3(std::max(1, num_sms * 8 / (node_blocks * n_trees)), node_blocks, n_trees), 256, 0, stream, level, b, columns(), cut_ptr.p, colb);
+                ++launches;
+            }
+            if (last) return;
             auto assign = [&](int order) {
                 launch_after(assign_kernel(level, float_sums), dim3(assign_ctas, 1, n_trees), ASSIGN_THREADS, assign_smem(level, assign_rpt), stream, level, b, N, binsT.p, Npad, sp_row_ptr.p,
                              sp_bin.p, cut_ptr.p, columns(), colb, order, assign_table.p);
@@ -1381,9 +1385,11 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
             } else assign(ASSIGN_ANY);
         });
     }
-    if (!one_launch) launch_after(k_prune, n_trees, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream, nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0,
-                                                                                              model.p, K, k0, rstate.p, leaf_weight.p, leaf_rule.p, b.rule_stride, colb,
-                                   seg_cnt[(depth - 1) & 1].p, b.seg_stride, cut_ptr.p, sparse ? col_ptr.p : nullptr);
+    if (!one_launch) {
+        launch_after(k_prune, n_trees, 1024, prune_in_smem ? sizeof(TreeNode) * (size_t)n_nodes : 0, stream, nodes.p, n_nodes, depth, p.gamma, prune_in_smem ? 1 : 0,
+                     model.p, K, k0, rstate.p, leaf_weight.p, leaf_rule.p, b.rule_stride, colb, seg_cnt[(depth - 1) & 1].p, b.seg_stride, cut_ptr.p, sparse ? col_ptr.p : nullptr);
+        ++launches;
+    }
     if (N) {
         float *yp = ypred.p + (size_t)k0 * N;
         int *nid_out = p.keep_nid ? nid_keep.p + ((size_t)round * K + k0) * N : nullptr;
@@ -1393,9 +1399,9 @@ void BoosterImpl::build_trees(int round, int k0, int n_trees) {
         const dim3 ctas(fuse ? metric_blocks() : std::min(ceil_div(N, 256), num_sms * 8), n_trees);
         launch_after(sparse ? k_apply_tree<true> : k_apply_tree<false>, ctas, 256, 0, stream, b, N, depth - 1, binsT.p, Npad, sp_row_ptr.p, sp_bin.p,
                      cut_ptr.p, p.learning_rate, yp, nid_out, y.p, fuse ? objective : -1, metric_partial.p, maxbits.p, colb);
+        ++launches;
         grad_max_ready = metric_partial_ready = fuse;
     }
-    launches += 2;
 }
 
 void BoosterImpl::round_metric(int round) {
@@ -1572,7 +1578,7 @@ HistProfile Booster::profile() {
     for (auto &e : m.events) {
         float ms = 0;
         cudaEventElapsedTime(&ms, e.a, e.b);
-        if (e.kind == 2) { r.partition_ms += ms; r.partition_launches += 1; }
+        if (e.kind == 2) { r.partition_ms += ms; r.partition_launches += e.launches; }
         else {
             r.hist_ms += ms; r.hist_launches += 1;
             if (e.kind == 0) { r.hist_root_ms += ms; r.hist_root_launches += 1; }
