@@ -322,7 +322,7 @@ k_bin_rows(const int *__restrict__ row_ptr, const int *__restrict__ col, const f
 // bins [row][feature] -> binsT [feature][row], to the end of the padded rows; a block transposes 128 rows of 32 features
 static __global__ void __launch_bounds__(256)
 k_bins_by_column(const unsigned char *__restrict__ bins, int n_rows, int F, int Fpad, size_t Npad, unsigned char *__restrict__ binsT) {
-    __shared__ unsigned char t[32][132];
+    __shared__ __align__(4) unsigned char t[32][132];   // (read four bytes at a time)
     const int f0 = blockIdx.y * 32;
     const size_t r0 = (size_t)blockIdx.x * 128;
     {
