@@ -858,7 +858,8 @@ __device__ inline void prune_tree(TreeNode *sn, int n_nodes, int depth, float ga
     __syncthreads();
 }
 // Does k_assign_stored move the rows of a node that store its split column, bins [span.x, span.y)?  Not if the column is much
-// longer than the node's list: searching the rows' values costs about as much as four entries of the column.
+// longer than the node's list.  Rounds of nine kinds of data with other factors than 4: 0 (always searched) 2 to 28 % longer, 1 up to
+// 4 % longer, 16 between 3 % shorter and 2 % longer, without a limit between 4 % shorter and 7 % longer (popular columns).
 __device__ __forceinline__ bool by_column(const int *bin_ptr, int2 span, int rows) {
     return bin_ptr && (long long)bin_ptr[span.y] - bin_ptr[span.x] <= 4ll * rows;
 }

@@ -518,7 +518,9 @@ struct SparseColumns {
 // sums per bin.  What it costs is the gradients, 8 bytes from anywhere in an array that stays in L2, a 32-byte sector each (popular
 // columns: up to four rows a sector): 36 M values of 1 M rows take 165 us, 5.6 TB/s of L2 sectors.  Row by row (k_hist_sparse) they
 // take 198 us: 181 for the 23 M values that meet in shared memory, where popular columns make the same few cells hot.  Bins of a
-// few values only: two reductions per value as there.  grid = (blocks, 1, trees)
+// few values only: two reductions per value as there.  Against the rows, 20 rounds, ms: 50 k rows x 30 values, two or one to a bin
+// 15.9 and 29.1 (16.3, 29.5), 1 M rows x 10 in 12 k bins 8.7 (9.5), 20 k rows x 40 in 10 k bins 3.6 (3.8), 200 k rows x 40 in 5 k bins,
+// all in shared memory there, 7.5 (7.2).  grid = (blocks, 1, trees)
 constexpr int COLUMN_RUN = 1024;
 static __global__ void __launch_bounds__(256)
 k_hist_columns(const Batch b, const SparseColumns c, int nnz) {
@@ -586,8 +588,6 @@ k_hist_columns(const Batch b, const SparseColumns c, int nnz) {
 template <typename T> __device__ __forceinline__ double cell_inv(const QuantInfo *q, int h);
 template <> __device__ __forceinline__ double cell_inv<long long>(const QuantInfo *q, int h) { return h ? q->inv_sh : q->inv_sg; }
 template <> __device__ __forceinline__ double cell_inv<float>(const QuantInfo *, int) { return 1.0; }
-__device__ __forceinline__ float cell_f(long long v, double inv_scale) { return q2f(v, inv_scale); }
-__device__ __forceinline__ float cell_f(float v, double) { return v; }
 __device__ __forceinline__ float cell_f(long long v, const GridScale &s) { return s(v); }
 __device__ __forceinline__ float cell_f(float v, const GridScale &) { return v; }
 __device__ __forceinline__ long long shfl_up_t(long long v, int d) { return shfl_up_ll(v, d); }
@@ -1038,7 +1038,7 @@ k_eval_chunk(int level, const Batch b_, int n_chunks, int B, const int *__restri
             const int lastb = cut_ptr[f + 1] - 1 - b0;
             const float mg = __fsub_rn(pg, cell_f(sg[warp][lastb], inv_sg)), mh = __fsub_rn(ph, cell_f(sh[warp][lastb], inv_sh));
             float gn, keep_g, keep_h;
-            if (multi) {  // inclusive prefix = right child, see eval_feature
+            if (multi) {  // inclusive prefix = right child, see k_eval
                 const float rg = cell_f(sg[warp][b], inv_sg), rh = cell_f(sh[warp][b], inv_sh);
                 const float gl = fmaxf(0.f, split_gain(parent, pg, ph, rg, rh, mcw, lam));
                 const float rg2 = __fadd_rn(rg, mg), rh2 = __fadd_rn(rh, mh);
@@ -1100,7 +1100,10 @@ __device__ __forceinline__ unsigned csr_bin(const int *__restrict__ row_ptr, con
 // order: ASSIGN_ANY as above.  The float rounds keep the lists in row order, as what their sums come to depends on it (with lists in
 // order to the chunk only, 7 % of trainings of 100 k rows fell on the other side of a near-tie that row order decides one
 // way): ASSIGN_COUNT leaves the children's rows of every block's run of chunks in `table` ([blocks][2 nl] a tree), ASSIGN_PLACE
-// starts from those of the blocks before, which it adds up (ASSIGN_PLACE_ADD) or finds there (k_assign_before has been).
+// starts from those of the blocks before, which it adds up (ASSIGN_PLACE_ADD) or finds there (k_assign_before has been).  1 M rows x 28:
+// 12 to 14 us each of the two, 7 to 10 the one launch of ASSIGN_ANY (counting and scattering records took 7 and 9).
+// RPT: rows per thread; eight where there are enough rows for it (BoosterImpl::assign_rpt).  The upper levels spill: 40 bytes with eight
+// rows (BITS 1 to 3), 48 with four (BITS 2 and 3), of 64 and 40 registers.
 // BITS: 1 to 3, the levels whose children (2^BITS) are few, ranked by ballots and one shared atomic per warp and child;
 // 0: many children, one shared atomic per row, the lanes seldom meet.
 enum AssignOrder { ASSIGN_ANY = 0, ASSIGN_COUNT = 1, ASSIGN_PLACE = 2, ASSIGN_PLACE_ADD = 3 };

@@ -10,7 +10,8 @@
 //
 // Bound by the shared-memory atomics of the rows x own features (four 32-bit halves per value, random banks; 12 k cycles a level
 // for 10000 rows x 2 features a CTA) and by the split search (128 units of 255 bins a tree, 8 k cycles for 32 of them).
-// 10000 rows x 32 features, depth 6: 121 us a tree (level kernels 185), 1605 rows x 119 features: 66 us (165).
+// 10000 rows x 32 features, depth 6: 121 us a tree (level kernels 185), 1605 rows x 119 features: 66 us (165).  64 registers, 88 bytes
+// of them spilled.
 // Same integer sums, gains, tie rules and node records as the level kernels, bit for bit.
 #pragma once
 #include <cooperative_groups.h>
@@ -31,7 +32,7 @@ struct SmallPost {   // a CTA's best candidate of a node: |gain| bits << 32 | (0
 __host__ __device__ constexpr int small_at(int bin) { return bin + (bin >> 3); }
 __host__ __device__ constexpr int small_feature_at(int first_bin, int f) { return small_at(first_bin) + f; }   // f-th feature of a CTA, bins before it
 
-struct SmallPlan {   // sizes fixed by the host (see small_plan in the booster)
+struct SmallPlan {   // sizes fixed by the host (BoosterImpl::plan_small_trees)
     int cluster, feats, bins;   // CTAs per tree, features per CTA, most bins of a CTA
     int cells;                  // words that these take
     int nodes_pass;             // nodes whose histograms are in shared memory at a time
