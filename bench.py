@@ -66,9 +66,9 @@ WORKLOADS = {
            dict(objective='rank:ndcg', depth=8, max_num_bin=255, learning_rate=0.1, **COMMON),
            'mslr-shape 2.27M x 136 f32 in query groups of Poisson(120), rank:ndcg, depth 8, 255 bins, lr 0.1'),
 }
-# dram__bytes_read.sum + dram__bytes_write.sum per launch (mean over a tree) of the histogram kernel of either mode on config 2: ncu at
-# 5 M rows (194 MB, profiles/k_assign_and_apply_higgs_5M_x28.md) times 2.1 (None: no capture of that kernel yet)
-NCU_TRAFFIC_BYTES_PER_LAUNCH = {'exact': 407e6, 'fp32': 407e6}
+# dram__bytes_read.sum + dram__bytes_write.sum per launch (mean over the second tree) of the histogram kernel of either mode on config 2,
+# captured with ncu at these 10.5 M rows (profiles/k_hist_fine_higgs_5M_x28.md)
+NCU_TRAFFIC_BYTES_PER_LAUNCH = {'exact': 423.7e6, 'fp32': 429.4e6}
 
 
 def hist_limiter(mode, csr, pairs_per_s):
