@@ -39,10 +39,10 @@ def _same_as_oracle(orc, d, **p):
     b.close()
 
 
-# one cluster builds the tree up to 32768 rows, the level kernels from there on
+# one cluster builds the tree up to 32768 rows (each of its CTAs moves them for itself up to 4096), the level kernels from there on
 @pytest.mark.parametrize('n,f,depth,classes,extra', [
     (1, 1, 1, 1, {}), (2, 3, 6, 1, {}), (31, 5, 4, 3, {}), (1023, 33, 6, 1, {}), (1025, 130, 9, 1, {}), (8191, 8, 10, 1, {}),
-    (3001, 600, 3, 1, {}), (4097, 17, 6, 7, dict(bagging=1, sample_seed=3)), (5000, 64, 7, 1, dict(column_sampling_rate=0.3, sample_seed=5)),
+    (3001, 600, 3, 1, {}), (4096, 20, 7, 1, {}), (4097, 17, 6, 7, dict(bagging=1, sample_seed=3)), (5000, 64, 7, 1, dict(column_sampling_rate=0.3, sample_seed=5)),
     (32768, 20, 6, 1, {}), (32769, 20, 6, 1, {})])
 def test_small_trees(gpu, orc, n, f, depth, classes, extra):
     d = _data(n, f, classes, n + f)

@@ -173,6 +173,7 @@ struct BoosterImpl {
     void gradient(int round);
     void build_trees(int round, int k0, int n_trees);
     SmallPlan small{};   // cluster > 0: trees of integer rounds are built by k_small_tree
+    auto small_kernel() const { return N <= SMALL_LOCAL ? k_small_tree<true> : k_small_tree<false>; }
     void plan_small_trees();
     void launch_small_trees(int k0, int n_trees);
     void round_metric(int round);
@@ -1213,7 +1214,7 @@ void BoosterImpl::plan_small_trees() {
     pl.cluster = 1;
     while (pl.cluster < 16 && pl.cluster < F) pl.cluster *= 2;
     const int max_nl = 1 << (depth - 1);
-    cudaFuncSetAttribute(k_small_tree, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(small_kernel(), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     for (; pl.cluster >= 1; pl.cluster /= 2) {
         pl.feats = ceil_div(F, pl.cluster);
         pl.bins = 1;
@@ -1222,12 +1223,13 @@ void BoosterImpl::plan_small_trees() {
         const size_t budget = 200 * 1024, fixed = (sizeof(TreeNode) * (size_t)n_nodes + 15) / 16 * 16 + sizeof(SmallPost) * 2 * max_nl + (size_t)(N + 7) / 8 * 16 +
                      4 * (size_t)((max_nl + 3) / 4 * 4) + 4 * (size_t)(pl.feats + 1 + pl.bins) + 64;   // (64: roundings)
         pl.cells = small_feature_at(pl.bins, pl.feats);
+        for (int f = 0; f < F; ++f) pl.most = std::max(pl.most, h_cut_ptr[f + 1] - h_cut_ptr[f]);
         const size_t per_node = 16 * (size_t)pl.cells + sizeof(SplitRec) * pl.feats;
         if (fixed + per_node > budget) return;
         pl.nodes_pass = (int)std::min<size_t>(max_nl, (budget - fixed) / per_node);
         if (max_nl > 8 * pl.nodes_pass) return;   // the rows would be walked over and over
         pl.smem = fixed + per_node * pl.nodes_pass;
-        allow_shared(k_small_tree, budget);
+        allow_shared(small_kernel(), budget);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = pl.cluster; cfg.blockDim = SMALL_THREADS; cfg.dynamicSmemBytes = pl.smem;
         cudaLaunchAttribute attr;
@@ -1235,7 +1237,7 @@ void BoosterImpl::plan_small_trees() {
         attr.val.clusterDim.x = pl.cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
         cfg.attrs = &attr; cfg.numAttrs = 1;
         int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, k_small_tree, &cfg) == cudaSuccess && fit >= 1) {
+        if (cudaOccupancyMaxActiveClusters(&fit, small_kernel(), &cfg) == cudaSuccess && fit >= 1) {
             small = pl;
             return;
         }
@@ -1254,7 +1256,7 @@ void BoosterImpl::launch_small_trees(int k0, int n_trees) {
     cfg.attrs = attr; cfg.numAttrs = 2;
     const int2 *gq = ghq.p + (size_t)k0 * N;
     const unsigned long long *roots = root_sum.p + 2 * (size_t)k0;
-    TGBM_CUDA(cudaLaunchKernelEx(&cfg, k_small_tree, (SmallPlan)small, N, Npad, F, depth, (const unsigned char *)binsT.p, (const int *)cut_ptr.p,
+    TGBM_CUDA(cudaLaunchKernelEx(&cfg, small_kernel(), (SmallPlan)small, N, Npad, F, depth, (const unsigned char *)binsT.p, (const int *)cut_ptr.p,
                                  (const float *)cut_val.p, gq, roots, (const QuantInfo *)qinfo.p, p.min_child_weight, p.lambda, p.rt_eps, p.gamma,
                                  (const unsigned char *)ignored_all.p, (const RoundState *)rstate.p, p.column_shards > 0 ? 1 : 0, nodes.p, model.p, K, k0,
                                  maxbits.p, f32 && k0 == 0 ? K : 0, ctl.p, hist_full.p, bufs.full_stride, nid.p, bufs.nid_stride, leaf_weight.p, leaf_rule.p, bufs.rule_stride));

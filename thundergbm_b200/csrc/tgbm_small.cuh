@@ -10,8 +10,9 @@
 //
 // Bound by the shared-memory atomics of the rows x own features (four 32-bit halves per value, random banks; 12 k cycles a level
 // for 10000 rows x 2 features a CTA) and by the split search (128 units of 255 bins a tree, 8 k cycles for 32 of them).
-// 10000 rows x 32 features, depth 6: 121 us a tree (level kernels 185), 1605 rows x 119 features: 66 us (165).  64 registers, 88 bytes
-// of them spilled.
+// 10000 rows x 32 features, depth 6: 124 us a tree (level kernels 185), 1605 rows x 119 features: 63 us (165).  64 registers, 28 to 32
+// bytes of them spilled.  LOCAL: up to SMALL_LOCAL rows, which every CTA moves for itself; a kernel of its own, as either way of moving
+// rows costs the other 3 % by its registers.
 // Same integer sums, gains, tie rules and node records as the level kernels, bit for bit.
 #pragma once
 #include <cooperative_groups.h>
@@ -21,6 +22,7 @@
 namespace tgbm {
 
 constexpr int SMALL_THREADS = 1024, SMALL_ROWS = 32768;   // most rows
+constexpr int SMALL_LOCAL = 4 * SMALL_THREADS;            // rows that every CTA moves for itself
 
 struct SmallPost {   // a CTA's best candidate of a node: |gain| bits << 32 | (0x7fffffff - feature), 0 = none
     unsigned long long key;
@@ -35,6 +37,7 @@ __host__ __device__ constexpr int small_feature_at(int first_bin, int f) { retur
 struct SmallPlan {   // sizes fixed by the host (BoosterImpl::plan_small_trees)
     int cluster, feats, bins;   // CTAs per tree, features per CTA, most bins of a CTA
     int cells;                  // words that these take
+    int most;                   // most bins of a feature
     int nodes_pass;             // nodes whose histograms are in shared memory at a time
     size_t smem;
 };
@@ -67,14 +70,15 @@ __device__ __forceinline__ void small_sums(const int *cell, int words, int nb, i
     for (int o = 16; o > 0; o >>= 1) { t.g += shfl_xor_ll(t.g, o); t.h += shfl_xor_ll(t.h, o); }
     if (lane == 0) sums[part] = t;
 }
-// (Functions of their own: inlined, their arrays and what the kernel holds meanwhile do not fit 64 registers.)
+// (Of up to four bins a lane in place, 0.4 us a level less than a call; the others are functions of their own: inlined, their arrays and
+// what the kernel holds meanwhile do not fit 64 registers.)
 struct SmallSearch {   // what is the same for all of them
     GridScale inv_sg, inv_sh;
     float mcw, lam;
     int multi, words;
 };
 template <int LANES, int BPL>
-__device__ __noinline__ void small_eval(const SmallSearch &x, const int *cell, int nb, float pg, float ph, int part, int parts, const SmallSums *sums, bool active,
+__device__ __forceinline__ void small_eval(const SmallSearch &x, const int *cell, int nb, float pg, float ph, int part, int parts, const SmallSums *sums, bool active,
                                         SplitRec *out) {
     const GridScale inv_sg = x.inv_sg, inv_sh = x.inv_sh;
     const float mcw = x.mcw, lam = x.lam;
@@ -134,7 +138,14 @@ __device__ __noinline__ void small_eval(const SmallSearch &x, const int *cell, i
     else if (key == top) *out = SplitRec{best, 0x7fffffff - (int)(unsigned)top, keep_g, keep_h, mg, mh, 0.f, 0};
 }
 
+template <int LANES, int BPL>
+__device__ __noinline__ void small_eval_call(const SmallSearch &x, const int *cell, int nb, float pg, float ph, int part, int parts, const SmallSums *sums, bool active,
+                                             SplitRec *out) {
+    small_eval<LANES, BPL>(x, cell, nb, pg, ph, part, parts, sums, active, out);
+}
+
 // grid = trees x plan.cluster, clusters of plan.cluster CTAs
+template <bool LOCAL>
 static __global__ void __launch_bounds__(SMALL_THREADS, 1)
 k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const unsigned char *__restrict__ binsT, const int *__restrict__ cut_ptr,
              const float *__restrict__ cut_val, const int2 *ghq, const unsigned long long *root_sum, const QuantInfo *q, float mcw, float lam,
@@ -143,7 +154,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
              unsigned short *nid, size_t nid_stride, float *weight, AssignRule *rule, size_t rule_stride) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char small_sm[];
-    __shared__ int scratch[33], s_split, s_most;
+    __shared__ int scratch[33], s_split;
     __shared__ __align__(8) unsigned char search_sm[sizeof(SmallSearch)];
     SmallSearch &s_search = *reinterpret_cast<SmallSearch *>(search_sm);
     __shared__ SmallSums s_sums[SMALL_THREADS / 32];
@@ -163,10 +174,6 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
     const int share = (N + plan.cluster - 1) / plan.cluster, share0 = min(N, rank * share), share1 = min(N, share0 + share);   // rows whose node this CTA reports
     for (int r = threadIdx.x; r < N; r += SMALL_THREADS) node_of[r] = 0;
     for (int f = threadIdx.x; f <= plan.feats; f += SMALL_THREADS) s_first[f] = cut_ptr[min(F, f0 + f)] - bin0;
-    for (int i = threadIdx.x; i < plan.bins; i += SMALL_THREADS) s_cut[i] = bin0 + i < cut_ptr[F] ? cut_val[bin0 + i] : 0.f;
-    if (threadIdx.x == 0) s_most = 0;
-    __syncthreads();
-    for (int f = threadIdx.x; f < nf; f += SMALL_THREADS) atomicMax(&s_most, s_first[f + 1] - s_first[f]);
     chain_wait();
     if (blockIdx.x == 0 && threadIdx.x == SMALL_THREADS - 1) next_maxima(root_sum, fine_K, maxbits, ctl);   // (a thread that has nothing else to do yet)
     const int2 *gq = ghq + (size_t)tree * N;
@@ -200,8 +207,12 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
             // -- histograms of nodes n0 .. n0 + here - 1 over the own features
             for (int i = threadIdx.x; i < here * plan.cells; i += SMALL_THREADS) { acc[i] = 0; acc[words + i] = 0; acc[2 * words + i] = 0; acc[3 * words + i] = 0; }
             __syncthreads();
+            if (level == 0)   // (on their way while the rows are added up)
+                for (int i = threadIdx.x; i < s_first[nf]; i += SMALL_THREADS)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(s_cut + i)), "l"(cut_val + bin0 + i) : "memory");
             const int first_node = off + n0;
-            // rows and features in flight per thread: a row's bins are loads that nothing waits for until all are on their way
+            // rows and features in flight per thread.  (Four rows and two features for one or two features: 5 % longer at 5000 rows, 1 %
+            // at 10000; four rows and one for eight features: 4 to 9 % longer)
             auto add = [&](auto rows_c, auto feats_c) {
                 constexpr int U = decltype(rows_c)::value, V = decltype(feats_c)::value;
                 for (int r0 = threadIdx.x; r0 < N; r0 += U * SMALL_THREADS) {
@@ -236,8 +247,9 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
                 }
             };
             if (nf > 2) add(std::integral_constant<int, 2>{}, std::integral_constant<int, 4>{});
-            else add(std::integral_constant<int, 4>{}, std::integral_constant<int, 2>{});
+            else add(std::integral_constant<int, 4>{}, std::integral_constant<int, 1>{});
             __syncthreads();
+            if (level == 0) asm volatile("cp.async.wait_all;" ::: "memory");
             if (level == 0) {   // the root's histogram stays readable (tgbm_booster_get_root_hist)
                 long long *full = hist_full + tree * full_stride;
                 for (int f = warp; f < nf; f += SMALL_THREADS / 32)
@@ -250,18 +262,18 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
             // -- best candidate of every (node, feature): a warp each; eight lanes where no feature has more than eight bins; several
             // warps where there are fewer units than warps (a unit of 255 bins is 15 k cycles for one warp alone; always two bins per lane and
             // four passes per warp were slower, 145 us a tree instead of 121)
-            const int units = here * nf, top_bins = s_most;
-            const int parts = top_bins > 128 && units * 4 <= SMALL_THREADS / 32 ? 4 : top_bins > 128 && units * 2 <= SMALL_THREADS / 32 ? 2 : 1;
-            const int lanes = top_bins <= 8 ? 8 : 32, per_block = SMALL_THREADS / (lanes * parts);
+            const int units = here * nf;
+            const int parts_log = plan.most <= 128 ? 0 : units * 4 <= SMALL_THREADS / 32 ? 2 : units * 2 <= SMALL_THREADS / 32 ? 1 : 0, parts = 1 << parts_log;
+            const int lanes_log = plan.most <= 8 ? 3 : 5;   // (shifts: a division by a variable is 200 cycles in every level's chain)
             auto unit = [&](int u, int &n, int &f, const int *&cell, int &nb) {
-                n = u / nf; f = u - n * nf;
+                n = nf == 1 ? u : u / nf; f = u - n * nf;
                 const int first = s_first[f];
                 nb = s_first[f + 1] - first;
                 cell = acc + n * plan.cells + small_feature_at(first, f);
                 return nodes[off + n0 + n].is_valid && nb > 0 && !(ignored && ignored[f0 + f]);
             };
             if (parts > 1) {   // (all units at once)
-                const int u = warp / parts, part = warp & (parts - 1);
+                const int u = warp >> parts_log, part = warp & (parts - 1);
                 int n = 0, f = 0, nb = 0;
                 const int *cell = acc;
                 const bool active = u < units && unit(u, n, f, cell, nb);
@@ -272,8 +284,8 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
                 __syncthreads();
                 if (active) {
                     const TreeNode &nd = nodes[off + n0 + n];
-                    if (parts == 4) small_eval<32, 2>(s_search, cell, nb, nd.sum_g, nd.sum_h, part, parts, s_sums + u * parts, true, s_parts + warp);
-                    else small_eval<32, 4>(s_search, cell, nb, nd.sum_g, nd.sum_h, part, parts, s_sums + u * parts, true, s_parts + warp);
+                    if (parts == 4) small_eval_call<32, 2>(s_search, cell, nb, nd.sum_g, nd.sum_h, part, parts, s_sums + u * parts, true, s_parts + warp);
+                    else small_eval_call<32, 4>(s_search, cell, nb, nd.sum_g, nd.sum_h, part, parts, s_sums + u * parts, true, s_parts + warp);
                 } else if (lane == 0) s_parts[warp].bin = -1;
                 __syncthreads();
                 for (int x = threadIdx.x; x < units; x += SMALL_THREADS) {   // the earlier part among equals
@@ -285,15 +297,15 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
                     recs[x / nf * plan.feats + x % nf] = best;
                 }
             } else {
-                for (int u0 = 0; u0 < units; u0 += per_block) {
-                    const int u = u0 + (int)threadIdx.x / lanes;
+                for (int u0 = 0; u0 < units; u0 += SMALL_THREADS >> lanes_log) {
+                    const int u = u0 + ((int)threadIdx.x >> lanes_log);
                     int n = 0, f = 0, nb = 0;
                     const int *cell = acc;
                     const bool active = u < units && unit(u, n, f, cell, nb);
                     const TreeNode &nd = nodes[off + n0 + n];
                     SplitRec *out = recs + n * plan.feats + f;
                     const float pg = nd.sum_g, ph = nd.sum_h;
-                    if (lanes == 8) {
+                    if (lanes_log == 3) {
                         if (u < units && !active && (lane & 7) == 0) out->bin = -1;
                         if (__any_sync(0xffffffffu, active)) small_eval<8, 1>(s_search, cell, nb, pg, ph, 0, 1, nullptr, active, out);
                         continue;
@@ -301,7 +313,7 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
                     if (!active) { if (u < units && lane == 0) out->bin = -1; continue; }   // (the same in the whole warp)
                     if (nb <= 32) small_eval<32, 1>(s_search, cell, nb, pg, ph, 0, 1, nullptr, true, out);
                     else if (nb <= 128) small_eval<32, 4>(s_search, cell, nb, pg, ph, 0, 1, nullptr, true, out);
-                    else small_eval<32, 8>(s_search, cell, nb, pg, ph, 0, 1, nullptr, true, out);
+                    else small_eval_call<32, 8>(s_search, cell, nb, pg, ph, 0, 1, nullptr, true, out);
                 }
             }
             __syncthreads();
@@ -351,7 +363,29 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
         }
         __syncthreads();
         if (!s_split || level == depth - 1) break;   // the same in every CTA (k_apply_tree makes the last move)
-        // -- rows to the children: a share of them per CTA, written to the table that the tree leaves behind and read back whole
+        // -- rows to the children.  Few of them: every CTA for itself, four rows a thread (a share each takes as long for 5000 rows and
+        // 1.2 k cycles longer for 200: what it writes has to be seen by the other CTAs)
+        if (LOCAL) {
+            unsigned at[4], sp[4];
+            unsigned char b[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int r = (int)threadIdx.x + u * SMALL_THREADS;
+                at[u] = r < N ? (unsigned)node_of[r] : 0u;
+                sp[u] = r < N && at[u] >= (unsigned)off ? split[at[u] - off] : 0u;   // 0: not split
+                b[u] = sp[u] ? binsT[(size_t)((sp[u] >> 8) & 0x3fffffu) * Npad + r] : (unsigned char)0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (!sp[u]) continue;
+                const unsigned char bid = (unsigned char)sp[u];
+                const bool left = b[u] == MISSING_BIN ? !(sp[u] & 0x40000000u) : (multi ? b[u] > bid : b[u] < bid);
+                node_of[threadIdx.x + u * SMALL_THREADS] = (unsigned short)(2 * at[u] + (left ? 1u : 2u));
+            }
+            __syncthreads();
+            continue;
+        }
+        // More: a share of them per CTA, written to the table that the tree leaves behind and read back whole
         // (every CTA for itself: a warp's 32 rows are in up to 32 nodes, so in as many columns; 10 k cycles a level for 10000 rows)
         for (int r = share0 + (int)threadIdx.x; r < share1; r += SMALL_THREADS) {
             const unsigned at = node_of[r], sp = at >= (unsigned)off ? split[at - off] : 0u;   // 0: not split
@@ -369,9 +403,9 @@ k_small_tree(const SmallPlan plan, int N, size_t Npad, int F, int depth, const u
         __syncthreads();
         moved = true;
     }
-    if (!moved)   // a tree that is its root
-        for (int r = share0 + (int)threadIdx.x; r < share1; r += SMALL_THREADS) my_nid[r] = 0;
     cluster.sync();   // nobody reads this CTA's candidates any more
+    if (!moved)   // moved here, or a tree that is its root
+        for (int r = share0 + (int)threadIdx.x; r < share1; r += SMALL_THREADS) my_nid[r] = node_of[r];
     if (rank != 0) return;
     // -- pruning and the finished tree (k_prune)
     if (threadIdx.x == 0) {
